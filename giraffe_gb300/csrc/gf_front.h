@@ -1,0 +1,121 @@
+// Multifrontal LU of K_AA under a nested-dissection ordering: the plan (host,
+// gf_order.cu), the device data and the launches (gf_front.cu).
+//
+// The graph of K_AA's nodes is split recursively by small vertex separators;
+// every separator (and every leaf) is a supernode, eliminated after the parts
+// it separates.  A supernode's front is the dense matrix over its own DOFs and
+// the DOFs of later supernodes its elimination touches (its boundary).  The
+// fronts form a forest; all fronts of one height are independent, so the
+// factorization is one sequence of launches per height, whatever the number
+// of structures.  For a mesh of m x m squares the dense fronts cost about
+// 20 (m d)^3 flops (d DOFs per grid line and square) and the longest dependent
+// chain is about 3.3 m d pivots, against 2 n kl^2 flops and n pivots of a
+// banded LU.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <vector>
+
+namespace gf {
+
+// One front, column-major: entry (i, j) at F[off + i + j ld], rows and columns
+// 0..s-1 the supernode's own DOFs, s..f-1 its boundary, column f the
+// right-hand side.
+struct Front {
+  int64_t off;
+  int f, s, ld;
+  int slot;    // structure
+  int dof0;    // its first own DOF in the elimination order (batch-wide index)
+  int bnd;     // boundary DOFs (batch-wide elimination positions, ascending): bnd[bnd .. bnd + f - s)
+  int rel;     // the parent's front index of every boundary DOF: rel[rel .. rel + f - s)
+  int parent;  // -1: a root
+};
+
+// Fronts whose whole matrix fits in a CTA's shared memory take one CTA for the
+// elimination (k_mf_small); the others run panel by panel on many.
+constexpr int MF_SMALL = 96;
+constexpr int MF_NB = 32;  // pivots per panel of a large front
+
+// Host schedule of one height.
+struct FrontLevel {
+  int small_off = 0, n_small = 0, small_f = 0;  // list range, largest small front
+  int big_off = 0, n_big = 0;                   // list range, by descending s
+  int big_f = 0;
+  std::vector<int> n_at;                        // large fronts that have panel k
+  std::vector<int> f_at;                        // largest f among them
+  std::vector<int> s_at;                        // largest s among them
+  std::vector<int> ext_off, ext_cnt;            // extend-add jobs of the k-th children
+  int schur_off = 0, schur_cnt = 0;
+};
+struct FrontSchedule {
+  std::vector<FrontLevel> level;
+  int launches = 0;  // of one factorization and solve
+};
+
+// Device arrays; the schedule is host memory owned by the batch.
+struct FrontData {
+  int n_fronts;
+  Front* fronts;
+  int* bnd;
+  int* rel;
+  int* list;        // front ids by height
+  int2* ext_jobs;   // (child front, column block)
+  int2* schur_jobs; // (front, row tile | column tile << 16)
+  int* pos;         // free DOF (batch-wide) -> elimination position (batch-wide)
+  int* dof_front;   // elimination position -> its front
+  int* map;         // [n_shells][729] destination of K_e entries in F, relative to the structure's first front (-1: none)
+  int64_t* base;    // per structure: offset of its fronts in F
+  int64_t* size;    // per structure: doubles of its fronts
+  double* F;
+  double* x;        // solution in the elimination order
+  const FrontSchedule* sched;
+};
+
+}  // namespace gf
+
+namespace gfh {
+
+// Vertices of a symmetric graph with weights (DOFs); the splits are taken
+// across level sets of the scalar fields, the first n_pref of them where those
+// give a separator as small as a surface mesh's.
+struct NdGraph {
+  int n = 0;
+  int n_pref = 0;
+  std::vector<int> ptr, adj, w;
+  std::vector<std::vector<float>> field;
+};
+
+// The fronts of one system of n DOFs; indices relative to the system.
+struct FrontPlan {
+  std::vector<gf::Front> fronts;
+  std::vector<int> bnd, rel, height;
+  std::vector<int> pos;        // DOF -> elimination position
+  std::vector<int> dof_front;  // elimination position -> front
+  int64_t size = 0;            // doubles
+  double flops = 0.0;
+};
+
+// Landmark fields of a graph without coordinates: differences of squared
+// distances to far-apart vertices (linear functions of the position where the
+// graph is a mesh).
+void nd_landmark_fields(NdGraph& g);
+// The plan of a graph whose vertex v holds the DOFs dofs[dptr[v] .. dptr[v + 1]).
+FrontPlan plan_fronts(const NdGraph& g, const std::vector<int>& dptr, const std::vector<int>& dofs);
+
+// Plans of several structures joined into one schedule; device offsets are
+// batch-wide.
+struct FrontBuild {
+  std::vector<gf::Front> fronts;
+  std::vector<int> bnd, rel, list, pos, dof_front;
+  std::vector<int2> ext_jobs, schur_jobs;
+  std::vector<int64_t> base, size;  // per structure (0 for the others)
+  int64_t total = 0;
+  gf::FrontSchedule sched;
+};
+// plans[k] belongs to structure slots[k], whose DOFs start at dof_off[k] of
+// n_dofs; base and size are sized for n_struct.
+void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<int>& slots,
+                 const std::vector<int>& dof_off, int n_struct, int n_dofs, FrontBuild& out);
+
+}  // namespace gfh

@@ -396,13 +396,61 @@ struct StructPlan {
   std::vector<char> node_free;      // chain structures: node fully free
   int nf = 0, kb = 0, kl_nat = 0, wkl = 0;
   bool has_f = false, has_m = false, wide = false, chain = false;
+  FrontPlan fronts;                 // wide structures: the multifrontal LU's plan
   int n_colors = 0, n_scolors = 0;  // set by the fill pass
 };
+
+// The multifrontal plan of a shell structure: the graph of its nodes with free
+// DOFs (adj: node adjacency), split across the nodes' coordinates and, for
+// meshes that those do not unfold, the landmark fields.
+void plan_shell_fronts(const gf_model_desc& m, const std::vector<std::vector<int>>& adj, const std::vector<int>& g6,
+                       StructPlan& P) {
+  const int nn = m.n_nodes;
+  NdGraph G;
+  std::vector<int> id(nn, -1), node, dptr(1, 0), dofs;
+  for (int i = 0; i < nn; ++i) {
+    const size_t before = dofs.size();
+    for (int k = 0; k < 6; ++k)
+      if (g6[6 * i + k] >= 0) dofs.push_back(g6[6 * i + k]);
+    if (dofs.size() == before) continue;
+    id[i] = G.n++;
+    node.push_back(i);
+    dptr.push_back((int)dofs.size());
+    G.w.push_back((int)(dofs.size() - before));
+  }
+  G.ptr.push_back(0);
+  for (int i : node) {
+    for (int j : adj[i])
+      if (id[j] >= 0) G.adj.push_back(id[j]);
+    G.ptr.push_back((int)G.adj.size());
+  }
+  double lo[3], hi[3], ext = 0.0;
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = 1e300;
+    hi[k] = -1e300;
+    for (int i : node) {
+      lo[k] = std::min(lo[k], m.node_xyz[3 * i + k]);
+      hi[k] = std::max(hi[k], m.node_xyz[3 * i + k]);
+    }
+    ext = std::max(ext, hi[k] - lo[k]);
+  }
+  for (int k = 0; k < 3; ++k)
+    if (hi[k] - lo[k] > 1e-3 * ext) {
+      std::vector<float> x;
+      // rounded to steps well below the mesh width, so that the nodes of a
+      // mesh line fall on one value
+      for (int i : node) x.push_back((float)std::rint((m.node_xyz[3 * i + k] - lo[k]) / ext * 65536.0));
+      G.field.push_back(std::move(x));
+    }
+  G.n_pref = (int)G.field.size();
+  nd_landmark_fields(G);
+  P.fronts = plan_fronts(G, dptr, dofs);
+}
 
 // Checks, activation and DOF numbering of one structure (SetGlobalDOFs,
 // reference src/Solution.cpp:40-118), its half-bandwidth and whether it is a
 // chain.
-void plan_structure(const gf_model_desc& m, int s, StructPlan& P) {
+void plan_structure(const gf_model_desc& m, int s, bool want_fronts, StructPlan& P) {
   if (m.solution.type != GF_STATIC && m.solution.type != GF_DYNAMIC) {
     P.err = strf("structure %d: unknown solution type", s);
     return;
@@ -534,6 +582,7 @@ void plan_structure(const gf_model_desc& m, int s, StructPlan& P) {
     P.perm.assign(nf, 0);
     for (int i = 0; i < nn * 6; ++i)
       if (g_nat[i] >= 0) P.perm[g_nat[i]] = g6[i];
+    if (want_fronts) plan_shell_fronts(m, adj, g6, P);
   } else {
     P.dofs.reserve((size_t)nn * 6);
     nf = number(natural, g6, &P.dofs);
@@ -623,7 +672,7 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
   size_t work = 0;
   for (int s = 0; s < n; ++s) work += (size_t)std::max(models[s].n_nodes, 0) + std::max(models[s].n_beams, 0) +
                                       std::max(models[s].n_shells, 0);
-  parallel_structures(n, work, [&](int s) { plan_structure(models[s], s, plan[s]); });
+  parallel_structures(n, work, [&](int s) { plan_structure(models[s], s, !B->band_view, plan[s]); });
   for (int s = 0; s < n; ++s)
     if (!plan[s].err.empty()) {
       set_err(ctx, "%s", plan[s].err.c_str());
@@ -1101,28 +1150,49 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       return GF_ERR_CUDA;
   }
   if (!wide_structs.empty()) {
-    if (!upload(B, &sd.wide_structs, wide_structs) || !balloc(B, &sd.wband, (size_t)wb_total) ||
-        !balloc(B, &sd.panel, 1))
+    const bool mixed = B->opts.precision == GF_PREC_MIXED && !B->band_view;
+    B->wb_total = wb_total;
+    if (!upload(B, &sd.wide_structs, wide_structs) || !balloc(B, &sd.panel, 1) ||
+        ((mixed || B->band_view) && !balloc(B, &sd.wband, (size_t)wb_total)))
       return GF_ERR_CUDA;
-    if (B->opts.precision == GF_PREC_MIXED) {
+    if (!B->band_view) {
+      // the fronts of all structures in one schedule
+      std::vector<const FrontPlan*> plans;
+      std::vector<int> offs;
+      for (int s : wide_structs) {
+        const FrontPlan& F = plan[s].fronts;
+        if (F.size > INT32_MAX) {
+          set_err(ctx, "structure %d: %lld entries of its fronts exceed 32-bit offsets", s, (long long)F.size);
+          return GF_ERR_ARG;
+        }
+        plans.push_back(&F);
+        offs.push_back(dof_offs[s]);
+      }
+      FrontBuild fb;
+      join_fronts(plans, wide_structs, offs, n, dof_off, fb);
+      FrontData& md = sd.mf;
+      md.n_fronts = (int)fb.fronts.size();
+      if (!upload(B, &md.fronts, fb.fronts) || !upload(B, &md.bnd, fb.bnd) || !upload(B, &md.rel, fb.rel) ||
+          !upload(B, &md.list, fb.list) || !upload(B, &md.ext_jobs, fb.ext_jobs) ||
+          !upload(B, &md.schur_jobs, fb.schur_jobs) || !upload(B, &md.pos, fb.pos) ||
+          !upload(B, &md.dof_front, fb.dof_front) || !upload(B, &md.base, fb.base) || !upload(B, &md.size, fb.size) ||
+          !balloc(B, &md.map, (size_t)shell_off * 729) || !balloc(B, &md.F, (size_t)fb.total) ||
+          !balloc(B, &md.x, (size_t)dof_off))
+        return GF_ERR_CUDA;
+      B->sched = std::move(fb.sched);
+      md.sched = &B->sched;
+    }
+    if (mixed) {
       // the FP32 LU beside the FP64 K_AA, its right-hand side and scratch,
       // the saved Newton right-hand side and the refinement state
       if (!balloc(B, &sd.wband32, (size_t)wb_total) || !balloc(B, &sd.r32, (size_t)dof_off) ||
           !balloc(B, &sd.y32, (size_t)dof_off) || !balloc(B, &sd.ir_rhs, (size_t)dof_off) ||
           !zeroed(B, &sd.ir, wide_structs.size()) || !zeroed(B, &sd.ir_more, 4))
         return GF_ERR_CUDA;
-    }
-    if (B->opts.wide_update == GF_WIDE_TENSOR || B->opts.wide_update == GF_WIDE_TENSOR_SYNC) {
-      // slices of one panel per wide structure for the tensor-core update
-      sd.oz_rows = (max_wkl + 127) / 128 * 128;  // whole 128-row tiles of the tensor-core update
-      const size_t nw = wide_structs.size(), R = (size_t)sd.oz_rows;
-      if (!zeroed(B, &sd.oz_slices, nw * 2 * 8 * R * GF_WB_NB) || !balloc(B, &sd.oz_exp, nw * 2 * R) ||
-          !zeroed(B, &sd.oz_kmax, nw * 2 * 2 * GF_WB_NB) || !zeroed(B, &sd.oz_error, 1))
-        return GF_ERR_CUDA;
-    }
-    if (!B->count_only) {
-      for (auto& a : sd.aux) CK(cudaStreamCreateWithFlags(&a, cudaStreamNonBlocking));
-      for (auto& e : sd.evt) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      if (!B->count_only) {
+        for (auto& a : sd.aux) CK(cudaStreamCreateWithFlags(&a, cudaStreamNonBlocking));
+        for (auto& e : sd.evt) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      }
     }
   }
   // device arrays
@@ -1176,19 +1246,21 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
   CK(cudaMemsetAsync(b.nodeK, 0, sizeof(double) * (size_t)std::max(node_off, 1) * 9, B->stream));
   b.mixed = B->opts.precision == GF_PREC_MIXED;
   b.sh.ir_max = B->opts.max_refine > 0 ? B->opts.max_refine : GF_IR_MAX;
-  b.sh.wide_tc = b.sh.oz_slices != nullptr ? B->opts.wide_update : GF_WIDE_FP64;
+  b.sh.wide_tc = GF_WIDE_FP64;  // the mixed path's factor is FP32
   if (b.sh.n_wide) {
     // tile shapes: the caller's entries, the others from the autotuner
     // (served waves, whose device memory comes from the server's budget,
     // take the defaults rather than time a synthetic band beside it)
     const int* wt = B->opts.wide_tiles;
     WideTiles t;
-    if (!(wt[0] && wt[1] && wt[2] && wt[3]) && !B->arena) t = tune_wide_tiles(B->ctx, b.sh.max_kl, b.sh.wide_tc);
+    if (!(wt[0] && wt[1] && wt[2] && wt[3]) && !B->arena && b.sh.wband32) t = tune_wide_tiles(B->ctx, b.sh.max_kl, b.sh.wide_tc);
     if (wt[0]) t.trsm_rb = wt[0];
     if (wt[1]) t.trsm_first = wt[1];
     if (wt[2]) t.corner = wt[2];
     if (wt[3]) t.sub_rows = wt[3];
     b.sh.tiles = t;
+    if (b.sh.mf.sched) launch_front_map(b, B->stream);
+    CK(cudaGetLastError());
   }
   return GF_OK;
 }
@@ -1239,6 +1311,34 @@ int batch_reset(gf_batch* B) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
+namespace gfh {
+gf_batch* create_batch(gf_ctx* ctx, int n, const gf_model_desc* models, const gf_solve_opts* opts, bool band_view) {
+  if (!ctx || n <= 0 || !models) {
+    set_err(ctx, "gf_batch_create: invalid arguments");
+    return nullptr;
+  }
+  cudaSetDevice(ctx->device);
+  gf_batch* B = new gf_batch();
+  B->ctx = ctx;
+  B->stream = ctx->stream;
+  B->band_view = band_view;
+  if (opts) B->opts = *opts; else gf_default_opts(&B->opts);
+  if (B->opts.poll_every <= 0) B->opts.poll_every = 8;
+  NvtxRange range("gf_batch_create");
+  const double t0 = host_now_ms();
+  if (build_batch(B, n, models) != GF_OK || cudaMallocHost(&B->h_running, sizeof(int)) != cudaSuccess ||
+      cudaEventCreate(&B->ev0) != cudaSuccess || cudaEventCreate(&B->ev1) != cudaSuccess) {
+    std::string e = ctx->err;
+    gf_batch_destroy(B);
+    ctx->err = e.empty() ? "gf_batch_create failed" : e;
+    return nullptr;
+  }
+  B->launches_per_pass = count_launches_per_pass(B);
+  B->host_ms[0] = host_now_ms() - t0 - B->host_ms[1] - B->host_ms[2];
+  return B;
+}
+}  // namespace gfh
+
 extern "C" {
 
 gf_ctx* gf_create(int device) {
@@ -1283,28 +1383,7 @@ void gf_default_opts(gf_solve_opts* o) {
 }
 
 gf_batch* gf_batch_create(gf_ctx* ctx, int n, const gf_model_desc* models, const gf_solve_opts* opts) {
-  if (!ctx || n <= 0 || !models) {
-    set_err(ctx, "gf_batch_create: invalid arguments");
-    return nullptr;
-  }
-  cudaSetDevice(ctx->device);
-  gf_batch* B = new gf_batch();
-  B->ctx = ctx;
-  B->stream = ctx->stream;
-  if (opts) B->opts = *opts; else gf_default_opts(&B->opts);
-  if (B->opts.poll_every <= 0) B->opts.poll_every = 8;
-  NvtxRange range("gf_batch_create");
-  const double t0 = host_now_ms();
-  if (build_batch(B, n, models) != GF_OK || cudaMallocHost(&B->h_running, sizeof(int)) != cudaSuccess ||
-      cudaEventCreate(&B->ev0) != cudaSuccess || cudaEventCreate(&B->ev1) != cudaSuccess) {
-    std::string e = ctx->err;
-    gf_batch_destroy(B);
-    ctx->err = e.empty() ? "gf_batch_create failed" : e;
-    return nullptr;
-  }
-  B->launches_per_pass = count_launches_per_pass(B);
-  B->host_ms[0] = host_now_ms() - t0 - B->host_ms[1] - B->host_ms[2];
-  return B;
+  return gfh::create_batch(ctx, n, models, opts, false);
 }
 
 void gf_batch_destroy(gf_batch* B) {
@@ -1846,6 +1925,8 @@ int first_pass_band(gf_batch* B, int s, std::vector<double>& band, std::vector<d
   const StructInfo& inf = B->info[s];
   int r = batch_reset(B);
   if (r != GF_OK) return r;
+  // the wide band of Shell_1 structures, which their solver does not keep
+  if (b.sh.n_wide && !b.sh.wband && !balloc(B, &B->b.sh.wband, (size_t)B->wb_total)) return GF_ERR_CUDA;
   // one partial pass: step start, zero, mount, loads, residual
   Batch bb = b;
   launch_iteration_partial(bb, B->stream);

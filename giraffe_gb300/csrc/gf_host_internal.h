@@ -132,10 +132,13 @@ struct gf_batch {
   DevArena* arena = nullptr;      // served waves: allocations come from the server's budget
   DevArena* host_stage = nullptr; // served waves: pinned staging for the uploads
   std::vector<void*> staged;      // staging blocks in use until the uploads land
+  bool band_view = false;         // K_AA is read by the caller or the modal analysis, in the band; never solved by the fronts
+  gf::FrontSchedule sched;        // of the multifrontal LU (b.sh.mf points to it)
   bool count_only = false;        // size the batch without touching the device
   size_t counted_bytes = 0;
   // host copies needed for results and resets
   std::vector<gf::StructInfo> info;
+  int64_t wb_total = 0;  // entries of the Shell_1 structures' wide bands
   std::vector<int> kb;  // true half-bandwidth per structure
   std::vector<void*> allocs;
   // initial configuration (device) for gf_batch_reset
@@ -197,6 +200,8 @@ bool set_err(gf_ctx* ctx, const char* fmt, ...);
 // Builds the device batch of n structures (or, with B->count_only, only
 // counts its device bytes).
 int build_batch(gf_batch* B, int n, const gf_model_desc* models);
+// gf_batch_create; band_view: for a caller that reads K_AA instead of solving.
+gf_batch* create_batch(gf_ctx* ctx, int n, const gf_model_desc* models, const gf_solve_opts* opts, bool band_view);
 // Initial configuration and step state, enqueued on B->stream.
 int batch_reset(gf_batch* B);
 // Captures one Newton pass as a CUDA graph on B->stream (opts.use_graph).

@@ -205,7 +205,7 @@ gf_structure* gf_upload_structure(gf_ctx* ctx, const gf_model_desc* model, const
   gf_solve_opts o;
   if (opts) o = *opts; else gf_default_opts(&o);
   o.use_graph = 0;
-  gf_batch* B = gf_batch_create(ctx, 1, model, &o);
+  gf_batch* B = create_batch(ctx, 1, model, &o, true);
   if (!B) return nullptr;
   gf_structure* S = new gf_structure();
   S->ctx = ctx;

@@ -281,7 +281,7 @@ __global__ void k_zero(Batch b) {
   // wide structures: k_wb_zero; chain structures keep no band (nodeK instead)
   const bool chain_only = inf.is_chain && !b.full_band;
   int64_t nb = (inf.wide || chain_only) ? 0 : (int64_t)inf.n_free * GF_LDB;
-  if (inf.is_chain) {
+  if (inf.is_chain || inf.wide) {
     double* nk = b.nodeK + (int64_t)inf.node_off * 9;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < inf.n_nodes * 9; i += gridDim.x * blockDim.x) nk[i] = 0.0;
   }
@@ -754,7 +754,8 @@ __global__ void k_loads(Batch b) {
   double time = st.last_converged_time + st.current_time_step;
   double* P = b.P + inf.dof_off;
   double* band = b.band + inf.band_off;
-  const bool to_nodeK = inf.is_chain && !b.full_band;
+  const bool to_nodeK = (inf.is_chain || inf.wide) && !b.full_band;
+  const bool to_wide = inf.wide && wide_band_filled(b);
   for (int l = inf.load_off; l < inf.load_off + inf.n_loads; ++l) {
     const LoadEntry L = b.loads[l];
     int node = L.node;
@@ -783,8 +784,8 @@ __global__ void k_loads(Batch b) {
         int gj = gl[3 + j];
         if (gi < 0 || gj < 0) continue;
         if (to_nodeK) b.nodeK[(int64_t)node * 9 + i * 3 + j] += -1.0 * V[i * 3 + j];
-        else if (inf.wide) b.sh.wband[inf.wb_off + (inf.wkl + gi - gj) + (int64_t)gj * (2 * inf.wkl + 1)] += -1.0 * V[i * 3 + j];
-        else band[(GF_KB + gi - gj) + (int64_t)gj * GF_LDB] += -1.0 * V[i * 3 + j];
+        if (to_wide) b.sh.wband[inf.wb_off + (inf.wkl + gi - gj) + (int64_t)gj * (2 * inf.wkl + 1)] += -1.0 * V[i * 3 + j];
+        else if (!to_nodeK) band[(GF_KB + gi - gj) + (int64_t)gj * GF_LDB] += -1.0 * V[i * 3 + j];
       }
     }
   }

@@ -72,6 +72,10 @@ struct ProfScope {
   }
 };
 
+// The wide band holds K_AA in the assembly view (gf_batch_assemble, the
+// Newton-iteration boundary) and in the mixed-precision path.
+__host__ __device__ inline bool wide_band_filled(const Batch& b) { return b.full_band || b.sh.wband32; }
+
 void launch_iteration(const Batch& b, cudaStream_t st, bool commit_kernels = true, LaunchProf* prof = nullptr);
 // FMA throughput probe: 8 independent chains per thread, `iters` steps.
 void launch_fp_probe(bool fp64, void* out, int blocks, int threads, int iters, cudaStream_t st);
@@ -107,6 +111,15 @@ void launch_shell_mount(const Batch& b, cudaStream_t st);
 void launch_wide_zero(const Batch& b, cudaStream_t st);
 void launch_wide_solve(const Batch& b, cudaStream_t st, LaunchProf* prof = nullptr);
 void launch_wide_subst(const Batch& b, int nrhs, cudaStream_t st);
+// Multifrontal LU (gf_front.cu): destinations of the element entries (once per
+// batch); assembly of K_AA, factorization and solution of P of the batch's
+// Shell_1 structures; the same on a one-structure batch from a CSR or LAPACK GB
+// matrix on the device; kernel launches of one solve.
+void launch_front_map(const Batch& b, cudaStream_t st);
+void launch_front_solve(const Batch& b, cudaStream_t st, LaunchProf* prof = nullptr);
+void launch_front_csr(const Batch& b, int n, const int* rp, const int* ci, const double* v, cudaStream_t st);
+void launch_front_band(const Batch& b, int n, int kl, int ku, int ldab, const double* ab, cudaStream_t st);
+int front_launches(const Batch& b);
 // The first error of a wide-band capture step (a conditional node or body
 // capture) since the last call on this thread; clears it.
 cudaError_t wide_capture_error();

@@ -1,0 +1,370 @@
+// Nested-dissection ordering and symbolic factorization for the multifrontal
+// LU (gf_front.h): host code.
+#include <algorithm>
+#include <atomic>
+#include <climits>
+#include <numeric>
+#include <thread>
+
+#include "gf_front.h"
+
+namespace gfh {
+
+namespace {
+
+// A part of at most this weight (DOFs) is not split further: below it a split
+// only adds fronts (a 2-element patch of the six-node mesh weighs 6 to 50).
+constexpr int ND_LEAF = 24;
+
+struct Dissection {
+  const NdGraph& g;
+  std::vector<int> perm;            // elimination order
+  std::vector<char> start;          // a supernode starts at this place of perm
+  std::vector<int> label;           // 2 id + side of the part a vertex is in
+  std::atomic<int> next_id{1};
+
+  explicit Dissection(const NdGraph& gr) : g(gr), perm(gr.n), start(gr.n, 0), label(gr.n, 0) {
+    std::iota(perm.begin(), perm.end(), 0);
+  }
+  // labels of other threads' parts are read but never equal the reader's own
+  int lab(int v) const { return __atomic_load_n(&label[v], __ATOMIC_RELAXED); }
+  void set(int v, int l) { __atomic_store_n(&label[v], l, __ATOMIC_RELAXED); }
+
+  // Splits perm[lo, hi) into [part A | part B | separator] and recurses.
+  void split(int lo, int hi, int depth) {
+    const int m = hi - lo;
+    if (m <= 0) return;
+    long long wt = 0;
+    for (int i = lo; i < hi; ++i) wt += g.w[perm[i]];
+    if (m == 1 || wt <= ND_LEAF) {
+      start[lo] = 1;
+      return;
+    }
+    double best = -1.0;
+    int bf = -1, bside = 0, bless = 0;
+    float bt = 0.f;
+    std::vector<float> val(m);
+    auto classify = [&](int f, float t, int less, int id) {
+      const std::vector<float>& x = g.field[f];
+      for (int i = lo; i < hi; ++i) {
+        const float v = x[perm[i]];
+        set(perm[i], 2 * id + ((less ? v < t : v <= t) ? 0 : 1));
+      }
+    };
+    // weights of the two boundary sets under the current labels
+    auto boundary = [&](int id, long long* wb, long long* wp) {
+      wb[0] = wb[1] = wp[0] = wp[1] = 0;
+      for (int i = lo; i < hi; ++i) {
+        const int v = perm[i], l = lab(v), side = l & 1;
+        wp[side] += g.w[v];
+        for (int k = g.ptr[v]; k < g.ptr[v + 1]; ++k)
+          if (lab(g.adj[k]) == (l ^ 1)) {
+            wb[side] += g.w[v];
+            break;
+          }
+      }
+    };
+    for (int f = 0; f < (int)g.field.size(); ++f) {
+      // a mesh of weight wt has separators of about 2 sqrt(wt)
+      if (f >= g.n_pref && best >= 0.0 && best * best < 9.0 * (double)wt) break;
+      const std::vector<float>& x = g.field[f];
+      for (int i = 0; i < m; ++i) val[i] = x[perm[lo + i]];
+      std::nth_element(val.begin(), val.begin() + m / 2, val.end());
+      const float t = val[m / 2];
+      int nl = 0, ne = 0;
+      for (int i = 0; i < m; ++i) {
+        nl += val[i] < t;
+        ne += val[i] == t;
+      }
+      if (ne == m) continue;
+      // the level set of t goes to the side that balances the parts
+      const int less = std::abs(2 * nl - m) <= std::abs(2 * (nl + ne) - m);
+      const int na = less ? nl : nl + ne;
+      if (na == 0 || na == m) continue;
+      const int id = next_id.fetch_add(1);
+      classify(f, t, less, id);
+      long long wb[2], wp[2];
+      boundary(id, wb, wp);
+      for (int side = 0; side < 2; ++side) {
+        const double a = (double)wp[side] - wb[side], b = (double)wp[1 - side];
+        const double imb = std::abs(a - b) / (double)wt;
+        // a smaller separator is worth some imbalance of the parts
+        const double cost = (double)wb[side] * (1.0 + 1.5 * imb * imb) + 1e-3 * imb;
+        if (best < 0.0 || cost < best) {
+          best = cost;
+          bf = f;
+          bt = t;
+          bless = less;
+          bside = side;
+        }
+      }
+    }
+    const int id = next_id.fetch_add(1);
+    if (bf < 0) {
+      // no field tells the vertices apart: halves of the present order
+      for (int i = lo; i < hi; ++i) set(perm[i], 2 * id + (i - lo < m / 2 ? 0 : 1));
+      bside = 0;
+    } else {
+      classify(bf, bt, bless, id);
+    }
+    std::vector<int> a, b, s;
+    for (int i = lo; i < hi; ++i) {
+      const int v = perm[i], l = lab(v), side = l & 1;
+      bool cut = false;
+      if (side == bside)
+        for (int k = g.ptr[v]; k < g.ptr[v + 1] && !cut; ++k) cut = lab(g.adj[k]) == (l ^ 1);
+      (cut ? s : side ? b : a).push_back(v);
+    }
+    if (a.empty() && b.empty()) {  // all of it is separator: one supernode
+      start[lo] = 1;
+      return;
+    }
+    std::copy(a.begin(), a.end(), perm.begin() + lo);
+    std::copy(b.begin(), b.end(), perm.begin() + lo + a.size());
+    std::copy(s.begin(), s.end(), perm.begin() + lo + a.size() + b.size());
+    const int ma = lo + (int)a.size(), mb = ma + (int)b.size();
+    if (!s.empty()) start[mb] = 1;
+    if (depth < 4 && m > 1000) {
+      std::thread t([&] { split(lo, ma, depth + 1); });
+      split(ma, mb, depth + 1);
+      t.join();
+    } else {
+      split(lo, ma, depth + 1);
+      split(ma, mb, depth + 1);
+    }
+  }
+};
+
+// Distances from vertex v0 (n where unreachable); returns the last vertex reached.
+int bfs(const NdGraph& g, int v0, std::vector<int>& dist, std::vector<int>& queue) {
+  std::fill(dist.begin(), dist.end(), g.n);
+  queue.clear();
+  queue.push_back(v0);
+  dist[v0] = 0;
+  for (size_t q = 0; q < queue.size(); ++q) {
+    const int v = queue[q];
+    for (int k = g.ptr[v]; k < g.ptr[v + 1]; ++k)
+      if (dist[g.adj[k]] == g.n) {
+        dist[g.adj[k]] = dist[v] + 1;
+        queue.push_back(g.adj[k]);
+      }
+  }
+  return queue.back();
+}
+
+}  // namespace
+
+void nd_landmark_fields(NdGraph& g) {
+  if (g.n == 0) return;
+  constexpr int L = 4;
+  std::vector<int> queue, d[L], far(g.n, INT_MAX), d0(g.n);
+  int v = bfs(g, bfs(g, 0, d0, queue), d0, queue);
+  for (int l = 0; l < L; ++l) {
+    d[l].resize(g.n);
+    bfs(g, v, d[l], queue);
+    // the next landmark: the vertex farthest from all so far, of those of the
+    // lowest degree (a corner of the mesh)
+    int best = 0;
+    for (int i = 0; i < g.n; ++i) {
+      far[i] = std::min(far[i], d[l][i]);
+      if (far[i] >= g.n) far[i] = -1;  // another component
+      const int deg = g.ptr[i + 1] - g.ptr[i], bd = g.ptr[best + 1] - g.ptr[best];
+      if (far[i] > far[best] || (far[i] == far[best] && deg < bd)) best = i;
+    }
+    v = best;
+  }
+  auto add = [&](auto f) {
+    std::vector<float> x(g.n);
+    for (int i = 0; i < g.n; ++i) x[i] = f(i);
+    g.field.push_back(std::move(x));
+  };
+  auto sq = [&](int l, int i) { return (float)d[l][i] * (float)d[l][i]; };
+  for (int a = 0; a < L; ++a)
+    for (int b = a + 1; b < L; ++b) add([&](int i) { return sq(a, i) - sq(b, i); });
+  add([&](int i) { return sq(0, i) + sq(1, i) - sq(2, i) - sq(3, i); });
+  add([&](int i) { return sq(0, i) + sq(2, i) - sq(1, i) - sq(3, i); });
+  add([&](int i) { return sq(0, i) + sq(3, i) - sq(1, i) - sq(2, i); });
+}
+
+FrontPlan plan_fronts(const NdGraph& g, const std::vector<int>& dptr, const std::vector<int>& dofs) {
+  FrontPlan P;
+  Dissection D(g);
+  D.split(0, g.n, 0);
+  const std::vector<int>& perm = D.perm;
+  std::vector<int> place(g.n), first, node_of(g.n);
+  for (int i = 0; i < g.n; ++i) {
+    place[perm[i]] = i;
+    if (D.start[i]) first.push_back(i);
+    node_of[i] = (int)first.size() - 1;
+  }
+  const int ns = (int)first.size();
+  first.push_back(g.n);
+  // boundary of every supernode (places of vertices, ascending); its parent
+  // holds the first of them
+  std::vector<std::vector<int>> bnd(ns), kids(ns);
+  std::vector<int> mark(g.n, -1), parent(ns, -1);
+  for (int k = 0; k < ns; ++k) {
+    const int end = first[k + 1];
+    std::vector<int>& B = bnd[k];
+    auto take = [&](int p) {
+      if (p >= end && mark[p] != k) {
+        mark[p] = k;
+        B.push_back(p);
+      }
+    };
+    for (int i = first[k]; i < end; ++i)
+      for (int q = g.ptr[perm[i]]; q < g.ptr[perm[i] + 1]; ++q) take(place[g.adj[q]]);
+    for (int c : kids[k])
+      for (int p : bnd[c]) take(p);
+    std::sort(B.begin(), B.end());
+    if (!B.empty()) {
+      parent[k] = node_of[B[0]];
+      kids[parent[k]].push_back(k);
+    }
+  }
+  // DOFs: elimination positions by place, then the fronts
+  const int nd = (int)dofs.size();
+  std::vector<int> dpos(g.n + 1, 0);  // first elimination position of a place
+  for (int i = 0; i < g.n; ++i) dpos[i + 1] = dpos[i] + dptr[perm[i] + 1] - dptr[perm[i]];
+  P.pos.assign(nd, -1);
+  P.dof_front.assign(nd, -1);
+  for (int i = 0; i < g.n; ++i)
+    for (int q = dptr[perm[i]], p = dpos[i]; q < dptr[perm[i] + 1]; ++q, ++p) P.pos[dofs[q]] = p;
+  P.fronts.resize(ns);
+  P.height.assign(ns, 0);
+  for (int k = 0; k < ns; ++k) {
+    gf::Front& F = P.fronts[k];
+    F.s = dpos[first[k + 1]] - dpos[first[k]];
+    F.dof0 = dpos[first[k]];
+    F.bnd = (int)P.bnd.size();
+    F.parent = parent[k];
+    F.slot = 0;
+    for (int p : bnd[k])
+      for (int d = dpos[p]; d < dpos[p + 1]; ++d) P.bnd.push_back(d);
+    F.f = F.s + (int)P.bnd.size() - F.bnd;
+    F.ld = (F.f + 1) & ~1;
+    F.off = P.size;
+    P.size += ((int64_t)F.ld * (F.f + 1) + 31) / 32 * 32;
+    for (int d = F.dof0; d < F.dof0 + F.s; ++d) P.dof_front[d] = k;
+    const double s = F.s, u = F.f - F.s;
+    P.flops += 2.0 * (s * s * s / 3.0 + s * s * u + s * u * u);
+    if (F.parent >= 0) P.height[F.parent] = std::max(P.height[F.parent], P.height[k] + 1);
+  }
+  // front index, in the parent, of every boundary DOF
+  P.rel.assign(P.bnd.size(), -1);
+  for (int k = 0; k < ns; ++k) {
+    gf::Front& F = P.fronts[k];
+    F.rel = F.bnd;
+    if (F.parent < 0) continue;
+    const gf::Front& Q = P.fronts[F.parent];
+    const int u = F.f - F.s, qu = Q.f - Q.s;
+    for (int i = 0, j = 0; i < u; ++i) {
+      const int d = P.bnd[F.bnd + i];
+      if (d < Q.dof0 + Q.s) {
+        P.rel[F.rel + i] = d - Q.dof0;
+      } else {
+        while (j < qu && P.bnd[Q.bnd + j] < d) ++j;
+        P.rel[F.rel + i] = Q.s + j;
+      }
+    }
+  }
+  return P;
+}
+
+void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<int>& slots,
+                 const std::vector<int>& dof_off, int n_struct, int n_dofs, FrontBuild& out) {
+  out.pos.assign(n_dofs, -1);
+  out.dof_front.assign(n_dofs, -1);
+  out.base.assign(n_struct, 0);
+  out.size.assign(n_struct, 0);
+  std::vector<int> height;
+  for (size_t q = 0; q < plans.size(); ++q) {
+    const FrontPlan& P = *plans[q];
+    const int f0 = (int)out.fronts.size(), b0 = (int)out.bnd.size(), d0 = dof_off[q];
+    out.base[slots[q]] = out.total;
+    out.size[slots[q]] = P.size;
+    for (gf::Front F : P.fronts) {
+      F.off += out.total;
+      F.slot = slots[q];
+      F.dof0 += d0;
+      F.bnd += b0;
+      F.rel += b0;
+      if (F.parent >= 0) F.parent += f0;
+      out.fronts.push_back(F);
+    }
+    for (int d : P.bnd) out.bnd.push_back(d + d0);
+    out.rel.insert(out.rel.end(), P.rel.begin(), P.rel.end());
+    height.insert(height.end(), P.height.begin(), P.height.end());
+    for (size_t i = 0; i < P.pos.size(); ++i) out.pos[d0 + i] = P.pos[i] + d0;
+    for (size_t i = 0; i < P.dof_front.size(); ++i) out.dof_front[d0 + i] = P.dof_front[i] + f0;
+    out.total += P.size;
+  }
+  const int nf = (int)out.fronts.size();
+  int nl = 0;
+  for (int h : height) nl = std::max(nl, h + 1);
+  std::vector<std::vector<int>> at(nl), kids(nf);
+  for (int k = 0; k < nf; ++k) {
+    at[height[k]].push_back(k);
+    if (out.fronts[k].parent >= 0 && out.fronts[k].f > out.fronts[k].s) kids[out.fronts[k].parent].push_back(k);
+  }
+  out.sched.level.resize(nl);
+  out.sched.launches = 3;  // zero, right-hand sides, gather of the solution
+  for (int l = 0; l < nl; ++l) {
+    gf::FrontLevel& V = out.sched.level[l];
+    std::vector<int> small, big;
+    size_t ords = 0;
+    for (int k : at[l]) {
+      (out.fronts[k].f <= gf::MF_SMALL ? small : big).push_back(k);
+      ords = std::max(ords, kids[k].size());
+    }
+    auto larger = [&](int a, int b) {
+      const gf::Front &A = out.fronts[a], &B = out.fronts[b];
+      return A.s != B.s ? A.s > B.s : a < b;
+    };
+    std::sort(big.begin(), big.end(), larger);
+    std::sort(small.begin(), small.end(), larger);
+    V.small_off = (int)out.list.size();
+    V.n_small = (int)small.size();
+    for (int k : small) V.small_f = std::max(V.small_f, out.fronts[k].f);
+    out.list.insert(out.list.end(), small.begin(), small.end());
+    V.big_off = (int)out.list.size();
+    V.n_big = (int)big.size();
+    out.list.insert(out.list.end(), big.begin(), big.end());
+    for (size_t o = 0; o < ords; ++o) {
+      V.ext_off.push_back((int)out.ext_jobs.size());
+      for (int k : at[l])
+        if (kids[k].size() > o) {
+          const gf::Front& C = out.fronts[kids[k][o]];
+          for (int c = 0; c <= C.f - C.s; c += 16) out.ext_jobs.push_back(make_int2(kids[k][o], c));
+        }
+      V.ext_cnt.push_back((int)out.ext_jobs.size() - V.ext_off.back());
+    }
+    const int panels = big.empty() ? 0 : (out.fronts[big[0]].s + gf::MF_NB - 1) / gf::MF_NB;
+    for (int p = 0; p < panels; ++p) {
+      int n = 0, f = 0, s = 0;
+      while (n < V.n_big && out.fronts[big[n]].s > p * gf::MF_NB) {
+        f = std::max(f, out.fronts[big[n]].f);
+        s = std::max(s, out.fronts[big[n]].s);
+        ++n;
+      }
+      V.n_at.push_back(n);
+      V.f_at.push_back(f);
+      V.s_at.push_back(s);
+    }
+    V.schur_off = (int)out.schur_jobs.size();
+    for (int k : big) {
+      const gf::Front& F = out.fronts[k];
+      const int u = F.f - F.s;
+      V.big_f = std::max(V.big_f, F.f);
+      if (u > 0)
+        for (int tj = 0; tj < (u + 1 + 31) / 32; ++tj)
+          for (int ti = 0; ti < (u + 31) / 32; ++ti) out.schur_jobs.push_back(make_int2(k, ti | (tj << 16)));
+    }
+    V.schur_cnt = (int)out.schur_jobs.size() - V.schur_off;
+    out.sched.launches += (int)ords + (V.n_small ? 1 : 0) + (V.schur_cnt ? 1 : 0) + 1;
+    for (int p = 0; p < panels; ++p)
+      out.sched.launches += 1 + (V.f_at[p] > p * gf::MF_NB ? 1 : 0) + (V.s_at[p] > (p + 1) * gf::MF_NB ? 1 : 0);
+  }
+}
+
+}  // namespace gfh

@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(64) k_shell_elements(int n, const ShellConst* 
 // MountGlobal: one warp per element of one colour (no two elements of a
 // colour share a node, so no two writers meet).  The element's free DOFs
 // (structure-local, in the structure's reverse Cuthill-McKee numbering) go
-// to the wide band and to P.
+// to the wide band (where one is kept) and to P.
 __global__ void k_shell_scatter(Batch b, int color) {
   int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
@@ -809,10 +809,11 @@ __global__ void k_shell_scatter(Batch b, int color) {
   }
   const double* K = b.sh.Ke + (int64_t)e * 729;
   const double* F = b.sh.Fe + (int64_t)e * 27;
+  if (lane < 27 && myg >= 0) b.P[inf.dof_off + myg] += F[lane];
+  if (!wide_band_filled(b)) return;  // the multifrontal LU assembles K_AA itself
   double* band = b.sh.wband + inf.wb_off;
   const int kl = inf.wkl;
   const int64_t W = 2 * kl + 1;
-  if (lane < 27 && myg >= 0) b.P[inf.dof_off + myg] += F[lane];
   for (int base = 0; base < 729; base += 32) {
     int idx = base + lane;
     bool valid = idx < 729;

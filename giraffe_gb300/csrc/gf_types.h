@@ -21,6 +21,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "gf_front.h"
+
 #define GF_KB 17
 #define GF_LDB (2 * GF_KB + 1)
 #define GF_UW (GF_KB + 1)
@@ -329,6 +331,8 @@ struct ShellData {
   // [0] panel start, [1] after trsm, [2] after the corner update, [3] after
   // diag, [4] end of forward, [5] after the bulk trsm
   cudaEvent_t evt[GF_WB_EVENTS];
+  // the multifrontal LU of the batch's Shell_1 structures (sched null: none)
+  FrontData mf;
 };
 
 // Device pointers of a batch.

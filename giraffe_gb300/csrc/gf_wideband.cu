@@ -1314,7 +1314,7 @@ __global__ void k_ir_restore(Batch b) {
 }
 
 void launch_wide_zero(const Batch& b, cudaStream_t st) {
-  if (b.sh.n_wide == 0) return;
+  if (b.sh.n_wide == 0 || !wide_band_filled(b)) return;
   k_wb_zero<<<dim3(4 * 152, b.sh.n_wide), 256, 0, st>>>(b);
 }
 
@@ -1561,29 +1561,6 @@ cudaError_t wide_capture_error() {
   return e;
 }
 
-// The same panel sequence on st alone, without the lookahead's helper
-// streams, in dependency order (the kernels and their results are those of
-// the lookahead form): the FP64 fallback inside the mixed path's captured
-// pass, whose helper streams already belong to that capture.
-template <typename F>
-static void wide_factor_solve_serial(const Batch& b, cudaStream_t st) {
-  const ShellData& sd = b.sh;
-  const int nw = sd.n_wide, nrest = trsm_rest_blocks(b);
-  k_wb_diag<F><<<nw, DIAG_THREADS, 0, st>>>(b, 0);
-  for (int p = 0; p < sd.max_panels; ++p) {
-    const bool next = p + 1 < sd.max_panels;
-    if (nrest) launch_trsm_rest<F>(b, p, st);
-    launch_trsm_first<F>(b, p, st);
-    if (next) {
-      wb_update(b, p, 1, st, (F*)nullptr);
-      k_wb_diag<F><<<nw, DIAG_THREADS, 0, st>>>(b, p + 1);
-    }
-    launch_fwd<F>(b, p, 1, st);
-    wb_update(b, p, next ? 2 : 0, st, (F*)nullptr);
-  }
-  for (int p = sd.max_panels - 1; p >= 0; --p) launch_bwd<F>(b, p, 1, st);
-}
-
 // Factor and solve in the factor's type F: FP64, the LU in place of K_AA
 // and the solve on P; FP32 (mixed path), the LU in wband32 and the solve on
 // r32.  Inside a served wave's capture the panel loops are graph loops
@@ -1710,7 +1687,7 @@ static void wide_solve_mixed(const Batch& b, cudaStream_t st, LaunchProf* prof) 
         cudaSuccess)
       return capture_fail(e);
     k_ir_restore<<<dim3(2 * 152, nw), 256, 0, sr>>>(fb);
-    wide_factor_solve_serial<double>(fb, sr);
+    launch_front_solve(fb, sr);
     if ((e = cudaStreamEndCapture(sr, &done)) != cudaSuccess) return capture_fail(e);
     return;
   }
@@ -1731,13 +1708,14 @@ static void wide_solve_mixed(const Batch& b, cudaStream_t st, LaunchProf* prof) 
     return;
   if (more[1]) {
     k_ir_restore<<<dim3(2 * 152, nw), 256, 0, st>>>(fb);
-    wide_factor_solve<double>(fb, st, prof);
+    launch_front_solve(fb, st, prof);
   }
 }
 
 void launch_wide_solve(const Batch& b, cudaStream_t st, LaunchProf* prof) {
   if (b.sh.n_wide == 0) return;
   if (b.mixed && b.sh.wband32) wide_solve_mixed(b, st, prof);
+  else if (b.sh.mf.sched) launch_front_solve(b, st, prof);
   else wide_factor_solve<double>(b, st, prof);
 }
 
@@ -1769,7 +1747,7 @@ static int wide_factor_launches(const Batch& b, bool fp64) {
 int wide_launches_per_pass(const Batch& b) {
   if (!b.sh.n_wide) return 0;
   if (b.mixed && b.sh.wband32) return wide_factor_launches(b, false) + 4;
-  return wide_factor_launches(b, true);
+  return b.sh.mf.sched ? front_launches(b) : wide_factor_launches(b, true);
 }
 
 // Launches of `sweeps` refinement sweeps (residual, forward and backward
@@ -1777,7 +1755,7 @@ int wide_launches_per_pass(const Batch& b) {
 long long wide_refine_launches(const Batch& b, long long sweeps, long long fallbacks) {
   const int P = b.sh.max_panels;
   const long long per_sweep = 3 + 2 * P;
-  return sweeps * per_sweep + fallbacks * (1 + wide_factor_launches(b, true));
+  return sweeps * per_sweep + fallbacks * (1 + front_launches(b));
 }
 
 }  // namespace gf
