@@ -1,0 +1,109 @@
+// One standalone system on the multifrontal LU: its plan, and the batch of one
+// structure around it that the kernels of gf_front.cu take.  Everything lives
+// in one block of the context's device workspace, its host data in one block
+// of pinned staging sent by one copy.  Internal to libgiraffe_gpu.so.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstring>
+#include <vector>
+
+#include "gf_front.h"
+#include "gf_host_internal.h"
+#include "gf_kernels.cuh"
+
+namespace gfh {
+
+struct FrontSystem {
+  gf::Batch b{};
+  FrontBuild fb;
+  // parts of the block: offset and, for host data, the source
+  struct Part {
+    size_t off, bytes;
+    const void* src;
+  };
+  std::vector<Part> parts;
+  size_t sent = 0, total = 0;
+  char* dev = nullptr;
+  gf::StructState state{};
+  gf::StructInfo info{};
+  int zero = 0;
+  int p_state = 0, p_rhs = 0;
+
+  // A host array to send (before any device-only part) or a device-only part.
+  int send(const void* src, size_t bytes) {
+    parts.push_back({sent, bytes, src});
+    sent += (bytes + 255) / 256 * 256;
+    return (int)parts.size() - 1;
+  }
+  template <typename T> T* at(int p) const { return reinterpret_cast<T*>(dev + parts[p].off); }
+
+  // plan: the system's fronts; extra: more arrays sent with it (their parts'
+  // numbers come back in order).  rhs: n doubles.
+  int init(gf_ctx* ctx, const FrontPlan& plan, int n, const double* rhs,
+           const std::vector<std::pair<const void*, size_t>>& extra, std::vector<int>* extra_parts) {
+    join_fronts({&plan}, {0}, {0}, 1, n, fb);
+    info.n_free = n;
+    info.wide = 1;
+    state.phase = gf::PH_ITER;
+    state.need_solve = 1;
+    auto vec = [&](const auto& v) { return send(v.data(), v.size() * sizeof(v[0])); };
+    const int p_fr = vec(fb.fronts), p_bnd = vec(fb.bnd), p_rel = vec(fb.rel), p_list = vec(fb.list),
+              p_ext = vec(fb.ext_jobs), p_sch = vec(fb.schur_jobs), p_pos = vec(fb.pos), p_df = vec(fb.dof_front),
+              p_base = vec(fb.base), p_size = vec(fb.size);
+    const int p_info = send(&info, sizeof(info)), p_ws = send(&zero, sizeof(int));
+    p_state = send(&state, sizeof(state));
+    p_rhs = send(rhs, sizeof(double) * (size_t)n);
+    for (const auto& x : extra) extra_parts->push_back(send(x.first, x.second));
+    const size_t off_F = sent, off_x = off_F + ((size_t)fb.total * sizeof(double) + 255) / 256 * 256;
+    total = off_x + sizeof(double) * (size_t)n;
+    dev = static_cast<char*>(ctx->device_work(total));
+    char* pin = static_cast<char*>(ctx->pinned(sent));
+    if (!dev || !pin) {
+      set_err(ctx, "linear solve: allocation of %zu device and %zu pinned bytes failed", total, sent);
+      return GF_ERR_CUDA;
+    }
+    for (const Part& p : parts) std::memcpy(pin + p.off, p.src, p.bytes);
+    GF_CK(cudaMemcpyAsync(dev, pin, sent, cudaMemcpyHostToDevice, ctx->stream));
+    b.n_struct = 1;
+    b.n_free = n;
+    b.info = at<gf::StructInfo>(p_info);
+    b.state = at<gf::StructState>(p_state);
+    b.P = at<double>(p_rhs);
+    b.sh.n_wide = 1;
+    b.sh.wide_structs = at<int>(p_ws);
+    gf::FrontData& d = b.sh.mf;
+    d.n_fronts = (int)fb.fronts.size();
+    d.fronts = at<gf::Front>(p_fr);
+    d.bnd = at<int>(p_bnd);
+    d.rel = at<int>(p_rel);
+    d.list = at<int>(p_list);
+    d.ext_jobs = at<int2>(p_ext);
+    d.schur_jobs = at<int2>(p_sch);
+    d.pos = at<int>(p_pos);
+    d.dof_front = at<int>(p_df);
+    d.base = at<int64_t>(p_base);
+    d.size = at<int64_t>(p_size);
+    d.F = reinterpret_cast<double*>(dev + off_F);
+    d.x = reinterpret_cast<double*>(dev + off_x);
+    d.sched = &fb.sched;
+    return GF_OK;
+  }
+
+  // The solution into x and the pivot status, after the solve's launches.
+  int finish(gf_ctx* ctx, int n, double* x, int* fail) {
+    GF_CK(cudaGetLastError());
+    char* pin = static_cast<char*>(ctx->pin);  // the staging is free again once the solve has run
+    const size_t xb = sizeof(double) * (size_t)n;
+    GF_CK(cudaMemcpyAsync(pin + parts[p_rhs].off, b.P, xb, cudaMemcpyDeviceToHost, ctx->stream));
+    GF_CK(cudaMemcpyAsync(pin + parts[p_state].off, b.state, sizeof(state), cudaMemcpyDeviceToHost, ctx->stream));
+    GF_CK(cudaStreamSynchronize(ctx->stream));
+    std::memcpy(x, pin + parts[p_rhs].off, xb);
+    std::memcpy(&state, pin + parts[p_state].off, sizeof(state));
+    *fail = state.info_fail;
+    ctx->trim_work();
+    return GF_OK;
+  }
+};
+
+}  // namespace gfh

@@ -1355,6 +1355,7 @@ void gf_destroy(gf_ctx* ctx) {
   if (!ctx) return;
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->pin) cudaFreeHost(ctx->pin);
+  if (ctx->work) cudaFree(ctx->work);
   delete ctx;
 }
 
@@ -2242,6 +2243,7 @@ int gf_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab
     set_err(ctx, "gf_band_solve: invalid arguments");
     return GF_ERR_ARG;
   }
+  if (band_takes_fronts(n, kl, ku)) return front_band_solve(ctx, n, kl, ku, ab, ldab, b, info);
   if (kl > GF_KB || ku > GF_KB) return wide_band_solve(ctx, n, kl, ku, ab, ldab, b, info);
   int npad = (n + 31) / 32 * 32;
   std::vector<double> band((size_t)npad * GF_LDB, 0.0);

@@ -27,6 +27,32 @@ struct gf_ctx {
   // with the context)
   void* pin = nullptr;
   size_t pin_bytes = 0;
+  // device workspace of the standalone solves (calls on one context do not
+  // overlap): grown on demand, kept between calls up to kKeepWork bytes, freed
+  // with the context
+  void* work = nullptr;
+  size_t work_bytes = 0;
+  static constexpr size_t kKeepWork = (size_t)512 << 20;
+  void* device_work(size_t n) {
+    if (n <= work_bytes) return work;
+    if (work) cudaFree(work);
+    work = nullptr;
+    work_bytes = 0;
+    if (cudaMalloc(&work, n) != cudaSuccess) {
+      cudaGetLastError();
+      work = nullptr;
+      return nullptr;
+    }
+    work_bytes = n;
+    return work;
+  }
+  void trim_work() {
+    if (work_bytes > kKeepWork) {
+      cudaFree(work);
+      work = nullptr;
+      work_bytes = 0;
+    }
+  }
   // a pinned block of at least n bytes, or nullptr when none can be had
   void* pinned(size_t n) {
     if (n <= pin_bytes) return pin;
@@ -223,6 +249,10 @@ std::vector<int> rcm_order(int nn, const std::vector<std::vector<int>>& adj);
 // gf_band_solve for half-bandwidths above 17: the blocked wide-band LU on a
 // one-structure batch (gf_sparse.cu).
 int wide_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, int* info);
+// gf_band_solve on the multifrontal LU, and whether it takes it
+// (gf_sparse.cu).
+bool band_takes_fronts(int n, int kl, int ku);
+int front_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, int* info);
 // Host PreCalc of one Beam_1 element (end nodes x0, x2; Hooke material E,
 // nu, rho; section A, I11, I22, I12, It, I33; CS rows E1, E3; pre-tension
 // T0) into its constants and initial Gauss-point history, and of one Shell_1

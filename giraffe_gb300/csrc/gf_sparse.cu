@@ -7,22 +7,23 @@
 //                     bandwidth above 17, the wide branch of gf_band_solve
 //                     (bandsystem, src/BandMatrix.cpp:257-287)
 //
-// Both factor on the GPU with the blocked no-pivot wide-band LU of the
-// Shell_1 path (gf_shell.cu) run on a batch of one structure; systems with
-// a half-bandwidth of at most 17 go to the 35-row band solver instead.
-// The CSR path picks the narrower of the natural ordering and reverse
-// Cuthill-McKee on the symmetrised pattern, as the batch path does for
-// shells.
+// Both factor on the GPU without pivoting: by the multifrontal LU of the
+// Shell_1 path (gf_front.cu) under a nested-dissection ordering of the CSR's
+// graph or of the band's blocks; by the 35-row band solver and the wide-band LU
+// (gf_wideband.cu) where those are estimated faster (short bands) or the fronts
+// would be too large.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
 #include "../../include/giraffe_gpu.h"
 #include "gf_host_internal.h"
+#include "gf_front_system.h"
 #include "gf_kernels.cuh"
 #include "gf_types.h"
 #include "gf_wide.h"
@@ -69,9 +70,110 @@ int csr_bandwidth(int n, const int* rp, const int* ci, const int* pos) {
   return w;
 }
 
+// Graph of the symmetrised CSR pattern, consecutive rows with the same columns
+// (the DOFs of a mesh node) as one vertex.
+void csr_graph(int n, const int* rp, const int* ci, NdGraph& g, std::vector<int>& dptr) {
+  std::vector<int> id(n);
+  for (int i = 0; i < n; ++i) {
+    const int len = rp[i + 1] - rp[i];
+    const bool same = i > 0 && len == rp[i] - rp[i - 1] && len > 0 &&
+                      std::memcmp(ci + rp[i], ci + rp[i - 1], sizeof(int) * (size_t)len) == 0;
+    if (!same) dptr.push_back(i);
+    id[i] = (int)dptr.size() - 1;
+  }
+  g.n = (int)dptr.size();
+  dptr.push_back(n);
+  for (int v = 0; v < g.n; ++v) g.w.push_back(dptr[v + 1] - dptr[v]);
+  // both directions of every edge, then each list sorted without repeats
+  std::vector<int> cnt(g.n + 1, 0);
+  auto edges = [&](auto f) {
+    for (int v = 0; v < g.n; ++v) {
+      int last = -1;
+      for (int k = rp[dptr[v]]; k < rp[dptr[v] + 1]; ++k) {
+        const int u = id[ci[k]];
+        if (u != v && u != last) f(v, u);
+        last = u;
+      }
+    }
+  };
+  edges([&](int v, int u) {
+    cnt[v + 1]++;
+    cnt[u + 1]++;
+  });
+  for (int v = 0; v < g.n; ++v) cnt[v + 1] += cnt[v];
+  std::vector<int> all(cnt[g.n]), at(cnt.begin(), cnt.end() - 1);
+  edges([&](int v, int u) {
+    all[at[v]++] = u;
+    all[at[u]++] = v;
+  });
+  g.ptr.assign(1, 0);
+  for (int v = 0; v < g.n; ++v) {
+    std::sort(all.begin() + cnt[v], all.begin() + cnt[v + 1]);
+    for (int k = cnt[v]; k < cnt[v + 1]; ++k)
+      if (k == cnt[v] || all[k] != all[k - 1]) g.adj.push_back(all[k]);
+    g.ptr.push_back((int)g.adj.size());
+  }
+}
+
+// What the multifrontal kernels take: 32-bit offsets, and a front's column of
+// the solution in shared memory.
+bool fronts_fit(const FrontPlan& P) {
+  int f = 0;
+  for (const Front& F : P.fronts) f = std::max(f, F.f);
+  return P.size < INT_MAX && f <= 16384;
+}
+
 }  // namespace
 
 namespace gfh {
+
+// The multifrontal LU eliminates a band of half-bandwidth w in blocks of w,
+// about 6.3 w^3 multiply-adds a block on a chain of log2(n / w) blocks; the
+// banded LU takes w^2 per column on a chain of n.  Measured: the 35-row band
+// solver takes 0.9 us a column and the wide-band LU about 85 us per 64 columns
+// plus its updates at 5.4 TFLOP/s, the fronts 0.8 TFLOP/s and about 0.6 us a
+// pivot of the chain.  Both are estimated at those rates.
+bool band_takes_fronts(int n, int kl, int ku) {
+  const double w = std::max(std::max(kl, ku), 12);
+  const double blocks = n / w;
+  if (blocks < 4.0) return false;
+  const double chain = w * (std::ceil(std::log2(blocks)) + 1.0);
+  const double t_front = 12.6 * w * w * n / 0.8e12 + 0.6e-6 * chain + 12e-6 * chain / w;
+  const double t_band = kl <= GF_KB && ku <= GF_KB ? 0.9e-6 * n : n / 64.0 * 85e-6 + 2.0 * n * w * w / 5.4e12;
+  return t_front < t_band;
+}
+
+int front_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, int* info) {
+  // blocks of at least the half-bandwidth: their graph is a path
+  const int B = std::max(std::max(kl, ku), 12), nb = (n + B - 1) / B, W = kl + ku + 1;
+  NdGraph g;
+  g.n = nb;
+  g.ptr.push_back(0);
+  g.field.resize(1);
+  std::vector<int> dptr(1, 0), dofs(n);
+  for (int v = 0; v < nb; ++v) {
+    if (v) g.adj.push_back(v - 1);
+    if (v + 1 < nb) g.adj.push_back(v + 1);
+    g.ptr.push_back((int)g.adj.size());
+    dptr.push_back(std::min(n, (v + 1) * B));
+    g.w.push_back(dptr[v + 1] - dptr[v]);
+    g.field[0].push_back((float)v);
+  }
+  for (int i = 0; i < n; ++i) dofs[i] = i;
+  const FrontPlan plan = plan_fronts(g, dptr, dofs);
+  std::vector<double> packed((size_t)n * W);
+  for (int j = 0; j < n; ++j)
+    std::memcpy(&packed[(size_t)j * W], ab + (size_t)j * ldab + kl, sizeof(double) * (size_t)W);
+  FrontSystem S;
+  std::vector<int> part;
+  int rc = S.init(ctx, plan, n, b, {{packed.data(), sizeof(double) * packed.size()}}, &part);
+  if (rc != GF_OK) return rc;
+  launch_front_band(S.b, n, kl, ku, W, S.at<double>(part[0]) - kl, ctx->stream);
+  int fail = 0;
+  rc = S.finish(ctx, n, b, &fail);
+  if (rc == GF_OK && info) *info = fail;
+  return rc;
+}
 
 // Wide branch of gf_band_solve: the GB array goes into the wide band with
 // one strided copy (each column's kl + ku + 1 stored entries keep their
@@ -131,8 +233,38 @@ int gf_sparse_solve(gf_ctx* ctx, int n, const int* row_ptr, const int* col_idx, 
       gfh::set_err(ctx, "gf_sparse_solve: column index %d out of range at entry %d", col_idx[k], k);
       return GF_ERR_ARG;
     }
-  // ordering: natural, or reverse Cuthill-McKee on the symmetrised pattern
-  // when that narrows the band
+  // a narrow band in the natural order goes to the band solvers, anything
+  // wider to the multifrontal LU under a nested-dissection ordering
+  bool wide = false;
+  for (int i = 0; i < n && !wide; ++i)
+    for (int k = row_ptr[i]; k < row_ptr[i + 1] && !wide; ++k) wide = std::abs(i - col_idx[k]) > GF_KB;
+  if (wide) {
+    NdGraph g;
+    std::vector<int> dptr, dofs(n);
+    csr_graph(n, row_ptr, col_idx, g, dptr);
+    for (int i = 0; i < n; ++i) dofs[i] = i;
+    nd_landmark_fields(g);
+    std::vector<float> place(g.n);
+    for (int v = 0; v < g.n; ++v) place[v] = (float)v;
+    g.field.push_back(std::move(place));
+    const FrontPlan plan = plan_fronts(g, dptr, dofs);
+    if (fronts_fit(plan)) {
+      FrontSystem S;
+      std::vector<int> part;
+      int rc = S.init(ctx, plan, n, b,
+                      {{row_ptr, sizeof(int) * ((size_t)n + 1)}, {col_idx, sizeof(int) * (size_t)nnz},
+                       {val, sizeof(double) * (size_t)nnz}}, &part);
+      if (rc != GF_OK) return rc;
+      launch_front_csr(S.b, n, S.at<int>(part[0]), S.at<int>(part[1]), S.at<double>(part[2]), ctx->stream);
+      int fail = 0;
+      rc = S.finish(ctx, n, b, &fail);
+      if (rc == GF_OK && info) *info = fail;
+      return rc;
+    }
+  }
+  // a system whose fronts exceed the multifrontal kernels' limits, or a narrow
+  // band: ordering natural, or reverse Cuthill-McKee on the symmetrised
+  // pattern when that narrows the band
   std::vector<int> perm(n);
   for (int i = 0; i < n; ++i) perm[i] = i;
   int w = csr_bandwidth(n, row_ptr, col_idx, perm.data());

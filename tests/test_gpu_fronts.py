@@ -74,3 +74,102 @@ def test_solves_as_the_oracle(gpu_ctx, make):
     assert np.array_equal(finals[0], finals[2])
     alone, _ = gpu.solve([make()])
     assert np.array_equal(finals[0], alone[0])
+
+
+def solve_dense(A, b):
+    return np.linalg.solve(A, b)
+
+
+def to_csr(A):
+    rows, cols = np.nonzero(A)
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=len(A)))]).astype(np.int32)
+    return rp, cols.astype(np.int32), A[rows, cols]
+
+
+def pattern(kind, seed):
+    """Diagonally dominant matrices (row sums 1.5 times the off-diagonal's, so
+    no pivoting is needed) whose graphs the ordering meets in earnest or not."""
+    rng = np.random.default_rng(seed)
+    if kind == "dense":
+        n = 150
+        M = np.ones((n, n), dtype=bool)
+    elif kind == "grid":
+        g, d = 13, 3
+        n = g * g * d
+        x = np.arange(n) // d
+        M = (np.abs(x[:, None] % g - x[None, :] % g) <= 1) & (np.abs(x[:, None] // g - x[None, :] // g) <= 1)
+    elif kind == "unsymmetric":
+        n = 400
+        M = rng.random((n, n)) < 4.0 / n
+    elif kind == "arrow":
+        n = 300
+        M = np.eye(n, dtype=bool)
+        M[-40:] = M[:, -40:] = True
+    elif kind == "blocks":  # three components and rows without off-diagonals
+        n = 330
+        c = np.arange(n) // 110
+        M = (c[:, None] == c[None, :]) & (rng.random((n, n)) < 0.05)
+    elif kind == "scrambled":
+        n = 500
+        p = rng.permutation(n)
+        M = np.abs(p[:, None] - p[None, :]) <= 5
+    else:  # one row past the narrow band
+        n = 100
+        M = np.abs(np.arange(n)[:, None] - np.arange(n)[None, :]) <= 18
+    A = np.where(M, rng.uniform(-1.0, 1.0, (n, n)), 0.0)
+    np.fill_diagonal(A, 0.0)
+    np.fill_diagonal(A, 1.5 * np.abs(A).sum(axis=1) + 0.1)
+    return A
+
+
+@pytest.mark.parametrize("kind", ["dense", "grid", "unsymmetric", "arrow", "blocks", "scrambled", "past17"])
+def test_sparse_patterns_match_dense(gpu_ctx, kind):
+    # forward error bound n eps cond with cond <= 5 for these row sums: 1e-13
+    A = pattern(kind, 3)
+    b = np.random.default_rng(4).normal(size=len(A))
+    x, info = gpu_ctx.sparse_solve(*to_csr(A), b)
+    assert info == 0
+    ref = solve_dense(A, b)
+    assert np.abs(x - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+def test_sparse_rows_in_any_order_and_repeated(gpu_ctx):
+    A = pattern("grid", 5)
+    rp, ci, v = to_csr(A)
+    rng = np.random.default_rng(6)
+    ci2, v2 = np.repeat(ci, 2), np.repeat(v, 2) * np.tile([0.25, 0.75], len(v))
+    rp2 = 2 * rp
+    for i in range(len(A)):
+        p = rp2[i] + rng.permutation(rp2[i + 1] - rp2[i])
+        ci2[rp2[i]:rp2[i + 1]], v2[rp2[i]:rp2[i + 1]] = ci2[p], v2[p]
+    b = rng.normal(size=len(A))
+    x, info = gpu_ctx.sparse_solve(rp2, ci2, v2, b)
+    ref = solve_dense(A, b)
+    assert info == 0 and np.abs(x - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n,kl,ku", [(2000, 17, 17), (2001, 3, 9), (1500, 0, 1), (800, 1, 0), (3000, 40, 33),
+                                     (2600, 97, 96), (1501, 300, 2), (700, 12, 13)])
+def test_bands_match_a_banded_lu(gpu_ctx, n, kl, ku):
+    from scipy.linalg import solve_banded
+
+    rng = np.random.default_rng(n + kl)
+    ab = np.full((n, 2 * kl + ku + 1), np.nan)  # unreferenced entries may hold anything
+    for j in range(n):
+        i = np.arange(max(0, j - ku), min(n, j + kl + 1))
+        ab[j, kl + ku + i - j] = rng.uniform(-1.0, 1.0, len(i))
+        ab[j, kl + ku] = 1.5 * (kl + ku + 1)
+    b = rng.normal(size=n)
+    x, info = gpu_ctx.band_solve(ab, kl, ku, b)
+    ref = solve_banded((kl, ku), np.nan_to_num(np.ascontiguousarray(ab[:, kl:].T)), b)
+    assert info == 0 and np.abs(x - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("at", [0, 777, 1999])
+def test_a_zero_pivot_is_reported(gpu_ctx, at):
+    n, kl = 2000, 17
+    ab = np.zeros((n, 3 * kl + 1))
+    ab[:, 2 * kl] = 1.0
+    ab[at, 2 * kl] = 0.0
+    _, info = gpu_ctx.band_solve(ab, kl, kl, np.ones(n))
+    assert info == 1
