@@ -4,7 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "gf_beam.cuh"
-#include "gf_df64.cuh"
+#include "gf_beam_gp.cuh"
 #include "gf_chain.cuh"
 #include "../../include/giraffe_model.h"
 #include "gf_kernels.cuh"
@@ -296,121 +296,142 @@ __global__ void k_zero(Batch b) {
 // Beam_1 Mount + MountElementLoads (k_beam_tangent) and MountGlobal
 // (k_beam_scatter).
 //
-// k_beam_tangent: one thread per element, every element of every iterating
-// structure.  The two rotated Gauss-point operators live in shared memory
-// ([g][entry][thread], conflict-free); the 18x18 tangent (column-major) and
-// the 18 internal forces go to per-element scratch.  Keeping the band
-// read-modify-write out of this FP64-bound kernel keeps global-load latency
-// off its dependency chains.
+// k_beam_tangent: 32 elements per CTA, an element per lane, so every warp runs
+// one code path and the element scratch (structure-of-arrays) is written
+// coalesced.  Warps 0 and 1 form the two Gauss points' operators and forces
+// (gf_beam_gp.cuh) in shared memory while warps 2 and 3 form the expansion's
+// coefficients and, in Dynamic steps, the points' inertial terms; then the
+// four warps share the entries of K_e and f_e.  K_e of the elastic terms is
+// symmetric: each pair of entries is formed once.  FP64 throughput bounds
+// large batches (about 1,900 FP64 operations an element, 4,250 with an element
+// per thread and full matrix products) and the chain of a point's 620 operations
+// small ones.  Keeping the band read-modify-write out of this kernel keeps
+// global-load latency off its dependency chains.
 // k_beam_scatter: one warp per element of one colour class; lanes walk the
 // 324 tangent entries in column order, so the band updates of a column are
 // contiguous.  Elements of one colour share no node, so the scatter needs no
 // atomics and is deterministic.
-constexpr int MOUNT_THREADS = 64;
-// per thread: the two operators (OP_N stored entries each) and the internal
-// force (18), so three CTAs fit on an SM; the inertial rotational tangents
-// of Dynamic steps go to the element scratch b.Dm instead
-constexpr int MOUNT_SMEM = (2 * OP_N + 18) * MOUNT_THREADS * (int)sizeof(double);
+constexpr int MOUNT_THREADS = 128;
+constexpr int MP_POINT = GP_COUNT + GC_COUNT;  // doubles per Gauss point and element
+// a Gauss point's inertial terms: rotational tangent, translational and
+// rotational force (global frame)
+constexpr int MI_D = 0, MI_FU = 9, MI_FA = 12, MI_COUNT = 15;
+constexpr int MOUNT_SMEM = 2 * MP_POINT * 32 * (int)sizeof(double);
+constexpr int MOUNT_SMEM_DYN = 2 * (MP_POINT + MI_COUNT) * 32 * (int)sizeof(double);
 
-template <typename TK>
+// The entries of K_e and f_e of lane's element, shared by the CTA's warps:
+// put(r, s, v) for one entry of every symmetric pair, force(q, v).
+template <typename Put, typename Force>
+__device__ __forceinline__ void beam_expand(const double* P, int warp, int lane, Put put, Force force) {
+  const double *M = P + lane, *C = P + GP_COUNT * 32 + lane;
+  constexpr int gs = MP_POINT * 32, ms = 32;
+#pragma unroll 1
+  for (int k = warp; k < 45; k += 4) {
+    int pair, I, J, i, j;
+    beam_aa_place(k, pair, I, J, i, j);
+    put(6 * I + 3 + i, 6 * J + 3 + j, beam_k_aa(M, C, gs, ms, pair, I, J, i, j));
+  }
+#pragma unroll 1
+  for (int k = warp; k < 81; k += 4) {
+    const int IJ = k / 9, x = k % 9;
+    put(6 * (IJ / 3) + x / 3, 6 * (IJ % 3) + 3 + x % 3, beam_k_ua(M, C, gs, ms, IJ, x));
+  }
+#pragma unroll 1
+  for (int k = warp; k < 36; k += 4) {
+    int pair, x, I, J, i, j;
+    beam_uu_place(k, pair, x, I, J, i, j);
+    const double v = beam_k_uu(M, C, gs, ms, pair, x);
+    put(6 * I + i, 6 * J + j, v);
+    if (I != J && i != j) put(6 * I + j, 6 * J + i, v);
+  }
+#pragma unroll 1
+  for (int k = warp; k < 18; k += 4) force(k, beam_f(M, C, gs, ms, k / 6, (k % 6) / 3, k % 3));
+}
+
 __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
-  extern __shared__ unsigned char smem_raw[];
-  TK* sM = reinterpret_cast<TK*>(smem_raw);
-  const int tid = threadIdx.x;
-  int e = blockIdx.x * MOUNT_THREADS + tid;
-  if (e >= b.n_elem) return;
-  int s = b.estruct[e];
-  if (!iterating(b.state[s])) return;
-  const BeamConst& c = b.bconst[e];
-  const BeamHist& h = b.bhist[e];
-  int nd[3] = {b.enodes[3 * e], b.enodes[3 * e + 1], b.enodes[3 * e + 2]};
-  double d[18];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* P = reinterpret_cast<double*>(smem_raw);  // [point][value][lane]
+  double* In = P + 2 * MP_POINT * 32;               // inertial terms, [point][value][lane]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int e = blockIdx.x * 32 + lane;
+  const int s = e < b.n_elem ? b.estruct[e] : -1;
+  const bool live = s >= 0 && iterating(b.state[s]);
+  const bool dyn = live && b.params[s].dynamic;
+  if (live) {
+    const BeamConst& c = b.bconst[e];
+    const int g = warp & 1;
+    if (warp >= 2) beam_gp_coef(c, g, P + (g * MP_POINT + GP_COUNT) * 32 + lane, 32);
+    if (warp < 2 || dyn) {
+      int nd[3] = {b.enodes[3 * e], b.enodes[3 * e + 1], b.enodes[3 * e + 2]};
+      double d[18];
 #pragma unroll
-  for (int j = 0; j < 3; ++j)
+      for (int j = 0; j < 3; ++j)
 #pragma unroll
-    for (int q = 0; q < 6; ++q) d[6 * j + q] = b.disp[(int64_t)nd[j] * 6 + q];
-  BeamInterp ip[2] = {beam_interp(c, d, 0), beam_interp(c, d, 1)};
-  double* f = reinterpret_cast<double*>(sM + (size_t)2 * OP_N * MOUNT_THREADS) + tid;
-  // inertial rotational tangents, 2 x 9, structure-of-arrays like K_e
-  double* Dm = b.Dm + e;
-  const int64_t dms = b.n_elem;
+        for (int q = 0; q < 6; ++q) d[6 * j + q] = b.disp[(int64_t)nd[j] * 6 + q];
+      if (warp < 2) {
+        beam_gp(c, b.bhist[e], d, g, P + g * MP_POINT * 32 + lane, 32);
+      } else {
+        // MountMass + MountDyn: inertial force and mass/gyroscopic tangent
+        double vel[18], acc[18], a6[6];
 #pragma unroll
-  for (int q = 0; q < 18; ++q) f[q * MOUNT_THREADS] = 0.0;
-  const StructParams& pr = b.params[s];
-  const bool dyn = pr.dynamic;
-  const double* an = b.state[s].a;
-#pragma unroll 1
-  for (int g = 0; g < 2; ++g) {
-    BeamGP kin;
-    beam_kinematics(c, h, ip[g], g, kin);
-    beam_gp_force(c, kin, g, f, MOUNT_THREADS);
-    TK* M = sM + (size_t)g * OP_N * MOUNT_THREADS + tid;
-    if constexpr (std::is_same<TK, double>::value) {
-      beam_gp_operator<TK>(c, kin, M, MOUNT_THREADS);
-      rotate_blocks9<TK>(c, M, MOUNT_THREADS);
-    } else {
-      // mixed precision: the operator in FP64, rounded to TK in place (a TK
-      // is as wide as a double), then its rotation and the K_e expansion in
-      // TK.  (Expanding in a kernel of its own, with many warps per SM, gains
-      // nothing here: its FP64 <-> FP32-pair conversions take the FP64 pipe
-      // as long as the products it moves off it.)
-      static_assert(sizeof(TK) == sizeof(double), "operator storage");
-      double* Md = reinterpret_cast<double*>(M);
-      beam_gp_operator<double>(c, kin, Md, MOUNT_THREADS);
-#pragma unroll 1
-      for (int q = 0; q < OP_N; ++q) {
-        const double v = Md[q * MOUNT_THREADS];
-        M[q * MOUNT_THREADS] = TK(v);
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+          for (int q = 0; q < 6; ++q) {
+            vel[6 * j + q] = b.copy_vel[(int64_t)nd[j] * 6 + q];
+            acc[6 * j + q] = b.copy_accel[(int64_t)nd[j] * 6 + q];
+          }
+#pragma unroll
+        for (int q = 0; q < 6; ++q) a6[q] = b.state[s].a[q];
+        double* I = In + g * MI_COUNT * 32 + lane;
+        beam_gp_inertia(c, b.baux[e], beam_interp(c, d, g), vel, acc, a6, g, I + MI_FU * 32, I + MI_FA * 32, I, 32);
       }
-      rotate_blocks9<TK>(c, M, MOUNT_THREADS);
     }
   }
-  double a1Mr = 0.0;
-  if (dyn) {
-    // MountMass + MountDyn: inertial force and mass/gyroscopic tangent
-    double vel[18], acc[18];
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        vel[6 * j + q] = b.copy_vel[(int64_t)nd[j] * 6 + q];
-        acc[6 * j + q] = b.copy_accel[(int64_t)nd[j] * 6 + q];
-      }
-    double a6[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) a6[q] = an[q];
-    const BeamHistAux& x = b.baux[e];
-#pragma unroll 1
-    for (int g = 0; g < 2; ++g)
-      beam_gp_inertia(c, x, ip[g], vel, acc, a6, g, f, MOUNT_THREADS, Dm + (int64_t)g * 9 * dms, (int)dms);
-    a1Mr = a6[0] * c.Mr;
-  }
-  // element scratch is structure-of-arrays (entry x of element e at
-  // [x * n_elem + e]): the writes of a warp and the per-item reads of the
-  // chain solver are coalesced
+  __syncthreads();
+  if (!live) return;
   double* Ke = b.Ke + e;
   const int64_t ne = b.n_elem;
-
-#pragma unroll 1
-  for (int J = 0; J < 3; ++J)
-#pragma unroll 1
-    for (int I = 0; I < 3; ++I)
-      beam_K_block<TK>(c, sM + tid, sM + OP_N * MOUNT_THREADS + tid, I, J, MOUNT_THREADS, Ke, dyn, Dm,
-                       Dm + 9 * dms, (int)dms, a1Mr, ne);
-  // Rayleigh damping: on the iterations that form C_e, the stiffness part
-  // of K_e alone (no inertial terms) goes to the damping scratch, where
-  // k_beam_rayleigh turns it into C_e = alpha M_modal + beta K_e
-  if (dyn && pr.ray_on && (pr.ray_update || !b.state[s].ray_init)) {
-    double* Ce = b.RD + e;
-#pragma unroll 1
-    for (int J = 0; J < 3; ++J)
-#pragma unroll 1
-      for (int I = 0; I < 3; ++I)
-        beam_K_block<TK>(c, sM + tid, sM + OP_N * MOUNT_THREADS + tid, I, J, MOUNT_THREADS, Ce, false, Dm,
-                         Dm + 9 * dms, (int)dms, 0.0, ne);
+  const double* Cf = P + GP_COUNT * 32 + lane;
+  if (!dyn) {
+    beam_expand(P, warp, lane,
+                [&](int r, int q, double v) {
+                  Ke[(r + 18 * q) * ne] = v;
+                  if (r != q) Ke[(q + 18 * r) * ne] = v;
+                },
+                [&](int q, double v) { b.Fe[q * ne + e] = v; });
+    return;
   }
-#pragma unroll
-  for (int q = 0; q < 18; ++q) b.Fe[q * ne + e] = f[q * MOUNT_THREADS];
+  // Dynamic steps: the inertial terms on top.  Rayleigh damping: on the
+  // iterations that form C_e, the stiffness part of K_e alone goes to the
+  // damping scratch, where k_beam_rayleigh turns it into C_e = alpha M_modal +
+  // beta K_e
+  const StructParams& pr = b.params[s];
+  double* Ce = pr.ray_on && (pr.ray_update || !b.state[s].ray_init) ? b.RD + e : nullptr;
+  const double a1Mr = rmul(b.state[s].a[0], b.bconst[e].Mr);
+  const double* I0 = In + lane;
+  auto mass = [&](int r, int q) {
+    const int I = r / 6, i = r % 6, J = q / 6, j = q % 6;
+    const int pair = tri3(I, J);
+    if (i < 3 && j < 3)
+      return i == j ? rmul(radd(Cf[(GC_NN + pair) * 32], Cf[(MP_POINT + GC_NN + pair) * 32]), a1Mr) : 0.0;
+    if (i < 3 || j < 3) return 0.0;
+    const int x = (i - 3) * 3 + j - 3;
+    return rfma(Cf[(MP_POINT + GC_NN + pair) * 32], I0[(MI_COUNT + MI_D + x) * 32],
+                rmul(Cf[(GC_NN + pair) * 32], I0[(MI_D + x) * 32]));
+  };
+  beam_expand(P, warp, lane,
+              [&](int r, int q, double v) {
+                Ke[(r + 18 * q) * ne] = radd(v, mass(r, q));
+                if (Ce) Ce[(r + 18 * q) * ne] = v;
+                if (r == q) return;
+                Ke[(q + 18 * r) * ne] = radd(v, mass(q, r));
+                if (Ce) Ce[(q + 18 * r) * ne] = v;
+              },
+              [&](int q, double v) {
+                const int I = q / 6, x = (q % 6) / 3 ? MI_FA + q % 3 : MI_FU + q % 3;
+                v = rfma(Cf[(GC_WN + I) * 32], I0[x * 32], v);
+                b.Fe[q * ne + e] = rfma(Cf[(MP_POINT + GC_WN + I) * 32], I0[(MI_COUNT + x) * 32], v);
+              });
 }
 
 // MountDamping and the damping part of MountDyn (reference
@@ -1155,9 +1176,9 @@ __global__ void k_control(Batch b) {
   }
 }
 
-// SaveConfiguration: element Gauss-point history ...
+// SaveConfiguration: element Gauss-point history, a thread per Gauss point ...
 __global__ void k_commit_elems(Batch b) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, e = t >> 1;
   if (e >= b.n_elem) return;
   int s = b.estruct[e];
   if (!b.state[s].commit) return;
@@ -1166,12 +1187,7 @@ __global__ void k_commit_elems(Batch b) {
     int nd = b.enodes[3 * e + j];
     for (int q = 0; q < 6; ++q) d[6 * j + q] = b.disp[(int64_t)nd * 6 + q];
   }
-  BeamConst c = b.bconst[e];
-  BeamHist h = b.bhist[e];
-  BeamHistAux x = b.baux[e];
-  beam_commit(c, h, x, d);
-  b.bhist[e] = h;
-  b.baux[e] = x;
+  beam_commit(b.bconst[e], b.bhist[e], b.baux[e], d, t & 1);
 }
 
 // ... and nodal configuration (reference src/Node.cpp:325-370)
@@ -1271,36 +1287,41 @@ __global__ void k_monitor_record(Batch b) {
   }
 }
 
-// Element-level entry (no batch): tangent and internal force, FP64.
+// Element-level entry (no batch): tangent and internal force, as
+// k_beam_tangent forms them.  The caller's K has an element's 324 entries
+// together, so the CTA's 32 matrices are put together in shared memory (an odd
+// stride apart) and written coalesced.
+constexpr int BE_LD = 325;
+constexpr int BE_SMEM = MOUNT_SMEM + 32 * BE_LD * (int)sizeof(double);
 __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_elements(int n, const BeamConst* cs, const BeamHist* hs,
                                                                  const double* ds, double* Ks, double* fs) {
-  extern __shared__ unsigned char smem_raw[];
-  double* sM = reinterpret_cast<double*>(smem_raw);
-  const int tid = threadIdx.x;
-  int e = blockIdx.x * blockDim.x + tid;
-  if (e >= n) return;
-  const BeamConst& c = cs[e];
-  const BeamHist& h = hs[e];
-  double d[18];
-  for (int q = 0; q < 18; ++q) d[q] = ds[(int64_t)e * 18 + q];
-  BeamInterp ip[2] = {beam_interp(c, d, 0), beam_interp(c, d, 1)};
-  double* f = sM + (size_t)2 * OP_N * MOUNT_THREADS + tid;
-  for (int q = 0; q < 18; ++q) f[q * MOUNT_THREADS] = 0.0;
-#pragma unroll 1
-  for (int g = 0; g < 2; ++g) {
-    BeamGP kin;
-    beam_kinematics(c, h, ip[g], g, kin);
-    beam_gp_force(c, kin, g, f, MOUNT_THREADS);
-    double* M = sM + (size_t)g * OP_N * MOUNT_THREADS + tid;
-    beam_gp_operator<double>(c, kin, M, MOUNT_THREADS);
-    rotate_blocks9<double>(c, M, MOUNT_THREADS);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* P = reinterpret_cast<double*>(smem_raw);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e = blockIdx.x * 32 + lane, g = warp & 1;
+  if (e < n) {
+    if (warp >= 2) {
+      beam_gp_coef(cs[e], g, P + (g * MP_POINT + GP_COUNT) * 32 + lane, 32);
+    } else {
+      double d[18];
+#pragma unroll
+      for (int q = 0; q < 18; ++q) d[q] = ds[(int64_t)e * 18 + q];
+      beam_gp(cs[e], hs[e], d, g, P + g * MP_POINT * 32 + lane, 32);
+    }
   }
-  double* K = Ks + (int64_t)e * 324;
-#pragma unroll 1
-  for (int J = 0; J < 3; ++J)
-#pragma unroll 1
-    for (int I = 0; I < 3; ++I) beam_K_block<double>(c, sM + tid, sM + OP_N * MOUNT_THREADS + tid, I, J, MOUNT_THREADS, K);
-  for (int q = 0; q < 18; ++q) fs[(int64_t)e * 18 + q] = f[q * MOUNT_THREADS];
+  __syncthreads();
+  double* tile = P + 2 * MP_POINT * 32;
+  double* K = tile + lane * BE_LD;
+  if (e < n)
+    beam_expand(P, warp, lane,
+                [&](int r, int q, double v) {
+                  K[r + 18 * q] = v;
+                  K[q + 18 * r] = v;
+                },
+                [&](int q, double v) { fs[(int64_t)e * 18 + q] = v; });
+  __syncthreads();
+  const int64_t k0 = (int64_t)blockIdx.x * 32 * 324;
+  const int m = min(32, n - (int)blockIdx.x * 32) * 324;
+  for (int x = threadIdx.x; x < m; x += MOUNT_THREADS) Ks[k0 + x] = tile[x / 324 * BE_LD + x % 324];
 }
 
 // Element-level inertia (no batch): M (18x18 column-major, global) and F.
@@ -1321,7 +1342,13 @@ __global__ void k_beam_inertia_elements(int n, const BeamConst* cs, const BeamHi
   for (int q = 0; q < 6; ++q) an[q] = a[q];
   for (int g = 0; g < 2; ++g) {
     BeamInterp ip = beam_interp(c, d, g);
-    beam_gp_inertia(c, xs[e], ip, vel, acc, an, g, f, 1, D + 9 * g, 1);
+    double fu[3], fa[3];
+    beam_gp_inertia(c, xs[e], ip, vel, acc, an, g, fu, fa, D + 9 * g, 1);
+    for (int I = 0; I < 3; ++I)
+      for (int i = 0; i < 3; ++i) {
+        f[6 * I + i] += c.jac * c.N[g][I] * fu[i];
+        f[6 * I + 3 + i] += c.jac * c.N[g][I] * fa[i];
+      }
   }
   for (int r = 0; r < 18; ++r)
     for (int q = 0; q < 18; ++q) Ms[(int64_t)e * 324 + r + 18 * q] = beam_M_entry(c, D, D + 9, 1, an[0] * c.Mr, r, q);
@@ -1329,15 +1356,11 @@ __global__ void k_beam_inertia_elements(int n, const BeamConst* cs, const BeamHi
 }
 
 __global__ void k_beam_commit(int n, const BeamConst* cs, BeamHist* hs, BeamHistAux* xs, const double* ds) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, e = t >> 1;
   if (e >= n) return;
   double d[18];
   for (int q = 0; q < 18; ++q) d[q] = ds[(int64_t)e * 18 + q];
-  BeamHist h = hs[e];
-  BeamHistAux x = xs[e];
-  beam_commit(cs[e], h, x, d);
-  hs[e] = h;
-  xs[e] = x;
+  beam_commit(cs[e], hs[e], xs[e], d, t & 1);
 }
 
 }  // namespace
@@ -1358,7 +1381,7 @@ void launch_beam_inertia(int n, const BeamConst* c, const BeamHistAux* x, const 
 }
 
 void launch_beam_commit(int n, const BeamConst* c, BeamHist* h, BeamHistAux* x, const double* d, cudaStream_t st) {
-  if (n > 0) k_beam_commit<<<(n + 127) / 128, 128, 0, st>>>(n, c, h, x, d);
+  if (n > 0) k_beam_commit<<<(n + 63) / 64, 128, 0, st>>>(n, c, h, x, d);
 }
 
 void launch_init_state(const Batch& b, cudaStream_t st) {
@@ -1406,7 +1429,7 @@ void launch_assembly(const Batch& b_in, cudaStream_t st) {
 void launch_increment(const Batch& b, cudaStream_t st) { k_update<<<b.n_chunks, 256, 0, st>>>(b); }
 
 void launch_commit(const Batch& b, cudaStream_t st) {
-  if (b.n_elem) k_commit_elems<<<(b.n_elem + 127) / 128, 128, 0, st>>>(b);
+  if (b.n_elem) k_commit_elems<<<(b.n_elem + 63) / 64, 128, 0, st>>>(b);
   if (b.sh.n_shells) launch_shell_commit(b, st);
   if (b.n_nodes) k_commit_nodes<<<(b.n_nodes + 127) / 128, 128, 0, st>>>(b);
 }
@@ -1416,8 +1439,6 @@ void launch_commit(const Batch& b, cudaStream_t st) {
 // function-local static is initialised by exactly one of them).
 static void set_attrs() {
   static const bool done = [] {
-    cudaFuncSetAttribute(k_beam_tangent<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOUNT_SMEM);
-    cudaFuncSetAttribute(k_beam_tangent<f2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOUNT_SMEM);
     cudaFuncSetAttribute(k_band_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (RING * GF_LDB + RING) * (int)sizeof(double));
     return true;
@@ -1438,13 +1459,9 @@ static void launch_mount(const Batch& b, cudaStream_t st, LaunchProf* prof) {
   if (b.n_elem == 0) return;
   {
     ProfScope q(prof, st, KC_MOUNT);
-    // mixed precision: the tangent operator in FP32-pair arithmetic on the
-    // FP32 pipe; kinematics, internal force and everything after stay FP64
-    const int smem = MOUNT_SMEM;
-    if (b.mixed)
-      k_beam_tangent<f2><<<(b.n_elem + MOUNT_THREADS - 1) / MOUNT_THREADS, MOUNT_THREADS, smem, st>>>(b);
-    else
-      k_beam_tangent<double><<<(b.n_elem + MOUNT_THREADS - 1) / MOUNT_THREADS, MOUNT_THREADS, smem, st>>>(b);
+    // 36.9 KB of shared memory a CTA (44.5 in Dynamic steps), under the 48 KB
+    // that needs no attribute
+    k_beam_tangent<<<(b.n_elem + 31) / 32, MOUNT_THREADS, b.any_dynamic ? MOUNT_SMEM_DYN : MOUNT_SMEM, st>>>(b);
     // the pressure's load stiffness is part of the K_e that Rayleigh damping
     // reads (the reference mounts loads before damping)
     if (b.n_pipe_press) k_pipe_pressure<<<(b.n_pipe_press + 127) / 128, 128, 0, st>>>(b);
@@ -1481,7 +1498,7 @@ void launch_iteration(const Batch& b, cudaStream_t st, bool commit_kernels, Laun
   { ProfScope q(prof, st, KC_UPDATE); k_update<<<b.n_chunks, 256, 0, st>>>(b); }
   { ProfScope q(prof, st, KC_CONTROL); k_control<<<(ns + 127) / 128, 128, 0, st>>>(b); }
   if (commit_kernels) {
-    if (b.n_elem) { ProfScope q(prof, st, KC_COMMIT_ELEMS); k_commit_elems<<<(b.n_elem + 127) / 128, 128, 0, st>>>(b); }
+    if (b.n_elem) { ProfScope q(prof, st, KC_COMMIT_ELEMS); k_commit_elems<<<(b.n_elem + 63) / 64, 128, 0, st>>>(b); }
     if (b.sh.n_shells) { ProfScope q(prof, st, KC_COMMIT_ELEMS); launch_shell_commit(b, st); }
     if (b.n_nodes) { ProfScope q(prof, st, KC_COMMIT_NODES); k_commit_nodes<<<(b.n_nodes + 127) / 128, 128, 0, st>>>(b); }
     if (b.mon_total) k_monitor_record<<<(b.mon_total + 127) / 128, 128, 0, st>>>(b);
@@ -1515,9 +1532,9 @@ void launch_beam_elements(int n, const BeamConst* c, const BeamHist* h, const do
                           double* f, cudaStream_t st) {
   if (n <= 0) return;
   static const bool attr =
-      cudaFuncSetAttribute(k_beam_elements, cudaFuncAttributeMaxDynamicSharedMemorySize, MOUNT_SMEM) == cudaSuccess;
+      cudaFuncSetAttribute(k_beam_elements, cudaFuncAttributeMaxDynamicSharedMemorySize, BE_SMEM) == cudaSuccess;
   (void)attr;
-  k_beam_elements<<<(n + MOUNT_THREADS - 1) / MOUNT_THREADS, MOUNT_THREADS, MOUNT_SMEM, st>>>(n, c, h, d, K, f);
+  k_beam_elements<<<(n + 31) / 32, MOUNT_THREADS, BE_SMEM, st>>>(n, c, h, d, K, f);
 }
 
 }  // namespace gf

@@ -406,16 +406,13 @@ struct Batch {
   // structure
   double* nodeK;
   int full_band;
-  int mixed;  // 1: Beam_1 tangent operator in FP32-pair arithmetic
+  int mixed;  // 1: GF_PREC_MIXED (Shell_1 factor in FP32; Beam_1 is FP64 in either)
   int* running;  // structures still running after the last pass
   // Rayleigh damping matrix per element (18x18, structure-of-arrays: entry
   // x of element e at [x * n_elem + e]); allocated when any_rayleigh
   double* RD;
   int any_rayleigh;
   int any_dynamic;  // a structure has a Dynamic solution step
-  // inertial rotational tangents of the Beam_1 Gauss points (2 x 9 per
-  // element, structure-of-arrays like Ke); allocated when any_dynamic
-  double* Dm;
   // reduction chunks: chunk k covers free DOFs [chunk_start[k],
   // chunk_start[k] + GF_RED_CHUNK) of structure chunk_struct[k]
   int n_chunks;
