@@ -14,6 +14,8 @@
 //                     even positions absorb them; the last survivor is
 //                     solved directly;
 //   4. back substitution level by level, then the midside nodes.
+// Corners may have fixed DOFs (a pinned end): their rows and columns are those
+// of the identity.
 // The critical path is O(log m) small dense solves instead of the O(n)
 // column recurrence of a banded LU, which on a GPU with slow FP64 latency
 // (~64 cycles per dependent FP64 operation) dominates long chains.  The
@@ -30,5 +32,6 @@
 namespace gf {
 
 void launch_chain_solve(const Batch& b, const ChainData& c, cudaStream_t st);
+int chain_launches(const ChainData& c);
 
 }  // namespace gf

@@ -19,6 +19,7 @@
 
 #include "../../include/giraffe_gpu.h"
 #include "gf_host_internal.h"
+#include "gf_chain.cuh"
 #include "gf_kernels.cuh"
 #include "gf_types.h"
 
@@ -393,7 +394,7 @@ struct StructPlan {
   std::vector<int> active, c6, g6;  // per node DOF: element-activated, constrained, free index (-1 fixed, -2 inactive)
   std::vector<int> dofs;            // local node DOF (6 node + k) of each free index, in the solver's order
   std::vector<int> perm;            // wide structures: the reference's free index -> the solver's
-  std::vector<char> node_free;      // chain structures: node fully free
+  std::vector<char> node_free;      // chain structures: node with free DOFs
   int nf = 0, kb = 0, kl_nat = 0, wkl = 0;
   bool has_f = false, has_m = false, wide = false, chain = false;
   FrontPlan fronts;                 // wide structures: the multifrontal LU's plan
@@ -616,8 +617,8 @@ void plan_structure(const gf_model_desc& m, int s, bool want_fronts, StructPlan&
         return;
       }
     }
-  // chain structure: elements on nodes (2e, 2e+1, 2e+2), every node fully
-  // free or fully fixed, midside and interior corner nodes free
+  // chain structure: elements on nodes (2e, 2e+1, 2e+2), midside nodes fully
+  // free and interior corners not fully fixed
   bool chain = m.n_beams > 0 && nn == 2 * m.n_beams + 1;
   for (int e = 0; chain && e < m.n_beams; ++e)
     chain = m.beams[6 * e] == 2 * e && m.beams[6 * e + 1] == 2 * e + 1 && m.beams[6 * e + 2] == 2 * e + 2;
@@ -625,10 +626,8 @@ void plan_structure(const gf_model_desc& m, int s, bool want_fronts, StructPlan&
   for (int i = 0; chain && i < nn; ++i) {
     int f = 0;
     for (int k = 0; k < 6; ++k) f += g6[6 * i + k] >= 0;
-    if (f != 0 && f != 6) chain = false;
-    P.node_free[i] = f == 6;
-    bool interior = i > 0 && i < nn - 1;
-    if (interior && !P.node_free[i]) chain = false;
+    P.node_free[i] = f > 0;
+    if (i % 2 ? f != 6 : (i > 0 && i < nn - 1 && f == 0)) chain = false;
   }
   P.chain = chain;
 }
@@ -996,6 +995,18 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       start = so.end_time;
     }
     params[s] = step_params[inf.step_off];
+    // K_AA of a chain is symmetric in Static steps unless a load adds its own
+    // stiffness: a pipe pressure (pipe_pressed) or a nodal moment
+    bool sym = inf.is_chain && pipe_pressed.empty();
+    for (int k = inf.step_off; k < inf.step_off + inf.n_steps; ++k) sym = sym && !step_params[k].dynamic;
+    for (int l = 0; l < m.n_loads && sym; ++l)
+      if (m.loads[l].type == GF_LOAD_NODAL) {
+        const gf_table& t = m.loads[l].table;
+        for (int i = 0; i < t.n_times && sym; ++i)
+          for (int q = 3; q < 6; ++q) sym = sym && t.values[(size_t)i * t.n_cols + q] == 0.0;
+      }
+    inf.sym = sym;
+    if (inf.is_chain) (sym ? b.chain.any_sym : b.chain.any_general) = 1;
   }
   b.n_struct = n;
   b.n_nodes = node_off;
@@ -1045,7 +1056,7 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       if (l < NL) { o += ocnt[l]; e += ecnt[l]; }
     }
     hvec<int> elem_list(n_t), eca(n_t), ecb(n_t), cnode(n_c), cstruct(n_c), cleft(n_c), cright(n_c), cprev(n_c),
-        cnext(n_c), roots(n_roots);
+        cnext(n_c), roots(n_roots), emask(n_t), cmask(n_c);
     hvec<CrItem> odd(cd.odd_off[NL]), even(cd.even_off[NL]);
     parallel_structures(n, work, [&](int s) {
       if (!plan[s].chain) return;
@@ -1067,6 +1078,11 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
         for (int h = hmax; h >= 1 && M > 1; h /= 2)
           for (int kp = h; kp < M; kp += 2 * h) slot[kp] = r++;
       }
+      auto mask6 = [&](int node) {
+        int k = 0;
+        for (int q = 0; q < 6; ++q) k |= (plan[s].g6[6 * node + q] >= 0) << q;
+        return k;
+      };
       std::vector<int> pos(mm + 1, -1);
       for (int ci = 0, k = 0; ci <= mm; ++ci)
         if (fr[2 * ci]) pos[ci] = slot[k++];
@@ -1074,12 +1090,14 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
         elem_list[tbase + e] = inf.elem_off + e;
         eca[tbase + e] = pos[e] >= 0 ? cbase + pos[e] : -1;
         ecb[tbase + e] = pos[e + 1] >= 0 ? cbase + pos[e + 1] : -1;
+        emask[tbase + e] = mask6(2 * e) | mask6(2 * e + 2) << 6;
       }
       for (int ci = 0, k = 0; ci <= mm; ++ci) {
         if (pos[ci] < 0) continue;
         const int c = cbase + pos[ci];
         cnode[c] = inf.node_off + 2 * ci;
         cstruct[c] = s;
+        cmask[c] = mask6(2 * ci);
         cleft[c] = ci >= 1 ? tbase + ci - 1 : -1;
         cright[c] = ci < mm ? tbase + ci : -1;
         cprev[c] = k > 0 ? cbase + slot[k - 1] : -1;
@@ -1110,9 +1128,11 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
           !upload(B, &cd.corner_struct, cstruct) || !upload(B, &cd.corner_left, cleft) ||
           !upload(B, &cd.corner_right, cright) || !upload(B, &cd.corner_prev, cprev) ||
           !upload(B, &cd.corner_next, cnext) || !upload(B, &cd.odd, odd) || !upload(B, &cd.even, even) ||
-          !upload(B, &cd.roots, roots) || !balloc(B, &cd.ez, ne * 78) || !balloc(B, &cd.ec, ne * 156) ||
-          !balloc(B, &cd.cD, nc * 36) || !balloc(B, &cd.cL, nc * 36) || !balloc(B, &cd.cU, nc * 36) ||
-          !balloc(B, &cd.cb, nc * 6) || !balloc(B, &cd.cz, nc * 78) || !balloc(B, &cd.cx, nc * 6))
+          !upload(B, &cd.roots, roots) || !upload(B, &cd.elem_mask, emask) || !upload(B, &cd.corner_mask, cmask) ||
+          !balloc(B, &cd.ez, ne * (cd.any_sym ? 99 : 78)) || !balloc(B, &cd.ec, ne * (cd.any_general ? 156 : 90)) ||
+          !balloc(B, &cd.cD, nc * (cd.any_general ? 36 : 21)) || !balloc(B, &cd.cL, nc * (cd.any_general ? 36 : 0)) ||
+          !balloc(B, &cd.cU, nc * 36) || !balloc(B, &cd.cb, nc * 6) || !balloc(B, &cd.cz, nc * (cd.any_sym ? 99 : 78)) ||
+          !balloc(B, &cd.ce, nc * (cd.any_general ? 114 : 90)) || !balloc(B, &cd.cx, nc * 6))
         return GF_ERR_CUDA;
     }
   }
@@ -1213,8 +1233,13 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       !dup(B, &B->copy0, b.copy, copy.size()) || !dup(B, &B->Qn0, b.Qn, Qn.size()) ||
       !dup(B, &B->bhist0, b.bhist, bhist.size()) || !dup(B, &B->baux0, b.baux, baux.size()))
     return GF_ERR_CUDA;
+  // the 35-row band and its factor, which only beam structures that are not
+  // chains solve with (the assembly views add the band when they are asked for)
+  bool banded = B->band_view;
+  for (int s = 0; s < n; ++s) banded = banded || (models[s].n_beams && !plan[s].chain);
+  B->band_total = (size_t)std::max(dof_off, 1) * GF_LDB;
   if (!balloc(B, &b.P, (size_t)dof_off) || !balloc(B, &b.y, (size_t)dof_off) ||
-      !balloc(B, &b.band, (size_t)dof_off * GF_LDB) || !balloc(B, &b.U, (size_t)dof_off * GF_UW) ||
+      (banded && (!balloc(B, &b.band, B->band_total) || !balloc(B, &b.U, (size_t)dof_off * GF_UW))) ||
       !balloc(B, &b.state, (size_t)n) || !balloc(B, &b.running, 1) ||
       !balloc(B, &b.Ke, (size_t)elem_off * 324) || !balloc(B, &b.Fe, (size_t)elem_off * 18) ||
       !balloc(B, &b.nodeK, (size_t)std::max(node_off, 1) * 9) ||
@@ -1240,7 +1265,7 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
   B->h_gl = std::move(gl);
   B->h_enodes = std::move(enodes);
   B->h_snodes = std::move(snodes);
-  CK(cudaMemsetAsync(b.band, 0, sizeof(double) * (size_t)std::max(dof_off, 1) * GF_LDB, B->stream));
+  if (b.band) CK(cudaMemsetAsync(b.band, 0, sizeof(double) * B->band_total, B->stream));
   CK(cudaMemsetAsync(b.P, 0, sizeof(double) * (size_t)std::max(dof_off, 1), B->stream));
   CK(cudaMemsetAsync(b.nodeK, 0, sizeof(double) * (size_t)std::max(node_off, 1) * 9, B->stream));
   b.mixed = B->opts.precision == GF_PREC_MIXED;
@@ -1270,16 +1295,7 @@ int count_launches_per_pass(const gf_batch* B) {
   const ChainData& cd = B->b.chain;
   // chains only: one gather launch in place of the colour passes
   if (B->b.n_elem && !B->b.full_band && cd.n_chain_elems == B->b.n_elem) colors = 1;
-  int chain_launches = 0;
-  if (cd.n_chain_elems) {
-    chain_launches = 2;
-    if (cd.n_corners) {
-      chain_launches += 3;
-      for (int l = 0; l < cd.n_levels; ++l)
-        chain_launches += 2 * (cd.odd_off[l + 1] > cd.odd_off[l]) + (cd.even_off[l + 1] > cd.even_off[l]);
-    }
-  }
-  return 10 + colors + chain_launches + shell_launches_per_pass(B->b) + (B->b.any_rayleigh ? 1 : 0) +
+  return 10 + colors + chain_launches(cd) + shell_launches_per_pass(B->b) + (B->b.any_rayleigh ? 1 : 0) +
          (B->b.n_pipe_press ? 1 : 0) + (B->b.mon_total ? 1 : 0);
 }
 
@@ -1927,6 +1943,10 @@ int first_pass_band(gf_batch* B, int s, std::vector<double>& band, std::vector<d
   if (r != GF_OK) return r;
   // the wide band of Shell_1 structures, which their solver does not keep
   if (b.sh.n_wide && !b.sh.wband && !balloc(B, &B->b.sh.wband, (size_t)B->wb_total)) return GF_ERR_CUDA;
+  if (!b.band) {
+    if (!balloc(B, &B->b.band, B->band_total)) return GF_ERR_CUDA;
+    CK(cudaMemsetAsync(B->b.band, 0, sizeof(double) * B->band_total, B->stream));
+  }
   // one partial pass: step start, zero, mount, loads, residual
   Batch bb = b;
   launch_iteration_partial(bb, B->stream);

@@ -164,6 +164,7 @@ struct gf_batch {
   size_t counted_bytes = 0;
   // host copies needed for results and resets
   std::vector<gf::StructInfo> info;
+  size_t band_total = 0;  // entries of the 35-row bands
   int64_t wb_total = 0;  // entries of the Shell_1 structures' wide bands
   std::vector<int> kb;  // true half-bandwidth per structure
   std::vector<void*> allocs;

@@ -393,10 +393,13 @@ __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
   const int64_t ne = b.n_elem;
   const double* Cf = P + GP_COUNT * 32 + lane;
   if (!dyn) {
+    // the symmetric chain elimination reads the lower triangle
+    const bool half = b.info[s].sym && !b.full_band;
     beam_expand(P, warp, lane,
                 [&](int r, int q, double v) {
-                  Ke[(r + 18 * q) * ne] = v;
-                  if (r != q) Ke[(q + 18 * r) * ne] = v;
+                  const int lo = r < q ? r : q, hi = r < q ? q : r;
+                  Ke[(hi + 18 * lo) * ne] = v;
+                  if (!half && hi != lo) Ke[(lo + 18 * hi) * ne] = v;
                 },
                 [&](int q, double v) { b.Fe[q * ne + e] = v; });
     return;

@@ -118,6 +118,8 @@ struct StructInfo {
   int has_force, has_moment;  // free translational / rotational DOFs exist
   int load_off, n_loads;  // nodal load entries of this structure
   int is_chain;  // solved by the chain solver (else by the band LU)
+  int sym;       // a chain whose K_AA is symmetric: Static steps only, no pipe
+                 // pressure and no nodal moments (whose stiffness is not)
   // wide-band structures (Shell_1): K_AA column-major with 2 wkl + 1 rows,
   // entry (i, j) at wband[wb_off + (wkl + i - j) + j (2 wkl + 1)]; the free
   // DOFs are numbered in reverse Cuthill-McKee node order
@@ -217,6 +219,9 @@ struct ChainData {
   int* elem_list;      // batch element ids of chain elements
   int* elem_corner_a;  // corner index of the element's first corner (-1 if fixed)
   int* elem_corner_b;  // corner index of the element's last corner (-1 if fixed)
+  int* elem_mask;      // free DOFs of the element's corners: bits 0-5 the first, 6-11 the last
+  int* corner_mask;    // free DOFs of the corner (bits 0-5)
+  int any_general, any_sym;  // chains of either kind in the batch
   int* corner_node;    // batch node id of each free corner
   int* corner_struct;
   int* corner_left;    // chain element to the left (-1 if none)
@@ -224,13 +229,15 @@ struct ChainData {
   int* corner_prev;    // previous free corner of the same chain (-1 if none)
   int* corner_next;    // next free corner (-1 if none)
   // scratch below is structure-of-arrays: entry x of item i at [x * n_items + i]
-  double* ez;          // [6*13][chain elem]  Z_s = A_ss^{-1}[b_s | A_sa | A_sb]
-  double* ec;          // [6*26][chain elem]  -A_as Z_s (13 cols), -A_bs Z_s (13 cols)
+  // (general elimination, then symmetric elimination)
+  double* ez;          // [6*13][chain elem]  Z_s = A_ss^{-1}[b_s | A_sa | A_sb]; [99] W, multipliers, reciprocals
+  double* ec;          // [6*26][chain elem]  -A_as Z_s (13 cols), -A_bs Z_s (13 cols); [90] contributions
   double* cD;          // [36][corner] (row-major 6x6 per corner)
   double* cL;          // [36][corner]
   double* cU;          // [36][corner]
   double* cb;          // [6][corner]
-  double* cz;          // [6*13][corner]  Z = D^{-1}[b | L | U] of an eliminated corner
+  double* cz;          // [6*13][corner]  Z = D^{-1}[b | L | U] of an eliminated corner; [99] as ez
+  double* ce;          // [114][corner]  outputs of the entry-per-thread update; [90] as ec
   double* cx;          // [6][corner]  solution
   CrItem* odd;         // per level: eliminated positions
   int odd_off[CR_MAX_LEVELS + 1];
