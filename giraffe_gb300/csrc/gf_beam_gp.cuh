@@ -286,6 +286,23 @@ GF_HD void beam_gp_coef(const BeamConst& c, int g, double* o, int os) {
     }
 }
 
+// Coefficients of the translations written as du = u_2 - u_0 and v = u_1 - (u_0 +
+// u_2) / 2, whose shape derivatives are N'_2 + N'_1 / 2 and N'_1: w D D, w D V, w
+// V V, then w D N_J and w V N_J.
+constexpr int GS_DD = 0, GS_DV = 1, GS_VV = 2, GS_DN = 3, GS_VN = 6, GS_COUNT = 9;
+GF_HD void beam_gp_coef_sym(const BeamConst& c, int g, double* o, int os) {
+  const double V = c.dN[g][1], D = rfma(0.5, V, c.dN[g][2]);
+  const double wD = rmul(c.jac, D), wV = rmul(c.jac, V);
+  o[GS_DD * os] = rmul(wD, D);
+  o[GS_DV * os] = rmul(wD, V);
+  o[GS_VV * os] = rmul(wV, V);
+#pragma unroll
+  for (int J = 0; J < 3; ++J) {
+    o[(GS_DN + J) * os] = rmul(wD, c.N[g][J]);
+    o[(GS_VN + J) * os] = rmul(wV, c.N[g][J]);
+  }
+}
+
 // Index of entry (i, j), i <= j, of a 3x3 upper triangle, and of either order.
 GF_HD int tri3(int i, int j) { return i <= j ? 3 * i - (i * (i - 1)) / 2 + j - i : 3 * j - (j * (j - 1)) / 2 + i - j; }
 

@@ -1,17 +1,12 @@
-// Chain solver kernels (see gf_chain.cuh).
-//
-// Two eliminations share the structure: the general one (Gauss-Jordan on
-// [D | b | L | U]) and, for structures whose K_AA is symmetric (StructInfo::
-// sym: Static steps without load stiffness), an LDL^T one that forms half of
-// every product: about 870 FP64 operations per condensed midside node or
-// eliminated corner against 1,520.  Each has two forms with the same
+// Chain solver kernels (see gf_chain.cuh): the general elimination, for Dynamic
+// steps and loads with stiffness of their own (the symmetric one is in
+// gf_chain_sym.cu).  Gauss-Jordan on [D | b | L | U], in two forms with the same
 // operations on every entry, so the same bits: one item per thread, whose FP64
 // warp instructions carry 32 items, for the large levels, and one item per
 // warp for the small ones, where an item's chain of dependent operations (64
 // cycles each on this part) is what counts.
 #include <cuda_runtime.h>
 
-#include "gf_beam_gp.cuh"
 #include "gf_chain.cuh"
 #include "gf_math.cuh"
 
@@ -100,7 +95,6 @@ __global__ void __launch_bounds__(CT) k_condense(Batch b, ChainData c) {
   int s = b.estruct[e];
   if (!solving(b, s)) return;
   const StructInfo& inf = b.info[s];
-  if (inf.sym) return;
   const double* P = b.P + inf.dof_off;
   double D[36];  // K_mm (+ the load stiffness)
   // K of the chain comes from the element tangents (column-major 18x18,
@@ -171,7 +165,6 @@ __global__ void __launch_bounds__(128) k_condense_w(Batch b, ChainData c) {
   const int e = c.elem_list[t], s = b.estruct[e];
   if (!solving(b, s)) return;
   const StructInfo& inf = b.info[s];
-  if (inf.sym) return;
   const double* P = b.P + inf.dof_off;
   const double* Kb = b.Ke + e;
   const int64_t ne = b.n_elem;
@@ -240,7 +233,6 @@ __global__ void k_corner_system(Batch b, ChainData c) {
   const int s = c.corner_struct[k];
   if (!solving(b, s)) return;
   const StructInfo& inf = b.info[s];
-  if (inf.sym) return;
   const int x = blockIdx.y % 36, i = x / 6, j = x % 6, part = blockIdx.y / 36;
   const int node = c.corner_node[k], eL = c.corner_left[k], eR = c.corner_right[k];
   const int64_t ne = b.n_elem;
@@ -286,7 +278,7 @@ __global__ void __launch_bounds__(CT) k_cr_eliminate(Batch b, ChainData c, int l
   int t = lo + blockIdx.x * CT + threadIdx.x;
   if (t >= hi) return;
   CrItem it = c.odd[t];
-  if (!solving(b, it.structure) || b.info[it.structure].sym) return;
+  if (!solving(b, it.structure)) return;
   int k = it.corner;
   double D[36];
 #pragma unroll
@@ -320,7 +312,7 @@ __global__ void k_cr_eliminate_w(Batch b, ChainData c, int lo, int hi) {
   const int t = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (t >= hi) return;
   CrItem it = c.odd[t];
-  if (!solving(b, it.structure) || b.info[it.structure].sym) return;
+  if (!solving(b, it.structure)) return;
   const int k = it.corner;
   double col[6];
 #pragma unroll
@@ -415,7 +407,7 @@ __global__ void k_cr_update_w(Batch b, ChainData c, int lo, int hi) {
   const int t = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
   if (t >= hi) return;
   CrItem it = c.even[t];
-  if (!solving(b, it.structure) || b.info[it.structure].sym) return;
+  if (!solving(b, it.structure)) return;
   cr_update_row(c, it, lane % 6);
 }
 
@@ -427,7 +419,7 @@ __global__ void k_cr_update_e(Batch b, ChainData c, int lo, int hi) {
   const int t = lo + blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= hi) return;
   const CrItem it = c.even[t];
-  if (!solving(b, it.structure) || b.info[it.structure].sym) return;
+  if (!solving(b, it.structure)) return;
   const int k = it.corner, i = blockIdx.y / 19, o = blockIdx.y % 19, q = (o - 1) % 6, what = o == 0 ? 0 : 1 + (o - 1) / 6;
   double v = what == 0 ? CRN(c.cb, k, i) : what == 1 ? CRN(c.cD, k, i * 6 + q) : 0.0;
   if (it.next >= 0 && what != 3) {
@@ -446,7 +438,7 @@ __global__ void k_cr_update_e2(Batch b, ChainData c, int lo, int hi) {
   const int t = lo + blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= hi) return;
   const CrItem it = c.even[t];
-  if (!solving(b, it.structure) || b.info[it.structure].sym) return;
+  if (!solving(b, it.structure)) return;
   const int k = it.corner, i = blockIdx.y / 19, o = blockIdx.y % 19, q = (o - 1) % 6;
   const double v = CRN(c.ce, k, blockIdx.y);
   if (o == 0) CRN(c.cb, k, i) = v;
@@ -461,7 +453,7 @@ __global__ void __launch_bounds__(CT) k_cr_root(Batch b, ChainData c) {
   if (t >= c.n_roots) return;
   int k = c.roots[t];
   int s = c.corner_struct[k];
-  if (!solving(b, s) || b.info[s].sym) return;
+  if (!solving(b, s)) return;
   double D[36], r[6];
 #pragma unroll
   for (int q = 0; q < 36; ++q) D[q] = CRN(c.cD, k, q);
@@ -482,7 +474,7 @@ __global__ void k_cr_back(Batch b, ChainData c, int lo, int hi) {
   const int t = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
   if (t >= hi) return;
   CrItem it = c.odd[t];
-  if (!solving(b, it.structure) || b.info[it.structure].sym) return;
+  if (!solving(b, it.structure)) return;
   const int k = it.corner, i = lane % 6;
   double x = CRN(c.cz, k, i * 13);
 #pragma unroll
@@ -503,7 +495,6 @@ __global__ void k_chain_scatter(Batch b, ChainData c) {
   int s = b.estruct[e];
   if (!solving(b, s)) return;
   const StructInfo& inf = b.info[s];
-  if (inf.sym) return;
   double* P = b.P + inf.dof_off;
   int ka = c.elem_corner_a[t], kb = c.elem_corner_b[t];
   double xa[6], xb[6];
@@ -540,393 +531,21 @@ __global__ void k_corner_scatter(Batch b, ChainData c) {
   }
 }
 
-// ---- the symmetric elimination ----
-// One item: the 6x6 matrix D (lower triangle) and 13 right-hand columns R = [b |
-// to the first neighbour a | to the second neighbour b].  D = L E L^T, W = L^-1
-// R, and the item's contributions -W^T E^-1 W to its neighbours: b_a, b_b, the
-// triangles aa and bb and the block ab, 90 values.  W, the multipliers and the
-// reciprocals of E (99 values) are kept for the back substitution.
-constexpr int SY_RA = 0, SY_RB = 6, SY_AA = 12, SY_AB = 33, SY_BB = 69, SY_OUT = 90;
-constexpr int SY_M = 78, SY_R = 93, SY_KEEP = 99;
-
-// (p, q), p <= q, of output o among the columns 0 (b), 1-6 (a), 7-12 (b side)
-__device__ __forceinline__ void sy_pair(int o, int& p, int& q) {
-  if (o < SY_AA) {
-    p = 0;
-    q = 1 + o;
-  } else if (o < SY_AB || o >= SY_BB) {
-    int x = o < SY_AB ? o - SY_AA : o - SY_BB, i = 0;
-    while (x > i) x -= ++i;  // row i, column x of the lower triangle
-    const int c0 = o < SY_AB ? 1 : 7;
-    p = c0 + x;
-    q = c0 + i;
-  } else {
-    p = 1 + (o - SY_AB) / 6;
-    q = 7 + (o - SY_AB) % 6;
-  }
-}
-
-__device__ __forceinline__ constexpr int lo6(int i, int j) { return i * (i + 1) / 2 + j; }
-
-// An item per thread.  load_d(i, j), j <= i; load_r(i, q); keep(x, v); out(o, v).
-template <typename LD, typename LR, typename Keep, typename Out>
-__device__ __forceinline__ bool sy_item(LD load_d, LR load_r, Keep keep, Out out) {
-  double D[21], r[6], m[15];
-#pragma unroll
-  for (int i = 0; i < 6; ++i)
-#pragma unroll
-    for (int j = 0; j <= i; ++j) D[lo6(i, j)] = load_d(i, j);
-  bool ok = true;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const double p = D[lo6(k, k)];
-    if (!(p != 0.0) || !isfinite(p)) ok = false;
-    r[k] = recip(p);
-#pragma unroll
-    for (int i = k + 1; i < 6; ++i) {
-      const double mi = rmul(D[lo6(i, k)], r[k]);
-      m[lo6(i - 1, k)] = mi;
-#pragma unroll
-      for (int j = k + 1; j <= i; ++j) D[lo6(i, j)] = rfma(-mi, D[lo6(j, k)], D[lo6(i, j)]);
-    }
-  }
-#pragma unroll
-  for (int x = 0; x < 15; ++x) keep(SY_M + x, m[x]);
-#pragma unroll
-  for (int k = 0; k < 6; ++k) keep(SY_R + k, r[k]);
-  double W[13][6];
-#pragma unroll
-  for (int q = 0; q < 13; ++q) {
-#pragma unroll
-    for (int i = 0; i < 6; ++i) W[q][i] = load_r(i, q);
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-#pragma unroll
-      for (int i = k + 1; i < 6; ++i) W[q][i] = rfma(-m[lo6(i - 1, k)], W[q][k], W[q][i]);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) keep(i * 13 + q, W[q][i]);
-  }
-#pragma unroll
-  for (int q = 1; q < 13; ++q) {
-    double v[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) v[i] = rmul(r[i], W[q][i]);
-#pragma unroll
-    for (int p = 0; p <= q; ++p) {
-      double acc = rmul(W[p][0], v[0]);
-#pragma unroll
-      for (int i = 1; i < 6; ++i) acc = rfma(W[p][i], v[i], acc);
-      const int o = p == 0 ? q - 1
-                  : q < 7  ? SY_AA + lo6(q - 1, p - 1)
-                  : p < 7  ? SY_AB + (p - 1) * 6 + q - 7
-                           : SY_BB + lo6(q - 7, p - 7);
-      out(o, -acc);
-    }
-  }
-  return ok;
-}
-
-// An item per warp: lane q < 13 holds column q of R, lane 13 + j column j of D
-// (rows from j on); W and E^-1 W go through shared memory (ws) to the lanes
-// that form the outputs.
-template <typename LD, typename LR, typename Keep, typename Out>
-__device__ __forceinline__ bool sy_item_w(int lane, double (*ws)[13][6], LD load_d, LR load_r, Keep keep, Out out) {
-  const int dj = lane - 13;  // column of D (0..5)
-  const bool rhs = lane < 13, mat = dj >= 0 && dj < 6;
-  double col[6], r[6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) col[i] = rhs ? load_r(i, lane) : (mat && i >= dj ? load_d(i, dj) : 0.0);
-  bool ok = true;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const double p = __shfl_sync(0xffffffffu, col[k], 13 + k);
-    if (!(p != 0.0) || !isfinite(p)) ok = false;
-    r[k] = recip(p);
-    double d[6], x = col[k];
-#pragma unroll
-    for (int i = k + 1; i < 6; ++i) {
-      d[i] = __shfl_sync(0xffffffffu, col[i], 13 + k);
-      if (dj == i) x = d[i];
-    }
-#pragma unroll
-    for (int i = k + 1; i < 6; ++i) {
-      const double mi = rmul(d[i], r[k]);
-      if (lane == 31) keep(SY_M + lo6(i - 1, k), mi);
-      if (rhs || (mat && dj > k && i >= dj)) col[i] = rfma(-mi, x, col[i]);
-    }
-    if (lane == 31) keep(SY_R + k, r[k]);
-  }
-  if (rhs)
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      ws[0][lane][i] = col[i];
-      ws[1][lane][i] = rmul(r[i], col[i]);
-      keep(i * 13 + lane, col[i]);
-    }
-  __syncwarp();
-  for (int o = lane; o < SY_OUT; o += 32) {
-    int p, q;
-    sy_pair(o, p, q);
-    double acc = rmul(ws[0][p][0], ws[1][q][0]);
-#pragma unroll
-    for (int i = 1; i < 6; ++i) acc = rfma(ws[0][p][i], ws[1][q][i], acc);
-    out(o, -acc);
-  }
-  __syncwarp();
-  return ok;
-}
-
-// Condensation of the midside node of element t.
-struct SymCondense {
-  const Batch& b;
-  const ChainData& c;
-  int t, mask, nm;
-  const double *K, *P;
-  int64_t ne;
-  __device__ bool init(int t_) {
-    t = t_;
-    const int e = c.elem_list[t], s = b.estruct[e];
-    if (!solving(b, s)) return false;
-    const StructInfo& inf = b.info[s];
-    if (!inf.sym) return false;
-    mask = c.elem_mask[t];
-    nm = b.enodes[3 * e + 1];
-    K = b.Ke + e;
-    P = b.P + inf.dof_off;
-    ne = b.n_elem;
-    return true;
-  }
-  // the lower triangle of K_e is what the tangent writes
-  __device__ double d(int i, int j) const { return K[((6 + i) + 18 * (6 + j)) * ne]; }
-  __device__ double r(int i, int q) const {
-    if (q == 0) return P[b.gl[(int64_t)nm * 6 + i]];
-    if (!(mask >> (q - 1) & 1)) return 0.0;
-    return q < 7 ? K[((6 + i) + 18 * (q - 1)) * ne] : K[((5 + q) + 18 * (6 + i)) * ne];
-  }
-  __device__ void keep(int x, double v) const { ELM(c.ez, t, x) = v; }
-  __device__ void out(int o, double v) const { ELM(c.ec, t, o) = v; }
-  __device__ void fail() const { b.state[b.estruct[c.elem_list[t]]].info_fail = 1; }
-};
-// Elimination of an odd corner: a the corner before it, b the one after.
-struct SymEliminate {
-  const Batch& b;
-  const ChainData& c;
-  CrItem it;
-  __device__ bool init(int t) {
-    it = c.odd[t];
-    return solving(b, it.structure) && b.info[it.structure].sym;
-  }
-  __device__ double d(int i, int j) const { return CRN(c.cD, it.corner, lo6(i, j)); }
-  __device__ double r(int i, int q) const {
-    if (q == 0) return CRN(c.cb, it.corner, i);
-    if (q < 7) return it.prev >= 0 ? CRN(c.cU, it.prev, (q - 1) * 6 + i) : 0.0;
-    return it.next >= 0 ? CRN(c.cU, it.corner, i * 6 + q - 7) : 0.0;
-  }
-  __device__ void keep(int x, double v) const { CRN(c.cz, it.corner, x) = v; }
-  __device__ void out(int o, double v) const { CRN(c.ce, it.corner, o) = v; }
-  __device__ void fail() const { b.state[it.structure].info_fail = 1; }
-};
-
-template <typename Item> __global__ void __launch_bounds__(CT) k_sy(Batch b, ChainData c, int lo, int hi) {
-  const int t = lo + blockIdx.x * CT + threadIdx.x;
-  if (t >= hi) return;
-  Item I{b, c};
-  if (!I.init(t)) return;
-  const bool ok = sy_item([&](int i, int j) { return I.d(i, j); }, [&](int i, int q) { return I.r(i, q); },
-                          [&](int x, double v) { I.keep(x, v); }, [&](int o, double v) { I.out(o, v); });
-  if (!ok) I.fail();
-}
-template <typename Item> __global__ void __launch_bounds__(128) k_sy_w(Batch b, ChainData c, int lo, int hi) {
-  __shared__ double ws[4][2][13][6];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lo + blockIdx.x * 4 + warp;
-  if (t >= hi) return;
-  Item I{b, c};
-  if (!I.init(t)) return;
-  const bool ok = sy_item_w(lane, ws[warp], [&](int i, int j) { return I.d(i, j); },
-                            [&](int i, int q) { return I.r(i, q); }, [&](int x, double v) { I.keep(x, v); },
-                            [&](int o, double v) { I.out(o, v); });
-  if (!ok && lane == 0) I.fail();
-}
-
-// Corner system, entry blockIdx.y of a corner per thread: 0-20 D (lower
-// triangle), 21-56 U (to the next corner), 57-62 b.
-__global__ void k_sy_corner(Batch b, ChainData c) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= c.n_corners) return;
-  const int s = c.corner_struct[k];
-  if (!solving(b, s)) return;
-  const StructInfo& inf = b.info[s];
-  if (!inf.sym) return;
-  const int eL = c.corner_left[k], eR = c.corner_right[k], mask = c.corner_mask[k];
-  const int64_t ne = b.n_elem;
-  int x = blockIdx.y;
-  if (x < 21) {
-    int i = 0, j = x;
-    while (j > i) j -= ++i;
-    double d = i == j ? 1.0 : 0.0;
-    if ((mask >> i & 1) && (mask >> j & 1)) {
-      const double kl = eL >= 0 ? b.Ke[((12 + i) + 18 * (12 + j)) * ne + c.elem_list[eL]] : 0.0;
-      const double kr = eR >= 0 ? b.Ke[(i + 18 * j) * ne + c.elem_list[eR]] : 0.0;
-      d = radd(kl, kr);
-      if (eL >= 0) d = radd(d, ELM(c.ec, eL, SY_BB + x));
-      if (eR >= 0) d = radd(d, ELM(c.ec, eR, SY_AA + x));
-    }
-    CRN(c.cD, k, x) = d;
-  } else if (x < 57) {
-    x -= 21;
-    const int i = x / 6, j = x % 6, kn = c.corner_next[k];
-    CRN(c.cU, k, x) = kn >= 0 && (mask >> i & 1) && (c.corner_mask[kn] >> j & 1)
-                          ? radd(b.Ke[((12 + j) + 18 * i) * ne + c.elem_list[eR]], ELM(c.ec, eR, SY_AB + x))
-                          : 0.0;
-  } else {
-    const int i = x - 57, g = b.gl[(int64_t)c.corner_node[k] * 6 + i];
-    double v = 0.0;
-    if (g >= 0) {
-      v = b.P[inf.dof_off + g];
-      if (eL >= 0) v = radd(v, ELM(c.ec, eL, SY_RB + i));
-      if (eR >= 0) v = radd(v, ELM(c.ec, eR, SY_RA + i));
-    }
-    CRN(c.cb, k, i) = v;
-  }
-}
-
-// Surviving positions absorb their neighbours' contributions, an entry per
-// thread (as k_sy_corner).
-__global__ void k_sy_update(Batch b, ChainData c, int lo, int hi) {
-  const int t = lo + blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= hi) return;
-  const CrItem it = c.even[t];
-  if (!solving(b, it.structure) || !b.info[it.structure].sym) return;
-  const int k = it.corner, x = blockIdx.y;
-  if (x < 21) {
-    double d = CRN(c.cD, k, x);
-    if (it.next >= 0) d = radd(d, CRN(c.ce, it.next, SY_AA + x));
-    if (it.prev >= 0) d = radd(d, CRN(c.ce, it.prev, SY_BB + x));
-    CRN(c.cD, k, x) = d;
-  } else if (x < 57) {
-    if (it.next >= 0) CRN(c.cU, k, x - 21) = CRN(c.ce, it.next, SY_AB + x - 21);
-  } else {
-    const int i = x - 57;
-    double v = CRN(c.cb, k, i);
-    if (it.next >= 0) v = radd(v, CRN(c.ce, it.next, SY_RA + i));
-    if (it.prev >= 0) v = radd(v, CRN(c.ce, it.prev, SY_RB + i));
-    CRN(c.cb, k, i) = v;
-  }
-}
-
-__global__ void __launch_bounds__(CT) k_sy_root(Batch b, ChainData c) {
-  const int t = blockIdx.x * CT + threadIdx.x;
-  if (t >= c.n_roots) return;
-  const int k = c.roots[t], s = c.corner_struct[k];
-  if (!solving(b, s) || !b.info[s].sym) return;
-  double D[21], y[6], r[6], m[15];
-#pragma unroll
-  for (int x = 0; x < 21; ++x) D[x] = CRN(c.cD, k, x);
-#pragma unroll
-  for (int i = 0; i < 6; ++i) y[i] = CRN(c.cb, k, i);
-  bool ok = true;
-#pragma unroll
-  for (int q = 0; q < 6; ++q) {
-    const double p = D[lo6(q, q)];
-    if (!(p != 0.0) || !isfinite(p)) ok = false;
-    r[q] = recip(p);
-#pragma unroll
-    for (int i = q + 1; i < 6; ++i) {
-      const double mi = rmul(D[lo6(i, q)], r[q]);
-      m[lo6(i - 1, q)] = mi;
-#pragma unroll
-      for (int j = q + 1; j <= i; ++j) D[lo6(i, j)] = rfma(-mi, D[lo6(j, q)], D[lo6(i, j)]);
-      y[i] = rfma(-mi, y[q], y[i]);
-    }
-  }
-#pragma unroll
-  for (int i = 5; i >= 0; --i) {
-    y[i] = rmul(y[i], r[i]);
-#pragma unroll
-    for (int q = i + 1; q < 6; ++q) y[i] = rfma(-m[lo6(q - 1, i)], y[q], y[i]);
-  }
-  if (!ok) b.state[s].info_fail = 1;
-#pragma unroll
-  for (int i = 0; i < 6; ++i) CRN(c.cx, k, i) = y[i];
-}
-
-// Back substitution of an item: x = L^-T E^-1 (W_b - W_a xa - W_b xb), a row
-// per lane, six lanes per item (the lanes of an item are l0 .. l0 + 5).
-template <typename Kept>
-__device__ __forceinline__ double sy_back(unsigned lanes, int l0, int i, const double (&xa)[6], const double (&xb)[6],
-                                          Kept kept) {
-  double y = kept(i * 13);
-#pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    y = rfma(-kept(i * 13 + 1 + j), xa[j], y);
-    y = rfma(-kept(i * 13 + 7 + j), xb[j], y);
-  }
-  y = rmul(y, kept(SY_R + i));
-#pragma unroll
-  for (int k = 5; k > 0; --k) {
-    const double xk = __shfl_sync(lanes, y, l0 + k);
-    if (i < k) y = rfma(-kept(SY_M + lo6(k - 1, i)), xk, y);
-  }
-  return y;
-}
-__global__ void k_sy_back(Batch b, ChainData c, int lo, int hi) {
-  const int lane = threadIdx.x & 31;
-  const int t = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
-  bool on = lane < 30 && t < hi;
-  CrItem it{};
-  if (on) {
-    it = c.odd[t];
-    on = solving(b, it.structure) && b.info[it.structure].sym;
-  }
-  const unsigned lanes = __ballot_sync(0xffffffffu, on);
-  if (!on) return;
-  const int k = it.corner;
-  double xa[6], xb[6];
-#pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    xa[j] = it.prev >= 0 ? CRN(c.cx, it.prev, j) : 0.0;
-    xb[j] = it.next >= 0 ? CRN(c.cx, it.next, j) : 0.0;
-  }
-  CRN(c.cx, k, lane % 6) = sy_back(lanes, lane / 6 * 6, lane % 6, xa, xb, [&](int x) { return CRN(c.cz, k, x); });
-}
-// Midside nodes, into P.
-__global__ void k_sy_scatter(Batch b, ChainData c) {
-  const int lane = threadIdx.x & 31;
-  const int t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
-  bool on = lane < 30 && t < c.n_chain_elems;
-  int e = 0, s = 0;
-  if (on) {
-    e = c.elem_list[t];
-    s = b.estruct[e];
-    on = solving(b, s) && b.info[s].sym;
-  }
-  const unsigned lanes = __ballot_sync(0xffffffffu, on);
-  if (!on) return;
-  const int ka = c.elem_corner_a[t], kb = c.elem_corner_b[t];
-  double xa[6], xb[6];
-#pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    xa[j] = ka >= 0 ? CRN(c.cx, ka, j) : 0.0;
-    xb[j] = kb >= 0 ? CRN(c.cx, kb, j) : 0.0;
-  }
-  const double x = sy_back(lanes, lane / 6 * 6, lane % 6, xa, xb, [&](int q) { return ELM(c.ez, t, q); });
-  b.P[b.info[s].dof_off + b.gl[(int64_t)b.enodes[3 * e + 1] * 6 + lane % 6]] = x;
-}
-
 }  // namespace
 
 // Items below which the item-per-warp forms are the faster ones: an item per
-// thread takes about 50 us however few there are (its chain of 870 to 1,520
-// operations of 64 cycles), an item per warp 5 to 8 us for as many as there are
-// sub-partitions (608) and then about 5 ns an item, three times the other's.
-constexpr int SMALL_GENERAL = 152 * 4 * 8, SMALL_SYM = 152 * 4 * 12;
+// thread takes about 50 us however few there are (its chain of 1,520 operations
+// of 64 cycles), an item per warp 8 us for as many as there are sub-partitions
+// (608), then about 8 ns an item, twice the other's.
+constexpr int SMALL_GENERAL = 152 * 4 * 8;
 // The update's row-per-lane form takes about 10 us below one wave, the
 // entry-per-thread form's two launches 2 us, at three times the loads.
 constexpr int SMALL_UPDATE = 152 * 4 * 4;
 
 static dim3 grid_for(int n, int per, int y = 1) { return dim3((n + per - 1) / per, y); }
 
-static void solve_general(const Batch& b, const ChainData& c, cudaStream_t st) {
+void launch_chain_solve(const Batch& b, const ChainData& c, cudaStream_t st) {
+  if (c.n_chain_elems == 0) return;
   const int ne = c.n_chain_elems;
   if (ne >= SMALL_GENERAL) k_condense<<<grid_for(ne, CT), CT, 0, st>>>(b, c);
   else k_condense_w<<<grid_for(ne, 4), 128, 0, st>>>(b, c);
@@ -951,50 +570,19 @@ static void solve_general(const Batch& b, const ChainData& c, cudaStream_t st) {
       if (hi > lo) k_cr_back<<<grid_for(hi - lo, 20), 128, 0, st>>>(b, c, lo, hi);
     }
   }
-  k_chain_scatter<<<grid_for(ne, 128), 128, 0, st>>>(b, c);
-}
-
-static void solve_sym(const Batch& b, const ChainData& c, cudaStream_t st) {
-  const int ne = c.n_chain_elems;
-  if (ne >= SMALL_SYM) k_sy<SymCondense><<<grid_for(ne, CT), CT, 0, st>>>(b, c, 0, ne);
-  else k_sy_w<SymCondense><<<grid_for(ne, 4), 128, 0, st>>>(b, c, 0, ne);
-  if (c.n_corners > 0) {
-    k_sy_corner<<<grid_for(c.n_corners, 128, 63), 128, 0, st>>>(b, c);
-    for (int l = 0; l < c.n_levels; ++l) {
-      const int lo = c.odd_off[l], hi = c.odd_off[l + 1];
-      if (hi - lo >= SMALL_SYM) k_sy<SymEliminate><<<grid_for(hi - lo, CT), CT, 0, st>>>(b, c, lo, hi);
-      else if (hi > lo) k_sy_w<SymEliminate><<<grid_for(hi - lo, 4), 128, 0, st>>>(b, c, lo, hi);
-      const int elo = c.even_off[l], ehi = c.even_off[l + 1];
-      if (ehi > elo) k_sy_update<<<grid_for(ehi - elo, 64, 63), 64, 0, st>>>(b, c, elo, ehi);
-    }
-    k_sy_root<<<grid_for(c.n_roots, CT), CT, 0, st>>>(b, c);
-    for (int l = c.n_levels - 1; l >= 0; --l) {
-      const int lo = c.odd_off[l], hi = c.odd_off[l + 1];
-      if (hi > lo) k_sy_back<<<grid_for(hi - lo, 20), 128, 0, st>>>(b, c, lo, hi);
-    }
-  }
-  k_sy_scatter<<<grid_for(ne, 20), 128, 0, st>>>(b, c);
-}
-
-void launch_chain_solve(const Batch& b, const ChainData& c, cudaStream_t st) {
-  if (c.n_chain_elems == 0) return;
-  if (c.any_general) solve_general(b, c, st);
-  if (c.any_sym) solve_sym(b, c, st);
   if (c.n_corners > 0) k_corner_scatter<<<grid_for(c.n_corners, 128), 128, 0, st>>>(b, c);
+  k_chain_scatter<<<grid_for(ne, 128), 128, 0, st>>>(b, c);
 }
 
 // Kernel launches of one chain solve.
 int chain_launches(const ChainData& c) {
   if (!c.n_chain_elems) return 0;
-  int n = c.n_corners ? 1 : 0;
-  for (int sym = 0; sym < 2; ++sym) {
-    if (!(sym ? c.any_sym : c.any_general)) continue;
-    n += 2;
-    if (!c.n_corners) continue;
-    n += 2;
+  int n = 2;
+  if (c.n_corners) {
+    n += 3;
     for (int l = 0; l < c.n_levels; ++l) {
       const int odd = c.odd_off[l + 1] - c.odd_off[l], even = c.even_off[l + 1] - c.even_off[l];
-      n += 2 * (odd > 0) + (even > 0) + (!sym && even > 0 && even < SMALL_UPDATE);
+      n += 2 * (odd > 0) + (even > 0) + (even > 0 && even < SMALL_UPDATE);
     }
   }
   return n;

@@ -33,5 +33,8 @@ namespace gf {
 
 void launch_chain_solve(const Batch& b, const ChainData& c, cudaStream_t st);
 int chain_launches(const ChainData& c);
+// The chains with a symmetric K_AA (gf_chain_sym.cu).
+void launch_sym_chains(const Batch& b, const SymChains& c, cudaStream_t st);
+int sym_chain_launches(const SymChains& c);
 
 }  // namespace gf

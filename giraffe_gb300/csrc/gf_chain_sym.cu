@@ -1,0 +1,508 @@
+// Symmetric elimination of Beam_1 chains: Static steps, whose K_AA is symmetric
+// and whose elements do not resist a common translation.
+//
+// The elements (and, as the elimination goes on, runs of elements) of such a
+// chain are "parts" between two corner nodes p and n: a symmetric 9x9 stiffness
+// over (du = u_n - u_p, a_p, a_n) and the forces they leave on the two nodes.
+//   condensation  a midside node, written u_1 = (u_p + u_n) / 2 + v, couples to
+//                 du, a_p, a_n: 6 unknowns against 9 columns
+//   merge         two parts p-k-n become one: with u_k = u_p + w the unknowns
+//                 (w, a_k) couple to du = u_n - u_p, a_p, a_n
+//   root          the last part of a chain with its end conditions (12 unknowns,
+//                 Gauss-Jordan: an end moment's stiffness is not symmetric)
+//   back          corners merge by merge, then the midside nodes
+// Merging pairs of parts level by level takes ceil(log2 m) levels.  Against a
+// cyclic reduction on 6x6 blocks with 12 coupling columns this halves the
+// coupling products (54 against 90 dot products of six per elimination by LDL^T,
+// 234 by Gauss-Jordan) and needs no separate update of the surviving corners:
+// about 700 FP64 operations per eliminated node against 1,100 and 1,520, in
+// kernels that FP64 throughput bounds.
+//
+// Two forms with the same operations on every entry, so the same bits: one item
+// per thread for the large levels and one per half warp for the small ones,
+// where an item's chain of dependent operations (64 cycles each on this part)
+// is what counts.
+#include <cuda_runtime.h>
+
+#include "gf_beam_gp.cuh"
+#include "gf_chain.cuh"
+#include "gf_math.cuh"
+
+namespace gf {
+
+namespace {
+
+constexpr int CT = 64;
+#define AT(arr, n, i, x) (arr)[(int64_t)(x) * (n) + (i)]
+
+__device__ __forceinline__ bool solving(const Batch& b, int s) {
+  const StructState& st = b.state[s];
+  return st.phase == PH_ITER && st.need_solve;
+}
+
+// Newton-Raphson reciprocal seeded by the FP32 hardware approximation (two
+// steps r <- r + r (1 - p r)); exact division outside the FP32 range.
+__device__ __forceinline__ double recip(double p) {
+  float pf = __double2float_rn(p);
+  float af = fabsf(pf);
+  if (!(af > 1e-30f && af < 1e30f)) return 1.0 / p;
+  float rf;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(pf));
+  double r = (double)rf;
+  double e = rfma(-p, r, 1.0);
+  r = rfma(r, e, r);
+  e = rfma(-p, r, 1.0);
+  return rfma(r, e, r);
+}
+
+__device__ __forceinline__ constexpr int lo6(int i, int j) { return i * (i + 1) / 2 + j; }
+
+// Part: lower triangle over (du 0-2, a_p 3-5, a_n 6-8), then the forces on p and
+// n (translation, rotation each).
+constexpr int PT_HP = 45, PT_HN = 51, PT_COUNT = 57;
+// Kept of an elimination: W = L^-1 R ([row * 10 + column]), the entries of L E below
+// the diagonal, the reciprocals of E.
+constexpr int KP_M = 60, KP_R = 75, KP_COUNT = 81;
+// Outputs: the 45 entries of the new stiffness, then the 9 forces h over (du,
+// a_p, a_n).
+constexpr int N_OUT = 54;
+
+// Columns (0: right-hand side, 1-9: du, a_p, a_n) of output o.
+__device__ __forceinline__ void out_pair(int o, int& p, int& q) {
+  if (o >= 45) {
+    p = 0;
+    q = o - 44;
+    return;
+  }
+  // row of the triangle: exact for o < 45, whose roots are at least 1/18 apart
+  const int i = (int)((sqrtf(8.0f * (float)o + 1.5f) - 1.0f) * 0.5f);
+  p = 1 + o - i * (i + 1) / 2;
+  q = 1 + i;
+}
+
+// One elimination of six unknowns: D = L E L^T (d(i, j), j <= i), W = L^-1 R (r(i,
+// q), ten columns), V = E^-1 W, and the outputs base(o) - W_p^T V_q.  L E stays
+// unscaled: W_i -= (L E)_ik V_k.
+template <typename Item> __device__ __forceinline__ bool eliminate(const Item& I) {
+  double D[21], r[6];
+#pragma unroll
+  for (int i = 0; i < 6; ++i)
+#pragma unroll
+    for (int j = 0; j <= i; ++j) D[lo6(i, j)] = I.d(i, j);
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const double p = D[lo6(k, k)];
+    if (!(p != 0.0) || !isfinite(p)) ok = false;
+    r[k] = recip(p);
+    I.keep(KP_R + k, r[k]);
+#pragma unroll
+    for (int j = k + 1; j < 6; ++j) {
+      const double t = rmul(r[k], D[lo6(j, k)]);
+      I.keep(KP_M + lo6(j - 1, k), D[lo6(j, k)]);
+#pragma unroll
+      for (int i = j; i < 6; ++i) D[lo6(i, j)] = rfma(-D[lo6(i, k)], t, D[lo6(i, j)]);
+    }
+  }
+  double W[10][6];
+#pragma unroll
+  for (int q = 0; q < 10; ++q) {
+    double v[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) W[q][i] = I.r(i, q);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      v[k] = rmul(r[k], W[q][k]);
+#pragma unroll
+      for (int i = k + 1; i < 6; ++i) W[q][i] = rfma(-D[lo6(i, k)], v[k], W[q][i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 6; ++i) I.keep(i * 10 + q, W[q][i]);
+    if (q == 0) continue;
+#pragma unroll
+    for (int p = 0; p <= q; ++p) {
+      const int o = p == 0 ? 44 + q : lo6(q - 1, p - 1);
+      double acc = I.base(o, p, q);
+#pragma unroll
+      for (int i = 0; i < 6; ++i) acc = rfma(-W[p][i], v[i], acc);
+      I.out(o, acc);
+    }
+  }
+  return ok;
+}
+
+// The same by a half warp (lanes 0-15 of its sixteen): lane q < 10 holds column q
+// of R, lane 10 + j column j of D from row j on; W and V go through shared memory
+// to the lanes that form the outputs.
+template <typename Item>
+__device__ __forceinline__ bool eliminate_h(const Item& I, int lane, unsigned lanes, double (*ws)[10][6]) {
+  const int dj = lane - 10;
+  const bool rhs = dj < 0;
+  double col[6], r[6], v[6];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) col[i] = rhs ? I.r(i, lane) : (i >= dj ? I.d(i, dj) : 0.0);
+  // the outputs' starting values, loaded ahead of the dependent chain
+  double base[4];
+  int op[4], oq[4];
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const int o = lane + 16 * x;
+    base[x] = 0.0;
+    if (o < N_OUT) {
+      out_pair(o, op[x], oq[x]);
+      base[x] = I.base(o, op[x], oq[x]);
+    }
+  }
+  if (!I.active()) return true;
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const double p = __shfl_sync(lanes, col[k], 10 + k, 16);
+    if (!(p != 0.0) || !isfinite(p)) ok = false;
+    r[k] = recip(p);
+    double d[6], x = col[k];
+#pragma unroll
+    for (int i = k + 1; i < 6; ++i) {
+      d[i] = __shfl_sync(lanes, col[i], 10 + k, 16);
+      if (dj == i) x = d[i];
+      if (lane == 15) I.keep(KP_M + lo6(i - 1, k), d[i]);
+    }
+    v[k] = rmul(r[k], x);
+#pragma unroll
+    for (int i = k + 1; i < 6; ++i)
+      if (rhs || (dj > k && i >= dj)) col[i] = rfma(-d[i], v[k], col[i]);
+    if (lane == 15) I.keep(KP_R + k, r[k]);
+  }
+  if (rhs)
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      ws[0][lane][i] = col[i];
+      ws[1][lane][i] = v[i];
+      I.keep(i * 10 + lane, col[i]);
+    }
+  __syncwarp(lanes);
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const int o = lane + 16 * x;
+    if (o >= N_OUT) break;
+    double acc = base[x];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) acc = rfma(-ws[0][op[x]][i], ws[1][oq[x]][i], acc);
+    I.out(o, acc);
+  }
+  __syncwarp(lanes);
+  return ok;
+}
+
+// Condensation of the midside node of part t.  The tangent kernel writes K_e of
+// such an element over (du, v, a_0, a_1, a_2), lower triangle (beam_expand_sym).
+struct Condense {
+  const Batch& b;
+  const SymChains& c;
+  int t, s;
+  const double *K, *P;
+  int64_t ne;
+  __device__ __forceinline__ void init(int t_) {
+    t = t_;
+    const int e = c.elem[t];
+    s = c.elem_struct[t];
+    K = b.Ke + e;
+    P = b.P + c.elem_dof[t];
+    ne = b.n_elem;
+  }
+  __device__ __forceinline__ bool active() const { return solving(b, s); }
+  // place of unknown i (v, a_1) and of column q (du, a_0, a_2) among the 15
+  __device__ static constexpr int row(int i) { return i < 3 ? 3 + i : 6 + i; }
+  __device__ static constexpr int place(int q) { return q < 4 ? q - 1 : q < 7 ? q + 2 : q + 5; }
+  __device__ static int tri(int i, int j) { return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i; }
+  __device__ __forceinline__ double k15(int i, int j) const { return K[(int64_t)tri(i, j) * ne]; }
+  __device__ __forceinline__ double d(int i, int j) const { return k15(row(i), row(j)); }
+  __device__ __forceinline__ double force(int i) const { return P[i]; }
+  __device__ __forceinline__ double r(int i, int q) const { return q == 0 ? force(i) : k15(row(i), place(q)); }
+  __device__ __forceinline__ double base(int o, int p, int q) const { return o >= 45 ? 0.0 : k15(place(q), place(p)); }
+  __device__ __forceinline__ void keep(int x, double v) const { AT(c.ez, c.n_elem, t, x) = v; }
+  __device__ __forceinline__ void put(int x, double v) const { AT(c.part, c.n_part, t, x) = v; }
+  __device__ __forceinline__ void out(int o, double h) const {
+    if (o < 45) {
+      put(o, h);
+    } else if (o < 48) {  // half of the midside force to each end, and the pull of du
+      const double f = rmul(0.5, force(o - 45));
+      put(PT_HP + o - 45, rsub(f, h));
+      put(PT_HN + o - 45, radd(f, h));
+    } else if (o < 51) {
+      put(PT_HP + 3 + o - 48, h);
+    } else {
+      put(PT_HN + 3 + o - 51, h);
+    }
+  }
+  __device__ void fail() const { b.state[s].info_fail = 1; }
+};
+
+// Elimination of corner k between parts e1 and e2.
+struct Merge {
+  const Batch& b;
+  const SymChains& c;
+  SymMerge m;
+  int t;
+  __device__ __forceinline__ void init(int t_) {
+    t = t_;
+    m = c.merge[t];
+  }
+  __device__ __forceinline__ bool active() const { return solving(b, m.structure); }
+  __device__ __forceinline__ double E(int e, int i, int j) const {
+    return AT(c.part, c.n_part, e, i >= j ? lo6(i, j) : lo6(j, i));
+  }
+  __device__ __forceinline__ double d(int i, int j) const {  // j <= i, unknowns (w, a_k)
+    if (i < 3) return radd(E(m.e1, i, j), E(m.e2, i, j));
+    if (j < 3) return rsub(E(m.e1, 3 + i, j), E(m.e2, i, j));  // a_k: a_n of e1, a_p of e2
+    return radd(E(m.e1, 3 + i, 3 + j), E(m.e2, i, j));
+  }
+  // the corner's own force with what both parts leave on it
+  __device__ __forceinline__ double force(int i) const {
+    return radd(radd(b.P[m.dof + i], AT(c.part, c.n_part, m.e1, PT_HN + i)), AT(c.part, c.n_part, m.e2, PT_HP + i));
+  }
+  __device__ __forceinline__ double r(int i, int q) const {
+    if (q == 0) return force(i);
+    if (q < 4) return i < 3 ? -E(m.e2, i, q - 1) : E(m.e2, i, q - 1);        // du = u_n - u_p
+    if (q < 7) return i < 3 ? E(m.e1, q - 1, i) : E(m.e1, 3 + i, q - 1);     // a_p (place 3 + q - 4)
+    return i < 3 ? -E(m.e2, q - 1, i) : E(m.e2, q - 1, i);                   // a_n (place 6 + q - 7)
+  }
+  __device__ __forceinline__ double base(int o, int p, int q) const {
+    if (o >= 45) return 0.0;
+    const int i = q - 1, j = p - 1;  // i >= j: places of the new part
+    if (i < 3) return E(m.e2, i, j);
+    if (i < 6) return j < 3 ? 0.0 : E(m.e1, i, j);
+    return j >= 3 && j < 6 ? 0.0 : E(m.e2, i, j);
+  }
+  __device__ __forceinline__ void keep(int x, double v) const { AT(c.mz, c.n_merge, t, x) = v; }
+  __device__ __forceinline__ void put(int x, double v) const { AT(c.part, c.n_part, m.out, x) = v; }
+  __device__ __forceinline__ void out(int o, double h) const {
+    if (o < 45) {
+      put(o, h);
+    } else if (o < 48) {  // u_k = u_p + w: the corner's force passes to p
+      const int i = o - 45;
+      put(PT_HP + i, radd(AT(c.part, c.n_part, m.e1, PT_HP + i), rsub(force(i), h)));
+      put(PT_HN + i, radd(AT(c.part, c.n_part, m.e2, PT_HN + i), h));
+    } else if (o < 51) {
+      put(PT_HP + o - 45, radd(AT(c.part, c.n_part, m.e1, PT_HP + o - 45), h));
+    } else {
+      put(PT_HN + o - 48, radd(AT(c.part, c.n_part, m.e2, PT_HN + o - 48), h));
+    }
+  }
+  __device__ void fail() const { b.state[m.structure].info_fail = 1; }
+};
+
+template <typename Item> __global__ void __launch_bounds__(CT) k_sym(Batch b, SymChains c, int lo, int hi) {
+  const int t = lo + blockIdx.x * CT + threadIdx.x;
+  if (t >= hi) return;
+  Item I{b, c};
+  I.init(t);
+  if (!I.active()) return;
+  if (!eliminate(I)) I.fail();
+}
+template <typename Item> __global__ void __launch_bounds__(128) k_sym_h(Batch b, SymChains c, int lo, int hi) {
+  __shared__ double ws[8][2][10][6];
+  const int half = threadIdx.x >> 4, lane = threadIdx.x & 15, t = lo + blockIdx.x * 8 + half;
+  const unsigned lanes = 0xFFFFu << (threadIdx.x & 16);
+  if (t >= hi) return;
+  Item I{b, c};
+  I.init(t);
+  const bool ok = eliminate_h(I, lane, lanes, ws[half]);
+  if (!ok && lane == 0) I.fail();
+}
+
+// The last part of a chain with its end nodes, by one warp: 12 unknowns (u_p, a_p, u_n,
+// a_n), lane j column j of the matrix, lane 12 the right-hand side; fixed DOFs
+// are identity rows and columns, their pivots skipped.
+__device__ void root(const Batch& b, const SymChains& c, const SymChain& ch, int lane) {
+  const int part = ch.root, s = ch.structure;
+  const int node[2] = {c.corner_node[ch.first], c.corner_node[ch.last]};
+  const int g = lane < 12 ? b.gl[(int64_t)node[lane / 6] * 6 + lane % 6] : -1;
+  const unsigned live = __ballot_sync(0xffffffffu, g >= 0);
+  double* P = b.P + b.info[s].dof_off;
+  // place of unknown x among (du, a_p, a_n), and the sign of u_p in du
+  auto place = [](int x) { return x < 3 ? x : x < 6 ? x : x < 9 ? x - 6 : x - 3; };
+  double col[12];
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    double v = 0.0;
+    if (lane < 12) {
+      if ((live >> i & 1) && (live >> lane & 1)) {
+        const int x = place(i), y = place(lane);
+        v = AT(c.part, c.n_part, part, x >= y ? lo6(x, y) : lo6(y, x));
+        if ((i < 3) != (lane < 3)) v = -v;
+        if (i % 6 >= 3 && lane % 6 >= 3 && i / 6 == lane / 6)
+          v = radd(v, b.nodeK[(int64_t)node[i / 6] * 9 + (i % 6 - 3) * 3 + lane % 6 - 3]);
+      } else {
+        v = i == lane ? 1.0 : 0.0;
+      }
+    } else if (lane == 12 && (live >> i & 1)) {
+      v = radd(P[b.gl[(int64_t)node[i / 6] * 6 + i % 6]],
+               AT(c.part, c.n_part, part, (i < 6 ? PT_HP : PT_HN) + i % 6));
+    }
+    col[i] = v;
+  }
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < 12; ++k) {
+    if (!(live >> k & 1)) continue;
+    const double p = __shfl_sync(0xffffffffu, col[k], k);
+    if (!(p != 0.0) || !isfinite(p)) ok = false;
+    const double inv = recip(p);
+    double m[12];
+#pragma unroll
+    for (int i = 0; i < 12; ++i) m[i] = __shfl_sync(0xffffffffu, col[i], k);
+    if (lane > k && lane < 13) {
+      const double rk = rmul(col[k], inv);
+      col[k] = rk;
+#pragma unroll
+      for (int i = 0; i < 12; ++i)
+        if (i != k) col[i] = rfma(-m[i], rk, col[i]);
+    }
+  }
+  if (!ok && lane == 0) b.state[s].info_fail = 1;
+  double x = 0.0;
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    const double v = __shfl_sync(0xffffffffu, col[i], 12);
+    if (lane == i) x = v;
+  }
+  if (lane < 12) {
+    AT(c.x, c.n_corner, lane < 6 ? ch.first : ch.last, lane % 6) = g >= 0 ? x : 0.0;
+    if (g >= 0) P[g] = x;
+  }
+}
+
+// Back substitution of one elimination: E x = L^-1-reduced right-hand side, i.e.
+// y = W_0 - W_du du - W_p a_p - W_n a_n, then x_k = y_k / E_k and y_i -= (L E)_ki x_k
+// from the last row up; a row per lane, six lanes from l0 on.  Returns row i.
+template <typename Kept>
+__device__ __forceinline__ double back(unsigned lanes, int l0, int i, const double (&z)[9], Kept kept) {
+  double w[10], le[6];
+#pragma unroll
+  for (int j = 0; j < 10; ++j) w[j] = kept(i * 10 + j);
+#pragma unroll
+  for (int k = 1; k < 6; ++k) le[k] = i < k ? kept(KP_M + lo6(k - 1, i)) : 0.0;
+  const double r = kept(KP_R + i);
+  double y = w[0];
+#pragma unroll
+  for (int j = 0; j < 9; ++j) y = rfma(-w[1 + j], z[j], y);
+#pragma unroll
+  for (int k = 5; k > 0; --k) {
+    const double xk = __shfl_sync(lanes, rmul(y, r), l0 + k);
+    if (i < k) y = rfma(-le[k], xk, y);
+  }
+  return rmul(y, r);
+}
+__device__ __forceinline__ void around(const SymChains& c, int p, int n, double (&z)[9]) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    z[j] = rsub(AT(c.x, c.n_corner, n, j), AT(c.x, c.n_corner, p, j));
+    z[3 + j] = AT(c.x, c.n_corner, p, 3 + j);
+    z[6 + j] = AT(c.x, c.n_corner, n, 3 + j);
+  }
+}
+// Corner of merge t, row i.
+__device__ __forceinline__ void back_corner(const Batch& b, const SymChains& c, int t, const SymMerge& m, unsigned lanes,
+                                            int l0, int i) {
+  double z[9];
+  around(c, m.p, m.n, z);
+  double x = back(lanes, l0, i, z, [&](int q) { return AT(c.mz, c.n_merge, t, q); });
+  if (i < 3) x = radd(x, AT(c.x, c.n_corner, m.p, i));  // u_k = u_p + w
+  AT(c.x, c.n_corner, m.k, i) = x;
+  b.P[m.dof + i] = x;
+}
+// Corners of one level, five per warp.
+__global__ void k_sym_back(Batch b, SymChains c, int lo, int hi) {
+  const int lane = threadIdx.x & 31, i = lane % 6;
+  const int t = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
+  bool on = lane < 30 && t < hi;
+  SymMerge m{};
+  if (on) {
+    m = c.merge[t];
+    on = solving(b, m.structure);
+  }
+  const unsigned lanes = __ballot_sync(0xffffffffu, on);
+  if (on) back_corner(b, c, t, m, lanes, lane - i, i);
+}
+// Midside nodes.
+__global__ void k_sym_mid(Batch b, SymChains c) {
+  const int lane = threadIdx.x & 31, i = lane % 6;
+  const int t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
+  const bool on = lane < 30 && t < c.n_elem && solving(b, c.elem_struct[t]);
+  const unsigned lanes = __ballot_sync(0xffffffffu, on);
+  if (!on) return;
+  const int p = c.elem_corner[t];
+  double z[9];
+  around(c, p, p + 1, z);
+  double x = back(lanes, lane - i, i, z, [&](int q) { return AT(c.ez, c.n_elem, t, q); });
+  if (i < 3) x = rfma(0.5, radd(AT(c.x, c.n_corner, p, i), AT(c.x, c.n_corner, p + 1, i)), x);
+  b.P[c.elem_dof[t] + i] = x;
+}
+
+// The last levels of a chain in one CTA, from at most SYM_TOP parts on: its
+// merges level by level (a half warp each), the root, and their back
+// substitution.  Against a launch per level this drops the launches and the
+// round trips through L2 between levels of a few items.
+__global__ void __launch_bounds__(128) k_sym_top(Batch b, SymChains c) {
+  __shared__ double ws[8][2][10][6];
+  const SymChain ch = c.chain[blockIdx.x];
+  if (!solving(b, ch.structure)) return;
+  const int half = threadIdx.x >> 4, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lanes = 0xFFFFu << (threadIdx.x & 16);
+  int t0 = ch.top;
+  for (int k = ch.n_top; k > 1; t0 += k / 2, k = (k + 1) / 2) {
+    if (half < k / 2) {
+      Merge I{b, c};
+      I.init(t0 + half);
+      const bool ok = eliminate_h(I, threadIdx.x & 15, lanes, ws[half]);
+      if (!ok && (threadIdx.x & 15) == 0) I.fail();
+    }
+    __syncthreads();
+  }
+  if (warp == 0) root(b, c, ch, lane);
+  __syncthreads();
+  // the levels again from the last: their merges end at t0
+  int cnt[5], n = 0;
+  for (int k = ch.n_top; k > 1; k = (k + 1) / 2) cnt[n++] = k / 2;
+  for (int l = n - 1; l >= 0; --l) {
+    t0 -= cnt[l];
+    const int i = lane % 6, q = warp * 5 + lane / 6;
+    const bool on = lane < 30 && q < cnt[l];
+    const unsigned on_lanes = __ballot_sync(0xffffffffu, on);
+    if (on) back_corner(b, c, t0 + q, c.merge[t0 + q], on_lanes, lane - i, i);
+    __syncthreads();
+  }
+}
+
+dim3 grid_for(int n, int per) { return dim3((n + per - 1) / per); }
+
+// Items below which an item per half warp is the faster form: it takes about 4
+// us for as many as there are half sub-partitions (1,216), then 3 ns an item;
+// an item per thread takes about 35 us however few there are, then half of that
+// per item.
+constexpr int SMALL = 152 * 4 * 20;
+
+}  // namespace
+
+void launch_sym_chains(const Batch& b, const SymChains& c, cudaStream_t st) {
+  if (c.n_elem == 0) return;
+  if (c.n_elem >= SMALL) k_sym<Condense><<<grid_for(c.n_elem, CT), CT, 0, st>>>(b, c, 0, c.n_elem);
+  else k_sym_h<Condense><<<grid_for(c.n_elem, 8), 128, 0, st>>>(b, c, 0, c.n_elem);
+  for (int l = 0; l < c.n_levels; ++l) {
+    const int lo = c.merge_off[l], hi = c.merge_off[l + 1];
+    if (hi - lo >= SMALL) k_sym<Merge><<<grid_for(hi - lo, CT), CT, 0, st>>>(b, c, lo, hi);
+    else k_sym_h<Merge><<<grid_for(hi - lo, 8), 128, 0, st>>>(b, c, lo, hi);
+  }
+  k_sym_top<<<c.n_chains, 128, 0, st>>>(b, c);
+  for (int l = c.n_levels - 1; l >= 0; --l) {
+    const int lo = c.merge_off[l], hi = c.merge_off[l + 1];
+    k_sym_back<<<grid_for(hi - lo, 20), 128, 0, st>>>(b, c, lo, hi);
+  }
+  k_sym_mid<<<grid_for(c.n_elem, 20), 128, 0, st>>>(b, c);
+}
+
+// Kernel launches of one solve.
+int sym_chain_launches(const SymChains& c) { return c.n_elem ? 3 + 2 * c.n_levels : 0; }
+
+}  // namespace gf

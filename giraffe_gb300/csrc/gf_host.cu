@@ -996,17 +996,22 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
     }
     params[s] = step_params[inf.step_off];
     // K_AA of a chain is symmetric in Static steps unless a load adds its own
-    // stiffness: a pipe pressure (pipe_pressed) or a nodal moment
+    // stiffness: a pipe pressure (pipe_pressed) or a nodal moment; the
+    // symmetric elimination takes moments at the chain's ends
     bool sym = inf.is_chain && pipe_pressed.empty();
     for (int k = inf.step_off; k < inf.step_off + inf.n_steps; ++k) sym = sym && !step_params[k].dynamic;
+    for (int i = 6; i < 6 * (m.n_nodes - 1) && sym; ++i) sym = g6[i] >= 0;
     for (int l = 0; l < m.n_loads && sym; ++l)
       if (m.loads[l].type == GF_LOAD_NODAL) {
         const gf_table& t = m.loads[l].table;
-        for (int i = 0; i < t.n_times && sym; ++i)
-          for (int q = 3; q < 6; ++q) sym = sym && t.values[(size_t)i * t.n_cols + q] == 0.0;
+        bool moment = false, inside = false;
+        for (int i = 0; i < t.n_times; ++i)
+          for (int q = 3; q < 6; ++q) moment = moment || t.values[(size_t)i * t.n_cols + q] != 0.0;
+        for (int q = 0; q < m.loads[l].n_items; ++q)
+          inside = inside || (m.loads[l].items[q] > 0 && m.loads[l].items[q] < m.n_nodes - 1);
+        sym = !(moment && inside);
       }
     inf.sym = sym;
-    if (inf.is_chain) (sym ? b.chain.any_sym : b.chain.any_general) = 1;
   }
   b.n_struct = n;
   b.n_nodes = node_off;
@@ -1028,7 +1033,7 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
     std::vector<int> ocnt(NL, 0), ecnt(NL, 0);
     int n_t = 0, n_c = 0, n_levels = 0, n_roots = 0;
     for (int s = 0; s < n; ++s) {
-      if (!plan[s].chain) continue;
+      if (!plan[s].chain || B->info[s].sym) continue;
       const int mm = B->info[s].n_elem;
       const std::vector<char>& fr = plan[s].node_free;
       int M = 0;
@@ -1059,7 +1064,7 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
         cnext(n_c), roots(n_roots), emask(n_t), cmask(n_c);
     hvec<CrItem> odd(cd.odd_off[NL]), even(cd.even_off[NL]);
     parallel_structures(n, work, [&](int s) {
-      if (!plan[s].chain) return;
+      if (!plan[s].chain || B->info[s].sym) return;
       const StructInfo& inf = B->info[s];
       const int mm = inf.n_elem, M = Mc[s], cbase = cb[s], tbase = tb[s];
       const std::vector<char>& fr = plan[s].node_free;
@@ -1129,10 +1134,85 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
           !upload(B, &cd.corner_right, cright) || !upload(B, &cd.corner_prev, cprev) ||
           !upload(B, &cd.corner_next, cnext) || !upload(B, &cd.odd, odd) || !upload(B, &cd.even, even) ||
           !upload(B, &cd.roots, roots) || !upload(B, &cd.elem_mask, emask) || !upload(B, &cd.corner_mask, cmask) ||
-          !balloc(B, &cd.ez, ne * (cd.any_sym ? 99 : 78)) || !balloc(B, &cd.ec, ne * (cd.any_general ? 156 : 90)) ||
-          !balloc(B, &cd.cD, nc * (cd.any_general ? 36 : 21)) || !balloc(B, &cd.cL, nc * (cd.any_general ? 36 : 0)) ||
-          !balloc(B, &cd.cU, nc * 36) || !balloc(B, &cd.cb, nc * 6) || !balloc(B, &cd.cz, nc * (cd.any_sym ? 99 : 78)) ||
-          !balloc(B, &cd.ce, nc * (cd.any_general ? 114 : 90)) || !balloc(B, &cd.cx, nc * 6))
+          !balloc(B, &cd.ez, ne * 78) || !balloc(B, &cd.ec, ne * 156) || !balloc(B, &cd.cD, nc * 36) ||
+          !balloc(B, &cd.cL, nc * 36) || !balloc(B, &cd.cU, nc * 36) || !balloc(B, &cd.cb, nc * 6) ||
+          !balloc(B, &cd.cz, nc * 78) || !balloc(B, &cd.ce, nc * 114) || !balloc(B, &cd.cx, nc * 6))
+        return GF_ERR_CUDA;
+    }
+    // the symmetric chains: parts of level 0 are the elements; each level
+    // merges neighbours in pairs, an odd last part passing up unchanged
+    SymChains& sy = cd.sy;
+    std::vector<int> sbase(n, 0), cbase(n, 0), mcnt(NL, 0), mpos((size_t)n * NL, 0), tpos(n, 0), chains;
+    int n_top = 0;
+    for (int s = 0; s < n; ++s) {
+      if (!plan[s].chain || !B->info[s].sym) continue;
+      const int mm = B->info[s].n_elem;
+      sbase[s] = sy.n_elem;
+      cbase[s] = sy.n_corner;
+      sy.n_elem += mm;
+      sy.n_corner += mm + 1;
+      chains.push_back(s);
+      int l = 0, k = mm;
+      for (; k > SYM_TOP; ++l, k = (k + 1) / 2) {
+        if (l >= NL) { set_err(ctx, "chain too long for %d elimination levels", NL); return GF_ERR_ARG; }
+        mpos[(size_t)s * NL + l] = mcnt[l];
+        mcnt[l] += k / 2;
+        sy.n_levels = std::max(sy.n_levels, l + 1);
+      }
+      tpos[s] = n_top;
+      n_top += k - 1;
+    }
+    for (int l = 0; l < NL; ++l) sy.merge_off[l + 1] = sy.merge_off[l] + mcnt[l];
+    sy.n_merge = sy.merge_off[NL] + n_top;
+    sy.n_part = sy.n_elem + sy.n_merge;
+    sy.n_chains = (int)chains.size();
+    if (sy.n_elem) {
+      hvec<int> selem(sy.n_elem), sstr(sy.n_elem), sdof(sy.n_elem), scorner(sy.n_elem), snode(sy.n_corner);
+      hvec<SymMerge> merge(sy.n_merge);
+      hvec<SymChain> schain(sy.n_chains);
+      parallel_structures(sy.n_chains, work, [&](int c) {
+        const int s = chains[c];
+        const StructInfo& inf = B->info[s];
+        const std::vector<int>& g6 = plan[s].g6;
+        const int mm = inf.n_elem, b0 = sbase[s], c0 = cbase[s];
+        std::vector<int> id(mm), end(mm);  // part, its last corner
+        for (int e = 0; e < mm; ++e) {
+          selem[b0 + e] = inf.elem_off + e;
+          sstr[b0 + e] = s;
+          sdof[b0 + e] = inf.dof_off + g6[6 * (2 * (size_t)e + 1)];
+          scorner[b0 + e] = c0 + e;
+          id[e] = b0 + e;
+          end[e] = c0 + e + 1;
+        }
+        for (int k = 0; k <= mm; ++k) snode[c0 + k] = inf.node_off + 2 * k;
+        SymChain& ch = schain[c];
+        ch = SymChain{0, sy.merge_off[NL] + tpos[s], 0, c0, c0 + mm, s};
+        int top = ch.top;
+        for (int l = 0, k = mm; k > 1; ++l, k = (k + 1) / 2) {
+          if (k <= SYM_TOP && !ch.n_top) ch.n_top = k;
+          int at = k > SYM_TOP ? sy.merge_off[l] + mpos[(size_t)s * NL + l] : top, first = c0;
+          for (int q = 0; q < k / 2; ++q, ++at) {
+            const int mid = end[2 * q];
+            merge[at] = SymMerge{id[2 * q], id[2 * q + 1], sy.n_elem + at, first, mid, end[2 * q + 1], s,
+                                 inf.dof_off + g6[6 * 2 * (size_t)(mid - c0)]};
+            first = end[2 * q + 1];
+            id[q] = sy.n_elem + at;
+            end[q] = first;
+          }
+          if (k <= SYM_TOP) top = at;
+          if (k % 2) {
+            id[k / 2] = id[k - 1];
+            end[k / 2] = end[k - 1];
+          }
+        }
+        if (!ch.n_top) ch.n_top = 1;
+        ch.root = id[0];
+      });
+      if (!upload(B, &sy.elem, selem) || !upload(B, &sy.elem_struct, sstr) || !upload(B, &sy.elem_dof, sdof) ||
+          !upload(B, &sy.elem_corner, scorner) || !upload(B, &sy.corner_node, snode) ||
+          !upload(B, &sy.merge, merge) || !upload(B, &sy.chain, schain) ||
+          !balloc(B, &sy.part, (size_t)sy.n_part * 57) || !balloc(B, &sy.ez, (size_t)sy.n_elem * 81) ||
+          !balloc(B, &sy.mz, (size_t)sy.n_merge * 81) || !balloc(B, &sy.x, (size_t)sy.n_corner * 6))
         return GF_ERR_CUDA;
     }
   }
@@ -1294,8 +1374,8 @@ int count_launches_per_pass(const gf_batch* B) {
   for (int c = 0; c < B->b.n_colors; ++c) colors += B->b.color_off[c + 1] > B->b.color_off[c];
   const ChainData& cd = B->b.chain;
   // chains only: one gather launch in place of the colour passes
-  if (B->b.n_elem && !B->b.full_band && cd.n_chain_elems == B->b.n_elem) colors = 1;
-  return 10 + colors + chain_launches(cd) + shell_launches_per_pass(B->b) + (B->b.any_rayleigh ? 1 : 0) +
+  if (B->b.n_elem && !B->b.full_band && cd.n_chain_elems + cd.sy.n_elem == B->b.n_elem) colors = 1;
+  return 10 + colors + chain_launches(cd) + sym_chain_launches(cd.sy) + shell_launches_per_pass(B->b) + (B->b.any_rayleigh ? 1 : 0) +
          (B->b.n_pipe_press ? 1 : 0) + (B->b.mon_total ? 1 : 0);
 }
 

@@ -317,7 +317,9 @@ constexpr int MP_POINT = GP_COUNT + GC_COUNT;  // doubles per Gauss point and el
 // rotational force (global frame)
 constexpr int MI_D = 0, MI_FU = 9, MI_FA = 12, MI_COUNT = 15;
 constexpr int MOUNT_SMEM = 2 * MP_POINT * 32 * (int)sizeof(double);
-constexpr int MOUNT_SMEM_DYN = 2 * (MP_POINT + MI_COUNT) * 32 * (int)sizeof(double);
+// the batch's kernel adds the inertial terms, or in static structures of the
+// symmetric chain solver their coefficients
+constexpr int MOUNT_SMEM_BATCH = 2 * (MP_POINT + MI_COUNT) * 32 * (int)sizeof(double);
 
 // The entries of K_e and f_e of lane's element, shared by the CTA's warps:
 // put(r, s, v) for one entry of every symmetric pair, force(q, v).
@@ -348,6 +350,44 @@ __device__ __forceinline__ void beam_expand(const double* P, int warp, int lane,
   for (int k = warp; k < 18; k += 4) force(k, beam_f(M, C, gs, ms, k / 6, (k % 6) / 3, k % 3));
 }
 
+// The same over (du 0-2, v 3-5, a_0 6-8, a_1 9-11, a_2 12-14), lower triangle, as
+// the symmetric chain solver condenses it: put(i, j, v), i >= j.  S: the
+// coefficients of du and v, point g at [g * ss].
+template <typename Put, typename Force>
+__device__ __forceinline__ void beam_expand_sym(const double* P, const double* S, int ss, int warp, int lane, Put put,
+                                                Force force) {
+  const double *M = P + lane, *C = P + GP_COUNT * 32 + lane;
+  constexpr int gs = MP_POINT * 32, ms = 32;
+#pragma unroll 1
+  for (int k = warp; k < 45; k += 4) {
+    int pair, I, J, i, j;
+    beam_aa_place(k, pair, I, J, i, j);
+    const double v = beam_k_aa(M, C, gs, ms, pair, I, J, i, j);
+    const int r = 6 + 3 * I + i, q = 6 + 3 * J + j;  // r <= q
+    put(q, r, v);
+  }
+#pragma unroll 1
+  for (int k = warp; k < 54; k += 4) {
+    const int B = k / 27, J = k % 27 / 9, x = k % 9, cf = (B ? GS_VN : GS_DN) + J;
+    put(6 + 3 * J + x % 3, 3 * B + x / 3,
+        rfma(S[ss + cf * ms], M[gs + (GP_M02 + x) * ms], rmul(S[cf * ms], M[(GP_M02 + x) * ms])));
+  }
+#pragma unroll 1
+  for (int k = warp; k < 18; k += 4) {
+    const int B = k / 6, x = k % 6;
+    const int i = x < 3 ? 0 : (x < 5 ? 1 : 2), j = x < 3 ? x : (x < 5 ? x - 2 : 2);  // i <= j
+    const double v = rfma(S[ss + B * ms], M[gs + (GP_M00 + x) * ms], rmul(S[B * ms], M[(GP_M00 + x) * ms]));
+    if (B == 1) {
+      put(3 + i, j, v);
+      if (i != j) put(3 + j, i, v);
+    } else {
+      put((B ? 3 : 0) + j, (B ? 3 : 0) + i, v);
+    }
+  }
+#pragma unroll 1
+  for (int k = warp; k < 18; k += 4) force(k, beam_f(M, C, gs, ms, k / 6, (k % 6) / 3, k % 3));
+}
+
 __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* P = reinterpret_cast<double*>(smem_raw);  // [point][value][lane]
@@ -360,7 +400,10 @@ __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
   if (live) {
     const BeamConst& c = b.bconst[e];
     const int g = warp & 1;
-    if (warp >= 2) beam_gp_coef(c, g, P + (g * MP_POINT + GP_COUNT) * 32 + lane, 32);
+    if (warp >= 2) {
+      beam_gp_coef(c, g, P + (g * MP_POINT + GP_COUNT) * 32 + lane, 32);
+      if (!dyn) beam_gp_coef_sym(c, g, In + g * MI_COUNT * 32 + lane, 32);
+    }
     if (warp < 2 || dyn) {
       int nd[3] = {b.enodes[3 * e], b.enodes[3 * e + 1], b.enodes[3 * e + 2]};
       double d[18];
@@ -393,13 +436,16 @@ __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
   const int64_t ne = b.n_elem;
   const double* Cf = P + GP_COUNT * 32 + lane;
   if (!dyn) {
-    // the symmetric chain elimination reads the lower triangle
-    const bool half = b.info[s].sym && !b.full_band;
+    if (b.info[s].sym && !b.full_band) {
+      beam_expand_sym(P, In + lane, MI_COUNT * 32, warp, lane,
+                      [&](int i, int j, double v) { Ke[(int64_t)(i * (i + 1) / 2 + j) * ne] = v; },
+                      [&](int q, double v) { b.Fe[q * ne + e] = v; });
+      return;
+    }
     beam_expand(P, warp, lane,
                 [&](int r, int q, double v) {
-                  const int lo = r < q ? r : q, hi = r < q ? q : r;
-                  Ke[(hi + 18 * lo) * ne] = v;
-                  if (!half && hi != lo) Ke[(lo + 18 * hi) * ne] = v;
+                  Ke[(r + 18 * q) * ne] = v;
+                  if (r != q) Ke[(q + 18 * r) * ne] = v;
                 },
                 [&](int q, double v) { b.Fe[q * ne + e] = v; });
     return;
@@ -1462,15 +1508,14 @@ static void launch_mount(const Batch& b, cudaStream_t st, LaunchProf* prof) {
   if (b.n_elem == 0) return;
   {
     ProfScope q(prof, st, KC_MOUNT);
-    // 36.9 KB of shared memory a CTA (44.5 in Dynamic steps), under the 48 KB
-    // that needs no attribute
-    k_beam_tangent<<<(b.n_elem + 31) / 32, MOUNT_THREADS, b.any_dynamic ? MOUNT_SMEM_DYN : MOUNT_SMEM, st>>>(b);
+    // 44.5 KB of shared memory a CTA, under the 48 KB that needs no attribute
+    k_beam_tangent<<<(b.n_elem + 31) / 32, MOUNT_THREADS, MOUNT_SMEM_BATCH, st>>>(b);
     // the pressure's load stiffness is part of the K_e that Rayleigh damping
     // reads (the reference mounts loads before damping)
     if (b.n_pipe_press) k_pipe_pressure<<<(b.n_pipe_press + 127) / 128, 128, 0, st>>>(b);
     if (b.any_rayleigh) k_beam_rayleigh<<<(b.n_elem + 127) / 128, 128, 0, st>>>(b);
   }
-  if (!b.full_band && b.chain.n_chain_elems == b.n_elem) {
+  if (!b.full_band && b.chain.n_chain_elems + b.chain.sy.n_elem == b.n_elem) {
     // chains only: the residual is all the scatter would assemble
     ProfScope q(prof, st, KC_SCATTER);
     const int64_t nt = (int64_t)b.n_nodes * 6;
@@ -1497,6 +1542,7 @@ void launch_iteration(const Batch& b, cudaStream_t st, bool commit_kernels, Laun
   { ProfScope q(prof, st, KC_RESIDUAL); k_residual<<<b.n_chunks, 256, 0, st>>>(b); }
   { ProfScope q(prof, st, KC_SOLVE); launch_band_solve(b, st); }
   if (b.chain.n_chain_elems) { ProfScope q(prof, st, KC_CHAIN); launch_chain_solve(b, b.chain, st); }
+  if (b.chain.sy.n_elem) { ProfScope q(prof, st, KC_CHAIN); launch_sym_chains(b, b.chain.sy, st); }
   if (b.sh.n_wide) launch_wide_solve(b, st, prof);
   { ProfScope q(prof, st, KC_UPDATE); k_update<<<b.n_chunks, 256, 0, st>>>(b); }
   { ProfScope q(prof, st, KC_CONTROL); k_control<<<(ns + 127) / 128, 128, 0, st>>>(b); }

@@ -118,8 +118,10 @@ struct StructInfo {
   int has_force, has_moment;  // free translational / rotational DOFs exist
   int load_off, n_loads;  // nodal load entries of this structure
   int is_chain;  // solved by the chain solver (else by the band LU)
-  int sym;       // a chain whose K_AA is symmetric: Static steps only, no pipe
-                 // pressure and no nodal moments (whose stiffness is not)
+  int sym;       // a chain whose K_AA is symmetric but for its end nodes: Static
+                 // steps only, no pipe pressure, nodal moments (whose
+                 // stiffness is not symmetric) at the ends only, interior
+                 // corners free
   // wide-band structures (Shell_1): K_AA column-major with 2 wkl + 1 rows,
   // entry (i, j) at wband[wb_off + (wkl + i - j) + j (2 wkl + 1)]; the free
   // DOFs are numbered in reverse Cuthill-McKee node order
@@ -212,6 +214,35 @@ struct CrItem {
   int structure;
 };
 
+// A merge of the symmetric chain elimination (gf_chain_sym.cu): the parts e1
+// (corners p to k) and e2 (k to n) become part `out`, corner k eliminated.
+// dof: corner k's first free DOF (batch-wide; its six are consecutive).
+struct SymMerge {
+  int e1, e2, out, p, k, n, structure, dof;
+};
+// A chain once SYM_TOP parts or fewer are left: their number, the merges that
+// are left (chain by chain, level by level), the last part and the end corners.
+#define SYM_TOP 16
+struct SymChain {
+  int n_top, top, root, first, last, structure;
+};
+struct SymChains {
+  int n_elem, n_part, n_corner, n_merge, n_levels, n_chains;
+  int* elem;         // batch element of each part of level 0
+  int* elem_struct;
+  int* elem_dof;     // first DOF (batch-wide) of its midside node
+  int* elem_corner;  // its first corner (the next index is its last)
+  int* corner_node;  // batch node of each corner
+  SymMerge* merge;   // the levels of more than SYM_TOP parts, level by level, then every chain's last ones
+  int merge_off[CR_MAX_LEVELS + 1];
+  SymChain* chain;
+  // structure-of-arrays, entry x of item i at [x * n + i]
+  double* part;      // [57][n_part]  condensed stiffness over (du, a0, a1) and nodal forces
+  double* ez;        // [81][n_elem]  kept for the midside nodes' back substitution
+  double* mz;        // [81][n_merge]  for the eliminated corners'
+  double* x;         // [6][n_corner]  solution at the corners
+};
+
 struct ChainData {
   int n_chain_elems;   // elements of chain structures
   int n_corners;       // free corners of chain structures
@@ -219,9 +250,9 @@ struct ChainData {
   int* elem_list;      // batch element ids of chain elements
   int* elem_corner_a;  // corner index of the element's first corner (-1 if fixed)
   int* elem_corner_b;  // corner index of the element's last corner (-1 if fixed)
+  SymChains sy;        // the chains solved by the symmetric elimination (the rest of this struct: the others)
   int* elem_mask;      // free DOFs of the element's corners: bits 0-5 the first, 6-11 the last
   int* corner_mask;    // free DOFs of the corner (bits 0-5)
-  int any_general, any_sym;  // chains of either kind in the batch
   int* corner_node;    // batch node id of each free corner
   int* corner_struct;
   int* corner_left;    // chain element to the left (-1 if none)
@@ -229,15 +260,14 @@ struct ChainData {
   int* corner_prev;    // previous free corner of the same chain (-1 if none)
   int* corner_next;    // next free corner (-1 if none)
   // scratch below is structure-of-arrays: entry x of item i at [x * n_items + i]
-  // (general elimination, then symmetric elimination)
-  double* ez;          // [6*13][chain elem]  Z_s = A_ss^{-1}[b_s | A_sa | A_sb]; [99] W, multipliers, reciprocals
-  double* ec;          // [6*26][chain elem]  -A_as Z_s (13 cols), -A_bs Z_s (13 cols); [90] contributions
+  double* ez;          // [6*13][chain elem]  Z_s = A_ss^{-1}[b_s | A_sa | A_sb]
+  double* ec;          // [6*26][chain elem]  -A_as Z_s (13 cols), -A_bs Z_s (13 cols)
   double* cD;          // [36][corner] (row-major 6x6 per corner)
   double* cL;          // [36][corner]
   double* cU;          // [36][corner]
   double* cb;          // [6][corner]
-  double* cz;          // [6*13][corner]  Z = D^{-1}[b | L | U] of an eliminated corner; [99] as ez
-  double* ce;          // [114][corner]  outputs of the entry-per-thread update; [90] as ec
+  double* cz;          // [6*13][corner]  Z = D^{-1}[b | L | U] of an eliminated corner
+  double* ce;          // [114][corner]  outputs of the entry-per-thread update
   double* cx;          // [6][corner]  solution
   CrItem* odd;         // per level: eliminated positions
   int odd_off[CR_MAX_LEVELS + 1];
