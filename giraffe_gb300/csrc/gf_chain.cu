@@ -28,22 +28,6 @@ __device__ __forceinline__ bool solving(const Batch& b, int s) {
   return st.phase == PH_ITER && st.need_solve;
 }
 
-// Newton-Raphson reciprocal seeded by the FP32 hardware approximation (two
-// steps r <- r + r (1 - p r)); exact division outside the FP32 range.
-__device__ __forceinline__ double recip(double p) {
-  float pf = __double2float_rn(p);
-  float af = fabsf(pf);
-  if (!(af > 1e-30f && af < 1e30f)) return 1.0 / p;
-  float rf;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(pf));
-  double r = (double)rf;
-  double e = fma(-p, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-p, r, 1.0);
-  r = fma(r, e, r);
-  return r;
-}
-
 // Gauss-Jordan on a thread's augmented matrix [D | R] in two phases, both in
 // registers: gj6_factor eliminates D (6x6, row-major, every index static under
 // the full unroll) and records each pivot's reciprocal and multipliers;
@@ -58,7 +42,7 @@ __device__ __forceinline__ bool gj6_factor(double (&D)[36], double (&inv)[6], do
   for (int k = 0; k < 6; ++k) {
     const double p = D[k * 6 + k];
     if (!(p != 0.0) || !isfinite(p)) ok = false;
-    inv[k] = recip(p);
+    inv[k] = rcp64(p);
     double dk[6];
 #pragma unroll
     for (int c = k + 1; c < 6; ++c) {
@@ -190,7 +174,7 @@ __global__ void __launch_bounds__(128) k_condense_w(Batch b, ChainData c) {
   for (int k = 0; k < 6; ++k) {
     const double p = __shfl_sync(0xffffffffu, col[k], k);
     if (!(p != 0.0) || !isfinite(p)) ok = false;
-    const double inv = recip(p);
+    const double inv = rcp64(p);
     double m[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) m[i] = __shfl_sync(0xffffffffu, col[i], k);
@@ -329,7 +313,7 @@ __global__ void k_cr_eliminate_w(Batch b, ChainData c, int lo, int hi) {
   for (int kk = 0; kk < 6; ++kk) {
     double p = __shfl_sync(0xffffffffu, col[kk], kk);
     if (!(p != 0.0) || !isfinite(p)) ok = false;
-    double inv = recip(p);
+    double inv = rcp64(p);
     double m[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) m[i] = __shfl_sync(0xffffffffu, col[i], kk);

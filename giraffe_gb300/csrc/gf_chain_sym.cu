@@ -40,21 +40,6 @@ __device__ __forceinline__ bool solving(const Batch& b, int s) {
   return st.phase == PH_ITER && st.need_solve;
 }
 
-// Newton-Raphson reciprocal seeded by the FP32 hardware approximation (two
-// steps r <- r + r (1 - p r)); exact division outside the FP32 range.
-__device__ __forceinline__ double recip(double p) {
-  float pf = __double2float_rn(p);
-  float af = fabsf(pf);
-  if (!(af > 1e-30f && af < 1e30f)) return 1.0 / p;
-  float rf;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(pf));
-  double r = (double)rf;
-  double e = rfma(-p, r, 1.0);
-  r = rfma(r, e, r);
-  e = rfma(-p, r, 1.0);
-  return rfma(r, e, r);
-}
-
 __device__ __forceinline__ constexpr int lo6(int i, int j) { return i * (i + 1) / 2 + j; }
 
 // Part: lower triangle over (du 0-2, a_p 3-5, a_n 6-8), then the forces on p and
@@ -94,7 +79,7 @@ template <typename Item> __device__ __forceinline__ bool eliminate(const Item& I
   for (int k = 0; k < 6; ++k) {
     const double p = D[lo6(k, k)];
     if (!(p != 0.0) || !isfinite(p)) ok = false;
-    r[k] = recip(p);
+    r[k] = rcp64(p);
     I.keep(KP_R + k, r[k]);
 #pragma unroll
     for (int j = k + 1; j < 6; ++j) {
@@ -159,7 +144,7 @@ __device__ __forceinline__ bool eliminate_h(const Item& I, int lane, unsigned la
   for (int k = 0; k < 6; ++k) {
     const double p = __shfl_sync(lanes, col[k], 10 + k, 16);
     if (!(p != 0.0) || !isfinite(p)) ok = false;
-    r[k] = recip(p);
+    r[k] = rcp64(p);
     double d[6], x = col[k];
 #pragma unroll
     for (int i = k + 1; i < 6; ++i) {
@@ -348,7 +333,7 @@ __device__ void root(const Batch& b, const SymChains& c, const SymChain& ch, int
     if (!(live >> k & 1)) continue;
     const double p = __shfl_sync(0xffffffffu, col[k], k);
     if (!(p != 0.0) || !isfinite(p)) ok = false;
-    const double inv = recip(p);
+    const double inv = rcp64(p);
     double m[12];
 #pragma unroll
     for (int i = 0; i < 12; ++i) m[i] = __shfl_sync(0xffffffffu, col[i], k);

@@ -29,6 +29,7 @@
 
 #include "gf_front.h"
 #include "gf_kernels.cuh"
+#include "gf_math.cuh"
 #include "gf_types.h"
 
 namespace gf {
@@ -42,26 +43,7 @@ __device__ __forceinline__ bool mf_active(const Batch& b, int s) {
   return st.phase == PH_ITER && st.need_solve && (!b.sh.fp64_pass || st.ir_fb);
 }
 
-// 1/p from a single-precision seed of p's own bits (r0, 2^-23) and one
-// third-order step r = r0 + r0 (e + e^2), e = 1 - p r0 (2^-69): three dependent
-// FP64 results in place of the six of two second-order steps and the two
-// conversions.  The division where the seed is out of range.
-__device__ __forceinline__ double mf_rcp(double p) {
-  const long long u = __double_as_longlong(p);
-  const int ex = (int)((u >> 52) & 0x7FF);
-  if (ex < 64 || ex > 1982) return 1.0 / p;
-  // m in [1, 2) from the leading bits of the fraction, its reciprocal in (0.5, 1]
-  const float m = __int_as_float(0x3F800000 | (int)((u >> 29) & 0x7FFFFF));
-  float rf;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(m));
-  const int rb = __float_as_int(rf);
-  // the seed's bits as a double, scaled by 2^(1023 - ex), with p's sign
-  const long long r0b = ((long long)((rb >> 23) - 127 + 1023 + 1023 - ex) << 52) | ((long long)(rb & 0x7FFFFF) << 29) |
-                        (u & (long long)0x8000000000000000ull);
-  const double r0 = __longlong_as_double(r0b);
-  const double e = fma(-p, r0, 1.0);
-  return fma(r0, fma(e, e, e), r0);
-}
+__device__ __forceinline__ double mf_rcp(double p) { return rcp64(p); }
 __device__ __forceinline__ float mf_rcp(float p) { return __frcp_rn(p); }
 __device__ __forceinline__ double mfma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float mfma(float a, float b, float c) { return fmaf(a, b, c); }

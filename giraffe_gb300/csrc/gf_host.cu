@@ -834,7 +834,8 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
     // tables and nodal loads (NodalLoad::UpdateforSolutionStep, reference
     // src/NodalLoad.cpp:235-263)
     auto add_table = [&](const gf_table& t) {
-      TableDev d{t.n_times, t.n_cols, (int64_t)tdata.size()};
+      TableDev d{t.n_times, t.n_cols, 1, 0, (int64_t)tdata.size()};
+      for (int i = 1; i < t.n_times; ++i) d.sorted = d.sorted && t.times[i] >= t.times[i - 1];
       for (int i = 0; i < t.n_times; ++i) tdata.push_back(t.times[i]);
       for (int i = 0; i < t.n_times * t.n_cols; ++i) tdata.push_back(t.values[i]);
       tables.push_back(d);
@@ -1012,6 +1013,13 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
         sym = !(moment && inside);
       }
     inf.sym = sym;
+  }
+  // prescribed displacements by node (their order kept within a node)
+  std::vector<int> disp_of;
+  if (!disps.empty()) {
+    std::stable_sort(disps.begin(), disps.end(), [](const DispEntry& x, const DispEntry& y) { return x.node < y.node; });
+    disp_of.assign(node_off, (int)disps.size());
+    for (size_t k = disps.size(); k-- > 0;) disp_of[disps[k].node] = (int)k;
   }
   b.n_struct = n;
   b.n_nodes = node_off;
@@ -1309,7 +1317,7 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       !upload(B, &b.mon_struct, mon_struct) || !upload(B, &b.mon_adj_off, mon_adj_off) ||
       !upload(B, &b.mon_adj, mon_adj) || !balloc(B, &b.mon_load, (size_t)b.mon_total * 6) ||
       !balloc(B, &b.mon_rec, (size_t)b.mon_total * b.mon_cap * 25) ||
-      !upload(B, &b.disps, disps) || !upload(B, &b.tables, tables) || !upload(B, &b.table_data, tdata) ||
+      !upload(B, &b.disps, disps) || !upload(B, &b.disp_of, disp_of) || !zeroed(B, &b.begin, (size_t)n) || !upload(B, &b.tables, tables) || !upload(B, &b.table_data, tdata) ||
       !dup(B, &B->copy0, b.copy, copy.size()) || !dup(B, &B->Qn0, b.Qn, Qn.size()) ||
       !dup(B, &B->bhist0, b.bhist, bhist.size()) || !dup(B, &B->baux0, b.baux, baux.size()))
     return GF_ERR_CUDA;
@@ -1375,7 +1383,8 @@ int count_launches_per_pass(const gf_batch* B) {
   const ChainData& cd = B->b.chain;
   // chains only: one gather launch in place of the colour passes
   if (B->b.n_elem && !B->b.full_band && cd.n_chain_elems + cd.sy.n_elem == B->b.n_elem) colors = 1;
-  return 10 + colors + chain_launches(cd) + sym_chain_launches(cd.sy) + shell_launches_per_pass(B->b) + (B->b.any_rayleigh ? 1 : 0) +
+  // step_begin, step_nodes, zero, tangent, residual, band solve, update, control, commits
+  return 10 + (B->b.n_loads ? 1 : 0) + (B->b.any_dynamic ? 1 : 0) + colors + chain_launches(cd) + sym_chain_launches(cd.sy) + shell_launches_per_pass(B->b) + (B->b.any_rayleigh ? 1 : 0) +
          (B->b.n_pipe_press ? 1 : 0) + (B->b.mon_total ? 1 : 0);
 }
 

@@ -22,66 +22,47 @@ __device__ __forceinline__ double table_at(const Batch& b, int t, double time, i
   if (T.n_times == 0) return 0.0;
   if (time >= times[T.n_times - 1]) return vals[(T.n_times - 1) * T.n_cols + col];
   if (time <= times[0]) return vals[col];
-  int idx = 0;
-  while (time >= times[idx]) idx++;
+  const int idx = table_row(T, times, time);
   double f = (time - times[idx - 1]) / (times[idx] - times[idx - 1]);
   double a = vals[(idx - 1) * T.n_cols + col], c = vals[idx * T.n_cols + col];
   return a + f * (c - a);
 }
 
-__device__ __forceinline__ double warp_max(double v) {
+// Magnitude bits of a double: they order like the magnitudes, with infinities
+// and then NaN above every finite value.  Maxima and the divergence test work on
+// them, since an FP64 comparison takes as long as an FP64 multiply-add here (16
+// cycles of an SM per warp) and these kernels compare eight times per DOF.
+typedef unsigned long long mag_t;
+__device__ __forceinline__ mag_t mag(double v) { return (mag_t)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull; }
+constexpr mag_t MAG_HUGE = 0x7E37E43C8800759Cull;  // 1e300
+constexpr mag_t MAG_INF = 0x7FF0000000000000ull;
+// the larger of m and v's magnitude; NaN does not count
+__device__ __forceinline__ void mag_max(mag_t& m, mag_t v) {
+  if (v > m && v <= MAG_INF) m = v;
+}
+__device__ __forceinline__ mag_t warp_max(mag_t v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) v = max(v, (mag_t)__shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ int warp_or(int v) { return __any_sync(0xffffffffu, v); }
-
-// Block-wide max of two values and an "any" flag (blockDim.x <= 1024).
-struct Red3 { double a, b; int f; };
-__device__ Red3 block_red(Red3 v) {
-  __shared__ double sa[32], sb[32];
-  __shared__ int sf[32];
-  v.a = warp_max(v.a);
-  v.b = warp_max(v.b);
-  v.f = warp_or(v.f);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) { sa[w] = v.a; sb[w] = v.b; sf[w] = v.f; }
-  __syncthreads();
-  int nw = (blockDim.x + 31) >> 5;
-  if (w == 0) {
-    v.a = l < nw ? sa[l] : 0.0;
-    v.b = l < nw ? sb[l] : 0.0;
-    v.f = l < nw ? sf[l] : 0;
-    v.a = warp_max(v.a);
-    v.b = warp_max(v.b);
-    v.f = warp_or(v.f);
-    if (l == 0) { sa[0] = v.a; sb[0] = v.b; sf[0] = v.f; }
-  }
-  __syncthreads();
-  Red3 r{sa[0], sb[0], sf[0]};
-  __syncthreads();
-  return r;
-}
-
-__device__ __forceinline__ bool nan_or_huge(double v) { return !(v == v) || v >= 1e300 || v <= -1e300; }
 
 // ---- reductions of one structure spread over several CTAs ----
 __device__ __forceinline__ int red_chunks(const StructInfo& inf) {
   return inf.n_free > 0 ? (inf.n_free + GF_RED_CHUNK - 1) / GF_RED_CHUNK : 1;
 }
-// Max of non-negative doubles through their bit patterns (exact, so the
-// result does not depend on the order in which CTAs arrive).
-__device__ __forceinline__ void red_max(unsigned long long* p, double v) {
-  atomicMax(p, (unsigned long long)__double_as_longlong(v));
+// Max of magnitudes through their bit patterns (exact, so the result does not
+// depend on the order in which warps arrive), a contribution per warp.
+__device__ __forceinline__ void red_max(mag_t* p, mag_t v) {
+  v = warp_max(v);
+  if ((threadIdx.x & 31) == 0 && v) atomicMax(p, v);
 }
-__device__ __forceinline__ double red_value(const unsigned long long* p) {
-  return __longlong_as_double((long long)*(volatile const unsigned long long*)p);
+__device__ __forceinline__ void red_flag(int* p, bool f) {
+  if (__any_sync(0xffffffffu, f) && (threadIdx.x & 31) == 0) atomicOr(p, 1);
 }
+__device__ __forceinline__ double red_value(const mag_t* p) {
+  return __longlong_as_double((long long)*(volatile const mag_t*)p);
+}
+struct Red3 { double a, b; int f; };
 // Counts this CTA in; true in every thread of the CTA that arrives last, to
 // which the other CTAs' global writes are then visible (each thread fences
 // its own writes before the count).
@@ -142,69 +123,74 @@ __global__ void k_init_state(Batch b) {
   st = z;
 }
 
-// reference src/Static.cpp:176-197 (+ NodalDisplacement::Mount, EulerAngles)
+// Start of a load / time step (reference src/Static.cpp:176-197): the step
+// machine, a thread per structure; begin[s] tells k_step_nodes what to do (bit 0
+// the step starts, bit 1 from zero velocities).
 __global__ void k_step_begin(Batch b) {
-  int s = blockIdx.x;
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= b.n_struct) return;
+  if (s == 0) *b.running = 0;
   StructState& st = b.state[s];
-  __shared__ int go, zero_va;
-  if (threadIdx.x == 0) {
-    if (s == 0) *b.running = 0;
-    go = st.phase == PH_START;
-    zero_va = go && st.zero_va;
-    if (go) {
-      st.zero_va = 0;
-      const StructParams& p = b.params[s];
-      if (st.host_step) {
-        // gf_begin_step: the caller's Static::Solve / Dynamic::Solve loop
-        // advanced the time itself
-        st.time_step = st.current_time_step;
-        st.time = st.last_converged_time + st.current_time_step;
-      } else {
-        st.last_converged_time = st.time;
-        st.time += st.time_step;
-        if (st.time > 0.99999999 * p.end_time) {
-          st.time = p.end_time;
-          st.time_step = p.end_time - st.last_converged_time;
-        }
-        st.current_time_step = st.time_step;
-      }
-      if (p.dynamic) {
-        // reference src/Dynamic.cpp:582-590
-        double dt = st.time_step;
-        st.a[0] = 1.0 / (dt * dt * p.beta);
-        st.a[1] = 1.0 / (dt * p.beta);
-        st.a[2] = 1.0 / (2.0 * p.beta) - 1.0;
-        st.a[3] = p.gamma / (dt * p.beta);
-        st.a[4] = 1.0 - p.gamma / p.beta;
-        st.a[5] = dt * (1.0 - p.gamma / (2.0 * p.beta));
-      }
-      st.it = 1;
-      st.res_conv = 0;
-      st.gl_conv = 0;
-      st.diverged = 0;
-      st.info_fail = 0;
-      st.phase = PH_ITER;
-    }
-  }
-  __syncthreads();
+  const bool go = st.phase == PH_START;
+  b.begin[s] = go ? 1 + 2 * (st.zero_va != 0) : 0;
   if (!go) return;
-  const StructInfo inf = b.info[s];
+  st.zero_va = 0;
+  const StructParams& p = b.params[s];
+  if (st.host_step) {
+    // gf_begin_step: the caller's Static::Solve / Dynamic::Solve loop
+    // advanced the time itself
+    st.time_step = st.current_time_step;
+    st.time = st.last_converged_time + st.current_time_step;
+  } else {
+    st.last_converged_time = st.time;
+    st.time += st.time_step;
+    if (st.time > 0.99999999 * p.end_time) {
+      st.time = p.end_time;
+      st.time_step = p.end_time - st.last_converged_time;
+    }
+    st.current_time_step = st.time_step;
+  }
+  if (p.dynamic) {
+    // reference src/Dynamic.cpp:582-590
+    double dt = st.time_step;
+    st.a[0] = 1.0 / (dt * dt * p.beta);
+    st.a[1] = 1.0 / (dt * p.beta);
+    st.a[2] = 1.0 / (2.0 * p.beta) - 1.0;
+    st.a[3] = p.gamma / (dt * p.beta);
+    st.a[4] = 1.0 - p.gamma / p.beta;
+    st.a[5] = dt * (1.0 - p.gamma / (2.0 * p.beta));
+  }
+  st.it = 1;
+  st.res_conv = 0;
+  st.gl_conv = 0;
+  st.diverged = 0;
+  st.info_fail = 0;
+  st.phase = PH_ITER;
+}
+
+// Zeros, the prescribed displacements of the step (NodalDisplacement::Mount,
+// Euler angles or vectors) and in Dynamic steps the Newmark predictor, a thread
+// per node.  disp_of[i]: the node's first entry of disps, sorted by node.
+__global__ void k_step_nodes(Batch b) {
+  const int node = blockIdx.x * blockDim.x + threadIdx.x;
+  if (node >= b.n_nodes) return;
+  const int s = b.node_struct[node], begin = b.begin[s];
+  if (!begin) return;
+  const StructState& st = b.state[s];
   const bool dyn = b.params[s].dynamic;
-  for (int i = threadIdx.x; i < inf.n_nodes * 6; i += blockDim.x) {
-    int64_t q = (int64_t)inf.node_off * 6 + i;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {
+    const int64_t q = (int64_t)node * 6 + j;
     b.disp[q] = 0.0;
-    if (zero_va) b.vel[q] = b.accel[q] = b.copy_vel[q] = b.copy_accel[q] = 0.0;
+    if (begin & 2) b.vel[q] = b.accel[q] = b.copy_vel[q] = b.copy_accel[q] = 0.0;
     if (dyn) {  // back to the converged velocities (a no-op after a commit)
       b.vel[q] = b.copy_vel[q];
       b.accel[q] = b.copy_accel[q];
     }
   }
-  __syncthreads();
   double time = st.last_converged_time + st.current_time_step, dt = st.current_time_step;
-  for (int e = threadIdx.x; e < b.n_disps; e += blockDim.x) {
-    const DispEntry D = b.disps[e];
-    if (D.structure != s) continue;
-    int node = D.node;
+  for (int e = b.n_disps ? b.disp_of[node] : b.n_disps; e < b.n_disps && b.disps[e].node == node; ++e) {
+    const DispEntry& D = b.disps[e];
     const int* cons = b.cons + (int64_t)node * 6;
     const int* gl = b.gl + (int64_t)node * 6;
     double dl[3], dg[3];
@@ -267,10 +253,17 @@ __global__ void k_step_begin(Batch b) {
         }
       }
   }
-  if (dyn) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < inf.n_nodes; i += blockDim.x) update_dyn_node(b, st.a, inf.node_off + i);
-  }
+  if (dyn) update_dyn_node(b, st.a, node);
+}
+
+// UpdateDyn after an increment (reference src/Dynamic.cpp:480-580), a thread per
+// node of the Dynamic structures that have just taken one.
+__global__ void k_update_dyn(Batch b) {
+  const int node = blockIdx.x * blockDim.x + threadIdx.x;
+  if (node >= b.n_nodes) return;
+  const int s = b.node_struct[node];
+  const StructState& st = b.state[s];
+  if (iterating(st) && st.need_solve && b.params[s].dynamic) update_dyn_node(b, st.a, node);
 }
 
 // clear band and P of iterating structures
@@ -548,8 +541,12 @@ __device__ void beam_modal_block(const BeamConst& c, const double (*D)[2][9], in
     for (int j = 0; j < 3; ++j) m[i * 3 + j] = T[i] * t2[j] + T[3 + i] * t2[3 + j] + T[6 + i] * t2[6 + j];
 }
 
-__global__ void k_beam_rayleigh(Batch b) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+// 32 elements per CTA, an element per lane (the scratch is structure-of-arrays)
+// and a row of C_e, K_e and f_e per warp, so that a row's 18 columns load side by
+// side.
+constexpr int RAY_THREADS = 18 * 32;
+__global__ void __launch_bounds__(RAY_THREADS) k_beam_rayleigh(Batch b) {
+  const int e = blockIdx.x * 32 + (threadIdx.x & 31), q = threadIdx.x >> 5;
   if (e >= b.n_elem) return;
   const int s = b.estruct[e];
   const StructState& st = b.state[s];
@@ -558,48 +555,40 @@ __global__ void k_beam_rayleigh(Batch b) {
   if (!p.dynamic || !p.ray_on) return;
   const int64_t ne = b.n_elem;
   double* C = b.RD + e;
+  double c[18], k[18];
+#pragma unroll
+  for (int x = 0; x < 18; ++x) {
+    c[x] = C[(int64_t)(q + 18 * x) * ne];
+    k[x] = b.Ke[(int64_t)(q + 18 * x) * ne + e];
+  }
   if (p.ray_update || !st.ray_init) {
-    const BeamConst& c = b.bconst[e];
+    const BeamConst& bc = b.bconst[e];
     double D[2][2][9];  // [Gauss point][translation, rotation][3x3 row-major]
-    beam_modal_D(c, b.baux[e], D);
-#pragma unroll 1
-    for (int I = 0; I < 3; ++I)
-#pragma unroll 1
-      for (int J = 0; J < 3; ++J)
-#pragma unroll 1
-        for (int bi = 0; bi < 2; ++bi)
-#pragma unroll 1
-          for (int bj = 0; bj < 2; ++bj) {
-            double m[9];
-            beam_modal_block(c, D, I, J, bi, bj, m);
+    beam_modal_D(bc, b.baux[e], D);
+    const int I = q / 6, bi = q % 6 / 3, i = q % 3;
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
+    for (int J = 0; J < 3; ++J)
 #pragma unroll
-              for (int j = 0; j < 3; ++j) {
-                const int64_t xi = (6 * I + 3 * bi + i) + 18 * (6 * J + 3 * bj + j);
-                C[xi * ne] = p.ray_alpha * m[i * 3 + j] + p.ray_beta * C[xi * ne];
-              }
-          }
+      for (int bj = 0; bj < 2; ++bj) {
+        double m[9];
+        beam_modal_block(bc, D, I, J, bi, bj, m);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const int x = 6 * J + 3 * bj + j;
+          const double mv = i == 0 ? m[j] : i == 1 ? m[3 + j] : m[6 + j];
+          c[x] = p.ray_alpha * mv + p.ray_beta * c[x];
+          C[(int64_t)(q + 18 * x) * ne] = c[x];
+        }
+      }
   }
   const double a4 = st.a[3];
-  double v[18];
+  double acc = 0.0;
 #pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const int64_t nd = b.enodes[3 * e + j];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) v[6 * j + q] = b.vel[nd * 6 + q];
+  for (int x = 0; x < 18; ++x) {
+    acc += c[x] * b.vel[(int64_t)b.enodes[3 * e + x / 6] * 6 + x % 6];
+    b.Ke[(int64_t)(q + 18 * x) * ne + e] = k[x] + a4 * c[x];
   }
-#pragma unroll 1
-  for (int q = 0; q < 18; ++q) {
-    double acc = 0.0;
-#pragma unroll 1
-    for (int k = 0; k < 18; ++k) {
-      const double cq = C[(int64_t)(q + 18 * k) * ne];
-      acc += cq * v[k];
-      b.Ke[(int64_t)(q + 18 * k) * ne + e] += a4 * cq;
-    }
-    b.Fe[(int64_t)q * ne + e] += acc;
-  }
+  b.Fe[(int64_t)q * ne + e] += acc;
 }
 
 // Pipe_1::MountPipeSpecialLoads (reference src/Pipe_1.cpp:1441-1494): the
@@ -611,44 +600,45 @@ __global__ void k_beam_rayleigh(Batch b) {
 // f_e -= jac T^T N^T (f, m) and K_e -= jac p0i Aint T^T N^T Kext Upsilon T.
 // Its O1 term reads the element's scalar g, which the reference's Mount
 // leaves at the second Gauss point's value (src/Pipe_1.cpp:890), for both
-// points.  One thread per pressurized element, after k_beam_tangent has
-// written K_e and f_e and before k_beam_rayleigh: in a Dynamic step the
-// reference mounts loads before damping, so on the iterations that form
-// C_e the load stiffness also goes into the stiffness part that C_e is
-// made from.
-__global__ void k_pipe_pressure(Batch b) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= b.n_pipe_press) return;
-  const int e = b.pp_elem[q];
-  const int s = b.estruct[e];
+// points.  After k_beam_tangent has written K_e and f_e and before
+// k_beam_rayleigh: in a Dynamic step the reference mounts loads before damping,
+// so on the iterations that form C_e the load stiffness also goes into the
+// stiffness part that C_e is made from.  32 elements per CTA, an element per
+// lane: warps 0 and 1 form the two Gauss points' blocks in shared memory, then
+// the eight warps share the entries of K_e.
+constexpr int PP_THREADS = 256;
+constexpr int PP_G = 0, PP_F = 36, PP_COUNT = 42;  // blocks G1..G4, then the force and moment
+__global__ void __launch_bounds__(PP_THREADS) k_pipe_pressure(Batch b) {
+  __shared__ double S[2][PP_COUNT][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * 32 + lane;
+  const int e = q < b.n_pipe_press ? b.pp_elem[q] : 0;
+  const int s = q < b.n_pipe_press ? b.estruct[e] : 0;
   const StructState& st = b.state[s];
-  if (!iterating(st)) return;
-  const StructParams& pr = b.params[s];
-  const bool form_c = pr.dynamic && pr.ray_on && (pr.ray_update || !st.ray_init);
-  const double p0i = table_at(b, b.pp_table[q], st.last_converged_time + st.current_time_step, 0);
-  const double Aint = b.pp_aint[q];
+  const bool on = q < b.n_pipe_press && iterating(st);
   const BeamConst& c = b.bconst[e];
-  const BeamHist& h = b.bhist[e];
-  double d[18];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const int64_t nd = b.enodes[3 * e + j];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) d[6 * j + k] = b.disp[nd * 6 + k];
+  double pa = 0.0, sK = 0.0;
+  if (on) {
+    const double p0i = table_at(b, b.pp_table[q], st.last_converged_time + st.current_time_step, 0);
+    const double Aint = b.pp_aint[q];
+    pa = -p0i * Aint;
+    sK = c.jac * p0i * Aint;
   }
-  M3<double> T;
+  if (on && warp < 2) {
+    const int g = warp;
+    const BeamHist& h = b.bhist[e];
+    double d[18];
 #pragma unroll
-  for (int i = 0; i < 9; ++i) T[i] = c.T3[i];
-  const V3<double> e3r = {{c.e3r[0], c.e3r[1], c.e3r[2]}};
-  const BeamInterp ip1 = beam_interp(c, d, 1);
-  const double g_last = 4.0 / (4.0 + dot(ip1.alpha, ip1.alpha));
-  const double pa = -p0i * Aint, sK = c.jac * p0i * Aint;
-  const int64_t ne = b.n_elem;
-  double* Ke = b.Ke + e;
-  double* Fe = b.Fe + e;
-  double* Ce = form_c ? b.RD + e : nullptr;
-#pragma unroll 1
-  for (int g = 0; g < 2; ++g) {
+    for (int j = 0; j < 3; ++j) {
+      const int64_t nd = b.enodes[3 * e + j];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) d[6 * j + k] = b.disp[nd * 6 + k];
+    }
+    M3<double> T;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) T[i] = c.T3[i];
+    const V3<double> e3r = {{c.e3r[0], c.e3r[1], c.e3r[2]}};
+    const BeamInterp ip1 = beam_interp(c, d, 1);
+    const double g_last = 4.0 / (4.0 + dot(ip1.alpha, ip1.alpha));
     const BeamInterp ip = beam_interp(c, d, g);
     double gg;
     M3<double> Qd, Xi, Qi;
@@ -686,39 +676,53 @@ __global__ void k_pipe_pressure(Batch b) {
     const M3<double> G1 = tmul(T, mul(K1ua, T)), G2 = tmul(T, mul(mul(E3, Xi), T));
     const M3<double> G3 = tmul(T, mul(tmul(Xi, E3), T)), G4 = tmul(T, mul(K1aa, T));
     const V3<double> fg = tmv(T, fl), mg = tmv(T, ml);
-#pragma unroll 1
-    for (int a = 0; a < 3; ++a) {
-      const double Na = c.N[g][a];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        Fe[(int64_t)(6 * a + i) * ne] -= c.jac * Na * (pa * fg[i]);
-        Fe[(int64_t)(6 * a + 3 + i) * ne] -= c.jac * Na * (pa * mg[i]);
-      }
-#pragma unroll 1
-      for (int n = 0; n < 3; ++n) {
-        const double Nb = c.N[g][n], dNb = c.dN[g][n];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            const int x = i * 3 + j;
-            // (u_a, alpha_b): K1ua Nb + K2ua dNb; (alpha_a, u_b): K2au dNb;
-            // (alpha_a, alpha_b): K1aa Nb
-            const int64_t x1 = (6 * a + i) + 18 * (6 * n + 3 + j), x2 = (6 * a + 3 + i) + 18 * (6 * n + j),
-                          x3 = (6 * a + 3 + i) + 18 * (6 * n + 3 + j);
-            const double v1 = sK * (Na * (Nb * G1[x] + dNb * G2[x])), v2 = sK * (Na * (dNb * G3[x])),
-                         v3 = sK * (Na * (Nb * G4[x]));
-            Ke[x1 * ne] -= v1;
-            Ke[x2 * ne] -= v2;
-            Ke[x3 * ne] -= v3;
-            if (Ce) {
-              Ce[x1 * ne] -= v1;
-              Ce[x2 * ne] -= v2;
-              Ce[x3 * ne] -= v3;
-            }
-          }
-      }
+    for (int x = 0; x < 9; ++x) {
+      S[g][PP_G + x][lane] = G1[x];
+      S[g][PP_G + 9 + x][lane] = G2[x];
+      S[g][PP_G + 18 + x][lane] = G3[x];
+      S[g][PP_G + 27 + x][lane] = G4[x];
     }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      S[g][PP_F + i][lane] = fg[i];
+      S[g][PP_F + 3 + i][lane] = mg[i];
+    }
+  }
+  __syncthreads();
+  if (!on) return;
+  const StructParams& pr = b.params[s];
+  const bool form_c = pr.dynamic && pr.ray_on && (pr.ray_update || !st.ray_init);
+  const int64_t ne = b.n_elem;
+  double* Ke = b.Ke + e;
+  double* Ce = form_c ? b.RD + e : nullptr;
+#pragma unroll 1
+  for (int k = warp; k < 18; k += 8) {
+    double f = b.Fe[(int64_t)k * ne + e];
+#pragma unroll
+    for (int g = 0; g < 2; ++g) f -= c.jac * c.N[g][k / 6] * (pa * S[g][PP_F + k % 6][lane]);
+    b.Fe[(int64_t)k * ne + e] = f;
+  }
+  // (u_a, alpha_n): K1ua Nb + K2ua dNb; (alpha_a, u_n): K2au dNb; (alpha_a,
+  // alpha_n): K1aa Nb
+#pragma unroll 1
+  for (int k = warp; k < 243; k += 8) {
+    const int kind = k / 81, a = k % 81 / 27, n = k % 27 / 9, x = k % 9, i = x / 3, j = x % 3;
+    const int64_t at =
+        kind == 0 ? (6 * a + i) + 18 * (6 * n + 3 + j)
+                  : kind == 1 ? (6 * a + 3 + i) + 18 * (6 * n + j) : (6 * a + 3 + i) + 18 * (6 * n + 3 + j);
+    double v = Ke[at * ne], w = Ce ? Ce[at * ne] : 0.0;
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      const double Na = c.N[g][a], Nb = c.N[g][n], dNb = c.dN[g][n];
+      const double t = kind == 0   ? sK * (Na * (Nb * S[g][PP_G + x][lane] + dNb * S[g][PP_G + 9 + x][lane]))
+                       : kind == 1 ? sK * (Na * (dNb * S[g][PP_G + 18 + x][lane]))
+                                   : sK * (Na * (Nb * S[g][PP_G + 27 + x][lane]));
+      v -= t;
+      w -= t;
+    }
+    Ke[at * ne] = v;
+    if (Ce) Ce[at * ne] = w;
   }
 }
 
@@ -815,49 +819,53 @@ __global__ void k_chain_gather_f(Batch b) {
 }
 
 // NodalLoad::Mount for every load entry of a structure, in entry order (one
-// thread per structure keeps the accumulation order fixed).
-__global__ void k_loads(Batch b) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
+// warp per structure keeps the accumulation order fixed; lanes 0-5 own the
+// entry's components, lanes 0-8 the entries of its load stiffness V(alpha,
+// Xi^T m)).
+__global__ void __launch_bounds__(128) k_loads(Batch b) {
+  const int s = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (s >= b.n_struct || !iterating(b.state[s])) return;
-  const StructInfo inf = b.info[s];
+  const StructInfo& inf = b.info[s];
   const StructState& st = b.state[s];
-  double time = st.last_converged_time + st.current_time_step;
+  const double time = st.last_converged_time + st.current_time_step;
   double* P = b.P + inf.dof_off;
   double* band = b.band + inf.band_off;
   const bool to_nodeK = (inf.is_chain || inf.wide) && !b.full_band;
   const bool to_wide = inf.wide && wide_band_filled(b);
+  const int c6 = lane < 6 ? lane : 0, i = lane < 9 ? lane / 3 : 0, j = lane % 3;
   for (int l = inf.load_off; l < inf.load_off + inf.n_loads; ++l) {
-    const LoadEntry L = b.loads[l];
-    int node = L.node;
+    const LoadEntry& L = b.loads[l];
+    const int node = L.node;
     const int* gl = b.gl + (int64_t)node * 6;
+    const double v = L.mult[c6] * table_at(b, L.table, time, c6);
     V3<double> fl, ml;
-    for (int i = 0; i < 3; ++i) {
-      fl[i] = L.mult[i] * table_at(b, L.table, time, i);
-      ml[i] = L.mult[3 + i] * table_at(b, L.table, time, i + 3);
+    for (int q = 0; q < 3; ++q) {
+      fl[q] = __shfl_sync(0xffffffffu, v, q);
+      ml[q] = __shfl_sync(0xffffffffu, v, 3 + q);
     }
-    M3<double> CQ;
-    for (int q = 0; q < 9; ++q) CQ[q] = L.CQ[q];
-    V3<double> fv = tmv(CQ, fl), mvv = tmv(CQ, ml);
-    V3<double> al = {{b.disp[(int64_t)node * 6 + 3], b.disp[(int64_t)node * 6 + 4], b.disp[(int64_t)node * 6 + 5]}};
-    double g = 4.0 / (4.0 + dot(al, al));
-    M3<double> A = skew(al), Xi;
-    for (int q = 0; q < 9; ++q) Xi[q] = g * 0.5 * A[q];
-    Xi[0] += g; Xi[4] += g; Xi[8] += g;
-    V3<double> mm = tmv(Xi, mvv);
-    M3<double> V = opV(al, mm, g);
-    for (int i = 0; i < 3; ++i)
-      if (gl[i] >= 0) P[gl[i]] += -1.0 * fv[i];
-    for (int i = 0; i < 3; ++i) {
-      int gi = gl[3 + i];
-      if (gi >= 0) P[gi] += -1.0 * mm[i];
-      for (int j = 0; j < 3; ++j) {
-        int gj = gl[3 + j];
-        if (gi < 0 || gj < 0) continue;
-        if (to_nodeK) b.nodeK[(int64_t)node * 9 + i * 3 + j] += -1.0 * V[i * 3 + j];
-        if (to_wide) b.sh.wband[inf.wb_off + (inf.wkl + gi - gj) + (int64_t)gj * (2 * inf.wkl + 1)] += -1.0 * V[i * 3 + j];
-        else if (!to_nodeK) band[(GF_KB + gi - gj) + (int64_t)gj * GF_LDB] += -1.0 * V[i * 3 + j];
-      }
+    const V3<double> al = {{b.disp[(int64_t)node * 6 + 3], b.disp[(int64_t)node * 6 + 4], b.disp[(int64_t)node * 6 + 5]}};
+    const double g = 4.0 / (4.0 + dot(al, al));
+    // component c6 of CQ^T (f, m): lanes 0-2 the force, 3-5 the moment
+    const V3<double>& w = lane < 3 ? fl : ml;
+    const int r = c6 % 3;
+    double comp = L.CQ[r] * w[0] + L.CQ[3 + r] * w[1] + L.CQ[6 + r] * w[2];
+    V3<double> mv3;
+    for (int q = 0; q < 3; ++q) mv3[q] = __shfl_sync(0xffffffffu, comp, 3 + q);
+    // Xi^T m = g (m - alpha x m / 2), and its cross product with alpha
+    V3<double> am = cross(al, mv3), mm;
+    for (int q = 0; q < 3; ++q) mm[q] = g * (mv3[q] - 0.5 * am[q]);
+    if (lane < 6) {
+      const int gi = gl[lane];
+      if (gi >= 0) P[gi] += -1.0 * (lane < 3 ? comp : mm[lane - 3]);
     }
+    const int gi = gl[3 + i], gj = gl[3 + j];
+    if (lane < 9 && gi >= 0 && gj >= 0) {
+      const double V = opV(al, mm, g)[lane];
+      if (to_nodeK) b.nodeK[(int64_t)node * 9 + lane] += -1.0 * V;
+      if (to_wide) b.sh.wband[inf.wb_off + (inf.wkl + gi - gj) + (int64_t)gj * (2 * inf.wkl + 1)] += -1.0 * V;
+      else if (!to_nodeK) band[(GF_KB + gi - gj) + (int64_t)gj * GF_LDB] += -1.0 * V;
+    }
+    __syncwarp();  // the next entry may add to the same DOFs from other lanes
   }
 }
 
@@ -873,23 +881,22 @@ __global__ void k_residual(Batch b) {
   double* P = b.P + inf.dof_off;
   const int* d6 = b.dof_node6 + inf.dof_off;
   const int i1 = min(inf.n_free, b.chunk_start[blockIdx.x] + GF_RED_CHUNK);
-  Red3 v{0.0, 0.0, 0};
+  mag_t va = 0, vb = 0;
+  bool vf = false;
   for (int i = b.chunk_start[blockIdx.x] + threadIdx.x; i < i1; i += blockDim.x) {
-    double x = -1.0 * P[i];
-    P[i] = x;
-    double a = fabs(x);
-    if (nan_or_huge(a)) v.f = 1;
-    if (d6[i] % 6 < 3) { if (a > v.a) v.a = a; }
-    else { if (a > v.b) v.b = a; }
+    const double p0 = P[i];
+    P[i] = -p0;
+    const mag_t a = mag(p0);
+    vf = vf || a >= MAG_HUGE;
+    if (d6[i] % 6 < 3) mag_max(va, a);
+    else mag_max(vb, a);
   }
-  Red3 r = block_red(v);
   RedScratch& R = b.red[s];
-  if (threadIdx.x == 0) {
-    red_max(&R.a, r.a);
-    red_max(&R.b, r.b);
-    if (r.f) atomicOr(&R.f, 1);
-  }
+  red_max(&R.a, va);
+  red_max(&R.b, vb);
+  red_flag(&R.f, vf);
   if (!red_arrive(R, red_chunks(inf))) return;
+  Red3 r{};
   if (threadIdx.x == 0) {
     r.a = red_value(&R.a);
     r.b = red_value(&R.b);
@@ -1094,31 +1101,31 @@ __global__ void k_update(Batch b) {
   const double* P = b.P + inf.dof_off;
   const int* d6 = b.dof_node6 + inf.dof_off;
   const int i1 = min(inf.n_free, b.chunk_start[blockIdx.x] + GF_RED_CHUNK);
-  Red3 inc{0.0, 0.0, 0}, val{0.0, 0.0, 0};
+  mag_t ia = 0, ib = 0, wa = 0, wb = 0;
+  bool vf = false;
   for (int i = b.chunk_start[blockIdx.x] + threadIdx.x; i < i1; i += blockDim.x) {
     int q = d6[i];
     double x = P[i];
     double nv = b.disp[q] + x;
     b.disp[q] = nv;
-    double a = fabs(x), v = fabs(nv);
-    if (nan_or_huge(a)) inc.f = 1;
-    if (q % 6 < 3) { if (a > inc.a) inc.a = a; if (v > val.a) val.a = v; }
-    else { if (a > inc.b) inc.b = a; if (v > val.b) val.b = v; }
+    const mag_t a = mag(x), v = mag(nv);
+    vf = vf || a >= MAG_HUGE;
+    if (q % 6 < 3) {
+      mag_max(ia, a);
+      mag_max(wa, v);
+    } else {
+      mag_max(ib, a);
+      mag_max(wb, v);
+    }
   }
-  Red3 ri = block_red(inc);
-  Red3 rv = block_red(val);
   RedScratch& R = b.red[s];
-  if (threadIdx.x == 0) {
-    red_max(&R.a, ri.a);
-    red_max(&R.b, ri.b);
-    red_max(&R.va, rv.a);
-    red_max(&R.vb, rv.b);
-    if (ri.f) atomicOr(&R.f, 1);
-  }
+  red_max(&R.a, ia);
+  red_max(&R.b, ib);
+  red_max(&R.va, wa);
+  red_max(&R.vb, wb);
+  red_flag(&R.f, vf);
   if (!red_arrive(R, red_chunks(inf))) return;
-  // the last CTA: every increment of the structure is in place
-  if (b.params[s].dynamic)
-    for (int i = threadIdx.x; i < inf.n_nodes; i += blockDim.x) update_dyn_node(b, st.a, inf.node_off + i);
+  Red3 ri{}, rv{};
   if (threadIdx.x == 0) {
     ri.a = red_value(&R.a);
     ri.b = red_value(&R.b);
@@ -1443,24 +1450,31 @@ static void set_attrs();
 
 static void launch_mount(const Batch& b, cudaStream_t st, LaunchProf* prof);
 
+static void launch_loads(const Batch& b, cudaStream_t st) {
+  if (b.n_loads) k_loads<<<(b.n_struct + 3) / 4, 128, 0, st>>>(b);
+}
+
 void launch_iteration_partial(const Batch& b_in, cudaStream_t st) {
   set_attrs();
   Batch b = b_in;
   b.full_band = 1;  // the assembly view: every structure's band is filled
   int ns = b.n_struct;
-  k_step_begin<<<ns, 256, 0, st>>>(b);
+  launch_step_begin(b, st);
   k_zero<<<dim3(8, ns), 256, 0, st>>>(b);
   launch_wide_zero(b, st);
   launch_mount(b, st, nullptr);
   launch_shell_mount(b, st);
-  k_loads<<<(ns + 63) / 64, 64, 0, st>>>(b);
+  launch_loads(b, st);
   k_residual<<<b.n_chunks, 256, 0, st>>>(b);
 }
 
 // The stages of one Newton iteration for a caller that runs its own step
 // control (gf_begin_step, gf_assemble, gf_set_increment, gf_commit): every
 // structure's band is filled (the assembly view), as the caller reads K_AA.
-void launch_step_begin(const Batch& b, cudaStream_t st) { k_step_begin<<<b.n_struct, 256, 0, st>>>(b); }
+void launch_step_begin(const Batch& b, cudaStream_t st) {
+  k_step_begin<<<(b.n_struct + 63) / 64, 64, 0, st>>>(b);
+  if (b.n_nodes) k_step_nodes<<<(b.n_nodes + 127) / 128, 128, 0, st>>>(b);
+}
 
 void launch_assembly(const Batch& b_in, cudaStream_t st) {
   set_attrs();
@@ -1471,11 +1485,14 @@ void launch_assembly(const Batch& b_in, cudaStream_t st) {
   launch_wide_zero(b, st);
   launch_mount(b, st, nullptr);
   launch_shell_mount(b, st);
-  k_loads<<<(ns + 63) / 64, 64, 0, st>>>(b);
+  launch_loads(b, st);
   k_residual<<<b.n_chunks, 256, 0, st>>>(b);
 }
 
-void launch_increment(const Batch& b, cudaStream_t st) { k_update<<<b.n_chunks, 256, 0, st>>>(b); }
+void launch_increment(const Batch& b, cudaStream_t st) {
+  k_update<<<b.n_chunks, 256, 0, st>>>(b);
+  if (b.any_dynamic) k_update_dyn<<<(b.n_nodes + 127) / 128, 128, 0, st>>>(b);
+}
 
 void launch_commit(const Batch& b, cudaStream_t st) {
   if (b.n_elem) k_commit_elems<<<(b.n_elem + 63) / 64, 128, 0, st>>>(b);
@@ -1512,8 +1529,8 @@ static void launch_mount(const Batch& b, cudaStream_t st, LaunchProf* prof) {
     k_beam_tangent<<<(b.n_elem + 31) / 32, MOUNT_THREADS, MOUNT_SMEM_BATCH, st>>>(b);
     // the pressure's load stiffness is part of the K_e that Rayleigh damping
     // reads (the reference mounts loads before damping)
-    if (b.n_pipe_press) k_pipe_pressure<<<(b.n_pipe_press + 127) / 128, 128, 0, st>>>(b);
-    if (b.any_rayleigh) k_beam_rayleigh<<<(b.n_elem + 127) / 128, 128, 0, st>>>(b);
+    if (b.n_pipe_press) k_pipe_pressure<<<(b.n_pipe_press + 31) / 32, PP_THREADS, 0, st>>>(b);
+    if (b.any_rayleigh) k_beam_rayleigh<<<(b.n_elem + 31) / 32, RAY_THREADS, 0, st>>>(b);
   }
   if (!b.full_band && b.chain.n_chain_elems + b.chain.sy.n_elem == b.n_elem) {
     // chains only: the residual is all the scatter would assemble
@@ -1533,18 +1550,18 @@ static void launch_mount(const Batch& b, cudaStream_t st, LaunchProf* prof) {
 void launch_iteration(const Batch& b, cudaStream_t st, bool commit_kernels, LaunchProf* prof) {
   set_attrs();
   int ns = b.n_struct;
-  { ProfScope q(prof, st, KC_STEP_BEGIN); k_step_begin<<<ns, 256, 0, st>>>(b); }
+  { ProfScope q(prof, st, KC_STEP_BEGIN); launch_step_begin(b, st); }
   { ProfScope q(prof, st, KC_ZERO); k_zero<<<dim3(8, ns), 256, 0, st>>>(b); }
   if (b.sh.n_wide) { ProfScope q(prof, st, KC_ZERO); launch_wide_zero(b, st); }
   launch_mount(b, st, prof);
   if (b.sh.n_shells) { ProfScope q(prof, st, KC_SHELL); launch_shell_mount(b, st); }
-  { ProfScope q(prof, st, KC_LOADS); k_loads<<<(ns + 63) / 64, 64, 0, st>>>(b); }
+  { ProfScope q(prof, st, KC_LOADS); launch_loads(b, st); }
   { ProfScope q(prof, st, KC_RESIDUAL); k_residual<<<b.n_chunks, 256, 0, st>>>(b); }
   { ProfScope q(prof, st, KC_SOLVE); launch_band_solve(b, st); }
   if (b.chain.n_chain_elems) { ProfScope q(prof, st, KC_CHAIN); launch_chain_solve(b, b.chain, st); }
   if (b.chain.sy.n_elem) { ProfScope q(prof, st, KC_CHAIN); launch_sym_chains(b, b.chain.sy, st); }
   if (b.sh.n_wide) launch_wide_solve(b, st, prof);
-  { ProfScope q(prof, st, KC_UPDATE); k_update<<<b.n_chunks, 256, 0, st>>>(b); }
+  { ProfScope q(prof, st, KC_UPDATE); launch_increment(b, st); }
   { ProfScope q(prof, st, KC_CONTROL); k_control<<<(ns + 127) / 128, 128, 0, st>>>(b); }
   if (commit_kernels) {
     if (b.n_elem) { ProfScope q(prof, st, KC_COMMIT_ELEMS); k_commit_elems<<<(b.n_elem + 63) / 64, 128, 0, st>>>(b); }

@@ -95,6 +95,30 @@ template <typename T, typename S> GF_HD V3<T> cvt(const V3<S>& a) {
   return r;
 }
 
+#ifdef __CUDACC__
+// 1/p from a single-precision seed of p's own bits (r0, 2^-23) and one
+// third-order step r = r0 + r0 (e + e^2), e = 1 - p r0 (2^-69): three dependent
+// FP64 results (64 cycles each on this part) in place of the six of two
+// second-order steps and the seed's two conversions.  The division where the
+// seed is out of range.
+__device__ __forceinline__ double rcp64(double p) {
+  const long long u = __double_as_longlong(p);
+  const int ex = (int)((u >> 52) & 0x7FF);
+  if (ex < 64 || ex > 1982) return 1.0 / p;
+  // m in [1, 2) from the leading bits of the fraction, its reciprocal in (0.5, 1]
+  const float m = __int_as_float(0x3F800000 | (int)((u >> 29) & 0x7FFFFF));
+  float rf;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(m));
+  const int rb = __float_as_int(rf);
+  // the seed's bits as a double, scaled by 2^(1023 - ex), with p's sign
+  const long long r0b = ((long long)((rb >> 23) - 127 + 1023 + 1023 - ex) << 52) | ((long long)(rb & 0x7FFFFF) << 29) |
+                        (u & (long long)0x8000000000000000ull);
+  const double r0 = __longlong_as_double(r0b);
+  const double e = fma(-p, r0, 1.0);
+  return fma(r0, fma(e, e, e), r0);
+}
+#endif
+
 // Rodrigues tensor Q = I + g (A + A^2 / 2), g = 4 / (4 + |a|^2)
 template <typename T> GF_HD M3<T> rodrigues(const V3<T>& a) {
   T n2 = dot(a, a);

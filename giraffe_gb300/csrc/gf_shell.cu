@@ -132,8 +132,7 @@ __device__ __forceinline__ double table_value(const Batch& b, int t, double time
   if (T.n_times == 0) return 0.0;
   if (time >= times[T.n_times - 1]) return vals[(int64_t)(T.n_times - 1) * T.n_cols];
   if (time <= times[0]) return vals[0];
-  int idx = 0;
-  while (time >= times[idx]) idx++;
+  const int idx = table_row(T, times, time);
   double f = (time - times[idx - 1]) / (times[idx] - times[idx - 1]);
   double a = vals[(int64_t)(idx - 1) * T.n_cols], c = vals[(int64_t)idx * T.n_cols];
   return a + f * (c - a);

@@ -199,8 +199,30 @@ struct DispEntry {
 
 struct TableDev {
   int n_times, n_cols;
+  int sorted, pad;  // times do not decrease (table_row's binary search)
   int64_t off;  // into the batch's table storage: times then values
 };
+
+#ifdef __CUDACC__
+// The first row of a table with times[row] > time, for times[0] < time <
+// times[n - 1]: by bisection where the times are sorted (a scan costs an FP64
+// comparison, 64 cycles here, per row passed), else by the scan of
+// Table::GetValueAt.
+__device__ __forceinline__ int table_row(const TableDev& T, const double* times, double time) {
+  int lo = 0;
+  if (!T.sorted) {
+    while (time >= times[lo]) lo++;
+    return lo;
+  }
+  int hi = T.n_times - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (time >= times[mid]) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+#endif
 
 // Chain solver data (see gf_chain.cuh).
 #define CR_MAX_LEVELS 24
@@ -433,7 +455,9 @@ struct Batch {
   double* mon_rec;
   // loads
   LoadEntry* loads;
-  DispEntry* disps;
+  DispEntry* disps;  // sorted by node
+  int* disp_of;      // per node: its first entry of disps (n_disps: none); only when n_disps
+  int* begin;        // per structure: this pass starts a step (k_step_begin)
   TableDev* tables;
   double* table_data;
   // chain structures: the nodal load stiffness (rotation block, row-major
