@@ -1,32 +1,30 @@
-// Chain solver kernels (see gf_chain.cuh): the general elimination, for Dynamic
-// steps and loads with stiffness of their own (the symmetric one is in
-// gf_chain_sym.cu).  Gauss-Jordan on [D | b | L | U], in two forms with the same
-// operations on every entry, so the same bits: one item per thread, whose FP64
-// warp instructions carry 32 items, for the large levels, and one item per
-// warp for the small ones, where an item's chain of dependent operations (64
-// cycles each on this part) is what counts.
+// General elimination of Beam_1 chains (see gf_chain.cuh): Dynamic steps and loads
+// with stiffness of their own, whose K_AA is not symmetric (the symmetric one is
+// in gf_chain_sym.cu).  Parts are 12x12 matrices over the DOFs (u_p, a_p, u_n,
+// a_n) of their two corners.  An elimination of six unknowns is Gauss-Jordan on
+// [D | b | K_p | K_n] (19 columns) and the products of the two coupling rows with
+// the 13 solved columns, about 1,550 FP64 operations that form the new part
+// outright.
+//
+// Two forms with the same operations on every entry, so the same bits: one item
+// per thread, whose FP64 warp instructions carry 32 items, for the large levels,
+// and one item per warp for the small ones, where an item's chain of dependent
+// operations (64 cycles each on this part) is what counts.
 #include <cuda_runtime.h>
 
 #include "gf_chain.cuh"
+#include "gf_chain_root.cuh"
 #include "gf_math.cuh"
 
 namespace gf {
 
 namespace {
 
-constexpr int CT = 64;   // threads per block
+constexpr int CT = 64;  // threads per block of the item-per-thread form
+constexpr int NC = 19;  // augmented columns: 6 (matrix) + 13 (right-hand sides)
 
-// Scratch arrays are structure-of-arrays: entry x of chain element t at
-// [x * n_chain_elems + t], entry x of corner k at [x * n_corners + k], so
-// that the threads of a warp (consecutive items) touch consecutive addresses.
-#define ELM(arr, t, x) (arr)[(int64_t)(x) * c.n_chain_elems + (t)]
-#define CRN(arr, k, x) (arr)[(int64_t)(x) * c.n_corners + (k)]
-constexpr int NC = 19;   // augmented columns: 6 (matrix) + 13 (right-hand sides)
-
-__device__ __forceinline__ bool solving(const Batch& b, int s) {
-  const StructState& st = b.state[s];
-  return st.phase == PH_ITER && st.need_solve;
-}
+// Part: the matrix ([row * 12 + column]), then the forces on p and n.
+constexpr int GP_F = 144;
 
 // Gauss-Jordan on a thread's augmented matrix [D | R] in two phases, both in
 // registers: gj6_factor eliminates D (6x6, row-major, every index static under
@@ -71,104 +69,153 @@ __device__ __forceinline__ void gj6_apply(const double (&inv)[6], const double (
   }
 }
 
-// ---- 1. condensation of the midside node of every chain element ----
-__global__ void __launch_bounds__(CT) k_condense(Batch b, ChainData c) {
-  int t = blockIdx.x * CT + threadIdx.x;
-  if (t >= c.n_chain_elems) return;
-  int e = c.elem_list[t];
-  int s = b.estruct[e];
-  if (!solving(b, s)) return;
-  const StructInfo& inf = b.info[s];
-  const double* P = b.P + inf.dof_off;
-  double D[36];  // K_mm (+ the load stiffness)
-  // K of the chain comes from the element tangents (column-major 18x18,
-  // DOFs of the first corner, the midside node, the last corner) plus the
-  // nodal load stiffness of the midside node: the midside rows belong to
-  // this element alone
-  const double* Kb = b.Ke + e;  // structure-of-arrays: entry x at Kb[x * n_elem]
-  const int64_t ne = b.n_elem;
-#define K(x) Kb[(int64_t)(x) * ne]
-  const double* nk = b.nodeK + (int64_t)b.enodes[3 * e + 1] * 9;
-  int nm = b.enodes[3 * e + 1];
-  const int mask = c.elem_mask[t];  // free DOFs of the two corners
-  int gm[6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) gm[i] = b.gl[(int64_t)nm * 6 + i];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) {
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      double kmm = K((6 + i) + 18 * (6 + j));
-      if (i >= 3 && j >= 3) kmm += nk[(i - 3) * 3 + j - 3];
-      D[i * 6 + j] = kmm;
-    }
+// Condensation of the midside node of part t: K_e (column-major 18x18, DOFs of
+// the first corner, the midside node, the last corner) and the midside node's
+// load stiffness.  Fixed DOFs of the corners have zero rows and columns.
+struct GenCondense {
+  const Batch& b;
+  const ChainParts& c;
+  int t, s, mask, nm;
+  const double *K, *P;
+  int64_t ne;
+  __device__ __forceinline__ void init(int t_) {
+    t = t_;
+    const int e = c.elem[t];
+    s = c.elem_struct[t];
+    mask = c.elem_mask[t];
+    nm = b.enodes[3 * e + 1];
+    K = b.Ke + e;
+    P = b.P + c.elem_dof[t];
+    ne = b.n_elem;
   }
-  double inv[6], mult[36];
-  if (!gj6_factor(D, inv, mult)) b.state[s].info_fail = 1;
-  // Z = K_mm^-1 [P_m | K_ma | K_mb] a column at a time, and with each column
-  // its share of -A_as Z and -A_bs Z (6 x 13 each: the same FMA chain over j
-  // for every entry)
+  __device__ __forceinline__ bool active() const { return solving(b, s); }
+  __device__ __forceinline__ static int place(int x) { return x < 6 ? x : 6 + x; }  // corner DOF 0..11 in K_e
+  __device__ __forceinline__ bool live(int x) const { return mask >> x & 1; }
+  __device__ __forceinline__ double ke(int i, int j) const { return K[(int64_t)(i + 18 * j) * ne]; }
+  __device__ __forceinline__ double d(int i, int j) const {
+    double v = ke(6 + i, 6 + j);
+    if (i >= 3 && j >= 3) v += b.nodeK[(int64_t)nm * 9 + (i - 3) * 3 + j - 3];
+    return v;
+  }
+  __device__ __forceinline__ double r(int i, int q) const {
+    return q == 0 ? P[i] : live(q - 1) ? ke(6 + i, place(q - 1)) : 0.0;
+  }
+  // coupling of corner DOF x to unknown k
+  __device__ __forceinline__ double left(int x, int k) const { return live(x) ? ke(place(x), 6 + k) : 0.0; }
+  __device__ __forceinline__ double base(int x, int q) const {
+    return q == 0 || !live(x) || !live(q - 1) ? 0.0 : ke(place(x), place(q - 1));
+  }
+  __device__ __forceinline__ void keep(int x, double v) const { chain_at(c.ez, c.elem_soa, CHAIN_GEN_KEEP, t, x) = v; }
+  __device__ __forceinline__ void out(int x, int q, double v) const {
+    chain_at(c.part, c.part_soa, CHAIN_GEN_PART, t, q == 0 ? GP_F + x : x * 12 + q - 1) = v;
+  }
+  __device__ void fail() const { b.state[s].info_fail = 1; }
+};
+
+// Elimination of corner k between parts e1 (p to k) and e2 (k to n).
+struct GenMerge {
+  const Batch& b;
+  const ChainParts& c;
+  ChainMerge m;
+  int t, node;
+  __device__ __forceinline__ void init(int t_) {
+    t = t_;
+    m = c.merge[t];
+    node = c.corner_node[m.k];
+  }
+  __device__ __forceinline__ bool active() const { return solving(b, m.structure); }
+  __device__ __forceinline__ double E(int e, int x) const { return chain_at(c.part, c.part_soa, CHAIN_GEN_PART, e, x); }
+  __device__ __forceinline__ bool live(int i) const { return m.mask >> i & 1; }
+  __device__ __forceinline__ double d(int i, int j) const {
+    if (!live(i) || !live(j)) return i == j ? 1.0 : 0.0;
+    double v = E(m.e1, (6 + i) * 12 + 6 + j) + E(m.e2, i * 12 + j);
+    if (i >= 3 && j >= 3) v += b.nodeK[(int64_t)node * 9 + (i - 3) * 3 + j - 3];
+    return v;
+  }
+  __device__ __forceinline__ double r(int i, int q) const {
+    if (q == 0)  // the corner's own force with what both parts leave on it
+      return live(i) ? b.P[m.dof + __popc(m.mask & ((1 << i) - 1))] + E(m.e1, GP_F + 6 + i) + E(m.e2, GP_F + i) : 0.0;
+    return q < 7 ? E(m.e1, (6 + i) * 12 + q - 1) : E(m.e2, i * 12 + q - 1);
+  }
+  __device__ __forceinline__ double left(int x, int k) const {
+    return x < 6 ? E(m.e1, x * 12 + 6 + k) : E(m.e2, x * 12 + k);
+  }
+  __device__ __forceinline__ double base(int x, int q) const {
+    if (q == 0) return x < 6 ? E(m.e1, GP_F + x) : E(m.e2, GP_F + x);
+    if ((x < 6) != (q < 7)) return 0.0;
+    return E(x < 6 ? m.e1 : m.e2, x * 12 + q - 1);
+  }
+  __device__ __forceinline__ void keep(int x, double v) const { chain_at(c.mz, c.merge_soa, CHAIN_GEN_KEEP, t, x) = v; }
+  __device__ __forceinline__ void out(int x, int q, double v) const {
+    chain_at(c.part, c.part_soa, CHAIN_GEN_PART, m.out, q == 0 ? GP_F + x : x * 12 + q - 1) = v;
+  }
+  __device__ void fail() const { b.state[m.structure].info_fail = 1; }
+};
+
+// An item per thread: Z = D^-1 R a column at a time into shared memory, then the
+// new part a row at a time, so that every coupling entry is loaded once.
+constexpr int GEN_SMEM = 78 * CT * (int)sizeof(double);
+template <typename Item> __global__ void __launch_bounds__(CT) k_gen(Batch b, ChainParts c, int lo, int hi) {
+  extern __shared__ double gen_z[];
+  double* z = gen_z + threadIdx.x;  // [row * 13 + column][thread]
+  const int t = lo + blockIdx.x * CT + threadIdx.x;
+  if (t >= hi) return;
+  Item I{b, c};
+  I.init(t);
+  if (!I.active()) return;
+  {
+    double D[36];
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+      for (int j = 0; j < 6; ++j) D[i * 6 + j] = I.d(i, j);
+    double inv[6], mult[36];
+    if (!gj6_factor(D, inv, mult)) I.fail();
 #pragma unroll 1
-  for (int q = 0; q < 13; ++q) {
-    double r[6];
+    for (int q = 0; q < 13; ++q) {
+      double r[6];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      if (q == 0) r[i] = P[gm[i]];
-      else if (!(mask >> (q - 1) & 1)) r[i] = 0.0;
-      else r[i] = K((6 + i) + 18 * (q < 7 ? q - 1 : 5 + q));
-    }
-    gj6_apply(inv, mult, r);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) ELM(c.ez, t, i * 13 + q) = r[i];
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {
-      const int r0 = side ? 12 : 0;
+      for (int i = 0; i < 6; ++i) r[i] = I.r(i, q);
+      gj6_apply(inv, mult, r);
 #pragma unroll
       for (int i = 0; i < 6; ++i) {
-        const bool live = mask >> (6 * side + i) & 1;
-        double acc = 0.0;
-#pragma unroll
-        for (int j = 0; j < 6; ++j) acc = fma(live ? K((r0 + i) + 18 * (6 + j)) : 0.0, r[j], acc);
-        ELM(c.ec, t, i * 26 + side * 13 + q) = -acc;
+        z[(i * 13 + q) * CT] = r[i];
+        I.keep(i * 13 + q, r[i]);
       }
+    }
+  }
+#pragma unroll 1
+  for (int x = 0; x < 12; ++x) {
+    double left[6], acc[13];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) left[k] = I.left(x, k);
+#pragma unroll
+    for (int q = 0; q < 13; ++q) acc[q] = I.base(x, q);
+#pragma unroll
+    for (int q = 0; q < 13; ++q) {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) acc[q] = fma(-left[k], z[(k * 13 + q) * CT], acc[q]);
+      I.out(x, q, acc[q]);
     }
   }
 }
 
-#undef K
-
-// Warp-per-element form of k_condense for small batches: lane q holds column q
-// of [K_mm | P_m | K_ma | K_mb] (lanes 0-5 the matrix), the pivot column is
-// broadcast by shuffle; then the lanes share the products A_as Z, A_bs Z.  The
-// same operations on every entry as k_condense.
-__global__ void __launch_bounds__(128) k_condense_w(Batch b, ChainData c) {
-  __shared__ double zs[4][6][13];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t = blockIdx.x * 4 + warp;
-  if (t >= c.n_chain_elems) return;
-  const int e = c.elem_list[t], s = b.estruct[e];
-  if (!solving(b, s)) return;
-  const StructInfo& inf = b.info[s];
-  const double* P = b.P + inf.dof_off;
-  const double* Kb = b.Ke + e;
-  const int64_t ne = b.n_elem;
-  const int nm = b.enodes[3 * e + 1], mask = c.elem_mask[t];
-  const double* nk = b.nodeK + (int64_t)nm * 9;
-  double col[6];
+// An item per warp: lane q < 19 holds column q of [D | R], the pivot column is
+// broadcast by shuffle; then the lanes share the entries of the new part.
+template <typename Item> __device__ __forceinline__ bool gen_item(const Item& I, int lane, double (*zs)[13]) {
+  double col[6], base[5], left[5][6];
 #pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    double v = 0.0;
-    if (lane < 6) {
-      v = Kb[((6 + i) + 18 * (6 + lane)) * ne];
-      if (i >= 3 && lane >= 3) v += nk[(i - 3) * 3 + lane - 3];
-    } else if (lane == 6) {
-      v = P[b.gl[(int64_t)nm * 6 + i]];
-    } else if (lane < NC && (mask >> (lane - 7) & 1)) {
-      const int q = lane - 6;
-      v = Kb[((6 + i) + 18 * (q < 7 ? q - 1 : 5 + q)) * ne];
-    }
-    col[i] = v;
+  for (int i = 0; i < 6; ++i) col[i] = lane < 6 ? I.d(i, lane) : lane < NC ? I.r(i, lane - 6) : 0.0;
+  // the products' operands, loaded ahead of the dependent chain
+#pragma unroll
+  for (int y = 0; y < 5; ++y) {
+    const int o = lane + 32 * y, x = o / 13, q = o % 13;
+    if (o >= 156) break;
+    base[y] = I.base(x, q);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) left[y][k] = I.left(x, k);
   }
+  if (!I.active()) return true;
   bool ok = true;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
@@ -186,390 +233,130 @@ __global__ void __launch_bounds__(128) k_condense_w(Batch b, ChainData c) {
         if (i != k) col[i] = fma(-m[i], rk, col[i]);
     }
   }
-  if (!ok && lane == 0) b.state[s].info_fail = 1;
   if (lane >= 6 && lane < NC)
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-      zs[warp][i][lane - 6] = col[i];
-      ELM(c.ez, t, i * 13 + lane - 6) = col[i];
+      zs[i][lane - 6] = col[i];
+      I.keep(i * 13 + lane - 6, col[i]);
     }
   __syncwarp();
-  for (int o = lane; o < 156; o += 32) {
-    const int i = o / 26, side = o % 26 / 13, q = o % 13;
-    const bool live = mask >> (6 * side + i) & 1;
-    double acc = 0.0;
 #pragma unroll
-    for (int j = 0; j < 6; ++j)
-      acc = fma(live ? Kb[(((side ? 12 : 0) + i) + 18 * (6 + j)) * ne] : 0.0, zs[warp][j][q], acc);
-    ELM(c.ec, t, o) = -acc;
+  for (int y = 0; y < 5; ++y) {
+    const int o = lane + 32 * y, x = o / 13, q = o % 13;
+    if (o >= 156) break;
+    double acc = base[y];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) acc = fma(-left[y][k], zs[k][q], acc);
+    I.out(x, q, acc);
   }
+  __syncwarp();
+  return ok;
 }
-
-// ---- 2. corner system: entry blockIdx.y of a corner per thread (0-35 D, 36-71
-// U, 72-107 L, 108-113 b).  K blocks come from the element tangents: the corner
-// is the last node of the element on its left and the first of the one on its
-// right (two terms, so the sum does not depend on their order), then the nodal
-// load stiffness.  A fixed DOF of a partly constrained corner is an identity
-// row and column. ----
-__global__ void k_corner_system(Batch b, ChainData c) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= c.n_corners) return;
-  const int s = c.corner_struct[k];
-  if (!solving(b, s)) return;
-  const StructInfo& inf = b.info[s];
-  const int x = blockIdx.y % 36, i = x / 6, j = x % 6, part = blockIdx.y / 36;
-  const int node = c.corner_node[k], eL = c.corner_left[k], eR = c.corner_right[k];
-  const int64_t ne = b.n_elem;
-  const double* KL = eL >= 0 ? b.Ke + c.elem_list[eL] : nullptr;
-  const double* KR = eR >= 0 ? b.Ke + c.elem_list[eR] : nullptr;
-  const int mask = c.corner_mask[k];
-  const bool live_i = mask >> i & 1;
-  if (part == 0) {
-    double d = i == j ? 1.0 : 0.0;
-    if (live_i && (mask >> j & 1)) {
-      const double kl = KL ? KL[((12 + i) + 18 * (12 + j)) * ne] : 0.0, kr = KR ? KR[(i + 18 * j) * ne] : 0.0;
-      d = kl + kr;
-      if (i >= 3 && j >= 3) d += b.nodeK[(int64_t)node * 9 + (i - 3) * 3 + j - 3];
-      if (eL >= 0) d += ELM(c.ec, eL, i * 26 + 13 + 7 + j);  // -A_bs Z_b of the left element
-      if (eR >= 0) d += ELM(c.ec, eR, i * 26 + 1 + j);       // -A_as Z_a of the right element
-    }
-    CRN(c.cD, k, x) = d;
-  } else if (part == 1) {
-    const int kn = c.corner_next[k];
-    CRN(c.cU, k, x) = kn >= 0 && live_i && (c.corner_mask[kn] >> j & 1)
-                          ? KR[(i + 18 * (12 + j)) * ne] + ELM(c.ec, eR, i * 26 + 7 + j)
-                          : 0.0;
-  } else if (part == 2) {
-    const int kp = c.corner_prev[k];
-    CRN(c.cL, k, x) = kp >= 0 && live_i && (c.corner_mask[kp] >> j & 1)
-                          ? KL[((12 + i) + 18 * j) * ne] + ELM(c.ec, eL, i * 26 + 13 + 1 + j)
-                          : 0.0;
-  } else {
-    const int r = blockIdx.y - 108;
-    const int g = b.gl[(int64_t)node * 6 + r];
-    double v = 0.0;
-    if (g >= 0) {
-      v = b.P[inf.dof_off + g];
-      if (eL >= 0) v += ELM(c.ec, eL, r * 26 + 13);
-      if (eR >= 0) v += ELM(c.ec, eR, r * 26);
-    }
-    CRN(c.cb, k, r) = v;
-  }
-}
-
-// ---- 3. cyclic reduction: eliminate odd positions ----
-__global__ void __launch_bounds__(CT) k_cr_eliminate(Batch b, ChainData c, int lo, int hi) {
-  int t = lo + blockIdx.x * CT + threadIdx.x;
+template <typename Item> __global__ void __launch_bounds__(128) k_gen_w(Batch b, ChainParts c, int lo, int hi) {
+  __shared__ double zs[4][6][13];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lo + blockIdx.x * 4 + warp;
   if (t >= hi) return;
-  CrItem it = c.odd[t];
-  if (!solving(b, it.structure)) return;
-  int k = it.corner;
-  double D[36];
-#pragma unroll
-  for (int q = 0; q < 36; ++q) D[q] = CRN(c.cD, k, q);
-  double inv[6], mult[36];
-  if (!gj6_factor(D, inv, mult)) b.state[it.structure].info_fail = 1;
-  // Z = D^-1 [b | L | U], a column at a time
-#pragma unroll 1
-  for (int q = 0; q < 13; ++q) {
-    double r[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      if (q == 0) r[i] = CRN(c.cb, k, i);
-      else if (q < 7) r[i] = it.prev >= 0 ? CRN(c.cL, k, i * 6 + q - 1) : 0.0;
-      else r[i] = it.next >= 0 ? CRN(c.cU, k, i * 6 + q - 7) : 0.0;
-    }
-    gj6_apply(inv, mult, r);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) CRN(c.cz, k, i * 13 + q) = r[i];
-  }
+  Item I{b, c};
+  I.init(t);
+  const bool ok = gen_item(I, lane, zs[warp]);
+  if (!ok && lane == 0) I.fail();
 }
 
-// Warp-per-item form of k_cr_eliminate for the small levels near the top of
-// the reduction, where one item per thread would leave most of the FP64
-// units idle: lane q holds column q of the augmented 6 x 19 matrix
-// [D | b | L | U] in registers and the pivot column is broadcast by shuffle.
-// The arithmetic is the same sequence as gj6_factor / gj6_apply (same products and
-// FMAs on every entry), so both forms give the same bits.
-__global__ void k_cr_eliminate_w(Batch b, ChainData c, int lo, int hi) {
-  const int lane = threadIdx.x & 31;
-  const int t = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (t >= hi) return;
-  CrItem it = c.odd[t];
-  if (!solving(b, it.structure)) return;
-  const int k = it.corner;
-  double col[6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    double v = 0.0;
-    if (lane < 6) v = CRN(c.cD, k, i * 6 + lane);
-    else if (lane == 6) v = CRN(c.cb, k, i);
-    else if (lane < 13) v = it.prev >= 0 ? CRN(c.cL, k, i * 6 + lane - 7) : 0.0;
-    else if (lane < NC) v = it.next >= 0 ? CRN(c.cU, k, i * 6 + lane - 13) : 0.0;
-    col[i] = v;
-  }
-  bool ok = true;
-#pragma unroll
-  for (int kk = 0; kk < 6; ++kk) {
-    double p = __shfl_sync(0xffffffffu, col[kk], kk);
-    if (!(p != 0.0) || !isfinite(p)) ok = false;
-    double inv = rcp64(p);
-    double m[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) m[i] = __shfl_sync(0xffffffffu, col[i], kk);
-    if (lane > kk && lane < NC) {
-      double rk = col[kk] * inv;
-      col[kk] = rk;
-#pragma unroll
-      for (int i = 0; i < 6; ++i)
-        if (i != kk) col[i] = fma(-m[i], rk, col[i]);
-    }
-  }
-  if (!ok && lane == 0) b.state[it.structure].info_fail = 1;
-  if (lane >= 6 && lane < NC)
-#pragma unroll
-    for (int i = 0; i < 6; ++i) CRN(c.cz, k, i * 13 + lane - 6) = col[i];
-}
+struct GenRoot {
+  const ChainParts& c;
+  int part;
+  __device__ __forceinline__ double k(int i, int j) const { return chain_at(c.part, c.part_soa, CHAIN_GEN_PART, part, i * 12 + j); }
+  __device__ __forceinline__ double f(int i) const { return chain_at(c.part, c.part_soa, CHAIN_GEN_PART, part, GP_F + i); }
+};
 
-// ---- 3b. cyclic reduction: surviving positions absorb their neighbours ----
-// D -= U ZL(next) + L ZU(prev);  b -= U Zb(next) + L Zb(prev);
-// U <- -U ZU(next);  L <- -L ZL(prev)
-__device__ __forceinline__ void cr_update_row(const ChainData& c, const CrItem& it, int i) {
-  const int k = it.corner;
-  const int zn = it.next, zp = it.prev;
-  {
-    double u[6], l[6];
+// Back substitution x = Z_0 - Z_p x_p - Z_n x_n, row i.
+template <typename Kept>
+__device__ __forceinline__ double gen_back(const ChainParts& c, int p, int n, int i, Kept kept) {
+  double z[13], xp[6], xn[6];
 #pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      u[j] = CRN(c.cU, k, i * 6 + j);
-      l[j] = CRN(c.cL, k, i * 6 + j);
-    }
-    double nb = CRN(c.cb, k, i), nD[6], nU[6], nL[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      nD[q] = CRN(c.cD, k, i * 6 + q);
-      nU[q] = 0.0;
-      nL[q] = 0.0;
-    }
-    if (zn >= 0) {
-#pragma unroll
-      for (int j = 0; j < 6; ++j) {
-        nb = fma(-u[j], CRN(c.cz, zn, j * 13), nb);
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-          nD[q] = fma(-u[j], CRN(c.cz, zn, j * 13 + 1 + q), nD[q]);
-          nU[q] = fma(-u[j], CRN(c.cz, zn, j * 13 + 7 + q), nU[q]);
-        }
-      }
-    }
-    if (zp >= 0) {
-#pragma unroll
-      for (int j = 0; j < 6; ++j) {
-        nb = fma(-l[j], CRN(c.cz, zp, j * 13), nb);
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-          nD[q] = fma(-l[j], CRN(c.cz, zp, j * 13 + 7 + q), nD[q]);
-          nL[q] = fma(-l[j], CRN(c.cz, zp, j * 13 + 1 + q), nL[q]);
-        }
-      }
-    }
-    CRN(c.cb, k, i) = nb;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      CRN(c.cD, k, i * 6 + q) = nD[q];
-      CRN(c.cU, k, i * 6 + q) = nU[q];
-      CRN(c.cL, k, i * 6 + q) = nL[q];
-    }
-  }
-}
-
-// Row per lane: six lanes per item (rows of the 6x6 blocks are
-// independent), five items per warp.
-__global__ void k_cr_update_w(Batch b, ChainData c, int lo, int hi) {
-  const int lane = threadIdx.x & 31;
-  if (lane >= 30) return;
-  const int t = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
-  if (t >= hi) return;
-  CrItem it = c.even[t];
-  if (!solving(b, it.structure)) return;
-  cr_update_row(c, it, lane % 6);
-}
-
-// Entry-per-thread form of the same update for the small levels: blockIdx.y is
-// a row and one of its 19 outputs (b, D, U, L), each the same chain of
-// multiply-adds as in cr_update_row.  The outputs go to scratch beside the
-// blocks they are formed from; k_cr_update_e2 puts them in place.
-__global__ void k_cr_update_e(Batch b, ChainData c, int lo, int hi) {
-  const int t = lo + blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= hi) return;
-  const CrItem it = c.even[t];
-  if (!solving(b, it.structure)) return;
-  const int k = it.corner, i = blockIdx.y / 19, o = blockIdx.y % 19, q = (o - 1) % 6, what = o == 0 ? 0 : 1 + (o - 1) / 6;
-  double v = what == 0 ? CRN(c.cb, k, i) : what == 1 ? CRN(c.cD, k, i * 6 + q) : 0.0;
-  if (it.next >= 0 && what != 3) {
-    const int z = what == 0 ? 0 : what == 1 ? 1 + q : 7 + q;
-#pragma unroll
-    for (int j = 0; j < 6; ++j) v = fma(-CRN(c.cU, k, i * 6 + j), CRN(c.cz, it.next, j * 13 + z), v);
-  }
-  if (it.prev >= 0 && what != 2) {
-    const int z = what == 0 ? 0 : what == 1 ? 7 + q : 1 + q;
-#pragma unroll
-    for (int j = 0; j < 6; ++j) v = fma(-CRN(c.cL, k, i * 6 + j), CRN(c.cz, it.prev, j * 13 + z), v);
-  }
-  CRN(c.ce, k, blockIdx.y) = v;
-}
-__global__ void k_cr_update_e2(Batch b, ChainData c, int lo, int hi) {
-  const int t = lo + blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= hi) return;
-  const CrItem it = c.even[t];
-  if (!solving(b, it.structure)) return;
-  const int k = it.corner, i = blockIdx.y / 19, o = blockIdx.y % 19, q = (o - 1) % 6;
-  const double v = CRN(c.ce, k, blockIdx.y);
-  if (o == 0) CRN(c.cb, k, i) = v;
-  else if (o < 7) CRN(c.cD, k, i * 6 + q) = v;
-  else if (o < 13) CRN(c.cU, k, i * 6 + q) = v;
-  else CRN(c.cL, k, i * 6 + q) = v;
-}
-
-// ---- 3c. the last position of each chain ----
-__global__ void __launch_bounds__(CT) k_cr_root(Batch b, ChainData c) {
-  int t = blockIdx.x * CT + threadIdx.x;
-  if (t >= c.n_roots) return;
-  int k = c.roots[t];
-  int s = c.corner_struct[k];
-  if (!solving(b, s)) return;
-  double D[36], r[6];
-#pragma unroll
-  for (int q = 0; q < 36; ++q) D[q] = CRN(c.cD, k, q);
-#pragma unroll
-  for (int i = 0; i < 6; ++i) r[i] = CRN(c.cb, k, i);
-  double inv[6], mult[36];
-  if (!gj6_factor(D, inv, mult)) b.state[s].info_fail = 1;
-  gj6_apply(inv, mult, r);
-#pragma unroll
-  for (int i = 0; i < 6; ++i) CRN(c.cx, k, i) = r[i];
-}
-
-// ---- 4. back substitution: x = Zb - ZL x_prev - ZU x_next ----
-// Row per lane: six lanes per item, five items per warp.
-__global__ void k_cr_back(Batch b, ChainData c, int lo, int hi) {
-  const int lane = threadIdx.x & 31;
-  if (lane >= 30) return;
-  const int t = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
-  if (t >= hi) return;
-  CrItem it = c.odd[t];
-  if (!solving(b, it.structure)) return;
-  const int k = it.corner, i = lane % 6;
-  double x = CRN(c.cz, k, i * 13);
+  for (int j = 0; j < 13; ++j) z[j] = kept(i * 13 + j);
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
-    double xp = it.prev >= 0 ? CRN(c.cx, it.prev, j) : 0.0;
-    double xn = it.next >= 0 ? CRN(c.cx, it.next, j) : 0.0;
-    x = fma(-CRN(c.cz, k, i * 13 + 1 + j), xp, x);
-    x = fma(-CRN(c.cz, k, i * 13 + 7 + j), xn, x);
+    xp[j] = c.x[6 * (int64_t)(p) + j];
+    xn[j] = c.x[6 * (int64_t)(n) + j];
   }
-  CRN(c.cx, k, i) = x;
-}
-
-// ---- 4b. midside nodes, and the solution into P ----
-__global__ void k_chain_scatter(Batch b, ChainData c) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= c.n_chain_elems) return;
-  int e = c.elem_list[t];
-  int s = b.estruct[e];
-  if (!solving(b, s)) return;
-  const StructInfo& inf = b.info[s];
-  double* P = b.P + inf.dof_off;
-  int ka = c.elem_corner_a[t], kb = c.elem_corner_b[t];
-  double xa[6], xb[6];
+  double x = z[0];
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
-    xa[j] = ka >= 0 ? CRN(c.cx, ka, j) : 0.0;
-    xb[j] = kb >= 0 ? CRN(c.cx, kb, j) : 0.0;
+    x = fma(-z[1 + j], xp[j], x);
+    x = fma(-z[7 + j], xn[j], x);
   }
-  int nm = b.enodes[3 * e + 1];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    double x = ELM(c.ez, t, i * 13);
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      x = fma(-ELM(c.ez, t, i * 13 + 1 + j), xa[j], x);
-      x = fma(-ELM(c.ez, t, i * 13 + 7 + j), xb[j], x);
+  return x;
+}
+__device__ __forceinline__ void gen_corner(const Batch& b, const ChainParts& c, int t, const ChainMerge& m, int i) {
+  const double x = gen_back(c, m.p, m.n, i, [&](int q) { return chain_at(c.mz, c.merge_soa, CHAIN_GEN_KEEP, t, q); });
+  c.x[6 * (int64_t)(m.k) + i] = x;
+  if (m.mask >> i & 1) b.P[m.dof + __popc(m.mask & ((1 << i) - 1))] = x;
+}
+// Corners of one level: a row per lane, six lanes per item, five items per warp.
+__global__ void k_gen_back(Batch b, ChainParts c, int lo, int hi) {
+  const int lane = threadIdx.x & 31;
+  const int t = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
+  if (lane >= 30 || t >= hi) return;
+  const ChainMerge m = c.merge[t];
+  if (solving(b, m.structure)) gen_corner(b, c, t, m, lane % 6);
+}
+__global__ void k_gen_mid(Batch b, ChainParts c) {
+  const int lane = threadIdx.x & 31, i = lane % 6;
+  const int t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
+  if (lane >= 30 || t >= c.n_elem || !solving(b, c.elem_struct[t])) return;
+  const int p = c.elem_corner[t];
+  b.P[c.elem_dof[t] + i] = gen_back(c, p, p + 1, i, [&](int q) { return chain_at(c.ez, c.elem_soa, CHAIN_GEN_KEEP, t, q); });
+}
+
+// The last levels of a chain, its root and their back substitution in one CTA, a
+// merge per warp.
+__global__ void __launch_bounds__(256) k_gen_top(Batch b, ChainParts c) {
+  __shared__ double zs[8][6][13];
+  const ChainTop ch = c.chain[blockIdx.x];
+  if (!solving(b, ch.structure)) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int t0 = ch.top;
+  for (int k = ch.n_top; k > 1; t0 += k / 2, k = (k + 1) / 2) {
+    if (warp < k / 2) {
+      GenMerge I{b, c};
+      I.init(t0 + warp);
+      const bool ok = gen_item(I, lane, zs[warp]);
+      if (!ok && lane == 0) I.fail();
     }
-    P[b.gl[(int64_t)nm * 6 + i]] = x;
+    __syncthreads();
+  }
+  if (warp == 0) chain_root(b, c, ch, lane, GenRoot{c, ch.root});
+  __syncthreads();
+  int cnt[5], n = 0;
+  for (int k = ch.n_top; k > 1; k = (k + 1) / 2) cnt[n++] = k / 2;
+  for (int l = n - 1; l >= 0; --l) {
+    t0 -= cnt[l];
+    const int q = warp * 5 + lane / 6;
+    if (lane < 30 && q < cnt[l]) gen_corner(b, c, t0 + q, c.merge[t0 + q], lane % 6);
+    __syncthreads();
   }
 }
 
-__global__ void k_corner_scatter(Batch b, ChainData c) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= c.n_corners) return;
-  int s = c.corner_struct[k];
-  if (!solving(b, s)) return;
-  const StructInfo inf = b.info[s];
-  double* P = b.P + inf.dof_off;
-  int node = c.corner_node[k];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    const int g = b.gl[(int64_t)node * 6 + i];
-    if (g >= 0) P[g] = CRN(c.cx, k, i);
-  }
-}
+dim3 grid_for(int n, int per) { return dim3((n + per - 1) / per); }
 
 }  // namespace
 
-// Items below which the item-per-warp forms are the faster ones: an item per
-// thread takes about 50 us however few there are (its chain of 1,520 operations
-// of 64 cycles), an item per warp 8 us for as many as there are sub-partitions
-// (608), then about 8 ns an item, twice the other's.
-constexpr int SMALL_GENERAL = 152 * 4 * 8;
-// The update's row-per-lane form takes about 10 us below one wave, the
-// entry-per-thread form's two launches 2 us, at three times the loads.
-constexpr int SMALL_UPDATE = 152 * 4 * 4;
-
-static dim3 grid_for(int n, int per, int y = 1) { return dim3((n + per - 1) / per, y); }
-
-void launch_chain_solve(const Batch& b, const ChainData& c, cudaStream_t st) {
-  if (c.n_chain_elems == 0) return;
-  const int ne = c.n_chain_elems;
-  if (ne >= SMALL_GENERAL) k_condense<<<grid_for(ne, CT), CT, 0, st>>>(b, c);
-  else k_condense_w<<<grid_for(ne, 4), 128, 0, st>>>(b, c);
-  if (c.n_corners > 0) {
-    k_corner_system<<<grid_for(c.n_corners, 128, 114), 128, 0, st>>>(b, c);
-    for (int l = 0; l < c.n_levels; ++l) {
-      const int lo = c.odd_off[l], hi = c.odd_off[l + 1];
-      if (hi - lo >= SMALL_GENERAL) k_cr_eliminate<<<grid_for(hi - lo, CT), CT, 0, st>>>(b, c, lo, hi);
-      else if (hi > lo) k_cr_eliminate_w<<<grid_for(hi - lo, 4), 128, 0, st>>>(b, c, lo, hi);
-      // a row of a block per lane, or at the small levels an entry per thread
-      const int elo = c.even_off[l], ehi = c.even_off[l + 1];
-      if (ehi - elo >= SMALL_UPDATE) {
-        k_cr_update_w<<<grid_for(ehi - elo, 20), 128, 0, st>>>(b, c, elo, ehi);
-      } else if (ehi > elo) {
-        k_cr_update_e<<<grid_for(ehi - elo, 32, 114), 32, 0, st>>>(b, c, elo, ehi);
-        k_cr_update_e2<<<grid_for(ehi - elo, 32, 114), 32, 0, st>>>(b, c, elo, ehi);
-      }
-    }
-    k_cr_root<<<grid_for(c.n_roots, CT), CT, 0, st>>>(b, c);
-    for (int l = c.n_levels - 1; l >= 0; --l) {
-      const int lo = c.odd_off[l], hi = c.odd_off[l + 1];
-      if (hi > lo) k_cr_back<<<grid_for(hi - lo, 20), 128, 0, st>>>(b, c, lo, hi);
-    }
+void launch_gen_chains(const Batch& b, const ChainParts& c, cudaStream_t st) {
+  if (c.n_elem == 0) return;
+  if (c.elem_soa) k_gen<GenCondense><<<grid_for(c.n_elem, CT), CT, GEN_SMEM, st>>>(b, c, 0, c.n_elem);
+  else k_gen_w<GenCondense><<<grid_for(c.n_elem, 4), 128, 0, st>>>(b, c, 0, c.n_elem);
+  for (int l = 0; l < c.n_levels; ++l) {
+    const int lo = c.merge_off[l], hi = c.merge_off[l + 1];
+    if (hi <= c.merge_soa) k_gen<GenMerge><<<grid_for(hi - lo, CT), CT, GEN_SMEM, st>>>(b, c, lo, hi);
+    else k_gen_w<GenMerge><<<grid_for(hi - lo, 4), 128, 0, st>>>(b, c, lo, hi);
   }
-  if (c.n_corners > 0) k_corner_scatter<<<grid_for(c.n_corners, 128), 128, 0, st>>>(b, c);
-  k_chain_scatter<<<grid_for(ne, 128), 128, 0, st>>>(b, c);
-}
-
-// Kernel launches of one chain solve.
-int chain_launches(const ChainData& c) {
-  if (!c.n_chain_elems) return 0;
-  int n = 2;
-  if (c.n_corners) {
-    n += 3;
-    for (int l = 0; l < c.n_levels; ++l) {
-      const int odd = c.odd_off[l + 1] - c.odd_off[l], even = c.even_off[l + 1] - c.even_off[l];
-      n += 2 * (odd > 0) + (even > 0) + (even > 0 && even < SMALL_UPDATE);
-    }
+  k_gen_top<<<c.n_chains, 256, 0, st>>>(b, c);
+  for (int l = c.n_levels - 1; l >= 0; --l) {
+    const int lo = c.merge_off[l], hi = c.merge_off[l + 1];
+    k_gen_back<<<grid_for(hi - lo, 20), 128, 0, st>>>(b, c, lo, hi);
   }
-  return n;
+  k_gen_mid<<<grid_for(c.n_elem, 20), 128, 0, st>>>(b, c);
 }
 
 }  // namespace gf

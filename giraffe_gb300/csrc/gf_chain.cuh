@@ -1,29 +1,23 @@
 // Direct solver for K_AA of Beam_1 chains (elements e = 0..m-1 on nodes
 // 2e, 2e+1, 2e+2; node-major DOF numbering), FP64, no pivoting.
 //
-// K_AA of such a chain is block-tridiagonal over the corner nodes once the
-// midside nodes are condensed: a midside node couples only to the two corner
-// nodes of its element.  The solve therefore runs as
-//   1. condensation   per element: Z_s = A_ss^{-1} [b_s | A_sa | A_sb] and the
-//                     Schur contributions to the two corners (parallel over
-//                     all elements of all chains);
-//   2. corner system  D_k, L_k (coupling to the previous corner), U_k (to the
-//                     next) and b_k per free corner;
-//   3. cyclic reduction over corner positions, one level per launch: odd
-//                     positions are eliminated (Z = D^{-1} [b | L | U]),
-//                     even positions absorb them; the last survivor is
-//                     solved directly;
-//   4. back substitution level by level, then the midside nodes.
-// Corners may have fixed DOFs (a pinned end): their rows and columns are those
-// of the identity.
-// The critical path is O(log m) small dense solves instead of the O(n)
-// column recurrence of a banded LU, which on a GPU with slow FP64 latency
-// (~64 cycles per dependent FP64 operation) dominates long chains.  The
-// solver never reads an assembled K_AA: it takes each element's tangent K_e
-// from the element scratch (plus the nodal load stiffness), which is the
-// same K_AA term by term.  Equations follow from block
-// Gaussian elimination on the assembled matrix; the reference solves the
-// same K_AA with PARDISO (reference src/SparseMatrix.cpp:74-166).
+// A midside node couples only to the two corner nodes of its element, so the
+// solve eliminates
+//   1. the midside node of every element (condensation): the element becomes a
+//      "part", a stiffness between two corners and the forces it leaves on them;
+//   2. corners, by merging pairs of neighbouring parts level by level, the last
+//      levels of a chain in one CTA;
+//   3. the last part with the chain's end nodes;
+// and substitutes back in reverse.  The critical path is O(log m) small dense
+// solves instead of the O(n) column recurrence of a banded LU, which on a GPU
+// with slow FP64 latency (~64 cycles per dependent FP64 operation) dominates
+// long chains.  The solver never reads an assembled K_AA: it takes each
+// element's tangent K_e from the element scratch (plus the nodal load
+// stiffness), which is the same K_AA term by term.  Corners may have fixed DOFs
+// (a pinned end): their rows and columns are those of the identity.  Equations
+// follow from block Gaussian elimination on the assembled matrix; the
+// reference solves the same K_AA with PARDISO (reference
+// src/SparseMatrix.cpp:74-166).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -31,10 +25,20 @@
 
 namespace gf {
 
-void launch_chain_solve(const Batch& b, const ChainData& c, cudaStream_t st);
-int chain_launches(const ChainData& c);
-// The chains with a symmetric K_AA (gf_chain_sym.cu).
-void launch_sym_chains(const Batch& b, const SymChains& c, cudaStream_t st);
-int sym_chain_launches(const SymChains& c);
+// Doubles per part and per kept elimination of the two kinds.
+constexpr int CHAIN_SYM_PART = 57, CHAIN_SYM_KEEP = 81, CHAIN_GEN_PART = 156, CHAIN_GEN_KEEP = 78;
+
+// Items below which an item per warp (half warp) is the faster form.  General: it
+// takes about 8 us for as many as there are sub-partitions (608), then 6 ns an
+// item, an item per thread about 55 us however few there are (its chain of 1,550
+// operations of 64 cycles), then half of that per item.  Symmetric: 4 us for
+// 1,216, then 3 ns, against 35 us.
+constexpr int CHAIN_GEN_SMALL = 152 * 4 * 16, CHAIN_SYM_SMALL = 152 * 4 * 20;
+
+// The chains of b.chain_gen (gf_chain.cu) and of b.chain_sym (gf_chain_sym.cu).
+void launch_gen_chains(const Batch& b, const ChainParts& c, cudaStream_t st);
+void launch_sym_chains(const Batch& b, const ChainParts& c, cudaStream_t st);
+// Kernel launches of one solve.
+inline int chain_launches(const ChainParts& c) { return c.n_elem ? 3 + 2 * c.n_levels : 0; }
 
 }  // namespace gf

@@ -26,6 +26,7 @@
 
 #include "gf_beam_gp.cuh"
 #include "gf_chain.cuh"
+#include "gf_chain_root.cuh"
 #include "gf_math.cuh"
 
 namespace gf {
@@ -33,21 +34,17 @@ namespace gf {
 namespace {
 
 constexpr int CT = 64;
-#define AT(arr, n, i, x) (arr)[(int64_t)(x) * (n) + (i)]
-
-__device__ __forceinline__ bool solving(const Batch& b, int s) {
-  const StructState& st = b.state[s];
-  return st.phase == PH_ITER && st.need_solve;
-}
 
 __device__ __forceinline__ constexpr int lo6(int i, int j) { return i * (i + 1) / 2 + j; }
 
 // Part: lower triangle over (du 0-2, a_p 3-5, a_n 6-8), then the forces on p and
 // n (translation, rotation each).
-constexpr int PT_HP = 45, PT_HN = 51, PT_COUNT = 57;
+constexpr int PT_HP = 45, PT_HN = 51;
+static_assert(PT_HN + 6 == CHAIN_SYM_PART, "a part's entries");
 // Kept of an elimination: W = L^-1 R ([row * 10 + column]), the entries of L E below
 // the diagonal, the reciprocals of E.
-constexpr int KP_M = 60, KP_R = 75, KP_COUNT = 81;
+constexpr int KP_M = 60, KP_R = 75;
+static_assert(KP_R + 6 == CHAIN_SYM_KEEP, "an elimination's kept entries");
 // Outputs: the 45 entries of the new stiffness, then the 9 forces h over (du,
 // a_p, a_n).
 constexpr int N_OUT = 54;
@@ -183,7 +180,7 @@ __device__ __forceinline__ bool eliminate_h(const Item& I, int lane, unsigned la
 // such an element over (du, v, a_0, a_1, a_2), lower triangle (beam_expand_sym).
 struct Condense {
   const Batch& b;
-  const SymChains& c;
+  const ChainParts& c;
   int t, s;
   const double *K, *P;
   int64_t ne;
@@ -205,8 +202,8 @@ struct Condense {
   __device__ __forceinline__ double force(int i) const { return P[i]; }
   __device__ __forceinline__ double r(int i, int q) const { return q == 0 ? force(i) : k15(row(i), place(q)); }
   __device__ __forceinline__ double base(int o, int p, int q) const { return o >= 45 ? 0.0 : k15(place(q), place(p)); }
-  __device__ __forceinline__ void keep(int x, double v) const { AT(c.ez, c.n_elem, t, x) = v; }
-  __device__ __forceinline__ void put(int x, double v) const { AT(c.part, c.n_part, t, x) = v; }
+  __device__ __forceinline__ void keep(int x, double v) const { chain_at(c.ez, c.elem_soa, CHAIN_SYM_KEEP, t, x) = v; }
+  __device__ __forceinline__ void put(int x, double v) const { chain_at(c.part, c.part_soa, CHAIN_SYM_PART, t, x) = v; }
   __device__ __forceinline__ void out(int o, double h) const {
     if (o < 45) {
       put(o, h);
@@ -226,8 +223,8 @@ struct Condense {
 // Elimination of corner k between parts e1 and e2.
 struct Merge {
   const Batch& b;
-  const SymChains& c;
-  SymMerge m;
+  const ChainParts& c;
+  ChainMerge m;
   int t;
   __device__ __forceinline__ void init(int t_) {
     t = t_;
@@ -235,7 +232,7 @@ struct Merge {
   }
   __device__ __forceinline__ bool active() const { return solving(b, m.structure); }
   __device__ __forceinline__ double E(int e, int i, int j) const {
-    return AT(c.part, c.n_part, e, i >= j ? lo6(i, j) : lo6(j, i));
+    return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, e, i >= j ? lo6(i, j) : lo6(j, i));
   }
   __device__ __forceinline__ double d(int i, int j) const {  // j <= i, unknowns (w, a_k)
     if (i < 3) return radd(E(m.e1, i, j), E(m.e2, i, j));
@@ -244,7 +241,7 @@ struct Merge {
   }
   // the corner's own force with what both parts leave on it
   __device__ __forceinline__ double force(int i) const {
-    return radd(radd(b.P[m.dof + i], AT(c.part, c.n_part, m.e1, PT_HN + i)), AT(c.part, c.n_part, m.e2, PT_HP + i));
+    return radd(radd(b.P[m.dof + i], chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e1, PT_HN + i)), chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e2, PT_HP + i));
   }
   __device__ __forceinline__ double r(int i, int q) const {
     if (q == 0) return force(i);
@@ -259,25 +256,25 @@ struct Merge {
     if (i < 6) return j < 3 ? 0.0 : E(m.e1, i, j);
     return j >= 3 && j < 6 ? 0.0 : E(m.e2, i, j);
   }
-  __device__ __forceinline__ void keep(int x, double v) const { AT(c.mz, c.n_merge, t, x) = v; }
-  __device__ __forceinline__ void put(int x, double v) const { AT(c.part, c.n_part, m.out, x) = v; }
+  __device__ __forceinline__ void keep(int x, double v) const { chain_at(c.mz, c.merge_soa, CHAIN_SYM_KEEP, t, x) = v; }
+  __device__ __forceinline__ void put(int x, double v) const { chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.out, x) = v; }
   __device__ __forceinline__ void out(int o, double h) const {
     if (o < 45) {
       put(o, h);
     } else if (o < 48) {  // u_k = u_p + w: the corner's force passes to p
       const int i = o - 45;
-      put(PT_HP + i, radd(AT(c.part, c.n_part, m.e1, PT_HP + i), rsub(force(i), h)));
-      put(PT_HN + i, radd(AT(c.part, c.n_part, m.e2, PT_HN + i), h));
+      put(PT_HP + i, radd(chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e1, PT_HP + i), rsub(force(i), h)));
+      put(PT_HN + i, radd(chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e2, PT_HN + i), h));
     } else if (o < 51) {
-      put(PT_HP + o - 45, radd(AT(c.part, c.n_part, m.e1, PT_HP + o - 45), h));
+      put(PT_HP + o - 45, radd(chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e1, PT_HP + o - 45), h));
     } else {
-      put(PT_HN + o - 48, radd(AT(c.part, c.n_part, m.e2, PT_HN + o - 48), h));
+      put(PT_HN + o - 48, radd(chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e2, PT_HN + o - 48), h));
     }
   }
   __device__ void fail() const { b.state[m.structure].info_fail = 1; }
 };
 
-template <typename Item> __global__ void __launch_bounds__(CT) k_sym(Batch b, SymChains c, int lo, int hi) {
+template <typename Item> __global__ void __launch_bounds__(CT) k_sym(Batch b, ChainParts c, int lo, int hi) {
   const int t = lo + blockIdx.x * CT + threadIdx.x;
   if (t >= hi) return;
   Item I{b, c};
@@ -285,7 +282,7 @@ template <typename Item> __global__ void __launch_bounds__(CT) k_sym(Batch b, Sy
   if (!I.active()) return;
   if (!eliminate(I)) I.fail();
 }
-template <typename Item> __global__ void __launch_bounds__(128) k_sym_h(Batch b, SymChains c, int lo, int hi) {
+template <typename Item> __global__ void __launch_bounds__(128) k_sym_h(Batch b, ChainParts c, int lo, int hi) {
   __shared__ double ws[8][2][10][6];
   const int half = threadIdx.x >> 4, lane = threadIdx.x & 15, t = lo + blockIdx.x * 8 + half;
   const unsigned lanes = 0xFFFFu << (threadIdx.x & 16);
@@ -296,67 +293,17 @@ template <typename Item> __global__ void __launch_bounds__(128) k_sym_h(Batch b,
   if (!ok && lane == 0) I.fail();
 }
 
-// The last part of a chain with its end nodes, by one warp: 12 unknowns (u_p, a_p, u_n,
-// a_n), lane j column j of the matrix, lane 12 the right-hand side; fixed DOFs
-// are identity rows and columns, their pivots skipped.
-__device__ void root(const Batch& b, const SymChains& c, const SymChain& ch, int lane) {
-  const int part = ch.root, s = ch.structure;
-  const int node[2] = {c.corner_node[ch.first], c.corner_node[ch.last]};
-  const int g = lane < 12 ? b.gl[(int64_t)node[lane / 6] * 6 + lane % 6] : -1;
-  const unsigned live = __ballot_sync(0xffffffffu, g >= 0);
-  double* P = b.P + b.info[s].dof_off;
-  // place of unknown x among (du, a_p, a_n), and the sign of u_p in du
-  auto place = [](int x) { return x < 3 ? x : x < 6 ? x : x < 9 ? x - 6 : x - 3; };
-  double col[12];
-#pragma unroll
-  for (int i = 0; i < 12; ++i) {
-    double v = 0.0;
-    if (lane < 12) {
-      if ((live >> i & 1) && (live >> lane & 1)) {
-        const int x = place(i), y = place(lane);
-        v = AT(c.part, c.n_part, part, x >= y ? lo6(x, y) : lo6(y, x));
-        if ((i < 3) != (lane < 3)) v = -v;
-        if (i % 6 >= 3 && lane % 6 >= 3 && i / 6 == lane / 6)
-          v = radd(v, b.nodeK[(int64_t)node[i / 6] * 9 + (i % 6 - 3) * 3 + lane % 6 - 3]);
-      } else {
-        v = i == lane ? 1.0 : 0.0;
-      }
-    } else if (lane == 12 && (live >> i & 1)) {
-      v = radd(P[b.gl[(int64_t)node[i / 6] * 6 + i % 6]],
-               AT(c.part, c.n_part, part, (i < 6 ? PT_HP : PT_HN) + i % 6));
-    }
-    col[i] = v;
+// The last part as a 12x12 matrix: the sign of u_p in du.
+struct SymRoot {
+  const ChainParts& c;
+  int part;
+  __device__ __forceinline__ double k(int i, int j) const {
+    const int x = i < 6 ? i : i < 9 ? i - 6 : i - 3, y = j < 6 ? j : j < 9 ? j - 6 : j - 3;
+    const double v = chain_at(c.part, c.part_soa, CHAIN_SYM_PART, part, x >= y ? lo6(x, y) : lo6(y, x));
+    return (i < 3) != (j < 3) ? -v : v;
   }
-  bool ok = true;
-#pragma unroll
-  for (int k = 0; k < 12; ++k) {
-    if (!(live >> k & 1)) continue;
-    const double p = __shfl_sync(0xffffffffu, col[k], k);
-    if (!(p != 0.0) || !isfinite(p)) ok = false;
-    const double inv = rcp64(p);
-    double m[12];
-#pragma unroll
-    for (int i = 0; i < 12; ++i) m[i] = __shfl_sync(0xffffffffu, col[i], k);
-    if (lane > k && lane < 13) {
-      const double rk = rmul(col[k], inv);
-      col[k] = rk;
-#pragma unroll
-      for (int i = 0; i < 12; ++i)
-        if (i != k) col[i] = rfma(-m[i], rk, col[i]);
-    }
-  }
-  if (!ok && lane == 0) b.state[s].info_fail = 1;
-  double x = 0.0;
-#pragma unroll
-  for (int i = 0; i < 12; ++i) {
-    const double v = __shfl_sync(0xffffffffu, col[i], 12);
-    if (lane == i) x = v;
-  }
-  if (lane < 12) {
-    AT(c.x, c.n_corner, lane < 6 ? ch.first : ch.last, lane % 6) = g >= 0 ? x : 0.0;
-    if (g >= 0) P[g] = x;
-  }
-}
+  __device__ __forceinline__ double f(int i) const { return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, part, PT_HP + i); }
+};
 
 // Back substitution of one elimination: E x = L^-1-reduced right-hand side, i.e.
 // y = W_0 - W_du du - W_p a_p - W_n a_n, then x_k = y_k / E_k and y_i -= (L E)_ki x_k
@@ -379,30 +326,30 @@ __device__ __forceinline__ double back(unsigned lanes, int l0, int i, const doub
   }
   return rmul(y, r);
 }
-__device__ __forceinline__ void around(const SymChains& c, int p, int n, double (&z)[9]) {
+__device__ __forceinline__ void around(const ChainParts& c, int p, int n, double (&z)[9]) {
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
-    z[j] = rsub(AT(c.x, c.n_corner, n, j), AT(c.x, c.n_corner, p, j));
-    z[3 + j] = AT(c.x, c.n_corner, p, 3 + j);
-    z[6 + j] = AT(c.x, c.n_corner, n, 3 + j);
+    z[j] = rsub(c.x[6 * (int64_t)(n) + j], c.x[6 * (int64_t)(p) + j]);
+    z[3 + j] = c.x[6 * (int64_t)(p) + 3 + j];
+    z[6 + j] = c.x[6 * (int64_t)(n) + 3 + j];
   }
 }
 // Corner of merge t, row i.
-__device__ __forceinline__ void back_corner(const Batch& b, const SymChains& c, int t, const SymMerge& m, unsigned lanes,
+__device__ __forceinline__ void back_corner(const Batch& b, const ChainParts& c, int t, const ChainMerge& m, unsigned lanes,
                                             int l0, int i) {
   double z[9];
   around(c, m.p, m.n, z);
-  double x = back(lanes, l0, i, z, [&](int q) { return AT(c.mz, c.n_merge, t, q); });
-  if (i < 3) x = radd(x, AT(c.x, c.n_corner, m.p, i));  // u_k = u_p + w
-  AT(c.x, c.n_corner, m.k, i) = x;
+  double x = back(lanes, l0, i, z, [&](int q) { return chain_at(c.mz, c.merge_soa, CHAIN_SYM_KEEP, t, q); });
+  if (i < 3) x = radd(x, c.x[6 * (int64_t)(m.p) + i]);  // u_k = u_p + w
+  c.x[6 * (int64_t)(m.k) + i] = x;
   b.P[m.dof + i] = x;
 }
 // Corners of one level, five per warp.
-__global__ void k_sym_back(Batch b, SymChains c, int lo, int hi) {
+__global__ void k_sym_back(Batch b, ChainParts c, int lo, int hi) {
   const int lane = threadIdx.x & 31, i = lane % 6;
   const int t = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
   bool on = lane < 30 && t < hi;
-  SymMerge m{};
+  ChainMerge m{};
   if (on) {
     m = c.merge[t];
     on = solving(b, m.structure);
@@ -411,7 +358,7 @@ __global__ void k_sym_back(Batch b, SymChains c, int lo, int hi) {
   if (on) back_corner(b, c, t, m, lanes, lane - i, i);
 }
 // Midside nodes.
-__global__ void k_sym_mid(Batch b, SymChains c) {
+__global__ void k_sym_mid(Batch b, ChainParts c) {
   const int lane = threadIdx.x & 31, i = lane % 6;
   const int t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
   const bool on = lane < 30 && t < c.n_elem && solving(b, c.elem_struct[t]);
@@ -420,18 +367,18 @@ __global__ void k_sym_mid(Batch b, SymChains c) {
   const int p = c.elem_corner[t];
   double z[9];
   around(c, p, p + 1, z);
-  double x = back(lanes, lane - i, i, z, [&](int q) { return AT(c.ez, c.n_elem, t, q); });
-  if (i < 3) x = rfma(0.5, radd(AT(c.x, c.n_corner, p, i), AT(c.x, c.n_corner, p + 1, i)), x);
+  double x = back(lanes, lane - i, i, z, [&](int q) { return chain_at(c.ez, c.elem_soa, CHAIN_SYM_KEEP, t, q); });
+  if (i < 3) x = rfma(0.5, radd(c.x[6 * (int64_t)(p) + i], c.x[6 * (int64_t)(p + 1) + i]), x);
   b.P[c.elem_dof[t] + i] = x;
 }
 
-// The last levels of a chain in one CTA, from at most SYM_TOP parts on: its
+// The last levels of a chain in one CTA, from at most CHAIN_TOP parts on: its
 // merges level by level (a half warp each), the root, and their back
 // substitution.  Against a launch per level this drops the launches and the
 // round trips through L2 between levels of a few items.
-__global__ void __launch_bounds__(128) k_sym_top(Batch b, SymChains c) {
+__global__ void __launch_bounds__(128) k_sym_top(Batch b, ChainParts c) {
   __shared__ double ws[8][2][10][6];
-  const SymChain ch = c.chain[blockIdx.x];
+  const ChainTop ch = c.chain[blockIdx.x];
   if (!solving(b, ch.structure)) return;
   const int half = threadIdx.x >> 4, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lanes = 0xFFFFu << (threadIdx.x & 16);
@@ -445,7 +392,7 @@ __global__ void __launch_bounds__(128) k_sym_top(Batch b, SymChains c) {
     }
     __syncthreads();
   }
-  if (warp == 0) root(b, c, ch, lane);
+  if (warp == 0) chain_root(b, c, ch, lane, SymRoot{c, ch.root});
   __syncthreads();
   // the levels again from the last: their merges end at t0
   int cnt[5], n = 0;
@@ -462,21 +409,15 @@ __global__ void __launch_bounds__(128) k_sym_top(Batch b, SymChains c) {
 
 dim3 grid_for(int n, int per) { return dim3((n + per - 1) / per); }
 
-// Items below which an item per half warp is the faster form: it takes about 4
-// us for as many as there are half sub-partitions (1,216), then 3 ns an item;
-// an item per thread takes about 35 us however few there are, then half of that
-// per item.
-constexpr int SMALL = 152 * 4 * 20;
-
 }  // namespace
 
-void launch_sym_chains(const Batch& b, const SymChains& c, cudaStream_t st) {
+void launch_sym_chains(const Batch& b, const ChainParts& c, cudaStream_t st) {
   if (c.n_elem == 0) return;
-  if (c.n_elem >= SMALL) k_sym<Condense><<<grid_for(c.n_elem, CT), CT, 0, st>>>(b, c, 0, c.n_elem);
+  if (c.elem_soa) k_sym<Condense><<<grid_for(c.n_elem, CT), CT, 0, st>>>(b, c, 0, c.n_elem);
   else k_sym_h<Condense><<<grid_for(c.n_elem, 8), 128, 0, st>>>(b, c, 0, c.n_elem);
   for (int l = 0; l < c.n_levels; ++l) {
     const int lo = c.merge_off[l], hi = c.merge_off[l + 1];
-    if (hi - lo >= SMALL) k_sym<Merge><<<grid_for(hi - lo, CT), CT, 0, st>>>(b, c, lo, hi);
+    if (hi <= c.merge_soa) k_sym<Merge><<<grid_for(hi - lo, CT), CT, 0, st>>>(b, c, lo, hi);
     else k_sym_h<Merge><<<grid_for(hi - lo, 8), 128, 0, st>>>(b, c, lo, hi);
   }
   k_sym_top<<<c.n_chains, 128, 0, st>>>(b, c);
@@ -486,8 +427,5 @@ void launch_sym_chains(const Batch& b, const SymChains& c, cudaStream_t st) {
   }
   k_sym_mid<<<grid_for(c.n_elem, 20), 128, 0, st>>>(b, c);
 }
-
-// Kernel launches of one solve.
-int sym_chain_launches(const SymChains& c) { return c.n_elem ? 3 + 2 * c.n_levels : 0; }
 
 }  // namespace gf

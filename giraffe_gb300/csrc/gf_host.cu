@@ -655,6 +655,108 @@ template <typename T> bool zeroed(gf_batch* B, T** p, size_t n) {
   return true;
 }
 
+// Chain solver tables of the batch's symmetric or general chains: parts of level
+// 0 are the elements; each level merges neighbours in pairs, an odd last part
+// passing up unchanged.  Sizes and offsets per structure first (serial), then the
+// tables of each structure in parallel.
+bool build_parts(gf_batch* B, const gf_model_desc* models, const std::vector<StructPlan>& plan, size_t work, bool sym,
+                 ChainParts& cp) {
+  constexpr int NL = CHAIN_MAX_LEVELS;
+  const int n = (int)plan.size();
+  std::vector<int> sbase(n, 0), cbase(n, 0), mcnt(NL, 0), mpos((size_t)n * NL, 0), tpos(n, 0), chains;
+  int n_top = 0;
+  for (int s = 0; s < n; ++s) {
+    if (!plan[s].chain || (B->info[s].sym != 0) != sym) continue;
+    const int mm = B->info[s].n_elem;
+    sbase[s] = cp.n_elem;
+    cbase[s] = cp.n_corner;
+    cp.n_elem += mm;
+    cp.n_corner += mm + 1;
+    chains.push_back(s);
+    int l = 0, k = mm;
+    for (; k > CHAIN_TOP; ++l, k = (k + 1) / 2) {
+      if (l >= NL) return set_err(B->ctx, "chain too long for %d elimination levels", NL);
+      mpos[(size_t)s * NL + l] = mcnt[l];
+      mcnt[l] += k / 2;
+      cp.n_levels = std::max(cp.n_levels, l + 1);
+    }
+    tpos[s] = n_top;
+    n_top += k - 1;
+  }
+  for (int l = 0; l < NL; ++l) cp.merge_off[l + 1] = cp.merge_off[l] + mcnt[l];
+  cp.n_merge = cp.merge_off[NL] + n_top;
+  cp.n_part = cp.n_elem + cp.n_merge;
+  cp.n_chains = (int)chains.size();
+  if (!cp.n_elem) return true;
+  // the levels taken an item per thread: the largest ones, so the first
+  const int small = sym ? CHAIN_SYM_SMALL : CHAIN_GEN_SMALL;
+  if (cp.n_elem >= small) {
+    cp.elem_soa = cp.n_elem;
+    int l = 0;
+    while (l < cp.n_levels && mcnt[l] >= small) ++l;
+    cp.merge_soa = cp.merge_off[l];
+    cp.part_soa = cp.n_elem + cp.merge_soa;
+  }
+  hvec<int> elem(cp.n_elem), estr(cp.n_elem), edof(cp.n_elem), ecorner(cp.n_elem), emask(cp.n_elem), cnode(cp.n_corner);
+  hvec<ChainMerge> merge(cp.n_merge);
+  hvec<ChainTop> top(cp.n_chains);
+  parallel_structures(cp.n_chains, work, [&](int c) {
+    const int s = chains[c];
+    const StructInfo& inf = B->info[s];
+    const std::vector<int>& g6 = plan[s].g6;
+    const int mm = inf.n_elem, b0 = sbase[s], c0 = cbase[s];
+    auto mask6 = [&](int node) {
+      int k = 0;
+      for (int q = 0; q < 6; ++q) k |= (g6[6 * (size_t)node + q] >= 0) << q;
+      return k;
+    };
+    auto first_dof = [&](int node) {
+      for (int q = 0; q < 6; ++q)
+        if (g6[6 * (size_t)node + q] >= 0) return inf.dof_off + g6[6 * (size_t)node + q];
+      return inf.dof_off;
+    };
+    std::vector<int> id(mm), end(mm);  // part, its last corner
+    for (int e = 0; e < mm; ++e) {
+      elem[b0 + e] = inf.elem_off + e;
+      estr[b0 + e] = s;
+      edof[b0 + e] = first_dof(2 * e + 1);
+      ecorner[b0 + e] = c0 + e;
+      emask[b0 + e] = mask6(2 * e) | mask6(2 * e + 2) << 6;
+      id[e] = b0 + e;
+      end[e] = c0 + e + 1;
+    }
+    for (int k = 0; k <= mm; ++k) cnode[c0 + k] = inf.node_off + 2 * k;
+    ChainTop& ch = top[c];
+    ch = ChainTop{0, cp.merge_off[NL] + tpos[s], 0, c0, c0 + mm, s};
+    int last = ch.top;
+    for (int l = 0, k = mm; k > 1; ++l, k = (k + 1) / 2) {
+      if (k <= CHAIN_TOP && !ch.n_top) ch.n_top = k;
+      int at = k > CHAIN_TOP ? cp.merge_off[l] + mpos[(size_t)s * NL + l] : last, first = c0;
+      for (int q = 0; q < k / 2; ++q, ++at) {
+        const int mid = end[2 * q], node = 2 * (mid - c0);
+        merge[at] = ChainMerge{id[2 * q], id[2 * q + 1], cp.n_elem + at, first, mid, end[2 * q + 1], s, first_dof(node),
+                               mask6(node)};
+        first = end[2 * q + 1];
+        id[q] = cp.n_elem + at;
+        end[q] = first;
+      }
+      if (k <= CHAIN_TOP) last = at;
+      if (k % 2) {
+        id[k / 2] = id[k - 1];
+        end[k / 2] = end[k - 1];
+      }
+    }
+    if (!ch.n_top) ch.n_top = 1;
+    ch.root = id[0];
+  });
+  const size_t np = sym ? CHAIN_SYM_PART : CHAIN_GEN_PART, nk = sym ? CHAIN_SYM_KEEP : CHAIN_GEN_KEEP;
+  return upload(B, &cp.elem, elem) && upload(B, &cp.elem_struct, estr) && upload(B, &cp.elem_dof, edof) &&
+         upload(B, &cp.elem_corner, ecorner) && upload(B, &cp.elem_mask, emask) && upload(B, &cp.corner_node, cnode) &&
+         upload(B, &cp.merge, merge) && upload(B, &cp.chain, top) && balloc(B, &cp.part, cp.n_part * np) &&
+         balloc(B, &cp.ez, cp.n_elem * nk) && balloc(B, &cp.mz, std::max(cp.n_merge, 1) * nk) &&
+         balloc(B, &cp.x, (size_t)cp.n_corner * 6);
+}
+
 int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
   gf_ctx* ctx = B->ctx;
   Batch& b = B->b;
@@ -1031,199 +1133,9 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
   b.mon_cap = b.mon_total ? B->opts.monitor_rows : 0;
   b.n_disps = (int)disps.size();
   b.n_tables = (int)tables.size();
-  // chain solver data: sizes and offsets per structure (serial), then the
-  // tables of each structure filled in parallel
-  {
-    ChainData& cd = b.chain;
-    const int NL = CR_MAX_LEVELS;
-    std::vector<int> Mc(n, 0), tb(n, 0), cb(n, 0), rpos(n, -1);
-    std::vector<int> opos((size_t)n * NL, 0), epos((size_t)n * NL, 0);
-    std::vector<int> ocnt(NL, 0), ecnt(NL, 0);
-    int n_t = 0, n_c = 0, n_levels = 0, n_roots = 0;
-    for (int s = 0; s < n; ++s) {
-      if (!plan[s].chain || B->info[s].sym) continue;
-      const int mm = B->info[s].n_elem;
-      const std::vector<char>& fr = plan[s].node_free;
-      int M = 0;
-      for (int ci = 0; ci <= mm; ++ci) M += fr[2 * ci] != 0;
-      Mc[s] = M;
-      tb[s] = n_t;
-      cb[s] = n_c;
-      n_t += mm;
-      n_c += M;
-      if (M >= 1) rpos[s] = n_roots++;
-      int l = 0;
-      for (int h = 1; h < M; h *= 2, ++l) {
-        if (l >= NL) { set_err(ctx, "chain too long for %d reduction levels", NL); return GF_ERR_ARG; }
-        // odd items kp = h, 3h, 5h, ... < M; even items kp = 0, 2h, 4h, ... < M
-        opos[(size_t)s * NL + l] = ocnt[l];
-        ocnt[l] += (M - h - 1) / (2 * h) + 1;
-        epos[(size_t)s * NL + l] = ecnt[l];
-        ecnt[l] += (M + 2 * h - 1) / (2 * h);
-      }
-      n_levels = std::max(n_levels, l);
-    }
-    for (int l = 0, o = 0, e = 0; l <= NL; ++l) {
-      cd.odd_off[l] = o;
-      cd.even_off[l] = e;
-      if (l < NL) { o += ocnt[l]; e += ecnt[l]; }
-    }
-    hvec<int> elem_list(n_t), eca(n_t), ecb(n_t), cnode(n_c), cstruct(n_c), cleft(n_c), cright(n_c), cprev(n_c),
-        cnext(n_c), roots(n_roots), emask(n_t), cmask(n_c);
-    hvec<CrItem> odd(cd.odd_off[NL]), even(cd.even_off[NL]);
-    parallel_structures(n, work, [&](int s) {
-      if (!plan[s].chain || B->info[s].sym) return;
-      const StructInfo& inf = B->info[s];
-      const int mm = inf.n_elem, M = Mc[s], cbase = cb[s], tbase = tb[s];
-      const std::vector<char>& fr = plan[s].node_free;
-      // corner slots: the chain's corners in the order of cyclic reduction,
-      // position 0, then the odd multiples of the largest power of two below
-      // M, ..., then the odd positions; at every level the items eliminated
-      // (the odd multiples of 2^l) are one contiguous run and the surviving
-      // ones the run before it, so a level's loads are contiguous in the
-      // structure-of-arrays scratch
-      std::vector<int> slot(std::max(M, 1));
-      {
-        int r = 0;
-        if (M > 0) slot[0] = r++;
-        int hmax = 1;
-        while (hmax * 2 < M) hmax *= 2;
-        for (int h = hmax; h >= 1 && M > 1; h /= 2)
-          for (int kp = h; kp < M; kp += 2 * h) slot[kp] = r++;
-      }
-      auto mask6 = [&](int node) {
-        int k = 0;
-        for (int q = 0; q < 6; ++q) k |= (plan[s].g6[6 * node + q] >= 0) << q;
-        return k;
-      };
-      std::vector<int> pos(mm + 1, -1);
-      for (int ci = 0, k = 0; ci <= mm; ++ci)
-        if (fr[2 * ci]) pos[ci] = slot[k++];
-      for (int e = 0; e < mm; ++e) {
-        elem_list[tbase + e] = inf.elem_off + e;
-        eca[tbase + e] = pos[e] >= 0 ? cbase + pos[e] : -1;
-        ecb[tbase + e] = pos[e + 1] >= 0 ? cbase + pos[e + 1] : -1;
-        emask[tbase + e] = mask6(2 * e) | mask6(2 * e + 2) << 6;
-      }
-      for (int ci = 0, k = 0; ci <= mm; ++ci) {
-        if (pos[ci] < 0) continue;
-        const int c = cbase + pos[ci];
-        cnode[c] = inf.node_off + 2 * ci;
-        cstruct[c] = s;
-        cmask[c] = mask6(2 * ci);
-        cleft[c] = ci >= 1 ? tbase + ci - 1 : -1;
-        cright[c] = ci < mm ? tbase + ci : -1;
-        cprev[c] = k > 0 ? cbase + slot[k - 1] : -1;
-        cnext[c] = k + 1 < M ? cbase + slot[k + 1] : -1;
-        ++k;
-      }
-      if (rpos[s] >= 0) roots[rpos[s]] = cbase + slot[0];
-      int l = 0;
-      for (int h = 1; h < M; h *= 2, ++l) {
-        CrItem* o = &odd[cd.odd_off[l] + opos[(size_t)s * NL + l]];
-        for (int kp = h; kp < M; kp += 2 * h)
-          *o++ = CrItem{cbase + slot[kp], cbase + slot[kp - h], kp + h < M ? cbase + slot[kp + h] : -1, s};
-        CrItem* v = &even[cd.even_off[l] + epos[(size_t)s * NL + l]];
-        for (int kp = 0; kp < M; kp += 2 * h) {
-          bool hp = kp - h >= 0, hn = kp + h < M;
-          *v++ = CrItem{cbase + slot[kp], hp ? cbase + slot[kp - h] : -1, hn ? cbase + slot[kp + h] : -1, s};
-        }
-      }
-    });
-    cd.n_chain_elems = (int)elem_list.size();
-    cd.n_corners = (int)cnode.size();
-    cd.n_levels = n_levels;
-    cd.n_roots = (int)roots.size();
-    if (cd.n_chain_elems) {
-      size_t ne = elem_list.size(), nc = std::max<size_t>(cnode.size(), 1);
-      if (!upload(B, &cd.elem_list, elem_list) || !upload(B, &cd.elem_corner_a, eca) ||
-          !upload(B, &cd.elem_corner_b, ecb) || !upload(B, &cd.corner_node, cnode) ||
-          !upload(B, &cd.corner_struct, cstruct) || !upload(B, &cd.corner_left, cleft) ||
-          !upload(B, &cd.corner_right, cright) || !upload(B, &cd.corner_prev, cprev) ||
-          !upload(B, &cd.corner_next, cnext) || !upload(B, &cd.odd, odd) || !upload(B, &cd.even, even) ||
-          !upload(B, &cd.roots, roots) || !upload(B, &cd.elem_mask, emask) || !upload(B, &cd.corner_mask, cmask) ||
-          !balloc(B, &cd.ez, ne * 78) || !balloc(B, &cd.ec, ne * 156) || !balloc(B, &cd.cD, nc * 36) ||
-          !balloc(B, &cd.cL, nc * 36) || !balloc(B, &cd.cU, nc * 36) || !balloc(B, &cd.cb, nc * 6) ||
-          !balloc(B, &cd.cz, nc * 78) || !balloc(B, &cd.ce, nc * 114) || !balloc(B, &cd.cx, nc * 6))
-        return GF_ERR_CUDA;
-    }
-    // the symmetric chains: parts of level 0 are the elements; each level
-    // merges neighbours in pairs, an odd last part passing up unchanged
-    SymChains& sy = cd.sy;
-    std::vector<int> sbase(n, 0), cbase(n, 0), mcnt(NL, 0), mpos((size_t)n * NL, 0), tpos(n, 0), chains;
-    int n_top = 0;
-    for (int s = 0; s < n; ++s) {
-      if (!plan[s].chain || !B->info[s].sym) continue;
-      const int mm = B->info[s].n_elem;
-      sbase[s] = sy.n_elem;
-      cbase[s] = sy.n_corner;
-      sy.n_elem += mm;
-      sy.n_corner += mm + 1;
-      chains.push_back(s);
-      int l = 0, k = mm;
-      for (; k > SYM_TOP; ++l, k = (k + 1) / 2) {
-        if (l >= NL) { set_err(ctx, "chain too long for %d elimination levels", NL); return GF_ERR_ARG; }
-        mpos[(size_t)s * NL + l] = mcnt[l];
-        mcnt[l] += k / 2;
-        sy.n_levels = std::max(sy.n_levels, l + 1);
-      }
-      tpos[s] = n_top;
-      n_top += k - 1;
-    }
-    for (int l = 0; l < NL; ++l) sy.merge_off[l + 1] = sy.merge_off[l] + mcnt[l];
-    sy.n_merge = sy.merge_off[NL] + n_top;
-    sy.n_part = sy.n_elem + sy.n_merge;
-    sy.n_chains = (int)chains.size();
-    if (sy.n_elem) {
-      hvec<int> selem(sy.n_elem), sstr(sy.n_elem), sdof(sy.n_elem), scorner(sy.n_elem), snode(sy.n_corner);
-      hvec<SymMerge> merge(sy.n_merge);
-      hvec<SymChain> schain(sy.n_chains);
-      parallel_structures(sy.n_chains, work, [&](int c) {
-        const int s = chains[c];
-        const StructInfo& inf = B->info[s];
-        const std::vector<int>& g6 = plan[s].g6;
-        const int mm = inf.n_elem, b0 = sbase[s], c0 = cbase[s];
-        std::vector<int> id(mm), end(mm);  // part, its last corner
-        for (int e = 0; e < mm; ++e) {
-          selem[b0 + e] = inf.elem_off + e;
-          sstr[b0 + e] = s;
-          sdof[b0 + e] = inf.dof_off + g6[6 * (2 * (size_t)e + 1)];
-          scorner[b0 + e] = c0 + e;
-          id[e] = b0 + e;
-          end[e] = c0 + e + 1;
-        }
-        for (int k = 0; k <= mm; ++k) snode[c0 + k] = inf.node_off + 2 * k;
-        SymChain& ch = schain[c];
-        ch = SymChain{0, sy.merge_off[NL] + tpos[s], 0, c0, c0 + mm, s};
-        int top = ch.top;
-        for (int l = 0, k = mm; k > 1; ++l, k = (k + 1) / 2) {
-          if (k <= SYM_TOP && !ch.n_top) ch.n_top = k;
-          int at = k > SYM_TOP ? sy.merge_off[l] + mpos[(size_t)s * NL + l] : top, first = c0;
-          for (int q = 0; q < k / 2; ++q, ++at) {
-            const int mid = end[2 * q];
-            merge[at] = SymMerge{id[2 * q], id[2 * q + 1], sy.n_elem + at, first, mid, end[2 * q + 1], s,
-                                 inf.dof_off + g6[6 * 2 * (size_t)(mid - c0)]};
-            first = end[2 * q + 1];
-            id[q] = sy.n_elem + at;
-            end[q] = first;
-          }
-          if (k <= SYM_TOP) top = at;
-          if (k % 2) {
-            id[k / 2] = id[k - 1];
-            end[k / 2] = end[k - 1];
-          }
-        }
-        if (!ch.n_top) ch.n_top = 1;
-        ch.root = id[0];
-      });
-      if (!upload(B, &sy.elem, selem) || !upload(B, &sy.elem_struct, sstr) || !upload(B, &sy.elem_dof, sdof) ||
-          !upload(B, &sy.elem_corner, scorner) || !upload(B, &sy.corner_node, snode) ||
-          !upload(B, &sy.merge, merge) || !upload(B, &sy.chain, schain) ||
-          !balloc(B, &sy.part, (size_t)sy.n_part * 57) || !balloc(B, &sy.ez, (size_t)sy.n_elem * 81) ||
-          !balloc(B, &sy.mz, (size_t)sy.n_merge * 81) || !balloc(B, &sy.x, (size_t)sy.n_corner * 6))
-        return GF_ERR_CUDA;
-    }
-  }
+  // chain solver data of the two kinds of chains
+  if (!build_parts(B, models, plan, work, true, b.chain_sym) || !build_parts(B, models, plan, work, false, b.chain_gen))
+    return GF_ERR_CUDA;
   // colour lists
   std::vector<int> color_elems;
   b.n_colors = max_color;
@@ -1380,11 +1292,11 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
 int count_launches_per_pass(const gf_batch* B) {
   int colors = 0;
   for (int c = 0; c < B->b.n_colors; ++c) colors += B->b.color_off[c + 1] > B->b.color_off[c];
-  const ChainData& cd = B->b.chain;
+  const ChainParts &cs = B->b.chain_sym, &cg = B->b.chain_gen;
   // chains only: one gather launch in place of the colour passes
-  if (B->b.n_elem && !B->b.full_band && cd.n_chain_elems + cd.sy.n_elem == B->b.n_elem) colors = 1;
+  if (B->b.n_elem && !B->b.full_band && cs.n_elem + cg.n_elem == B->b.n_elem) colors = 1;
   // step_begin, step_nodes, zero, tangent, residual, band solve, update, control, commits
-  return 10 + (B->b.n_loads ? 1 : 0) + (B->b.any_dynamic ? 1 : 0) + colors + chain_launches(cd) + sym_chain_launches(cd.sy) + shell_launches_per_pass(B->b) + (B->b.any_rayleigh ? 1 : 0) +
+  return 10 + (B->b.n_loads ? 1 : 0) + (B->b.any_dynamic ? 1 : 0) + colors + chain_launches(cs) + chain_launches(cg) + shell_launches_per_pass(B->b) + (B->b.any_rayleigh ? 1 : 0) +
          (B->b.n_pipe_press ? 1 : 0) + (B->b.mon_total ? 1 : 0);
 }
 

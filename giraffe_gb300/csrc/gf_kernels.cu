@@ -1532,7 +1532,7 @@ static void launch_mount(const Batch& b, cudaStream_t st, LaunchProf* prof) {
     if (b.n_pipe_press) k_pipe_pressure<<<(b.n_pipe_press + 31) / 32, PP_THREADS, 0, st>>>(b);
     if (b.any_rayleigh) k_beam_rayleigh<<<(b.n_elem + 31) / 32, RAY_THREADS, 0, st>>>(b);
   }
-  if (!b.full_band && b.chain.n_chain_elems + b.chain.sy.n_elem == b.n_elem) {
+  if (!b.full_band && b.chain_sym.n_elem + b.chain_gen.n_elem == b.n_elem) {
     // chains only: the residual is all the scatter would assemble
     ProfScope q(prof, st, KC_SCATTER);
     const int64_t nt = (int64_t)b.n_nodes * 6;
@@ -1558,8 +1558,8 @@ void launch_iteration(const Batch& b, cudaStream_t st, bool commit_kernels, Laun
   { ProfScope q(prof, st, KC_LOADS); launch_loads(b, st); }
   { ProfScope q(prof, st, KC_RESIDUAL); k_residual<<<b.n_chunks, 256, 0, st>>>(b); }
   { ProfScope q(prof, st, KC_SOLVE); launch_band_solve(b, st); }
-  if (b.chain.n_chain_elems) { ProfScope q(prof, st, KC_CHAIN); launch_chain_solve(b, b.chain, st); }
-  if (b.chain.sy.n_elem) { ProfScope q(prof, st, KC_CHAIN); launch_sym_chains(b, b.chain.sy, st); }
+  if (b.chain_gen.n_elem) { ProfScope q(prof, st, KC_CHAIN); launch_gen_chains(b, b.chain_gen, st); }
+  if (b.chain_sym.n_elem) { ProfScope q(prof, st, KC_CHAIN); launch_sym_chains(b, b.chain_sym, st); }
   if (b.sh.n_wide) launch_wide_solve(b, st, prof);
   { ProfScope q(prof, st, KC_UPDATE); launch_increment(b, st); }
   { ProfScope q(prof, st, KC_CONTROL); k_control<<<(ns + 127) / 128, 128, 0, st>>>(b); }

@@ -225,78 +225,40 @@ __device__ __forceinline__ int table_row(const TableDev& T, const double* times,
 #endif
 
 // Chain solver data (see gf_chain.cuh).
-#define CR_MAX_LEVELS 24
+#define CHAIN_MAX_LEVELS 24
 
-// One cyclic-reduction item: a corner position with its neighbours at the
-// item's level (-1 when absent).
-struct CrItem {
-  int corner;  // batch-wide corner index
-  int prev;
-  int next;
-  int structure;
+// A merge: the parts e1 (corners p to k) and e2 (k to n) become part `out`, corner
+// k eliminated.  mask: k's free DOFs; dof: the first of them (batch-wide; the
+// others follow in order).
+struct ChainMerge {
+  int e1, e2, out, p, k, n, structure, dof, mask;
 };
-
-// A merge of the symmetric chain elimination (gf_chain_sym.cu): the parts e1
-// (corners p to k) and e2 (k to n) become part `out`, corner k eliminated.
-// dof: corner k's first free DOF (batch-wide; its six are consecutive).
-struct SymMerge {
-  int e1, e2, out, p, k, n, structure, dof;
-};
-// A chain once SYM_TOP parts or fewer are left: their number, the merges that
+// A chain once CHAIN_TOP parts or fewer are left: their number, the merges that
 // are left (chain by chain, level by level), the last part and the end corners.
-#define SYM_TOP 16
-struct SymChain {
+#define CHAIN_TOP 16
+struct ChainTop {
   int n_top, top, root, first, last, structure;
 };
-struct SymChains {
+// The chains of one kind (symmetric or general elimination).
+struct ChainParts {
   int n_elem, n_part, n_corner, n_merge, n_levels, n_chains;
   int* elem;         // batch element of each part of level 0
   int* elem_struct;
   int* elem_dof;     // first DOF (batch-wide) of its midside node
   int* elem_corner;  // its first corner (the next index is its last)
+  int* elem_mask;    // free DOFs of its corners: bits 0-5 the first, 6-11 the last
   int* corner_node;  // batch node of each corner
-  SymMerge* merge;   // the levels of more than SYM_TOP parts, level by level, then every chain's last ones
-  int merge_off[CR_MAX_LEVELS + 1];
-  SymChain* chain;
-  // structure-of-arrays, entry x of item i at [x * n + i]
-  double* part;      // [57][n_part]  condensed stiffness over (du, a0, a1) and nodal forces
-  double* ez;        // [81][n_elem]  kept for the midside nodes' back substitution
-  double* mz;        // [81][n_merge]  for the eliminated corners'
-  double* x;         // [6][n_corner]  solution at the corners
-};
-
-struct ChainData {
-  int n_chain_elems;   // elements of chain structures
-  int n_corners;       // free corners of chain structures
-  int n_levels;
-  int* elem_list;      // batch element ids of chain elements
-  int* elem_corner_a;  // corner index of the element's first corner (-1 if fixed)
-  int* elem_corner_b;  // corner index of the element's last corner (-1 if fixed)
-  SymChains sy;        // the chains solved by the symmetric elimination (the rest of this struct: the others)
-  int* elem_mask;      // free DOFs of the element's corners: bits 0-5 the first, 6-11 the last
-  int* corner_mask;    // free DOFs of the corner (bits 0-5)
-  int* corner_node;    // batch node id of each free corner
-  int* corner_struct;
-  int* corner_left;    // chain element to the left (-1 if none)
-  int* corner_right;   // chain element to the right (-1 if none)
-  int* corner_prev;    // previous free corner of the same chain (-1 if none)
-  int* corner_next;    // next free corner (-1 if none)
-  // scratch below is structure-of-arrays: entry x of item i at [x * n_items + i]
-  double* ez;          // [6*13][chain elem]  Z_s = A_ss^{-1}[b_s | A_sa | A_sb]
-  double* ec;          // [6*26][chain elem]  -A_as Z_s (13 cols), -A_bs Z_s (13 cols)
-  double* cD;          // [36][corner] (row-major 6x6 per corner)
-  double* cL;          // [36][corner]
-  double* cU;          // [36][corner]
-  double* cb;          // [6][corner]
-  double* cz;          // [6*13][corner]  Z = D^{-1}[b | L | U] of an eliminated corner
-  double* ce;          // [114][corner]  outputs of the entry-per-thread update
-  double* cx;          // [6][corner]  solution
-  CrItem* odd;         // per level: eliminated positions
-  int odd_off[CR_MAX_LEVELS + 1];
-  CrItem* even;        // per level: surviving positions with at least one eliminated neighbour
-  int even_off[CR_MAX_LEVELS + 1];
-  int* roots;          // per chain structure: the corner left after all levels
-  int n_roots;
+  ChainMerge* merge; // the levels of more than CHAIN_TOP parts, level by level, then every chain's last ones
+  int merge_off[CHAIN_MAX_LEVELS + 1];
+  ChainTop* chain;
+  // What the item-per-thread kernels write is structure-of-arrays (the items
+  // below *_soa), what the item-per-warp ones write item by item (chain_at), so
+  // that either form's loads and stores are contiguous over its lanes.
+  int elem_soa, part_soa, merge_soa;
+  double* part;      // 57 or 156 per part: condensed stiffness and the forces on the two corners
+  double* ez;        // 81 or 78 per element: kept for the midside nodes' back substitution
+  double* mz;        // 81 or 78 per merge: for the eliminated corners'
+  double* x;         // 6 per corner: the solution
 };
 
 // Shell_1 elements and the wide-band storage of their structures.
@@ -480,7 +442,7 @@ struct Batch {
   int* chunk_struct;
   int* chunk_start;
   RedScratch* red;  // [n_struct], zero between kernels
-  ChainData chain;
+  ChainParts chain_sym, chain_gen;  // chains with a symmetric K_AA (StructInfo::sym), and the others
   ShellData sh;
 };
 
