@@ -527,6 +527,55 @@ template <typename T> __global__ void __launch_bounds__(MF_BACK_THREADS) k_mf_ba
   }
 }
 
+// Forward substitution alone, on fronts that hold their LU: every front of a
+// height, one CTA each.  w = the right-hand side of the own DOFs with what the
+// children leave (their column f, read through their parent indices, one child
+// after the other), then y1 = L11^-1 w1 in blocks of 32 and w2 -= L21 y1; both
+// into column f.
+template <typename T> __global__ void __launch_bounds__(MF_BACK_THREADS) k_mf_fwd(Batch b, int off) {
+  const FrontData& d = b.sh.mf;
+  const int id = d.list[off + blockIdx.x];
+  const Front F = d.fronts[id];
+  if (!mf_active(b, F.slot)) return;
+  const int f = F.f, s = F.s, ld = F.ld, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  T* G = mf_mat<T>(b, F);
+  extern __shared__ __align__(16) unsigned char mf_raw[];
+  T* w = reinterpret_cast<T*>(mf_raw);  // [f]
+  const T* P = mf_rhs(b, (T*)nullptr);
+  for (int i = tid; i < f; i += MF_BACK_THREADS) w[i] = i < s ? P[d.dof_at[F.dof0 + i]] : T(0);
+  for (int k = d.kid_off[id]; k < d.kid_off[id + 1]; ++k) {
+    __syncthreads();
+    const Front C = d.fronts[d.kids[k]];
+    const T* cw = mf_mat<T>(b, C) + (int64_t)C.f * C.ld + C.s;
+    const int* rel = d.rel + C.rel;
+    for (int i = tid; i < C.f - C.s; i += MF_BACK_THREADS) w[rel[i]] += cw[i];
+  }
+  __syncthreads();
+  for (int j0 = 0; j0 < s; j0 += 32) {
+    const int nb = min(32, s - j0);
+    if (warp == 0) {
+      T v = lane < nb ? w[j0 + lane] : T(0);
+      for (int k = 0; k + 1 < nb; ++k) {
+        const T l = lane > k && lane < nb ? G[j0 + lane + (int64_t)(j0 + k) * ld] : T(0);
+        const T yk = __shfl_sync(0xffffffffu, v, k);
+        if (lane > k) v = mfma(-l, yk, v);
+      }
+      if (lane < nb) w[j0 + lane] = v;
+    }
+    __syncthreads();
+    for (int i = j0 + nb + tid; i < f; i += MF_BACK_THREADS) {
+      T a0 = T(0), a1 = T(0);
+      for (int k = 0; k < nb; k += 2) {
+        a0 = mfma(G[i + (int64_t)(j0 + k) * ld], w[j0 + k], a0);
+        if (k + 1 < nb) a1 = mfma(G[i + (int64_t)(j0 + k + 1) * ld], w[j0 + k + 1], a1);
+      }
+      w[i] -= a0 + a1;
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < f; i += MF_BACK_THREADS) G[i + (int64_t)f * ld] = w[i];
+}
+
 // ---- standalone systems (one structure): matrix entries into the fronts ----
 
 // A CSR row per thread: distinct rows own distinct entries, and the entries of
@@ -560,6 +609,7 @@ template <typename T> void mf_attrs() {
   static const bool done = [] {
     cudaFuncSetAttribute(k_mf_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          MF_SMALL * (MF_SMALL + 1) * (int)sizeof(T));
+    cudaFuncSetAttribute(k_mf_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k_mf_back<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     return true;
   }();
@@ -635,6 +685,22 @@ void launch_front_solve(const Batch& b, cudaStream_t st, LaunchProf* prof) {
   { ProfScope q(prof, st, KC_WIDE_UPDATE); launch_front_factor<double>(b, st); }
   { ProfScope q(prof, st, KC_WIDE_SUBST); launch_front_back<double>(b, st); }
 }
+
+// The same with the FP32 factor, on r32.
+void launch_front_solve32(const Batch& b, cudaStream_t st, LaunchProf* prof) {
+  { ProfScope q(prof, st, KC_WIDE_DIAG); launch_front_assemble<float>(b, st); }
+  { ProfScope q(prof, st, KC_WIDE_UPDATE); launch_front_factor<float>(b, st); }
+  { ProfScope q(prof, st, KC_WIDE_SUBST); launch_front_back<float>(b, st); }
+}
+// Another right-hand side (r32) with the FP32 factor.
+void launch_front_resolve32(const Batch& b, cudaStream_t st) {
+  for (const FrontLevel& V : b.sh.mf.sched->level) {
+    const int f = std::max(V.small_f, V.big_f);
+    k_mf_fwd<float><<<V.n_small + V.n_big, MF_BACK_THREADS, (size_t)f * sizeof(float), st>>>(b, V.small_off);
+  }
+  launch_front_back<float>(b, st);
+}
+int front_resolve_launches(const Batch& b) { return b.sh.mf.sched ? 2 * (int)b.sh.mf.sched->level.size() + 1 : 0; }
 
 void launch_front_csr(const Batch& b, int n, const int* rp, const int* ci, const double* v, cudaStream_t st) {
   launch_front_zero<double>(b, st);

@@ -62,6 +62,9 @@ struct FrontData {
   int* list;        // front ids by height
   int2* ext_jobs;   // (child front, column block)
   int2* schur_jobs; // (front, row tile | column tile << 16)
+  int* kid_off;     // children of front i: kids[kid_off[i] .. kid_off[i + 1])
+  int* kids;
+  int* dof_at;      // elimination position -> free DOF (batch-wide)
   int* pos;         // free DOF (batch-wide) -> elimination position (batch-wide)
   int* dof_front;   // elimination position -> its front
   int* map;         // [n_shells][729] destination of K_e entries in F, relative to the structure's first front (-1: none)
@@ -107,7 +110,7 @@ FrontPlan plan_fronts(const NdGraph& g, const std::vector<int>& dptr, const std:
 // batch-wide.
 struct FrontBuild {
   std::vector<gf::Front> fronts;
-  std::vector<int> bnd, rel, list, pos, dof_front;
+  std::vector<int> bnd, rel, list, pos, dof_front, kid_off, kids, dof_at;
   std::vector<int2> ext_jobs, schur_jobs;
   std::vector<int64_t> base, size;  // per structure (0 for the others)
   int64_t total = 0;

@@ -1172,8 +1172,8 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
   if (!wide_structs.empty()) {
     const bool mixed = B->opts.precision == GF_PREC_MIXED && !B->band_view;
     B->wb_total = wb_total;
-    if (!upload(B, &sd.wide_structs, wide_structs) || !balloc(B, &sd.panel, 1) ||
-        ((mixed || B->band_view) && !balloc(B, &sd.wband, (size_t)wb_total)))
+    if (!upload(B, &sd.wide_structs, wide_structs) ||
+        (B->band_view && !balloc(B, &sd.wband, (size_t)wb_total)))
       return GF_ERR_CUDA;
     if (!B->band_view) {
       // the fronts of all structures in one schedule
@@ -1195,7 +1195,9 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       if (!upload(B, &md.fronts, fb.fronts) || !upload(B, &md.bnd, fb.bnd) || !upload(B, &md.rel, fb.rel) ||
           !upload(B, &md.list, fb.list) || !upload(B, &md.ext_jobs, fb.ext_jobs) ||
           !upload(B, &md.schur_jobs, fb.schur_jobs) || !upload(B, &md.pos, fb.pos) ||
-          !upload(B, &md.dof_front, fb.dof_front) || !upload(B, &md.base, fb.base) || !upload(B, &md.size, fb.size) ||
+          !upload(B, &md.dof_front, fb.dof_front) || !upload(B, &md.kid_off, fb.kid_off) ||
+          !upload(B, &md.kids, fb.kids) || !upload(B, &md.dof_at, fb.dof_at) ||
+          !upload(B, &md.base, fb.base) || !upload(B, &md.size, fb.size) ||
           !balloc(B, &md.map, (size_t)shell_off * 729) || !balloc(B, &md.F, (size_t)fb.total) ||
           !balloc(B, &md.x, (size_t)dof_off))
         return GF_ERR_CUDA;
@@ -1203,16 +1205,15 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       md.sched = &B->sched;
     }
     if (mixed) {
-      // the FP32 LU beside the FP64 K_AA, its right-hand side and scratch,
-      // the saved Newton right-hand side and the refinement state
-      if (!balloc(B, &sd.wband32, (size_t)wb_total) || !balloc(B, &sd.r32, (size_t)dof_off) ||
-          !balloc(B, &sd.y32, (size_t)dof_off) || !balloc(B, &sd.ir_rhs, (size_t)dof_off) ||
+      // the FP32 LU's right-hand side (its factor takes the fronts' storage),
+      // the saved Newton right-hand side, the residual and the refinement state
+      std::vector<int> slot(n, -1);
+      for (size_t z = 0; z < wide_structs.size(); ++z) slot[wide_structs[z]] = (int)z;
+      if (!balloc(B, &sd.r32, (size_t)dof_off) || !balloc(B, &sd.ir_res, (size_t)dof_off) ||
+          !balloc(B, &sd.ir_rhs, (size_t)dof_off) || !upload(B, &sd.wide_slot, slot) ||
           !zeroed(B, &sd.ir, wide_structs.size()) || !zeroed(B, &sd.ir_more, 4))
         return GF_ERR_CUDA;
-      if (!B->count_only) {
-        for (auto& a : sd.aux) CK(cudaStreamCreateWithFlags(&a, cudaStreamNonBlocking));
-        for (auto& e : sd.evt) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      }
+      if (!B->count_only) CK(cudaStreamCreateWithFlags(&sd.ir_stream, cudaStreamNonBlocking));
     }
   }
   // device arrays
@@ -1270,14 +1271,11 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
   CK(cudaMemsetAsync(b.nodeK, 0, sizeof(double) * (size_t)std::max(node_off, 1) * 9, B->stream));
   b.mixed = B->opts.precision == GF_PREC_MIXED;
   b.sh.ir_max = B->opts.max_refine > 0 ? B->opts.max_refine : GF_IR_MAX;
-  b.sh.wide_tc = GF_WIDE_FP64;  // the mixed path's factor is FP32
   if (b.sh.n_wide) {
-    // tile shapes: the caller's entries, the others from the autotuner
-    // (served waves, whose device memory comes from the server's budget,
-    // take the defaults rather than time a synthetic band beside it)
+    // tile shapes of the wide-band LU: the caller's entries, else the defaults
+    // (the structures' own solves do not run it)
     const int* wt = B->opts.wide_tiles;
     WideTiles t;
-    if (!(wt[0] && wt[1] && wt[2] && wt[3]) && !B->arena && b.sh.wband32) t = tune_wide_tiles(B->ctx, b.sh.max_kl, b.sh.wide_tc);
     if (wt[0]) t.trsm_rb = wt[0];
     if (wt[1]) t.trsm_first = wt[1];
     if (wt[2]) t.corner = wt[2];
@@ -1406,10 +1404,7 @@ gf_batch* gf_batch_create(gf_ctx* ctx, int n, const gf_model_desc* models, const
 void gf_batch_destroy(gf_batch* B) {
   if (!B) return;
   if (B->graph) cudaGraphExecDestroy(B->graph);
-  for (auto& a : B->b.sh.aux)
-    if (a) cudaStreamDestroy(a);
-  for (auto& e : B->b.sh.evt)
-    if (e) cudaEventDestroy(e);
+  if (B->b.sh.ir_stream) cudaStreamDestroy(B->b.sh.ir_stream);
   for (void* p : B->allocs) {
     if (B->arena) B->arena->release(p);
     else cudaFree(p);
@@ -1492,12 +1487,12 @@ int run_passes(gf_batch* B, long long* passes_out, LaunchProf* prof = nullptr) {
 
 // Launches of the mixed path's refinement sweeps and FP64 fallbacks since
 // the last call, from the device counters (the stream is idle here).
-static long long refine_launches(gf_batch* B) {
+static long long refine_launch_count(gf_batch* B) {
   const int* cnt = B->b.sh.ir_more;
   if (!cnt) return 0;
   int c[4];
   if (cudaMemcpy(c, cnt, sizeof(c), cudaMemcpyDeviceToHost) != cudaSuccess) return 0;
-  const long long n = gf::wide_refine_launches(B->b, c[2] - B->ir_seen[0], c[3] - B->ir_seen[1]);
+  const long long n = gf::refine_launches(B->b, c[2] - B->ir_seen[0], c[3] - B->ir_seen[1]);
   B->ir_seen[0] = c[2];
   B->ir_seen[1] = c[3];
   return n;
@@ -1521,7 +1516,7 @@ int gf_batch_run(gf_batch* B) {
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, B->ev0, B->ev1));
   B->last_ms = ms;
-  B->last_launches = passes * B->launches_per_pass + refine_launches(B);
+  B->last_launches = passes * B->launches_per_pass + refine_launch_count(B);
   return GF_OK;
 }
 
@@ -1673,7 +1668,7 @@ int gf_batch_solve_timed(gf_batch* B, int steps, double* ms_out) {
   CK(cudaEventElapsedTime(&ms, B->ev0, B->ev1));
   *ms_out = ms;
   B->last_ms = ms / steps;
-  B->last_launches = launches + refine_launches(B);
+  B->last_launches = launches + refine_launch_count(B);
   return GF_OK;
 }
 

@@ -1560,7 +1560,7 @@ void launch_iteration(const Batch& b, cudaStream_t st, bool commit_kernels, Laun
   { ProfScope q(prof, st, KC_SOLVE); launch_band_solve(b, st); }
   if (b.chain_gen.n_elem) { ProfScope q(prof, st, KC_CHAIN); launch_gen_chains(b, b.chain_gen, st); }
   if (b.chain_sym.n_elem) { ProfScope q(prof, st, KC_CHAIN); launch_sym_chains(b, b.chain_sym, st); }
-  if (b.sh.n_wide) launch_wide_solve(b, st, prof);
+  launch_shell_solve(b, st, prof);
   { ProfScope q(prof, st, KC_UPDATE); launch_increment(b, st); }
   { ProfScope q(prof, st, KC_CONTROL); k_control<<<(ns + 127) / 128, 128, 0, st>>>(b); }
   if (commit_kernels) {

@@ -72,9 +72,9 @@ struct ProfScope {
   }
 };
 
-// The wide band holds K_AA in the assembly view (gf_batch_assemble, the
-// Newton-iteration boundary) and in the mixed-precision path.
-__host__ __device__ inline bool wide_band_filled(const Batch& b) { return b.full_band || b.sh.wband32; }
+// The wide band holds K_AA in the assembly view only (gf_batch_assemble, the
+// Newton-iteration boundary).
+__host__ __device__ inline bool wide_band_filled(const Batch& b) { return b.full_band; }
 
 void launch_iteration(const Batch& b, cudaStream_t st, bool commit_kernels = true, LaunchProf* prof = nullptr);
 // FMA throughput probe: 8 independent chains per thread, `iters` steps.
@@ -120,6 +120,14 @@ void launch_front_solve(const Batch& b, cudaStream_t st, LaunchProf* prof = null
 void launch_front_csr(const Batch& b, int n, const int* rp, const int* ci, const double* v, cudaStream_t st);
 void launch_front_band(const Batch& b, int n, int kl, int ku, int ldab, const double* ab, cudaStream_t st);
 int front_launches(const Batch& b);
+// FP32: the same on r32, and another right-hand side with that factor.
+void launch_front_solve32(const Batch& b, cudaStream_t st, LaunchProf* prof = nullptr);
+void launch_front_resolve32(const Batch& b, cudaStream_t st);
+int front_resolve_launches(const Batch& b);
+// The solve of a batch's Shell_1 structures at its precision (gf_refine.cu).
+void launch_shell_solve(const Batch& b, cudaStream_t st, LaunchProf* prof = nullptr);
+int shell_solve_launches(const Batch& b);
+long long refine_launches(const Batch& b, long long sweeps, long long fallbacks);
 // The first error of a wide-band capture step (a conditional node or body
 // capture) since the last call on this thread; clears it.
 cudaError_t wide_capture_error();
@@ -139,8 +147,6 @@ void launch_shell_inertia_elements(int n, const ShellConst* c, const ShellHistAu
                                    cudaStream_t st);
 // Kernel launches of one pass of the shell and wide-band kernels.
 int shell_launches_per_pass(const Batch& b);
-int wide_launches_per_pass(const Batch& b);
-long long wide_refine_launches(const Batch& b, long long sweeps, long long fallbacks);
 
 // Band factor + solve of independent systems in the batch layout
 // (GF_LDB rows); FP64.  Returns per-system info in state[].info_fail.

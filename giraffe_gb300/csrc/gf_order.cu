@@ -307,6 +307,14 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
     at[height[k]].push_back(k);
     if (out.fronts[k].parent >= 0 && out.fronts[k].f > out.fronts[k].s) kids[out.fronts[k].parent].push_back(k);
   }
+  out.kid_off.assign(1, 0);
+  for (int k = 0; k < nf; ++k) {
+    out.kids.insert(out.kids.end(), kids[k].begin(), kids[k].end());
+    out.kid_off.push_back((int)out.kids.size());
+  }
+  out.dof_at.assign(n_dofs, -1);
+  for (int i = 0; i < n_dofs; ++i)
+    if (out.pos[i] >= 0) out.dof_at[out.pos[i]] = i;
   out.sched.level.resize(nl);
   out.sched.launches = 3;  // zero, right-hand sides, gather of the solution
   for (int l = 0; l < nl; ++l) {

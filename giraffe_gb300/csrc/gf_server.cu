@@ -77,14 +77,13 @@ constexpr size_t kWaveSlack = 1 << 16;
 // pageable memory (uploads).
 constexpr size_t kHostStage = (size_t)256 << 20;
 
-// Handles of a retired Shell_1 wave kept until the device is idle:
+// Handles of a retired wave kept until the device is idle:
 // destroying an executable graph with conditional nodes waits for the
 // device's other work, which would stall the polling loop behind the
 // running waves.
 struct Parked {
   cudaGraphExec_t graph = nullptr;
-  cudaStream_t aux[GF_WB_STREAMS] = {};
-  cudaEvent_t evt[GF_WB_EVENTS] = {};
+  cudaStream_t ir_stream = nullptr;
 };
 // Parked handles beyond this many are destroyed at once, waiting or not.
 constexpr size_t kMaxParked = 64;
@@ -297,10 +296,7 @@ int read_chunk(gf_server* S, Wave& w, bool* progressed) {
 
 void destroy_parked(Parked& p) {
   if (p.graph) cudaGraphExecDestroy(p.graph);
-  for (auto& a : p.aux)
-    if (a) cudaStreamDestroy(a);
-  for (auto& e : p.evt)
-    if (e) cudaEventDestroy(e);
+  if (p.ir_stream) cudaStreamDestroy(p.ir_stream);
 }
 
 // Destroys the parked handles (the device is idle, or too many wait).
@@ -314,11 +310,10 @@ void retire(gf_server* S, size_t i) {
   for (int s = 0; s < (int)w->reqs.size(); ++s)
     if (!w->reported[s]) report(S, *w, s, nullptr, GF_ERR_TIMEOUT);
   gf_batch* B = w->B;
-  if (B->b.sh.loops_in_graph) {
+  if (B->graph) {
     Parked p;
     std::swap(p.graph, B->graph);
-    for (int k = 0; k < GF_WB_STREAMS; ++k) std::swap(p.aux[k], B->b.sh.aux[k]);
-    for (int k = 0; k < GF_WB_EVENTS; ++k) std::swap(p.evt[k], B->b.sh.evt[k]);
+    std::swap(p.ir_stream, B->b.sh.ir_stream);
     S->parked.push_back(p);
     if (S->parked.size() > kMaxParked) {
       destroy_parked(S->parked.front());
@@ -405,7 +400,6 @@ void build_wave(gf_server* S, Wave& w) {
   B->host_stage = &S->stage;
   B->stream = S->capture_stream;
   int r = build_batch(B, take, models.data());
-  B->b.sh.loops_in_graph = 1;
   // the uploads must land before the staging blocks are reused
   if (cudaStreamSynchronize(S->capture_stream) != cudaSuccess && r == GF_OK) r = GF_ERR_CUDA;
   for (void* h : B->staged) S->stage.release(h);

@@ -939,6 +939,6 @@ int shell_launches_per_pass(const Batch& b) {
     n += 2 + (b.sh.any_rayleigh ? 1 : 0);  // tangent (+ Rayleigh damping) + commit
     for (int c = 0; c < b.sh.n_colors; ++c) n += b.sh.color_off[c + 1] > b.sh.color_off[c];
   }
-  return n + wide_launches_per_pass(b);
+  return n + shell_solve_launches(b);
 }
 }  // namespace gf

@@ -26,7 +26,7 @@
 #define GF_KB 17
 #define GF_LDB (2 * GF_KB + 1)
 #define GF_UW (GF_KB + 1)
-#define GF_WB_STREAMS 5  // helper streams of the wide-band lookahead
+#define GF_WB_STREAMS 3  // helper streams of the wide-band lookahead
 #define GF_WB_EVENTS 6
 
 namespace gf {
@@ -261,13 +261,11 @@ struct ChainParts {
   double* x;         // 6 per corner: the solution
 };
 
-// Shell_1 elements and the wide-band storage of their structures.
 // Tile shapes of the wide-band LU that leave every entry's arithmetic as it
 // is (so any choice gives the same bits): rows per CTA of the bulk trsm (4,
 // 8 or 16) and of the first trsm on the critical path (1, 2 or 4), the
 // output tile edge of the corner update (4 or 8), rows per CTA of the
-// triangular solves (32 or 64).  Picked by timing (the autotuner) or pinned
-// by the caller.
+// triangular solves (32 or 64).
 struct WideTiles {
   int trsm_rb = 8;
   int trsm_first = 2;
@@ -286,7 +284,7 @@ struct WideIr {
 
 struct ShellData {
   int n_shells;
-  int n_wide;       // structures solved by the wide-band LU
+  int n_wide;       // structures with Shell_1 elements (the wide-band LU's, in the assembly view and modal analysis)
   int max_panels;   // over those structures
   int max_kl;       // over those structures
   int* wide_structs;  // [n_wide] structure indices
@@ -308,24 +306,22 @@ struct ShellData {
   int color_off[17];
   int n_colors;
   double* wband;
-  // mixed precision (GF_PREC_MIXED): K_AA stays in wband (FP64) for the
-  // residuals; its LU is formed in wband32 (FP32, same geometry) and the
-  // solution refined in FP64: r32 / y32 the FP32 right-hand side and the
-  // forward-substitution scratch, ir_rhs the Newton right-hand side, ir the
-  // per-slot refinement state.  fp64_pass is set on the host's copy of the
-  // batch for the FP64 fallback launches (only structures with ir_fb run).
-  float* wband32;
+  // mixed precision (GF_PREC_MIXED): the LU is formed in FP32 and the solution
+  // refined in FP64: r32 the FP32 right-hand side and solution, ir_rhs the
+  // Newton right-hand side, ir_res the FP64 residual, ir the per-slot refinement
+  // state, wide_slot the slot of each structure.  fp64_pass is set on the host's
+  // copy of the batch for the FP64 fallback launches (only structures with ir_fb
+  // run).
   float* r32;
-  float* y32;
   double* ir_rhs;
+  double* ir_res;
+  int* wide_slot;
   struct WideIr* ir;
   WideTiles tiles;   // tile shapes of this batch's wide-band LU
   int* ir_more;      // [0] a slot still refines, [1] a slot needs the FP64 fallback,
                      // [2] sweeps run, [3] fallbacks run (both cumulative)
   int fp64_pass;
   int ir_max;        // refinement sweeps before the FP64 fallback
-  int* panel;       // device panel counter of the captured panel loops
-  int loops_in_graph;  // capture the panel loops as graph WHILE loops (served waves)
   int wide_tc;         // trailing update: 0 FP64 FMA, 1 tcgen05 Ozaki slices, 2 mma.sync Ozaki slices
   // the tensor-core update's slices of a panel: per wide structure slot,
   // [2 operands][8 slices][oz_rows][64] bf16 and [2][oz_rows] exponents;
@@ -343,11 +339,12 @@ struct ShellData {
   // nonzero when a bounded wait of the tensor-core update gave up (its
   // structures are then reported as failed solves)
   int* oz_error;
+  // host handle of the mixed path: the stream that roots the captured bodies of
+  // the refinement loop and of the FP64 fallback
+  cudaStream_t ir_stream;
   // host handles of the wide-band lookahead: helper streams and the events
-  // that fork from and join into the pass's stream; aux[2] roots the
-  // captured panel-loop bodies, aux[3] runs the bulk trsm beside the first
-  // blocks and the corner update, aux[4] roots the captured bodies of the
-  // refinement loop and of the FP64 fallback
+  // that fork from and join into the solve's stream; aux[2] runs the bulk trsm
+  // beside the first blocks and the corner update
   cudaStream_t aux[GF_WB_STREAMS];
   // [0] panel start, [1] after trsm, [2] after the corner update, [3] after
   // diag, [4] end of forward, [5] after the bulk trsm

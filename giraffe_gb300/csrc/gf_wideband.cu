@@ -46,68 +46,39 @@ __device__ __forceinline__ double wb_recip(double p) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Wide-band LU.  Band pointer and geometry of wide structure w, in the
-// factor's arithmetic type F (double: the FP64 LU in place of K_AA; float:
-// the FP32 LU of the mixed-precision path, beside K_AA).
+// Wide-band LU.  Band pointer and geometry of wide structure w.
 namespace {
-template <typename F>
-struct WBT {
-  F* a;
+struct WB {
+  double* a;
   int n, kl;
   int64_t W;
-  __device__ __forceinline__ F& at(int i, int j) const { return a[(kl + i - j) + (int64_t)j * W]; }
+  __device__ __forceinline__ double& at(int i, int j) const { return a[(kl + i - j) + (int64_t)j * W]; }
 };
-typedef WBT<double> WB;
 
-// A structure whose K_AA this launch factors: iterating, asking for a
-// solve, and in the FP64 fallback launches of the mixed path only those
-// whose refinement did not finish.
+// A structure whose K_AA this launch factors: iterating and asking for a solve.
 __device__ __forceinline__ bool wide_active(const Batch& b, int s) {
   const StructState& st = b.state[s];
-  return iterating_s(st) && st.need_solve && (!b.sh.fp64_pass || st.ir_fb);
+  return iterating_s(st) && st.need_solve;
 }
 
-__device__ __forceinline__ double* wb_base(const Batch& b, double*) { return b.sh.wband; }
-__device__ __forceinline__ float* wb_base(const Batch& b, float*) { return b.sh.wband32; }
-
-template <typename F = double>
-__device__ __forceinline__ WBT<F> wb_of(const Batch& b, const StructInfo& inf) {
-  WBT<F> w;
-  w.a = wb_base(b, (F*)nullptr) + inf.wb_off;
+__device__ __forceinline__ WB wb_of(const Batch& b, const StructInfo& inf) {
+  WB w;
+  w.a = b.sh.wband + inf.wb_off;
   w.n = inf.n_free;
   w.kl = inf.wkl;
   w.W = 2 * (int64_t)inf.wkl + 1;
   return w;
 }
 
-// 1/p in the factor's type: FP64 by Newton steps from the FP32 seed, FP32
-// correctly rounded.
-__device__ __forceinline__ double wb_rcp(double p) { return wb_recip(p); }
-__device__ __forceinline__ float wb_rcp(float p) { return __frcp_rn(p); }
-// fused multiply-add in the factor's own type (no promotion of FP32 to FP64)
-__device__ __forceinline__ double wfma(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float wfma(float a, float b, float c) { return fmaf(a, b, c); }
-
-// Right-hand side and forward-substitution scratch of the solves in type F:
-// the batch's P / y (FP64, column q of a multi-column solve at q rhs_ld), or
-// the mixed path's FP32 r32 / y32.
-__device__ __forceinline__ double* wb_rhs(const Batch& b, const StructInfo& inf, int q, double*) {
+// Right-hand side and forward-substitution scratch of the solves: the batch's
+// P / y, column q of a multi-column solve at q rhs_ld.
+__device__ __forceinline__ double* wb_rhs(const Batch& b, const StructInfo& inf, int q) {
   return b.P + inf.dof_off + (int64_t)q * b.rhs_ld;
 }
-__device__ __forceinline__ double* wb_scratch(const Batch& b, const StructInfo& inf, int q, double*) {
+__device__ __forceinline__ double* wb_scratch(const Batch& b, const StructInfo& inf, int q) {
   return b.y + inf.dof_off + (int64_t)q * b.rhs_ld;
 }
-__device__ __forceinline__ float* wb_rhs(const Batch& b, const StructInfo& inf, int, float*) {
-  return b.sh.r32 + inf.dof_off;
-}
-__device__ __forceinline__ float* wb_scratch(const Batch& b, const StructInfo& inf, int, float*) {
-  return b.sh.y32 + inf.dof_off;
-}
 constexpr int NB = GF_WB_NB;
-
-// Panel index of a wide-band kernel: p >= 0 as given; inside a captured
-// panel loop p = -1 - d, meaning the device counter plus d.
-__device__ __forceinline__ int wb_panel(const Batch& b, int p) { return p >= 0 ? p : *b.sh.panel + (-1 - p); }
 }  // namespace
 
 // Column / row maxima of panel p's L21 and U12 for wide structure slot z
@@ -142,34 +113,32 @@ __global__ void k_wb_zero(Batch b) {
 // sees the same operations in the same order as the textbook kij loop:
 // multiplier l = a_ik * (1 / a_kk), then a_ij = fma(-l, a_kj, a_ij).
 constexpr int DIAG_THREADS = 288;
-template <typename F>
 __global__ void __launch_bounds__(DIAG_THREADS) k_wb_diag(Batch b, int p) {
-  p = wb_panel(b, p);
   if (p < 0) return;
   int s = b.sh.wide_structs[blockIdx.x];
   if (!wide_active(b, s)) return;
   const StructInfo& inf = b.info[s];
   if (p >= inf.n_panels) return;
-  WBT<F> w = wb_of<F>(b, inf);
+  WB w = wb_of(b, inf);
   const int j0 = p * NB, nb = min(NB, w.n - j0);
-  __shared__ F Ac[NB][NB + 1];  // Ac[j][i] = A(i, j)
+  __shared__ double Ac[NB][NB + 1];  // Ac[j][i] = A(i, j)
   __shared__ int fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) fail = 0;
   // this panel's L21 / U12 maxima start at zero (the buffer of its parity
   // was last read by the slicing of panel p - 2, which precedes this kernel)
-  if (sizeof(F) == 8 && b.sh.wide_tc && tid < 2 * NB) wb_kmax(b, blockIdx.x, p)[tid] = 0ull;
+  if (b.sh.wide_tc && tid < 2 * NB) wb_kmax(b, blockIdx.x, p)[tid] = 0ull;
   for (int x = tid; x < NB * NB; x += blockDim.x) {
     const int i = x % NB, j = x / NB;
-    F v = F(0);
+    double v = 0.0;
     if (i < nb && j < nb && abs(i - j) <= w.kl) v = w.at(j0 + i, j0 + j);
     Ac[j][i] = v;
   }
   __syncthreads();
   if (warp == 8 && nb > 0) {  // the multipliers of column 0
-    const F piv = Ac[0][0];
+    const double piv = Ac[0][0];
     if (lane == 0 && (!(piv != 0.0) || !isfinite(piv))) fail = 1;
-    const F r = wb_rcp(piv);
+    const double r = wb_recip(piv);
     if (1 + lane < nb) Ac[0][1 + lane] *= r;
     if (33 + lane < nb) Ac[0][33 + lane] *= r;
   }
@@ -179,13 +148,13 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_wb_diag(Batch b, int p) {
     if (warp == 8) {
       // column k + 1: its update, then the next pivot and multipliers
       const int j = k + 1, i0 = j + lane, i1 = i0 + 32;
-      const F u = Ac[j][k];
-      if (i0 < nb) Ac[j][i0] = wfma(-Ac[k][i0], u, Ac[j][i0]);
-      if (i1 < nb) Ac[j][i1] = wfma(-Ac[k][i1], u, Ac[j][i1]);
+      const double u = Ac[j][k];
+      if (i0 < nb) Ac[j][i0] = fma(-Ac[k][i0], u, Ac[j][i0]);
+      if (i1 < nb) Ac[j][i1] = fma(-Ac[k][i1], u, Ac[j][i1]);
       __syncwarp();
-      const F piv = Ac[j][j];
+      const double piv = Ac[j][j];
       if (lane == 0 && (!(piv != 0.0) || !isfinite(piv))) fail = 1;
-      const F r = wb_rcp(piv);
+      const double r = wb_recip(piv);
       if (i0 > j && i0 < nb) Ac[j][i0] *= r;
       if (i1 < nb) Ac[j][i1] *= r;
     } else {
@@ -196,7 +165,7 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_wb_diag(Batch b, int p) {
         const int jj = __float2int_rz(((float)e + 0.5f) * inv_m);  // e / m, exact for e < 4096
         const int ii = e - jj * m;
         const int i = k + 1 + ii, j = k + 2 + jj;
-        Ac[j][i] = wfma(-Ac[k][i], Ac[j][k], Ac[j][i]);
+        Ac[j][i] = fma(-Ac[k][i], Ac[j][k], Ac[j][i]);
       }
     }
     __syncthreads();
@@ -208,8 +177,7 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_wb_diag(Batch b, int p) {
   // a zero or non-finite pivot: the FP64 LU's solver failure; the FP32 LU
   // of the mixed path hands the solve to the FP64 fallback instead
   if (tid == 0 && fail) {
-    if (sizeof(F) == 8) b.state[s].info_fail = 1;
-    else b.state[s].ir_fb = 1;
+    b.state[s].info_fail = 1;
   }
 }
 
@@ -223,36 +191,35 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_wb_diag(Batch b, int p) {
 // critical path) are a launch of their own with two rows per CTA, spread
 // over 64 SMs; the bulk runs beside it with eight.  Each CTA loads the half
 // of the diagonal block its side reads (U11 for L21, L11 for U12).
-template <typename F, int RB>
+template <int RB>
 __global__ void __launch_bounds__(32 * RB) k_wb_trsm(Batch b, int p, int row0, int nblk) {
-  p = wb_panel(b, p);
   if (p < 0) return;
   int s = b.sh.wide_structs[blockIdx.y];
   if (!wide_active(b, s)) return;
   const StructInfo& inf = b.info[s];
   if (p >= inf.n_panels) return;
-  WBT<F> w = wb_of<F>(b, inf);
+  WB w = wb_of(b, inf);
   const int j0 = p * NB, nb = min(NB, w.n - j0);
   const int m = min(w.kl, w.n - j0 - nb);  // rows below / columns right of the panel
   if (m <= 0) return;
   const bool lower = (int)blockIdx.x < nblk;
   const int rowb = row0 + RB * (lower ? (int)blockIdx.x : (int)blockIdx.x - nblk);
   if (rowb >= m) return;
-  __shared__ F T[NB][NB + 1];  // the diagonal block's LU (the half this side reads)
-  __shared__ F X[RB][NB + 1];
-  __shared__ F rd[NB];         // reciprocals of U11's diagonal
+  __shared__ double T[NB][NB + 1];  // the diagonal block's LU (the half this side reads)
+  __shared__ double X[RB][NB + 1];
+  __shared__ double rd[NB];         // reciprocals of U11's diagonal
   const int tid = threadIdx.x;
   for (int x = tid; x < NB * NB; x += blockDim.x) {
     int i = x % NB, j = x / NB;
-    T[i][j] = ((lower ? i <= j : i > j) && i < nb && j < nb && abs(i - j) <= w.kl) ? w.at(j0 + i, j0 + j) : F(0);
+    T[i][j] = ((lower ? i <= j : i > j) && i < nb && j < nb && abs(i - j) <= w.kl) ? w.at(j0 + i, j0 + j) : 0.0;
   }
   if (lower)
-    for (int k = tid; k < nb; k += blockDim.x) rd[k] = wb_rcp(w.at(j0 + k, j0 + k));
+    for (int k = tid; k < nb; k += blockDim.x) rd[k] = wb_recip(w.at(j0 + k, j0 + k));
   const int r = tid >> 5, c = tid & 31;  // row (or column) r of the block, lane c
   const int g = j0 + nb + rowb + r;      // global row (lower) or column (upper)
   const bool live = g < j0 + nb + m;
   for (int k = c; k < NB; k += 32) {
-    F v = F(0);
+    double v = 0.0;
     if (live && k < nb) {
       if (lower) { if (g - (j0 + k) <= w.kl) v = w.at(g, j0 + k); }
       else { if (g - (j0 + k) <= w.kl) v = w.at(j0 + k, g); }
@@ -265,11 +232,11 @@ __global__ void __launch_bounds__(32 * RB) k_wb_trsm(Batch b, int p, int row0, i
   // takes about 64 cycles on this part, a shuffle far less), and the half
   // with no live entry left (k >= 31 for the first) is skipped by a
   // warp-uniform branch instead of issued masked
-  F v0 = X[r][c], v1 = X[r][c + 32];
+  double v0 = X[r][c], v1 = X[r][c + 32];
   if (lower) {
     // x U11 = a: x_k = a_k / u_kk, then a_j -= x_k u_kj (j > k)
     for (int k = 0; k < nb; ++k) {
-      const F xk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31) * rd[k];
+      const double xk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31) * rd[k];
       if (k < 32) {
         if (c == k) v0 = xk;
       } else if (c == k - 32) {
@@ -281,7 +248,7 @@ __global__ void __launch_bounds__(32 * RB) k_wb_trsm(Batch b, int p, int row0, i
   } else {
     // L11 y = a (unit lower): y_k = a_k, then a_i -= l_ik y_k (i > k)
     for (int k = 0; k < nb; ++k) {
-      const F yk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
+      const double yk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
       if (k < 31 && c > k) v0 -= T[c][k] * yk;
       if (c + 32 > k && c + 32 < nb) v1 -= T[c + 32][k] * yk;
     }
@@ -294,7 +261,7 @@ __global__ void __launch_bounds__(32 * RB) k_wb_trsm(Batch b, int p, int row0, i
     if (lower) w.at(g, j0 + k) = X[r][k];
     else w.at(j0 + k, g) = X[r][k];
   }
-  if (sizeof(F) == 8 && b.sh.wide_tc)
+  if (b.sh.wide_tc)
   for (int k = tid; k < nb; k += blockDim.x) {
     // largest magnitude of column k of this block's L21 rows (row k of its
     // U12 columns), as FP64 bits, which order like the magnitudes; the
@@ -316,7 +283,6 @@ constexpr int UT = 32;
 // part: 0 every tile, 1 only the tiles of the next panel's diagonal block
 // (the first NB rows and columns of the window), 2 every other tile.
 __global__ void __launch_bounds__(256) k_wb_update(Batch b, int p, int part) {
-  p = wb_panel(b, p);
   if (p < 0) return;
   int s = b.sh.wide_structs[blockIdx.z];
   if (!wide_active(b, s)) return;
@@ -369,7 +335,6 @@ __global__ void __launch_bounds__(256) k_wb_update(Batch b, int p, int part) {
 // sub-partitions finish the 64 terms four times sooner than one.
 template <int CT>
 __global__ void __launch_bounds__(4 * CT * CT) k_wb_corner(Batch b, int p) {
-  p = wb_panel(b, p);
   if (p < 0) return;
   int s = b.sh.wide_structs[blockIdx.z];
   if (!wide_active(b, s)) return;
@@ -506,7 +471,6 @@ __device__ __forceinline__ OzSlices oz_slices(const Batch& b, int z) {
 // work is a few loads and integer operations per entry, bound by latency.
 constexpr int SL_ROWS = 16;
 __global__ void __launch_bounds__(256) k_wb_slice(Batch b, int p) {
-  p = wb_panel(b, p);
   if (p < 0) return;
   const int s = b.sh.wide_structs[blockIdx.z];
   if (!wide_active(b, s)) return;
@@ -585,7 +549,6 @@ __device__ __forceinline__ void oz_wait(int pending) {
 }
 
 __global__ void __launch_bounds__(OZ_THREADS) k_wb_update_tc(Batch b, int p, int part) {
-  p = wb_panel(b, p);
   if (p < 0) return;
   const int s = b.sh.wide_structs[blockIdx.z];
   if (!wide_active(b, s)) return;
@@ -789,7 +752,6 @@ __device__ __forceinline__ void t5_ld8(uint32_t taddr, uint32_t (&v)[8]) {
 __device__ __forceinline__ void t5_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
 __global__ void __launch_bounds__(T5_THREADS, 1) k_wb_update_t5(Batch b, int p, int part) {
-  p = wb_panel(b, p);
   if (p < 0) return;
   const int s = b.sh.wide_structs[blockIdx.z];
   if (!wide_active(b, s)) return;
@@ -953,41 +915,40 @@ __global__ void __launch_bounds__(T5_THREADS, 1) k_wb_update_t5(Batch b, int p, 
 // Forward substitution for panel p: y_p = L11^-1 b_p into y; then the rows
 // below the panel: P_i -= L21(i, :) y_p.  Every CTA solves the small
 // triangle redundantly; CTA 0 writes y_p.
-template <typename F, int SR>
+template <int SR>
 __global__ void __launch_bounds__(4 * SR) k_wb_fwd(Batch b, int p) {
-  p = wb_panel(b, p);
   if (p < 0) return;
   int s = b.sh.wide_structs[blockIdx.y];
   if (!wide_active(b, s)) return;
   const StructInfo& inf = b.info[s];
   if (p >= inf.n_panels) return;
-  WBT<F> w = wb_of<F>(b, inf);
+  WB w = wb_of(b, inf);
   const int j0 = p * NB, nb = min(NB, w.n - j0);
   const int m = min(w.kl, w.n - j0 - nb);
   // right-hand side blockIdx.z of a multi-column solve (columns rhs_ld apart)
-  F* P = wb_rhs(b, inf, blockIdx.z, (F*)nullptr);
-  F* Y = wb_scratch(b, inf, blockIdx.z, (F*)nullptr);
-  __shared__ F T[NB][NB + 1];  // the panel's diagonal block (L11 below the diagonal)
-  __shared__ F ys[NB];
-  __shared__ F part[4][SR];
+  double* P = wb_rhs(b, inf, blockIdx.z);
+  double* Y = wb_scratch(b, inf, blockIdx.z);
+  __shared__ double T[NB][NB + 1];  // the panel's diagonal block (L11 below the diagonal)
+  __shared__ double ys[NB];
+  __shared__ double part[4][SR];
   const int tid = threadIdx.x, r = tid % SR, q = tid / SR;
   const int row = blockIdx.x * SR + r, gi = j0 + nb + row;  // row below the panel
-  F lv[16];
+  double lv[16];
 #pragma unroll
   for (int u = 0; u < 16; ++u) {
     const int k = 16 * q + u;
-    lv[u] = (row < m && k < nb && gi - (j0 + k) <= w.kl) ? w.at(gi, j0 + k) : F(0);
+    lv[u] = (row < m && k < nb && gi - (j0 + k) <= w.kl) ? w.at(gi, j0 + k) : 0.0;
   }
   for (int x = tid; x < NB * NB; x += blockDim.x) {
     int i = x % NB, j = x / NB;
-    T[i][j] = (i < nb && j < nb && abs(i - j) <= w.kl) ? w.at(j0 + i, j0 + j) : F(0);
+    T[i][j] = (i < nb && j < nb && abs(i - j) <= w.kl) ? w.at(j0 + i, j0 + j) : 0.0;
   }
   __syncthreads();
   if (tid < 32) {
     // lanes hold entries k = lane and lane + 32
-    F v0 = tid < nb ? P[j0 + tid] : F(0), v1 = tid + 32 < nb ? P[j0 + tid + 32] : F(0);
+    double v0 = tid < nb ? P[j0 + tid] : 0.0, v1 = tid + 32 < nb ? P[j0 + tid + 32] : 0.0;
     for (int k = 0; k < nb; ++k) {
-      F yk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
+      double yk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
       if (tid > k) v0 -= T[tid][k] * yk;
       if (tid + 32 > k) v1 -= T[tid + 32][k] * yk;
     }
@@ -997,9 +958,9 @@ __global__ void __launch_bounds__(4 * SR) k_wb_fwd(Batch b, int p) {
   __syncthreads();
   if (blockIdx.x == 0)
     for (int k = tid; k < nb; k += blockDim.x) Y[j0 + k] = ys[k];
-  F acc = F(0);
+  double acc = 0.0;
 #pragma unroll
-  for (int u = 0; u < 16; ++u) acc = wfma(lv[u], ys[16 * q + u], acc);
+  for (int u = 0; u < 16; ++u) acc = fma(lv[u], ys[16 * q + u], acc);
   part[q][r] = acc;
   __syncthreads();
   if (q == 0 && row < m) P[gi] -= (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
@@ -1007,44 +968,43 @@ __global__ void __launch_bounds__(4 * SR) k_wb_fwd(Batch b, int p) {
 
 // Backward substitution for panel p (last panel first): x_p = U11^-1 y_p into
 // P; then the rows above the panel: y_i -= U(i, panel) x_p.
-template <typename F, int SR>
+template <int SR>
 __global__ void __launch_bounds__(4 * SR) k_wb_bwd(Batch b, int p) {
-  p = wb_panel(b, p);
   if (p < 0) return;
   int s = b.sh.wide_structs[blockIdx.y];
   if (!wide_active(b, s)) return;
   const StructInfo& inf = b.info[s];
   if (p >= inf.n_panels) return;
-  WBT<F> w = wb_of<F>(b, inf);
+  WB w = wb_of(b, inf);
   const int j0 = p * NB, nb = min(NB, w.n - j0);
   // right-hand side blockIdx.z of a multi-column solve (columns rhs_ld apart)
-  F* P = wb_rhs(b, inf, blockIdx.z, (F*)nullptr);
-  F* Y = wb_scratch(b, inf, blockIdx.z, (F*)nullptr);
-  __shared__ F T[NB][NB + 1];  // the panel's diagonal block (U11 on and above the diagonal)
-  __shared__ F rdiag[NB];
-  __shared__ F xs[NB];
-  __shared__ F part[4][SR];
+  double* P = wb_rhs(b, inf, blockIdx.z);
+  double* Y = wb_scratch(b, inf, blockIdx.z);
+  __shared__ double T[NB][NB + 1];  // the panel's diagonal block (U11 on and above the diagonal)
+  __shared__ double rdiag[NB];
+  __shared__ double xs[NB];
+  __shared__ double part[4][SR];
   const int tid = threadIdx.x, r = tid % SR, q = tid / SR;
   const int top = max(0, j0 - w.kl);
   const int gi = top + blockIdx.x * SR + r;  // row above the panel
-  F lv[16];
+  double lv[16];
 #pragma unroll
   for (int u = 0; u < 16; ++u) {
     const int k = 16 * q + u;
-    lv[u] = (gi < j0 && k < nb && j0 + k - gi <= w.kl) ? w.at(gi, j0 + k) : F(0);
+    lv[u] = (gi < j0 && k < nb && j0 + k - gi <= w.kl) ? w.at(gi, j0 + k) : 0.0;
   }
   for (int x = tid; x < NB * NB; x += blockDim.x) {
     int i = x % NB, j = x / NB;
-    T[i][j] = (i < nb && j < nb && abs(i - j) <= w.kl) ? w.at(j0 + i, j0 + j) : F(0);
+    T[i][j] = (i < nb && j < nb && abs(i - j) <= w.kl) ? w.at(j0 + i, j0 + j) : 0.0;
   }
   __syncthreads();
-  if (tid < nb) rdiag[tid] = wb_rcp(T[tid][tid]);
+  if (tid < nb) rdiag[tid] = wb_recip(T[tid][tid]);
   __syncthreads();
   if (tid < 32) {
-    F v0 = tid < nb ? Y[j0 + tid] : F(0), v1 = tid + 32 < nb ? Y[j0 + tid + 32] : F(0);
+    double v0 = tid < nb ? Y[j0 + tid] : 0.0, v1 = tid + 32 < nb ? Y[j0 + tid + 32] : 0.0;
     for (int k = nb - 1; k >= 0; --k) {
-      F mine = k < 32 ? v0 : v1;
-      F xk = __shfl_sync(0xffffffffu, mine, k & 31) * rdiag[k];
+      double mine = k < 32 ? v0 : v1;
+      double xk = __shfl_sync(0xffffffffu, mine, k & 31) * rdiag[k];
       if (k < 32) { if (tid == k) v0 = xk; }
       else { if (tid + 32 == k) v1 = xk; }
       if (tid < k) v0 -= T[tid][k] * xk;
@@ -1056,261 +1016,12 @@ __global__ void __launch_bounds__(4 * SR) k_wb_bwd(Batch b, int p) {
   __syncthreads();
   if (blockIdx.x == 0)
     for (int k = tid; k < nb; k += blockDim.x) P[j0 + k] = xs[k];
-  F acc = F(0);
+  double acc = 0.0;
 #pragma unroll
-  for (int u = 0; u < 16; ++u) acc = wfma(lv[u], xs[16 * q + u], acc);
+  for (int u = 0; u < 16; ++u) acc = fma(lv[u], xs[16 * q + u], acc);
   part[q][r] = acc;
   __syncthreads();
   if (q == 0 && gi < j0) Y[gi] -= (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
-}
-
-// ---- mixed precision: FP32 factor, FP64 refinement ----
-// The trailing update of the FP32 factor: A22 -= L21 U12 over panel p's
-// window in 64x64 tiles on the FP32 pipe, each of 256 threads a 4x4 block
-// of outputs (four consecutive rows of four columns, so the 16 lanes along a
-// column write 256 contiguous bytes).  part as k_wb_update; the corner (the
-// next panel's diagonal block, part 1) is the single tile (0, 0).
-constexpr int U32T = 64;
-__global__ void __launch_bounds__(256) k_wb_update32(Batch b, int p, int part) {
-  p = wb_panel(b, p);
-  if (p < 0) return;
-  int s = b.sh.wide_structs[blockIdx.z];
-  if (!wide_active(b, s)) return;
-  const StructInfo& inf = b.info[s];
-  if (p >= inf.n_panels) return;
-  WBT<float> w = wb_of<float>(b, inf);
-  const int j0 = p * NB, nb = min(NB, w.n - j0);
-  const int m = min(w.kl, w.n - j0 - nb);
-  if (m <= 0) return;
-  const int r0 = blockIdx.x * U32T, c0 = blockIdx.y * U32T;
-  if (r0 >= m || c0 >= m) return;
-  const bool corner = blockIdx.x == 0 && blockIdx.y == 0;
-  if ((part == 1 && !corner) || (part == 2 && corner)) return;
-  __shared__ __align__(16) float Ls[NB][U32T + 4];  // [k][row]
-  __shared__ __align__(16) float Us[NB][U32T + 4];  // [k][col]
-  const int tid = threadIdx.x, base = j0 + nb;
-  for (int x = tid; x < NB * U32T; x += 256) {
-    // rows of L21 along a band column are contiguous; U12's k too
-    const int i = x % U32T, k = x / U32T;
-    const int gk = j0 + k, gi = base + r0 + i;
-    Ls[k][i] = (k < nb && r0 + i < m && gi - gk <= w.kl) ? w.at(gi, gk) : 0.0f;
-    const int kk = x % NB, c = x / NB, gj = base + c0 + c;
-    Us[kk][c] = (kk < nb && c0 + c < m && gj - (j0 + kk) <= w.kl) ? w.at(j0 + kk, gj) : 0.0f;
-  }
-  __syncthreads();
-  const int tr = tid & 15, tc = tid >> 4;  // rows 4 tr .. 4 tr + 3, columns 4 tc .. 4 tc + 3
-  float acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[a][c] = 0.0f;
-#pragma unroll 4
-  for (int k = 0; k < NB; ++k) {
-    const float4 l = *reinterpret_cast<const float4*>(&Ls[k][4 * tr]);
-    const float4 u = *reinterpret_cast<const float4*>(&Us[k][4 * tc]);
-    const float lv[4] = {l.x, l.y, l.z, l.w}, uv[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[a][c] = fmaf(lv[a], uv[c], acc[a][c]);
-  }
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int col = c0 + 4 * tc + c;
-    if (col >= m) continue;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int row = r0 + 4 * tr + a;
-      if (row < m) w.at(base + row, base + col) -= acc[a][c];
-    }
-  }
-}
-
-// Start of a mixed solve: K_AA rounded into wband32 (where the FP32 LU then
-// forms), the Newton right-hand side saved in FP64 (ir_rhs) and rounded into
-// r32, the slot's refinement state reset.
-__global__ void __launch_bounds__(256) k_ir_begin(Batch b) {
-  const int z = blockIdx.y, s = b.sh.wide_structs[z];
-  if (!wide_active(b, s)) return;
-  const StructInfo& inf = b.info[s];
-  const int64_t nband = (int64_t)inf.n_free * (2 * (int64_t)inf.wkl + 1);
-  const double* src = b.sh.wband + inf.wb_off;
-  float* dst = b.sh.wband32 + inf.wb_off;
-  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, dt = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = t0; i < nband; i += dt) dst[i] = __double2float_rn(src[i]);
-  const double* P = b.P + inf.dof_off;
-  for (int64_t i = t0; i < inf.n_free; i += dt) {
-    b.sh.ir_rhs[inf.dof_off + i] = P[i];
-    b.sh.r32[inf.dof_off + i] = __double2float_rn(P[i]);
-  }
-  if (t0 == 0) {
-    WideIr& q = b.sh.ir[z];
-    q.dn = 0;
-    q.xn = 0;
-    q.dprev = 0.0;
-    q.k = 0;
-    q.done = 0;
-    b.state[s].ir_fb = 0;
-  }
-}
-
-// r = b - K x in FP64 (K_AA in wband, x in P, b in ir_rhs), rounded into
-// r32 for the next FP32 correction solve.  A CTA takes 256 rows and walks
-// the columns j of their band, 256 at a time through shared memory; at each
-// j its threads read K(i, j) of consecutive rows, contiguous in the
-// column-major band.  Two accumulators per row halve the dependent FP64
-// chain.
-__global__ void __launch_bounds__(256) k_ir_residual(Batch b) {
-  const int z = blockIdx.y, s = b.sh.wide_structs[z];
-  if (!wide_active(b, s) || b.sh.ir[z].done) return;
-  const StructInfo& inf = b.info[s];
-  const int n = inf.n_free, kl = inf.wkl;
-  const int i0 = blockIdx.x * 256;
-  if (i0 >= n) return;
-  const int i = i0 + threadIdx.x;
-  const double* x = b.P + inf.dof_off;
-  const WB w = wb_of(b, inf);
-  __shared__ double xs[256];
-  double acc0 = 0.0, acc1 = 0.0;
-  const int jlo = max(0, i0 - kl), jhi = min(n, i0 + 256 + kl);
-  for (int jt = jlo; jt < jhi; jt += 256) {
-    __syncthreads();
-    if (jt + (int)threadIdx.x < jhi) xs[threadIdx.x] = x[jt + threadIdx.x];
-    __syncthreads();
-    if (i >= n) continue;
-    // the columns of this tile inside row i's band: |i - j| <= kl
-    const int ta = max(0, i - kl - jt), te = min(min(256, jhi - jt), i + kl + 1 - jt);
-    int t = ta;
-    for (; t + 1 < te; t += 2) {
-      acc0 = fma(w.at(i, jt + t), xs[t], acc0);
-      acc1 = fma(w.at(i, jt + t + 1), xs[t + 1], acc1);
-    }
-    if (t < te) acc0 = fma(w.at(i, jt + t), xs[t], acc0);
-  }
-  if (i < n) b.sh.r32[inf.dof_off + i] = __double2float_rn(b.sh.ir_rhs[inf.dof_off + i] - (acc0 + acc1));
-}
-
-__device__ __forceinline__ double warp_max(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
-// x += d in FP64 (d: the FP32 correction the solve left in r32; first: x =
-// d, the first solve); the sweep's largest |d| and |x| raise the slot's
-// maxima (FP64 bits of non-negative values order like the values, so the
-// maxima do not depend on the CTAs' order).  A non-finite entry counts as
-// an infinite |d|.
-__global__ void __launch_bounds__(256) k_ir_correct(Batch b, int first) {
-  const int z = blockIdx.y, s = b.sh.wide_structs[z];
-  if (!wide_active(b, s) || b.sh.ir[z].done) return;
-  const StructInfo& inf = b.info[s];
-  double* x = b.P + inf.dof_off;
-  const float* d = b.sh.r32 + inf.dof_off;
-  double dm = 0.0, xm = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < inf.n_free; i += gridDim.x * blockDim.x) {
-    const double di = (double)d[i], xi = first ? di : x[i] + di;
-    x[i] = xi;
-    if (!isfinite(xi)) dm = INFINITY;
-    dm = fmax(dm, fabs(di));
-    xm = fmax(xm, fabs(xi));
-  }
-  __shared__ double red[2][8];
-  dm = warp_max(dm);
-  xm = warp_max(xm);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) {
-    red[0][warp] = dm;
-    red[1][warp] = xm;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 1; q < (int)(blockDim.x >> 5); ++q) {
-      dm = fmax(dm, red[0][q]);
-      xm = fmax(xm, red[1][q]);
-    }
-    WideIr& q = b.sh.ir[z];
-    if (dm > 0.0) atomicMax(&q.dn, (unsigned long long)__double_as_longlong(dm));
-    if (xm > 0.0) atomicMax(&q.xn, (unsigned long long)__double_as_longlong(xm));
-  }
-}
-
-// After a correction, per slot: converged (|d| <= 2^-52 |x|), stalled
-// (|d| > |d_prev| / 2: at the FP64 floor, or a factor too poor to refine),
-// or out of sweeps (ir_max).  A stall above 2^-30 |x|, the sweep limit, a
-// non-finite value or a failed FP32 pivot hand the solve to the FP64
-// fallback (ir_fb).  ir_more[0]: a slot refines on (inside a captured pass
-// also the refinement loop's condition h); ir_more[1]: a slot takes the
-// fallback; ir_more[2] counts the sweeps run (sweep: called after one).
-__global__ void k_ir_check(Batch b, cudaGraphConditionalHandle h, int use_h, int sweep) {
-  __shared__ int more, fb;
-  if (threadIdx.x == 0) {
-    more = 0;
-    fb = 0;
-  }
-  __syncthreads();
-  for (int z = threadIdx.x; z < b.sh.n_wide; z += blockDim.x) {
-    const int s = b.sh.wide_structs[z];
-    if (!wide_active(b, s)) continue;
-    WideIr& q = b.sh.ir[z];
-    StructState& st = b.state[s];
-    if (!q.done) {
-      const double dn = __longlong_as_double((long long)q.dn), xn = __longlong_as_double((long long)q.xn);
-      q.dn = 0;
-      q.xn = 0;
-      bool stop = false, bad = false;
-      if (st.ir_fb || !(dn <= DBL_MAX) || !(xn <= DBL_MAX)) {
-        stop = true;
-        bad = true;
-      } else if (q.k > 0) {
-        st.ir_sweeps += 1;
-        if (dn <= 0x1p-52 * xn) {
-          stop = true;
-        } else if (dn > 0.5 * q.dprev) {
-          stop = true;
-          bad = dn > 0x1p-30 * xn;
-        } else if (q.k >= b.sh.ir_max) {
-          stop = true;
-          bad = true;
-        }
-      }
-      q.dprev = dn;
-      q.k += 1;
-      if (stop) {
-        q.done = 1;
-        if (bad) {
-          st.ir_fb = 1;
-          st.ir_fallbacks += 1;
-        }
-      }
-    }
-    if (!q.done) atomicOr(&more, 1);
-    if (st.ir_fb) atomicOr(&fb, 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    b.sh.ir_more[0] = more;
-    b.sh.ir_more[1] = fb;
-    if (sweep) b.sh.ir_more[2] += 1;
-    if (use_h) cudaGraphSetConditional(h, more ? 1u : 0u);
-  }
-}
-
-// The FP64 fallback's condition: a slot whose refinement did not finish.
-__global__ void k_ir_fb_cond(Batch b, cudaGraphConditionalHandle h) {
-  cudaGraphSetConditional(h, b.sh.ir_more[1] ? 1u : 0u);
-}
-
-// The FP64 fallback's right-hand side: P = the saved Newton right-hand side
-// (b: the fallback's view, so only structures with ir_fb are active);
-// ir_more[3] counts the fallbacks run.
-__global__ void k_ir_restore(Batch b) {
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) b.sh.ir_more[3] += 1;
-  const int z = blockIdx.y, s = b.sh.wide_structs[z];
-  if (!wide_active(b, s)) return;
-  const StructInfo& inf = b.info[s];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < inf.n_free; i += gridDim.x * blockDim.x)
-    b.P[inf.dof_off + i] = b.sh.ir_rhs[inf.dof_off + i];
 }
 
 void launch_wide_zero(const Batch& b, cudaStream_t st) {
@@ -1326,26 +1037,25 @@ static int trsm_rest_blocks(const Batch& b) {
   const int kl = b.sh.max_kl, rb = b.sh.tiles.trsm_rb;
   return kl > NB ? (kl - NB + rb - 1) / rb : 0;
 }
-template <typename F, int RB>
+template <int RB>
 static void trsm_at(const Batch& b, int p, int row0, int nblk, cudaStream_t st) {
-  k_wb_trsm<F, RB><<<dim3(2 * nblk, b.sh.n_wide), 32 * RB, 0, st>>>(b, p, row0, nblk);
+  k_wb_trsm<RB><<<dim3(2 * nblk, b.sh.n_wide), 32 * RB, 0, st>>>(b, p, row0, nblk);
 }
 // rows row0 .. of panel p (and as many columns) in nblk CTAs of rb rows
-template <typename F>
 static void launch_trsm(const Batch& b, int p, int row0, int nblk, int rb, cudaStream_t st) {
   switch (rb) {
-    case 1: trsm_at<F, 1>(b, p, row0, nblk, st); break;
-    case 2: trsm_at<F, 2>(b, p, row0, nblk, st); break;
-    case 4: trsm_at<F, 4>(b, p, row0, nblk, st); break;
-    case 16: trsm_at<F, 16>(b, p, row0, nblk, st); break;
-    default: trsm_at<F, 8>(b, p, row0, nblk, st); break;
+    case 1: trsm_at<1>(b, p, row0, nblk, st); break;
+    case 2: trsm_at<2>(b, p, row0, nblk, st); break;
+    case 4: trsm_at<4>(b, p, row0, nblk, st); break;
+    case 16: trsm_at<16>(b, p, row0, nblk, st); break;
+    default: trsm_at<8>(b, p, row0, nblk, st); break;
   }
 }
-template <typename F> static void launch_trsm_first(const Batch& b, int p, cudaStream_t st) {
-  launch_trsm<F>(b, p, 0, trsm_first_blocks(b), b.sh.tiles.trsm_first, st);
+static void launch_trsm_first(const Batch& b, int p, cudaStream_t st) {
+  launch_trsm(b, p, 0, trsm_first_blocks(b), b.sh.tiles.trsm_first, st);
 }
-template <typename F> static void launch_trsm_rest(const Batch& b, int p, cudaStream_t st) {
-  launch_trsm<F>(b, p, NB, trsm_rest_blocks(b), b.sh.tiles.trsm_rb, st);
+static void launch_trsm_rest(const Batch& b, int p, cudaStream_t st) {
+  launch_trsm(b, p, NB, trsm_rest_blocks(b), b.sh.tiles.trsm_rb, st);
 }
 static void launch_corner(const Batch& b, int p, cudaStream_t st) {
   const int nw = b.sh.n_wide;
@@ -1354,15 +1064,15 @@ static void launch_corner(const Batch& b, int p, cudaStream_t st) {
 }
 // the triangular solves of panel p: rows of tiles.sub_rows per CTA, nrhs
 // right-hand sides
-template <typename F> static void launch_fwd(const Batch& b, int p, int nrhs, cudaStream_t st) {
+static void launch_fwd(const Batch& b, int p, int nrhs, cudaStream_t st) {
   const int sr = b.sh.tiles.sub_rows, kl = b.sh.max_kl, nb = kl > 0 ? (kl + sr - 1) / sr : 1;
-  if (sr == 32) k_wb_fwd<F, 32><<<dim3(nb, b.sh.n_wide, nrhs), 128, 0, st>>>(b, p);
-  else k_wb_fwd<F, 64><<<dim3(nb, b.sh.n_wide, nrhs), 256, 0, st>>>(b, p);
+  if (sr == 32) k_wb_fwd<32><<<dim3(nb, b.sh.n_wide, nrhs), 128, 0, st>>>(b, p);
+  else k_wb_fwd<64><<<dim3(nb, b.sh.n_wide, nrhs), 256, 0, st>>>(b, p);
 }
-template <typename F> static void launch_bwd(const Batch& b, int p, int nrhs, cudaStream_t st) {
+static void launch_bwd(const Batch& b, int p, int nrhs, cudaStream_t st) {
   const int sr = b.sh.tiles.sub_rows, kl = b.sh.max_kl, nb = kl > 0 ? (kl + sr - 1) / sr : 1;
-  if (sr == 32) k_wb_bwd<F, 32><<<dim3(nb, b.sh.n_wide, nrhs), 128, 0, st>>>(b, p);
-  else k_wb_bwd<F, 64><<<dim3(nb, b.sh.n_wide, nrhs), 256, 0, st>>>(b, p);
+  if (sr == 32) k_wb_bwd<32><<<dim3(nb, b.sh.n_wide, nrhs), 128, 0, st>>>(b, p);
+  else k_wb_bwd<64><<<dim3(nb, b.sh.n_wide, nrhs), 256, 0, st>>>(b, p);
 }
 
 // Panel loop with lookahead on three helper streams (fork / join by events,
@@ -1406,66 +1116,13 @@ static void launch_wb_update(const Batch& b, int p, int part, cudaStream_t st) {
   }
 }
 
-// Panel-loop control inside a captured pass: the counter's start value,
-// and the step at the end of each loop body, which also sets the loop's
-// condition (continue while the counter stays in [0, limit)).
-__global__ void k_wb_loop_set(int* counter, int v) { *counter = v; }
-__global__ void k_wb_loop_step(int* counter, int step, int limit, cudaGraphConditionalHandle h) {
-  const int c = *counter + step;
-  *counter = c;
-  cudaGraphSetConditional(h, (c >= 0 && c < limit) ? 1u : 0u);
-}
-
 namespace {
-// A conditional handle on the graph that st captures into, its value reset
-// to dflt at every launch of the graph.
-cudaError_t make_cond(cudaStream_t st, cudaGraphConditionalHandle* h, unsigned dflt) {
-  cudaStreamCaptureStatus cs;
-  cudaGraph_t g = nullptr;
-  cudaError_t e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, nullptr, nullptr, nullptr);
-  if (e != cudaSuccess) return e;
-  return cudaGraphConditionalHandleCreate(h, g, dflt, cudaGraphCondAssignDefault);
-}
-
-// Appends a conditional node of the given type on handle h to the capture
-// of st and returns its body graph, into which the caller captures the body.
-cudaError_t add_cond(cudaStream_t st, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type,
-                     cudaGraph_t* body) {
-  cudaStreamCaptureStatus cs;
-  cudaGraph_t g = nullptr;
-  const cudaGraphNode_t* deps = nullptr;
-  size_t nd = 0;
-  cudaError_t e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, nullptr, &nd);
-  if (e != cudaSuccess) return e;
-  std::vector<cudaGraphNode_t> dv(deps, deps + nd);
-  cudaGraphNodeParams np{};
-  np.type = cudaGraphNodeTypeConditional;
-  np.conditional.handle = h;
-  np.conditional.type = type;
-  np.conditional.size = 1;
-  cudaGraphNode_t node;
-  if ((e = cudaGraphAddNode(&node, g, dv.data(), nullptr, dv.size(), &np)) != cudaSuccess) return e;
-  *body = np.conditional.phGraph_out[0];
-  return cudaStreamUpdateCaptureDependencies(st, &node, nullptr, 1, cudaStreamSetCaptureDependencies);
-}
-
-// A WHILE node whose condition starts at 1 on every launch.
-cudaError_t add_while(cudaStream_t st, cudaGraphConditionalHandle* h, cudaGraph_t* body) {
-  cudaError_t e = make_cond(st, h, 1);
-  return e != cudaSuccess ? e : add_cond(st, *h, cudaGraphCondTypeWhile, body);
-}
-
-// The trailing update of panel p in the factor's type (FP64: launch_wb_update
-// with the batch's choice of kernel; FP32: k_wb_update32, the corner as its
-// single tile).
-void wb_update(const Batch& b, int p, int part, cudaStream_t st, double*) { launch_wb_update(b, p, part, st); }
-
 // The next panel's diagonal LU, one CTA per structure on the lookahead's
 // critical path, launched at the device's highest stream priority: the
 // block scheduler then gives it the first free SM ahead of the trailing
 // update's and the helper streams' CTAs (a captured launch keeps the
 // priority as a node attribute).
-template <typename F> void launch_diag(const Batch& b, int p, cudaStream_t st) {
+void launch_diag(const Batch& b, int p, cudaStream_t st) {
   static const int prio = [] {
     int lo = 0, hi = 0;
     return cudaDeviceGetStreamPriorityRange(&lo, &hi) == cudaSuccess ? hi : 0;
@@ -1479,140 +1136,51 @@ template <typename F> void launch_diag(const Batch& b, int p, cudaStream_t st) {
   at[0].val.priority = prio;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_wb_diag<F>, b, p);
-}
-void wb_update(const Batch& b, int p, int part, cudaStream_t st, float*) {
-  const int t = part == 1 ? 1 : (b.sh.max_kl + U32T - 1) / U32T;
-  k_wb_update32<<<dim3(t, t, b.sh.n_wide), 256, 0, st>>>(b, p, part);
+  cudaLaunchKernelEx(&cfg, k_wb_diag, b, p);
 }
 }  // namespace
 
-// The panel loops as two graph-resident WHILE loops (forward: factor and
-// forward substitution, one panel per iteration; backward substitution, last
-// panel first), used when a served wave's pass is captured: the pass graph
-// then holds a dozen nodes whatever the panel count, instead of six launches
-// per panel, and instantiates in a millisecond even while other waves run
-// (a graph of thousands of launches took hundreds of milliseconds then, and
-// held up the server's other CUDA calls).  One iteration keeps the
-// lookahead of the launched form (next panel's diagonal LU and this panel's
-// forward step beside the trailing update); it ends with the counter step.
-// Each iteration costs a few microseconds more than the unrolled panel
-// sequence, so the batch path, which captures once on an idle device, keeps
-// the unrolled form.  F: the factor's type.
-template <typename F>
-static cudaError_t capture_wide_loops(const Batch& b, cudaStream_t st) {
-  const ShellData& sd = b.sh;
-  const int nw = sd.n_wide, mr = sd.max_kl, P = sd.max_panels;
-  const int nrest = trsm_rest_blocks(b);
-  (void)mr;
-  cudaStream_t sb = sd.aux[2], s2 = sd.aux[0], s3 = sd.aux[1], s4 = sd.aux[3];
-  cudaEvent_t e_start = sd.evt[0], e_trsm = sd.evt[1], e_corner = sd.evt[2], e_diag = sd.evt[3], e_fwd = sd.evt[4],
-              e_rest = sd.evt[5];
-  if (P <= 0) return cudaSuccess;
-  cudaError_t e;
-  cudaGraphConditionalHandle h;
-  cudaGraph_t body, done;
-  k_wb_loop_set<<<1, 1, 0, st>>>(sd.panel, 0);
-  k_wb_diag<F><<<nw, DIAG_THREADS, 0, st>>>(b, 0);
-  if ((e = add_while(st, &h, &body)) != cudaSuccess) return e;
-  if ((e = cudaStreamBeginCaptureToGraph(sb, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
-    return e;
-  if (nrest) {
-    cudaEventRecord(e_start, sb);
-    cudaStreamWaitEvent(s4, e_start, 0);
-    launch_trsm_rest<F>(b, -1, s4);
-    cudaEventRecord(e_rest, s4);
-  }
-  launch_trsm_first<F>(b, -1, sb);
-  wb_update(b, -1, 1, sb, (F*)nullptr);
-  cudaEventRecord(e_corner, sb);
-  cudaStreamWaitEvent(s2, e_corner, 0);
-  launch_diag<F>(b, -2, s2);
-  cudaEventRecord(e_diag, s2);
-  if (nrest) cudaStreamWaitEvent(sb, e_rest, 0);
-  cudaEventRecord(e_trsm, sb);
-  cudaStreamWaitEvent(s3, e_trsm, 0);
-  launch_fwd<F>(b, -1, 1, s3);
-  cudaEventRecord(e_fwd, s3);
-  wb_update(b, -1, 2, sb, (F*)nullptr);
-  cudaStreamWaitEvent(sb, e_diag, 0);
-  cudaStreamWaitEvent(sb, e_fwd, 0);
-  k_wb_loop_step<<<1, 1, 0, sb>>>(sd.panel, 1, P, h);
-  if ((e = cudaStreamEndCapture(sb, &done)) != cudaSuccess) return e;
-  k_wb_loop_set<<<1, 1, 0, st>>>(sd.panel, P - 1);
-  if ((e = add_while(st, &h, &body)) != cudaSuccess) return e;
-  if ((e = cudaStreamBeginCaptureToGraph(sb, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
-    return e;
-  launch_bwd<F>(b, -1, 1, sb);
-  k_wb_loop_step<<<1, 1, 0, sb>>>(sd.panel, -1, P, h);
-  return cudaStreamEndCapture(sb, &done);
-}
-
-// The first error of a wide-band capture step on this thread (a failed
-// conditional node or body capture), which the capturing caller reports:
-// capture_error() returns it and clears it.
-static thread_local cudaError_t g_capture_error = cudaSuccess;
-static void capture_fail(cudaError_t e) {
-  if (e != cudaSuccess && g_capture_error == cudaSuccess) g_capture_error = e;
-}
-cudaError_t wide_capture_error() {
-  const cudaError_t e = g_capture_error;
-  g_capture_error = cudaSuccess;
-  return e;
-}
-
-// Factor and solve in the factor's type F: FP64, the LU in place of K_AA
-// and the solve on P; FP32 (mixed path), the LU in wband32 and the solve on
-// r32.  Inside a served wave's capture the panel loops are graph loops
-// (capture_wide_loops), else one launch sequence per panel with lookahead.
-template <typename F>
+// Factor and solve, one launch sequence per panel with lookahead: the LU in place
+// of K_AA, the solution in P.
 static void wide_factor_solve(const Batch& b, cudaStream_t st, LaunchProf* prof) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (!prof && b.sh.loops_in_graph && b.sh.panel && cudaStreamIsCapturing(st, &cs) == cudaSuccess &&
-      cs == cudaStreamCaptureStatusActive) {
-    capture_fail(capture_wide_loops<F>(b, st));
-    return;
-  }
   const ShellData& sd = b.sh;
   const int nw = sd.n_wide;
-  const int mr = sd.max_kl;  // largest kl over the wide structures
   const int nrest = trsm_rest_blocks(b);
-  (void)mr;
-  cudaStream_t s2 = sd.aux[0], s3 = sd.aux[1], s4 = sd.aux[3];
+  cudaStream_t s2 = sd.aux[0], s3 = sd.aux[1], s4 = sd.aux[2];
   // the helpers fork from the main stream at their first wait and join it
   // again before the backward substitution
   cudaEvent_t e_start = sd.evt[0], e_trsm = sd.evt[1], e_corner = sd.evt[2], e_diag = sd.evt[3], e_fwd = sd.evt[4],
               e_rest = sd.evt[5];
-  { ProfScope q(prof, st, KC_WIDE_DIAG); k_wb_diag<F><<<nw, DIAG_THREADS, 0, st>>>(b, 0); }
+  { ProfScope q(prof, st, KC_WIDE_DIAG); k_wb_diag<<<nw, DIAG_THREADS, 0, st>>>(b, 0); }
   for (int p = 0; p < sd.max_panels; ++p) {
     bool next = p + 1 < sd.max_panels;
     if (nrest) {
       cudaEventRecord(e_start, st);
       cudaStreamWaitEvent(s4, e_start, 0);
       ProfScope q(prof, s4, KC_WIDE_TRSM);
-      launch_trsm_rest<F>(b, p, s4);
+      launch_trsm_rest(b, p, s4);
       cudaEventRecord(e_rest, s4);
     }
     {
       ProfScope q(prof, st, KC_WIDE_TRSM);
-      launch_trsm_first<F>(b, p, st);
+      launch_trsm_first(b, p, st);
     }
     if (next) {
-      { ProfScope q(prof, st, KC_WIDE_UPDATE); wb_update(b, p, 1, st, (F*)nullptr); }
+      { ProfScope q(prof, st, KC_WIDE_UPDATE); launch_wb_update(b, p, 1, st); }
       cudaEventRecord(e_corner, st);
       cudaStreamWaitEvent(s2, e_corner, 0);
-      { ProfScope q(prof, s2, KC_WIDE_DIAG); launch_diag<F>(b, p + 1, s2); }
+      { ProfScope q(prof, s2, KC_WIDE_DIAG); launch_diag(b, p + 1, s2); }
       cudaEventRecord(e_diag, s2);
     }
     if (nrest) cudaStreamWaitEvent(st, e_rest, 0);
     cudaEventRecord(e_trsm, st);
     cudaStreamWaitEvent(s3, e_trsm, 0);
-    { ProfScope q(prof, s3, KC_WIDE_SUBST); launch_fwd<F>(b, p, 1, s3); }
+    { ProfScope q(prof, s3, KC_WIDE_SUBST); launch_fwd(b, p, 1, s3); }
     if (next) {
-      { ProfScope q(prof, st, KC_WIDE_UPDATE); wb_update(b, p, 2, st, (F*)nullptr); }
+      { ProfScope q(prof, st, KC_WIDE_UPDATE); launch_wb_update(b, p, 2, st); }
       cudaStreamWaitEvent(st, e_diag, 0);
     } else {
-      { ProfScope q(prof, st, KC_WIDE_UPDATE); wb_update(b, p, 0, st, (F*)nullptr); }
+      { ProfScope q(prof, st, KC_WIDE_UPDATE); launch_wb_update(b, p, 0, st); }
     }
   }
   // join: every forward step is done before the backward substitution
@@ -1620,103 +1188,12 @@ static void wide_factor_solve(const Batch& b, cudaStream_t st, LaunchProf* prof)
   cudaStreamWaitEvent(st, e_fwd, 0);
   for (int p = sd.max_panels - 1; p >= 0; --p) {
     ProfScope q(prof, st, KC_WIDE_SUBST);
-    launch_bwd<F>(b, p, 1, st);
-  }
-}
-
-// One refinement sweep of the mixed path: the FP64 residual into r32, the
-// FP32 forward and backward substitution with the FP32 LU (one launch per
-// panel), x += d and the check, which sets the refinement loop's condition
-// h when use_h.  (Served waves, whose passes hold the panel loops as graph
-// loops, are built with the FP64 options and never refine.)
-static void ir_sweep(const Batch& b, cudaStream_t st, cudaGraphConditionalHandle h, int use_h, LaunchProf* prof) {
-  const ShellData& sd = b.sh;
-  const int nw = sd.n_wide, P = sd.max_panels;
-  const int rows = (P * NB + 255) / 256;
-  { ProfScope q(prof, st, KC_WIDE_REFINE); k_ir_residual<<<dim3(rows, nw), 256, 0, st>>>(b); }
-  for (int p = 0; p < P; ++p) {
-    ProfScope q(prof, st, KC_WIDE_SUBST);
-    launch_fwd<float>(b, p, 1, st);
-  }
-  for (int p = P - 1; p >= 0; --p) {
-    ProfScope q(prof, st, KC_WIDE_SUBST);
-    launch_bwd<float>(b, p, 1, st);
-  }
-  {
-    ProfScope q(prof, st, KC_WIDE_REFINE);
-    k_ir_correct<<<dim3(2 * 152, nw), 256, 0, st>>>(b, 0);
-    k_ir_check<<<1, 128, 0, st>>>(b, h, use_h, 1);
-  }
-}
-
-// Mixed precision (GF_PREC_MIXED): the FP32 LU of K_AA, its solve, then FP64
-// iterative refinement against the FP64 K_AA until the corrections stop
-// shrinking; a structure whose refinement does not reach the FP64 level is
-// solved again by the FP64 LU.  Inside a captured pass the refinement loop
-// is a WHILE node and the fallback an IF node, so the pass needs no host
-// round trip; otherwise the host reads the loop's flags after each sweep.
-static void wide_solve_mixed(const Batch& b, cudaStream_t st, LaunchProf* prof) {
-  const ShellData& sd = b.sh;
-  const int nw = sd.n_wide;
-  Batch fb = b;  // the FP64 fallback's view
-  fb.sh.fp64_pass = 1;
-  { ProfScope q(prof, st, KC_WIDE_REFINE); k_ir_begin<<<dim3(4 * 152, nw), 256, 0, st>>>(b); }
-  wide_factor_solve<float>(b, st, prof);
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  const bool capturing = !prof && cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive;
-  if (capturing) {
-    // the bodies are captured on aux[4], which the pass's capture has not
-    // forked into; a failed step is recorded for the capturing caller
-    cudaStream_t sr = sd.aux[4];
-    cudaGraphConditionalHandle h, hf;
-    cudaGraph_t body, done;
-    cudaError_t e;
-    if ((e = make_cond(st, &h, 0)) != cudaSuccess) return capture_fail(e);
-    k_ir_correct<<<dim3(2 * 152, nw), 256, 0, st>>>(b, 1);
-    k_ir_check<<<1, 128, 0, st>>>(b, h, 1, 0);
-    if ((e = add_cond(st, h, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return capture_fail(e);
-    if ((e = cudaStreamBeginCaptureToGraph(sr, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
-        cudaSuccess)
-      return capture_fail(e);
-    ir_sweep(b, sr, h, 1, nullptr);
-    if ((e = cudaStreamEndCapture(sr, &done)) != cudaSuccess) return capture_fail(e);
-    if ((e = make_cond(st, &hf, 0)) != cudaSuccess) return capture_fail(e);
-    k_ir_fb_cond<<<1, 1, 0, st>>>(b, hf);
-    if ((e = add_cond(st, hf, cudaGraphCondTypeIf, &body)) != cudaSuccess) return capture_fail(e);
-    if ((e = cudaStreamBeginCaptureToGraph(sr, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
-        cudaSuccess)
-      return capture_fail(e);
-    k_ir_restore<<<dim3(2 * 152, nw), 256, 0, sr>>>(fb);
-    launch_front_solve(fb, sr);
-    if ((e = cudaStreamEndCapture(sr, &done)) != cudaSuccess) return capture_fail(e);
-    return;
-  }
-  {
-    ProfScope q(prof, st, KC_WIDE_REFINE);
-    k_ir_correct<<<dim3(2 * 152, nw), 256, 0, st>>>(b, 1);
-    k_ir_check<<<1, 128, 0, st>>>(b, 0, 0, 0);
-  }
-  int more[2] = {0, 0};
-  for (int k = 0; k <= sd.ir_max; ++k) {
-    if (cudaMemcpyAsync(more, sd.ir_more, sizeof(more), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess || !more[0])
-      break;
-    ir_sweep(b, st, 0, 0, prof);
-  }
-  if (cudaMemcpyAsync(more, sd.ir_more, sizeof(more), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return;
-  if (more[1]) {
-    k_ir_restore<<<dim3(2 * 152, nw), 256, 0, st>>>(fb);
-    launch_front_solve(fb, st, prof);
+    launch_bwd(b, p, 1, st);
   }
 }
 
 void launch_wide_solve(const Batch& b, cudaStream_t st, LaunchProf* prof) {
-  if (b.sh.n_wide == 0) return;
-  if (b.mixed && b.sh.wband32) wide_solve_mixed(b, st, prof);
-  else if (b.sh.mf.sched) launch_front_solve(b, st, prof);
-  else wide_factor_solve<double>(b, st, prof);
+  if (b.sh.n_wide) wide_factor_solve(b, st, prof);
 }
 
 // Forward and backward substitution alone on a wide band that already holds
@@ -1725,37 +1202,8 @@ void launch_wide_solve(const Batch& b, cudaStream_t st, LaunchProf* prof) {
 // launch_wide_solve without the factor, every column per launch.
 void launch_wide_subst(const Batch& b, int nrhs, cudaStream_t st) {
   if (b.sh.n_wide == 0 || nrhs <= 0) return;
-  for (int p = 0; p < b.sh.max_panels; ++p) launch_fwd<double>(b, p, nrhs, st);
-  for (int p = b.sh.max_panels - 1; p >= 0; --p) launch_bwd<double>(b, p, nrhs, st);
-}
-
-// Launches of the panel loops: unrolled, the first diagonal LU, then per
-// panel the first trsm blocks, update corner + next diagonal, the other trsm
-// blocks, forward step, update rest, backward step (the last panel has no
-// corner or next diagonal); graph loops, two loop-control kernels, the first
-// diagonal LU, the same six or seven kernels and a counter step per forward
-// iteration, and two kernels per backward one; the FP64 tensor-core update
-// adds its slicing kernel per panel.
-static int wide_factor_launches(const Batch& b, bool fp64) {
-  const int P = b.sh.max_panels, per = 6 + (trsm_rest_blocks(b) ? 1 : 0);
-  return (b.sh.loops_in_graph ? 3 + (per + 2) * P : 1 + per * P - 2) + (fp64 && b.sh.wide_tc ? P : 0);
-}
-
-// Per Newton pass; the mixed path adds its start, first correction and
-// check and the fallback's condition, and its sweeps and fallbacks come on
-// top (wide_refine_launches).
-int wide_launches_per_pass(const Batch& b) {
-  if (!b.sh.n_wide) return 0;
-  if (b.mixed && b.sh.wband32) return wide_factor_launches(b, false) + 4;
-  return b.sh.mf.sched ? front_launches(b) : wide_factor_launches(b, true);
-}
-
-// Launches of `sweeps` refinement sweeps (residual, forward and backward
-// substitution, correction, check) and `fallbacks` FP64 fallbacks.
-long long wide_refine_launches(const Batch& b, long long sweeps, long long fallbacks) {
-  const int P = b.sh.max_panels;
-  const long long per_sweep = 3 + 2 * P;
-  return sweeps * per_sweep + fallbacks * (1 + front_launches(b));
+  for (int p = 0; p < b.sh.max_panels; ++p) launch_fwd(b, p, nrhs, st);
+  for (int p = b.sh.max_panels - 1; p >= 0; --p) launch_bwd(b, p, nrhs, st);
 }
 
 }  // namespace gf

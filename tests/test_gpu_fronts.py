@@ -173,3 +173,26 @@ def test_a_zero_pivot_is_reported(gpu_ctx, at):
     ab[at, 2 * kl] = 0.0
     _, info = gpu_ctx.band_solve(ab, kl, kl, np.ones(n))
     assert info == 1
+
+
+@pytest.mark.parametrize("make", [
+    lambda: configs.square_plate(1, steps=2), lambda: strip(12, 3), lambda: two_plates(2, 5), lambda: loaded(9),
+    lambda: configs.square_plate(13, steps=2),
+], ids=["plate1", "strip12x3", "two", "loaded9", "plate13"])
+def test_mixed_fronts_refine_to_the_fp64_solve(gpu_ctx, make):
+    """The FP32 fronts' forward and backward sweeps against the element
+    matrices' residual (and the nodal load stiffness'): the FP64 path's counts
+    and, refined to the FP64 floor, its states to 1e-10 of the displacement
+    scale, every solve without the FP64 fallback."""
+    run = {}
+    for p in (gpu.GF_PREC_MIXED, gpu.GF_PREC_FP64):
+        b = gpu.BatchSolver(gpu_ctx, [make()], gpu_ctx.opts(precision=p))
+        b.reset()
+        b.run()
+        run[p] = b.results() + (b.solve_stats(),)
+        b.close()
+    (fm, sm, em), (ff, sf, _) = run[gpu.GF_PREC_MIXED], run[gpu.GF_PREC_FP64]
+    assert np.array_equal(sm, sf)
+    scale = np.abs(ff[0][:, :3] - make().nodes).max()
+    assert np.abs(fm[0][:, :3] - ff[0][:, :3]).max() <= 1e-10 * scale
+    assert em[0][2] == 0 and em[0][1] >= em[0][0] > 0
