@@ -61,7 +61,16 @@ template <typename T> __device__ __forceinline__ void mf_fail(const Batch& b, in
   if (sizeof(T) == 8) b.state[s].info_fail = 1;
   else b.state[s].ir_fb = 1;
 }
-template <typename T> __device__ __forceinline__ bool mf_bad(T p) { return !(p != T(0)) || !isfinite(p); }
+// Zero, infinite or NaN, from the bits: an FP64 comparison would hold the pivot's
+// chain up for 64 cycles.
+__device__ __forceinline__ bool mf_bad(double p) {
+  const int h = __double2hiint(p) & 0x7FFFFFFF;
+  return (h | __double2loint(p)) == 0 || h >= 0x7FF00000;
+}
+__device__ __forceinline__ bool mf_bad(float p) {
+  const int h = __float_as_int(p) & 0x7FFFFFFF;
+  return h == 0 || h >= 0x7F800000;
+}
 
 // Index of elimination position q in front F (own DOFs, then the boundary).
 __device__ __forceinline__ int mf_local(const FrontData& d, const Front& F, int q) {
@@ -127,9 +136,22 @@ template <typename T> __global__ void k_mf_elements(Batch b, int color) {
   const double* K = b.sh.Ke + (int64_t)e * 729;
   const int* map = b.sh.mf.map + (int64_t)e * 729;
   T* F = reinterpret_cast<T*>(b.sh.mf.F) + b.sh.mf.base[s];
-  for (int x = lane; x < 729; x += 32) {
-    const int to = map[x];
-    if (to >= 0) F[to] += (T)K[x];
+  // twelve entries in flight a lane (one at a time: 17 us a colour for 6)
+#pragma unroll 1
+  for (int x0 = lane; x0 < 729; x0 += 12 * 32) {
+    int to[12];
+    T k[12], f[12];
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {
+      const int x = x0 + 32 * q;
+      to[q] = x < 729 ? map[x] : -1;
+      k[q] = x < 729 ? (T)K[x] : T(0);
+    }
+#pragma unroll
+    for (int q = 0; q < 12; ++q) f[q] = to[q] >= 0 ? F[to[q]] : T(0);
+#pragma unroll
+    for (int q = 0; q < 12; ++q)
+      if (to[q] >= 0) F[to[q]] = f[q] + k[q];
   }
 }
 
@@ -172,40 +194,80 @@ template <typename T> __global__ void k_mf_out(Batch b) {
     P[i] = mf_x<T>(b)[b.sh.mf.pos[inf.dof_off + i]];
 }
 
-// Extend-add: sixteen columns of a child's Schur complement (and right-hand
-// side) into its parent, a warp per column.
+// Extend-add: eight columns of a large front with its children's Schur
+// complements, a warp per column, two children at a time (the small fronts gather
+// theirs as they load).
 template <typename T> __global__ void __launch_bounds__(256) k_mf_extend(Batch b, int job0) {
   const FrontData& d = b.sh.mf;
   const int2 job = d.ext_jobs[job0 + blockIdx.x];
-  const Front C = d.fronts[job.x];
-  if (!mf_active(b, C.slot)) return;
-  const Front P = d.fronts[C.parent];
-  const int u = C.f - C.s, lane = threadIdx.x & 31;
-  const int* rel = d.rel + C.rel;
-  const T* S = mf_mat<T>(b, C);
-  T* Q = mf_mat<T>(b, P);
-  for (int j = job.y + (threadIdx.x >> 5); j < min(job.y + 16, u + 1); j += 8) {
-    const T* sc = S + (int64_t)(C.s + j) * C.ld + C.s;
-    T* qc = Q + (int64_t)(j < u ? rel[j] : P.f) * P.ld;
-    for (int i = lane; i < u; i += 32) qc[rel[i]] += sc[i];
+  const Front F = d.fronts[job.x];
+  if (!mf_active(b, F.slot)) return;
+  const int lane = threadIdx.x & 31, j = job.y + (threadIdx.x >> 5), kid1 = F.kid1;
+  if (j > F.f) return;
+  T* g = mf_mat<T>(b, F) + (int64_t)j * F.ld;
+  for (int k = F.kid0; k < kid1; k += 2) {
+    const int* inv[2];
+    const T* sc[2];
+    bool on[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int2 kid = d.kids[min(k + q, kid1 - 1)];
+      const Front& C = d.fronts[kid.x];
+      inv[q] = d.inv + kid.y;
+      const int cj = j < F.f ? inv[q][j] : C.f - C.s;
+      on[q] = cj >= 0 && k + q < kid1;
+      sc[q] = reinterpret_cast<const T*>(d.F) + C.off + C.s + (int64_t)(C.s + cj) * C.ld;
+    }
+    if (!on[0] && !on[1]) continue;
+#pragma unroll 4
+    for (int i = lane; i < F.f; i += 32) {
+      const int c0 = on[0] ? inv[0][i] : -1, c1 = on[1] ? inv[1][i] : -1;
+      if (c0 < 0 && c1 < 0) continue;
+      T v = g[i];
+      if (c0 >= 0) v += sc[0][c0];
+      if (c1 >= 0) v += sc[1][c1];
+      g[i] = v;
+    }
   }
 }
 
-// Partial LU of a front held in shared memory, s pivots, one CTA: the pivot
-// warp (warp 3) owns column k + 1 at step k (its update, the next pivot's
-// reciprocal and multipliers) while the others update the rest of the trailing
-// block, packed densely over their lanes; one barrier closes the step.  Many
-// CTAs share an SM, so one front's pivot chain runs beside another's updates.
-constexpr int MF_SMALL_THREADS = 128;
+// Partial LU of a front held in shared memory, s pivots, one CTA: the front and its
+// children's Schur complements are summed as they load, then warp 3, the pivot
+// warp, owns column k + 1 at step k (its update, the next pivot's reciprocal and
+// multipliers) while the others update the rest of the trailing block, packed
+// densely over their lanes; one barrier closes the step.  Bound by its SM's FP64
+// rate, for which one CTA needs two warps a sub-partition (f = 87, s = 15, a CTA an
+// SM: four warps 80 us, eight 50).
+constexpr int MF_SMALL_THREADS = 256;
 template <typename T> __global__ void __launch_bounds__(MF_SMALL_THREADS) k_mf_small(Batch b, int off) {
   const FrontData& d = b.sh.mf;
-  const Front F = d.fronts[d.list[off + blockIdx.x]];
+  const Front F = d.list[off + blockIdx.x];
   if (!mf_active(b, F.slot)) return;
   extern __shared__ __align__(16) unsigned char mf_raw[];
   T* A = reinterpret_cast<T*>(mf_raw);
   const int f = F.f, s = F.s, ld = F.ld, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int WARPS = MF_SMALL_THREADS / 32;
   T* G = mf_mat<T>(b, F);
   for (int x = tid; x < ld * (f + 1); x += MF_SMALL_THREADS) A[x] = G[x];
+  for (int k = F.kid0; k < F.kid1; ++k) {
+    const int2 kid = d.kids[k];
+    const int* inv = d.inv + kid.y;
+    const Front& C = d.fronts[kid.x];
+    const int u = C.f - C.s, cld = C.ld;
+    const T* S = reinterpret_cast<const T*>(d.F) + C.off + C.s + (int64_t)C.s * cld;
+    int ci[MF_SMALL / 32];
+#pragma unroll
+    for (int q = 0; q < MF_SMALL / 32; ++q) ci[q] = lane + 32 * q < f ? inv[lane + 32 * q] : -1;
+    __syncthreads();  // A is complete, or holds the child before
+#pragma unroll 2
+    for (int j = warp; j <= f; j += WARPS) {
+      const int cj = j < f ? inv[j] : u;
+      if (cj < 0) continue;
+#pragma unroll
+      for (int q = 0; q < MF_SMALL / 32; ++q)
+        if (ci[q] >= 0) A[lane + 32 * q + j * ld] += S[ci[q] + (int64_t)cj * cld];
+    }
+  }
   __syncthreads();
   bool bad = false;
   auto pivot = [&](int k) {  // reciprocal and multipliers of column k
@@ -227,10 +289,10 @@ template <typename T> __global__ void __launch_bounds__(MF_SMALL_THREADS) k_mf_s
       __syncwarp();
       pivot(k + 1);
     } else if (m > 0) {
-      const int c0 = next ? k + 2 : k + 1, nt = next ? 96 : 128;
+      const int c0 = next ? k + 2 : k + 1, nt = MF_SMALL_THREADS - (next ? 32 : 0);
       const int tot = m * (f + 1 - c0);
       const float inv_m = 1.0f / (float)m;
-      for (int e = tid; e < tot; e += nt) {
+      for (int e = next && warp > 3 ? tid - 32 : tid; e < tot; e += nt) {
         const int jj = __float2int_rz(((float)e + 0.5f) * inv_m);  // e / m, exact for e < 2^14
         const int i = k + 1 + e - jj * m, j = c0 + jj;
         A[i + j * ld] = mfma(-A[i + k * ld], A[k + j * ld], A[i + j * ld]);
@@ -243,68 +305,81 @@ template <typename T> __global__ void __launch_bounds__(MF_SMALL_THREADS) k_mf_s
 }
 
 // LU of the diagonal block of panel p of the large fronts of a height, one CTA
-// each; as k_mf_small, on the panel's block alone.
-constexpr int MF_DIAG_THREADS = 160;
+// each: a chain of pivots (update of a column, reciprocal, multipliers), 540 cycles
+// each if nothing holds them up.  The pivot warp (warp 3) has a sub-partition to
+// itself; six warps on the other three update the remaining columns, lane i row i,
+// a column at a time (FP64 instructions take their 64 cycles even where a predicate
+// turns every lane off, so the loop ends at the last column; three warps with the
+// columns in registers took 1,120 cycles a pivot, packed lanes 1,150, this 700).
+constexpr int MF_DIAG_THREADS = 224;
 template <typename T> __global__ void __launch_bounds__(MF_DIAG_THREADS) k_mf_diag(Batch b, int off, int p) {
   const FrontData& d = b.sh.mf;
-  const Front F = d.fronts[d.list[off + blockIdx.x]];
-  if (!mf_active(b, F.slot)) return;
+  const Front F = d.list[off + blockIdx.x];
+  const bool on = mf_active(b, F.slot);
+  constexpr int WARPS = MF_DIAG_THREADS / 32;
   const int k0 = p * MF_NB, nb = min(MF_NB, F.s - k0), ld = F.ld, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   T* G = mf_mat<T>(b, F) + k0 + (int64_t)k0 * ld;
   __shared__ T A[MF_NB][MF_NB + 1];  // A[j][i]: column j, row i
-  for (int x = tid; x < nb * MF_NB; x += MF_DIAG_THREADS) {
-    const int i = x % MF_NB, j = x / MF_NB;
-    if (i < nb) A[j][i] = G[i + (int64_t)j * ld];
+#pragma unroll
+  for (int q = 0; q < (MF_NB + WARPS - 1) / WARPS; ++q) {
+    const int j = warp + WARPS * q;
+    if (j < nb) A[j][lane] = lane < nb ? G[lane + (int64_t)j * ld] : T(0);
   }
+  if (!on) return;
   __syncthreads();
   bool bad = false;
+  T a = T(0), l = T(0);
+  // pivot k of the updated column a: lane i keeps the multiplier of row i
   auto pivot = [&](int k) {
-    const T q = A[k][k];
+    const T q = __shfl_sync(0xffffffffu, a, k);
     bad = bad || mf_bad(q);
     const T r = mf_rcp(q);
-    __syncwarp();
-    if (lane > k && lane < nb) A[k][lane] *= r;
+    l = a * r;
+    if (lane > k && lane < nb) A[k][lane] = l;
     if (lane == k) A[k][k] = r;
   };
-  if (warp == 4) pivot(0);
+  if (warp == 3) {
+    a = A[0][lane];
+    pivot(0);
+  }
   __syncthreads();
   for (int k = 0; k + 1 < nb; ++k) {
-    const int m = nb - 1 - k;
-    if (warp == 4) {
-      const T u = A[k + 1][k];
-      if (lane > k && lane < nb) A[k + 1][lane] = mfma(-A[k][lane], u, A[k + 1][lane]);
-      __syncwarp();
+    if (warp == 3) {
+      a = A[k + 1][lane];
+      const T u = __shfl_sync(0xffffffffu, a, k);
+      if (lane > k) a = mfma(-l, u, a);
       pivot(k + 1);
     } else {
-      const int tot = m * (m - 1);
-      const float inv_m = 1.0f / (float)m;
-      for (int e = tid; e < tot; e += 128) {
-        const int jj = __float2int_rz(((float)e + 0.5f) * inv_m);
-        const int i = k + 1 + e - jj * m, j = k + 2 + jj;
-        A[j][i] = mfma(-A[k][i], A[j][k], A[j][i]);
+      const T x = -A[k][lane];
+      for (int j = k + 2 + (warp < 3 ? warp : warp - 1); j < nb; j += WARPS - 1) {
+        const T v = mfma(x, A[j][k], A[j][lane]);
+        if (lane > k) A[j][lane] = v;
       }
     }
     __syncthreads();
   }
-  for (int x = tid; x < nb * MF_NB; x += MF_DIAG_THREADS) {
-    const int i = x % MF_NB, j = x / MF_NB;
-    if (i < nb) G[i + (int64_t)j * ld] = A[j][i];
+#pragma unroll
+  for (int q = 0; q < (MF_NB + WARPS - 1) / WARPS; ++q) {
+    const int j = warp + WARPS * q;
+    if (lane < nb && j < nb) G[lane + (int64_t)j * ld] = A[j][lane];
   }
   if (bad && lane == 0) mf_fail<T>(b, F.slot);
 }
 
-// L21 = A21 U11^-1 (blockIdx.x < nlow: 32 rows below the panel) and U12 =
-// L11^-1 A12 (32 columns right of it, the right-hand side among them).  Four
-// lanes per row (column), lane q holding its entries 4 j + q in registers, the
-// finished entry broadcast within the four: 176 FP64 warp instructions per
-// eight rows (132 with a thread per row, but four times the latency).
-template <typename T> __global__ void __launch_bounds__(128) k_mf_trsm(Batch b, int off, int p, int nlow) {
+// L21 = A21 U11^-1 (blockIdx.x < nlow: the rows below the panel, 128 / L a CTA) and
+// U12 = L11^-1 A12 (the columns right of it, the right-hand side among them).  L
+// lanes per row (column), lane q holding its entries L j + q in registers, the
+// finished entry broadcast within the L: 176 FP64 warp instructions per eight rows
+// with L = 4 (132 with a thread per row, but four times the latency), 80 per two
+// with L = 16, which has half the latency where the rows leave SMs idle.
+template <typename T, int L> __global__ void __launch_bounds__(128) k_mf_trsm(Batch b, int off, int p, int nlow) {
   const FrontData& d = b.sh.mf;
-  const Front F = d.fronts[d.list[off + blockIdx.y]];
-  if (!mf_active(b, F.slot)) return;
+  const Front F = d.list[off + blockIdx.y];
+  const bool on = mf_active(b, F.slot);
   const int k0 = p * MF_NB, nb = min(MF_NB, F.s - k0), k1 = k0 + nb, ld = F.ld, tid = threadIdx.x;
   const bool lower = (int)blockIdx.x < nlow;
-  const int first = k1 + 32 * (lower ? (int)blockIdx.x : (int)blockIdx.x - nlow);
+  constexpr int R = 128 / L, E = MF_NB / L;
+  const int first = k1 + R * (lower ? (int)blockIdx.x : (int)blockIdx.x - nlow);
   if (first >= (lower ? F.f : F.f + 1)) return;
   T* G = mf_mat<T>(b, F);
   __shared__ T U[MF_NB][MF_NB + 1];  // U[k][j]: the factor this side reads, identity beyond nb
@@ -315,29 +390,31 @@ template <typename T> __global__ void __launch_bounds__(128) k_mf_trsm(Batch b, 
     if (lower) U[i][j] = v;  // U11(i, j), the reciprocal on the diagonal
     else U[j][i] = v;        // L11(i, j) at [j][i]
   }
-  const int r = tid >> 2, q = tid & 3, g = first + r;  // row (lower) or column of the front
+  const int r = tid / L, q = tid % L, g = first + r;  // row (lower) or column of the front
   const bool live = g < (lower ? F.f : F.f + 1);
-  T v[8];
+  T v[E];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int c = 4 * j + q;
+  for (int j = 0; j < E; ++j) {
+    const int c = L * j + q;
     v[j] = (live && c < nb) ? (lower ? G[g + (int64_t)(k0 + c) * ld] : G[k0 + c + (int64_t)g * ld]) : T(0);
   }
+  if (!on) return;
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < MF_NB; ++k) {
+    if (k >= nb) break;
     // the finished entry k, from the lane that holds it
-    T x = v[k >> 2];
+    T x = v[k / L];
     if (lower) x *= U[k][k];
-    x = __shfl_sync(0xffffffffu, x, k & 3, 4);
-    if (lower && q == (k & 3)) v[k >> 2] = x;
+    x = __shfl_sync(0xffffffffu, x, k % L, L);
+    if (lower && q == k % L) v[k / L] = x;
 #pragma unroll
-    for (int j = k >> 2; j < 8; ++j)
-      if (4 * j + q > k) v[j] = mfma(-x, U[k][4 * j + q], v[j]);
+    for (int j = k / L; j < E; ++j)
+      if (L * j + q > k) v[j] = mfma(-x, U[k][L * j + q], v[j]);
   }
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int c = 4 * j + q;
+  for (int j = 0; j < E; ++j) {
+    const int c = L * j + q;
     if (!live || c >= nb) continue;
     if (lower) G[g + (int64_t)(k0 + c) * ld] = v[j];
     else G[k0 + c + (int64_t)g * ld] = v[j];
@@ -352,8 +429,8 @@ template <typename T> __global__ void __launch_bounds__(128) k_mf_trsm(Batch b, 
 template <typename T>
 __global__ void __launch_bounds__(128) k_mf_panel(Batch b, int off, int p, int na, int nca, int ncb) {
   const FrontData& d = b.sh.mf;
-  const Front F = d.fronts[d.list[off + blockIdx.y]];
-  if (!mf_active(b, F.slot)) return;
+  const Front F = d.list[off + blockIdx.y];
+  const bool on = mf_active(b, F.slot);
   const int k0 = p * MF_NB, k1 = k0 + MF_NB, ld = F.ld, tid = threadIdx.x;
   if (k1 >= F.s) return;
   int r0, c0, r1, c1;
@@ -386,6 +463,7 @@ __global__ void __launch_bounds__(128) k_mf_panel(Batch b, int off, int p, int n
 #pragma unroll
   for (int q = 0; q < 4; ++q)
     acc[q] = (r0 + i < r1 && c0 + cg + 8 * q < c1) ? G[r0 + i + (int64_t)(c0 + cg + 8 * q) * ld] : T(0);
+  if (!on) return;
   __syncthreads();
 #pragma unroll 8
   for (int k = 0; k < MF_NB; ++k) {
@@ -399,126 +477,195 @@ __global__ void __launch_bounds__(128) k_mf_panel(Batch b, int off, int p, int n
 }
 
 // The Schur complement of the large fronts of a height: C -= L21 U12 over all
-// pivots, 32 x 32 tiles, 2 x 4 outputs per thread, the next 32 pivots' operands
-// loading into registers while this one's products run.
-template <typename T> __global__ void __launch_bounds__(128) k_mf_schur(Batch b, int job0) {
+// pivots, R x R tiles, 2 x 4 (R = 32) or 1 x 2 (16) outputs per thread, the next 32
+// pivots' operands loading into registers while this one's products run.  Bound by
+// the FP64 pipes.
+template <typename T, int R> __global__ void __launch_bounds__(128) k_mf_schur(Batch b, int job0) {
   const FrontData& d = b.sh.mf;
   const int2 job = d.schur_jobs[job0 + blockIdx.x];
   const Front F = d.fronts[job.x];
-  if (!mf_active(b, F.slot)) return;
-  const int r0 = F.s + 32 * (job.y & 0xFFFF), c0 = F.s + 32 * (job.y >> 16), ld = F.ld, s = F.s, tid = threadIdx.x;
+  const bool on = mf_active(b, F.slot);
+  constexpr int H = R / 16, Q = R / 8, N = R / 4;  // row halves, column groups, entries a thread loads
+  const int r0 = F.s + R * (job.y & 0xFFFF), c0 = F.s + R * (job.y >> 16), ld = F.ld, s = F.s, tid = threadIdx.x;
   T* G = mf_mat<T>(b, F);
-  __shared__ T Ls[2][32][33];  // [k][row]
-  __shared__ T Us[2][32][33];  // [column][k]
-  const int lx = tid & 31, ly = tid >> 5;
-  const bool row_ok = r0 + lx < F.f;
-  T lr[8], ur[8];
+  __shared__ T Ls[2][32][R + 1];  // [k][row]
+  __shared__ T Us[2][R][33];      // [column][k]
+  const int lr_ = tid % R, lk = tid / R;      // L: row, pivots lk + (128 / R) q
+  const int uk = tid & 31, uc = tid >> 5;     // U: pivot, columns uc + 4 q
+  const bool row_ok = r0 + lr_ < F.f;
+  const int rows = F.f - r0, cols = F.f + 1 - c0;
+  const bool full = rows > R - 16 && cols > R - 8;
+  T lr[N], ur[N];
   auto fetch = [&](int k0) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int y = ly + 4 * q;
-      lr[q] = (row_ok && k0 + y < s) ? G[r0 + lx + (int64_t)(k0 + y) * ld] : T(0);
-      ur[q] = (c0 + y <= F.f && k0 + lx < s) ? G[k0 + lx + (int64_t)(c0 + y) * ld] : T(0);
+    for (int q = 0; q < N; ++q) {
+      const int k = lk + 128 / R * q, c = uc + 4 * q;
+      lr[q] = (row_ok && k0 + k < s) ? G[r0 + lr_ + (int64_t)(k0 + k) * ld] : T(0);
+      ur[q] = (c0 + c <= F.f && k0 + uk < s) ? G[k0 + uk + (int64_t)(c0 + c) * ld] : T(0);
     }
   };
   auto stash = [&](int w) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      Ls[w][ly + 4 * q][lx] = lr[q];
-      Us[w][ly + 4 * q][lx] = ur[q];
+    for (int q = 0; q < N; ++q) {
+      Ls[w][lk + 128 / R * q][lr_] = lr[q];
+      Us[w][uc + 4 * q][uk] = ur[q];
     }
   };
-  const int ti = tid & 15, tj = tid >> 4;  // rows ti, ti + 16; columns tj + 8 q
-  T acc[2][4];
+  const int ti = tid & 15, tj = tid >> 4;  // rows ti + 16 h; columns tj + 8 q
+  T acc[H][Q];
   fetch(0);
 #pragma unroll
-  for (int h = 0; h < 2; ++h)
+  for (int h = 0; h < H; ++h)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < Q; ++q) {
       const int r = r0 + ti + 16 * h, c = c0 + tj + 8 * q;
       acc[h][q] = (r < F.f && c <= F.f) ? G[r + (int64_t)c * ld] : T(0);
     }
+  if (!on) return;
   stash(0);
   __syncthreads();
   for (int k0 = 0, w = 0; k0 < s; k0 += 32, w ^= 1) {
     if (k0 + 32 < s) fetch(k0 + 32);
     const int kn = min(32, s - k0);
-    for (int k = 0; k < kn; ++k) {
-      const T l0 = -Ls[w][k][ti], l1 = -Ls[w][k][ti + 16];
+    if (full) {
+      for (int k = 0; k < kn; ++k) {
+        T l[H];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const T u = Us[w][tj + 8 * q][k];
-        acc[0][q] = mfma(l0, u, acc[0][q]);
-        acc[1][q] = mfma(l1, u, acc[1][q]);
+        for (int h = 0; h < H; ++h) l[h] = -Ls[w][k][ti + 16 * h];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const T u = Us[w][tj + 8 * q][k];
+#pragma unroll
+          for (int h = 0; h < H; ++h) acc[h][q] = mfma(l[h], u, acc[h][q]);
+        }
       }
+    } else {
+      // the halves and column groups of an edge tile that hold entries
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+          if (16 * h < rows && 8 * q < cols)
+#pragma unroll 8
+            for (int k = 0; k < kn; ++k) acc[h][q] = mfma(-Ls[w][k][ti + 16 * h], Us[w][tj + 8 * q][k], acc[h][q]);
     }
     if (k0 + 32 < s) stash(w ^ 1);
     __syncthreads();
   }
 #pragma unroll
-  for (int h = 0; h < 2; ++h)
+  for (int h = 0; h < H; ++h)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < Q; ++q) {
       const int r = r0 + ti + 16 * h, c = c0 + tj + 8 * q;
       if (r < F.f && c <= F.f) G[r + (int64_t)c * ld] = acc[h][q];
     }
 }
 
+// Substitution on a 32 x 32 diagonal block: D[j][i] its column j, row i.  Lane i
+// holds w_i of the block.
+template <typename T> __device__ __forceinline__ T mf_block_back(const T (*D)[33], int nb, int lane, T v) {
+  for (int k = nb - 1; k >= 0; --k) {
+    const T xk = __shfl_sync(0xffffffffu, v, k) * D[k][k];  // the reciprocal
+    if (lane == k) v = xk;
+    if (lane < k) v = mfma(-D[k][lane], xk, v);
+  }
+  return v;
+}
+template <typename T> __device__ __forceinline__ T mf_block_fwd(const T (*D)[33], int nb, int lane, T v) {
+  for (int k = 0; k + 1 < nb; ++k) {
+    const T yk = __shfl_sync(0xffffffffu, v, k);
+    if (lane > k) v = mfma(-D[k][lane], yk, v);
+  }
+  return v;
+}
+
 // Back substitution of every front of a height, one CTA each: w = y - U12 x2,
-// then x1 = U11^-1 w in blocks of 32 (warp 0 solves a block's triangle, then
-// every thread takes its rows above it).
-constexpr int MF_BACK_THREADS = 256;
+// then x1 = U11^-1 w in blocks of 32: warp 0 solves a block's triangle while the
+// others load the next one's and every thread its row above the block, then every
+// thread takes its rows.  The blocks' chain (150 cycles a DOF) bounds the tall
+// fronts; with the triangle's entries read from memory it was 600.
+constexpr int MF_BACK_THREADS = 256, MF_PART = 512;
 template <typename T> __global__ void __launch_bounds__(MF_BACK_THREADS) k_mf_back(Batch b, int off) {
   const FrontData& d = b.sh.mf;
-  const Front F = d.fronts[d.list[off + blockIdx.x]];
+  const Front F = d.list[off + blockIdx.x];
   if (!mf_active(b, F.slot)) return;
   const int f = F.f, s = F.s, u = f - s, ld = F.ld, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const T* G = mf_mat<T>(b, F);
   T* x = mf_x<T>(b);
   const int* B = d.bnd + F.bnd;
+  __shared__ T D[2][32][33];
   extern __shared__ __align__(16) unsigned char mf_raw[];
   T* w = reinterpret_cast<T*>(mf_raw);  // [f]: w of the own DOFs, then x2
-  T* part = w + f + (f & 1);            // [8][32]
+  T* part = w + f + (f & 1);            // [8][rows of a chunk]
+  const int sp = min((s + 31) / 32 * 32, MF_PART);
+  auto block = [&](T (*E)[33], int j0) {  // the diagonal block at j0 into E
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = lane, j = warp + 8 * q;
+      E[j][i] = (j0 + i < s && j0 + j < s) ? G[j0 + i + (int64_t)(j0 + j) * ld] : T(0);
+    }
+  };
+  const int last = (s - 1) / 32 * 32;
+  block(D[0], last);
   for (int i = tid; i < s; i += MF_BACK_THREADS) w[i] = G[i + (int64_t)f * ld];
   for (int i = tid; i < u; i += MF_BACK_THREADS) w[s + i] = x[B[i]];
   __syncthreads();
-  if (u > 0)
-    for (int i0 = 0; i0 < s; i0 += 32) {
-      // 32 rows, the eight warps an eighth of the columns each
+  for (int c0 = 0; u > 0 && c0 < s; c0 += MF_PART) {
+    // 32 rows at a time, the eight warps an eighth of the columns each
+    for (int i0 = c0; i0 < min(s, c0 + MF_PART); i0 += 32) {
       const int i = i0 + lane;
-      T acc = T(0);
-      if (i < s)
-        for (int j = s + warp; j < f; j += 8) acc = mfma(G[i + (int64_t)j * ld], w[j], acc);
-      part[warp * 32 + lane] = acc;
-      __syncthreads();
-      if (warp == 0 && i < s) {
-        T t = part[lane];
-        for (int q = 1; q < 8; ++q) t += part[q * 32 + lane];
-        w[i] -= t;
+      T acc[4] = {T(0), T(0), T(0), T(0)};
+      if (i < s) {
+        const T* g = G + i;
+        int j = s + warp;
+        for (; j + 24 < f; j += 32) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc[q] = mfma(g[(int64_t)(j + 8 * q) * ld], w[j + 8 * q], acc[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          if (j + 8 * q < f) acc[q] = mfma(g[(int64_t)(j + 8 * q) * ld], w[j + 8 * q], acc[q]);
       }
-      __syncthreads();
+      part[warp * sp + i - c0] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
     }
-  for (int j0 = (s - 1) / 32 * 32; j0 >= 0; j0 -= 32) {
+    __syncthreads();
+    for (int i = c0 + tid; i < min(s, c0 + MF_PART); i += MF_BACK_THREADS) {
+      T t = part[i - c0];
+      for (int q = 1; q < 8; ++q) t += part[q * sp + i - c0];
+      w[i] -= t;
+    }
+    __syncthreads();
+  }
+  int cur = 0;
+  for (int j0 = last; j0 >= 0; j0 -= 32, cur ^= 1) {
     const int nb = min(32, s - j0);
+    T g[32];
+    const bool mine = tid < j0;  // this thread's first row above the block
+#pragma unroll
+    for (int k = 0; k < 32; ++k) g[k] = (mine && k < nb) ? G[tid + (int64_t)(j0 + k) * ld] : T(0);
     if (warp == 0) {
-      T v = lane < nb ? w[j0 + lane] : T(0);
-      for (int k = nb - 1; k >= 0; --k) {
-        const T ukk = G[j0 + k + (int64_t)(j0 + k) * ld];  // the reciprocal
-        const T uk = lane < k ? G[j0 + lane + (int64_t)(j0 + k) * ld] : T(0);
-        const T xk = __shfl_sync(0xffffffffu, v, k) * ukk;
-        if (lane == k) v = xk;
-        if (lane < k) v = mfma(-uk, xk, v);
-      }
+      const T v = mf_block_back<T>(D[cur], nb, lane, lane < nb ? w[j0 + lane] : T(0));
       if (lane < nb) {
         w[j0 + lane] = v;
         x[F.dof0 + j0 + lane] = v;
       }
     }
+    if (j0 > 0) block(D[cur ^ 1], j0 - 32);
     __syncthreads();
-    for (int i = tid; i < j0; i += MF_BACK_THREADS) {
+    if (mine) {
       T a0 = T(0), a1 = T(0);
-      for (int k = 0; k < nb; k += 2) {
-        a0 = mfma(G[i + (int64_t)(j0 + k) * ld], w[j0 + k], a0);
+#pragma unroll
+      for (int k = 0; k < 32; k += 2) {
+        if (k < nb) a0 = mfma(g[k], w[j0 + k], a0);
+        if (k + 1 < nb) a1 = mfma(g[k + 1], w[j0 + k + 1], a1);
+      }
+      w[tid] -= a0 + a1;
+    }
+    for (int i = tid + MF_BACK_THREADS; i < j0; i += MF_BACK_THREADS) {
+      T a0 = T(0), a1 = T(0);
+#pragma unroll 8
+      for (int k = 0; k < 32; k += 2) {
+        if (k < nb) a0 = mfma(G[i + (int64_t)(j0 + k) * ld], w[j0 + k], a0);
         if (k + 1 < nb) a1 = mfma(G[i + (int64_t)(j0 + k + 1) * ld], w[j0 + k + 1], a1);
       }
       w[i] -= a0 + a1;
@@ -529,44 +676,64 @@ template <typename T> __global__ void __launch_bounds__(MF_BACK_THREADS) k_mf_ba
 
 // Forward substitution alone, on fronts that hold their LU: every front of a
 // height, one CTA each.  w = the right-hand side of the own DOFs with what the
-// children leave (their column f, read through their parent indices, one child
-// after the other), then y1 = L11^-1 w1 in blocks of 32 and w2 -= L21 y1; both
-// into column f.
+// children leave (column f of theirs, one child after the other), then y1 =
+// L11^-1 w1 in blocks of 32 and w2 -= L21 y1, as in k_mf_back; both into column f.
 template <typename T> __global__ void __launch_bounds__(MF_BACK_THREADS) k_mf_fwd(Batch b, int off) {
   const FrontData& d = b.sh.mf;
-  const int id = d.list[off + blockIdx.x];
-  const Front F = d.fronts[id];
+  const Front F = d.list[off + blockIdx.x];
   if (!mf_active(b, F.slot)) return;
   const int f = F.f, s = F.s, ld = F.ld, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   T* G = mf_mat<T>(b, F);
+  __shared__ T D[2][32][33];
   extern __shared__ __align__(16) unsigned char mf_raw[];
   T* w = reinterpret_cast<T*>(mf_raw);  // [f]
   const T* P = mf_rhs(b, (T*)nullptr);
-  for (int i = tid; i < f; i += MF_BACK_THREADS) w[i] = i < s ? P[d.dof_at[F.dof0 + i]] : T(0);
-  for (int k = d.kid_off[id]; k < d.kid_off[id + 1]; ++k) {
-    __syncthreads();
-    const Front C = d.fronts[d.kids[k]];
-    const T* cw = mf_mat<T>(b, C) + (int64_t)C.f * C.ld + C.s;
-    const int* rel = d.rel + C.rel;
-    for (int i = tid; i < C.f - C.s; i += MF_BACK_THREADS) w[rel[i]] += cw[i];
+  auto block = [&](T (*E)[33], int j0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = lane, j = warp + 8 * q;
+      E[j][i] = (j0 + i < s && j0 + j < s) ? G[j0 + i + (int64_t)(j0 + j) * ld] : T(0);
+    }
+  };
+  block(D[0], 0);
+  for (int i = tid; i < f; i += MF_BACK_THREADS) {
+    T v = i < s ? P[d.dof_at[F.dof0 + i]] : T(0);
+    for (int k = F.kid0; k < F.kid1; ++k) {
+      const int2 kid = d.kids[k];
+      const Front& C = d.fronts[kid.x];
+      const int ci = d.inv[kid.y + i];
+      if (ci >= 0) v += reinterpret_cast<const T*>(d.F)[C.off + C.s + ci + (int64_t)C.f * C.ld];
+    }
+    w[i] = v;
   }
   __syncthreads();
-  for (int j0 = 0; j0 < s; j0 += 32) {
-    const int nb = min(32, s - j0);
+  int cur = 0;
+  for (int j0 = 0; j0 < s; j0 += 32, cur ^= 1) {
+    const int nb = min(32, s - j0), r = j0 + nb + tid;
+    T g[32];
+    const bool mine = r < f;  // this thread's first row below the block
+#pragma unroll
+    for (int k = 0; k < 32; ++k) g[k] = (mine && k < nb) ? G[r + (int64_t)(j0 + k) * ld] : T(0);
     if (warp == 0) {
-      T v = lane < nb ? w[j0 + lane] : T(0);
-      for (int k = 0; k + 1 < nb; ++k) {
-        const T l = lane > k && lane < nb ? G[j0 + lane + (int64_t)(j0 + k) * ld] : T(0);
-        const T yk = __shfl_sync(0xffffffffu, v, k);
-        if (lane > k) v = mfma(-l, yk, v);
-      }
+      const T v = mf_block_fwd<T>(D[cur], nb, lane, lane < nb ? w[j0 + lane] : T(0));
       if (lane < nb) w[j0 + lane] = v;
     }
+    if (j0 + 32 < s) block(D[cur ^ 1], j0 + 32);
     __syncthreads();
-    for (int i = j0 + nb + tid; i < f; i += MF_BACK_THREADS) {
+    if (mine) {
       T a0 = T(0), a1 = T(0);
-      for (int k = 0; k < nb; k += 2) {
-        a0 = mfma(G[i + (int64_t)(j0 + k) * ld], w[j0 + k], a0);
+#pragma unroll
+      for (int k = 0; k < 32; k += 2) {
+        if (k < nb) a0 = mfma(g[k], w[j0 + k], a0);
+        if (k + 1 < nb) a1 = mfma(g[k + 1], w[j0 + k + 1], a1);
+      }
+      w[r] -= a0 + a1;
+    }
+    for (int i = r + MF_BACK_THREADS; i < f; i += MF_BACK_THREADS) {
+      T a0 = T(0), a1 = T(0);
+#pragma unroll 8
+      for (int k = 0; k < 32; k += 2) {
+        if (k < nb) a0 = mfma(G[i + (int64_t)(j0 + k) * ld], w[j0 + k], a0);
         if (k + 1 < nb) a1 = mfma(G[i + (int64_t)(j0 + k + 1) * ld], w[j0 + k + 1], a1);
       }
       w[i] -= a0 + a1;
@@ -646,7 +813,7 @@ template <typename T> void launch_front_factor(const Batch& b, cudaStream_t st) 
   const dim3 dofs(dof_blocks(b), b.sh.n_wide);
   k_mf_rhs<T><<<dofs, 256, 0, st>>>(b);
   for (const FrontLevel& V : sc.level) {
-    for (size_t o = 0; o < V.ext_off.size(); ++o) k_mf_extend<T><<<V.ext_cnt[o], 256, 0, st>>>(b, V.ext_off[o]);
+    if (V.ext_cnt) k_mf_extend<T><<<V.ext_cnt, 256, 0, st>>>(b, V.ext_off);
     if (V.n_small)
       k_mf_small<T><<<V.n_small, MF_SMALL_THREADS, (size_t)((V.small_f + 1) & ~1) * (V.small_f + 1) * sizeof(T), st>>>(
           b, V.small_off);
@@ -656,8 +823,14 @@ template <typename T> void launch_front_factor(const Batch& b, cudaStream_t st) 
       // the panels of fronts whose last panel this is end before k1
       const int m = f - k0 - 1;
       if (m >= 0) {
-        const int nlow = (m + 31) / 32, nup = (m + 1 + 31) / 32;
-        k_mf_trsm<T><<<dim3(nlow + nup, n), 128, 0, st>>>(b, V.big_off, (int)p, nlow);
+        // sixteen lanes a row while that leaves an SM at most one CTA
+        if ((2 * m + 1) * n <= 8 * 152) {
+          const int nlow = (m + 7) / 8, nup = (m + 1 + 7) / 8;
+          k_mf_trsm<T, 16><<<dim3(nlow + nup, n), 128, 0, st>>>(b, V.big_off, (int)p, nlow);
+        } else {
+          const int nlow = (m + 31) / 32, nup = (m + 1 + 31) / 32;
+          k_mf_trsm<T, 4><<<dim3(nlow + nup, n), 128, 0, st>>>(b, V.big_off, (int)p, nlow);
+        }
       }
       if (s > k1) {
         const int nca = (f + 1 - k1 + 31) / 32, na = (s - k1 + 15) / 16 * nca;
@@ -665,7 +838,10 @@ template <typename T> void launch_front_factor(const Batch& b, cudaStream_t st) 
         k_mf_panel<T><<<dim3(na + nb, n), 128, 0, st>>>(b, V.big_off, (int)p, na, nca, ncb);
       }
     }
-    if (V.schur_cnt) k_mf_schur<T><<<V.schur_cnt, 128, 0, st>>>(b, V.schur_off);
+    if (V.schur_cnt) {
+      if (V.tile == 16) k_mf_schur<T, 16><<<V.schur_cnt, 128, 0, st>>>(b, V.schur_off);
+      else k_mf_schur<T, 32><<<V.schur_cnt, 128, 0, st>>>(b, V.schur_off);
+    }
   }
 }
 
@@ -673,8 +849,8 @@ template <typename T> void launch_front_back(const Batch& b, cudaStream_t st) {
   const FrontSchedule& sc = *b.sh.mf.sched;
   for (size_t l = sc.level.size(); l-- > 0;) {
     const FrontLevel& V = sc.level[l];
-    const int f = std::max(V.small_f, V.big_f);
-    k_mf_back<T><<<V.n_small + V.n_big, MF_BACK_THREADS, (size_t)(f + 2 + 8 * 32) * sizeof(T), st>>>(b, V.small_off);
+    const size_t n = (size_t)std::max(V.small_f, V.big_f) + 2 + 8 * (size_t)std::min((V.max_s + 31) / 32 * 32, MF_PART);
+    k_mf_back<T><<<V.n_small + V.n_big, MF_BACK_THREADS, n * sizeof(T), st>>>(b, V.small_off);
   }
   k_mf_out<T><<<dim3(dof_blocks(b), b.sh.n_wide), 256, 0, st>>>(b);
 }

@@ -30,10 +30,11 @@ struct Front {
   int bnd;     // boundary DOFs (batch-wide elimination positions, ascending): bnd[bnd .. bnd + f - s)
   int rel;     // the parent's front index of every boundary DOF: rel[rel .. rel + f - s)
   int parent;  // -1: a root
+  int kid0, kid1;  // its children: kids[kid0 .. kid1)
 };
 
-// Fronts whose whole matrix fits in a CTA's shared memory take one CTA for the
-// elimination (k_mf_small); the others run panel by panel on many.
+// Fronts up to this size may take one CTA for the elimination, the whole matrix
+// in its shared memory (k_mf_small); the others run panel by panel on many.
 constexpr int MF_SMALL = 96;
 constexpr int MF_NB = 32;  // pivots per panel of a large front
 
@@ -41,12 +42,12 @@ constexpr int MF_NB = 32;  // pivots per panel of a large front
 struct FrontLevel {
   int small_off = 0, n_small = 0, small_f = 0;  // list range, largest small front
   int big_off = 0, n_big = 0;                   // list range, by descending s
-  int big_f = 0;
+  int big_f = 0, max_s = 0;                     // largest large front, most own DOFs of any
   std::vector<int> n_at;                        // large fronts that have panel k
   std::vector<int> f_at;                        // largest f among them
   std::vector<int> s_at;                        // largest s among them
-  std::vector<int> ext_off, ext_cnt;            // extend-add jobs of the k-th children
-  int schur_off = 0, schur_cnt = 0;
+  int ext_off = 0, ext_cnt = 0;                 // extend-add jobs of the large fronts
+  int schur_off = 0, schur_cnt = 0, tile = 32;  // Schur jobs and the rows and columns of one
 };
 struct FrontSchedule {
   std::vector<FrontLevel> level;
@@ -59,11 +60,11 @@ struct FrontData {
   Front* fronts;
   int* bnd;
   int* rel;
-  int* list;        // front ids by height
-  int2* ext_jobs;   // (child front, column block)
-  int2* schur_jobs; // (front, row tile | column tile << 16)
-  int* kid_off;     // children of front i: kids[kid_off[i] .. kid_off[i + 1])
-  int* kids;
+  Front* list;      // the fronts by height
+  int2* ext_jobs;   // (front, column block)
+  int2* schur_jobs; // (front, row tile | column tile << 16), tiles of FrontLevel::tile rows
+  int2* kids;       // (child front, offset in inv)
+  int* inv;         // per child: its boundary index of every row of the parent (-1: none)
   int* dof_at;      // elimination position -> free DOF (batch-wide)
   int* pos;         // free DOF (batch-wide) -> elimination position (batch-wide)
   int* dof_front;   // elimination position -> its front
@@ -110,8 +111,9 @@ FrontPlan plan_fronts(const NdGraph& g, const std::vector<int>& dptr, const std:
 // batch-wide.
 struct FrontBuild {
   std::vector<gf::Front> fronts;
-  std::vector<int> bnd, rel, list, pos, dof_front, kid_off, kids, dof_at;
-  std::vector<int2> ext_jobs, schur_jobs;
+  std::vector<gf::Front> list;
+  std::vector<int> bnd, rel, pos, dof_front, inv, dof_at;
+  std::vector<int2> kids, ext_jobs, schur_jobs;
   std::vector<int64_t> base, size;  // per structure (0 for the others)
   int64_t total = 0;
   gf::FrontSchedule sched;

@@ -48,7 +48,8 @@ struct FrontSystem {
     state.phase = gf::PH_ITER;
     state.need_solve = 1;
     auto vec = [&](const auto& v) { return send(v.data(), v.size() * sizeof(v[0])); };
-    const int p_fr = vec(fb.fronts), p_bnd = vec(fb.bnd), p_rel = vec(fb.rel), p_list = vec(fb.list),
+    const int p_fr = vec(fb.fronts), p_bnd = vec(fb.bnd), p_kids = vec(fb.kids),
+              p_inv = vec(fb.inv), p_list = vec(fb.list),
               p_ext = vec(fb.ext_jobs), p_sch = vec(fb.schur_jobs), p_pos = vec(fb.pos), p_df = vec(fb.dof_front),
               p_base = vec(fb.base), p_size = vec(fb.size);
     const int p_info = send(&info, sizeof(info)), p_ws = send(&zero, sizeof(int));
@@ -76,8 +77,9 @@ struct FrontSystem {
     d.n_fronts = (int)fb.fronts.size();
     d.fronts = at<gf::Front>(p_fr);
     d.bnd = at<int>(p_bnd);
-    d.rel = at<int>(p_rel);
-    d.list = at<int>(p_list);
+    d.kids = at<int2>(p_kids);
+    d.inv = at<int>(p_inv);
+    d.list = at<gf::Front>(p_list);
     d.ext_jobs = at<int2>(p_ext);
     d.schur_jobs = at<int2>(p_sch);
     d.pos = at<int>(p_pos);

@@ -1195,8 +1195,8 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       if (!upload(B, &md.fronts, fb.fronts) || !upload(B, &md.bnd, fb.bnd) || !upload(B, &md.rel, fb.rel) ||
           !upload(B, &md.list, fb.list) || !upload(B, &md.ext_jobs, fb.ext_jobs) ||
           !upload(B, &md.schur_jobs, fb.schur_jobs) || !upload(B, &md.pos, fb.pos) ||
-          !upload(B, &md.dof_front, fb.dof_front) || !upload(B, &md.kid_off, fb.kid_off) ||
-          !upload(B, &md.kids, fb.kids) || !upload(B, &md.dof_at, fb.dof_at) ||
+          !upload(B, &md.dof_front, fb.dof_front) ||
+          !upload(B, &md.kids, fb.kids) || !upload(B, &md.inv, fb.inv) || !upload(B, &md.dof_at, fb.dof_at) ||
           !upload(B, &md.base, fb.base) || !upload(B, &md.size, fb.size) ||
           !balloc(B, &md.map, (size_t)shell_off * 729) || !balloc(B, &md.F, (size_t)fb.total) ||
           !balloc(B, &md.x, (size_t)dof_off))

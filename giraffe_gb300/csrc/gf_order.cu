@@ -271,6 +271,43 @@ FrontPlan plan_fronts(const NdGraph& g, const std::vector<int>& dptr, const std:
   return P;
 }
 
+// The largest front of a height that takes one CTA.  One CTA runs at its SM's FP64
+// rate (16 cycles a warp instruction) and has no launches between its steps: the
+// way for many fronts.  Panel by panel a front spreads over the SMs at about 30 us
+// a panel (diagonal block, rows and columns, update): the way for a few, whose one
+// CTA each would take longer (a front of 96 with 69 pivots 190 us, panel by panel
+// 90).  Both give the same bits.  Estimates in us; W is the elimination's time on
+// an SM of its own.
+static int small_limit(const std::vector<gf::Front>& fronts, const std::vector<int>& at) {
+  static const int lims[] = {gf::MF_SMALL, 88, 80, 72, 64, 48, 32, 0};
+  int best = gf::MF_SMALL;
+  double best_t = -1.0;
+  for (int lim : lims) {
+    double one = 0.0, ws = 0.0, wb = 0.0;
+    int sb = 0, n_small = 0, n_big = 0;
+    for (int k : at) {
+      const double f = fronts[k].f, s = fronts[k].s, w = (s * f * f - s * s * f + s * s * s / 3.0) * (0.5 / 1930.0);
+      if (fronts[k].f <= lim) {
+        one = std::max(one, 1.6 * w + 0.5 * s);
+        ws += w;
+        ++n_small;
+      } else {
+        sb = std::max(sb, fronts[k].s);
+        wb += w;
+        ++n_big;
+      }
+    }
+    double t = 0.0;
+    if (n_small) t += 5.0 + std::max(one, 1.4 * ws / 152.0);
+    if (n_big) t += 10.0 + 30.0 * ((sb + gf::MF_NB - 1) / gf::MF_NB) + 1.5 * wb / 152.0;
+    if (best_t < 0.0 || t < best_t) {
+      best_t = t;
+      best = lim;
+    }
+  }
+  return best;
+}
+
 void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<int>& slots,
                  const std::vector<int>& dof_off, int n_struct, int n_dofs, FrontBuild& out) {
   out.pos.assign(n_dofs, -1);
@@ -307,10 +344,16 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
     at[height[k]].push_back(k);
     if (out.fronts[k].parent >= 0 && out.fronts[k].f > out.fronts[k].s) kids[out.fronts[k].parent].push_back(k);
   }
-  out.kid_off.assign(1, 0);
   for (int k = 0; k < nf; ++k) {
-    out.kids.insert(out.kids.end(), kids[k].begin(), kids[k].end());
-    out.kid_off.push_back((int)out.kids.size());
+    out.fronts[k].kid0 = (int)out.kids.size();
+    for (int c : kids[k]) {
+      const gf::Front& C = out.fronts[c];
+      out.kids.push_back(make_int2(c, (int)out.inv.size()));
+      out.inv.resize(out.inv.size() + out.fronts[k].f, -1);
+      int* inv = out.inv.data() + out.inv.size() - out.fronts[k].f;
+      for (int i = 0; i < C.f - C.s; ++i) inv[out.rel[C.rel + i]] = i;
+    }
+    out.fronts[k].kid1 = (int)out.kids.size();
   }
   out.dof_at.assign(n_dofs, -1);
   for (int i = 0; i < n_dofs; ++i)
@@ -320,33 +363,27 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
   for (int l = 0; l < nl; ++l) {
     gf::FrontLevel& V = out.sched.level[l];
     std::vector<int> small, big;
-    size_t ords = 0;
-    for (int k : at[l]) {
-      (out.fronts[k].f <= gf::MF_SMALL ? small : big).push_back(k);
-      ords = std::max(ords, kids[k].size());
-    }
+    const int lim = small_limit(out.fronts, at[l]);
+    for (int k : at[l]) (out.fronts[k].f <= lim ? small : big).push_back(k);
     auto larger = [&](int a, int b) {
       const gf::Front &A = out.fronts[a], &B = out.fronts[b];
       return A.s != B.s ? A.s > B.s : a < b;
     };
     std::sort(big.begin(), big.end(), larger);
     std::sort(small.begin(), small.end(), larger);
+    for (int k : at[l]) V.max_s = std::max(V.max_s, out.fronts[k].s);
     V.small_off = (int)out.list.size();
     V.n_small = (int)small.size();
     for (int k : small) V.small_f = std::max(V.small_f, out.fronts[k].f);
-    out.list.insert(out.list.end(), small.begin(), small.end());
+    for (int k : small) out.list.push_back(out.fronts[k]);
     V.big_off = (int)out.list.size();
     V.n_big = (int)big.size();
-    out.list.insert(out.list.end(), big.begin(), big.end());
-    for (size_t o = 0; o < ords; ++o) {
-      V.ext_off.push_back((int)out.ext_jobs.size());
-      for (int k : at[l])
-        if (kids[k].size() > o) {
-          const gf::Front& C = out.fronts[kids[k][o]];
-          for (int c = 0; c <= C.f - C.s; c += 16) out.ext_jobs.push_back(make_int2(kids[k][o], c));
-        }
-      V.ext_cnt.push_back((int)out.ext_jobs.size() - V.ext_off.back());
-    }
+    for (int k : big) out.list.push_back(out.fronts[k]);
+    V.ext_off = (int)out.ext_jobs.size();
+    for (int k : big)
+      if (!kids[k].empty())
+        for (int c = 0; c <= out.fronts[k].f; c += 8) out.ext_jobs.push_back(make_int2(k, c));
+    V.ext_cnt = (int)out.ext_jobs.size() - V.ext_off;
     const int panels = big.empty() ? 0 : (out.fronts[big[0]].s + gf::MF_NB - 1) / gf::MF_NB;
     for (int p = 0; p < panels; ++p) {
       int n = 0, f = 0, s = 0;
@@ -360,16 +397,27 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
       V.s_at.push_back(s);
     }
     V.schur_off = (int)out.schur_jobs.size();
+    // 32 x 32 tiles, or 16 x 16 while those leave SMs idle in the last wave: a tile
+    // holds an SM's FP64 units for its whole product
+    auto tiles = [&](int t) {
+      int64_t n = 0;
+      for (int k : big) {
+        const int u = out.fronts[k].f - out.fronts[k].s;
+        if (u > 0) n += (int64_t)((u + t) / t) * ((u + t - 1) / t);
+      }
+      return n;
+    };
+    if (4 * ((tiles(32) + 151) / 152) * 10 > 13 * ((tiles(16) + 151) / 152)) V.tile = 16;
     for (int k : big) {
       const gf::Front& F = out.fronts[k];
       const int u = F.f - F.s;
       V.big_f = std::max(V.big_f, F.f);
       if (u > 0)
-        for (int tj = 0; tj < (u + 1 + 31) / 32; ++tj)
-          for (int ti = 0; ti < (u + 31) / 32; ++ti) out.schur_jobs.push_back(make_int2(k, ti | (tj << 16)));
+        for (int tj = 0; tj < (u + V.tile) / V.tile; ++tj)
+          for (int ti = 0; ti < (u + V.tile - 1) / V.tile; ++ti) out.schur_jobs.push_back(make_int2(k, ti | (tj << 16)));
     }
     V.schur_cnt = (int)out.schur_jobs.size() - V.schur_off;
-    out.sched.launches += (int)ords + (V.n_small ? 1 : 0) + (V.schur_cnt ? 1 : 0) + 1;
+    out.sched.launches += (V.ext_cnt ? 1 : 0) + (V.n_small ? 1 : 0) + (V.schur_cnt ? 1 : 0) + 1;
     for (int p = 0; p < panels; ++p)
       out.sched.launches += 1 + (V.f_at[p] > p * gf::MF_NB ? 1 : 0) + (V.s_at[p] > (p + 1) * gf::MF_NB ? 1 : 0);
   }
