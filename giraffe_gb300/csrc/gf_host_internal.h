@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/giraffe_gpu.h"
+#include "gf_beam_setup.cuh"
 #include "gf_types.h"
 
 struct gf_ctx {
@@ -248,12 +249,10 @@ int wide_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ld
 // (gf_sparse.cu).
 bool band_takes_fronts(int n, int kl, int ku);
 int front_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, int* info);
-// Host PreCalc of one Beam_1 element (end nodes x0, x2; Hooke material E,
-// nu, rho; section A, I11, I22, I12, It, I33; CS rows E1, E3; pre-tension
-// T0) into its constants and initial Gauss-point history, and of one Shell_1
-// element (six nodes, material, thickness).
-void beam_precalc(const double* x0, const double* x2, const double* mat, const double* sec, const double* cs,
-                  gf::BeamConst& c, gf::BeamHist& h, gf::BeamHistAux& x, double T0);
+using gf::beam_precalc;
+using gf::beam_state_in;
+using gf::cs_rows;
+// Host PreCalc of one Shell_1 element (six nodes, material, thickness).
 void shell_precalc(const double* xyz, const double* mat, double thick, gf::ShellConst& c, gf::ShellHist& h,
                    gf::ShellHistAux& x);
 // CSR pattern of structure s's K_AA in the reference's free-DOF numbering
