@@ -26,6 +26,11 @@ constexpr int NC = 19;  // augmented columns: 6 (matrix) + 13 (right-hand sides)
 // Part: the matrix ([row * 12 + column]), then the forces on p and n.
 constexpr int GP_F = 144;
 
+// The item-per-warp form's staging area (doubles): two parts or an 18x18 K_e, a
+// zero, the forces of a midside node.
+constexpr int GEN_E2 = CHAIN_GEN_PART, GEN_ZERO = 324, GEN_F = 325, GEN_STAGE = 332;
+static_assert(2 * CHAIN_GEN_PART <= GEN_ZERO, "two parts");
+
 // Gauss-Jordan on a thread's augmented matrix [D | R] in two phases, both in
 // registers: gj6_factor eliminates D (6x6, row-major, every index static under
 // the full unroll) and records each pivot's reciprocal and multipliers;
@@ -39,7 +44,7 @@ __device__ __forceinline__ bool gj6_factor(double (&D)[36], double (&inv)[6], do
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     const double p = D[k * 6 + k];
-    if (!(p != 0.0) || !isfinite(p)) ok = false;
+    ok = ok && !bad_pivot(p);
     inv[k] = rcp64(p);
     double dk[6];
 #pragma unroll
@@ -105,6 +110,39 @@ struct GenCondense {
   __device__ __forceinline__ double base(int x, int q) const {
     return q == 0 || !live(x) || !live(q - 1) ? 0.0 : ke(place(x), place(q - 1));
   }
+  // The item-per-warp form: K_e with its fixed corner DOFs cleared at s[0], the
+  // midside node's forces at s[GEN_F], its load stiffness added.
+  __device__ __forceinline__ void stage(int lane, double* s) const {
+    double v[11], extra = 0.0;
+#pragma unroll
+    for (int q = 0; q < 11; ++q) {
+      const int x = lane + 32 * q, i = x % 18, j = x / 18;
+      const bool fixed = (i < 6 && !live(i)) || (i >= 12 && !live(i - 6)) || (j < 6 && !live(j)) || (j >= 12 && !live(j - 6));
+      v[q] = x < 324 && !fixed ? K[(int64_t)x * ne] : 0.0;
+    }
+    const double* at = lane < 9 ? b.nodeK + (int64_t)nm * 9 + lane : P + lane - 9;
+    if (lane < 15) extra = *at;
+#pragma unroll
+    for (int q = 0; q < 11; ++q)
+      if (lane + 32 * q < 324) s[lane + 32 * q] = v[q];
+    if (lane == 31) s[GEN_ZERO] = 0.0;
+    if (lane >= 9 && lane < 15) s[GEN_F + lane - 9] = extra;
+    __syncwarp();
+    if (lane < 9) s[9 + lane / 3 + 18 * (9 + lane % 3)] += extra;
+    __syncwarp();
+  }
+  // where column `lane` of [D | R] is the sum of: entries a + i sa and o + i so
+  __device__ __forceinline__ void column(int lane, int& a, int& sa, int& o, int& so) const {
+    a = lane < 6 ? 6 + 18 * (6 + lane) : lane == 6 ? GEN_F : lane < NC ? 6 + 18 * place(lane - 7) : GEN_ZERO;
+    sa = lane < NC ? 1 : 0;
+    o = GEN_ZERO;
+    so = 0;
+  }
+  __device__ __forceinline__ static double pinned(int, int, double v) { return v; }
+  __device__ __forceinline__ static double left_s(const double* s, int x, int k) { return s[place(x) + 18 * (6 + k)]; }
+  __device__ __forceinline__ static double base_s(const double* s, int x, int q) {
+    return s[q == 0 ? GEN_ZERO : place(x) + 18 * place(q - 1)];
+  }
   __device__ __forceinline__ void keep(int x, double v) const { chain_at(c.ez, c.elem_soa, CHAIN_GEN_KEEP, t, x) = v; }
   __device__ __forceinline__ void out(int x, int q, double v) const {
     chain_at(c.part, c.part_soa, CHAIN_GEN_PART, t, q == 0 ? GP_F + x : x * 12 + q - 1) = v;
@@ -128,9 +166,9 @@ struct GenMerge {
   __device__ __forceinline__ bool live(int i) const { return m.mask >> i & 1; }
   __device__ __forceinline__ double d(int i, int j) const {
     if (!live(i) || !live(j)) return i == j ? 1.0 : 0.0;
-    double v = E(m.e1, (6 + i) * 12 + 6 + j) + E(m.e2, i * 12 + j);
+    double v = E(m.e1, (6 + i) * 12 + 6 + j);
     if (i >= 3 && j >= 3) v += b.nodeK[(int64_t)node * 9 + (i - 3) * 3 + j - 3];
-    return v;
+    return v + E(m.e2, i * 12 + j);
   }
   __device__ __forceinline__ double r(int i, int q) const {
     if (q == 0)  // the corner's own force with what both parts leave on it
@@ -144,6 +182,52 @@ struct GenMerge {
     if (q == 0) return x < 6 ? E(m.e1, GP_F + x) : E(m.e2, GP_F + x);
     if ((x < 6) != (q < 7)) return 0.0;
     return E(x < 6 ? m.e1 : m.e2, x * 12 + q - 1);
+  }
+  // The item-per-warp form: e1 at s[0], e2 at s[GEN_E2], the corner's load stiffness
+  // and force added to e1.
+  __device__ __forceinline__ void stage(int lane, double* s) const {
+    double v1[5], v2[5], extra = 0.0;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      const int x = lane + 32 * q;
+      v1[q] = x < CHAIN_GEN_PART ? E(m.e1, x) : 0.0;
+      v2[q] = x < CHAIN_GEN_PART ? E(m.e2, x) : 0.0;
+    }
+    const int f = lane - 9;
+    const double* at = lane < 9 ? b.nodeK + (int64_t)node * 9 + lane : b.P + m.dof + __popc(m.mask & ((1 << f) - 1));
+    if (lane < 9 || (lane < 15 && live(f))) extra = *at;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      const int x = lane + 32 * q;
+      if (x < CHAIN_GEN_PART) {
+        s[x] = v1[q];
+        s[GEN_E2 + x] = v2[q];
+      }
+    }
+    if (lane == 31) s[GEN_ZERO] = 0.0;
+    __syncwarp();
+    if (lane < 15) s[lane < 9 ? (9 + lane / 3) * 12 + 9 + lane % 3 : GP_F + 6 + f] += extra;
+    __syncwarp();
+  }
+  __device__ __forceinline__ void column(int lane, int& a, int& sa, int& o, int& so) const {
+    const int q = lane - 6;
+    const bool first = lane < 6 || q == 0 || (q > 0 && q < 7), second = lane < 6 || q == 0 || (q >= 7 && lane < NC);
+    a = !first ? GEN_ZERO : q == 0 ? GP_F + 6 : 72 + (lane < 6 ? 6 + lane : q - 1);
+    sa = !first ? 0 : q == 0 ? 1 : 12;
+    o = !second ? GEN_ZERO : GEN_E2 + (q == 0 ? GP_F : lane < 6 ? lane : q - 1);
+    so = !second ? 0 : q == 0 ? 1 : 12;
+  }
+  // entry i of column `lane` where the corner is fixed
+  __device__ __forceinline__ double pinned(int i, int lane, double v) const {
+    if (lane < 6 && !(live(i) && live(lane))) return i == lane ? 1.0 : 0.0;
+    return lane == 6 && !live(i) ? 0.0 : v;
+  }
+  __device__ __forceinline__ static double left_s(const double* s, int x, int k) {
+    return s[x < 6 ? x * 12 + 6 + k : GEN_E2 + x * 12 + k];
+  }
+  __device__ __forceinline__ static double base_s(const double* s, int x, int q) {
+    const int o = (x < 6 ? 0 : GEN_E2) + (q == 0 ? GP_F + x : x * 12 + q - 1);
+    return s[q != 0 && (x < 6) != (q < 7) ? GEN_ZERO : o];
   }
   __device__ __forceinline__ void keep(int x, double v) const { chain_at(c.mz, c.merge_soa, CHAIN_GEN_KEEP, t, x) = v; }
   __device__ __forceinline__ void out(int x, int q, double v) const {
@@ -200,27 +284,25 @@ template <typename Item> __global__ void __launch_bounds__(CT) k_gen(Batch b, Ch
   }
 }
 
-// An item per warp: lane q < 19 holds column q of [D | R], the pivot column is
+// An item per warp: its operands go to shared memory in one round of loads (read
+// entry by entry under the conditions of each column they took a memory round
+// trip per condition), lane q < 19 holds column q of [D | R], the pivot column is
 // broadcast by shuffle; then the lanes share the entries of the new part.
-template <typename Item> __device__ __forceinline__ bool gen_item(const Item& I, int lane, double (*zs)[13]) {
-  double col[6], base[5], left[5][6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) col[i] = lane < 6 ? I.d(i, lane) : lane < NC ? I.r(i, lane - 6) : 0.0;
-  // the products' operands, loaded ahead of the dependent chain
-#pragma unroll
-  for (int y = 0; y < 5; ++y) {
-    const int o = lane + 32 * y, x = o / 13, q = o % 13;
-    if (o >= 156) break;
-    base[y] = I.base(x, q);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) left[y][k] = I.left(x, k);
-  }
+template <typename Item> __device__ __forceinline__ bool gen_item(const Item& I, int lane, double* st, double (*zs)[13]) {
+  I.stage(lane, st);
   if (!I.active()) return true;
+  double col[6];
+  {
+    int a, sa, o, so;
+    I.column(lane, a, sa, o, so);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) col[i] = I.pinned(i, lane, st[a + i * sa] + st[o + i * so]);
+  }
   bool ok = true;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     const double p = __shfl_sync(0xffffffffu, col[k], k);
-    if (!(p != 0.0) || !isfinite(p)) ok = false;
+    ok = ok && !bad_pivot(p);
     const double inv = rcp64(p);
     double m[6];
 #pragma unroll
@@ -240,25 +322,24 @@ template <typename Item> __device__ __forceinline__ bool gen_item(const Item& I,
       I.keep(i * 13 + lane - 6, col[i]);
     }
   __syncwarp();
+#pragma unroll 1
+  for (int o = lane; o < 156; o += 32) {
+    const int x = o / 13, q = o % 13;
+    double acc = I.base_s(st, x, q);
 #pragma unroll
-  for (int y = 0; y < 5; ++y) {
-    const int o = lane + 32 * y, x = o / 13, q = o % 13;
-    if (o >= 156) break;
-    double acc = base[y];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) acc = fma(-left[y][k], zs[k][q], acc);
+    for (int k = 0; k < 6; ++k) acc = fma(-I.left_s(st, x, k), zs[k][q], acc);
     I.out(x, q, acc);
   }
   __syncwarp();
   return ok;
 }
 template <typename Item> __global__ void __launch_bounds__(128) k_gen_w(Batch b, ChainParts c, int lo, int hi) {
-  __shared__ double zs[4][6][13];
+  __shared__ double zs[4][6][13], stage[4][GEN_STAGE];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lo + blockIdx.x * 4 + warp;
   if (t >= hi) return;
   Item I{b, c};
   I.init(t);
-  const bool ok = gen_item(I, lane, zs[warp]);
+  const bool ok = gen_item(I, lane, stage[warp], zs[warp]);
   if (!ok && lane == 0) I.fail();
 }
 
@@ -267,6 +348,7 @@ struct GenRoot {
   int part;
   __device__ __forceinline__ double k(int i, int j) const { return chain_at(c.part, c.part_soa, CHAIN_GEN_PART, part, i * 12 + j); }
   __device__ __forceinline__ double f(int i) const { return chain_at(c.part, c.part_soa, CHAIN_GEN_PART, part, GP_F + i); }
+  __device__ __forceinline__ static bool minus(int, int) { return false; }
 };
 
 // Back substitution x = Z_0 - Z_p x_p - Z_n x_n, row i.
@@ -312,7 +394,7 @@ __global__ void k_gen_mid(Batch b, ChainParts c) {
 // The last levels of a chain, its root and their back substitution in one CTA, a
 // merge per warp.
 __global__ void __launch_bounds__(256) k_gen_top(Batch b, ChainParts c) {
-  __shared__ double zs[8][6][13];
+  __shared__ double zs[8][6][13], stage[8][GEN_STAGE];
   const ChainTop ch = c.chain[blockIdx.x];
   if (!solving(b, ch.structure)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -321,7 +403,7 @@ __global__ void __launch_bounds__(256) k_gen_top(Batch b, ChainParts c) {
     if (warp < k / 2) {
       GenMerge I{b, c};
       I.init(t0 + warp);
-      const bool ok = gen_item(I, lane, zs[warp]);
+      const bool ok = gen_item(I, lane, stage[warp], zs[warp]);
       if (!ok && lane == 0) I.fail();
     }
     __syncthreads();

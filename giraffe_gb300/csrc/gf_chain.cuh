@@ -29,11 +29,11 @@ namespace gf {
 constexpr int CHAIN_SYM_PART = 57, CHAIN_SYM_KEEP = 81, CHAIN_GEN_PART = 156, CHAIN_GEN_KEEP = 78;
 
 // Items below which an item per warp (half warp) is the faster form.  General: it
-// takes about 8 us for as many as there are sub-partitions (608), then 6 ns an
-// item, an item per thread about 55 us however few there are (its chain of 1,550
-// operations of 64 cycles), then half of that per item.  Symmetric: 4 us for
-// 1,216, then 3 ns, against 35 us.
-constexpr int CHAIN_GEN_SMALL = 152 * 4 * 16, CHAIN_SYM_SMALL = 152 * 4 * 20;
+// takes 8 us for as many as there are sub-partitions (608), then 5.3 ns an item, an
+// item per thread 98 us for anything up to 19,456 (its chain of 1,550 operations of
+// 64 cycles).  Symmetric: 7 us for 1,216, then 3.1 ns, against 41 us for 16,000 and
+// 55 us for 33,000.
+constexpr int CHAIN_GEN_SMALL = 152 * 4 * 28, CHAIN_SYM_SMALL = 152 * 4 * 20;
 
 // The chains of b.chain_gen (gf_chain.cu) and of b.chain_sym (gf_chain_sym.cu).
 void launch_gen_chains(const Batch& b, const ChainParts& c, cudaStream_t st);

@@ -19,57 +19,63 @@ __device__ __forceinline__ bool solving(const Batch& b, int s) {
 }
 
 // The last part of a chain with its end nodes, by one warp: 12 unknowns (u_p, a_p, u_n,
-// a_n), lane j column j of the matrix, lane 12 the right-hand side; fixed DOFs
-// are identity rows and columns, their pivots skipped.
+// a_n) by Gauss-Jordan, column j of the matrix in lanes j (rows 0-5) and 16 + j
+// (rows 6-11), column 12 the right-hand side; fixed DOFs are identity rows and
+// columns, their pivots skipped.  Bound by the chain of its pivots, 64 cycles an
+// FP64 operation: six updates a pivot here against eleven with a lane per column.
 template <typename Root>
 __device__ void chain_root(const Batch& b, const ChainParts& c, const ChainTop& ch, int lane, Root R) {
-  const int s = ch.structure;
-  const int node[2] = {c.corner_node[ch.first], c.corner_node[ch.last]};
-  const int g = lane < 12 ? b.gl[(int64_t)node[lane / 6] * 6 + lane % 6] : -1;
+  const int s = ch.structure, j = lane & 15, half = lane >> 4;
+  const int node0 = c.corner_node[ch.first], node1 = c.corner_node[ch.last];
+  const int g = lane < 12 ? b.gl[(int64_t)(lane < 6 ? node0 : node1) * 6 + lane % 6] : -1;
   const unsigned live = __ballot_sync(0xffffffffu, g >= 0);
   double* P = b.P + b.info[s].dof_off;
-  double col[12];
+  const double* nk = b.nodeK + (int64_t)(half ? node1 : node0) * 9;
+  // an entry and what comes on top of it, every load before the first sum
+  double col[6], add[6];
+  bool on[6], more[6];
 #pragma unroll
-  for (int i = 0; i < 12; ++i) {
-    double v = 0.0;
-    if (lane < 12) {
-      if ((live >> i & 1) && (live >> lane & 1)) {
-        v = R.k(i, lane);
-        if (i % 6 >= 3 && lane % 6 >= 3 && i / 6 == lane / 6)
-          v = radd(v, b.nodeK[(int64_t)node[i / 6] * 9 + (i % 6 - 3) * 3 + lane % 6 - 3]);
-      } else {
-        v = i == lane ? 1.0 : 0.0;
-      }
-    } else if (lane == 12 && (live >> i & 1)) {
-      v = radd(P[b.gl[(int64_t)node[i / 6] * 6 + i % 6]],
-               R.f(i));
-    }
-    col[i] = v;
+  for (int i = 0; i < 6; ++i) {
+    const int r = 6 * half + i, gi = __shfl_sync(0xffffffffu, g, r);
+    on[i] = (live >> r & 1) && (j == 12 || (j < 12 && (live >> j & 1)));
+    more[i] = on[i] && (j == 12 || (i >= 3 && j - 6 * half >= 3 && j - 6 * half < 6));
+    col[i] = on[i] ? (j == 12 ? R.f(r) : R.k(r, j)) : 0.0;
+    const double* at = j == 12 ? P + gi : nk + (i - 3) * 3 + j - 6 * half - 3;
+    add[i] = more[i] ? *at : 0.0;
+  }
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    if (j < 12 && R.minus(6 * half + i, j)) col[i] = -col[i];
+    if (!on[i]) col[i] = 6 * half + i == j ? 1.0 : 0.0;
+    if (more[i]) col[i] = radd(col[i], add[i]);
   }
   bool ok = true;
 #pragma unroll
   for (int k = 0; k < 12; ++k) {
     if (!(live >> k & 1)) continue;
-    const double p = __shfl_sync(0xffffffffu, col[k], k);
-    if (!(p != 0.0) || !isfinite(p)) ok = false;
+    const int kh = k / 6, kr = k % 6;
+    const double p = __shfl_sync(0xffffffffu, col[kr], 16 * kh + k);
+    ok = ok && !bad_pivot(p);
     const double inv = rcp64(p);
-    double m[12];
+    const double xk = __shfl_sync(0xffffffffu, col[kr], 16 * kh + j);
+    double m[6];
 #pragma unroll
-    for (int i = 0; i < 12; ++i) m[i] = __shfl_sync(0xffffffffu, col[i], k);
-    if (lane > k && lane < 13) {
-      const double rk = rmul(col[k], inv);
-      col[k] = rk;
+    for (int i = 0; i < 6; ++i) m[i] = __shfl_sync(0xffffffffu, col[i], 16 * half + k);
+    if (j > k && j < 13) {
+      const double rk = rmul(xk, inv);
 #pragma unroll
-      for (int i = 0; i < 12; ++i)
-        if (i != k) col[i] = rfma(-m[i], rk, col[i]);
+      for (int i = 0; i < 6; ++i) {
+        if (i == kr && half == kh) col[i] = rk;
+        else col[i] = rfma(-m[i], rk, col[i]);
+      }
     }
   }
   if (!ok && lane == 0) b.state[s].info_fail = 1;
   double x = 0.0;
 #pragma unroll
-  for (int i = 0; i < 12; ++i) {
-    const double v = __shfl_sync(0xffffffffu, col[i], 12);
-    if (lane == i) x = v;
+  for (int i = 0; i < 6; ++i) {
+    const double v = __shfl_sync(0xffffffffu, col[i], lane < 6 ? 12 : 28);
+    if (lane % 6 == i) x = v;
   }
   if (lane < 12) {
     c.x[6 * (int64_t)(lane < 6 ? ch.first : ch.last) + lane % 6] = g >= 0 ? x : 0.0;

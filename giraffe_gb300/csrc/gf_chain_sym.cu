@@ -45,6 +45,9 @@ static_assert(PT_HN + 6 == CHAIN_SYM_PART, "a part's entries");
 // the diagonal, the reciprocals of E.
 constexpr int KP_M = 60, KP_R = 75;
 static_assert(KP_R + 6 == CHAIN_SYM_KEEP, "an elimination's kept entries");
+// The half-warp form's staging area (doubles): two parts or K_e's triangle, zeros,
+// the forces of a midside node.
+constexpr int SYM_E2 = CHAIN_SYM_PART, SYM_ZERO = 120, SYM_F = 128, SYM_STAGE = 134;
 // Outputs: the 45 entries of the new stiffness, then the 9 forces h over (du,
 // a_p, a_n).
 constexpr int N_OUT = 54;
@@ -75,7 +78,7 @@ template <typename Item> __device__ __forceinline__ bool eliminate(const Item& I
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     const double p = D[lo6(k, k)];
-    if (!(p != 0.0) || !isfinite(p)) ok = false;
+    ok = ok && !bad_pivot(p);
     r[k] = rcp64(p);
     I.keep(KP_R + k, r[k]);
 #pragma unroll
@@ -115,32 +118,22 @@ template <typename Item> __device__ __forceinline__ bool eliminate(const Item& I
 
 // The same by a half warp (lanes 0-15 of its sixteen): lane q < 10 holds column q
 // of R, lane 10 + j column j of D from row j on; W and V go through shared memory
-// to the lanes that form the outputs.
+// to the lanes that form the outputs.  The operands go to shared memory first (st),
+// in one round of loads.
 template <typename Item>
-__device__ __forceinline__ bool eliminate_h(const Item& I, int lane, unsigned lanes, double (*ws)[10][6]) {
+__device__ __forceinline__ bool eliminate_h(const Item& I, int lane, unsigned lanes, double* st, double (*ws)[10][6]) {
   const int dj = lane - 10;
   const bool rhs = dj < 0;
+  I.stage(lane, lanes, st);
+  if (!I.active()) return true;
   double col[6], r[6], v[6];
 #pragma unroll
-  for (int i = 0; i < 6; ++i) col[i] = rhs ? I.r(i, lane) : (i >= dj ? I.d(i, dj) : 0.0);
-  // the outputs' starting values, loaded ahead of the dependent chain
-  double base[4];
-  int op[4], oq[4];
-#pragma unroll
-  for (int x = 0; x < 4; ++x) {
-    const int o = lane + 16 * x;
-    base[x] = 0.0;
-    if (o < N_OUT) {
-      out_pair(o, op[x], oq[x]);
-      base[x] = I.base(o, op[x], oq[x]);
-    }
-  }
-  if (!I.active()) return true;
+  for (int i = 0; i < 6; ++i) col[i] = I.column(st, i, lane);
   bool ok = true;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     const double p = __shfl_sync(lanes, col[k], 10 + k, 16);
-    if (!(p != 0.0) || !isfinite(p)) ok = false;
+    ok = ok && !bad_pivot(p);
     r[k] = rcp64(p);
     double d[6], x = col[k];
 #pragma unroll
@@ -163,14 +156,14 @@ __device__ __forceinline__ bool eliminate_h(const Item& I, int lane, unsigned la
       I.keep(i * 10 + lane, col[i]);
     }
   __syncwarp(lanes);
+#pragma unroll 1
+  for (int o = lane; o < N_OUT; o += 16) {
+    int p, q;
+    out_pair(o, p, q);
+    double acc = I.base_s(st, o, p, q);
 #pragma unroll
-  for (int x = 0; x < 4; ++x) {
-    const int o = lane + 16 * x;
-    if (o >= N_OUT) break;
-    double acc = base[x];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) acc = rfma(-ws[0][op[x]][i], ws[1][oq[x]][i], acc);
-    I.out(o, acc);
+    for (int i = 0; i < 6; ++i) acc = rfma(-ws[0][p][i], ws[1][q][i], acc);
+    I.out_s(st, o, acc);
   }
   __syncwarp(lanes);
   return ok;
@@ -204,11 +197,12 @@ struct Condense {
   __device__ __forceinline__ double base(int o, int p, int q) const { return o >= 45 ? 0.0 : k15(place(q), place(p)); }
   __device__ __forceinline__ void keep(int x, double v) const { chain_at(c.ez, c.elem_soa, CHAIN_SYM_KEEP, t, x) = v; }
   __device__ __forceinline__ void put(int x, double v) const { chain_at(c.part, c.part_soa, CHAIN_SYM_PART, t, x) = v; }
-  __device__ __forceinline__ void out(int o, double h) const {
+  __device__ __forceinline__ void out(int o, double h) const { out_f(o, h, [&](int i) { return force(i); }); }
+  template <typename Force> __device__ __forceinline__ void out_f(int o, double h, Force fo) const {
     if (o < 45) {
       put(o, h);
     } else if (o < 48) {  // half of the midside force to each end, and the pull of du
-      const double f = rmul(0.5, force(o - 45));
+      const double f = rmul(0.5, fo(o - 45));
       put(PT_HP + o - 45, rsub(f, h));
       put(PT_HN + o - 45, radd(f, h));
     } else if (o < 51) {
@@ -217,6 +211,26 @@ struct Condense {
       put(PT_HN + 3 + o - 51, h);
     }
   }
+  // The half-warp form: K_e's triangle at st[0], the midside node's forces at
+  // st[SYM_F].
+  __device__ __forceinline__ void stage(int lane, unsigned lanes, double* st) const {
+    double v[8], f = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = lane + 16 * q < 120 ? K[(int64_t)(lane + 16 * q) * ne] : 0.0;
+    if (lane < 6) f = P[lane];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) st[lane + 16 * q] = v[q];  // st[120 ..]: zeros
+    if (lane < 6) st[SYM_F + lane] = f;
+    __syncwarp(lanes);
+  }
+  __device__ __forceinline__ double column(const double* st, int i, int lane) const {
+    const int x = row(i), y = lane < 10 ? place(lane) : row(lane - 10);
+    return st[lane == 0 ? SYM_F + i : tri(x, y)];
+  }
+  __device__ __forceinline__ double base_s(const double* st, int o, int p, int q) const {
+    return st[o >= 45 ? SYM_ZERO : tri(place(q), place(p))];
+  }
+  __device__ __forceinline__ void out_s(const double* st, int o, double h) const { out_f(o, h, [&](int i) { return st[SYM_F + i]; }); }
   __device__ void fail() const { b.state[s].info_fail = 1; }
 };
 
@@ -259,17 +273,68 @@ struct Merge {
   __device__ __forceinline__ void keep(int x, double v) const { chain_at(c.mz, c.merge_soa, CHAIN_SYM_KEEP, t, x) = v; }
   __device__ __forceinline__ void put(int x, double v) const { chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.out, x) = v; }
   __device__ __forceinline__ void out(int o, double h) const {
+    out_f(o, h, [&](int i) { return force(i); }, [&](int x) { return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e1, x); },
+          [&](int x) { return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e2, x); });
+  }
+  template <typename Force, typename E1, typename E2>
+  __device__ __forceinline__ void out_f(int o, double h, Force fo, E1 e1, E2 e2) const {
     if (o < 45) {
       put(o, h);
     } else if (o < 48) {  // u_k = u_p + w: the corner's force passes to p
       const int i = o - 45;
-      put(PT_HP + i, radd(chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e1, PT_HP + i), rsub(force(i), h)));
-      put(PT_HN + i, radd(chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e2, PT_HN + i), h));
+      put(PT_HP + i, radd(e1(PT_HP + i), rsub(fo(i), h)));
+      put(PT_HN + i, radd(e2(PT_HN + i), h));
     } else if (o < 51) {
-      put(PT_HP + o - 45, radd(chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e1, PT_HP + o - 45), h));
+      put(PT_HP + o - 45, radd(e1(PT_HP + o - 45), h));
     } else {
-      put(PT_HN + o - 48, radd(chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e2, PT_HN + o - 48), h));
+      put(PT_HN + o - 48, radd(e2(PT_HN + o - 48), h));
     }
+  }
+  // The half-warp form: e1 at st[0], the corner's force added to its force on n,
+  // e2 at st[SYM_E2].
+  __device__ __forceinline__ void stage(int lane, unsigned lanes, double* st) const {
+    double v1[4], v2[4], f = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int x = lane + 16 * q;
+      v1[q] = x < CHAIN_SYM_PART ? chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e1, x) : 0.0;
+      v2[q] = x < CHAIN_SYM_PART ? chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e2, x) : 0.0;
+    }
+    if (lane < 6) f = b.P[m.dof + lane];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int x = lane + 16 * q;
+      if (x < CHAIN_SYM_PART) {
+        st[x] = v1[q];
+        st[SYM_E2 + x] = v2[q];
+      }
+    }
+    if (lane == 15) st[SYM_ZERO] = 0.0;
+    __syncwarp(lanes);
+    if (lane < 6) st[PT_HN + lane] = radd(f, st[PT_HN + lane]);
+    __syncwarp(lanes);
+  }
+  // Entry i of column lane (0: force, 1-3 du, 4-6 a_p, 7-9 a_n, 10 + j: column j of
+  // D): e1's entry plus or minus e2's.
+  __device__ __forceinline__ double column(const double* st, int i, int lane) const {
+    const int j = lane - 10, x1 = i < 3 ? i : 3 + i;  // the unknown among e1's places
+    const bool d = j >= 0, first = d || lane == 0 || (lane >= 4 && lane < 7), second = d || lane < 4 || lane >= 7;
+    const int y1 = d ? (j < 3 ? j : 3 + j) : lane - 1, y2 = d ? j : lane - 1;
+    const int p1 = lane == 0 ? PT_HN + i : x1 >= y1 ? lo6(x1, y1) : lo6(y1, x1);
+    const int p2 = SYM_E2 + (lane == 0 ? PT_HP + i : i >= y2 ? lo6(i, y2) : lo6(y2, i));
+    double v2 = st[second ? p2 : SYM_ZERO];
+    if (d ? (i >= 3 && j < 3) : (i < 3 && lane > 0)) v2 = -v2;
+    const double v1 = st[first ? p1 : SYM_ZERO];
+    return first ? radd(v1, v2) : v2;
+  }
+  __device__ __forceinline__ double base_s(const double* st, int o, int p, int q) const {
+    const int i = q - 1, j = p - 1;  // i >= j: places of the new part
+    const bool none = o >= 45 || (i >= 3 && i < 6 ? j < 3 : i >= 6 && j >= 3 && j < 6);
+    return st[none ? SYM_ZERO : (i >= 3 && i < 6 ? 0 : SYM_E2) + lo6(i, j)];
+  }
+  __device__ __forceinline__ void out_s(const double* st, int o, double h) const {
+    out_f(o, h, [&](int i) { return radd(st[PT_HN + i], st[SYM_E2 + PT_HP + i]); }, [&](int x) { return st[x]; },
+          [&](int x) { return st[SYM_E2 + x]; });
   }
   __device__ void fail() const { b.state[m.structure].info_fail = 1; }
 };
@@ -283,13 +348,13 @@ template <typename Item> __global__ void __launch_bounds__(CT) k_sym(Batch b, Ch
   if (!eliminate(I)) I.fail();
 }
 template <typename Item> __global__ void __launch_bounds__(128) k_sym_h(Batch b, ChainParts c, int lo, int hi) {
-  __shared__ double ws[8][2][10][6];
+  __shared__ double ws[8][2][10][6], stage[8][SYM_STAGE];
   const int half = threadIdx.x >> 4, lane = threadIdx.x & 15, t = lo + blockIdx.x * 8 + half;
   const unsigned lanes = 0xFFFFu << (threadIdx.x & 16);
   if (t >= hi) return;
   Item I{b, c};
   I.init(t);
-  const bool ok = eliminate_h(I, lane, lanes, ws[half]);
+  const bool ok = eliminate_h(I, lane, lanes, stage[half], ws[half]);
   if (!ok && lane == 0) I.fail();
 }
 
@@ -299,9 +364,9 @@ struct SymRoot {
   int part;
   __device__ __forceinline__ double k(int i, int j) const {
     const int x = i < 6 ? i : i < 9 ? i - 6 : i - 3, y = j < 6 ? j : j < 9 ? j - 6 : j - 3;
-    const double v = chain_at(c.part, c.part_soa, CHAIN_SYM_PART, part, x >= y ? lo6(x, y) : lo6(y, x));
-    return (i < 3) != (j < 3) ? -v : v;
+    return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, part, x >= y ? lo6(x, y) : lo6(y, x));
   }
+  __device__ __forceinline__ static bool minus(int i, int j) { return (i < 3) != (j < 3); }
   __device__ __forceinline__ double f(int i) const { return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, part, PT_HP + i); }
 };
 
@@ -377,7 +442,7 @@ __global__ void k_sym_mid(Batch b, ChainParts c) {
 // substitution.  Against a launch per level this drops the launches and the
 // round trips through L2 between levels of a few items.
 __global__ void __launch_bounds__(128) k_sym_top(Batch b, ChainParts c) {
-  __shared__ double ws[8][2][10][6];
+  __shared__ double ws[8][2][10][6], stage[8][SYM_STAGE];
   const ChainTop ch = c.chain[blockIdx.x];
   if (!solving(b, ch.structure)) return;
   const int half = threadIdx.x >> 4, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -387,7 +452,7 @@ __global__ void __launch_bounds__(128) k_sym_top(Batch b, ChainParts c) {
     if (half < k / 2) {
       Merge I{b, c};
       I.init(t0 + half);
-      const bool ok = eliminate_h(I, threadIdx.x & 15, lanes, ws[half]);
+      const bool ok = eliminate_h(I, threadIdx.x & 15, lanes, stage[half], ws[half]);
       if (!ok && (threadIdx.x & 15) == 0) I.fail();
     }
     __syncthreads();

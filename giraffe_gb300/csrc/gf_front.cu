@@ -61,12 +61,7 @@ template <typename T> __device__ __forceinline__ void mf_fail(const Batch& b, in
   if (sizeof(T) == 8) b.state[s].info_fail = 1;
   else b.state[s].ir_fb = 1;
 }
-// Zero, infinite or NaN, from the bits: an FP64 comparison would hold the pivot's
-// chain up for 64 cycles.
-__device__ __forceinline__ bool mf_bad(double p) {
-  const int h = __double2hiint(p) & 0x7FFFFFFF;
-  return (h | __double2loint(p)) == 0 || h >= 0x7FF00000;
-}
+__device__ __forceinline__ bool mf_bad(double p) { return bad_pivot(p); }
 __device__ __forceinline__ bool mf_bad(float p) {
   const int h = __float_as_int(p) & 0x7FFFFFFF;
   return h == 0 || h >= 0x7F800000;

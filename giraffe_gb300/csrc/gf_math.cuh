@@ -96,6 +96,12 @@ template <typename T, typename S> GF_HD V3<T> cvt(const V3<S>& a) {
 }
 
 #ifdef __CUDACC__
+// Zero, infinite or NaN, from the bits: an FP64 comparison takes the 64 cycles of
+// any FP64 instruction out of a pivot's chain.
+__device__ __forceinline__ bool bad_pivot(double p) {
+  const int h = __double2hiint(p) & 0x7FFFFFFF;
+  return (h | __double2loint(p)) == 0 || h >= 0x7FF00000;
+}
 // 1/p from a single-precision seed of p's own bits (r0, 2^-23) and one
 // third-order step r = r0 + r0 (e + e^2), e = 1 - p r0 (2^-69): three dependent
 // FP64 results (64 cycles each on this part) in place of the six of two
