@@ -209,7 +209,7 @@ struct GenMerge {
     if (lane < 15) s[lane < 9 ? (9 + lane / 3) * 12 + 9 + lane % 3 : GP_F + 6 + f] += extra;
     __syncwarp();
   }
-  __device__ __forceinline__ void column(int lane, int& a, int& sa, int& o, int& so) const {
+  __device__ __forceinline__ static void column(int lane, int& a, int& sa, int& o, int& so) {
     const int q = lane - 6;
     const bool first = lane < 6 || q == 0 || (q > 0 && q < 7), second = lane < 6 || q == 0 || (q >= 7 && lane < NC);
     a = !first ? GEN_ZERO : q == 0 ? GP_F + 6 : 72 + (lane < 6 ? 6 + lane : q - 1);
@@ -218,9 +218,10 @@ struct GenMerge {
     so = !second ? 0 : q == 0 ? 1 : 12;
   }
   // entry i of column `lane` where the corner is fixed
-  __device__ __forceinline__ double pinned(int i, int lane, double v) const {
-    if (lane < 6 && !(live(i) && live(lane))) return i == lane ? 1.0 : 0.0;
-    return lane == 6 && !live(i) ? 0.0 : v;
+  __device__ __forceinline__ double pinned(int i, int lane, double v) const { return pinned(m.mask, i, lane, v); }
+  __device__ __forceinline__ static double pinned(int mask, int i, int lane, double v) {
+    if (lane < 6 && !((mask >> i & 1) && (mask >> lane & 1))) return i == lane ? 1.0 : 0.0;
+    return lane == 6 && !(mask >> i & 1) ? 0.0 : v;
   }
   __device__ __forceinline__ static double left_s(const double* s, int x, int k) {
     return s[x < 6 ? x * 12 + 6 + k : GEN_E2 + x * 12 + k];
@@ -344,23 +345,22 @@ template <typename Item> __global__ void __launch_bounds__(128) k_gen_w(Batch b,
 }
 
 struct GenRoot {
-  const ChainParts& c;
-  int part;
-  __device__ __forceinline__ double k(int i, int j) const { return chain_at(c.part, c.part_soa, CHAIN_GEN_PART, part, i * 12 + j); }
-  __device__ __forceinline__ double f(int i) const { return chain_at(c.part, c.part_soa, CHAIN_GEN_PART, part, GP_F + i); }
+  const double* part;
+  __device__ __forceinline__ double k(int i, int j) const { return part[i * 12 + j]; }
+  __device__ __forceinline__ double f(int i) const { return part[GP_F + i]; }
   __device__ __forceinline__ static bool minus(int, int) { return false; }
 };
 
 // Back substitution x = Z_0 - Z_p x_p - Z_n x_n, row i.
 template <typename Kept>
-__device__ __forceinline__ double gen_back(const ChainParts& c, int p, int n, int i, Kept kept) {
+__device__ __forceinline__ double gen_back(const double* xps, const double* xns, int i, Kept kept) {
   double z[13], xp[6], xn[6];
 #pragma unroll
   for (int j = 0; j < 13; ++j) z[j] = kept(i * 13 + j);
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
-    xp[j] = c.x[6 * (int64_t)(p) + j];
-    xn[j] = c.x[6 * (int64_t)(n) + j];
+    xp[j] = xps[j];
+    xn[j] = xns[j];
   }
   double x = z[0];
 #pragma unroll
@@ -371,7 +371,7 @@ __device__ __forceinline__ double gen_back(const ChainParts& c, int p, int n, in
   return x;
 }
 __device__ __forceinline__ void gen_corner(const Batch& b, const ChainParts& c, int t, const ChainMerge& m, int i) {
-  const double x = gen_back(c, m.p, m.n, i, [&](int q) { return chain_at(c.mz, c.merge_soa, CHAIN_GEN_KEEP, t, q); });
+  const double x = gen_back(c.x + 6 * (int64_t)m.p, c.x + 6 * (int64_t)m.n, i, [&](int q) { return chain_at(c.mz, c.merge_soa, CHAIN_GEN_KEEP, t, q); });
   c.x[6 * (int64_t)(m.k) + i] = x;
   if (m.mask >> i & 1) b.P[m.dof + __popc(m.mask & ((1 << i) - 1))] = x;
 }
@@ -388,34 +388,87 @@ __global__ void k_gen_mid(Batch b, ChainParts c) {
   const int t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 5 + lane / 6;
   if (lane >= 30 || t >= c.n_elem || !solving(b, c.elem_struct[t])) return;
   const int p = c.elem_corner[t];
-  b.P[c.elem_dof[t] + i] = gen_back(c, p, p + 1, i, [&](int q) { return chain_at(c.ez, c.elem_soa, CHAIN_GEN_KEEP, t, q); });
+  b.P[c.elem_dof[t] + i] = gen_back(c.x + 6 * (int64_t)p, c.x + 6 * (int64_t)(p + 1), i, [&](int q) { return chain_at(c.ez, c.elem_soa, CHAIN_GEN_KEEP, t, q); });
 }
 
 // The last levels of a chain, its root and their back substitution in one CTA, a
-// merge per warp.
-__global__ void __launch_bounds__(256) k_gen_top(Batch b, ChainParts c) {
-  __shared__ double zs[8][6][13], stage[8][GEN_STAGE];
+// merge per warp, as k_sym_top.
+struct GenTopShared {
+  ChainTopShared t;
+  double nk[TOP_MERGES][9];  // load stiffness of the corners
+  double part[TOP_MERGES][CHAIN_GEN_PART];
+  double kept[TOP_MERGES][CHAIN_GEN_KEEP];
+  double zs[TOP_THREADS / 32][6][13], stage[TOP_THREADS / 32][GEN_STAGE];
+};
+struct GenTopMerge {
+  const ChainParts& c;
+  GenTopShared& S;
+  int t;
+  __device__ __forceinline__ static bool active() { return true; }
+  __device__ __forceinline__ void stage(int lane, double* s) const {
+    double v[10];
+#pragma unroll
+    for (int q = 0; q < 10; ++q) {
+      const int y = lane + 32 * (q % 5), o = q < 5 ? S.t.part1[t] : S.t.part2[t], e = q < 5 ? S.t.m[t].e1 : S.t.m[t].e2;
+      v[q] = y >= CHAIN_GEN_PART ? 0.0 : o >= 0 ? S.part[o][y] : chain_at(c.part, c.part_soa, CHAIN_GEN_PART, e, y);
+    }
+#pragma unroll
+    for (int q = 0; q < 10; ++q)
+      if (lane + 32 * (q % 5) < CHAIN_GEN_PART) s[(q < 5 ? 0 : GEN_E2) + lane + 32 * (q % 5)] = v[q];
+    if (lane == 31) s[GEN_ZERO] = 0.0;
+    __syncwarp();
+    if (lane < 15)
+      s[lane < 9 ? (9 + lane / 3) * 12 + 9 + lane % 3 : GP_F + 6 + lane - 9] += lane < 9 ? S.nk[t][lane] : S.t.f[t][lane - 9];
+    __syncwarp();
+  }
+  __device__ __forceinline__ static void column(int lane, int& a, int& sa, int& o, int& so) { GenMerge::column(lane, a, sa, o, so); }
+  __device__ __forceinline__ double pinned(int i, int lane, double v) const { return GenMerge::pinned(S.t.m[t].mask, i, lane, v); }
+  __device__ __forceinline__ static double left_s(const double* s, int x, int k) { return GenMerge::left_s(s, x, k); }
+  __device__ __forceinline__ static double base_s(const double* s, int x, int q) { return GenMerge::base_s(s, x, q); }
+  __device__ __forceinline__ void keep(int x, double v) const { S.kept[t][x] = v; }
+  __device__ __forceinline__ void out(int x, int q, double v) const { S.part[t][q == 0 ? GP_F + x : x * 12 + q - 1] = v; }
+};
+__global__ void __launch_bounds__(TOP_THREADS) k_gen_top(Batch b, ChainParts c) {
+  extern __shared__ __align__(16) unsigned char gen_top_raw[];
+  GenTopShared& S = *reinterpret_cast<GenTopShared*>(gen_top_raw);
   const ChainTop ch = c.chain[blockIdx.x];
   if (!solving(b, ch.structure)) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int t0 = ch.top;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = ch.n_top - 1;
+  top_load(b, c, ch, tid, S.t);
+  for (int y = tid; y < 9 * n; y += TOP_THREADS)
+    S.nk[y / 9][y % 9] = b.nodeK[(int64_t)c.corner_node[S.t.m[y / 9].k] * 9 + y % 9];
+  __syncthreads();
+  int t0 = 0;
   for (int k = ch.n_top; k > 1; t0 += k / 2, k = (k + 1) / 2) {
-    if (warp < k / 2) {
-      GenMerge I{b, c};
-      I.init(t0 + warp);
-      const bool ok = gen_item(I, lane, stage[warp], zs[warp]);
-      if (!ok && lane == 0) I.fail();
+    for (int w = warp; w < k / 2; w += TOP_THREADS / 32) {
+      const GenTopMerge I{c, S, t0 + w};
+      const bool ok = gen_item(I, lane, S.stage[warp], S.zs[warp]);
+      if (!ok && lane == 0) b.state[ch.structure].info_fail = 1;
     }
     __syncthreads();
   }
-  if (warp == 0) chain_root(b, c, ch, lane, GenRoot{c, ch.root});
+  if (warp == 0) {
+    if (n == 0) {
+      for (int x = lane; x < CHAIN_GEN_PART; x += 32)
+        S.part[0][x] = chain_at(c.part, c.part_soa, CHAIN_GEN_PART, ch.root, x);
+      __syncwarp();
+    }
+    chain_root(b, c, ch, lane, GenRoot{S.part[max(n - 1, 0)]}, S.t.x[TOP_FIRST]);
+  }
   __syncthreads();
-  int cnt[5], n = 0;
-  for (int k = ch.n_top; k > 1; k = (k + 1) / 2) cnt[n++] = k / 2;
-  for (int l = n - 1; l >= 0; --l) {
+  int cnt[6], nl = 0;
+  for (int k = ch.n_top; k > 1; k = (k + 1) / 2) cnt[nl++] = k / 2;
+  for (int l = nl - 1; l >= 0; --l) {
     t0 -= cnt[l];
-    const int q = warp * 5 + lane / 6;
-    if (lane < 30 && q < cnt[l]) gen_corner(b, c, t0 + q, c.merge[t0 + q], lane % 6);
+    const int i = lane % 6, q = warp * 5 + lane / 6;
+    if (lane < 30 && q < cnt[l]) {
+      const int t = t0 + q;
+      const ChainMerge& m = S.t.m[t];
+      const double x = gen_back(S.t.x[S.t.p[t]], S.t.x[S.t.n[t]], i, [&](int y) { return S.kept[t][y]; });
+      S.t.x[t][i] = x;
+      c.x[6 * (int64_t)m.k + i] = x;
+      if (m.mask >> i & 1) b.P[m.dof + __popc(m.mask & ((1 << i) - 1))] = x;
+    }
     __syncthreads();
   }
 }
@@ -433,7 +486,12 @@ void launch_gen_chains(const Batch& b, const ChainParts& c, cudaStream_t st) {
     if (hi <= c.merge_soa) k_gen<GenMerge><<<grid_for(hi - lo, CT), CT, GEN_SMEM, st>>>(b, c, lo, hi);
     else k_gen_w<GenMerge><<<grid_for(hi - lo, 4), 128, 0, st>>>(b, c, lo, hi);
   }
-  k_gen_top<<<c.n_chains, 256, 0, st>>>(b, c);
+  static const bool done = [] {  // once per process, thread-safe
+    cudaFuncSetAttribute(k_gen_top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GenTopShared));
+    return true;
+  }();
+  (void)done;
+  k_gen_top<<<c.n_chains, TOP_THREADS, sizeof(GenTopShared), st>>>(b, c);
   for (int l = c.n_levels - 1; l >= 0; --l) {
     const int lo = c.merge_off[l], hi = c.merge_off[l + 1];
     k_gen_back<<<grid_for(hi - lo, 20), 128, 0, st>>>(b, c, lo, hi);

@@ -107,7 +107,7 @@ template <typename Item> __device__ __forceinline__ bool eliminate(const Item& I
 #pragma unroll
     for (int p = 0; p <= q; ++p) {
       const int o = p == 0 ? 44 + q : lo6(q - 1, p - 1);
-      double acc = I.base(o, p, q);
+      double acc = I.start(o, p, q);
 #pragma unroll
       for (int i = 0; i < 6; ++i) acc = rfma(-W[p][i], v[i], acc);
       I.out(o, acc);
@@ -116,53 +116,87 @@ template <typename Item> __device__ __forceinline__ bool eliminate(const Item& I
   return ok;
 }
 
-// The same by a half warp (lanes 0-15 of its sixteen): lane q < 10 holds column q
-// of R, lane 10 + j column j of D from row j on; W and V go through shared memory
-// to the lanes that form the outputs.  The operands go to shared memory first (st),
-// in one round of loads.
-template <typename Item>
-__device__ __forceinline__ bool eliminate_h(const Item& I, int lane, unsigned lanes, double* st, double (*ws)[10][6]) {
-  const int dj = lane - 10;
-  const bool rhs = dj < 0;
+// What a lane of the half-warp form reads of an item's staged operands, the same for
+// every item: entry i of its column is st[a[i]] plus (minus where neg's bit i is
+// set) st[b[i]]; output o[x] & 63 starts from st[o[x] >> 16] and takes columns p, q
+// (bits 6-9, 10-13).
+template <int LANES> struct SymLane {
+  static constexpr int OUTS = (N_OUT + LANES - 1) / LANES;
+  int a[6], b[6], o[OUTS];
+  unsigned neg;
+  bool sum;  // both terms (else the first alone)
+  template <typename Item> __device__ __forceinline__ void init(int lane) {
+    neg = 0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) Item::column(i, lane & 15, a[i], b[i], neg, sum);
+#pragma unroll
+    for (int x = 0; x < OUTS; ++x) {
+      const int y = lane + LANES * x;
+      int p = 0, q = 1;
+      if (y < N_OUT) out_pair(y, p, q);
+      o[x] = min(y, N_OUT) | p << 6 | q << 10 | Item::base(min(y, N_OUT - 1), p, q) << 16;
+    }
+  }
+};
+
+// The same by a half warp (lane 0-15; LANES = 16) or by both halves of a warp, which
+// then share the outputs (LANES = 32): lane q < 10 holds column q of R, lane 10 + j
+// column j of D from row j on; W and V go through shared memory to the lanes that
+// form the outputs.  The operands go to shared memory first (st), in one round of
+// loads.
+template <int LANES, typename Item>
+__device__ __forceinline__ bool eliminate_h(const Item& I, const SymLane<LANES>& L, int lane, unsigned lanes, double* st,
+                                            double (*ws)[10][6]) {
+  const int x = lane & 15, dj = x - 10;
+  const bool rhs = dj < 0, writes = lane == x;
   I.stage(lane, lanes, st);
   if (!I.active()) return true;
   double col[6], r[6], v[6];
 #pragma unroll
-  for (int i = 0; i < 6; ++i) col[i] = I.column(st, i, lane);
+  for (int i = 0; i < 6; ++i) {
+    col[i] = st[L.a[i]];
+    if (Item::SUMS) {
+      double y = st[L.b[i]];
+      if (L.neg >> i & 1) y = -y;
+      y = radd(col[i], y);
+      col[i] = L.sum ? y : L.neg >> i & 1 ? -col[i] : col[i];
+    }
+  }
   bool ok = true;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     const double p = __shfl_sync(lanes, col[k], 10 + k, 16);
     ok = ok && !bad_pivot(p);
     r[k] = rcp64(p);
-    double d[6], x = col[k];
+    double d[6], y = col[k];
 #pragma unroll
     for (int i = k + 1; i < 6; ++i) {
       d[i] = __shfl_sync(lanes, col[i], 10 + k, 16);
-      if (dj == i) x = d[i];
+      if (dj == i) y = d[i];
       if (lane == 15) I.keep(KP_M + lo6(i - 1, k), d[i]);
     }
-    v[k] = rmul(r[k], x);
+    v[k] = rmul(r[k], y);
 #pragma unroll
     for (int i = k + 1; i < 6; ++i)
       if (rhs || (dj > k && i >= dj)) col[i] = rfma(-d[i], v[k], col[i]);
     if (lane == 15) I.keep(KP_R + k, r[k]);
   }
-  if (rhs)
+  if (rhs && writes)
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-      ws[0][lane][i] = col[i];
-      ws[1][lane][i] = v[i];
-      I.keep(i * 10 + lane, col[i]);
+      ws[0][x][i] = col[i];
+      ws[1][x][i] = v[i];
+      I.keep(i * 10 + x, col[i]);
     }
   __syncwarp(lanes);
-#pragma unroll 1
-  for (int o = lane; o < N_OUT; o += 16) {
-    int p, q;
-    out_pair(o, p, q);
-    double acc = I.base_s(st, o, p, q);
 #pragma unroll
-    for (int i = 0; i < 6; ++i) acc = rfma(-ws[0][p][i], ws[1][q][i], acc);
+  for (int y = 0; y < SymLane<LANES>::OUTS; ++y) {
+    const int o = L.o[y] & 63;
+    if (o >= N_OUT) break;
+    const double *w = ws[0][L.o[y] >> 6 & 15], *u = ws[1][L.o[y] >> 10 & 15];
+    double acc = st[L.o[y] >> 16];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) acc = rfma(-w[i], u[i], acc);
     I.out_s(st, o, acc);
   }
   __syncwarp(lanes);
@@ -194,7 +228,7 @@ struct Condense {
   __device__ __forceinline__ double d(int i, int j) const { return k15(row(i), row(j)); }
   __device__ __forceinline__ double force(int i) const { return P[i]; }
   __device__ __forceinline__ double r(int i, int q) const { return q == 0 ? force(i) : k15(row(i), place(q)); }
-  __device__ __forceinline__ double base(int o, int p, int q) const { return o >= 45 ? 0.0 : k15(place(q), place(p)); }
+  __device__ __forceinline__ double start(int o, int p, int q) const { return o >= 45 ? 0.0 : k15(place(q), place(p)); }
   __device__ __forceinline__ void keep(int x, double v) const { chain_at(c.ez, c.elem_soa, CHAIN_SYM_KEEP, t, x) = v; }
   __device__ __forceinline__ void put(int x, double v) const { chain_at(c.part, c.part_soa, CHAIN_SYM_PART, t, x) = v; }
   __device__ __forceinline__ void out(int o, double h) const { out_f(o, h, [&](int i) { return force(i); }); }
@@ -223,13 +257,14 @@ struct Condense {
     if (lane < 6) st[SYM_F + lane] = f;
     __syncwarp(lanes);
   }
-  __device__ __forceinline__ double column(const double* st, int i, int lane) const {
+  static constexpr bool SUMS = false;
+  __device__ __forceinline__ static void column(int i, int lane, int& a, int& b, unsigned& neg, bool& sum) {
     const int x = row(i), y = lane < 10 ? place(lane) : row(lane - 10);
-    return st[lane == 0 ? SYM_F + i : tri(x, y)];
+    a = lane == 0 ? SYM_F + i : tri(x, y);
+    b = SYM_ZERO;
+    sum = false;
   }
-  __device__ __forceinline__ double base_s(const double* st, int o, int p, int q) const {
-    return st[o >= 45 ? SYM_ZERO : tri(place(q), place(p))];
-  }
+  __device__ __forceinline__ static int base(int o, int p, int q) { return o >= 45 ? SYM_ZERO : tri(place(q), place(p)); }
   __device__ __forceinline__ void out_s(const double* st, int o, double h) const { out_f(o, h, [&](int i) { return st[SYM_F + i]; }); }
   __device__ void fail() const { b.state[s].info_fail = 1; }
 };
@@ -263,7 +298,7 @@ struct Merge {
     if (q < 7) return i < 3 ? E(m.e1, q - 1, i) : E(m.e1, 3 + i, q - 1);     // a_p (place 3 + q - 4)
     return i < 3 ? -E(m.e2, q - 1, i) : E(m.e2, q - 1, i);                   // a_n (place 6 + q - 7)
   }
-  __device__ __forceinline__ double base(int o, int p, int q) const {
+  __device__ __forceinline__ double start(int o, int p, int q) const {
     if (o >= 45) return 0.0;
     const int i = q - 1, j = p - 1;  // i >= j: places of the new part
     if (i < 3) return E(m.e2, i, j);
@@ -272,17 +307,14 @@ struct Merge {
   }
   __device__ __forceinline__ void keep(int x, double v) const { chain_at(c.mz, c.merge_soa, CHAIN_SYM_KEEP, t, x) = v; }
   __device__ __forceinline__ void put(int x, double v) const { chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.out, x) = v; }
+  __device__ __forceinline__ double e1(int x) const { return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e1, x); }
+  __device__ __forceinline__ double e2(int x) const { return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e2, x); }
   __device__ __forceinline__ void out(int o, double h) const {
-    out_f(o, h, [&](int i) { return force(i); }, [&](int x) { return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e1, x); },
-          [&](int x) { return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, m.e2, x); });
-  }
-  template <typename Force, typename E1, typename E2>
-  __device__ __forceinline__ void out_f(int o, double h, Force fo, E1 e1, E2 e2) const {
     if (o < 45) {
       put(o, h);
     } else if (o < 48) {  // u_k = u_p + w: the corner's force passes to p
       const int i = o - 45;
-      put(PT_HP + i, radd(e1(PT_HP + i), rsub(fo(i), h)));
+      put(PT_HP + i, radd(e1(PT_HP + i), rsub(force(i), h)));
       put(PT_HN + i, radd(e2(PT_HN + i), h));
     } else if (o < 51) {
       put(PT_HP + o - 45, radd(e1(PT_HP + o - 45), h));
@@ -314,27 +346,39 @@ struct Merge {
     if (lane < 6) st[PT_HN + lane] = radd(f, st[PT_HN + lane]);
     __syncwarp(lanes);
   }
-  // Entry i of column lane (0: force, 1-3 du, 4-6 a_p, 7-9 a_n, 10 + j: column j of
-  // D): e1's entry plus or minus e2's.
-  __device__ __forceinline__ double column(const double* st, int i, int lane) const {
+  // Column lane (0: force, 1-3 du, 4-6 a_p, 7-9 a_n, 10 + j: column j of D): e1's
+  // entry plus or minus e2's, or one of them.
+  static constexpr bool SUMS = true;
+  __device__ __forceinline__ static void column(int i, int lane, int& a, int& b, unsigned& neg, bool& sum) {
     const int j = lane - 10, x1 = i < 3 ? i : 3 + i;  // the unknown among e1's places
-    const bool d = j >= 0, first = d || lane == 0 || (lane >= 4 && lane < 7), second = d || lane < 4 || lane >= 7;
+    const bool d = j >= 0, first = d || lane == 0 || (lane >= 4 && lane < 7);
     const int y1 = d ? (j < 3 ? j : 3 + j) : lane - 1, y2 = d ? j : lane - 1;
     const int p1 = lane == 0 ? PT_HN + i : x1 >= y1 ? lo6(x1, y1) : lo6(y1, x1);
     const int p2 = SYM_E2 + (lane == 0 ? PT_HP + i : i >= y2 ? lo6(i, y2) : lo6(y2, i));
-    double v2 = st[second ? p2 : SYM_ZERO];
-    if (d ? (i >= 3 && j < 3) : (i < 3 && lane > 0)) v2 = -v2;
-    const double v1 = st[first ? p1 : SYM_ZERO];
-    return first ? radd(v1, v2) : v2;
+    sum = d || lane == 0;
+    a = first ? p1 : p2;
+    b = sum ? p2 : SYM_ZERO;
+    if (d ? (i >= 3 && j < 3) : (i < 3 && lane > 0 && !first)) neg |= 1u << i;
   }
-  __device__ __forceinline__ double base_s(const double* st, int o, int p, int q) const {
+  __device__ __forceinline__ static int base(int o, int p, int q) {
     const int i = q - 1, j = p - 1;  // i >= j: places of the new part
     const bool none = o >= 45 || (i >= 3 && i < 6 ? j < 3 : i >= 6 && j >= 3 && j < 6);
-    return st[none ? SYM_ZERO : (i >= 3 && i < 6 ? 0 : SYM_E2) + lo6(i, j)];
+    return none ? SYM_ZERO : (i >= 3 && i < 6 ? 0 : SYM_E2) + lo6(i, j);
   }
   __device__ __forceinline__ void out_s(const double* st, int o, double h) const {
-    out_f(o, h, [&](int i) { return radd(st[PT_HN + i], st[SYM_E2 + PT_HP + i]); }, [&](int x) { return st[x]; },
-          [&](int x) { return st[SYM_E2 + x]; });
+    out_st(st, o, h, [&](int x, double v) { put(x, v); });
+  }
+  // out() from the staged parts, the force outputs along one path
+  template <typename Put> __device__ __forceinline__ static void out_st(const double* st, int o, double h, Put put) {
+    if (o < 45) {
+      put(o, h);
+      return;
+    }
+    const int i = o - 45;
+    double t = h;
+    if (i < 3) t = rsub(radd(st[PT_HN + i], st[SYM_E2 + PT_HP + i]), h);
+    put(i < 6 ? PT_HP + i : PT_HN + i - 3, radd(st[i < 6 ? PT_HP + i : SYM_E2 + PT_HN + i - 3], t));
+    if (i < 3) put(PT_HN + i, radd(st[SYM_E2 + PT_HN + i], h));
   }
   __device__ void fail() const { b.state[m.structure].info_fail = 1; }
 };
@@ -354,20 +398,21 @@ template <typename Item> __global__ void __launch_bounds__(128) k_sym_h(Batch b,
   if (t >= hi) return;
   Item I{b, c};
   I.init(t);
-  const bool ok = eliminate_h(I, lane, lanes, stage[half], ws[half]);
+  SymLane<16> L;
+  L.init<Item>(lane);
+  const bool ok = eliminate_h<16>(I, L, lane, lanes, stage[half], ws[half]);
   if (!ok && lane == 0) I.fail();
 }
 
 // The last part as a 12x12 matrix: the sign of u_p in du.
 struct SymRoot {
-  const ChainParts& c;
-  int part;
+  const double* part;
   __device__ __forceinline__ double k(int i, int j) const {
     const int x = i < 6 ? i : i < 9 ? i - 6 : i - 3, y = j < 6 ? j : j < 9 ? j - 6 : j - 3;
-    return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, part, x >= y ? lo6(x, y) : lo6(y, x));
+    return part[x >= y ? lo6(x, y) : lo6(y, x)];
   }
   __device__ __forceinline__ static bool minus(int i, int j) { return (i < 3) != (j < 3); }
-  __device__ __forceinline__ double f(int i) const { return chain_at(c.part, c.part_soa, CHAIN_SYM_PART, part, PT_HP + i); }
+  __device__ __forceinline__ double f(int i) const { return part[PT_HP + i]; }
 };
 
 // Back substitution of one elimination: E x = L^-1-reduced right-hand side, i.e.
@@ -391,19 +436,19 @@ __device__ __forceinline__ double back(unsigned lanes, int l0, int i, const doub
   }
   return rmul(y, r);
 }
-__device__ __forceinline__ void around(const ChainParts& c, int p, int n, double (&z)[9]) {
+__device__ __forceinline__ void around(const double* xp, const double* xn, double (&z)[9]) {
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
-    z[j] = rsub(c.x[6 * (int64_t)(n) + j], c.x[6 * (int64_t)(p) + j]);
-    z[3 + j] = c.x[6 * (int64_t)(p) + 3 + j];
-    z[6 + j] = c.x[6 * (int64_t)(n) + 3 + j];
+    z[j] = rsub(xn[j], xp[j]);
+    z[3 + j] = xp[3 + j];
+    z[6 + j] = xn[3 + j];
   }
 }
 // Corner of merge t, row i.
 __device__ __forceinline__ void back_corner(const Batch& b, const ChainParts& c, int t, const ChainMerge& m, unsigned lanes,
                                             int l0, int i) {
   double z[9];
-  around(c, m.p, m.n, z);
+  around(c.x + 6 * (int64_t)m.p, c.x + 6 * (int64_t)m.n, z);
   double x = back(lanes, l0, i, z, [&](int q) { return chain_at(c.mz, c.merge_soa, CHAIN_SYM_KEEP, t, q); });
   if (i < 3) x = radd(x, c.x[6 * (int64_t)(m.p) + i]);  // u_k = u_p + w
   c.x[6 * (int64_t)(m.k) + i] = x;
@@ -431,43 +476,119 @@ __global__ void k_sym_mid(Batch b, ChainParts c) {
   if (!on) return;
   const int p = c.elem_corner[t];
   double z[9];
-  around(c, p, p + 1, z);
+  around(c.x + 6 * (int64_t)p, c.x + 6 * (int64_t)(p + 1), z);
   double x = back(lanes, lane - i, i, z, [&](int q) { return chain_at(c.ez, c.elem_soa, CHAIN_SYM_KEEP, t, q); });
   if (i < 3) x = rfma(0.5, radd(c.x[6 * (int64_t)(p) + i], c.x[6 * (int64_t)(p + 1) + i]), x);
   b.P[c.elem_dof[t] + i] = x;
 }
 
 // The last levels of a chain in one CTA, from at most CHAIN_TOP parts on: its
-// merges level by level (a half warp each), the root, and their back
-// substitution.  Against a launch per level this drops the launches and the
-// round trips through L2 between levels of a few items.
-__global__ void __launch_bounds__(128) k_sym_top(Batch b, ChainParts c) {
-  __shared__ double ws[8][2][10][6], stage[8][SYM_STAGE];
+// merges level by level, the root, and their back substitution, the
+// parts, kept entries and solutions in shared memory all along.  Bound by the chain
+// of dependent FP64 operations: the roll-up's 20 parts take 38 us, 50 when the last
+// 10 went through L2 between the levels and the first level had its own launches.
+struct SymTopShared {
+  ChainTopShared t;
+  double part[TOP_MERGES][CHAIN_SYM_PART + 1];
+  double kept[TOP_MERGES][CHAIN_SYM_KEEP + 1];
+  double ws[TOP_THREADS / 16][2][10][6], stage[TOP_THREADS / 16][SYM_STAGE];
+};
+struct TopMerge {
+  static constexpr bool SUMS = true;
+  const ChainParts& c;
+  SymTopShared& S;
+  int t;
+  int width;  // lanes of an item
+  __device__ __forceinline__ static bool active() { return true; }
+  __device__ __forceinline__ void stage(int lane, unsigned lanes, double* st) const {
+    const int o1 = S.t.part1[t], o2 = S.t.part2[t], e1 = S.t.m[t].e1, e2 = S.t.m[t].e2;
+    double v1[4], v2[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int y = lane + width * q;
+      const bool on = y < CHAIN_SYM_PART;
+      v1[q] = !on ? 0.0 : o1 >= 0 ? S.part[o1][y] : chain_at(c.part, c.part_soa, CHAIN_SYM_PART, e1, y);
+      v2[q] = !on ? 0.0 : o2 >= 0 ? S.part[o2][y] : chain_at(c.part, c.part_soa, CHAIN_SYM_PART, e2, y);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int y = lane + width * q;
+      if (y < CHAIN_SYM_PART) {
+        st[y] = v1[q];
+        st[SYM_E2 + y] = v2[q];
+      }
+    }
+    if (lane == 15) st[SYM_ZERO] = 0.0;
+    __syncwarp(lanes);
+    if (lane < 6) st[PT_HN + lane] = radd(S.t.f[t][lane], st[PT_HN + lane]);
+    __syncwarp(lanes);
+  }
+  __device__ __forceinline__ void keep(int x, double v) const { S.kept[t][x] = v; }
+  __device__ __forceinline__ void out_s(const double* st, int o, double h) const {
+    Merge::out_st(st, o, h, [&](int x, double v) { S.part[t][x] = v; });
+  }
+};
+__global__ void __launch_bounds__(TOP_THREADS) k_sym_top(Batch b, ChainParts c) {
+  extern __shared__ __align__(16) unsigned char sym_top_raw[];
+  SymTopShared& S = *reinterpret_cast<SymTopShared*>(sym_top_raw);
   const ChainTop ch = c.chain[blockIdx.x];
   if (!solving(b, ch.structure)) return;
-  const int half = threadIdx.x >> 4, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned lanes = 0xFFFFu << (threadIdx.x & 16);
-  int t0 = ch.top;
-  for (int k = ch.n_top; k > 1; t0 += k / 2, k = (k + 1) / 2) {
-    if (half < k / 2) {
-      Merge I{b, c};
-      I.init(t0 + half);
-      const bool ok = eliminate_h(I, threadIdx.x & 15, lanes, stage[half], ws[half]);
-      if (!ok && (threadIdx.x & 15) == 0) I.fail();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = ch.n_top - 1;
+  top_load(b, c, ch, tid, S.t);
+  int t0 = 0;
+  {
+    // two items a warp while there are more than sub-partitions, then one
+    SymLane<16> L;
+    L.init<Merge>(lane & 15);
+    const int half = tid >> 4;
+    int k = ch.n_top;
+    for (; k / 2 > 4; t0 += k / 2, k = (k + 1) / 2) {
+      if (half < k / 2) {
+        const TopMerge I{c, S, t0 + half, 16};
+        const bool ok = eliminate_h<16>(I, L, lane & 15, 0xFFFFu << (tid & 16), S.stage[half], S.ws[half]);
+        if (!ok && (lane & 15) == 0) b.state[ch.structure].info_fail = 1;
+      }
+      __syncthreads();
     }
-    __syncthreads();
+    SymLane<32> W;
+    W.init<Merge>(lane);
+    for (; k > 1; t0 += k / 2, k = (k + 1) / 2) {
+      if (warp < k / 2) {
+        const TopMerge I{c, S, t0 + warp, 32};
+        const bool ok = eliminate_h<32>(I, W, lane, 0xffffffffu, S.stage[warp], S.ws[warp]);
+        if (!ok && lane == 0) b.state[ch.structure].info_fail = 1;
+      }
+      __syncthreads();
+    }
   }
-  if (warp == 0) chain_root(b, c, ch, lane, SymRoot{c, ch.root});
+  if (warp == 0) {
+    if (n == 0) {
+      for (int x = lane; x < CHAIN_SYM_PART; x += 32)
+        S.part[0][x] = chain_at(c.part, c.part_soa, CHAIN_SYM_PART, ch.root, x);
+      __syncwarp();
+    }
+    chain_root(b, c, ch, lane, SymRoot{S.part[max(n - 1, 0)]}, S.t.x[TOP_FIRST]);
+  }
   __syncthreads();
   // the levels again from the last: their merges end at t0
-  int cnt[5], n = 0;
-  for (int k = ch.n_top; k > 1; k = (k + 1) / 2) cnt[n++] = k / 2;
-  for (int l = n - 1; l >= 0; --l) {
+  int cnt[6], nl = 0;
+  for (int k = ch.n_top; k > 1; k = (k + 1) / 2) cnt[nl++] = k / 2;
+  for (int l = nl - 1; l >= 0; --l) {
     t0 -= cnt[l];
     const int i = lane % 6, q = warp * 5 + lane / 6;
     const bool on = lane < 30 && q < cnt[l];
     const unsigned on_lanes = __ballot_sync(0xffffffffu, on);
-    if (on) back_corner(b, c, t0 + q, c.merge[t0 + q], on_lanes, lane - i, i);
+    if (on) {
+      const int t = t0 + q;
+      const ChainMerge& m = S.t.m[t];
+      double z[9];
+      around(S.t.x[S.t.p[t]], S.t.x[S.t.n[t]], z);
+      double x = back(on_lanes, lane - i, i, z, [&](int y) { return S.kept[t][y]; });
+      if (i < 3) x = radd(x, S.t.x[S.t.p[t]][i]);  // u_k = u_p + w
+      S.t.x[t][i] = x;
+      c.x[6 * (int64_t)m.k + i] = x;
+      b.P[m.dof + i] = x;
+    }
     __syncthreads();
   }
 }
@@ -485,7 +606,12 @@ void launch_sym_chains(const Batch& b, const ChainParts& c, cudaStream_t st) {
     if (hi <= c.merge_soa) k_sym<Merge><<<grid_for(hi - lo, CT), CT, 0, st>>>(b, c, lo, hi);
     else k_sym_h<Merge><<<grid_for(hi - lo, 8), 128, 0, st>>>(b, c, lo, hi);
   }
-  k_sym_top<<<c.n_chains, 128, 0, st>>>(b, c);
+  static const bool done = [] {  // once per process, thread-safe
+    cudaFuncSetAttribute(k_sym_top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SymTopShared));
+    return true;
+  }();
+  (void)done;
+  k_sym_top<<<c.n_chains, TOP_THREADS, sizeof(SymTopShared), st>>>(b, c);
   for (int l = c.n_levels - 1; l >= 0; --l) {
     const int lo = c.merge_off[l], hi = c.merge_off[l + 1];
     k_sym_back<<<grid_for(hi - lo, 20), 128, 0, st>>>(b, c, lo, hi);

@@ -605,6 +605,11 @@ bool build_parts(gf_batch* B, const gf_model_desc* models, const std::vector<Str
   constexpr int NL = CHAIN_MAX_LEVELS;
   const int n = (int)plan.size();
   std::vector<int> sbase(n, 0), cbase(n, 0), mcnt(NL, 0), mpos((size_t)n * NL, 0), tpos(n, 0), chains;
+  // The parts from which one CTA takes a chain.  32 spares a few chains a level's
+  // launches and its round trip (one of 20 elements 38 us for 50); with more chains
+  // than SMs the level's own launch fills the chip better (512: 53 ms for 54)
+  for (int s = 0; s < n; ++s) cp.n_chains += plan[s].chain && (B->info[s].sym != 0) == sym;
+  const int top_parts = cp.n_chains > 152 ? CHAIN_TOP / 2 : CHAIN_TOP;
   int n_top = 0;
   for (int s = 0; s < n; ++s) {
     if (!plan[s].chain || (B->info[s].sym != 0) != sym) continue;
@@ -615,7 +620,7 @@ bool build_parts(gf_batch* B, const gf_model_desc* models, const std::vector<Str
     cp.n_corner += mm + 1;
     chains.push_back(s);
     int l = 0, k = mm;
-    for (; k > CHAIN_TOP; ++l, k = (k + 1) / 2) {
+    for (; k > top_parts; ++l, k = (k + 1) / 2) {
       if (l >= NL) return set_err(B->ctx, "chain too long for %d elimination levels", NL);
       mpos[(size_t)s * NL + l] = mcnt[l];
       mcnt[l] += k / 2;
@@ -627,7 +632,6 @@ bool build_parts(gf_batch* B, const gf_model_desc* models, const std::vector<Str
   for (int l = 0; l < NL; ++l) cp.merge_off[l + 1] = cp.merge_off[l] + mcnt[l];
   cp.n_merge = cp.merge_off[NL] + n_top;
   cp.n_part = cp.n_elem + cp.n_merge;
-  cp.n_chains = (int)chains.size();
   if (!cp.n_elem) return true;
   // the levels taken an item per thread: the largest ones, so the first
   const int small = sym ? CHAIN_SYM_SMALL : CHAIN_GEN_SMALL;
@@ -671,8 +675,8 @@ bool build_parts(gf_batch* B, const gf_model_desc* models, const std::vector<Str
     ch = ChainTop{0, cp.merge_off[NL] + tpos[s], 0, c0, c0 + mm, s};
     int last = ch.top;
     for (int l = 0, k = mm; k > 1; ++l, k = (k + 1) / 2) {
-      if (k <= CHAIN_TOP && !ch.n_top) ch.n_top = k;
-      int at = k > CHAIN_TOP ? cp.merge_off[l] + mpos[(size_t)s * NL + l] : last, first = c0;
+      if (k <= top_parts && !ch.n_top) ch.n_top = k;
+      int at = k > top_parts ? cp.merge_off[l] + mpos[(size_t)s * NL + l] : last, first = c0;
       for (int q = 0; q < k / 2; ++q, ++at) {
         const int mid = end[2 * q], node = 2 * (mid - c0);
         merge[at] = ChainMerge{id[2 * q], id[2 * q + 1], cp.n_elem + at, first, mid, end[2 * q + 1], s, first_dof(node),
@@ -681,7 +685,7 @@ bool build_parts(gf_batch* B, const gf_model_desc* models, const std::vector<Str
         id[q] = cp.n_elem + at;
         end[q] = first;
       }
-      if (k <= CHAIN_TOP) last = at;
+      if (k <= top_parts) last = at;
       if (k % 2) {
         id[k / 2] = id[k - 1];
         end[k / 2] = end[k - 1];

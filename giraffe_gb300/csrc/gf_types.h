@@ -233,9 +233,9 @@ __device__ __forceinline__ int table_row(const TableDev& T, const double* times,
 struct ChainMerge {
   int e1, e2, out, p, k, n, structure, dof, mask;
 };
-// A chain once CHAIN_TOP parts or fewer are left: their number, the merges that
+// A chain once CHAIN_TOP parts (half as many in large batches) or fewer are left: their number, the merges that
 // are left (chain by chain, level by level), the last part and the end corners.
-#define CHAIN_TOP 16
+#define CHAIN_TOP 32
 struct ChainTop {
   int n_top, top, root, first, last, structure;
 };
@@ -248,7 +248,7 @@ struct ChainParts {
   int* elem_corner;  // its first corner (the next index is its last)
   int* elem_mask;    // free DOFs of its corners: bits 0-5 the first, 6-11 the last
   int* corner_node;  // batch node of each corner
-  ChainMerge* merge; // the levels of more than CHAIN_TOP parts, level by level, then every chain's last ones
+  ChainMerge* merge; // the levels of more parts than ChainTop takes, level by level, then every chain's last ones
   int merge_off[CHAIN_MAX_LEVELS + 1];
   ChainTop* chain;
   // What the item-per-thread kernels write is structure-of-arrays (the items

@@ -38,6 +38,7 @@ def solve(structs):
 CASES = {
     # the symmetric elimination: part counts around powers of two, moments and fixed DOFs at the ends
     "1": lambda: chain(1), "2": lambda: chain(2), "3": lambda: chain(3), "8": lambda: chain(8), "17": lambda: chain(17),
+    "31": lambda: chain(31), "32": lambda: chain(32), "65": lambda: chain(65),
     "1_tip_moment": lambda: chain(1, -1), "33_tip_moment": lambda: chain(33, -1),
     "roller_tip": lambda: chain(20, fix={40: (0, 1, 0, 0, 0, 0)}),
     "pinned_tip_moment": lambda: chain(11, -1, fix={22: (1, 0, 1, 0, 0, 0)}),
@@ -45,6 +46,7 @@ CASES = {
     "2_moment": lambda: chain(2, 2), "3_midside_moment": lambda: chain(3, 3), "33_moment": lambda: chain(33, 20),
     "guided": lambda: chain(21, fix={42: (1, 1, 0, 0, 0, 0), 20: (0, 0, 1, 0, 0, 0)}),
     "guided_moment": lambda: chain(12, 8, fix={24: (1, 0, 0, 0, 0, 0), 12: (0, 1, 0, 0, 0, 0)}),
+    "31_moment": lambda: chain(31, 6), "65_moment": lambda: chain(65, 64),
     "riser": lambda: riser(9, False), "riser_pinned": lambda: riser(10, True),
 }
 
@@ -63,10 +65,10 @@ def test_solves_as_the_oracle(gpu_ctx, make):
 @pytest.mark.parametrize("make", [lambda: chain(57), lambda: chain(57, -1), lambda: chain(57, 30), lambda: riser(57, True)],
                          ids=["symmetric", "tip_moment", "general", "dynamic"])
 def test_same_bits_in_a_batch_of_either_size(gpu_ctx, make):
-    """One structure alone (every level below the thresholds), and among 600
-    chains of 40 to 75 elements of both kinds (17,000 elements of each: the
+    """One structure alone (every level below the thresholds), and among 1,300
+    chains of 40 to 75 elements of both kinds (37,000 elements of each: the
     first levels above them)."""
     alone, _ = solve([make()])
-    many = [chain(40 + i % 36, 20 if i % 2 else None, steps=1) for i in range(600)]
+    many = [chain(40 + i % 36, 20 if i % 2 else None, steps=1) for i in range(1300)]
     batch, _ = solve(many[:100] + [make()] + many[100:])
     assert np.array_equal(alone[0], batch[100])
