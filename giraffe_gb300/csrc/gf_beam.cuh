@@ -3,6 +3,7 @@
 // 1564-1638 (MountMass) and 1494-1506 (SaveLagrange)), FP64.  The tangent and
 // the internal force are in gf_beam_gp.cuh.
 #pragma once
+#include "gf_beam_gp.cuh"
 #include "gf_math.cuh"
 #include "gf_types.h"
 
@@ -52,7 +53,7 @@ GF_HD void beam_rot(const V3<double>& alpha, double& g, M3<double>& Qd, M3<doubl
 
 // Inertial contribution of one Gauss point (Beam_1::MountMass, reference
 // src/Beam_1.cpp:1564-1638, Hooke sections: no offset of the mass centre).
-// In the element frame, with Newmark coefficients a[0..5] = a1..a6:
+// With Newmark coefficients a[0..5] = a1..a6:
 //   dT_u = Mr (a1 du - a2 v_i - a3 acc_i)
 //   dT_a = Xi(da) h,  h = J_i w2 + w1 x J_i w1,  J_i = Q(alpha_i) Jr Q(alpha_i)^T,
 //   w1 = a4 da + a5 w_i + a6 dw_i,  w2 = a1 da - a2 w_i - a3 dw_i
@@ -61,70 +62,77 @@ GF_HD void beam_rot(const V3<double>& alpha, double& g, M3<double>& Qd, M3<doubl
 //   d dT_u/d du = a1 Mr I,
 //   d dT_a/d da = Xi (a1 J_i + a4 (skew(w1) J_i - skew(J_i w1)))
 //                 - g^2/2 (h + da x h / 2) da^T - g/2 skew(h).
-// Returns dT_u and dT_a in the global frame (fu[i * ds], fa[i * ds]; the element
-// force is their sum with wJ N_I) and the rotated rotational tangent T3^T (d
-// dT_a/d da) T3 in Daa[q * ds]; the translational tangent is a1 Mr I in every
-// frame.
-GF_HD void beam_gp_inertia(const BeamConst& c, const BeamHistAux& x, const BeamInterp& ip, const double* vel,
+// All in the global frame, the element frame entering through T3^T Q(alpha_i), and
+// J_i symmetric: about 330 operations against 560 in the element frame with its
+// rotations.  d: the nodal increments.  Returns dT_u and dT_a (fu[i * ds], fa[i *
+// ds]; the element force is their sum with wJ N_I) and the rotational tangent in
+// Daa[q * ds]; the translational tangent is a1 Mr I.
+GF_HD void beam_gp_inertia(const BeamConst& c, const BeamHistAux& x, const double* d, const double* vel,
                            const double* acc, const double* a, int g, double* fu_out, double* fa_out, double* Daa,
                            int ds) {
-  const double* N = c.N[g];
-  M3<double> T;
-#pragma unroll
-  for (int i = 0; i < 9; ++i) T[i] = c.T3[i];
-  V3<double> wi, dwi, vi, ai;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    wi[i] = vel[3 + i] * N[0] + vel[9 + i] * N[1] + vel[15 + i] * N[2];
-    dwi[i] = acc[3 + i] * N[0] + acc[9 + i] * N[1] + acc[15 + i] * N[2];
-    vi[i] = vel[i] * N[0] + vel[6 + i] * N[1] + vel[12 + i] * N[2];
-    ai[i] = acc[i] * N[0] + acc[6 + i] * N[1] + acc[12 + i] * N[2];
-  }
-  wi = mv(T, wi);
-  dwi = mv(T, dwi);
-  vi = mv(T, vi);
-  ai = mv(T, ai);
+  const double N0 = c.N[g][0], N1 = c.N[g][1], N2 = c.N[g][2];
   const double a1 = a[0], a2 = a[1], a3 = a[2], a4 = a[3], a5 = a[4], a6 = a[5];
-  V3<double> fu;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) fu[i] = c.Mr * (a1 * ip.u[i] - a2 * vi[i] - a3 * ai[i]);
-  V3<double> al = {{x.alpha[g][0], x.alpha[g][1], x.alpha[g][2]}};
-  M3<double> Qi = rodrigues(al), Jr;
-#pragma unroll
-  for (int i = 0; i < 9; ++i) Jr[i] = c.Jr[i];
-  M3<double> Ji = mul(mul(Qi, Jr), transpose(Qi));
-  V3<double> w1, w2;
+  d3 al, w1, w2;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    w1[i] = a4 * ip.alpha[i] + a5 * wi[i] + a6 * dwi[i];
-    w2[i] = a1 * ip.alpha[i] - a2 * wi[i] - a3 * dwi[i];
+    auto at = [&](const double* v, int k) { return fma(v[12 + k], N2, fma(v[6 + k], N1, v[k] * N0)); };
+    fu_out[i * ds] = c.Mr * fma(-a3, at(acc, i), fma(-a2, at(vel, i), a1 * at(d, i)));
+    const double wi = at(vel, 3 + i), dwi = at(acc, 3 + i);
+    al[i] = at(d, 3 + i);
+    w1[i] = fma(a6, dwi, fma(a5, wi, a4 * al[i]));
+    w2[i] = fma(-a3, dwi, fma(-a2, wi, a1 * al[i]));
   }
-  V3<double> Jw1 = mv(Ji, w1), Jw2 = mv(Ji, w2), cr = cross(w1, Jw1), h;
+  // J = R Jr R^T with R = T3^T Q(alpha_i): Jr has the two bending inertias and their
+  // product, and the polar one
+  d3 J[3];  // columns
+  {
+    M3<double> T;
 #pragma unroll
-  for (int i = 0; i < 3; ++i) h[i] = Jw2[i] + cr[i];
-  double gg;
-  M3<double> Qd, Xi;
-  beam_rot(ip.alpha, gg, Qd, Xi);
-  V3<double> m = mv(Xi, h);
-  M3<double> t = mul(skew(w1), Ji), SJw1 = skew(Jw1), Dh;
+    for (int i = 0; i < 9; ++i) T[i] = c.T3[i];
+    const M3<double> Q = rodrigues(V3<double>{{x.alpha[g][0], x.alpha[g][1], x.alpha[g][2]}});
+    d3 R[3], S[3];
 #pragma unroll
-  for (int q = 0; q < 9; ++q) Dh[q] = a1 * Ji[q] + a4 * (t[q] - SJw1[q]);
-  M3<double> D = mul(Xi, Dh);
-  V3<double> axh = cross(ip.alpha, h);
-  M3<double> Sh = skew(h);
+    for (int j = 0; j < 3; ++j) R[j] = tmv(T, d3{{Q[j], Q[3 + j], Q[6 + j]}});
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+    for (int i = 0; i < 3; ++i) {
+      S[0][i] = fma(c.Jr[3], R[1][i], c.Jr[0] * R[0][i]);
+      S[1][i] = fma(c.Jr[4], R[1][i], c.Jr[1] * R[0][i]);
+      S[2][i] = c.Jr[8] * R[2][i];
+    }
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
-      D[i * 3 + j] += -0.5 * gg * gg * (h[i] + 0.5 * axh[i]) * ip.alpha[j] - 0.5 * gg * Sh[i * 3 + j];
-  M3<double> Dg = tmul(T, mul(D, T));
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-  for (int q = 0; q < 9; ++q) Daa[q * ds] = Dg[q];
-  V3<double> gu = tmv(T, fu), ga = tmv(T, m);
+      for (int j = i; j < 3; ++j) {
+        const double v = fma(S[2][i], R[2][j], fma(S[1][i], R[1][j], S[0][i] * R[0][j]));
+        J[j][i] = v;
+        J[i][j] = v;
+      }
+  }
+  const d3 Jw1 = rmv(J, w1), Jw2 = rmv(J, w2), cr = rcross(w1, Jw1);
+  const d3 h = {{Jw2[0] + cr[0], Jw2[1] + cr[1], Jw2[2] + cr[2]}};
+  const double gg = 4.0 / (4.0 + dot(al, al)), hg = 0.5 * gg;
+  const d3 m = rxi(al, h, gg, 0.5), axh = rcross(al, h);
+  d3 p;  // -g^2/2 (h + da x h / 2)
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    fu_out[i * ds] = gu[i];
-    fa_out[i * ds] = ga[i];
+    fa_out[i * ds] = m[i];
+    p[i] = -hg * gg * fma(0.5, axh[i], h[i]);
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const d3 t = rcross(w1, J[j]);
+    // columns j of skew(J w1) and skew(h)
+    const d3 sj = j == 0 ? d3{{0.0, Jw1[2], -Jw1[1]}} : j == 1 ? d3{{-Jw1[2], 0.0, Jw1[0]}} : d3{{Jw1[1], -Jw1[0], 0.0}};
+    const d3 sh = j == 0 ? d3{{0.0, h[2], -h[1]}} : j == 1 ? d3{{-h[2], 0.0, h[0]}} : d3{{h[1], -h[0], 0.0}};
+    d3 col;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) col[i] = fma(a4, i == j ? t[i] : t[i] - sj[i], a1 * J[j][i]);
+    const d3 y = rxi(al, col, gg, 0.5);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double v = fma(p[i], al[j], y[i]);
+      Daa[(3 * i + j) * ds] = i == j ? v : fma(-hg, sh[i], v);
+    }
   }
 }
 

@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
 #pragma unroll
         for (int q = 0; q < 6; ++q) a6[q] = b.state[s].a[q];
         double* I = In + g * MI_COUNT * 32 + lane;
-        beam_gp_inertia(c, b.baux[e], beam_interp(c, d, g), vel, acc, a6, g, I + MI_FU * 32, I + MI_FA * 32, I, 32);
+        beam_gp_inertia(c, b.baux[e], d, vel, acc, a6, g, I + MI_FU * 32, I + MI_FA * 32, I, 32);
       }
     }
   }
@@ -451,22 +451,24 @@ __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
   double* Ce = pr.ray_on && (pr.ray_update || !b.state[s].ray_init) ? b.RD + e : nullptr;
   const double a1Mr = rmul(b.state[s].a[0], b.bconst[e].Mr);
   const double* I0 = In + lane;
-  auto mass = [&](int r, int q) {
+  // K_e's entry with its inertial term, if it has one: couplings of translations
+  // and rotations and of different translations do not (a zero added would take an
+  // FP64 instruction's 64 cycles)
+  auto with_mass = [&](int r, int q, double v) {
     const int I = r / 6, i = r % 6, J = q / 6, j = q % 6;
     const int pair = tri3(I, J);
-    if (i < 3 && j < 3)
-      return i == j ? rmul(radd(Cf[(GC_NN + pair) * 32], Cf[(MP_POINT + GC_NN + pair) * 32]), a1Mr) : 0.0;
-    if (i < 3 || j < 3) return 0.0;
+    if ((i < 3) != (j < 3) || (i < 3 && i != j)) return v;
+    if (i < 3) return radd(v, rmul(radd(Cf[(GC_NN + pair) * 32], Cf[(MP_POINT + GC_NN + pair) * 32]), a1Mr));
     const int x = (i - 3) * 3 + j - 3;
-    return rfma(Cf[(MP_POINT + GC_NN + pair) * 32], I0[(MI_COUNT + MI_D + x) * 32],
-                rmul(Cf[(GC_NN + pair) * 32], I0[(MI_D + x) * 32]));
+    return radd(v, rfma(Cf[(MP_POINT + GC_NN + pair) * 32], I0[(MI_COUNT + MI_D + x) * 32],
+                        rmul(Cf[(GC_NN + pair) * 32], I0[(MI_D + x) * 32])));
   };
   beam_expand(P, warp, lane,
               [&](int r, int q, double v) {
-                Ke[(r + 18 * q) * ne] = radd(v, mass(r, q));
+                Ke[(r + 18 * q) * ne] = with_mass(r, q, v);
                 if (Ce) Ce[(r + 18 * q) * ne] = v;
                 if (r == q) return;
-                Ke[(q + 18 * r) * ne] = radd(v, mass(q, r));
+                Ke[(q + 18 * r) * ne] = with_mass(q, r, v);
                 if (Ce) Ce[(q + 18 * r) * ne] = v;
               },
               [&](int q, double v) {
@@ -604,10 +606,80 @@ __global__ void __launch_bounds__(RAY_THREADS) k_beam_rayleigh(Batch b) {
 // k_beam_rayleigh: in a Dynamic step the reference mounts loads before damping,
 // so on the iterations that form C_e the load stiffness also goes into the
 // stiffness part that C_e is made from.  32 elements per CTA, an element per
-// lane: warps 0 and 1 form the two Gauss points' blocks in shared memory, then
-// the eight warps share the entries of K_e.
+// lane: warps 0 and 1 form the two Gauss points' blocks in shared memory (in the
+// global frame, where K2au = -K2ua^T and kappa x e3's commutator spares the products
+// of three skew matrices: 300 operations for 800), the other six the products of
+// the shape functions, then the eight warps share the entries of K_e, four loads in
+// flight.  Bound by these chains of FP64 operations: 500 elements 58 us with the
+// element frame's matrix products and an entry at a time, 24 here.
 constexpr int PP_THREADS = 256;
-constexpr int PP_G = 0, PP_F = 36, PP_COUNT = 42;  // blocks G1..G4, then the force and moment
+// blocks G1 (K1ua), G2 (K2ua), G4 (K1aa), the force and the moment; the products
+// jac p0i Aint N_a N_n and N_a N'_n and jac p0i Aint N_a
+constexpr int PP_G1 = 0, PP_G2 = 9, PP_G4 = 18, PP_F = 27, PP_NN = 33, PP_ND = 42, PP_N = 51, PP_COUNT = 54;
+__device__ __forceinline__ void pipe_press_point(const BeamConst& c, const BeamHist& h, const double* d, int g, double* S) {
+  d3 a, b, z;
+  beam_gp_interp(c, d, g, a, b, z);
+  const double gq = 4.0 / radd(4.0, rdot(a, a)), hg = 0.5 * gq;
+  double g_last = gq;
+  if (g == 0) {
+    d3 y;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) y[i] = fma(d[15 + i], c.N[1][2], fma(d[9 + i], c.N[1][1], d[3 + i] * c.N[1][0]));
+    g_last = 4.0 / (4.0 + dot(y, y));
+  }
+  // kappa and e3 before the increment's rotation, then through it
+  d3 kip = {{0.0, 0.0, 0.0}}, e3 = {{0.0, 0.0, 0.0}};
+  {
+    d3 T[3];  // rows of T3
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) T[i][j] = c.T3[i * 3 + j];
+    const d3 w = rmv(T, d3{{h.dz[g][0], h.dz[g][1], h.dz[g][2]}}), beta = rxi(a, b, gq, -0.5);
+    d3 k0 = kip, e0 = e3;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const d3 r = rmv(T, d3{{h.Q[g][j], h.Q[g][3 + j], h.Q[g][6 + j]}});
+      const double kj = radd(rdot(r, beta), h.kap[g][j]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        k0[i] = fma(r[i], kj, k0[i]);
+        e0[i] = fma(r[i], c.e3r[j], e0[i]);
+      }
+      z[j] += w[j];
+    }
+    const d3 ck = rcross(a, k0), ck2 = rcross(a, ck), ce = rcross(a, e0), ce2 = rcross(a, ce);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      kip[i] = fma(gq, fma(0.5, ck2[i], ck[i]), k0[i]);
+      e3[i] = fma(gq, fma(0.5, ce2[i], ce[i]), e0[i]);
+    }
+  }
+  const d3 fl = rcross(kip, e3), c2 = rcross(e3, z);
+  const d3 w = rxi(a, c2, gq, -0.5), eps = rxi(a, e3, gq, -0.5), zeta = rxi(a, z, gq, -0.5);
+  const d3 ha = {{hg * a[0], hg * a[1], hg * a[2]}};
+  const d3 X[3] = {{{gq, ha[2], -ha[1]}}, {{-ha[2], gq, ha[0]}}, {{ha[1], -ha[0], gq}}};  // columns of Xi
+  const double hab = hg * dot(a, b), heb = hg * dot(e3, b), ze = dot(z, e3);
+  const double sk[9] = {0.0, -c2[2], c2[1], c2[2], 0.0, -c2[0], -c2[1], c2[0], 0.0};
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const d3 y = rcross(e3, X[j]), f = rcross(fl, X[j]);
+    const double hej = hg * e3[j], aj = ze * hg * ha[j];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      S[(PP_G2 + 3 * i + j) * 32] = y[i];
+      double v = fma(hej, b[i], fma(-hab, y[i], f[i]));
+      if (i == j) v -= heb;
+      S[(PP_G1 + 3 * i + j) * 32] = v;
+      double u = i == j ? w[i] * a[j] : fma(w[i], a[j], -sk[3 * i + j]);
+      u = fma(-0.5 * g_last, u, fma(eps[i], zeta[j], aj * a[i]));
+      if (i == j) u = fma(-ze, gq, u);
+      S[(PP_G4 + 3 * i + j) * 32] = u;
+    }
+    S[(PP_F + j) * 32] = fl[j];
+    S[(PP_F + 3 + j) * 32] = -w[j];
+  }
+}
 __global__ void __launch_bounds__(PP_THREADS) k_pipe_pressure(Batch b) {
   __shared__ double S[2][PP_COUNT][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * 32 + lane;
@@ -616,77 +688,27 @@ __global__ void __launch_bounds__(PP_THREADS) k_pipe_pressure(Batch b) {
   const StructState& st = b.state[s];
   const bool on = q < b.n_pipe_press && iterating(st);
   const BeamConst& c = b.bconst[e];
-  double pa = 0.0, sK = 0.0;
   if (on) {
-    const double p0i = table_at(b, b.pp_table[q], st.last_converged_time + st.current_time_step, 0);
-    const double Aint = b.pp_aint[q];
-    pa = -p0i * Aint;
-    sK = c.jac * p0i * Aint;
-  }
-  if (on && warp < 2) {
-    const int g = warp;
-    const BeamHist& h = b.bhist[e];
-    double d[18];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const int64_t nd = b.enodes[3 * e + j];
-#pragma unroll
-      for (int k = 0; k < 6; ++k) d[6 * j + k] = b.disp[nd * 6 + k];
-    }
-    M3<double> T;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) T[i] = c.T3[i];
-    const V3<double> e3r = {{c.e3r[0], c.e3r[1], c.e3r[2]}};
-    const BeamInterp ip1 = beam_interp(c, d, 1);
-    const double g_last = 4.0 / (4.0 + dot(ip1.alpha, ip1.alpha));
-    const BeamInterp ip = beam_interp(c, d, g);
-    double gg;
-    M3<double> Qd, Xi, Qi;
-    beam_rot(ip.alpha, gg, Qd, Xi);
-    const M3<double> dA = skew(ip.dalpha);
-    const double ad = dot(ip.alpha, ip.dalpha);
-    M3<double> dXi;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) dXi[i] = -0.5 * gg * (ad * Xi[i] - dA[i]);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) Qi[i] = h.Q[g][i];
-    V3<double> dz;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) dz[i] = ip.du[i] + h.dz[g][i];
-    const M3<double> Q = mul(Qd, Qi);
-    V3<double> kap = tmv(Qi, tmv(Xi, ip.dalpha));
-#pragma unroll
-    for (int i = 0; i < 3; ++i) kap[i] += h.kap[g][i];
-    const V3<double> kip = mv(Q, kap), e3 = mv(Q, e3r);
-    const V3<double> fl = cross(kip, e3), ml = tmv(Xi, cross(dz, e3));
-    const M3<double> E3 = skew(e3), Kp = skew(kip), dZ = skew(dz);
-    const V3<double> c2 = cross(e3, dz), w = tmv(Xi, c2);
-    const M3<double> S2 = skew(c2);
-    const M3<double> A1 = mul(mul(Kp, E3), Xi), A2 = mul(E3, dXi), A3 = mul(mul(E3, Kp), Xi);
-    const M3<double> B1 = tmul(Xi, mul(mul(dZ, E3), Xi));
-    M3<double> K1ua, K1aa;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
+    const int g = warp & 1;
+    if (warp < 2) {
+      double d[18];
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
-        K1ua[i * 3 + j] = A1[i * 3 + j] + A2[i * 3 + j] - A3[i * 3 + j];
-        K1aa[i * 3 + j] = -0.5 * g_last * (w[i] * ip.alpha[j] - S2[i * 3 + j]) + B1[i * 3 + j];
+        const int64_t nd = b.enodes[3 * e + j];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) d[6 * j + k] = b.disp[nd * 6 + k];
       }
-    // blocks of Kext in the global frame: T^T X T
-    const M3<double> G1 = tmul(T, mul(K1ua, T)), G2 = tmul(T, mul(mul(E3, Xi), T));
-    const M3<double> G3 = tmul(T, mul(tmul(Xi, E3), T)), G4 = tmul(T, mul(K1aa, T));
-    const V3<double> fg = tmv(T, fl), mg = tmv(T, ml);
-#pragma unroll
-    for (int x = 0; x < 9; ++x) {
-      S[g][PP_G + x][lane] = G1[x];
-      S[g][PP_G + 9 + x][lane] = G2[x];
-      S[g][PP_G + 18 + x][lane] = G3[x];
-      S[g][PP_G + 27 + x][lane] = G4[x];
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      S[g][PP_F + i][lane] = fg[i];
-      S[g][PP_F + 3 + i][lane] = mg[i];
+      pipe_press_point(c, b.bhist[e], d, g, &S[g][0][lane]);
+    } else {
+      const double p0i = table_at(b, b.pp_table[q], st.last_converged_time + st.current_time_step, 0);
+      const double sK = c.jac * p0i * b.pp_aint[q];
+#pragma unroll 1
+      for (int x = (warp >> 1) - 1; x < 9; x += 3) {  // warps 2-7: three for each point
+        const double t = sK * c.N[g][x / 3];
+        S[g][PP_NN + x][lane] = t * c.N[g][x % 3];
+        S[g][PP_ND + x][lane] = t * c.dN[g][x % 3];
+        if (x % 3 == 0) S[g][PP_N + x / 3][lane] = t;
+      }
     }
   }
   __syncthreads();
@@ -696,33 +718,44 @@ __global__ void __launch_bounds__(PP_THREADS) k_pipe_pressure(Batch b) {
   const int64_t ne = b.n_elem;
   double* Ke = b.Ke + e;
   double* Ce = form_c ? b.RD + e : nullptr;
+  // f_e -= jac N (f, m) with the line load's -p0i Aint
 #pragma unroll 1
   for (int k = warp; k < 18; k += 8) {
     double f = b.Fe[(int64_t)k * ne + e];
 #pragma unroll
-    for (int g = 0; g < 2; ++g) f -= c.jac * c.N[g][k / 6] * (pa * S[g][PP_F + k % 6][lane]);
+    for (int g = 0; g < 2; ++g) f = fma(S[g][PP_N + k / 6][lane], S[g][PP_F + k % 6][lane], f);
     b.Fe[(int64_t)k * ne + e] = f;
   }
-  // (u_a, alpha_n): K1ua Nb + K2ua dNb; (alpha_a, u_n): K2au dNb; (alpha_a,
-  // alpha_n): K1aa Nb
+  // (u_a, alpha_n): K1ua Nb + K2ua dNb; (alpha_a, u_n): K2au dNb = -K2ua^T dNb;
+  // (alpha_a, alpha_n): K1aa Nb
 #pragma unroll 1
-  for (int k = warp; k < 243; k += 8) {
-    const int kind = k / 81, a = k % 81 / 27, n = k % 27 / 9, x = k % 9, i = x / 3, j = x % 3;
-    const int64_t at =
-        kind == 0 ? (6 * a + i) + 18 * (6 * n + 3 + j)
-                  : kind == 1 ? (6 * a + 3 + i) + 18 * (6 * n + j) : (6 * a + 3 + i) + 18 * (6 * n + 3 + j);
-    double v = Ke[at * ne], w = Ce ? Ce[at * ne] : 0.0;
+  for (int k0 = warp; k0 < 243; k0 += 32) {
+    int64_t at[4];
+    double v[4], w[4], t[4];
 #pragma unroll
-    for (int g = 0; g < 2; ++g) {
-      const double Na = c.N[g][a], Nb = c.N[g][n], dNb = c.dN[g][n];
-      const double t = kind == 0   ? sK * (Na * (Nb * S[g][PP_G + x][lane] + dNb * S[g][PP_G + 9 + x][lane]))
-                       : kind == 1 ? sK * (Na * (dNb * S[g][PP_G + 18 + x][lane]))
-                                   : sK * (Na * (Nb * S[g][PP_G + 27 + x][lane]));
-      v -= t;
-      w -= t;
+    for (int y = 0; y < 4; ++y) {
+      const int k = k0 + 8 * y, kind = k / 81, an = k % 81 / 9, x = k % 9, i = x / 3, j = x % 3, a = an / 3, n = an % 3;
+      at[y] = ((kind == 0 ? 6 * a + i : 6 * a + 3 + i) + 18 * (kind == 1 ? 6 * n + j : 6 * n + 3 + j)) * ne;
+      v[y] = k < 243 ? Ke[at[y]] : 0.0;
+      w[y] = k < 243 && Ce ? Ce[at[y]] : 0.0;
     }
-    Ke[at * ne] = v;
-    if (Ce) Ce[at * ne] = w;
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+      const int k = k0 + 8 * y, kind = k / 81, an = k % 81 / 9, x = k % 9, xt = 3 * (x % 3) + x / 3;
+      if (k >= 243) break;
+      if (kind == 0) {
+        t[y] = S[0][PP_NN + an][lane] * S[0][PP_G1 + x][lane];
+        t[y] = fma(S[0][PP_ND + an][lane], S[0][PP_G2 + x][lane], t[y]);
+        t[y] = fma(S[1][PP_NN + an][lane], S[1][PP_G1 + x][lane], t[y]);
+        t[y] = fma(S[1][PP_ND + an][lane], S[1][PP_G2 + x][lane], t[y]);
+      } else {
+        const int cf = (kind == 1 ? PP_ND : PP_NN) + an, m = kind == 1 ? PP_G2 + xt : PP_G4 + x;
+        t[y] = fma(S[1][cf][lane], S[1][m][lane], S[0][cf][lane] * S[0][m][lane]);
+      }
+      // (K2au's sign)
+      Ke[at[y]] = kind == 1 ? v[y] + t[y] : v[y] - t[y];
+      if (Ce) Ce[at[y]] = kind == 1 ? w[y] + t[y] : w[y] - t[y];
+    }
   }
 }
 
@@ -1397,9 +1430,8 @@ __global__ void k_beam_inertia_elements(int n, const BeamConst* cs, const BeamHi
   double an[6];
   for (int q = 0; q < 6; ++q) an[q] = a[q];
   for (int g = 0; g < 2; ++g) {
-    BeamInterp ip = beam_interp(c, d, g);
     double fu[3], fa[3];
-    beam_gp_inertia(c, xs[e], ip, vel, acc, an, g, fu, fa, D + 9 * g, 1);
+    beam_gp_inertia(c, xs[e], d, vel, acc, an, g, fu, fa, D + 9 * g, 1);
     for (int I = 0; I < 3; ++I)
       for (int i = 0; i < 3; ++i) {
         f[6 * I + i] += c.jac * c.N[g][I] * fu[i];
