@@ -84,7 +84,12 @@ GF_HD void beam_gp_interp(const BeamConst& c, const double* d, int g, d3& a, d3&
 }
 
 // The point's operator and forces at the nodal increments d (18, global),
-// written to o[x * os].
+// written to o[x * os].  Parts: 1 the blocks 00, 02 and the share Y^T W of 22, 2 the
+// blocks 11, 12 and the share S^T D S, 4 the geometric share of 22 and the forces;
+// 22 is (Y^T W + S^T D S) + the geometric share.  A part alone writes its share at
+// GP_PART + 6 (0, 1, 2) and forms what it needs of the kinematics itself.
+constexpr int GP_PART = GP_COUNT;
+template <int PARTS = 7>
 GF_HD void beam_gp(const BeamConst& c, const BeamHist& h, const double* d, int g, double* o, int os) {
   d3 a, b, z;
   beam_gp_interp(c, d, g, a, b, z);
@@ -142,8 +147,8 @@ GF_HD void beam_gp(const BeamConst& c, const BeamHist& h, const double* d, int g
   }
   // M00 = Q Dt Q^T; Y = skew(z) Xi, W = M00 Y; M02 = W - skew(n) Xi; the part
   // Y^T W of M22
-  double m22[6];
-  {
+  double m22[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  if constexpr (PARTS & 1) {
     d3 DQ[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j)
@@ -171,7 +176,10 @@ GF_HD void beam_gp(const BeamConst& c, const BeamHist& h, const double* d, int g
 #pragma unroll
     for (int i = 0, x = 0; i < 3; ++i)
 #pragma unroll
-      for (int j = i; j < 3; ++j, ++x) m22[x] = rdot(Y[i], W[j]);
+      for (int j = i; j < 3; ++j, ++x) {
+        m22[x] = rdot(Y[i], W[j]);
+        if constexpr (PARTS != 7) o[(GP_PART + x) * os] = m22[x];
+      }
   }
   const double ab = rdot(a, b);
   const d3 mu = rxi(a, m, gq, -0.5);  // Xi^T m
@@ -179,7 +187,7 @@ GF_HD void beam_gp(const BeamConst& c, const BeamHist& h, const double* d, int g
   const d3 w = {{rmul(-hg, mu[0]), rmul(-hg, mu[1]), rmul(-hg, mu[2])}};
   // R = Q^T Xi and S = Q^T dXi by rows; M11 = R^T Dr R, M12 = R^T Dr S + V^T,
   // the part S^T Dr S of M22
-  {
+  if constexpr (PARTS & 2) {
     d3 R[3], S[3], DR[3], DS[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -210,11 +218,14 @@ GF_HD void beam_gp(const BeamConst& c, const BeamHist& h, const double* d, int g
         o[(GP_M12 + 3 * i + j) * os] = v;
         if (j >= i) {
           o[(GP_M11 + x) * os] = rfma(R[2][i], DR[2][j], rfma(R[1][i], DR[1][j], rmul(R[0][i], DR[0][j])));
-          m22[x] = rfma(S[2][i], DS[2][j], rfma(S[1][i], DS[1][j], rfma(S[0][i], DS[0][j], m22[x])));
+          const double y = rfma(S[2][i], DS[2][j], rfma(S[1][i], DS[1][j], rmul(S[0][i], DS[0][j])));
+          if constexpr (PARTS == 7) m22[x] = radd(m22[x], y);
+          else o[(GP_PART + 6 + x) * os] = y;
           ++x;
         }
       }
   }
+  if constexpr (!(PARTS & 4)) return;
   // the geometric part of M22, its symmetric part:
   //   Xi^T skew(z) skew(n) Xi        = nu zeta^T - (z.n) (g I - (g/2)^2 a a^T)
   //   -V(a, z x n)                   = g/2 kappa a^T + antisymmetric
@@ -247,7 +258,8 @@ GF_HD void beam_gp(const BeamConst& c, const BeamHist& h, const double* d, int g
           v = rfma(w[i], b[j], rfma(w[j], b[i], v));
           v = rmul(0.5, rfma(rmul(hg, m[i]), beta[j], rfma(rmul(hg, m[j]), beta[i], v)));
         }
-        o[(GP_M22 + x) * os] = radd(m22[x], v);
+        if constexpr (PARTS == 7) o[(GP_M22 + x) * os] = radd(m22[x], v);
+        else o[(GP_PART + 12 + x) * os] = v;
       }
   }
   // force terms (reference src/Beam_1.cpp:828): n, Xi^T m and Xi^T skew(z)^T n

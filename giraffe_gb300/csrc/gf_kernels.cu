@@ -1,6 +1,7 @@
 // Device-resident Newton loop for batches of Beam_1 structures (see
 // gf_kernels.cuh for the pass structure and the reference lines each kernel
 // follows).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "gf_beam.cuh"
@@ -306,6 +307,8 @@ __global__ void k_zero(Batch b) {
 // atomics and is deterministic.
 constexpr int MOUNT_THREADS = 128;
 constexpr int MP_POINT = GP_COUNT + GC_COUNT;  // doubles per Gauss point and element
+// with a point's parts on three warps: their shares of block 22 before the coefficients
+constexpr int MP_COEF_SPLIT = GP_PART + 18, MP_POINT_SPLIT = MP_COEF_SPLIT + GC_COUNT;
 // a Gauss point's inertial terms: rotational tangent, translational and
 // rotational force (global frame)
 constexpr int MI_D = 0, MI_FU = 9, MI_FA = 12, MI_COUNT = 15;
@@ -313,26 +316,28 @@ constexpr int MOUNT_SMEM = 2 * MP_POINT * 32 * (int)sizeof(double);
 // the batch's kernel adds the inertial terms, or in static structures of the
 // symmetric chain solver their coefficients
 constexpr int MOUNT_SMEM_BATCH = 2 * (MP_POINT + MI_COUNT) * 32 * (int)sizeof(double);
+constexpr int MOUNT_SMEM_SPLIT = 2 * (MP_POINT_SPLIT + MI_COUNT) * 32 * (int)sizeof(double);
+// Elements up to which two CTAs take 32 of them: every CTA its own SM
+constexpr int MOUNT_SPLIT = 152 / 2 * 32;
 
-// The entries of K_e and f_e of lane's element, shared by the CTA's warps:
-// put(r, s, v) for one entry of every symmetric pair, force(q, v).
-template <typename Put, typename Force>
-__device__ __forceinline__ void beam_expand(const double* P, int warp, int lane, Put put, Force force) {
-  const double *M = P + lane, *C = P + GP_COUNT * 32 + lane;
-  constexpr int gs = MP_POINT * 32, ms = 32;
+// The entries of K_e and f_e of lane's element, shared by `step` warps: put(r, s, v) for one entry of every symmetric pair, force(q, v).
+template <int PT, int CO, typename Put, typename Force>
+__device__ __forceinline__ void beam_expand(const double* P, int warp, int step, int lane, Put put, Force force) {
+  const double *M = P + lane, *C = P + CO * 32 + lane;
+  constexpr int gs = PT * 32, ms = 32;
 #pragma unroll 1
-  for (int k = warp; k < 45; k += 4) {
+  for (int k = warp; k < 45; k += step) {
     int pair, I, J, i, j;
     beam_aa_place(k, pair, I, J, i, j);
     put(6 * I + 3 + i, 6 * J + 3 + j, beam_k_aa(M, C, gs, ms, pair, I, J, i, j));
   }
 #pragma unroll 1
-  for (int k = warp; k < 81; k += 4) {
+  for (int k = warp; k < 81; k += step) {
     const int IJ = k / 9, x = k % 9;
     put(6 * (IJ / 3) + x / 3, 6 * (IJ % 3) + 3 + x % 3, beam_k_ua(M, C, gs, ms, IJ, x));
   }
 #pragma unroll 1
-  for (int k = warp; k < 36; k += 4) {
+  for (int k = warp; k < 36; k += step) {
     int pair, x, I, J, i, j;
     beam_uu_place(k, pair, x, I, J, i, j);
     const double v = beam_k_uu(M, C, gs, ms, pair, x);
@@ -340,19 +345,19 @@ __device__ __forceinline__ void beam_expand(const double* P, int warp, int lane,
     if (I != J && i != j) put(6 * I + j, 6 * J + i, v);
   }
 #pragma unroll 1
-  for (int k = warp; k < 18; k += 4) force(k, beam_f(M, C, gs, ms, k / 6, (k % 6) / 3, k % 3));
+  for (int k = warp; k < 18; k += step) force(k, beam_f(M, C, gs, ms, k / 6, (k % 6) / 3, k % 3));
 }
 
 // The same over (du 0-2, v 3-5, a_0 6-8, a_1 9-11, a_2 12-14), lower triangle, as
 // the symmetric chain solver condenses it: put(i, j, v), i >= j.  S: the
 // coefficients of du and v, point g at [g * ss].
-template <typename Put, typename Force>
-__device__ __forceinline__ void beam_expand_sym(const double* P, const double* S, int ss, int warp, int lane, Put put,
+template <int PT, int CO, typename Put, typename Force>
+__device__ __forceinline__ void beam_expand_sym(const double* P, const double* S, int ss, int warp, int step, int lane, Put put,
                                                 Force force) {
-  const double *M = P + lane, *C = P + GP_COUNT * 32 + lane;
-  constexpr int gs = MP_POINT * 32, ms = 32;
+  const double *M = P + lane, *C = P + CO * 32 + lane;
+  constexpr int gs = PT * 32, ms = 32;
 #pragma unroll 1
-  for (int k = warp; k < 45; k += 4) {
+  for (int k = warp; k < 45; k += step) {
     int pair, I, J, i, j;
     beam_aa_place(k, pair, I, J, i, j);
     const double v = beam_k_aa(M, C, gs, ms, pair, I, J, i, j);
@@ -360,13 +365,13 @@ __device__ __forceinline__ void beam_expand_sym(const double* P, const double* S
     put(q, r, v);
   }
 #pragma unroll 1
-  for (int k = warp; k < 54; k += 4) {
+  for (int k = warp; k < 54; k += step) {
     const int B = k / 27, J = k % 27 / 9, x = k % 9, cf = (B ? GS_VN : GS_DN) + J;
     put(6 + 3 * J + x % 3, 3 * B + x / 3,
         rfma(S[ss + cf * ms], M[gs + (GP_M02 + x) * ms], rmul(S[cf * ms], M[(GP_M02 + x) * ms])));
   }
 #pragma unroll 1
-  for (int k = warp; k < 18; k += 4) {
+  for (int k = warp; k < 18; k += step) {
     const int B = k / 6, x = k % 6;
     const int i = x < 3 ? 0 : (x < 5 ? 1 : 2), j = x < 3 ? x : (x < 5 ? x - 2 : 2);  // i <= j
     const double v = rfma(S[ss + B * ms], M[gs + (GP_M00 + x) * ms], rmul(S[B * ms], M[(GP_M00 + x) * ms]));
@@ -378,34 +383,49 @@ __device__ __forceinline__ void beam_expand_sym(const double* P, const double* S
     }
   }
 #pragma unroll 1
-  for (int k = warp; k < 18; k += 4) force(k, beam_f(M, C, gs, ms, k / 6, (k % 6) / 3, k % 3));
+  for (int k = warp; k < 18; k += step) force(k, beam_f(M, C, gs, ms, k / 6, (k % 6) / 3, k % 3));
 }
 
-__global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
+// k_beam_tangent<2>: a cluster of two CTAs takes 32 elements, each one Gauss point,
+// whose three parts (beam_gp) and coefficients or inertia fill the SM's four
+// sub-partitions; the points' values are then exchanged and the eight warps share
+// K_e.  The parts repeat the kinematics, so this is for batches that leave SMs idle.
+template <int CTAS> __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int PT = CTAS == 2 ? MP_POINT_SPLIT : MP_POINT;
   double* P = reinterpret_cast<double*>(smem_raw);  // [point][value][lane]
-  double* In = P + 2 * MP_POINT * 32;               // inertial terms, [point][value][lane]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int e = blockIdx.x * 32 + lane;
+  double* In = P + 2 * PT * 32;                     // inertial terms, [point][value][lane]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = CTAS == 2 ? blockIdx.x & 1 : 0;
+  const int e = blockIdx.x / CTAS * 32 + lane;
   const int s = e < b.n_elem ? b.estruct[e] : -1;
   const bool live = s >= 0 && iterating(b.state[s]);
   const bool dyn = live && b.params[s].dynamic;
   if (live) {
     const BeamConst& c = b.bconst[e];
-    const int g = warp & 1;
-    if (warp >= 2) {
-      beam_gp_coef(c, g, P + (g * MP_POINT + GP_COUNT) * 32 + lane, 32);
+    // one CTA: warps 0, 1 the points, 2, 3 the rest; two: warps 0-2 the parts of
+    // point `rank`, 3 the rest
+    const int g = CTAS == 2 ? rank : warp & 1;
+    const bool point = CTAS == 2 ? warp < 3 : warp < 2;
+    double* M = P + g * PT * 32 + lane;
+    if (!point) {
+      beam_gp_coef(c, g, M + (CTAS == 2 ? MP_COEF_SPLIT : GP_COUNT) * 32, 32);
       if (!dyn) beam_gp_coef_sym(c, g, In + g * MI_COUNT * 32 + lane, 32);
     }
-    if (warp < 2 || dyn) {
+    if (point || dyn) {
       int nd[3] = {b.enodes[3 * e], b.enodes[3 * e + 1], b.enodes[3 * e + 2]};
       double d[18];
 #pragma unroll
       for (int j = 0; j < 3; ++j)
 #pragma unroll
         for (int q = 0; q < 6; ++q) d[6 * j + q] = b.disp[(int64_t)nd[j] * 6 + q];
-      if (warp < 2) {
-        beam_gp(c, b.bhist[e], d, g, P + g * MP_POINT * 32 + lane, 32);
+      if (point) {
+        if constexpr (CTAS == 1) {
+          beam_gp(c, b.bhist[e], d, g, M, 32);
+        } else {
+          if (warp == 0) beam_gp<1>(c, b.bhist[e], d, g, M, 32);
+          else if (warp == 1) beam_gp<2>(c, b.bhist[e], d, g, M, 32);
+          else beam_gp<4>(c, b.bhist[e], d, g, M, 32);
+        }
       } else {
         // MountMass + MountDyn: inertial force and mass/gyroscopic tangent
         double vel[18], acc[18], a6[6];
@@ -423,19 +443,38 @@ __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
       }
     }
   }
-  __syncthreads();
+  if constexpr (CTAS == 2) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __syncthreads();
+    // 22 of this CTA's point, then the other's values
+    double* M = P + rank * PT * 32;
+    for (int x = threadIdx.x; x < 6 * 32; x += MOUNT_THREADS)
+      M[GP_M22 * 32 + x] = radd(radd(M[GP_PART * 32 + x], M[(GP_PART + 6) * 32 + x]), M[(GP_PART + 12) * 32 + x]);
+    cluster.sync();
+    const double* other = cluster.map_shared_rank(P, rank ^ 1);
+    const int o = (rank ^ 1) * PT * 32, oi = (2 * PT + (rank ^ 1) * MI_COUNT) * 32;
+    for (int x = threadIdx.x; x < GP_COUNT * 32; x += MOUNT_THREADS) P[o + x] = other[o + x];
+    for (int x = threadIdx.x; x < GC_COUNT * 32; x += MOUNT_THREADS)
+      P[o + MP_COEF_SPLIT * 32 + x] = other[o + MP_COEF_SPLIT * 32 + x];
+    for (int x = threadIdx.x; x < MI_COUNT * 32; x += MOUNT_THREADS) P[oi + x] = other[oi + x];
+    cluster.sync();  // neither leaves while the other reads
+  }
+  if constexpr (CTAS == 1) __syncthreads();
   if (!live) return;
+  const int first = warp + 4 * rank, step = 4 * CTAS;
   double* Ke = b.Ke + e;
   const int64_t ne = b.n_elem;
-  const double* Cf = P + GP_COUNT * 32 + lane;
+  constexpr int CO = CTAS == 2 ? MP_COEF_SPLIT : GP_COUNT;
+  const double* Cf = P + CO * 32 + lane;
   if (!dyn) {
     if (b.info[s].sym && !b.full_band) {
-      beam_expand_sym(P, In + lane, MI_COUNT * 32, warp, lane,
+      beam_expand_sym<PT, CO>(P, In + lane, MI_COUNT * 32, first, step, lane,
                       [&](int i, int j, double v) { Ke[(int64_t)(i * (i + 1) / 2 + j) * ne] = v; },
                       [&](int q, double v) { b.Fe[q * ne + e] = v; });
       return;
     }
-    beam_expand(P, warp, lane,
+    beam_expand<PT, CO>(P, first, step, lane,
                 [&](int r, int q, double v) {
                   Ke[(r + 18 * q) * ne] = v;
                   if (r != q) Ke[(q + 18 * r) * ne] = v;
@@ -458,12 +497,12 @@ __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
     const int I = r / 6, i = r % 6, J = q / 6, j = q % 6;
     const int pair = tri3(I, J);
     if ((i < 3) != (j < 3) || (i < 3 && i != j)) return v;
-    if (i < 3) return radd(v, rmul(radd(Cf[(GC_NN + pair) * 32], Cf[(MP_POINT + GC_NN + pair) * 32]), a1Mr));
+    if (i < 3) return radd(v, rmul(radd(Cf[(GC_NN + pair) * 32], Cf[(PT + GC_NN + pair) * 32]), a1Mr));
     const int x = (i - 3) * 3 + j - 3;
-    return radd(v, rfma(Cf[(MP_POINT + GC_NN + pair) * 32], I0[(MI_COUNT + MI_D + x) * 32],
+    return radd(v, rfma(Cf[(PT + GC_NN + pair) * 32], I0[(MI_COUNT + MI_D + x) * 32],
                         rmul(Cf[(GC_NN + pair) * 32], I0[(MI_D + x) * 32])));
   };
-  beam_expand(P, warp, lane,
+  beam_expand<PT, CO>(P, first, step, lane,
               [&](int r, int q, double v) {
                 Ke[(r + 18 * q) * ne] = with_mass(r, q, v);
                 if (Ce) Ce[(r + 18 * q) * ne] = v;
@@ -474,7 +513,7 @@ __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_tangent(Batch b) {
               [&](int q, double v) {
                 const int I = q / 6, x = (q % 6) / 3 ? MI_FA + q % 3 : MI_FU + q % 3;
                 v = rfma(Cf[(GC_WN + I) * 32], I0[x * 32], v);
-                b.Fe[q * ne + e] = rfma(Cf[(MP_POINT + GC_WN + I) * 32], I0[(MI_COUNT + x) * 32], v);
+                b.Fe[q * ne + e] = rfma(Cf[(PT + GC_WN + I) * 32], I0[(MI_COUNT + x) * 32], v);
               });
 }
 
@@ -1401,7 +1440,7 @@ __global__ void __launch_bounds__(MOUNT_THREADS) k_beam_elements(int n, const Be
   double* tile = P + 2 * MP_POINT * 32;
   double* K = tile + lane * BE_LD;
   if (e < n)
-    beam_expand(P, warp, lane,
+    beam_expand<MP_POINT, GP_COUNT>(P, warp, 4, lane,
                 [&](int r, int q, double v) {
                   K[r + 18 * q] = v;
                   K[q + 18 * r] = v;
@@ -1537,6 +1576,7 @@ void launch_commit(const Batch& b, cudaStream_t st) {
 // function-local static is initialised by exactly one of them).
 static void set_attrs() {
   static const bool done = [] {
+    cudaFuncSetAttribute(k_beam_tangent<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOUNT_SMEM_SPLIT);
     cudaFuncSetAttribute(k_band_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (RING * GF_LDB + RING) * (int)sizeof(double));
     return true;
@@ -1557,8 +1597,24 @@ static void launch_mount(const Batch& b, cudaStream_t st, LaunchProf* prof) {
   if (b.n_elem == 0) return;
   {
     ProfScope q(prof, st, KC_MOUNT);
-    // 44.5 KB of shared memory a CTA, under the 48 KB that needs no attribute
-    k_beam_tangent<<<(b.n_elem + 31) / 32, MOUNT_THREADS, MOUNT_SMEM_BATCH, st>>>(b);
+    const int n = (b.n_elem + 31) / 32;
+    if (b.n_elem <= MOUNT_SPLIT) {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(2 * n);
+      cfg.blockDim = dim3(MOUNT_THREADS);
+      cfg.dynamicSmemBytes = MOUNT_SMEM_SPLIT;
+      cfg.stream = st;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = 2;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      cudaLaunchKernelEx(&cfg, k_beam_tangent<2>, b);
+    } else {
+      k_beam_tangent<1><<<n, MOUNT_THREADS, MOUNT_SMEM_BATCH, st>>>(b);
+    }
     // the pressure's load stiffness is part of the K_e that Rayleigh damping
     // reads (the reference mounts loads before damping)
     if (b.n_pipe_press) k_pipe_pressure<<<(b.n_pipe_press + 31) / 32, PP_THREADS, 0, st>>>(b);
