@@ -833,9 +833,11 @@ template <typename T> void launch_front_factor(const Batch& b, cudaStream_t st) 
         k_mf_panel<T><<<dim3(na + nb, n), 128, 0, st>>>(b, V.big_off, (int)p, na, nca, ncb);
       }
     }
-    if (V.schur_cnt) {
-      if (V.tile == 16) k_mf_schur<T, 16><<<V.schur_cnt, 128, 0, st>>>(b, V.schur_off);
-      else k_mf_schur<T, 32><<<V.schur_cnt, 128, 0, st>>>(b, V.schur_off);
+    if constexpr (sizeof(T) == 8) launch_front_t5(b, V, st);
+    const int jobs = sizeof(T) == 8 ? V.schur_cnt : V.schur_all;
+    if (jobs) {
+      if (V.tile == 16) k_mf_schur<T, 16><<<jobs, 128, 0, st>>>(b, V.schur_off);
+      else k_mf_schur<T, 32><<<jobs, 128, 0, st>>>(b, V.schur_off);
     }
   }
 }

@@ -12,6 +12,7 @@
 // chain is about 3.3 m d pivots, against 2 n kl^2 flops and n pivots of a
 // banded LU.
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -38,6 +39,20 @@ struct Front {
 constexpr int MF_SMALL = 96;
 constexpr int MF_NB = 32;  // pivots per panel of a large front
 
+// Large fronts whose Schur complement takes this many multiply-adds run it on the
+// tensor cores (gf_front_t5.cu) where the caller lets them (GF_WIDE_TENSOR, the
+// default): a 128 x 64 tile takes about 10 us for 64 pivots, an SM's FP64 units 40.
+// Below, the tiles are too few and the slicing's launches (15 us a height) too dear.
+// A rule on the front alone, so a structure is eliminated the same way in any batch.
+constexpr double MF_T5_WORK = 1.5e6;
+// Such a front: its slices, exponents (per 128 pivots) and pivot maxima.
+struct FrontT5 {
+  int64_t slices;  // L21's at oz[slices], U12's behind: [64 pivots][slice][rows][64]
+  int exps, kmax;  // [operand][128 pivots][rows], [operand][s]
+  int rows;        // rows of L21 and columns of U12, padded to 128
+  int front;
+};
+
 // Host schedule of one height.
 struct FrontLevel {
   int small_off = 0, n_small = 0, small_f = 0;  // list range, largest small front
@@ -47,7 +62,11 @@ struct FrontLevel {
   std::vector<int> f_at;                        // largest f among them
   std::vector<int> s_at;                        // largest s among them
   int ext_off = 0, ext_cnt = 0;                 // extend-add jobs of the large fronts
-  int schur_off = 0, schur_cnt = 0, tile = 32;  // Schur jobs and the rows and columns of one
+  int t5_off = 0, t5_cnt = 0, t5_rows = 0, t5_s = 0;  // fronts on the tensor cores, their most rows and pivots
+  int t5_job_off = 0, t5_job_cnt = 0;
+  // Schur jobs (FP32: all of them, the tensor-core fronts' too) and the rows and columns
+  // of one
+  int schur_off = 0, schur_cnt = 0, schur_all = 0, tile = 32;
 };
 struct FrontSchedule {
   std::vector<FrontLevel> level;
@@ -71,6 +90,11 @@ struct FrontData {
   int* map;         // [n_shells][729] destination of K_e entries in F, relative to the structure's first front (-1: none)
   int64_t* base;    // per structure: offset of its fronts in F
   int64_t* size;    // per structure: doubles of its fronts
+  FrontT5* t5;      // by height
+  int2* t5_jobs;    // (t5 entry, row tile | column tile << 16)
+  __nv_bfloat16* oz;
+  int* oz_exp;
+  unsigned long long* oz_kmax;
   double* F;
   double* x;        // solution in the elimination order
   const FrontSchedule* sched;
@@ -116,11 +140,15 @@ struct FrontBuild {
   std::vector<int2> kids, ext_jobs, schur_jobs;
   std::vector<int64_t> base, size;  // per structure (0 for the others)
   int64_t total = 0;
+  std::vector<gf::FrontT5> t5;
+  std::vector<int2> t5_jobs;
+  int64_t oz = 0, oz_exp = 0, oz_kmax = 0;  // entries of the slice buffers (every height uses them in turn)
   gf::FrontSchedule sched;
 };
 // plans[k] belongs to structure slots[k], whose DOFs start at dof_off[k] of
-// n_dofs; base and size are sized for n_struct.
+// n_dofs; base and size are sized for n_struct.  tensor: large Schur complements on
+// the tensor cores.
 void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<int>& slots,
-                 const std::vector<int>& dof_off, int n_struct, int n_dofs, FrontBuild& out);
+                 const std::vector<int>& dof_off, int n_struct, int n_dofs, bool tensor, FrontBuild& out);
 
 }  // namespace gfh

@@ -42,7 +42,7 @@ struct FrontSystem {
   // numbers come back in order).  rhs: n doubles.
   int init(gf_ctx* ctx, const FrontPlan& plan, int n, const double* rhs,
            const std::vector<std::pair<const void*, size_t>>& extra, std::vector<int>* extra_parts) {
-    join_fronts({&plan}, {0}, {0}, 1, n, fb);
+    join_fronts({&plan}, {0}, {0}, 1, n, ctx->wide_update == GF_WIDE_TENSOR, fb);
     info.n_free = n;
     info.wide = 1;
     state.phase = gf::PH_ITER;
@@ -50,14 +50,17 @@ struct FrontSystem {
     auto vec = [&](const auto& v) { return send(v.data(), v.size() * sizeof(v[0])); };
     const int p_fr = vec(fb.fronts), p_bnd = vec(fb.bnd), p_kids = vec(fb.kids),
               p_inv = vec(fb.inv), p_list = vec(fb.list),
-              p_ext = vec(fb.ext_jobs), p_sch = vec(fb.schur_jobs), p_pos = vec(fb.pos), p_df = vec(fb.dof_front),
+              p_ext = vec(fb.ext_jobs), p_sch = vec(fb.schur_jobs), p_t5 = vec(fb.t5), p_t5j = vec(fb.t5_jobs), p_pos = vec(fb.pos), p_df = vec(fb.dof_front),
               p_base = vec(fb.base), p_size = vec(fb.size);
     const int p_info = send(&info, sizeof(info)), p_ws = send(&zero, sizeof(int));
     p_state = send(&state, sizeof(state));
     p_rhs = send(rhs, sizeof(double) * (size_t)n);
     for (const auto& x : extra) extra_parts->push_back(send(x.first, x.second));
-    const size_t off_F = sent, off_x = off_F + ((size_t)fb.total * sizeof(double) + 255) / 256 * 256;
-    total = off_x + sizeof(double) * (size_t)n;
+    auto after = [](size_t at, size_t bytes) { return at + (bytes + 255) / 256 * 256; };
+    const size_t off_F = sent, off_x = after(off_F, (size_t)fb.total * sizeof(double));
+    const size_t off_oz = after(off_x, sizeof(double) * (size_t)n), off_km = after(off_oz, (size_t)fb.oz * 2);
+    const size_t off_ex = after(off_km, (size_t)fb.oz_kmax * sizeof(unsigned long long));
+    total = off_ex + (size_t)fb.oz_exp * sizeof(int);
     dev = static_cast<char*>(ctx->device_work(total));
     char* pin = static_cast<char*>(ctx->pinned(sent));
     if (!dev || !pin) {
@@ -88,6 +91,11 @@ struct FrontSystem {
     d.size = at<int64_t>(p_size);
     d.F = reinterpret_cast<double*>(dev + off_F);
     d.x = reinterpret_cast<double*>(dev + off_x);
+    d.t5 = at<gf::FrontT5>(p_t5);
+    d.t5_jobs = at<int2>(p_t5j);
+    d.oz = reinterpret_cast<__nv_bfloat16*>(dev + off_oz);
+    d.oz_kmax = reinterpret_cast<unsigned long long*>(dev + off_km);
+    d.oz_exp = reinterpret_cast<int*>(dev + off_ex);
     d.sched = &fb.sched;
     return GF_OK;
   }

@@ -1134,7 +1134,7 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
         offs.push_back(dof_offs[s]);
       }
       FrontBuild fb;
-      join_fronts(plans, wide_structs, offs, n, dof_off, fb);
+      join_fronts(plans, wide_structs, offs, n, dof_off, B->opts.wide_update == GF_WIDE_TENSOR, fb);
       FrontData& md = sd.mf;
       md.n_fronts = (int)fb.fronts.size();
       if (!upload(B, &md.fronts, fb.fronts) || !upload(B, &md.bnd, fb.bnd) || !upload(B, &md.rel, fb.rel) ||
@@ -1144,6 +1144,8 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
           !upload(B, &md.kids, fb.kids) || !upload(B, &md.inv, fb.inv) || !upload(B, &md.dof_at, fb.dof_at) ||
           !upload(B, &md.base, fb.base) || !upload(B, &md.size, fb.size) ||
           !balloc(B, &md.map, (size_t)shell_off * 729) || !balloc(B, &md.F, (size_t)fb.total) ||
+          !upload(B, &md.t5, fb.t5) || !upload(B, &md.t5_jobs, fb.t5_jobs) || !balloc(B, &md.oz, (size_t)fb.oz) ||
+          !balloc(B, &md.oz_exp, (size_t)fb.oz_exp) || !balloc(B, &md.oz_kmax, (size_t)fb.oz_kmax) ||
           !balloc(B, &md.x, (size_t)dof_off))
         return GF_ERR_CUDA;
       B->sched = std::move(fb.sched);

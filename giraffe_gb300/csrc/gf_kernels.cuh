@@ -120,6 +120,8 @@ void launch_front_solve(const Batch& b, cudaStream_t st, LaunchProf* prof = null
 void launch_front_csr(const Batch& b, int n, const int* rp, const int* ci, const double* v, cudaStream_t st);
 void launch_front_band(const Batch& b, int n, int kl, int ku, int ldab, const double* ab, cudaStream_t st);
 int front_launches(const Batch& b);
+// The Schur complements of a height's fronts on the tensor cores (gf_front_t5.cu).
+void launch_front_t5(const Batch& b, const FrontLevel& V, cudaStream_t st);
 // FP32: the same on r32, and another right-hand side with that factor.
 void launch_front_solve32(const Batch& b, cudaStream_t st, LaunchProf* prof = nullptr);
 void launch_front_resolve32(const Batch& b, cudaStream_t st);

@@ -309,7 +309,7 @@ static int small_limit(const std::vector<gf::Front>& fronts, const std::vector<i
 }
 
 void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<int>& slots,
-                 const std::vector<int>& dof_off, int n_struct, int n_dofs, FrontBuild& out) {
+                 const std::vector<int>& dof_off, int n_struct, int n_dofs, bool tensor, FrontBuild& out) {
   out.pos.assign(n_dofs, -1);
   out.dof_front.assign(n_dofs, -1);
   out.base.assign(n_struct, 0);
@@ -399,25 +399,56 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
     V.schur_off = (int)out.schur_jobs.size();
     // 32 x 32 tiles, or 16 x 16 while those leave SMs idle in the last wave: a tile
     // holds an SM's FP64 units for its whole product
+    auto on_t5 = [&](int k) {
+      const double u = out.fronts[k].f - out.fronts[k].s;
+      return tensor && out.fronts[k].s * u * u >= gf::MF_T5_WORK;
+    };
     auto tiles = [&](int t) {
       int64_t n = 0;
       for (int k : big) {
+        if (on_t5(k)) continue;
         const int u = out.fronts[k].f - out.fronts[k].s;
         if (u > 0) n += (int64_t)((u + t) / t) * ((u + t - 1) / t);
       }
       return n;
     };
     if (4 * ((tiles(32) + 151) / 152) * 10 > 13 * ((tiles(16) + 151) / 152)) V.tile = 16;
-    for (int k : big) {
-      const gf::Front& F = out.fronts[k];
-      const int u = F.f - F.s;
-      V.big_f = std::max(V.big_f, F.f);
+    auto jobs = [&](int k) {
+      const int u = out.fronts[k].f - out.fronts[k].s;
       if (u > 0)
         for (int tj = 0; tj < (u + V.tile) / V.tile; ++tj)
           for (int ti = 0; ti < (u + V.tile - 1) / V.tile; ++ti) out.schur_jobs.push_back(make_int2(k, ti | (tj << 16)));
+    };
+    for (int k : big) {
+      V.big_f = std::max(V.big_f, out.fronts[k].f);
+      if (!on_t5(k)) jobs(k);
     }
     V.schur_cnt = (int)out.schur_jobs.size() - V.schur_off;
-    out.sched.launches += (V.ext_cnt ? 1 : 0) + (V.n_small ? 1 : 0) + (V.schur_cnt ? 1 : 0) + 1;
+    for (int k : big)
+      if (on_t5(k)) jobs(k);
+    V.schur_all = (int)out.schur_jobs.size() - V.schur_off;
+    V.t5_off = (int)out.t5.size();
+    V.t5_job_off = (int)out.t5_jobs.size();
+    int64_t oz = 0, exps = 0, kmax = 0;
+    for (int k : big) {
+      if (!on_t5(k)) continue;
+      const gf::Front& F = out.fronts[k];
+      const int u = F.f - F.s, rows = (u + 127) / 128 * 128, id = (int)out.t5.size();
+      out.t5.push_back(gf::FrontT5{oz, (int)exps, (int)kmax, rows, k});
+      oz += (int64_t)2 * ((F.s + 63) / 64) * 8 * rows * 64;
+      exps += (int64_t)2 * ((F.s + 127) / 128) * rows;
+      kmax += 2 * F.s;
+      V.t5_rows = std::max(V.t5_rows, rows);
+      V.t5_s = std::max(V.t5_s, F.s);
+      for (int tj = 0; tj < (u + 63) / 64; ++tj)
+        for (int ti = 0; ti < (u + 127) / 128; ++ti) out.t5_jobs.push_back(make_int2(id, ti | (tj << 16)));
+    }
+    out.oz = std::max(out.oz, oz);
+    out.oz_exp = std::max(out.oz_exp, exps);
+    out.oz_kmax = std::max(out.oz_kmax, kmax);
+    V.t5_cnt = (int)out.t5.size() - V.t5_off;
+    V.t5_job_cnt = (int)out.t5_jobs.size() - V.t5_job_off;
+    out.sched.launches += (V.ext_cnt ? 1 : 0) + (V.n_small ? 1 : 0) + (V.schur_cnt ? 1 : 0) + (V.t5_cnt ? 3 : 0) + 1;
     for (int p = 0; p < panels; ++p)
       out.sched.launches += 1 + (V.f_at[p] > p * gf::MF_NB ? 1 : 0) + (V.s_at[p] > (p + 1) * gf::MF_NB ? 1 : 0);
   }

@@ -196,3 +196,60 @@ def test_mixed_fronts_refine_to_the_fp64_solve(gpu_ctx, make):
     scale = np.abs(ff[0][:, :3] - make().nodes).max()
     assert np.abs(fm[0][:, :3] - ff[0][:, :3]).max() <= 1e-10 * scale
     assert em[0][2] == 0 and em[0][1] >= em[0][0] > 0
+
+
+@pytest.mark.parametrize("n", [28, 36])
+def test_tensor_core_fronts(gpu_ctx, n):
+    """Plates whose top fronts take the tensor cores (288 boundary DOFs and 69
+    pivots on), beside a small one: the FP64 fronts' counts and states to 1e-10
+    of the displacement scale (the plain path's stated tolerance), the same bits
+    alone, and the mixed path's fallback still the FP64 path exactly."""
+    def run(structs, **kw):
+        b = gpu.BatchSolver(gpu_ctx, structs, gpu_ctx.opts(**kw))
+        b.reset()
+        b.run()
+        out = b.results()
+        b.close()
+        return out
+
+    make = lambda: configs.square_plate(n, steps=2)
+    ft, st = run([configs.square_plate(5, steps=2), make()], wide_update=gpu.GF_WIDE_TENSOR)
+    ff, sf = run([make()], wide_update=gpu.GF_WIDE_FP64)
+    fa, _ = run([make()])
+    fb, _ = run([make()], precision=gpu.GF_PREC_MIXED, max_refine=1)
+    assert np.array_equal(st[1], sf[0])
+    scale = np.abs(ff[0][:, :3] - make().nodes).max()
+    assert np.abs(ft[1][:, :3] - ff[0][:, :3]).max() <= 1e-10 * scale
+    assert np.array_equal(ft[1], fa[0]) and np.array_equal(fa[0], fb[0])
+
+
+def test_tensor_core_fronts_of_a_sparse_system(gpu_ctx):
+    # rows scaled over eight decades; forward error bound n eps cond with cond <= 5
+    # for these row sums once the scaling is taken out: 1e-12
+    g, d = 40, 3
+    n = g * g * d
+    x = np.arange(n) // d
+    rng = np.random.default_rng(9)
+    rows, cols = [], []
+    for v in range(g * g):
+        for a in (-1, 0, 1):
+            for b in (-1, 0, 1):
+                if 0 <= v % g + a < g and 0 <= v // g + b < g:
+                    w = v + a + g * b
+                    for i in range(d):
+                        rows += [v * d + i] * d
+                        cols += list(range(w * d, w * d + d))
+    rows, cols = np.array(rows), np.array(cols)
+    val = rng.uniform(-1.0, 1.0, len(rows))
+    val[rows == cols] = 0.0
+    sums = np.bincount(rows, np.abs(val), n)
+    val[rows == cols] = 1.5 * sums[rows[rows == cols]] + 0.1
+    val = val * 10.0 ** rng.integers(-4, 5, n)[rows]
+    order = np.lexsort((cols, rows))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.int32)
+    ref = rng.normal(size=n)
+    b = np.zeros(n)
+    np.add.at(b, rows, val * ref[cols])
+    sol, info = gpu_ctx.sparse_solve(rp, cols[order].astype(np.int32), val[order], b)
+    assert info == 0
+    assert np.abs(sol - ref).max() <= 1e-12 * np.abs(ref).max()
