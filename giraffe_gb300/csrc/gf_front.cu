@@ -299,29 +299,16 @@ template <typename T> __global__ void __launch_bounds__(MF_SMALL_THREADS) k_mf_s
   if (bad && lane == 0) mf_fail<T>(b, F.slot);
 }
 
-// LU of the diagonal block of panel p of the large fronts of a height, one CTA
-// each: a chain of pivots (update of a column, reciprocal, multipliers), 540 cycles
-// each if nothing holds them up.  The pivot warp (warp 3) has a sub-partition to
-// itself; six warps on the other three update the remaining columns, lane i row i,
-// a column at a time (FP64 instructions take their 64 cycles even where a predicate
-// turns every lane off, so the loop ends at the last column; three warps with the
-// columns in registers took 1,120 cycles a pivot, packed lanes 1,150, this 700).
-constexpr int MF_DIAG_THREADS = 224;
-template <typename T> __global__ void __launch_bounds__(MF_DIAG_THREADS) k_mf_diag(Batch b, int off, int p) {
-  const FrontData& d = b.sh.mf;
-  const Front F = d.list[off + blockIdx.x];
-  const bool on = mf_active(b, F.slot);
-  constexpr int WARPS = MF_DIAG_THREADS / 32;
-  const int k0 = p * MF_NB, nb = min(MF_NB, F.s - k0), ld = F.ld, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  T* G = mf_mat<T>(b, F) + k0 + (int64_t)k0 * ld;
-  __shared__ T A[MF_NB][MF_NB + 1];  // A[j][i]: column j, row i
-#pragma unroll
-  for (int q = 0; q < (MF_NB + WARPS - 1) / WARPS; ++q) {
-    const int j = warp + WARPS * q;
-    if (j < nb) A[j][lane] = lane < nb ? G[lane + (int64_t)j * ld] : T(0);
-  }
-  if (!on) return;
-  __syncthreads();
+// LU of a 32 x 32 diagonal block in shared memory (A[j][i]: column j, row i; nb of it)
+// by a CTA of MF_DIAG_THREADS: a chain of pivots (update of a column, reciprocal,
+// multipliers), 540 cycles each if nothing holds them up.  The pivot warp (warp 3) has
+// a sub-partition to itself; six warps on the other three update the remaining
+// columns, lane i row i, a column at a time (FP64 instructions take their 64 cycles
+// even where a predicate turns every lane off, so the loop ends at the last column;
+// three warps with the columns in registers took 1,120 cycles a pivot, packed lanes
+// 1,150, this 700).  True where a pivot failed.
+constexpr int MF_DIAG_THREADS = 256;
+template <typename T> __device__ __forceinline__ bool mf_block_lu(T (*A)[MF_NB + 1], int nb, int warp, int lane) {
   bool bad = false;
   T a = T(0), l = T(0);
   // pivot k of the updated column a: lane i keeps the multiplier of row i
@@ -344,18 +331,38 @@ template <typename T> __global__ void __launch_bounds__(MF_DIAG_THREADS) k_mf_di
       const T u = __shfl_sync(0xffffffffu, a, k);
       if (lane > k) a = mfma(-l, u, a);
       pivot(k + 1);
-    } else {
+    } else if (warp < 7) {
       const T x = -A[k][lane];
-      for (int j = k + 2 + (warp < 3 ? warp : warp - 1); j < nb; j += WARPS - 1) {
+      for (int j = k + 2 + (warp < 3 ? warp : warp - 1); j < nb; j += 6) {
         const T v = mfma(x, A[j][k], A[j][lane]);
         if (lane > k) A[j][lane] = v;
       }
     }
     __syncthreads();
   }
+  return bad;
+}
+
+// The first diagonal block of the large fronts of a height, one CTA each (k_mf_panel
+// factors the next one of a front as it forms it).
+template <typename T> __global__ void __launch_bounds__(MF_DIAG_THREADS) k_mf_diag(Batch b, int off) {
+  const FrontData& d = b.sh.mf;
+  const Front F = d.list[off + blockIdx.x];
+  const bool on = mf_active(b, F.slot);
+  const int nb = min(MF_NB, F.s), ld = F.ld, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  T* G = mf_mat<T>(b, F);
+  __shared__ T A[MF_NB][MF_NB + 1];
 #pragma unroll
-  for (int q = 0; q < (MF_NB + WARPS - 1) / WARPS; ++q) {
-    const int j = warp + WARPS * q;
+  for (int q = 0; q < MF_NB / 8; ++q) {
+    const int j = warp + 8 * q;
+    if (j < nb) A[j][lane] = lane < nb ? G[lane + (int64_t)j * ld] : T(0);
+  }
+  if (!on) return;
+  __syncthreads();
+  const bool bad = mf_block_lu<T>(A, nb, warp, lane);
+#pragma unroll
+  for (int q = 0; q < MF_NB / 8; ++q) {
+    const int j = warp + 8 * q;
     if (lane < nb && j < nb) G[lane + (int64_t)j * ld] = A[j][lane];
   }
   if (bad && lane == 0) mf_fail<T>(b, F.slot);
@@ -420,20 +427,63 @@ template <typename T, int L> __global__ void __launch_bounds__(128) k_mf_trsm(Ba
 // later columns (blockIdx.x < na) and the boundary rows of the later pivot
 // columns, minus L U over the panel's pivots.  16 x 32 tiles, so that the few
 // tiles of the top fronts spread over the SMs (a tile holds an SM's FP64 units
-// for 512 warp instructions, about 5 us).
+// for 512 warp instructions, about 5 us).  The first CTA of a front takes the 32 x 32
+// tile of the next diagonal block and factors it (mf_block_lu) while the others run:
+// a launch per panel and 14 us less on the chain of panels.
+constexpr int MF_PANEL_THREADS = 256;
+static_assert(MF_PANEL_THREADS == MF_DIAG_THREADS, "the panel's first CTA factors a block");
 template <typename T>
-__global__ void __launch_bounds__(128) k_mf_panel(Batch b, int off, int p, int na, int nca, int ncb) {
+__global__ void __launch_bounds__(MF_PANEL_THREADS) k_mf_panel(Batch b, int off, int p, int na, int nca, int ncb) {
   const FrontData& d = b.sh.mf;
   const Front F = d.list[off + blockIdx.y];
   const bool on = mf_active(b, F.slot);
   const int k0 = p * MF_NB, k1 = k0 + MF_NB, ld = F.ld, tid = threadIdx.x;
   if (k1 >= F.s) return;
+  T* G = mf_mat<T>(b, F);
+  __shared__ T Ls[MF_NB][33];  // [k][row]
+  __shared__ T Us[32][MF_NB + 1];  // [column][k]
+  if (blockIdx.x == 0) {
+    const int lane = tid & 31, warp = tid >> 5, r1 = F.s, c1 = F.f + 1, nb = min(MF_NB, F.s - k1);
+    T acc[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int y = warp + 8 * q;  // pivot of L, column of U and of the tile
+      Ls[y][lane] = k1 + lane < r1 ? G[k1 + lane + (int64_t)(k0 + y) * ld] : T(0);
+      Us[y][lane] = k1 + y < c1 ? G[k0 + lane + (int64_t)(k1 + y) * ld] : T(0);
+      acc[q] = (k1 + lane < r1 && k1 + y < c1) ? G[k1 + lane + (int64_t)(k1 + y) * ld] : T(0);
+    }
+    if (!on) return;
+    __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < MF_NB; ++k) {
+      const T l = -Ls[k][lane];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = mfma(l, Us[warp + 8 * q][k], acc[q]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int y = warp + 8 * q;
+      if (y < nb) Ls[y][lane] = acc[q];  // the diagonal block, column y
+      else if (lane < nb && k1 + y < c1) G[k1 + lane + (int64_t)(k1 + y) * ld] = acc[q];
+    }
+    __syncthreads();
+    const bool bad = mf_block_lu<T>(Ls, nb, warp, lane);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int y = warp + 8 * q;
+      if (lane < nb && y < nb) G[k1 + lane + (int64_t)(k1 + y) * ld] = Ls[y][lane];
+    }
+    if (bad && lane == 0) mf_fail<T>(b, F.slot);
+    return;
+  }
   int r0, c0, r1, c1;
   if ((int)blockIdx.x < na) {
     r0 = k1 + 16 * ((int)blockIdx.x / nca);
     c0 = k1 + 32 * ((int)blockIdx.x % nca);
     r1 = F.s;
     c1 = F.f + 1;
+    if (r0 == k1 + 16 && c0 == k1) return;  // the first CTA's other half
   } else {
     const int x = (int)blockIdx.x - na;
     r0 = F.s + 16 * (x / ncb);
@@ -442,33 +492,29 @@ __global__ void __launch_bounds__(128) k_mf_panel(Batch b, int off, int p, int n
     c1 = F.s;
   }
   if (r0 >= r1 || c0 >= c1) return;
-  T* G = mf_mat<T>(b, F);
-  __shared__ T Ls[MF_NB][17];  // [k][row]
-  __shared__ T Us[32][MF_NB + 1];  // [column][k]
-  for (int x = tid; x < MF_NB * 16; x += 128) {
-    const int i = x & 15, k = x >> 4;
-    Ls[k][i] = r0 + i < r1 ? G[r0 + i + (int64_t)(k0 + k) * ld] : T(0);
-  }
-  for (int x = tid; x < 32 * MF_NB; x += 128) {
-    const int k = x & 31, c = x >> 5;
+  const int i = tid & 15, cg = tid >> 4;  // row, columns cg + 16 q
+#pragma unroll
+  for (int q = 0; q < 2; ++q) Ls[cg + 16 * q][i] = r0 + i < r1 ? G[r0 + i + (int64_t)(k0 + cg + 16 * q) * ld] : T(0);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int k = tid & 31, c = (tid >> 5) + 8 * q;
     Us[c][k] = c0 + c < c1 ? G[k0 + k + (int64_t)(c0 + c) * ld] : T(0);
   }
-  const int i = tid & 15, cg = tid >> 4;  // row, columns cg + 8 q
-  T acc[4];
+  T acc[2];
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
-    acc[q] = (r0 + i < r1 && c0 + cg + 8 * q < c1) ? G[r0 + i + (int64_t)(c0 + cg + 8 * q) * ld] : T(0);
+  for (int q = 0; q < 2; ++q)
+    acc[q] = (r0 + i < r1 && c0 + cg + 16 * q < c1) ? G[r0 + i + (int64_t)(c0 + cg + 16 * q) * ld] : T(0);
   if (!on) return;
   __syncthreads();
 #pragma unroll 8
   for (int k = 0; k < MF_NB; ++k) {
     const T l = -Ls[k][i];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[q] = mfma(l, Us[cg + 8 * q][k], acc[q]);
+    for (int q = 0; q < 2; ++q) acc[q] = mfma(l, Us[cg + 16 * q][k], acc[q]);
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
-    if (r0 + i < r1 && c0 + cg + 8 * q < c1) G[r0 + i + (int64_t)(c0 + cg + 8 * q) * ld] = acc[q];
+  for (int q = 0; q < 2; ++q)
+    if (r0 + i < r1 && c0 + cg + 16 * q < c1) G[r0 + i + (int64_t)(c0 + cg + 16 * q) * ld] = acc[q];
 }
 
 // The Schur complement of the large fronts of a height: C -= L21 U12 over all
@@ -814,7 +860,7 @@ template <typename T> void launch_front_factor(const Batch& b, cudaStream_t st) 
           b, V.small_off);
     for (size_t p = 0; p < V.n_at.size(); ++p) {
       const int n = V.n_at[p], k0 = (int)p * MF_NB, k1 = k0 + MF_NB, f = V.f_at[p], s = V.s_at[p];
-      k_mf_diag<T><<<n, MF_DIAG_THREADS, 0, st>>>(b, V.big_off, (int)p);
+      if (p == 0) k_mf_diag<T><<<n, MF_DIAG_THREADS, 0, st>>>(b, V.big_off);
       // the panels of fronts whose last panel this is end before k1
       const int m = f - k0 - 1;
       if (m >= 0) {
@@ -830,7 +876,7 @@ template <typename T> void launch_front_factor(const Batch& b, cudaStream_t st) 
       if (s > k1) {
         const int nca = (f + 1 - k1 + 31) / 32, na = (s - k1 + 15) / 16 * nca;
         const int ncb = (s - k1 + 31) / 32, nb = (f + 15) / 16 * ncb;
-        k_mf_panel<T><<<dim3(na + nb, n), 128, 0, st>>>(b, V.big_off, (int)p, na, nca, ncb);
+        k_mf_panel<T><<<dim3(na + nb, n), MF_PANEL_THREADS, 0, st>>>(b, V.big_off, (int)p, na, nca, ncb);
       }
     }
     if constexpr (sizeof(T) == 8) launch_front_t5(b, V, st);
