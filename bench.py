@@ -37,6 +37,8 @@ UNIT = "Newton solves/s"
 # DRAM bytes per element mount of k_beam_tangent, from one ncu capture on 128
 # chains: (54.9 MB read + 173.1 MB written) / 79,322 elements
 TANGENT_DRAM_BYTES_PER_ELEMENT = (55.088384e6 + 202.853120e6) / 79322
+# FP64 flops of one element in k_beam_tangent (an FMA counts two)
+TANGENT_FLOPS = 3270.0
 
 
 def parse():
@@ -276,9 +278,8 @@ def plain_leg(ctx, structs, sample_n):
 
 
 def mixed_leg(ctx, structs, args, f64_finals, f64_stats):
-    """The same batched workload with GF_PREC_MIXED (the Beam_1 tangent
-    operator in FP32-pair arithmetic; force, residual, rotations and solves
-    FP64), device-timed like the headline, with its deviation from the FP64
+    """The same batched workload with GF_PREC_MIXED (which changes Shell_1
+    solves only: chains stay FP64 throughout), device-timed like the headline, with its deviation from the FP64
     path: max over chains of |u_mixed - u_fp64| / |u_fp64| (translations,
     2-norm) and of the nodal rotation tensors."""
     import ctypes as C
@@ -301,9 +302,7 @@ def mixed_leg(ctx, structs, args, f64_finals, f64_stats):
         rel_u = max(rel_u, float(np.linalg.norm(u_m - u_f) / np.linalg.norm(u_f)))
         dq = max(dq, float(np.abs(fm[k][:, 6:] - f64_finals[k][:, 6:]).max()))
     return {"value": solves / (ms.value / 1e3), "unit": UNIT, "ms_per_step": ms.value / args.mixed_steps,
-            "precision": "Beam_1 tangent: rotation to the global frame and K_e expansion in FP32-pair (~48-bit) "
-                         "arithmetic on the FP32 pipe; Gauss-point operator, internal force, residual, rotation "
-                         "updates, chain/band solves and convergence checks FP64",
+            "precision": "FP64 throughout: the mixed option's FP32 factor applies to Shell_1 structures",
             "max_rel_err_displacement_vs_fp64": rel_u, "max_abs_err_rotation_vs_fp64": dq,
             "same_step_and_iteration_counts": bool(np.array_equal(sm, f64_stats)),
             "structures_with_other_counts": int((sm != f64_stats).any(axis=1).sum())}
@@ -313,7 +312,7 @@ def shell_leg(ctx, args, fp64_peak):
     """The Shell_1 plate (64x64 squares x 2 six-node triangles, 84,867 free
     DOFs, clamped edges, follower pressure ramped to 1e5 Pa over 20 load
     steps): the first `shell_steps` load steps, device-timed, with the
-    wide-band LU's FP64 rate; and an 8x8 plate solved completely by the GPU
+    LU's rate in banded-LU-equivalent flops; and an 8x8 plate solved completely by the GPU
     and by the oracle on the host cores, like for like."""
     import ctypes as C
 
@@ -323,8 +322,7 @@ def shell_leg(ctx, args, fp64_peak):
     L = ctx.L
     s = configs.square_plate(args.shell_n, steps=20)
     s.solution.end_time = args.shell_steps / 20.0
-    # the first two steps with the trailing update in FP64 FMA and in the
-    # mma.sync form, for comparison
+    # the first two steps with every product in FP64 FMA, for comparison
     s2 = configs.square_plate(args.shell_n, steps=20)
     s2.solution.end_time = min(args.shell_steps, 2) / 20.0
     b2 = gpu.BatchSolver(ctx, [s2])
@@ -337,7 +335,7 @@ def shell_leg(ctx, args, fp64_peak):
     ms_fp64 = bf.run()
     st_fp64 = bf.results()[1]
     bf.close()
-    # and with the warp-level mma.sync form of the tensor-core update
+    # and with the warp-level mma.sync option (FP64 FMA in the multifrontal LU)
     bsy = gpu.BatchSolver(ctx, [s2], ctx.opts(wide_update=gpu.GF_WIDE_TENSOR_SYNC))
     bsy.reset()
     ms_sync = bsy.run()
@@ -354,8 +352,7 @@ def shell_leg(ctx, args, fp64_peak):
     launches = b.launches()
     tiles = b.wide_tiles()
     # per-kernel-class device time of a pass over the first load step (events
-    # around every launch, no graph; classes on the lookahead's helper
-    # streams overlap the main stream, so the classes sum to more than a pass)
+    # around every launch, no graph)
     L.gf_batch_profile.argtypes = [C.c_void_p, C.POINTER(C.c_double), C.POINTER(C.c_longlong)]
     L.gf_kernel_name.restype = C.c_char_p
     s1 = configs.square_plate(args.shell_n, steps=20)
@@ -367,7 +364,7 @@ def shell_leg(ctx, args, fp64_peak):
     bp.close()
     split = {L.gf_kernel_name(i).decode(): round(kms[i] / passes, 3) for i in range(gpu.GF_N_KERNELS) if kl[i]}
     # the sparsesystem drop-in on the same plate: the first pass's K_AA as a
-    # host CSR, solved through gf_sparse_solve (ordering, upload, wide-band
+    # host CSR, solved through gf_sparse_solve (ordering, upload, multifrontal
     # LU, solution back to the host)
     rp, ci, v, P = b.assemble_csr(0)
     b.close()
@@ -382,9 +379,10 @@ def shell_leg(ctx, args, fp64_peak):
                           f"nnz {len(v)}, "
                           f"half-bandwidth {kl_sp}", "ms": t_sp * 1e3, "linear_solves_per_s": 1.0 / t_sp,
               "info": int(info), "lu_tflops_end_to_end": 2.0 * n_sp * kl_sp * kl_sp / t_sp / 1e12,
-              "note": "host CSR in, x out; includes the RCM trial, CSR upload, scatter, factor and "
-                      "substitutions (2 n kl^2 flops counted)"}
-    # FP32 band factor with FP64 iterative refinement (GF_PREC_MIXED), the
+              "note": "host CSR in, x out; includes the nested dissection, CSR upload, scatter, factor and "
+                      "substitutions (a banded LU's 2 n kl^2 flops counted; the multifrontal LU does about "
+                      "a fortieth of them)"}
+    # FP32 factor with FP64 iterative refinement (GF_PREC_MIXED), the
     # same plate and load steps
     sm_ = configs.square_plate(args.shell_n, steps=20)
     sm_.solution.end_time = args.shell_steps / 20.0
@@ -403,7 +401,7 @@ def shell_leg(ctx, args, fp64_peak):
     bpm.close()
     split_mx = {L.gf_kernel_name(i).decode(): round(kms[i] / passes_m, 3) for i in range(gpu.GF_N_KERNELS) if kl[i]}
     u64 = fin[0][:, :3] - s.nodes
-    mixed = {"precision": "FP32 wide-band LU (FP32 FMA panel kernels and trailing update) beside the FP64 K_AA; "
+    mixed = {"precision": "FP32 multifrontal LU beside the FP64 element matrices; "
                           "FP64 residual b - K x and x += K32^-1 r until a correction is below 2^-52 |x| or "
                           "shrinks by less than half; FP64 refactor when refinement stalls above 2^-30 |x| or "
                           "exceeds 30 sweeps",
@@ -432,8 +430,9 @@ def shell_leg(ctx, args, fp64_peak):
                         f"{dims[1]}, first {args.shell_steps} of 20 load steps",
             "newton_solves": int(st[0][0]), "newton_passes": int(st[0][1]), "ms": ms,
             "solves_per_s": st[0][0] / (ms / 1e3), "ms_per_pass": ms / max(1, st[0][1]),
-            "wide_update": "tensor cores: FP64 products from exact bf16 slices (Ozaki), tcgen05.mma 128x64x16 with "
-                           "TMEM accumulators, bulk-copy (TMA) staged slices",
+            "wide_update": "multifrontal LU, Schur complements of the largest fronts on the tensor cores: FP64 "
+                           "products from exact bf16 slices (Ozaki), tcgen05.mma 128x64x16 with TMEM accumulators, "
+                           "bulk-copy (TMA) staged slices; wide_lu_tflops counts a banded LU's 2 n kl^2 flops",
             "wide_lu_tflops": lu.value / (ms / 1e3) / 1e12, "fp64_peak_tflops": fp64_peak,
             "wide_lu_frac_of_measured_fp64": lu.value / (ms / 1e3) / 1e12 / fp64_peak,
             "first_two_steps": {"tcgen05_ms_per_pass": ms_tc2 / max(1, st_tc2[0][1]),
@@ -448,8 +447,7 @@ def shell_leg(ctx, args, fp64_peak):
                                     float(np.abs(f_sync[0][:, :3] - f_tc2[0][:, :3]).max())},
             "gpu_launches": launches, "center_deflection_m": float(fin[0][:, 2].min()),
             "wide_tiles": {"trsm_rows": tiles[0], "first_trsm_rows": tiles[1], "corner_tile": tiles[2],
-                           "solve_rows": tiles[3], "how": "picked by the library's autotuner (timed on a "
-                                                         "synthetic band of the plate's half-bandwidth)"},
+                           "solve_rows": tiles[3], "how": "defaults (the multifrontal LU does not use them)"},
             "pass_split_ms": split,
             "sparse_solve": sparse,
             "mixed_precision": mixed,
@@ -711,10 +709,12 @@ def run_ours(args, rank, world):
     peaks, tag = measured_peaks()
     # The dominant single kernel is k_beam_tangent (the chain solver is a
     # class of nine kernels, none as large); its roofline is the headline one,
-    # the chain solver's is reported beside it.
+    # the chain solver's is reported beside it.  The library counts 9,000 flops
+    # per mount, those of the 3x3 matrix products as written in the reference;
+    # the kernel's symmetric form takes 1,930 FP64 operations, 1,340 of them FMA.
     def tangent_roof(name):
         t = kernels[name]["ms"] / 1e3
-        achieved = mnt_f.value / t / 1e12
+        achieved = mnt_f.value / 9000.0 * TANGENT_FLOPS / t / 1e12
         mounts_per_launch = mnt_f.value / 9000.0 / max(kernels[name]["launches"], 1)
         return {"kernel": name, "bound": "fp64", "achieved": achieved, "peak": fp64.value, "unit": "TFLOP/s",
                 "frac": achieved / fp64.value,
@@ -724,7 +724,7 @@ def run_ours(args, rank, world):
                                   f"{TANGENT_DRAM_BYTES_PER_ELEMENT:.0f} B per element, scaled by the "
                                   f"{mounts_per_launch:.0f} element mounts of an average launch here",
                 "note": "FP64 CUDA-core bound (no HBM or tensor-core bound applies: per-element 18x18 algebra); "
-                        "achieved counts 9000 FP64 flops per Beam_1 Mount (both Gauss points); peak = FP64 FMA "
+                        f"achieved counts the kernel's own {TANGENT_FLOPS:.0f} FP64 flops per Beam_1 Mount; peak = FP64 FMA "
                         "throughput measured live by gf_device_fp_peaks (of measured); HBM view: "
                         f"{TANGENT_DRAM_BYTES_PER_ELEMENT * mnt_f.value / 9000.0 / t / 1e9:.1f} GB/s of "
                         f"{peaks.get('hbm_gbs')} GB/s {tag}"}
@@ -736,8 +736,8 @@ def run_ours(args, rank, world):
                 "frac": achieved / fp64.value, "traffic": None,
                 "note": "FP64 CUDA-core bound; achieved counts the banded-LU-equivalent flops 2 n kl ku + "
                         "2 n (kl+ku) per Newton solve of each structure (the chain solver's own count, "
-                        "condensation + cyclic reduction, is about 0.8 of it); peak = FP64 FMA throughput "
-                        "measured live (of measured)"}
+                        "condensation and merges, is about 0.4 of it, so the fraction can pass 1); peak = FP64 "
+                        "FMA throughput measured live (of measured)"}
 
     if "beam_tangent" in kernels:
         roof = tangent_roof("beam_tangent")

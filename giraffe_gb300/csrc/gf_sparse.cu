@@ -129,17 +129,22 @@ namespace gfh {
 
 // The multifrontal LU eliminates a band of half-bandwidth w in blocks of w,
 // about 6.3 w^3 multiply-adds a block on a chain of log2(n / w) blocks; the
-// banded LU takes w^2 per column on a chain of n.  Measured: the 35-row band
-// solver takes 0.9 us a column and the wide-band LU about 85 us per 64 columns
-// plus its updates at 5.4 TFLOP/s, the fronts 0.8 TFLOP/s and about 0.6 us a
-// pivot of the chain.  Both are estimated at those rates.
+// banded LU takes w^2 per column on a chain of n.  Both are estimated: the 35-row
+// band solver at 0.9 us a column, the wide-band LU at 85 us per 64 columns plus its
+// updates at 5.4 TFLOP/s, either with 0.17 ms of allocations and copies; the fronts
+// at 0.9 TFLOP/s, 0.6 us a pivot of the chain and 12 us a height.  Measured, band
+// against fronts, half-bandwidth and n: 2 and 60 0.26 / 0.09 ms, 12 and 2,000 1.92 /
+// 0.32, 17 and 60,000 52.5 / 5.0, 60 and 20,000 30.0 / 4.5, 120 and 600 1.20 / 0.76,
+// 240 and 2,000 3.42 / 2.78, 240 and 60,000 92.9 / 71.8; the other way 480 and 2,000
+// 3.56 / 5.07, 480 and 60,000 98 / 166, 900 and 20,000 34 / 130.
 bool band_takes_fronts(int n, int kl, int ku) {
   const double w = std::max(std::max(kl, ku), 12);
   const double blocks = n / w;
   if (blocks < 4.0) return false;
   const double chain = w * (std::ceil(std::log2(blocks)) + 1.0);
-  const double t_front = 12.6 * w * w * n / 0.8e12 + 0.6e-6 * chain + 12e-6 * chain / w;
-  const double t_band = kl <= GF_KB && ku <= GF_KB ? 0.9e-6 * n : n / 64.0 * 85e-6 + 2.0 * n * w * w / 5.4e12;
+  const double t_front = 12.6 * w * w * n / 0.9e12 + 0.6e-6 * chain + 12e-6 * chain / w;
+  const double t_band =
+      0.17e-3 + (kl <= GF_KB && ku <= GF_KB ? 0.9e-6 * n : n / 64.0 * 85e-6 + 2.0 * n * w * w / 5.4e12);
   return t_front < t_band;
 }
 

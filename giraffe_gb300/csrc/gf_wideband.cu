@@ -1,4 +1,6 @@
-// The wide-band LU of Shell_1 structures' K_AA and its triangular solves.
+// The wide-band LU and its triangular solves: the factor of modal analysis, and the
+// solve of linear systems whose band or graph the multifrontal LU (gf_front.cu) does
+// not suit.
 //
 // Wide band: K_AA of a structure with free-DOF half-bandwidth kl is stored
 // column-major with 2 kl + 1 rows.  No pivoting (the reference's tangent

@@ -273,7 +273,7 @@ class Context:
         return x, info.value
 
     def set_standalone_opts(self, wide_update=GF_WIDE_TENSOR):
-        """gf_ctx_set_opts: the wide-band trailing update of this context's
+        """gf_ctx_set_opts: how the large products are formed in this context's
         standalone solves (band_solve, sparse_solve)."""
         o = self.opts(wide_update=wide_update)
         self.check(self.L.gf_ctx_set_opts(self.h, C.byref(o)), "gf_ctx_set_opts")
@@ -499,7 +499,7 @@ class BatchSolver:
 
     def solve_stats(self):
         """Per structure, after results(): linear solves, FP64 refinement
-        sweeps of the FP32 wide-band factor and solves refactored in FP64
+        sweeps of the FP32 factor and solves refactored in FP64
         (GF_PREC_MIXED), as rows [linear_solves, refine_sweeps,
         fp64_fallbacks]."""
         return np.array([[x.linear_solves, x.refine_sweeps, x.fp64_fallbacks] for x in self.last_stats])

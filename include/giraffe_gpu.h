@@ -77,16 +77,18 @@ typedef struct gf_solve_opts {
                       iterative refinement) */
   int poll_every;  /* Newton passes between host checks for completion */
   int use_graph;   /* capture one Newton pass as a CUDA graph */
-  int wide_update; /* Shell_1 wide-band LU trailing update: GF_WIDE_TENSOR (the
+  int wide_update; /* how the large products of the LU of Shell_1 structures
+                      and of wide linear systems are formed: GF_WIDE_TENSOR (the
                       default: FP64 products emulated from exact bf16 slices
                       on the tensor cores, Ozaki scheme, tcgen05.mma with
-                      tensor-memory accumulators), GF_WIDE_TENSOR_SYNC (the
-                      same emulation on warp-level mma.sync) or GF_WIDE_FP64
-                      (FP64 FMA).  The emulated product of row i of L21 and
-                      column j of U12 (K = 64 terms) errs by at most about
-                      2^-52 K max_k |L_ik 2^-f_k| max_k |2^f_k U_kj|, where
-                      2^f_k is a power-of-two balancing of the panel's column
-                      k of L21 against row k of U12 (chosen per panel); for
+                      tensor-memory accumulators) or GF_WIDE_FP64 (FP64 FMA);
+                      GF_WIDE_TENSOR_SYNC runs the same emulation on warp-level
+                      mma.sync where the wide-band LU is used, FP64 FMA in the
+                      multifrontal LU.  The emulated product of row i of L21 and
+                      column j of U12 (K <= 128 terms at a time) errs by at most
+                      about 2^-52 K max_k |L_ik 2^-f_k| max_k |2^f_k U_kj|, where
+                      2^f_k is a power-of-two balancing of pivot k's column
+                      of L21 against its row of U12; for
                       rows whose terms differ greatly in magnitude that can
                       exceed the FP64 rounding of the product sum */
   int max_passes;  /* host cap on the Newton passes of one gf_batch_run;
@@ -94,16 +96,14 @@ typedef struct gf_solve_opts {
                       default of 4,000,000) */
   int monitor_rows; /* monitor lines kept per structure with a Monitor
                       (gf_model_desc monitor_nodes; 0: none recorded) */
-  int max_refine;  /* GF_PREC_MIXED: FP64 refinement sweeps of a wide-band
+  int max_refine;  /* GF_PREC_MIXED: FP64 refinement sweeps of a Shell_1
                       solve before its FP64 fallback (0: the default of 30) */
-  int wide_tiles[4]; /* Shell_1 wide-band LU tile shapes: rows per CTA of the
-                      bulk trsm (4, 8, 16) and of the first trsm (1, 2, 4),
+  int wide_tiles[4]; /* tile shapes of the blocked wide-band LU: rows per CTA of
+                      the bulk trsm (4, 8, 16) and of the first trsm (1, 2, 4),
                       the corner update's tile edge (4, 8), rows per CTA of
-                      the triangular solves (32, 64).  An entry of 0 is picked
-                      by the autotuner, which times the shapes on a synthetic
-                      band of the structures' half-bandwidth once per context
-                      (served waves take the defaults 8, 2, 8, 64).  No
-                      choice changes any result. */
+                      the triangular solves (32, 64); 0: the defaults 8, 2, 8,
+                      64.  Checked and reported; Shell_1 structures are solved
+                      by the multifrontal LU, which does not use them. */
 } gf_solve_opts;
 enum { GF_WIDE_FP64 = 0, GF_WIDE_TENSOR = 1, GF_WIDE_TENSOR_SYNC = 2 };
 
@@ -114,8 +114,8 @@ typedef struct gf_stats {
   int bisections;         /* rolled-back steps */
   int aborted;            /* 1 when the step size fell below MinTimeStep */
   int linear_solves;      /* linear solves performed */
-  int refine_sweeps;      /* GF_PREC_MIXED: FP64 refinement sweeps of the FP32 wide-band factor */
-  int fp64_fallbacks;     /* GF_PREC_MIXED: wide-band solves refactored in FP64 */
+  int refine_sweeps;      /* GF_PREC_MIXED: FP64 refinement sweeps of the FP32 factor */
+  int fp64_fallbacks;     /* GF_PREC_MIXED: solves refactored in FP64 */
 } gf_stats;
 
 /* Context on CUDA device `device`; NULL on failure. */
@@ -125,7 +125,7 @@ const char* gf_last_error(const gf_ctx* ctx);
 void gf_default_opts(gf_solve_opts* opts);
 /* Options of the context's standalone solves (gf_band_solve and
  * gf_sparse_solve, which have no options argument, as bandsystem and
- * sparsesystem have none): their wide-band trailing update follows
+ * sparsesystem have none): their large products follow
  * opts->wide_update (GF_WIDE_TENSOR until set).  The batch entry points take
  * their own options. */
 int gf_ctx_set_opts(gf_ctx* ctx, const gf_solve_opts* opts);
@@ -133,8 +133,8 @@ int gf_ctx_set_opts(gf_ctx* ctx, const gf_solve_opts* opts);
 /* Uploads n structures into one device batch: each a sequence of Static and
  * Dynamic solution steps of Beam_1 elements or of Shell_1 elements (with
  * follower pressures), with nodal loads, constraints and prescribed
- * displacements.  Shell_1 structures are solved by the wide-band LU on the
- * narrower of the reference's numbering and reverse Cuthill-McKee. */
+ * displacements.  Shell_1 structures are solved by a multifrontal LU under a
+ * nested-dissection ordering of their nodes. */
 gf_batch* gf_batch_create(gf_ctx* ctx, int n, const gf_model_desc* models, const gf_solve_opts* opts);
 void gf_batch_destroy(gf_batch* batch);
 /* Restores the initial configuration of every structure (device side). */
@@ -261,8 +261,9 @@ int gf_shell_inertia_elements(gf_ctx* ctx, int n, const double* xyz, const doubl
 
 /* Solves A x = b for a banded matrix given in the reference's BandMatrix
  * storage (LAPACK GB: entry (i,j) at ab[(kl+ku+i-j) + j*ldab], ldab >=
- * 2*kl+ku+1), without pivoting, FP64.  kl, ku <= 17 run on the 35-row band
- * solver; wider bands on the blocked wide-band LU with half-bandwidth
+ * 2*kl+ku+1), without pivoting, FP64: by a multifrontal LU under a
+ * nested-dissection ordering where that is the faster way, else by the 35-row
+ * band solver (kl, ku <= 17) or the blocked wide-band LU with half-bandwidth
  * max(kl, ku).  b is overwritten by x.  *info receives 0 or 1 (zero or
  * non-finite pivot), as bandsystem's info_fail. */
 int gf_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, int* info);
@@ -270,10 +271,10 @@ int gf_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab
 /* Replaces sparsesystem (src/SparseMatrix.cpp:74-166, the Newton step's
  * solve) for one system K x = b, K in SparseMatrix's layout: Eigen
  * row-major CSR, 0-based (row_ptr[n+1], col_idx[nnz], val[nnz]; entries
- * repeated within a row are summed).  The unknowns are ordered by the
- * narrower of their natural order and reverse Cuthill-McKee on the
- * symmetrised pattern; the factorization is the no-pivot banded LU of
- * gf_band_solve on the GPU, FP64.  b (n) is overwritten by x.  *info
+ * repeated within a row are summed).  A natural half-bandwidth up to 17 is
+ * solved as gf_band_solve does; any other pattern by a no-pivot multifrontal LU
+ * under a nested dissection of the symmetrised pattern (where its fronts do not
+ * fit, by the blocked wide-band LU in reverse Cuthill-McKee order), FP64.  b (n) is overwritten by x.  *info
  * receives 0 or 1 (zero or non-finite pivot), as sparsesystem's info_fail;
  * the return value reports argument and CUDA errors. */
 int gf_sparse_solve(gf_ctx* ctx, int n, const int* row_ptr, const int* col_idx, const double* val, double* b,

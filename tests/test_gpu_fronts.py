@@ -200,8 +200,7 @@ def test_mixed_fronts_refine_to_the_fp64_solve(gpu_ctx, make):
 
 @pytest.mark.parametrize("n", [28, 36])
 def test_tensor_core_fronts(gpu_ctx, n):
-    """Plates whose top fronts take the tensor cores (288 boundary DOFs and 69
-    pivots on), beside a small one: the FP64 fronts' counts and states to 1e-10
+    """Plates whose larger fronts take the tensor cores, beside a small one: the FP64 fronts' counts and states to 1e-10
     of the displacement scale (the plain path's stated tolerance), the same bits
     alone, and the mixed path's fallback still the FP64 path exactly."""
     def run(structs, **kw):
