@@ -23,6 +23,7 @@
 // every 64 cycles at any instruction-level parallelism, an SM one every 19),
 // so the large fronts are bound by FP64 throughput and the chain of panels by
 // the dependent results of each pivot.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cfloat>
@@ -35,6 +36,8 @@
 namespace gf {
 
 namespace {
+
+namespace cg = cooperative_groups;
 
 // A structure whose K_AA this launch factors (in the FP64 fallback launches of
 // the mixed path only those whose refinement did not finish).
@@ -620,168 +623,237 @@ template <typename T> __device__ __forceinline__ T mf_block_fwd(const T (*D)[33]
   return v;
 }
 
-// Back substitution of every front of a height, one CTA each: w = y - U12 x2,
-// then x1 = U11^-1 w in blocks of 32: warp 0 solves a block's triangle while the
-// others load the next one's and every thread its row above the block, then every
-// thread takes its rows.  The blocks' chain (150 cycles a DOF) bounds the tall
-// fronts; with the triangle's entries read from memory it was 600.
+// The substitutions take a front by a cluster of C CTAs (C = 1, 2, 4 or 8, see
+// subst_ctas); its rows go in groups of 32 to the ranks in turn, and every row's
+// sums are in the same order whatever C is.  A block of 32 own DOFs is solved by
+// warp 0 of the rank that owns it and handed to all of them in their shared memory
+// (xb); then four warps take a group's rows, a quarter of the block's columns each
+// from registers that were loaded while the block was solved.
+//
+// Bound by latency: the blocks' chain (150 cycles a DOF in FP64, 35 in FP32) and the
+// rounds of loads before it.  One CTA a front took 70 us a height on the 64x64x2
+// plate (0.84 ms of a 6.2 ms pass), where the top fronts' U12 alone is 44 us of one
+// SM's FP64 rate, and 11 us a height and sweep on the 24x24x2 plate's FP32 fronts,
+// most of it four loads at a time from L2 over U12's columns.
 constexpr int MF_BACK_THREADS = 256, MF_PART = 512;
-template <typename T> __global__ void __launch_bounds__(MF_BACK_THREADS) k_mf_back(Batch b, int off) {
+
+template <typename T> struct MfSubst {
+  T D[2][32][33];   // diagonal blocks: column j, row i
+  T xb[2][32];      // a solved block
+  T part[8 * 32];   // quarter sums of two groups
+};
+
+__device__ __forceinline__ void mf_sync(cg::cluster_group& cl, int C) {
+  if (C == 1) __syncthreads();
+  else cl.sync();
+}
+
+// The rows of group h (one per lane) less a solved block's columns: quarter q of the
+// columns j0 .. j0 + 31 into g, zero outside the front's s columns.
+template <typename T> __device__ __forceinline__ void mf_cols(T* g, const T* G, int ld, int row, bool in, int j0, int s, int q) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int k = j0 + q + 4 * i;
+    g[i] = (in && k < s) ? G[row + (int64_t)k * ld] : T(0);
+  }
+}
+
+// One step of either substitution: the block's x in xb, the rank's groups first,
+// first + dir C, ... (n of them) less its columns, two groups at a time; rows in
+// [lo, hi).  g: the quarter of the first pair's columns that this warp loaded ahead.
+template <typename T>
+__device__ __forceinline__ void mf_apply(MfSubst<T>& m, T* w, const T* g0, const T* xb, const T* G, int ld, int first,
+                                         int step, int n, int lo, int hi, int j0, int s) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = warp & 3;
+  T g[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) g[i] = g0[i];
+  for (int t = 0; t < n; t += 2) {
+    const int mine = t + (warp >> 2);
+    if (t > 0) {
+      const int row = 32 * (first + step * mine) + lane;
+      mf_cols(g, G, ld, row, mine < n && row >= lo && row < hi, j0, s, q);
+    }
+    if (mine < n) {
+      T a = T(0);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a = mfma(g[i], xb[q + 4 * i], a);
+      m.part[warp * 32 + lane] = a;
+    }
+    __syncthreads();
+    // group t by warp 0, which solves the next block from it, and t + 1 by warp 4
+    if (q == 0 && mine < n) {
+      const int row = 32 * (first + step * mine) + lane;
+      const T* z = m.part + warp * 32 + lane;
+      if (row >= lo && row < hi) w[row] -= (z[0] + z[32]) + (z[64] + z[96]);
+    }
+    if (t + 2 < n) __syncthreads();
+  }
+}
+
+// Back substitution of every front of a height: w = y - U12 x2, the eight warps an
+// eighth of the columns each, then x1 = U11^-1 w in blocks of 32.
+template <typename T> __global__ void __launch_bounds__(MF_BACK_THREADS) k_mf_back(Batch b, int off, int C) {
   const FrontData& d = b.sh.mf;
-  const Front F = d.list[off + blockIdx.x];
+  const Front F = d.list[off + blockIdx.x / C];
   if (!mf_active(b, F.slot)) return;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = C == 1 ? 0 : (int)cl.block_rank();
   const int f = F.f, s = F.s, u = f - s, ld = F.ld, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const T* G = mf_mat<T>(b, F);
   T* x = mf_x<T>(b);
   const int* B = d.bnd + F.bnd;
-  __shared__ T D[2][32][33];
+  __shared__ MfSubst<T> m;
   extern __shared__ __align__(16) unsigned char mf_raw[];
-  T* w = reinterpret_cast<T*>(mf_raw);  // [f]: w of the own DOFs, then x2
-  T* part = w + f + (f & 1);            // [8][rows of a chunk]
-  const int sp = min((s + 31) / 32 * 32, MF_PART);
-  auto block = [&](T (*E)[33], int j0) {  // the diagonal block at j0 into E
+  T* w = reinterpret_cast<T*>(mf_raw);  // [f]: w of the rank's own DOFs, then x2
+  T* part = w + f + (f & 1);            // [8][rows of a chunk of the rank's groups]
+  const int ng = (s + 31) / 32, own = (ng - rank + C - 1) / C;
+  const int sp = min(own * 32, MF_PART);
+  // the diagonal block of group h into E, by warps w0 to 7
+  auto block = [&](T (*E)[33], int h, int w0) {
+    const int j0 = 32 * h, i = lane;
+    if (warp < w0) return;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = lane, j = warp + 8 * q;
-      E[j][i] = (j0 + i < s && j0 + j < s) ? G[j0 + i + (int64_t)(j0 + j) * ld] : T(0);
+    for (int q = 0; q < 5; ++q) {
+      const int j = warp - w0 + (8 - w0) * q;
+      if (j < 32) E[j][i] = (j0 + i < s && j0 + j < s) ? G[j0 + i + (int64_t)(j0 + j) * ld] : T(0);
     }
   };
-  const int last = (s - 1) / 32 * 32;
-  block(D[0], last);
-  for (int i = tid; i < s; i += MF_BACK_THREADS) w[i] = G[i + (int64_t)f * ld];
-  for (int i = tid; i < u; i += MF_BACK_THREADS) w[s + i] = x[B[i]];
-  __syncthreads();
-  for (int c0 = 0; u > 0 && c0 < s; c0 += MF_PART) {
-    // 32 rows at a time, the eight warps an eighth of the columns each
-    for (int i0 = c0; i0 < min(s, c0 + MF_PART); i0 += 32) {
-      const int i = i0 + lane;
+  if (own > 0) block(m.D[0], rank + C * (own - 1), 0);
+  for (int i = tid; i < own * 32; i += MF_BACK_THREADS) {
+    const int r = 32 * (rank + C * (i / 32)) + i % 32;
+    if (r < s) w[r] = G[r + (int64_t)f * ld];
+  }
+  if (own > 0)
+    for (int i = tid; i < u; i += MF_BACK_THREADS) w[s + i] = x[B[i]];
+  mf_sync(cl, C);  // every rank runs before the first block is handed over
+  for (int c0 = 0; u > 0 && c0 < own * 32; c0 += MF_PART) {
+    const int c1 = min(own * 32, c0 + MF_PART);
+    for (int i0 = c0; i0 < c1; i0 += 32) {
+      const int r = 32 * (rank + C * (i0 / 32)) + lane;
       T acc[4] = {T(0), T(0), T(0), T(0)};
-      if (i < s) {
-        const T* g = G + i;
-        int j = s + warp;
-        for (; j + 24 < f; j += 32) {
+      const T* g = G + min(r, s - 1);
+      for (int j = s + warp; j < f; j += 128) {
+        T v[16];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) acc[q] = mfma(g[(int64_t)(j + 8 * q) * ld], w[j + 8 * q], acc[q]);
-        }
+        for (int q = 0; q < 16; ++q) v[q] = j + 8 * q < f ? g[(int64_t)(j + 8 * q) * ld] : T(0);
 #pragma unroll
-        for (int q = 0; q < 3; ++q)
-          if (j + 8 * q < f) acc[q] = mfma(g[(int64_t)(j + 8 * q) * ld], w[j + 8 * q], acc[q]);
+        for (int q = 0; q < 16; ++q)
+          if (j + 8 * q < f) acc[q & 3] = mfma(v[q], w[j + 8 * q], acc[q & 3]);
       }
-      part[warp * sp + i - c0] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+      part[warp * sp + i0 - c0 + lane] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
     }
     __syncthreads();
-    for (int i = c0 + tid; i < min(s, c0 + MF_PART); i += MF_BACK_THREADS) {
+    for (int i = c0 + tid; i < c1; i += MF_BACK_THREADS) {
+      const int r = 32 * (rank + C * (i / 32)) + i % 32;
       T t = part[i - c0];
       for (int q = 1; q < 8; ++q) t += part[q * sp + i - c0];
-      w[i] -= t;
+      if (r < s) w[r] -= t;
     }
     __syncthreads();
   }
   int cur = 0;
-  for (int j0 = last; j0 >= 0; j0 -= 32, cur ^= 1) {
-    const int nb = min(32, s - j0);
-    T g[32];
-    const bool mine = tid < j0;  // this thread's first row above the block
-#pragma unroll
-    for (int k = 0; k < 32; ++k) g[k] = (mine && k < nb) ? G[tid + (int64_t)(j0 + k) * ld] : T(0);
-    if (warp == 0) {
-      const T v = mf_block_back<T>(D[cur], nb, lane, lane < nb ? w[j0 + lane] : T(0));
-      if (lane < nb) {
-        w[j0 + lane] = v;
-        x[F.dof0 + j0 + lane] = v;
-      }
+  for (int h = ng - 1; h >= 0; --h) {
+    const int j0 = 32 * h, nb = min(32, s - j0), p = h & 1;
+    // the rank's groups below h, downwards
+    const int n = (h - rank + C - 1) / C, first = rank + C * (n - 1);
+    T g[8];
+    {
+      const int mine = warp >> 2, row = 32 * (first - C * mine) + lane;
+      mf_cols(g, G, ld, row, mine < n, j0, s, warp & 3);
     }
-    if (j0 > 0) block(D[cur ^ 1], j0 - 32);
-    __syncthreads();
-    if (mine) {
-      T a0 = T(0), a1 = T(0);
-#pragma unroll
-      for (int k = 0; k < 32; k += 2) {
-        if (k < nb) a0 = mfma(g[k], w[j0 + k], a0);
-        if (k + 1 < nb) a1 = mfma(g[k + 1], w[j0 + k + 1], a1);
+    if (h % C == rank) {
+      if (warp == 0) {
+        const T v = mf_block_back<T>(m.D[cur], nb, lane, lane < nb ? w[j0 + lane] : T(0));
+        if (lane < nb) x[F.dof0 + j0 + lane] = v;
+        if (C == 1) m.xb[p][lane] = v;
+        else
+          for (int c = 0; c < C; ++c) cl.map_shared_rank(&m.xb[p][0], c)[lane] = v;
       }
-      w[tid] -= a0 + a1;
+      cur ^= 1;
+      if (n > 0) block(m.D[cur], first, 1);
     }
-    for (int i = tid + MF_BACK_THREADS; i < j0; i += MF_BACK_THREADS) {
-      T a0 = T(0), a1 = T(0);
-#pragma unroll 8
-      for (int k = 0; k < 32; k += 2) {
-        if (k < nb) a0 = mfma(G[i + (int64_t)(j0 + k) * ld], w[j0 + k], a0);
-        if (k + 1 < nb) a1 = mfma(G[i + (int64_t)(j0 + k + 1) * ld], w[j0 + k + 1], a1);
-      }
-      w[i] -= a0 + a1;
-    }
-    __syncthreads();
+    mf_sync(cl, C);
+    if (n > 0) mf_apply(m, w, g, m.xb[p], G, ld, first, -C, n, 0, s, j0, s);
   }
 }
 
-// Forward substitution alone, on fronts that hold their LU: every front of a
-// height, one CTA each.  w = the right-hand side of the own DOFs with what the
-// children leave (column f of theirs, one child after the other), then y1 =
-// L11^-1 w1 in blocks of 32 and w2 -= L21 y1, as in k_mf_back; both into column f.
-template <typename T> __global__ void __launch_bounds__(MF_BACK_THREADS) k_mf_fwd(Batch b, int off) {
+// Forward substitution alone, on fronts that hold their LU: every front of a height.
+// w = the right-hand side of the own DOFs with what the children leave (column f of
+// theirs, one child after the other), then y1 = L11^-1 w1 in blocks of 32 and w2 -=
+// L21 y1; both into column f.
+template <typename T> __global__ void __launch_bounds__(MF_BACK_THREADS) k_mf_fwd(Batch b, int off, int C) {
   const FrontData& d = b.sh.mf;
-  const Front F = d.list[off + blockIdx.x];
+  const Front F = d.list[off + blockIdx.x / C];
   if (!mf_active(b, F.slot)) return;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = C == 1 ? 0 : (int)cl.block_rank();
   const int f = F.f, s = F.s, ld = F.ld, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   T* G = mf_mat<T>(b, F);
-  __shared__ T D[2][32][33];
+  __shared__ MfSubst<T> m;
   extern __shared__ __align__(16) unsigned char mf_raw[];
-  T* w = reinterpret_cast<T*>(mf_raw);  // [f]
+  T* w = reinterpret_cast<T*>(mf_raw);  // [f], the rank's rows used
   const T* P = mf_rhs(b, (T*)nullptr);
-  auto block = [&](T (*E)[33], int j0) {
+  const int ng = (s + 31) / 32, nr = (f + 31) / 32, own = (nr - rank + C - 1) / C;
+  auto block = [&](T (*E)[33], int h, int w0) {
+    const int j0 = 32 * h, i = lane;
+    if (warp < w0) return;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = lane, j = warp + 8 * q;
-      E[j][i] = (j0 + i < s && j0 + j < s) ? G[j0 + i + (int64_t)(j0 + j) * ld] : T(0);
+    for (int q = 0; q < 5; ++q) {
+      const int j = warp - w0 + (8 - w0) * q;
+      if (j < 32) E[j][i] = (j0 + i < s && j0 + j < s) ? G[j0 + i + (int64_t)(j0 + j) * ld] : T(0);
     }
   };
-  block(D[0], 0);
-  for (int i = tid; i < f; i += MF_BACK_THREADS) {
-    T v = i < s ? P[d.dof_at[F.dof0 + i]] : T(0);
-    for (int k = F.kid0; k < F.kid1; ++k) {
-      const int2 kid = d.kids[k];
-      const Front& C = d.fronts[kid.x];
-      const int ci = d.inv[kid.y + i];
-      if (ci >= 0) v += reinterpret_cast<const T*>(d.F)[C.off + C.s + ci + (int64_t)C.f * C.ld];
+  if (rank < ng) block(m.D[0], rank, 0);
+  for (int i = tid; i < own * 32; i += MF_BACK_THREADS) {
+    const int r = 32 * (rank + C * (i / 32)) + i % 32;
+    if (r >= f) continue;
+    T v = r < s ? P[d.dof_at[F.dof0 + r]] : T(0);
+    for (int k = F.kid0; k < F.kid1; k += 2) {  // two children's loads side by side
+      const bool two = k + 1 < F.kid1;
+      const int2 k0 = d.kids[k], k1 = d.kids[two ? k + 1 : k];
+      const Front &C0 = d.fronts[k0.x], &C1 = d.fronts[k1.x];
+      const int i0 = d.inv[k0.y + r], i1 = two ? d.inv[k1.y + r] : -1;
+      const T* X = reinterpret_cast<const T*>(d.F);
+      const T v0 = i0 >= 0 ? X[C0.off + C0.s + i0 + (int64_t)C0.f * C0.ld] : T(0);
+      const T v1 = i1 >= 0 ? X[C1.off + C1.s + i1 + (int64_t)C1.f * C1.ld] : T(0);
+      if (i0 >= 0) v += v0;
+      if (i1 >= 0) v += v1;
     }
-    w[i] = v;
+    w[r] = v;
+  }
+  mf_sync(cl, C);
+  int cur = 0;
+  for (int h = 0; h < ng; ++h) {
+    const int j0 = 32 * h, nb = min(32, s - j0), p = h & 1;
+    // the rank's groups with rows below the block, upwards: the block's own where it
+    // is short
+    const int g0 = nb < 32 ? h : h + 1, first = g0 + (rank - g0 % C + C) % C;
+    const int n = first < nr ? (nr - first + C - 1) / C : 0;
+    T g[8];
+    {
+      const int mine = warp >> 2, row = 32 * (first + C * mine) + lane;
+      mf_cols(g, G, ld, row, mine < n && row >= j0 + nb && row < f, j0, s, warp & 3);
+    }
+    if (h % C == rank) {
+      if (warp == 0) {
+        const T v = mf_block_fwd<T>(m.D[cur], nb, lane, lane < nb ? w[j0 + lane] : T(0));
+        if (lane < nb) w[j0 + lane] = v;
+        if (C == 1) m.xb[p][lane] = v;
+        else
+          for (int c = 0; c < C; ++c) cl.map_shared_rank(&m.xb[p][0], c)[lane] = v;
+      }
+      cur ^= 1;
+      if (h + C < ng) block(m.D[cur], h + C, 1);
+    }
+    mf_sync(cl, C);
+    if (n > 0) mf_apply(m, w, g, m.xb[p], G, ld, first, C, n, j0 + nb, f, j0, s);
   }
   __syncthreads();
-  int cur = 0;
-  for (int j0 = 0; j0 < s; j0 += 32, cur ^= 1) {
-    const int nb = min(32, s - j0), r = j0 + nb + tid;
-    T g[32];
-    const bool mine = r < f;  // this thread's first row below the block
-#pragma unroll
-    for (int k = 0; k < 32; ++k) g[k] = (mine && k < nb) ? G[r + (int64_t)(j0 + k) * ld] : T(0);
-    if (warp == 0) {
-      const T v = mf_block_fwd<T>(D[cur], nb, lane, lane < nb ? w[j0 + lane] : T(0));
-      if (lane < nb) w[j0 + lane] = v;
-    }
-    if (j0 + 32 < s) block(D[cur ^ 1], j0 + 32);
-    __syncthreads();
-    if (mine) {
-      T a0 = T(0), a1 = T(0);
-#pragma unroll
-      for (int k = 0; k < 32; k += 2) {
-        if (k < nb) a0 = mfma(g[k], w[j0 + k], a0);
-        if (k + 1 < nb) a1 = mfma(g[k + 1], w[j0 + k + 1], a1);
-      }
-      w[r] -= a0 + a1;
-    }
-    for (int i = r + MF_BACK_THREADS; i < f; i += MF_BACK_THREADS) {
-      T a0 = T(0), a1 = T(0);
-#pragma unroll 8
-      for (int k = 0; k < 32; k += 2) {
-        if (k < nb) a0 = mfma(G[i + (int64_t)(j0 + k) * ld], w[j0 + k], a0);
-        if (k + 1 < nb) a1 = mfma(G[i + (int64_t)(j0 + k + 1) * ld], w[j0 + k + 1], a1);
-      }
-      w[i] -= a0 + a1;
-    }
-    __syncthreads();
+  for (int i = tid; i < own * 32; i += MF_BACK_THREADS) {
+    const int r = 32 * (rank + C * (i / 32)) + i % 32;
+    if (r < f) G[r + (int64_t)f * ld] = w[r];
   }
-  for (int i = tid; i < f; i += MF_BACK_THREADS) G[i + (int64_t)f * ld] = w[i];
 }
 
 // ---- standalone systems (one structure): matrix entries into the fronts ----
@@ -888,12 +960,38 @@ template <typename T> void launch_front_factor(const Batch& b, cudaStream_t st) 
   }
 }
 
+namespace {
+// CTAs of a front in the substitutions: as many as leave an SM one, up to a group of
+// 32 rows each.
+int subst_ctas(int n, int rows) {
+  int C = 1;
+  while (C < 8 && 2 * C * n <= 152 && C * 32 < rows) C *= 2;
+  return C;
+}
+template <typename K> void launch_subst(K kernel, const Batch& b, int off, int n, int C, size_t smem, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(n * C);
+  cfg.blockDim = dim3(MF_BACK_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, b, off, C);
+}
+}  // namespace
+
 template <typename T> void launch_front_back(const Batch& b, cudaStream_t st) {
   const FrontSchedule& sc = *b.sh.mf.sched;
   for (size_t l = sc.level.size(); l-- > 0;) {
     const FrontLevel& V = sc.level[l];
-    const size_t n = (size_t)std::max(V.small_f, V.big_f) + 2 + 8 * (size_t)std::min((V.max_s + 31) / 32 * 32, MF_PART);
-    k_mf_back<T><<<V.n_small + V.n_big, MF_BACK_THREADS, n * sizeof(T), st>>>(b, V.small_off);
+    const int n = V.n_small + V.n_big, C = subst_ctas(n, V.max_s), f = std::max(V.small_f, V.big_f);
+    const size_t w = (size_t)f + 2 + 8 * (size_t)std::min(((V.max_s + 31) / 32 + C - 1) / C * 32, MF_PART);
+    launch_subst(k_mf_back<T>, b, V.small_off, n, C, w * sizeof(T), st);
   }
   k_mf_out<T><<<dim3(dof_blocks(b), b.sh.n_wide), 256, 0, st>>>(b);
 }
@@ -914,8 +1012,8 @@ void launch_front_solve32(const Batch& b, cudaStream_t st, LaunchProf* prof) {
 // Another right-hand side (r32) with the FP32 factor.
 void launch_front_resolve32(const Batch& b, cudaStream_t st) {
   for (const FrontLevel& V : b.sh.mf.sched->level) {
-    const int f = std::max(V.small_f, V.big_f);
-    k_mf_fwd<float><<<V.n_small + V.n_big, MF_BACK_THREADS, (size_t)f * sizeof(float), st>>>(b, V.small_off);
+    const int n = V.n_small + V.n_big, f = std::max(V.small_f, V.big_f);
+    launch_subst(k_mf_fwd<float>, b, V.small_off, n, subst_ctas(n, f), (size_t)f * sizeof(float), st);
   }
   launch_front_back<float>(b, st);
 }

@@ -252,3 +252,34 @@ def test_tensor_core_fronts_of_a_sparse_system(gpu_ctx):
     sol, info = gpu_ctx.sparse_solve(rp, cols[order].astype(np.int32), val[order], b)
     assert info == 0
     assert np.abs(sol - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 65, 97, 257, 600])
+def test_substitution_of_one_front(gpu_ctx, n):
+    # a full matrix is one front of n own DOFs: clusters of one to eight CTAs, blocks
+    # of 32 with and without a remainder; diagonally dominant, forward error n eps cond
+    # with cond <= 5: 1e-12
+    rng = np.random.default_rng(n)
+    A = rng.uniform(-1.0, 1.0, (n, n))
+    A[np.arange(n), np.arange(n)] = 1.5 * np.abs(A).sum(1) + 0.1
+    ref = rng.normal(size=n)
+    rp = np.arange(0, n * n + 1, n, dtype=np.int32)
+    sol, info = gpu_ctx.sparse_solve(rp, np.tile(np.arange(n, dtype=np.int32), n), A.ravel(), A @ ref)
+    assert info == 0
+    assert np.abs(sol - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("n,copies", [(3, 160), (9, 30), (13, 12)])
+def test_substitution_does_not_depend_on_the_batch(gpu_ctx, n, copies, mixed):
+    # a front's CTAs follow from the fronts of its height, its bits do not
+    opts = gpu_ctx.opts(precision=gpu.GF_PREC_MIXED if mixed else gpu.GF_PREC_FP64)
+    out = []
+    for k in (1, copies):
+        b = gpu.BatchSolver(gpu_ctx, [configs.square_plate(n, steps=2)] * k, opts)
+        b.reset()
+        b.run()
+        out.append(b.results())
+        b.close()
+    for q in range(copies):
+        assert np.array_equal(out[0][0][0], out[1][0][q]) and np.array_equal(out[0][1][0], out[1][1][q])
