@@ -605,20 +605,39 @@ template <typename T, int R> __global__ void __launch_bounds__(128) k_mf_schur(B
     }
 }
 
-// Substitution on a 32 x 32 diagonal block: D[j][i] its column j, row i.  Lane i
-// holds w_i of the block.
+// Substitution on a 32 x 32 diagonal block: D[j][i] its column j, row i (zero outside
+// the nb used).  Lane i holds w_i of the block.  Eight columns at a time from
+// registers, so that no load waits on the chain.
 template <typename T> __device__ __forceinline__ T mf_block_back(const T (*D)[33], int nb, int lane, T v) {
-  for (int k = nb - 1; k >= 0; --k) {
-    const T xk = __shfl_sync(0xffffffffu, v, k) * D[k][k];  // the reciprocal
-    if (lane == k) v = xk;
-    if (lane < k) v = mfma(-D[k][lane], xk, v);
+  const T r = D[lane][lane];  // the reciprocal
+#pragma unroll
+  for (int k0 = 24; k0 >= 0; k0 -= 8) {
+    if (k0 >= nb) continue;
+    T c[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) c[q] = -D[k0 + q][lane];
+#pragma unroll
+    for (int q = 7; q >= 0; --q) {
+      if (k0 + q >= nb) continue;
+      const T xk = __shfl_sync(0xffffffffu, v * r, k0 + q);
+      if (lane == k0 + q) v = xk;
+      if (lane < k0 + q) v = mfma(c[q], xk, v);
+    }
   }
   return v;
 }
 template <typename T> __device__ __forceinline__ T mf_block_fwd(const T (*D)[33], int nb, int lane, T v) {
-  for (int k = 0; k + 1 < nb; ++k) {
-    const T yk = __shfl_sync(0xffffffffu, v, k);
-    if (lane > k) v = mfma(-D[k][lane], yk, v);
+#pragma unroll
+  for (int k0 = 0; k0 < 32; k0 += 8) {
+    if (k0 >= nb) continue;
+    T c[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) c[q] = -D[k0 + q][lane];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const T yk = __shfl_sync(0xffffffffu, v, k0 + q);
+      if (lane > k0 + q) v = mfma(c[q], yk, v);
+    }
   }
   return v;
 }
@@ -630,8 +649,8 @@ template <typename T> __device__ __forceinline__ T mf_block_fwd(const T (*D)[33]
 // (xb); then four warps take a group's rows, a quarter of the block's columns each
 // from registers that were loaded while the block was solved.
 //
-// Bound by latency: the blocks' chain (150 cycles a DOF in FP64, 35 in FP32) and the
-// rounds of loads before it.  One CTA a front took 70 us a height on the 64x64x2
+// Bound by latency: the blocks' chain (two dependent FP64 operations and a shuffle a
+// DOF) and the rounds of loads before it.  One CTA a front took 70 us a height on the 64x64x2
 // plate (0.84 ms of a 6.2 ms pass), where the top fronts' U12 alone is 44 us of one
 // SM's FP64 rate, and 11 us a height and sweep on the 24x24x2 plate's FP32 fronts,
 // most of it four loads at a time from L2 over U12's columns.
@@ -993,7 +1012,7 @@ template <typename T> void launch_front_back(const Batch& b, cudaStream_t st) {
     const size_t w = (size_t)f + 2 + 8 * (size_t)std::min(((V.max_s + 31) / 32 + C - 1) / C * 32, MF_PART);
     launch_subst(k_mf_back<T>, b, V.small_off, n, C, w * sizeof(T), st);
   }
-  k_mf_out<T><<<dim3(dof_blocks(b), b.sh.n_wide), 256, 0, st>>>(b);
+  if constexpr (sizeof(T) == 8) k_mf_out<T><<<dim3(dof_blocks(b), b.sh.n_wide), 256, 0, st>>>(b);
 }
 
 void launch_front_solve(const Batch& b, cudaStream_t st, LaunchProf* prof) {
@@ -1003,7 +1022,7 @@ void launch_front_solve(const Batch& b, cudaStream_t st, LaunchProf* prof) {
   { ProfScope q(prof, st, KC_WIDE_SUBST); launch_front_back<double>(b, st); }
 }
 
-// The same with the FP32 factor, on r32.
+// The same with the FP32 factor, on r32; the solution stays in the fronts' order.
 void launch_front_solve32(const Batch& b, cudaStream_t st, LaunchProf* prof) {
   { ProfScope q(prof, st, KC_WIDE_DIAG); launch_front_assemble<float>(b, st); }
   { ProfScope q(prof, st, KC_WIDE_UPDATE); launch_front_factor<float>(b, st); }
@@ -1017,7 +1036,7 @@ void launch_front_resolve32(const Batch& b, cudaStream_t st) {
   }
   launch_front_back<float>(b, st);
 }
-int front_resolve_launches(const Batch& b) { return b.sh.mf.sched ? 2 * (int)b.sh.mf.sched->level.size() + 1 : 0; }
+int front_resolve_launches(const Batch& b) { return b.sh.mf.sched ? 2 * (int)b.sh.mf.sched->level.size() : 0; }
 
 void launch_front_csr(const Batch& b, int n, const int* rp, const int* ci, const double* v, cudaStream_t st) {
   launch_front_zero<double>(b, st);

@@ -1104,12 +1104,21 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       if (scolor[e] == c) scolor_elems.push_back(e);
   }
   sd.color_off[max_scolor] = (int)scolor_elems.size();
+  std::vector<int> nref_off(shell_off ? (size_t)b.n_nodes + 1 : 0, 0), nref((size_t)shell_off * 6);
+  if (shell_off) {
+    for (size_t q = 0; q < nref.size(); ++q) ++nref_off[snodes[q] + 1];
+    for (int i = 0; i < b.n_nodes; ++i) nref_off[i + 1] += nref_off[i];
+    std::vector<int> at(nref_off.begin(), nref_off.end() - 1);
+    for (int e : scolor_elems)
+      for (int a = 0; a < 6; ++a) nref[at[snodes[(size_t)6 * e + a]]++] = 8 * e + a;
+  }
   if (shell_off) {
     if (!upload(B, &sd.snodes, snodes) || !upload(B, &sd.sstruct, sstruct) || !upload(B, &sd.spress, spress) ||
         !upload(B, &sd.sarea, sarea) || !upload(B, &sd.sconst, sconst) || !upload(B, &sd.shist, shist) ||
         !upload(B, &sd.saux, saux) || !dup(B, &B->shist0, sd.shist, shist.size()) ||
         !dup(B, &B->saux0, sd.saux, saux.size()) ||
-        !upload(B, &sd.color_elems, scolor_elems) || !balloc(B, &sd.Ke, (size_t)shell_off * 729) ||
+        !upload(B, &sd.color_elems, scolor_elems) || !upload(B, &sd.nref_off, nref_off) ||
+        !upload(B, &sd.nref, nref) || !balloc(B, &sd.Ke, (size_t)shell_off * 729) ||
         !balloc(B, &sd.Fe, (size_t)shell_off * 27) ||
         (sd.any_rayleigh && !balloc(B, &sd.RD, (size_t)shell_off * 729)))
       return GF_ERR_CUDA;
@@ -1156,7 +1165,7 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       // the saved Newton right-hand side, the residual and the refinement state
       std::vector<int> slot(n, -1);
       for (size_t z = 0; z < wide_structs.size(); ++z) slot[wide_structs[z]] = (int)z;
-      if (!balloc(B, &sd.r32, (size_t)dof_off) || !balloc(B, &sd.ir_res, (size_t)dof_off) ||
+      if (!balloc(B, &sd.r32, (size_t)dof_off) || !balloc(B, &sd.ir_fe, (size_t)shell_off * 27) ||
           !balloc(B, &sd.ir_rhs, (size_t)dof_off) || !upload(B, &sd.wide_slot, slot) ||
           !zeroed(B, &sd.ir, wide_structs.size()) || !zeroed(B, &sd.ir_more, 4))
         return GF_ERR_CUDA;

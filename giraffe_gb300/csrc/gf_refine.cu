@@ -3,9 +3,9 @@
 // corrections stop shrinking, r = b - K x formed from the element matrices; a
 // solve that does not reach the FP64 level is done again in FP64.
 //
-// Bound by the latency of the sweep's launches (a height of the tree at a time
-// down and up, a colour of elements at a time): the 24x24x2 plate's step, 177 ms
-// with the FP32 wide-band LU and a residual from the FP64 band, 27 ms here.
+// Bound by the latency of the sweep's launches, a height of the tree at a time down
+// and up: the 24x24x2 plate's step, 177 ms with the FP32 wide-band LU and a residual
+// from the FP64 band, 10.5 ms here.
 #include <cuda_runtime.h>
 
 #include <cfloat>
@@ -48,31 +48,18 @@ __global__ void __launch_bounds__(256) k_ir_begin(Batch b) {
   }
 }
 
-// The residual's start, r = b (ir_rhs); a thread per DOF.
-__global__ void k_ir_rhs(Batch b) {
-  const int s = b.sh.wide_structs[blockIdx.y];
-  if (!wide_active(b, s) || b.sh.ir[blockIdx.y].done) return;
-  const StructInfo& inf = b.info[s];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < inf.n_free; i += gridDim.x * blockDim.x)
-    b.sh.ir_res[inf.dof_off + i] = b.sh.ir_rhs[inf.dof_off + i];
-}
-
-// r -= K_e x_e in FP64 from the element matrices, x in P, r in ir_res: a warp per
-// element of one colour (no two elements of a colour share a node), lane r < 27
-// row r of K_e x_e.
-__global__ void __launch_bounds__(128) k_ir_color(Batch b, int color) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  const int lo = b.sh.color_off[color], hi = b.sh.color_off[color + 1];
-  if (lo + w >= hi) return;
-  const int e = b.sh.color_elems[lo + w], s = b.sh.sstruct[e];
+// y_e = K_e x_e in FP64 into ir_fe, x in P: a warp per element, lane r < 27 row r.
+__global__ void __launch_bounds__(128) k_ir_elements(Batch b) {
+  const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (e >= b.sh.n_shells) return;
+  const int s = b.sh.sstruct[e];
   if (!wide_active(b, s) || b.sh.ir[b.sh.wide_slot[s]].done) return;
   const int off = b.info[s].dof_off;
   const int* nd = b.sh.snodes + 6 * e;
-  int g = -1;
   double x = 0.0;
   if (lane < 27) {
     const int node = lane < 18 ? nd[lane / 3] : nd[3 + (lane - 18) / 3];
-    g = b.gl[(int64_t)node * 6 + (lane < 18 ? lane % 3 : 3 + (lane - 18) % 3)];
+    const int g = b.gl[(int64_t)node * 6 + (lane < 18 ? lane % 3 : 3 + (lane - 18) % 3)];
     if (g >= 0) x = b.P[off + g];
   }
   const double* K = b.sh.Ke + (int64_t)e * 729 + lane;
@@ -84,19 +71,36 @@ __global__ void __launch_bounds__(128) k_ir_color(Batch b, int color) {
     y1 = fma(k1, __shfl_sync(0xffffffffu, x, q + 1), y1);
   }
   y0 = fma(lane < 27 ? K[27 * 26] : 0.0, __shfl_sync(0xffffffffu, x, 26), y0);
-  if (g >= 0) b.sh.ir_res[off + g] -= y0 + y1;
+  if (lane < 27) b.sh.ir_fe[(int64_t)e * 27 + lane] = y0 + y1;
 }
-// The nodal load stiffness' share, and r rounded into r32 for the FP32 solve; a
-// thread per DOF.
+
+// r = b - K x, b in ir_rhs: a thread per DOF takes its elements' y_e in colour order
+// and the nodal load stiffness' share; r rounded into r32 for the FP32 solve.  (A
+// launch per colour that subtracts in place, and one to start r, took 41 us a sweep on
+// the 24x24x2 plate.)
 __global__ void k_ir_round(Batch b) {
   const int s = b.sh.wide_structs[blockIdx.y];
   if (!wide_active(b, s) || b.sh.ir[blockIdx.y].done) return;
   const StructInfo& inf = b.info[s];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < inf.n_free; i += gridDim.x * blockDim.x) {
-    double r = b.sh.ir_res[inf.dof_off + i];
-    const int q = b.dof_node6[inf.dof_off + i], k = q % 6;
+    double r = b.sh.ir_rhs[inf.dof_off + i];
+    const int n6 = b.dof_node6[inf.dof_off + i], k = n6 % 6;
+    const int64_t node = n6 / 6;
+    const int o0 = b.sh.nref_off[node], o1 = b.sh.nref_off[node + 1];
+    for (int o = o0; o < o1; o += 4) {
+      double y[4];
+      bool in[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int t = o + q < o1 ? b.sh.nref[o + q] : 0, x = shell_dof(t & 7, k);
+        in[q] = o + q < o1 && x >= 0;
+        y[q] = in[q] ? b.sh.ir_fe[(int64_t)(t >> 3) * 27 + x] : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (in[q]) r -= y[q];
+    }
     if (inf.n_loads && k >= 3) {
-      const int64_t node = q / 6;
       for (int j = 0; j < 3; ++j) {
         const int gj = b.gl[node * 6 + 3 + j];
         if (gj >= 0) r -= b.nodeK[node * 9 + (k - 3) * 3 + j] * b.P[inf.dof_off + gj];
@@ -105,32 +109,35 @@ __global__ void k_ir_round(Batch b) {
     b.sh.r32[inf.dof_off + i] = __double2float_rn(r);
   }
 }
-__device__ __forceinline__ double warp_max(double v) {
+
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
 
-// x += d in FP64 (d: the FP32 correction the solve left in r32; first: x =
-// d, the first solve); the sweep's largest |d| and |x| raise the slot's
-// maxima (FP64 bits of non-negative values order like the values, so the
-// maxima do not depend on the CTAs' order).  A non-finite entry counts as
-// an infinite |d|.
+// x += d in FP64 (d: the FP32 correction, in the fronts' order; first: x = d, the
+// first solve); the sweep's largest |d| and |x| raise the slot's maxima (FP64 bits of
+// non-negative values order like the values, so the maxima do not depend on the
+// CTAs' order, and take no FP64 comparison).  A non-finite entry counts as an
+// infinite |d|.
 __global__ void __launch_bounds__(256) k_ir_correct(Batch b, int first) {
   const int z = blockIdx.y, s = b.sh.wide_structs[z];
   if (!wide_active(b, s) || b.sh.ir[z].done) return;
   const StructInfo& inf = b.info[s];
   double* x = b.P + inf.dof_off;
-  const float* d = b.sh.r32 + inf.dof_off;
-  double dm = 0.0, xm = 0.0;
+  const float* d = reinterpret_cast<const float*>(b.sh.mf.x);
+  const int* pos = b.sh.mf.pos + inf.dof_off;
+  unsigned long long dm = 0, xm = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < inf.n_free; i += gridDim.x * blockDim.x) {
-    const double di = (double)d[i], xi = first ? di : x[i] + di;
+    const double di = (double)d[pos[i]], xi = first ? di : x[i] + di;
     x[i] = xi;
-    if (!isfinite(xi)) dm = INFINITY;
-    dm = fmax(dm, fabs(di));
-    xm = fmax(xm, fabs(xi));
+    const unsigned long long db = (unsigned long long)__double_as_longlong(di) & 0x7fffffffffffffffull;
+    const unsigned long long xb = (unsigned long long)__double_as_longlong(xi) & 0x7fffffffffffffffull;
+    dm = max(dm, xb < 0x7ff0000000000000ull ? db : 0x7ff0000000000000ull);
+    xm = max(xm, xb);
   }
-  __shared__ double red[2][8];
+  __shared__ unsigned long long red[2][8];
   dm = warp_max(dm);
   xm = warp_max(xm);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -141,12 +148,12 @@ __global__ void __launch_bounds__(256) k_ir_correct(Batch b, int first) {
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int q = 1; q < (int)(blockDim.x >> 5); ++q) {
-      dm = fmax(dm, red[0][q]);
-      xm = fmax(xm, red[1][q]);
+      dm = max(dm, red[0][q]);
+      xm = max(xm, red[1][q]);
     }
     WideIr& q = b.sh.ir[z];
-    if (dm > 0.0) atomicMax(&q.dn, (unsigned long long)__double_as_longlong(dm));
-    if (xm > 0.0) atomicMax(&q.xn, (unsigned long long)__double_as_longlong(xm));
+    if (dm) atomicMax(&q.dn, dm);
+    if (xm) atomicMax(&q.xn, xm);
   }
 }
 
@@ -284,11 +291,7 @@ static void ir_sweep(const Batch& b, cudaStream_t st, cudaGraphConditionalHandle
   const dim3 dofs(2 * 152, sd.n_wide);
   {
     ProfScope q(prof, st, KC_WIDE_REFINE);
-    k_ir_rhs<<<dofs, 256, 0, st>>>(b);
-    for (int c = 0; c < sd.n_colors; ++c) {
-      const int cnt = sd.color_off[c + 1] - sd.color_off[c];
-      if (cnt > 0) k_ir_color<<<(cnt + 3) / 4, 128, 0, st>>>(b, c);
-    }
+    k_ir_elements<<<(sd.n_shells + 3) / 4, 128, 0, st>>>(b);
     k_ir_round<<<dofs, 256, 0, st>>>(b);
   }
   {
@@ -372,16 +375,14 @@ void launch_shell_solve(const Batch& b, cudaStream_t st, LaunchProf* prof) {
   else launch_front_solve(b, st, prof);
 }
 
-// Kernel launches per Newton pass; the mixed path adds its start, first
-// correction and check and the fallback's condition, and its sweeps and
+// Kernel launches per Newton pass; the mixed path adds its start, check and the
+// fallback's condition (its first correction takes the place of k_mf_out), and its sweeps and
 // fallbacks come on top (refine_launches).
-int shell_solve_launches(const Batch& b) { return front_launches(b) + (b.sh.n_wide && b.mixed ? 4 : 0); }
+int shell_solve_launches(const Batch& b) { return front_launches(b) + (b.sh.n_wide && b.mixed ? 3 : 0); }
 
 // Launches of `sweeps` refinement sweeps and `fallbacks` FP64 fallbacks.
 long long refine_launches(const Batch& b, long long sweeps, long long fallbacks) {
-  int colors = 0;
-  for (int c = 0; c < b.sh.n_colors; ++c) colors += b.sh.color_off[c + 1] > b.sh.color_off[c];
-  return sweeps * (4 + colors + front_resolve_launches(b)) + fallbacks * (1 + front_launches(b));
+  return sweeps * (4 + front_resolve_launches(b)) + fallbacks * (1 + front_launches(b));
 }
 
 }  // namespace gf

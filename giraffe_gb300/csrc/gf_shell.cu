@@ -1,7 +1,7 @@
 // Shell_1 structures on the device: element tangent and internal force with
 // the follower pressure and, in Dynamic steps, the inertial terms
 // (k_shell_mount, on the Gauss points of gf_shell_gp.cuh), Rayleigh damping
-// (k_shell_rayleigh), colour scatter of the forces (k_shell_scatter) and
+// (k_shell_rayleigh), the forces into P (k_shell_gather_f; k_shell_scatter with a band) and
 // SaveLagrange (k_shell_commit; reference src/Shell_1.cpp:1650-1664).  The LU of
 // the assembled operator is in gf_front.cu.
 #include <cuda_bf16.h>
@@ -522,7 +522,6 @@ __global__ void k_shell_scatter(Batch b, int color) {
   const double* K = b.sh.Ke + (int64_t)e * 729;
   const double* F = b.sh.Fe + (int64_t)e * 27;
   if (lane < 27 && myg >= 0) b.P[inf.dof_off + myg] += F[lane];
-  if (!wide_band_filled(b)) return;  // the multifrontal LU assembles K_AA itself
   double* band = b.sh.wband + inf.wb_off;
   const int kl = inf.wkl;
   const int64_t W = 2 * kl + 1;
@@ -534,6 +533,35 @@ __global__ void k_shell_scatter(Batch b, int color) {
     int gq = __shfl_sync(0xffffffffu, myg, q);
     if (valid && gr >= 0 && gq >= 0) band[(kl + gr - gq) + (int64_t)gq * W] += K[idx];
   }
+}
+
+// The forces alone, where K_AA is not asked for: a thread per node DOF adds its
+// elements' in colour order, so P has the colour scatter's bits in one launch (for 7
+// of 3.3 us on the 24x24x2 plate).
+__global__ void k_shell_gather_f(Batch b) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= (int64_t)b.n_nodes * 6) return;
+  const int g = b.gl[t], i = (int)(t / 6), k = (int)(t - (int64_t)i * 6);
+  const int o0 = b.sh.nref_off[i], o1 = b.sh.nref_off[i + 1];
+  if (g < 0 || o0 == o1) return;
+  const int s = b.node_struct[i];
+  if (!iterating_s(b.state[s])) return;
+  double* P = b.P + b.info[s].dof_off + g;
+  double v = *P;
+  for (int o = o0; o < o1; o += 4) {
+    double f[4];
+    bool in[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = o + q < o1 ? b.sh.nref[o + q] : 0, x = shell_dof(r & 7, k);
+      in[q] = o + q < o1 && x >= 0;
+      f[q] = in[q] ? b.sh.Fe[(int64_t)(r >> 3) * 27 + x] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (in[q]) v += f[q];
+  }
+  *P = v;
 }
 
 // SaveLagrange of Gauss point g at the converged increment d.
@@ -578,6 +606,10 @@ void launch_shell_mount(const Batch& b, cudaStream_t st) {
   if (b.sh.n_shells == 0) return;
   launch_mount(ShellBatchSrc{b}, b.sh.n_shells, st);
   if (b.sh.any_rayleigh) k_shell_rayleigh<<<(b.sh.n_shells + 3) / 4, 128, 0, st>>>(b);
+  if (!wide_band_filled(b)) {
+    k_shell_gather_f<<<(unsigned)(((int64_t)b.n_nodes * 6 + 255) / 256), 256, 0, st>>>(b);
+    return;
+  }
   for (int c = 0; c < b.sh.n_colors; ++c) {
     int cnt = b.sh.color_off[c + 1] - b.sh.color_off[c];
     if (cnt <= 0) continue;
@@ -651,7 +683,9 @@ int shell_launches_per_pass(const Batch& b) {
   int n = 0;
   if (b.sh.n_shells) {
     n += 2 + (b.sh.any_rayleigh ? 1 : 0);  // tangent (+ Rayleigh damping) + commit
-    for (int c = 0; c < b.sh.n_colors; ++c) n += b.sh.color_off[c + 1] > b.sh.color_off[c];
+    if (!wide_band_filled(b)) n += 1;
+    else
+      for (int c = 0; c < b.sh.n_colors; ++c) n += b.sh.color_off[c + 1] > b.sh.color_off[c];
   }
   return n + shell_solve_launches(b);
 }

@@ -305,16 +305,20 @@ struct ShellData {
   int* color_elems;
   int color_off[17];
   int n_colors;
+  // the elements on every node, in colour order: nref[nref_off[node] .. nref_off[node + 1])
+  // = 8 element + local node
+  int* nref_off;
+  int* nref;
   double* wband;
   // mixed precision (GF_PREC_MIXED): the LU is formed in FP32 and the solution
-  // refined in FP64: r32 the FP32 right-hand side and solution, ir_rhs the
-  // Newton right-hand side, ir_res the FP64 residual, ir the per-slot refinement
+  // refined in FP64: r32 the FP32 right-hand side, ir_rhs the Newton
+  // right-hand side, ir_fe the elements' K_e x_e [n_shells][27], ir the per-slot refinement
   // state, wide_slot the slot of each structure.  fp64_pass is set on the host's
   // copy of the batch for the FP64 fallback launches (only structures with ir_fb
   // run).
   float* r32;
   double* ir_rhs;
-  double* ir_res;
+  double* ir_fe;
   int* wide_slot;
   struct WideIr* ir;
   WideTiles tiles;   // tile shapes of this batch's wide-band LU
