@@ -193,13 +193,14 @@ template <typename T> __global__ void k_mf_out(Batch b) {
 }
 
 // Extend-add: eight columns of a large front with its children's Schur
-// complements, a warp per column, two children at a time (the small fronts gather
-// theirs as they load).
+// complements, a warp per column, two children and four rows a lane at a time (the
+// small fronts gather theirs as they load).  Bound by dependent loads from L2: front,
+// child, its index of the column, of the rows, the entries.
 template <typename T> __global__ void __launch_bounds__(256) k_mf_extend(Batch b, int job0) {
   const FrontData& d = b.sh.mf;
   const int2 job = d.ext_jobs[job0 + blockIdx.x];
   const Front F = d.fronts[job.x];
-  if (!mf_active(b, F.slot)) return;
+  const bool active = mf_active(b, F.slot);
   const int lane = threadIdx.x & 31, j = job.y + (threadIdx.x >> 5), kid1 = F.kid1;
   if (j > F.f) return;
   T* g = mf_mat<T>(b, F) + (int64_t)j * F.ld;
@@ -217,14 +218,27 @@ template <typename T> __global__ void __launch_bounds__(256) k_mf_extend(Batch b
       sc[q] = reinterpret_cast<const T*>(d.F) + C.off + C.s + (int64_t)(C.s + cj) * C.ld;
     }
     if (!on[0] && !on[1]) continue;
-#pragma unroll 4
-    for (int i = lane; i < F.f; i += 32) {
-      const int c0 = on[0] ? inv[0][i] : -1, c1 = on[1] ? inv[1][i] : -1;
-      if (c0 < 0 && c1 < 0) continue;
-      T v = g[i];
-      if (c0 >= 0) v += sc[0][c0];
-      if (c1 >= 0) v += sc[1][c1];
-      g[i] = v;
+    for (int i0 = lane; i0 < F.f; i0 += 128) {
+      int c[2][4];
+      T v[4], a[2][4];
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const int i = i0 + 32 * y;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) c[q][y] = on[q] && i < F.f ? inv[q][i] : -1;
+        v[y] = i < F.f ? g[i] : T(0);
+      }
+      if (!active) return;
+#pragma unroll
+      for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) a[q][y] = c[q][y] >= 0 ? sc[q][c[q][y]] : T(0);
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        if (c[0][y] >= 0) v[y] += a[0][y];
+        if (c[1][y] >= 0) v[y] += a[1][y];
+        if (c[0][y] >= 0 || c[1][y] >= 0) g[i0 + 32 * y] = v[y];
+      }
     }
   }
 }
@@ -246,7 +260,15 @@ template <typename T> __global__ void __launch_bounds__(MF_SMALL_THREADS) k_mf_s
   const int f = F.f, s = F.s, ld = F.ld, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr int WARPS = MF_SMALL_THREADS / 32;
   T* G = mf_mat<T>(b, F);
-  for (int x = tid; x < ld * (f + 1); x += MF_SMALL_THREADS) A[x] = G[x];
+  const int size = ld * (f + 1);
+  for (int x0 = tid; x0 < size; x0 += 8 * MF_SMALL_THREADS) {
+    T v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = x0 + q * MF_SMALL_THREADS < size ? G[x0 + q * MF_SMALL_THREADS] : T(0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (x0 + q * MF_SMALL_THREADS < size) A[x0 + q * MF_SMALL_THREADS] = v[q];
+  }
   for (int k = F.kid0; k < F.kid1; ++k) {
     const int2 kid = d.kids[k];
     const int* inv = d.inv + kid.y;
@@ -256,14 +278,24 @@ template <typename T> __global__ void __launch_bounds__(MF_SMALL_THREADS) k_mf_s
     int ci[MF_SMALL / 32];
 #pragma unroll
     for (int q = 0; q < MF_SMALL / 32; ++q) ci[q] = lane + 32 * q < f ? inv[lane + 32 * q] : -1;
+    // the child's column of each of the warp's columns, one a lane
+    const int jl = warp + WARPS * lane, cjl = jl < f ? inv[jl] : jl == f ? u : -1;
     __syncthreads();  // A is complete, or holds the child before
-#pragma unroll 2
-    for (int j = warp; j <= f; j += WARPS) {
-      const int cj = j < f ? inv[j] : u;
-      if (cj < 0) continue;
+    for (int y0 = 0; warp + WARPS * y0 <= f; y0 += 4) {
+      T a[4][MF_SMALL / 32];
+      int cj[4];
 #pragma unroll
-      for (int q = 0; q < MF_SMALL / 32; ++q)
-        if (ci[q] >= 0) A[lane + 32 * q + j * ld] += S[ci[q] + (int64_t)cj * cld];
+      for (int y = 0; y < 4; ++y) {
+        cj[y] = __shfl_sync(0xffffffffu, cjl, y0 + y);
+#pragma unroll
+        for (int q = 0; q < MF_SMALL / 32; ++q)
+          a[y][q] = cj[y] >= 0 && ci[q] >= 0 ? S[ci[q] + (int64_t)cj[y] * cld] : T(0);
+      }
+#pragma unroll
+      for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int q = 0; q < MF_SMALL / 32; ++q)
+          if (cj[y] >= 0 && ci[q] >= 0) A[lane + 32 * q + (warp + WARPS * (y0 + y)) * ld] += a[y][q];
     }
   }
   __syncthreads();
@@ -388,12 +420,12 @@ template <typename T, int L> __global__ void __launch_bounds__(128) k_mf_trsm(Ba
   if (first >= (lower ? F.f : F.f + 1)) return;
   T* G = mf_mat<T>(b, F);
   __shared__ T U[MF_NB][MF_NB + 1];  // U[k][j]: the factor this side reads, identity beyond nb
-  for (int x = tid; x < MF_NB * MF_NB; x += 128) {
-    const int i = x % MF_NB, j = x / MF_NB;
-    T v = i == j ? T(1) : T(0);
-    if (i < nb && j < nb && (lower ? i <= j : i > j)) v = G[k0 + i + (int64_t)(k0 + j) * ld];
-    if (lower) U[i][j] = v;  // U11(i, j), the reciprocal on the diagonal
-    else U[j][i] = v;        // L11(i, j) at [j][i]
+  T u[MF_NB / 4];
+#pragma unroll
+  for (int y = 0; y < MF_NB / 4; ++y) {
+    const int i = tid % MF_NB, j = tid / MF_NB + 4 * y;
+    u[y] = i == j ? T(1) : T(0);
+    if (i < nb && j < nb && (lower ? i <= j : i > j)) u[y] = G[k0 + i + (int64_t)(k0 + j) * ld];
   }
   const int r = tid / L, q = tid % L, g = first + r;  // row (lower) or column of the front
   const bool live = g < (lower ? F.f : F.f + 1);
@@ -403,11 +435,17 @@ template <typename T, int L> __global__ void __launch_bounds__(128) k_mf_trsm(Ba
     const int c = L * j + q;
     v[j] = (live && c < nb) ? (lower ? G[g + (int64_t)(k0 + c) * ld] : G[k0 + c + (int64_t)g * ld]) : T(0);
   }
+#pragma unroll
+  for (int y = 0; y < MF_NB / 4; ++y) {
+    const int i = tid % MF_NB, j = tid / MF_NB + 4 * y;
+    if (lower) U[i][j] = u[y];  // U11(i, j), the reciprocal on the diagonal
+    else U[j][i] = u[y];        // L11(i, j) at [j][i]
+  }
   if (!on) return;
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < MF_NB; ++k) {
-    if (k >= nb) break;
+    if (k % 8 == 0 && k >= nb) break;  // the factor is the identity beyond nb
     // the finished entry k, from the lane that holds it
     T x = v[k / L];
     if (lower) x *= U[k][k];
