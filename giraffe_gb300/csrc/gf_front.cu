@@ -465,15 +465,18 @@ template <typename T, int L> __global__ void __launch_bounds__(128) k_mf_trsm(Ba
 }
 
 // The pivot rows and columns right of and below panel p: rows k1..s-1 of all
-// later columns (blockIdx.x < na) and the boundary rows of the later pivot
+// later columns (the first na tiles) and the boundary rows of the later pivot
 // columns, minus L U over the panel's pivots.  16 x 32 tiles, so that the few
 // tiles of the top fronts spread over the SMs (a tile holds an SM's FP64 units
-// for 512 warp instructions, about 5 us).  The first CTA of a front takes the 32 x 32
-// tile of the next diagonal block and factors it (mf_block_lu) while the others run:
-// a launch per panel and 14 us less on the chain of panels.
+// for 512 warp instructions, about 5 us).  The first C CTAs of a front, a cluster, take
+// the 32 x 32 tile of the next diagonal block, 32 / C columns each, and the first of
+// them factors it (mf_block_lu) while the others run: a launch per panel and 14 us less
+// on the chain of panels.  On one CTA the tile takes 8 us of its SM's FP64 rate, all of
+// them on the chain where a height has few fronts (24 us a panel with one, 17 with
+// four).
 constexpr int MF_PANEL_THREADS = 256;
 static_assert(MF_PANEL_THREADS == MF_DIAG_THREADS, "the panel's first CTA factors a block");
-template <typename T>
+template <typename T, int C>
 __global__ void __launch_bounds__(MF_PANEL_THREADS) k_mf_panel(Batch b, int off, int p, int na, int nca, int ncb) {
   const FrontData& d = b.sh.mf;
   const Front F = d.list[off + blockIdx.y];
@@ -483,50 +486,63 @@ __global__ void __launch_bounds__(MF_PANEL_THREADS) k_mf_panel(Batch b, int off,
   T* G = mf_mat<T>(b, F);
   __shared__ T Ls[MF_NB][33];  // [k][row]
   __shared__ T Us[32][MF_NB + 1];  // [column][k]
-  if (blockIdx.x == 0) {
+  if (blockIdx.x < C) {
+    constexpr int Q = 4 / C;
+    __shared__ T Ds[MF_NB][MF_NB + 1];  // the diagonal block (the first CTA's)
+    cg::cluster_group cl = cg::this_cluster();
     const int lane = tid & 31, warp = tid >> 5, r1 = F.s, c1 = F.f + 1, nb = min(MF_NB, F.s - k1);
-    T acc[4];
+    const int y0 = warp + 8 * Q * (int)blockIdx.x;  // this warp's columns y0 + 8 q
+    T acc[Q];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int y = warp + 8 * q;  // pivot of L, column of U and of the tile
-      Ls[y][lane] = k1 + lane < r1 ? G[k1 + lane + (int64_t)(k0 + y) * ld] : T(0);
+      const int k = warp + 8 * q;
+      Ls[k][lane] = k1 + lane < r1 ? G[k1 + lane + (int64_t)(k0 + k) * ld] : T(0);
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int y = y0 + 8 * q;
       Us[y][lane] = k1 + y < c1 ? G[k0 + lane + (int64_t)(k1 + y) * ld] : T(0);
       acc[q] = (k1 + lane < r1 && k1 + y < c1) ? G[k1 + lane + (int64_t)(k1 + y) * ld] : T(0);
     }
     if (!on) return;
+    if (C > 1) cl.barrier_arrive();
     __syncthreads();
 #pragma unroll 8
     for (int k = 0; k < MF_NB; ++k) {
       const T l = -Ls[k][lane];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] = mfma(l, Us[warp + 8 * q][k], acc[q]);
+      for (int q = 0; q < Q; ++q) acc[q] = mfma(l, Us[y0 + 8 * q][k], acc[q]);
     }
-    __syncthreads();
+    if (C > 1) cl.barrier_wait();  // every CTA of the cluster runs
+    T* D0 = C > 1 ? cl.map_shared_rank(&Ds[0][0], 0) : &Ds[0][0];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int y = warp + 8 * q;
-      if (y < nb) Ls[y][lane] = acc[q];  // the diagonal block, column y
+    for (int q = 0; q < Q; ++q) {
+      const int y = y0 + 8 * q;
+      if (y < nb) D0[y * (MF_NB + 1) + lane] = acc[q];
       else if (lane < nb && k1 + y < c1) G[k1 + lane + (int64_t)(k1 + y) * ld] = acc[q];
     }
-    __syncthreads();
-    const bool bad = mf_block_lu<T>(Ls, nb, warp, lane);
+    if (C > 1) cl.sync();
+    else __syncthreads();
+    if (blockIdx.x > 0) return;
+    const bool bad = mf_block_lu<T>(Ds, nb, warp, lane);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int y = warp + 8 * q;
-      if (lane < nb && y < nb) G[k1 + lane + (int64_t)(k1 + y) * ld] = Ls[y][lane];
+      if (lane < nb && y < nb) G[k1 + lane + (int64_t)(k1 + y) * ld] = Ds[y][lane];
     }
     if (bad && lane == 0) mf_fail<T>(b, F.slot);
     return;
   }
+  const int tile = (int)blockIdx.x - C;
   int r0, c0, r1, c1;
-  if ((int)blockIdx.x < na) {
-    r0 = k1 + 16 * ((int)blockIdx.x / nca);
-    c0 = k1 + 32 * ((int)blockIdx.x % nca);
+  if (tile < na) {
+    r0 = k1 + 16 * (tile / nca);
+    c0 = k1 + 32 * (tile % nca);
     r1 = F.s;
     c1 = F.f + 1;
-    if (r0 == k1 + 16 && c0 == k1) return;  // the first CTA's other half
+    if (r0 <= k1 + 16 && c0 == k1) return;  // the first CTAs'
   } else {
-    const int x = (int)blockIdx.x - na;
+    const int x = tile - na;
     r0 = F.s + 16 * (x / ncb);
     c0 = k1 + 32 * (x % ncb);
     r1 = F.f;
@@ -953,6 +969,24 @@ template <typename T> void mf_attrs() {
   (void)done;
 }
 
+// A launch in clusters of C CTAs along x.
+template <typename... P, typename... A>
+void launch_clusters(void (*kernel)(P...), dim3 grid, int threads, int C, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 int dof_blocks(const Batch& b) { return std::max(1, std::min(152, (b.n_free + 255) / 256)); }
 }  // namespace
 
@@ -1005,7 +1039,11 @@ template <typename T> void launch_front_factor(const Batch& b, cudaStream_t st) 
       if (s > k1) {
         const int nca = (f + 1 - k1 + 31) / 32, na = (s - k1 + 15) / 16 * nca;
         const int ncb = (s - k1 + 31) / 32, nb = (f + 15) / 16 * ncb;
-        k_mf_panel<T><<<dim3(na + nb, n), MF_PANEL_THREADS, 0, st>>>(b, V.big_off, (int)p, na, nca, ncb);
+        if (sizeof(T) == 8 && 4 * n <= 152)
+          launch_clusters(k_mf_panel<T, 4>, dim3((na + nb + 4 + 3) / 4 * 4, n), MF_PANEL_THREADS, 4, 0, st, b, V.big_off,
+                          (int)p, na, nca, ncb);
+        else
+          k_mf_panel<T, 1><<<dim3(na + nb + 1, n), MF_PANEL_THREADS, 0, st>>>(b, V.big_off, (int)p, na, nca, ncb);
       }
     }
     if constexpr (sizeof(T) == 8) launch_front_t5(b, V, st);
@@ -1025,21 +1063,6 @@ int subst_ctas(int n, int rows) {
   while (C < 8 && 2 * C * n <= 152 && C * 32 < rows) C *= 2;
   return C;
 }
-template <typename K> void launch_subst(K kernel, const Batch& b, int off, int n, int C, size_t smem, cudaStream_t st) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(n * C);
-  cfg.blockDim = dim3(MF_BACK_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = C;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, b, off, C);
-}
 }  // namespace
 
 template <typename T> void launch_front_back(const Batch& b, cudaStream_t st) {
@@ -1048,7 +1071,7 @@ template <typename T> void launch_front_back(const Batch& b, cudaStream_t st) {
     const FrontLevel& V = sc.level[l];
     const int n = V.n_small + V.n_big, C = subst_ctas(n, V.max_s), f = std::max(V.small_f, V.big_f);
     const size_t w = (size_t)f + 2 + 8 * (size_t)std::min(((V.max_s + 31) / 32 + C - 1) / C * 32, MF_PART);
-    launch_subst(k_mf_back<T>, b, V.small_off, n, C, w * sizeof(T), st);
+    launch_clusters(k_mf_back<T>, dim3(n * C), MF_BACK_THREADS, C, w * sizeof(T), st, b, V.small_off, C);
   }
   if constexpr (sizeof(T) == 8) k_mf_out<T><<<dim3(dof_blocks(b), b.sh.n_wide), 256, 0, st>>>(b);
 }
@@ -1070,7 +1093,8 @@ void launch_front_solve32(const Batch& b, cudaStream_t st, LaunchProf* prof) {
 void launch_front_resolve32(const Batch& b, cudaStream_t st) {
   for (const FrontLevel& V : b.sh.mf.sched->level) {
     const int n = V.n_small + V.n_big, f = std::max(V.small_f, V.big_f);
-    launch_subst(k_mf_fwd<float>, b, V.small_off, n, subst_ctas(n, f), (size_t)f * sizeof(float), st);
+    const int C = subst_ctas(n, f);
+    launch_clusters(k_mf_fwd<float>, dim3(n * C), MF_BACK_THREADS, C, (size_t)f * sizeof(float), st, b, V.small_off, C);
   }
   launch_front_back<float>(b, st);
 }
