@@ -91,25 +91,55 @@ __device__ __forceinline__ int64_t mf_entry(const FrontData& d, int pr, int pc) 
 
 }  // namespace
 
-// Destinations of the element matrices' entries, once per batch.
+// Destinations of the element matrices' entries and the chains of entries that share
+// one, in colour order, once per batch: a thread per pair of an element's nodes.  The
+// elements with both nodes are among the first one's (nref).
 __global__ void k_mf_map(Batch b) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= (int64_t)b.sh.n_shells * 729) return;
-  const int e = (int)(t / 729), x = (int)(t % 729), r = x % 27, q = x / 27;
-  const int s = b.sh.sstruct[e];
+  if (t >= (int64_t)b.sh.n_shells * 36) return;
+  const int e = (int)(t / 36), la = (int)(t % 36) / 6, lb = (int)(t % 6), s = b.sh.sstruct[e];
   const StructInfo& inf = b.info[s];
-  const int* nd = b.sh.snodes + 6 * e;
-  auto dof = [&](int a) {
-    const int node = a < 18 ? nd[a / 3] : nd[3 + (a - 18) / 3];
-    return b.gl[(int64_t)node * 6 + (a < 18 ? a % 3 : 3 + (a - 18) % 3)];
-  };
-  const int gr = dof(r), gq = dof(q);
-  int to = -1;
-  if (gr >= 0 && gq >= 0) {
-    const FrontData& d = b.sh.mf;
-    to = (int)(mf_entry(d, d.pos[inf.dof_off + gr], d.pos[inf.dof_off + gq]) - d.base[s]);
-  }
-  b.sh.mf.map[t] = to;
+  const FrontData& d = b.sh.mf;
+  const int na = b.sh.snodes[6 * (int64_t)e + la], nb = b.sh.snodes[6 * (int64_t)e + lb];
+  const int o0 = b.sh.nref_off[na], o1 = b.sh.nref_off[na + 1];
+  // translations or rotations of either node
+  for (int ka = 0; ka < (la < 3 ? 1 : 2); ++ka)
+    for (int kb = 0; kb < (lb < 3 ? 1 : 2); ++kb) {
+      bool first = true, past = false;
+      int ne = -1, xa = 0, xb = 0;  // the next element and its rows of the first DOFs
+      for (int o = o0; o < o1 && ne < 0; ++o) {
+        const int v = b.sh.nref[o];
+        if (v == 8 * e + la) {
+          past = true;
+          continue;
+        }
+        const int ra = shell_dof(v & 7, 3 * ka);
+        if (ra < 0) continue;
+        for (int m = 0; m < 6; ++m) {
+          if (b.sh.snodes[6 * (int64_t)(v >> 3) + m] != nb) continue;
+          const int rb = shell_dof(m, 3 * kb);
+          if (rb < 0) continue;
+          if (!past) first = false;
+          else {
+            ne = v >> 3;
+            xa = ra;
+            xb = rb;
+          }
+          break;
+        }
+      }
+      for (int ca = 0; ca < 3; ++ca)
+        for (int cb = 0; cb < 3; ++cb) {
+          const int x = shell_dof(la, 3 * ka + ca) + 27 * shell_dof(lb, 3 * kb + cb);
+          const int gr = b.gl[(int64_t)na * 6 + 3 * ka + ca], gq = b.gl[(int64_t)nb * 6 + 3 * kb + cb];
+          int2 to = make_int2(-1, 0);
+          if (gr >= 0 && gq >= 0) {
+            if (first) to.x = (int)(mf_entry(d, d.pos[inf.dof_off + gr], d.pos[inf.dof_off + gq]) - d.base[s]);
+            if (ne >= 0) to.y = (ne - e) * 729 + xa + ca + 27 * (xb + cb) - x;
+          }
+          d.map[(int64_t)e * 729 + x] = to;
+        }
+    }
 }
 
 // Clears the fronts of the structures that solve.
@@ -123,33 +153,58 @@ template <typename T> __global__ void k_mf_zero(Batch b) {
     p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// MountGlobal into the fronts: a warp per element of one colour (no two
-// elements of a colour share a node, so no two writers meet).
-template <typename T> __global__ void k_mf_elements(Batch b, int color) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  const int lo = b.sh.color_off[color], hi = b.sh.color_off[color + 1];
-  if (lo + w >= hi) return;
-  const int e = b.sh.color_elems[lo + w], s = b.sh.sstruct[e];
-  if (!mf_active(b, s)) return;
+// MountGlobal into the fronts: a warp per element; the first entry of a destination
+// takes the others' along its chain (at most as long as the elements on a node), so an
+// entry of the fronts is written once, with the bits of one colour of elements after the
+// other.  Bound by the chains' loads, twelve entries in flight a lane; a launch per
+// colour that adds in place took 5.6 us for each of 7 on small meshes, 13 on the 64x64x2
+// plate.
+template <typename T> __global__ void __launch_bounds__(128) k_mf_elements(Batch b) {
+  const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (e >= b.sh.n_shells) return;
+  const int s = b.sh.sstruct[e];
+  const bool active = mf_active(b, s);
   const double* K = b.sh.Ke + (int64_t)e * 729;
-  const int* map = b.sh.mf.map + (int64_t)e * 729;
+  const int2* map = b.sh.mf.map + (int64_t)e * 729;
   T* F = reinterpret_cast<T*>(b.sh.mf.F) + b.sh.mf.base[s];
-  // twelve entries in flight a lane (one at a time: 17 us a colour for 6)
 #pragma unroll 1
   for (int x0 = lane; x0 < 729; x0 += 12 * 32) {
-    int to[12];
-    T k[12], f[12];
+    int2 m[12];
+    int at[12];
+    T v[12];
 #pragma unroll
     for (int q = 0; q < 12; ++q) {
-      const int x = x0 + 32 * q;
-      to[q] = x < 729 ? map[x] : -1;
-      k[q] = x < 729 ? (T)K[x] : T(0);
+      at[q] = x0 + 32 * q;
+      m[q] = at[q] < 729 ? map[at[q]] : make_int2(-1, 0);
+      v[q] = at[q] < 729 ? (T)K[at[q]] : T(0);
+    }
+    if (!active) return;
+    bool more = false;
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {
+      if (m[q].x < 0) m[q].y = 0;
+      more = more || m[q].y != 0;
+    }
+    while (more) {
+      T k[12];
+      int next[12];
+#pragma unroll
+      for (int q = 0; q < 12; ++q) {
+        at[q] += m[q].y;
+        k[q] = m[q].y ? (T)K[at[q]] : T(0);
+        next[q] = m[q].y ? map[at[q]].y : 0;
+      }
+      more = false;
+#pragma unroll
+      for (int q = 0; q < 12; ++q) {
+        if (m[q].y) v[q] += k[q];
+        m[q].y = next[q];
+        more = more || next[q] != 0;
+      }
     }
 #pragma unroll
-    for (int q = 0; q < 12; ++q) f[q] = to[q] >= 0 ? F[to[q]] : T(0);
-#pragma unroll
     for (int q = 0; q < 12; ++q)
-      if (to[q] >= 0) F[to[q]] = f[q] + k[q];
+      if (m[q].x >= 0) F[m[q].x] = v[q];
   }
 }
 
@@ -991,7 +1046,7 @@ int dof_blocks(const Batch& b) { return std::max(1, std::min(152, (b.n_free + 25
 }  // namespace
 
 void launch_front_map(const Batch& b, cudaStream_t st) {
-  const int64_t n = (int64_t)b.sh.n_shells * 729;
+  const int64_t n = (int64_t)b.sh.n_shells * 36;
   if (n) k_mf_map<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(b);
 }
 
@@ -1002,10 +1057,7 @@ template <typename T> void launch_front_zero(const Batch& b, cudaStream_t st) {
 // K_AA of the wide structures from the element matrices and nodal loads.
 template <typename T> void launch_front_assemble(const Batch& b, cudaStream_t st) {
   launch_front_zero<T>(b, st);
-  for (int c = 0; c < b.sh.n_colors; ++c) {
-    const int cnt = b.sh.color_off[c + 1] - b.sh.color_off[c];
-    if (cnt > 0) k_mf_elements<T><<<(cnt + 3) / 4, 128, 0, st>>>(b, c);
-  }
+  if (b.sh.n_shells) k_mf_elements<T><<<(b.sh.n_shells + 3) / 4, 128, 0, st>>>(b);
   if (b.n_loads) k_mf_nodes<T><<<(b.n_nodes + 127) / 128, 128, 0, st>>>(b);
 }
 
@@ -1118,9 +1170,7 @@ void launch_front_band(const Batch& b, int n, int kl, int ku, int ldab, const do
 // Launches of one assembly, factorization and solve of the batch.
 int front_launches(const Batch& b) {
   if (!b.sh.n_wide || !b.sh.mf.sched) return 0;
-  int n = b.sh.mf.sched->launches + (b.n_loads ? 1 : 0);
-  for (int c = 0; c < b.sh.n_colors; ++c) n += b.sh.color_off[c + 1] > b.sh.color_off[c];
-  return n;
+  return b.sh.mf.sched->launches + (b.n_loads ? 1 : 0) + (b.sh.n_shells ? 1 : 0);
 }
 
 }  // namespace gf

@@ -87,7 +87,10 @@ struct FrontData {
   int* dof_at;      // elimination position -> free DOF (batch-wide)
   int* pos;         // free DOF (batch-wide) -> elimination position (batch-wide)
   int* dof_front;   // elimination position -> its front
-  int* map;         // [n_shells][729] destination of K_e entries in F, relative to the structure's first front (-1: none)
+  // [n_shells][729] per K_e entry: x, its destination in F relative to the structure's first
+  // front (-1: none, or an earlier element's entry takes the sum); y, the distance in K_e
+  // entries to the next one of the same destination (0: the last)
+  int2* map;
   int64_t* base;    // per structure: offset of its fronts in F
   int64_t* size;    // per structure: doubles of its fronts
   FrontT5* t5;      // by height
