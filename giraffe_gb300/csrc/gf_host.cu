@@ -1072,6 +1072,8 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
   b.n_nodes = node_off;
   b.n_elem = elem_off;
   b.n_free = dof_off;
+  b.n_band = 0;
+  for (const StructInfo& q : B->info) b.n_band += !q.is_chain && !q.wide;
   b.n_loads = (int)loads.size();
   b.n_pipe_press = (int)pp_elem.size();
   b.mon_total = (int)mon_node.size();
@@ -1249,8 +1251,8 @@ int count_launches_per_pass(const gf_batch* B) {
   const ChainParts &cs = B->b.chain_sym, &cg = B->b.chain_gen;
   // chains only: one gather launch in place of the colour passes
   if (B->b.n_elem && !B->b.full_band && cs.n_elem + cg.n_elem == B->b.n_elem) colors = 1;
-  // step_begin, step_nodes, zero, tangent, residual, band solve, update, control, commits
-  return 10 + (B->b.n_loads ? 1 : 0) + (B->b.any_dynamic ? 1 : 0) + colors + chain_launches(cs) + chain_launches(cg) + shell_launches_per_pass(B->b) + (B->b.any_rayleigh ? 1 : 0) +
+  // step_begin, step_nodes, zero, tangent, residual, update, control, commit
+  return 8 + (B->b.n_band ? 1 : 0) + (B->b.n_loads ? 1 : 0) + (B->b.any_dynamic ? 1 : 0) + colors + chain_launches(cs) + chain_launches(cg) + shell_launches_per_pass(B->b) + (B->b.any_rayleigh ? 1 : 0) +
          (B->b.n_pipe_press ? 1 : 0) + (B->b.mon_total ? 1 : 0);
 }
 

@@ -1305,8 +1305,8 @@ __global__ void k_control(Batch b) {
 }
 
 // SaveConfiguration: element Gauss-point history, a thread per Gauss point ...
-__global__ void k_commit_elems(Batch b) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, e = t >> 1;
+__device__ __forceinline__ void commit_elem(const Batch& b, int t) {
+  const int e = t >> 1;
   if (e >= b.n_elem) return;
   int s = b.estruct[e];
   if (!b.state[s].commit) return;
@@ -1319,8 +1319,7 @@ __global__ void k_commit_elems(Batch b) {
 }
 
 // ... and nodal configuration (reference src/Node.cpp:325-370)
-__global__ void k_commit_nodes(Batch b) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void commit_node(const Batch& b, int i) {
   if (i >= b.n_nodes) return;
   int s = b.node_struct[i];
   if (!b.state[s].commit) return;
@@ -1339,6 +1338,13 @@ __global__ void k_commit_nodes(Batch b) {
       b.copy_vel[(int64_t)i * 6 + k] = b.vel[(int64_t)i * 6 + k];
       b.copy_accel[(int64_t)i * 6 + k] = b.accel[(int64_t)i * 6 + k];
     }
+}
+
+// Both, the nodes in the first node_ctas CTAs: neither reads what the other writes, and
+// most passes commit nothing (a launch of 2.4 us a pass less).
+__global__ void __launch_bounds__(128) k_commit(Batch b, int node_ctas) {
+  if ((int)blockIdx.x < node_ctas) commit_node(b, blockIdx.x * blockDim.x + threadIdx.x);
+  else commit_elem(b, (blockIdx.x - node_ctas) * blockDim.x + threadIdx.x);
 }
 
 // Monitor line of one monitored node (Node::WriteMonitor, reference
@@ -1565,10 +1571,14 @@ void launch_increment(const Batch& b, cudaStream_t st) {
   if (b.any_dynamic) k_update_dyn<<<(b.n_nodes + 127) / 128, 128, 0, st>>>(b);
 }
 
+static void launch_commit_nodes(const Batch& b, cudaStream_t st) {
+  const int nodes = (b.n_nodes + 127) / 128, elems = (b.n_elem + 63) / 64;
+  if (nodes + elems) k_commit<<<nodes + elems, 128, 0, st>>>(b, nodes);
+}
+
 void launch_commit(const Batch& b, cudaStream_t st) {
-  if (b.n_elem) k_commit_elems<<<(b.n_elem + 63) / 64, 128, 0, st>>>(b);
   if (b.sh.n_shells) launch_shell_commit(b, st);
-  if (b.n_nodes) k_commit_nodes<<<(b.n_nodes + 127) / 128, 128, 0, st>>>(b);
+  launch_commit_nodes(b, st);
 }
 
 // Shared-memory limits of the large kernels, once per process (the served
@@ -1645,16 +1655,15 @@ void launch_iteration(const Batch& b, cudaStream_t st, bool commit_kernels, Laun
   if (b.sh.n_shells) { ProfScope q(prof, st, KC_SHELL); launch_shell_mount(b, st); }
   { ProfScope q(prof, st, KC_LOADS); launch_loads(b, st); }
   { ProfScope q(prof, st, KC_RESIDUAL); k_residual<<<b.n_chunks, 256, 0, st>>>(b); }
-  { ProfScope q(prof, st, KC_SOLVE); launch_band_solve(b, st); }
+  if (b.n_band) { ProfScope q(prof, st, KC_SOLVE); launch_band_solve(b, st); }
   if (b.chain_gen.n_elem) { ProfScope q(prof, st, KC_CHAIN); launch_gen_chains(b, b.chain_gen, st); }
   if (b.chain_sym.n_elem) { ProfScope q(prof, st, KC_CHAIN); launch_sym_chains(b, b.chain_sym, st); }
   launch_shell_solve(b, st, prof);
   { ProfScope q(prof, st, KC_UPDATE); launch_increment(b, st); }
   { ProfScope q(prof, st, KC_CONTROL); k_control<<<(ns + 127) / 128, 128, 0, st>>>(b); }
   if (commit_kernels) {
-    if (b.n_elem) { ProfScope q(prof, st, KC_COMMIT_ELEMS); k_commit_elems<<<(b.n_elem + 63) / 64, 128, 0, st>>>(b); }
     if (b.sh.n_shells) { ProfScope q(prof, st, KC_COMMIT_ELEMS); launch_shell_commit(b, st); }
-    if (b.n_nodes) { ProfScope q(prof, st, KC_COMMIT_NODES); k_commit_nodes<<<(b.n_nodes + 127) / 128, 128, 0, st>>>(b); }
+    { ProfScope q(prof, st, KC_COMMIT_NODES); launch_commit_nodes(b, st); }
     if (b.mon_total) k_monitor_record<<<(b.mon_total + 127) / 128, 128, 0, st>>>(b);
   }
 }

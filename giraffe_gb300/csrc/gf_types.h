@@ -361,6 +361,7 @@ struct ShellData {
 struct Batch {
   int n_struct, n_nodes, n_elem, n_free;
   int n_loads, n_disps, n_tables;
+  int n_band;  // structures that the band LU solves (neither a chain nor with shells)
   // nodes
   double* disp;
   double* copy;
