@@ -1341,7 +1341,7 @@ __device__ __forceinline__ void commit_node(const Batch& b, int i) {
 }
 
 // Both, the nodes in the first node_ctas CTAs: neither reads what the other writes, and
-// most passes commit nothing (a launch of 2.4 us a pass less).
+// most passes commit nothing (a launch less: 1.3 us of the roll-up's 93 us a pass).
 __global__ void __launch_bounds__(128) k_commit(Batch b, int node_ctas) {
   if ((int)blockIdx.x < node_ctas) commit_node(b, blockIdx.x * blockDim.x + threadIdx.x);
   else commit_elem(b, (blockIdx.x - node_ctas) * blockDim.x + threadIdx.x);
