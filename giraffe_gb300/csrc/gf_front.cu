@@ -158,7 +158,7 @@ template <typename T> __global__ void k_mf_zero(Batch b) {
 // entry of the fronts is written once, with the bits of one colour of elements after the
 // other.  Bound by the chains' loads, twelve entries in flight a lane; a launch per
 // colour that adds in place took 5.6 us for each of 7 on small meshes, 13 on the 64x64x2
-// plate.
+// plate; this 11 and 45 in all.
 template <typename T> __global__ void __launch_bounds__(128) k_mf_elements(Batch b) {
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (e >= b.sh.n_shells) return;
@@ -1108,8 +1108,9 @@ template <typename T> void launch_front_factor(const Batch& b, cudaStream_t st) 
 }
 
 namespace {
-// CTAs of a front in the substitutions: as many as leave an SM one, up to a group of
-// 32 rows each.
+// CTAs of a front in the substitutions: as many as leave an SM one, up to eight and a
+// group of 32 rows each (the 24x24x2 mixed plate's step with at most two 10.9 ms, four
+// 10.3, eight 10.3; the 64x64x2 plate's with one 33.0, eight 31.4).
 int subst_ctas(int n, int rows) {
   int C = 1;
   while (C < 8 && 2 * C * n <= 152 && C * 32 < rows) C *= 2;
