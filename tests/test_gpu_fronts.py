@@ -283,3 +283,39 @@ def test_substitution_does_not_depend_on_the_batch(gpu_ctx, n, copies, mixed):
         b.close()
     for q in range(copies):
         assert np.array_equal(out[0][0][0], out[1][0][q]) and np.array_equal(out[0][1][0], out[1][1][q])
+
+
+def junction():
+    """A plate of 2x2 squares and one of half its size beside it: a midside node of the
+    coarse one's edge is a corner of the fine one's elements."""
+    a, b = configs.square_plate(2, steps=2, pressure=1e3), configs.square_plate(2, side=0.5, steps=2)
+    xy = [tuple(p) for p in a.nodes]
+    new = []
+    for p in b.nodes + [1.0, 0.0, 0.0]:
+        if p[1] in (0.0, 0.25, 0.5) and p[0] == 1.0:
+            new.append(xy.index(tuple(p)))
+        else:
+            new.append(len(xy))
+            xy.append(tuple(p))
+    a.nodes = np.array(xy)
+    a.shells.extend([tuple(new[q] for q in row[:6]) + tuple(row[6:]) for row in b.shells])
+    a.constraints = np.zeros((len(xy), 6), dtype=np.int32)
+    a.constraints[(a.nodes[:, 0] == 0.0) | (a.nodes[:, 0] == 1.5) | (a.nodes[:, 1] == 0.0)] = 1
+    a.loads[0].shells = list(range(len(a.shells)))
+    return a
+
+
+@pytest.mark.parametrize("precision", [gpu.GF_PREC_FP64, gpu.GF_PREC_MIXED])
+def test_a_node_that_is_corner_and_midside(gpu_ctx, precision):
+    # forces and matrices are gathered per node: a node with rotations in some of its
+    # elements only
+    fo, so, _ = oracle.solve(junction(), 0)
+    b = gpu.BatchSolver(gpu_ctx, [junction()], gpu_ctx.opts(precision=precision))
+    b.reset()
+    b.run()
+    finals, stats = b.results()
+    b.close()
+    assert tuple(stats[0]) == tuple(so)
+    scale = np.abs(fo[:, :3]).max()
+    assert np.abs(finals[0][:, :3] - fo[:, :3]).max() <= 1e-10 * scale
+    assert np.abs(finals[0][:, 6:] - fo[:, 6:]).max() <= 1e-9
