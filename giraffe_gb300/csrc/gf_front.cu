@@ -1008,6 +1008,62 @@ __global__ void k_mf_band(Batch b, int n, int kl, int ku, int ldab, const double
   d.F[mf_entry(d, d.pos[i], d.pos[j])] = ab[kl + ku + i - j + (int64_t)j * ldab];
 }
 
+// r = rhs - A x and whether a row's backward error is above the limit; a non-finite
+// one is.  mx: the largest |x_j| of the row's columns as its bits.
+__device__ __forceinline__ void mf_judge(int i, double rhs, double ax, double sum, unsigned long long mx, double* r, int* bad) {
+  const double res = rhs - ax, d = fma(sum, __longlong_as_double((long long)mx), fabs(rhs));
+  r[i] = res;
+  if (!(fabs(res) <= MF_ERROR_LIMIT * d && d <= DBL_MAX)) *bad = 1;
+}
+__device__ __forceinline__ unsigned long long mf_mag(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+}
+
+// Eight lanes a row of a CSR matrix.
+__global__ void __launch_bounds__(128) k_csr_residual(int n, const int* rp, const int* ci, const double* v, const double* rhs,
+                                                      const double* x, double* r, int* bad) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, lane = threadIdx.x & 7;
+  double ax = 0.0, sum = 0.0;
+  unsigned long long mx = 0;
+  const int k1 = i < n ? rp[i + 1] : 0;
+  for (int k = i < n ? rp[i] + lane : 0; k < k1; k += 8) {
+    const double a = v[k], xk = x[ci[k]];
+    ax = fma(a, xk, ax);
+    sum += fabs(a);
+    mx = max(mx, mf_mag(xk));
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    ax += __shfl_xor_sync(0xffffffffu, ax, o);
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    mx = max(mx, (unsigned long long)__shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  if (i < n && lane == 0) mf_judge(i, rhs[i], ax, sum, mx, r, bad);
+}
+
+// A thread a row of LAPACK GB columns.
+__global__ void __launch_bounds__(64) k_band_residual(int n, int kl, int ku, int ldab, const double* ab, const double* rhs,
+                                                      const double* x, double* r, int* bad) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double ax = 0.0, sum = 0.0;
+  unsigned long long mx = 0;
+  const int j1 = min(n - 1, i + ku);
+#pragma unroll 4
+  for (int j = max(0, i - kl); j <= j1; ++j) {
+    const double a = ab[kl + ku + i - j + (int64_t)j * ldab], xj = x[j];
+    ax = fma(a, xj, ax);
+    sum += fabs(a);
+    mx = max(mx, mf_mag(xj));
+  }
+  mf_judge(i, rhs[i], ax, sum, mx, r, bad);
+}
+
+__global__ void k_mf_add(int n, const double* d, double* x) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) x[i] += d[i];
+}
+
 // ---------------------------------------------------------------------------
 namespace {
 constexpr int ZERO_CTAS = 8 * 152;
@@ -1142,30 +1198,51 @@ void launch_front_solve32(const Batch& b, cudaStream_t st, LaunchProf* prof) {
   { ProfScope q(prof, st, KC_WIDE_UPDATE); launch_front_factor<float>(b, st); }
   { ProfScope q(prof, st, KC_WIDE_SUBST); launch_front_back<float>(b, st); }
 }
-// Another right-hand side (r32) with the FP32 factor.
-void launch_front_resolve32(const Batch& b, cudaStream_t st) {
+// Another right-hand side (P or r32) with the factor that the fronts hold.
+template <typename T> void launch_front_resolve(const Batch& b, cudaStream_t st) {
   for (const FrontLevel& V : b.sh.mf.sched->level) {
     const int n = V.n_small + V.n_big, f = std::max(V.small_f, V.big_f);
     const int C = subst_ctas(n, f);
-    launch_clusters(k_mf_fwd<float>, dim3(n * C), MF_BACK_THREADS, C, (size_t)f * sizeof(float), st, b, V.small_off, C);
+    launch_clusters(k_mf_fwd<T>, dim3(n * C), MF_BACK_THREADS, C, (size_t)f * sizeof(T), st, b, V.small_off, C);
   }
-  launch_front_back<float>(b, st);
+  launch_front_back<T>(b, st);
 }
+void launch_front_resolve32(const Batch& b, cudaStream_t st) { launch_front_resolve<float>(b, st); }
 int front_resolve_launches(const Batch& b) { return b.sh.mf.sched ? 2 * (int)b.sh.mf.sched->level.size() : 0; }
 
 void launch_front_csr(const Batch& b, int n, const int* rp, const int* ci, const double* v, cudaStream_t st) {
   launch_front_zero<double>(b, st);
   k_mf_csr<<<(n + 127) / 128, 128, 0, st>>>(b, n, rp, ci, v);
-  launch_front_factor<double>(b, st);
-  launch_front_back<double>(b, st);
 }
 
 void launch_front_band(const Batch& b, int n, int kl, int ku, int ldab, const double* ab, cudaStream_t st) {
   launch_front_zero<double>(b, st);
   const int64_t t = (int64_t)n * (kl + ku + 1);
   k_mf_band<<<(unsigned)((t + 255) / 256), 256, 0, st>>>(b, n, kl, ku, ldab, ab);
+}
+
+void launch_front_lu(const Batch& b, double* x, cudaStream_t st) {
   launch_front_factor<double>(b, st);
-  launch_front_back<double>(b, st);
+  Batch out = b;
+  out.P = x;
+  launch_front_back<double>(out, st);
+}
+
+void launch_front_refine(const Batch& b, int n, double* r, double* x, cudaStream_t st) {
+  Batch rb = b;
+  rb.P = r;
+  launch_front_resolve<double>(rb, st);
+  k_mf_add<<<(n + 255) / 256, 256, 0, st>>>(n, r, x);
+}
+
+void launch_csr_residual(int n, const int* rp, const int* ci, const double* v, const double* rhs, const double* x,
+                         double* r, int* bad, cudaStream_t st) {
+  k_csr_residual<<<(n + 15) / 16, 128, 0, st>>>(n, rp, ci, v, rhs, x, r, bad);
+}
+
+void launch_band_residual(int n, int kl, int ku, int ldab, const double* ab, const double* rhs, const double* x, double* r,
+                          int* bad, cudaStream_t st) {
+  k_band_residual<<<(n + 63) / 64, 64, 0, st>>>(n, kl, ku, ldab, ab, rhs, x, r, bad);
 }
 
 // Launches of one assembly, factorization and solve of the batch.

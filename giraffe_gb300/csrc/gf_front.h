@@ -45,6 +45,11 @@ constexpr int MF_NB = 32;  // pivots per panel of a large front
 // Below, the tiles are too few and the slicing's launches (15 us a height) too dear.
 // A rule on the front alone, so a structure is eliminated the same way in any batch.
 constexpr double MF_T5_WORK = 1.5e6;
+// Largest backward error of a row of a standalone system, in units of sum_j |a_ij| max_j
+// |x_j| + |b_i| (j over the row's entries): sixteen roundings.  Dominant matrices, mesh
+// and beam tangents reach 1 to 8 of them in either order, a tridiagonal system with a
+// diagonal entry of 1e-3 that the dissection puts first 130, one of 1e-6 350,000.
+constexpr double MF_ERROR_LIMIT = 0x1p-49;
 // Such a front: its slices, exponents (per 128 pivots) and pivot maxima.
 struct FrontT5 {
   int64_t slices;  // L21's at oz[slices], U12's behind: [64 pivots][slice][rows][64]

@@ -25,8 +25,12 @@ struct FrontSystem {
   std::vector<Part> parts;
   size_t sent = 0, total = 0;
   char* dev = nullptr;
-  gf::StructState state{};
+  struct {
+    gf::StructState st;
+    int bad;  // the solution's backward error passes the limit
+  } state{};
   gf::StructInfo info{};
+  double *xs = nullptr, *r = nullptr;  // solution and residual (device)
   int zero = 0;
   int p_state = 0, p_rhs = 0;
 
@@ -45,13 +49,13 @@ struct FrontSystem {
     join_fronts({&plan}, {0}, {0}, 1, n, ctx->wide_update == GF_WIDE_TENSOR, fb);
     info.n_free = n;
     info.wide = 1;
-    state.phase = gf::PH_ITER;
-    state.need_solve = 1;
+    state.st.phase = gf::PH_ITER;
+    state.st.need_solve = 1;
     auto vec = [&](const auto& v) { return send(v.data(), v.size() * sizeof(v[0])); };
     const int p_fr = vec(fb.fronts), p_bnd = vec(fb.bnd), p_kids = vec(fb.kids),
               p_inv = vec(fb.inv), p_list = vec(fb.list),
               p_ext = vec(fb.ext_jobs), p_sch = vec(fb.schur_jobs), p_t5 = vec(fb.t5), p_t5j = vec(fb.t5_jobs), p_pos = vec(fb.pos), p_df = vec(fb.dof_front),
-              p_base = vec(fb.base), p_size = vec(fb.size);
+              p_base = vec(fb.base), p_size = vec(fb.size), p_da = vec(fb.dof_at);
     const int p_info = send(&info, sizeof(info)), p_ws = send(&zero, sizeof(int));
     p_state = send(&state, sizeof(state));
     p_rhs = send(rhs, sizeof(double) * (size_t)n);
@@ -60,7 +64,8 @@ struct FrontSystem {
     const size_t off_F = sent, off_x = after(off_F, (size_t)fb.total * sizeof(double));
     const size_t off_oz = after(off_x, sizeof(double) * (size_t)n), off_km = after(off_oz, (size_t)fb.oz * 2);
     const size_t off_ex = after(off_km, (size_t)fb.oz_kmax * sizeof(unsigned long long));
-    total = off_ex + (size_t)fb.oz_exp * sizeof(int);
+    const size_t off_xs = after(off_ex, (size_t)fb.oz_exp * sizeof(int)), off_r = after(off_xs, sizeof(double) * (size_t)n);
+    total = off_r + sizeof(double) * (size_t)n;
     dev = static_cast<char*>(ctx->device_work(total));
     char* pin = static_cast<char*>(ctx->pinned(sent));
     if (!dev || !pin) {
@@ -96,21 +101,45 @@ struct FrontSystem {
     d.oz = reinterpret_cast<__nv_bfloat16*>(dev + off_oz);
     d.oz_kmax = reinterpret_cast<unsigned long long*>(dev + off_km);
     d.oz_exp = reinterpret_cast<int*>(dev + off_ex);
+    d.dof_at = at<int>(p_da);
     d.sched = &fb.sched;
+    xs = reinterpret_cast<double*>(dev + off_xs);
+    r = reinterpret_cast<double*>(dev + off_r);
     return GF_OK;
   }
 
-  // The solution into x and the pivot status, after the solve's launches.
-  int finish(gf_ctx* ctx, int n, double* x, int* fail) {
-    GF_CK(cudaGetLastError());
-    char* pin = static_cast<char*>(ctx->pin);  // the staging is free again once the solve has run
+  // Factorization and solution: assemble(b) puts the matrix into the fronts, check(x,
+  // r, bad) forms r = rhs - A x and sets *bad where a row's backward error passes
+  // MF_ERROR_LIMIT.  No elimination pivots, so an order of its own can meet pivots that
+  // the caller's does not: small ones lose digits without failing.  A solution above the
+  // limit is refined with the factor (r as the right-hand side) up to twice; one that is
+  // still above it, or a failed pivot, leaves *done false and x as it was, and the caller
+  // solves in the natural order.
+  template <typename Assemble, typename Check>
+  int solve(gf_ctx* ctx, int n, Assemble assemble, Check check, double* x, bool* done) {
+    cudaStream_t st = ctx->stream;
+    int* bad = reinterpret_cast<int*>(b.state + 1);
     const size_t xb = sizeof(double) * (size_t)n;
-    GF_CK(cudaMemcpyAsync(pin + parts[p_rhs].off, b.P, xb, cudaMemcpyDeviceToHost, ctx->stream));
-    GF_CK(cudaMemcpyAsync(pin + parts[p_state].off, b.state, sizeof(state), cudaMemcpyDeviceToHost, ctx->stream));
-    GF_CK(cudaStreamSynchronize(ctx->stream));
-    std::memcpy(x, pin + parts[p_rhs].off, xb);
-    std::memcpy(&state, pin + parts[p_state].off, sizeof(state));
-    *fail = state.info_fail;
+    char* pin = static_cast<char*>(ctx->pin);  // the staging is free again once the factorization has run
+    assemble(b);
+    gf::launch_front_lu(b, xs, st);
+    *done = false;
+    for (int sweep = 0;; ++sweep) {
+      check(xs, r, bad);
+      GF_CK(cudaGetLastError());
+      GF_CK(cudaMemcpyAsync(pin + parts[p_rhs].off, xs, xb, cudaMemcpyDeviceToHost, st));
+      GF_CK(cudaMemcpyAsync(pin + parts[p_state].off, b.state, sizeof(state), cudaMemcpyDeviceToHost, st));
+      GF_CK(cudaStreamSynchronize(st));
+      std::memcpy(&state, pin + parts[p_state].off, sizeof(state));
+      if (state.st.info_fail || !state.bad) {
+        *done = !state.st.info_fail;
+        break;
+      }
+      if (sweep == 2) break;
+      GF_CK(cudaMemsetAsync(bad, 0, sizeof(int), st));
+      gf::launch_front_refine(b, n, r, xs, st);
+    }
+    if (*done) std::memcpy(x, pin + parts[p_rhs].off, xb);
     ctx->trim_work();
     return GF_OK;
   }

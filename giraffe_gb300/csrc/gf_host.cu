@@ -2216,7 +2216,12 @@ int gf_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab
     set_err(ctx, "gf_band_solve: invalid arguments");
     return GF_ERR_ARG;
   }
-  if (band_takes_fronts(n, kl, ku)) return front_band_solve(ctx, n, kl, ku, ab, ldab, b, info);
+  if (band_takes_fronts(n, kl, ku)) {
+    bool done = false;
+    const int rc = front_band_solve(ctx, n, kl, ku, ab, ldab, b, &done);
+    if (rc == GF_OK && done && info) *info = 0;
+    if (rc != GF_OK || done) return rc;
+  }
   if (kl > GF_KB || ku > GF_KB) return wide_band_solve(ctx, n, kl, ku, ab, ldab, b, info);
   int npad = (n + 31) / 32 * 32;
   std::vector<double> band((size_t)npad * GF_LDB, 0.0);

@@ -117,13 +117,22 @@ void launch_wide_solve(const Batch& b, cudaStream_t st, LaunchProf* prof = nullp
 void launch_wide_subst(const Batch& b, int nrhs, cudaStream_t st);
 // Multifrontal LU (gf_front.cu): destinations of the element entries (once per
 // batch); assembly of K_AA, factorization and solution of P of the batch's
-// Shell_1 structures; the same on a one-structure batch from a CSR or LAPACK GB
-// matrix on the device; kernel launches of one solve.
+// Shell_1 structures; kernel launches of one solve.
 void launch_front_map(const Batch& b, cudaStream_t st);
 void launch_front_solve(const Batch& b, cudaStream_t st, LaunchProf* prof = nullptr);
+int front_launches(const Batch& b);
+// Standalone systems (a one-structure batch): a CSR or LAPACK GB matrix on the device into
+// the fronts, their LU and the solution x of P, a refinement step x += A^-1 r with that LU
+// (r overwritten); the residual r = rhs - A x, *bad set where a row's backward error passes
+// MF_ERROR_LIMIT.
 void launch_front_csr(const Batch& b, int n, const int* rp, const int* ci, const double* v, cudaStream_t st);
 void launch_front_band(const Batch& b, int n, int kl, int ku, int ldab, const double* ab, cudaStream_t st);
-int front_launches(const Batch& b);
+void launch_front_lu(const Batch& b, double* x, cudaStream_t st);
+void launch_front_refine(const Batch& b, int n, double* r, double* x, cudaStream_t st);
+void launch_csr_residual(int n, const int* rp, const int* ci, const double* v, const double* rhs, const double* x,
+                         double* r, int* bad, cudaStream_t st);
+void launch_band_residual(int n, int kl, int ku, int ldab, const double* ab, const double* rhs, const double* x, double* r,
+                          int* bad, cudaStream_t st);
 // The Schur complements of a height's fronts on the tensor cores (gf_front_t5.cu).
 void launch_front_t5(const Batch& b, const FrontLevel& V, cudaStream_t st);
 // FP32: the same on r32, and another right-hand side with that factor.

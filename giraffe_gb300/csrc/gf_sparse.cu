@@ -148,7 +148,8 @@ bool band_takes_fronts(int n, int kl, int ku) {
   return t_front < t_band;
 }
 
-int front_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, int* info) {
+int front_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, bool* done) {
+  *done = false;
   // blocks of at least the half-bandwidth: their graph is a path
   const int B = std::max(std::max(kl, ku), 12), nb = (n + B - 1) / B, W = kl + ku + 1;
   NdGraph g;
@@ -166,18 +167,17 @@ int front_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int l
   }
   for (int i = 0; i < n; ++i) dofs[i] = i;
   const FrontPlan plan = plan_fronts(g, dptr, dofs);
+  if (!fronts_fit(plan)) return GF_OK;
   std::vector<double> packed((size_t)n * W);
   for (int j = 0; j < n; ++j)
     std::memcpy(&packed[(size_t)j * W], ab + (size_t)j * ldab + kl, sizeof(double) * (size_t)W);
   FrontSystem S;
   std::vector<int> part;
-  int rc = S.init(ctx, plan, n, b, {{packed.data(), sizeof(double) * packed.size()}}, &part);
-  if (rc != GF_OK) return rc;
-  launch_front_band(S.b, n, kl, ku, W, S.at<double>(part[0]) - kl, ctx->stream);
-  int fail = 0;
-  rc = S.finish(ctx, n, b, &fail);
-  if (rc == GF_OK && info) *info = fail;
-  return rc;
+  if (S.init(ctx, plan, n, b, {{packed.data(), sizeof(double) * packed.size()}}, &part) != GF_OK) return GF_OK;
+  const double* A = S.at<double>(part[0]) - kl;
+  return S.solve(ctx, n, [&](const Batch& q) { launch_front_band(q, n, kl, ku, W, A, ctx->stream); },
+                 [&](const double* x, double* r, int* bad) { launch_band_residual(n, kl, ku, W, A, S.b.P, x, r, bad, ctx->stream); },
+                 b, done);
 }
 
 // Wide branch of gf_band_solve: the GB array goes into the wide band with
@@ -256,20 +256,25 @@ int gf_sparse_solve(gf_ctx* ctx, int n, const int* row_ptr, const int* col_idx, 
     if (fronts_fit(plan)) {
       FrontSystem S;
       std::vector<int> part;
-      int rc = S.init(ctx, plan, n, b,
-                      {{row_ptr, sizeof(int) * ((size_t)n + 1)}, {col_idx, sizeof(int) * (size_t)nnz},
-                       {val, sizeof(double) * (size_t)nnz}}, &part);
-      if (rc != GF_OK) return rc;
-      launch_front_csr(S.b, n, S.at<int>(part[0]), S.at<int>(part[1]), S.at<double>(part[2]), ctx->stream);
-      int fail = 0;
-      rc = S.finish(ctx, n, b, &fail);
-      if (rc == GF_OK && info) *info = fail;
-      return rc;
+      if (S.init(ctx, plan, n, b,
+                 {{row_ptr, sizeof(int) * ((size_t)n + 1)}, {col_idx, sizeof(int) * (size_t)nnz},
+                  {val, sizeof(double) * (size_t)nnz}}, &part) == GF_OK) {
+        const int *rp = S.at<int>(part[0]), *ci = S.at<int>(part[1]);
+        const double* v = S.at<double>(part[2]);
+        bool done = false;
+        const int rc = S.solve(ctx, n, [&](const Batch& q) { launch_front_csr(q, n, rp, ci, v, ctx->stream); },
+                               [&](const double* x, double* r, int* bad) {
+                                 launch_csr_residual(n, rp, ci, v, S.b.P, x, r, bad, ctx->stream);
+                               },
+                               b, &done);
+        if (rc == GF_OK && done && info) *info = 0;
+        if (rc != GF_OK || done) return rc;
+      }
     }
   }
-  // a system whose fronts exceed the multifrontal kernels' limits, or a narrow
-  // band: ordering natural, or reverse Cuthill-McKee on the symmetrised
-  // pattern when that narrows the band
+  // a system that the multifrontal LU does not take or not solve to the accuracy that it
+  // asks of it, or a narrow band: ordering natural, or reverse Cuthill-McKee on the
+  // symmetrised pattern when that narrows the band
   std::vector<int> perm(n);
   for (int i = 0; i < n; ++i) perm[i] = i;
   int w = csr_bandwidth(n, row_ptr, col_idx, perm.data());

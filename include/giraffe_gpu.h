@@ -264,8 +264,12 @@ int gf_shell_inertia_elements(gf_ctx* ctx, int n, const double* xyz, const doubl
  * 2*kl+ku+1), without pivoting, FP64: by a multifrontal LU under a
  * nested-dissection ordering where that is the faster way, else by the 35-row
  * band solver (kl, ku <= 17) or the blocked wide-band LU with half-bandwidth
- * max(kl, ku).  b is overwritten by x.  *info receives 0 or 1 (zero or
- * non-finite pivot), as bandsystem's info_fail. */
+ * max(kl, ku).  The dissection's solution is returned where every row's residual is
+ * within 2^-49 (sum_j |a_ij| max_j |x_j| + |b_i|), if need be after up to two steps of
+ * refinement with its factor; otherwise, or where one of its pivots fails, the natural
+ * order's, so a matrix that the natural order solves is solved.  b is overwritten by x.
+ * *info receives 0 or 1 (zero or non-finite pivot in the natural order), as
+ * bandsystem's info_fail. */
 int gf_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, int* info);
 
 /* Replaces sparsesystem (src/SparseMatrix.cpp:74-166, the Newton step's
@@ -273,9 +277,10 @@ int gf_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab
  * row-major CSR, 0-based (row_ptr[n+1], col_idx[nnz], val[nnz]; entries
  * repeated within a row are summed).  A natural half-bandwidth up to 17 is
  * solved as gf_band_solve does; any other pattern by a no-pivot multifrontal LU
- * under a nested dissection of the symmetrised pattern (where its fronts do not
- * fit, by the blocked wide-band LU in reverse Cuthill-McKee order), FP64.  b (n) is overwritten by x.  *info
- * receives 0 or 1 (zero or non-finite pivot), as sparsesystem's info_fail;
+ * under a nested dissection of the symmetrised pattern.  Where its fronts do not fit
+ * or its solution is not within gf_band_solve's limit, the blocked wide-band LU takes the
+ * narrower of the natural and the reverse Cuthill-McKee order.  FP64.  b (n) is
+ * overwritten by x.  *info receives 0 or 1 (zero or non-finite pivot), as sparsesystem's info_fail;
  * the return value reports argument and CUDA errors. */
 int gf_sparse_solve(gf_ctx* ctx, int n, const int* row_ptr, const int* col_idx, const double* val, double* b,
                     int* info);
