@@ -1130,28 +1130,31 @@ template <typename T> void launch_front_factor(const Batch& b, cudaStream_t st) 
       k_mf_small<T><<<V.n_small, MF_SMALL_THREADS, (size_t)((V.small_f + 1) & ~1) * (V.small_f + 1) * sizeof(T), st>>>(
           b, V.small_off);
     for (size_t p = 0; p < V.n_at.size(); ++p) {
-      const int n = V.n_at[p], k0 = (int)p * MF_NB, k1 = k0 + MF_NB, f = V.f_at[p], s = V.s_at[p];
-      if (p == 0) k_mf_diag<T><<<n, MF_DIAG_THREADS, 0, st>>>(b, V.big_off);
-      // the panels of fronts whose last panel this is end before k1
-      const int m = f - k0 - 1;
-      if (m >= 0) {
-        // sixteen lanes a row while that leaves an SM at most one CTA
-        if ((2 * m + 1) * n <= 8 * 152) {
-          const int nlow = (m + 7) / 8, nup = (m + 1 + 7) / 8;
-          k_mf_trsm<T, 16><<<dim3(nlow + nup, n), 128, 0, st>>>(b, V.big_off, (int)p, nlow);
-        } else {
-          const int nlow = (m + 31) / 32, nup = (m + 1 + 31) / 32;
-          k_mf_trsm<T, 4><<<dim3(nlow + nup, n), 128, 0, st>>>(b, V.big_off, (int)p, nlow);
+      if (p == 0) k_mf_diag<T><<<V.n_at[p], MF_DIAG_THREADS, 0, st>>>(b, V.big_off);
+      for (int q = 0; q < front_grids(V.n_at[p]); ++q) {
+        const int n = std::min(V.n_at[p] - q * MF_GRID_FRONTS, MF_GRID_FRONTS), off = V.big_off + q * MF_GRID_FRONTS;
+        const int k0 = (int)p * MF_NB, k1 = k0 + MF_NB, f = V.f_at[p], s = V.s_at[p];
+        // the panels of fronts whose last panel this is end before k1
+        const int m = f - k0 - 1;
+        if (m >= 0) {
+          // sixteen lanes a row while that leaves an SM at most one CTA
+          if ((2 * m + 1) * (int64_t)n <= 8 * 152) {
+            const int nlow = (m + 7) / 8, nup = (m + 1 + 7) / 8;
+            k_mf_trsm<T, 16><<<dim3(nlow + nup, n), 128, 0, st>>>(b, off, (int)p, nlow);
+          } else {
+            const int nlow = (m + 31) / 32, nup = (m + 1 + 31) / 32;
+            k_mf_trsm<T, 4><<<dim3(nlow + nup, n), 128, 0, st>>>(b, off, (int)p, nlow);
+          }
         }
-      }
-      if (s > k1) {
-        const int nca = (f + 1 - k1 + 31) / 32, na = (s - k1 + 15) / 16 * nca;
-        const int ncb = (s - k1 + 31) / 32, nb = (f + 15) / 16 * ncb;
-        if (sizeof(T) == 8 && 4 * n <= 152)
-          launch_clusters(k_mf_panel<T, 4>, dim3((na + nb + 4 + 3) / 4 * 4, n), MF_PANEL_THREADS, 4, 0, st, b, V.big_off,
-                          (int)p, na, nca, ncb);
-        else
-          k_mf_panel<T, 1><<<dim3(na + nb + 1, n), MF_PANEL_THREADS, 0, st>>>(b, V.big_off, (int)p, na, nca, ncb);
+        if (s > k1) {
+          const int nca = (f + 1 - k1 + 31) / 32, na = (s - k1 + 15) / 16 * nca;
+          const int ncb = (s - k1 + 31) / 32, nb = (f + 15) / 16 * ncb;
+          if (sizeof(T) == 8 && 4 * n <= 152)
+            launch_clusters(k_mf_panel<T, 4>, dim3((na + nb + 4 + 3) / 4 * 4, n), MF_PANEL_THREADS, 4, 0, st, b, off,
+                            (int)p, na, nca, ncb);
+          else
+            k_mf_panel<T, 1><<<dim3(na + nb + 1, n), MF_PANEL_THREADS, 0, st>>>(b, off, (int)p, na, nca, ncb);
+        }
       }
     }
     if constexpr (sizeof(T) == 8) launch_front_t5(b, V, st);

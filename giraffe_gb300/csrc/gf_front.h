@@ -38,6 +38,10 @@ struct Front {
 // in its shared memory (k_mf_small); the others run panel by panel on many.
 constexpr int MF_SMALL = 96;
 constexpr int MF_NB = 32;  // pivots per panel of a large front
+// Large fronts of a height that one launch takes where they are its grid's y or z (which
+// end at 65,535): more of them, as a band of 200,000 blocks has, take several.
+constexpr int MF_GRID_FRONTS = 65535;
+inline int front_grids(int n) { return (n + MF_GRID_FRONTS - 1) / MF_GRID_FRONTS; }
 
 // Large fronts whose Schur complement takes this many multiply-adds run it on the
 // tensor cores (gf_front_t5.cu) where the caller lets them (GF_WIDE_TENSOR, the

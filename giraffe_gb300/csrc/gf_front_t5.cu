@@ -354,8 +354,11 @@ void launch_front_t5(const Batch& b, const FrontLevel& V, cudaStream_t st) {
     return true;
   }();
   (void)done;
-  k_mf_kmax<<<dim3((V.t5_s + 7) / 8, 2, V.t5_cnt), 256, 0, st>>>(b, V.t5_off);
-  k_mf_slice<<<dim3(V.t5_rows / SL_ROWS, 2 * ((V.t5_s + T5_CHUNK - 1) / T5_CHUNK), V.t5_cnt), 256, 0, st>>>(b, V.t5_off);
+  for (int q = 0; q < front_grids(V.t5_cnt); ++q) {
+    const int n = min(V.t5_cnt - q * MF_GRID_FRONTS, MF_GRID_FRONTS), off = V.t5_off + q * MF_GRID_FRONTS;
+    k_mf_kmax<<<dim3((V.t5_s + 7) / 8, 2, n), 256, 0, st>>>(b, off);
+    k_mf_slice<<<dim3(V.t5_rows / SL_ROWS, 2 * ((V.t5_s + T5_CHUNK - 1) / T5_CHUNK), n), 256, 0, st>>>(b, off);
+  }
   k_mf_t5<<<min(V.t5_job_cnt, 152), T5_THREADS, MF_T5_SMEM, st>>>(b, V.t5_job_off, V.t5_job_cnt);
 }
 

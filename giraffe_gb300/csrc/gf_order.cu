@@ -448,9 +448,11 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
     out.oz_kmax = std::max(out.oz_kmax, kmax);
     V.t5_cnt = (int)out.t5.size() - V.t5_off;
     V.t5_job_cnt = (int)out.t5_jobs.size() - V.t5_job_off;
-    out.sched.launches += (V.ext_cnt ? 1 : 0) + (V.n_small ? 1 : 0) + (V.schur_cnt ? 1 : 0) + (V.t5_cnt ? 3 : 0) + 1;
+    out.sched.launches += (V.ext_cnt ? 1 : 0) + (V.n_small ? 1 : 0) + (V.schur_cnt ? 1 : 0) +
+                          (V.t5_cnt ? 1 + 2 * gf::front_grids(V.t5_cnt) : 0) + 1;
     for (int p = 0; p < panels; ++p)
-      out.sched.launches += (p == 0 ? 1 : 0) + (V.f_at[p] > p * gf::MF_NB ? 1 : 0) + (V.s_at[p] > (p + 1) * gf::MF_NB ? 1 : 0);
+      out.sched.launches += (p == 0 ? 1 : 0) + gf::front_grids(V.n_at[p]) * ((V.f_at[p] > p * gf::MF_NB ? 1 : 0) +
+                                                                           (V.s_at[p] > (p + 1) * gf::MF_NB ? 1 : 0));
   }
 }
 

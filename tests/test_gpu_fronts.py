@@ -319,3 +319,16 @@ def test_a_node_that_is_corner_and_midside(gpu_ctx, precision):
     scale = np.abs(fo[:, :3]).max()
     assert np.abs(finals[0][:, :3] - fo[:, :3]).max() <= 1e-10 * scale
     assert np.abs(finals[0][:, 6:] - fo[:, 6:]).max() <= 1e-9
+
+
+def test_more_fronts_of_a_height_than_a_grid_has_rows(gpu_ctx):
+    # a band of 200,000 blocks of 33: 65,535 fronts of 99 rows and more at the lowest
+    # heights, beyond the y of a grid; unit sums, so x is a sum of the row's terms exactly
+    n, kl = 33 * 200000, 33
+    ab = np.zeros((n, 2 * kl + 1))
+    ab[:, kl] = 2.0
+    ab[:, 2 * kl] = -0.5
+    b = np.full(n, 1.5)
+    b[:kl] = 2.0
+    x, info = gpu_ctx.band_solve(ab, kl, 0, b)
+    assert info == 0 and np.array_equal(x, np.ones(n))
