@@ -14,6 +14,7 @@
 
 #include "gf_chain.cuh"
 #include "gf_chain_root.cuh"
+#include "gf_kernels.cuh"
 #include "gf_math.cuh"
 
 namespace gf {
@@ -486,11 +487,8 @@ void launch_gen_chains(const Batch& b, const ChainParts& c, cudaStream_t st) {
     if (hi <= c.merge_soa) k_gen<GenMerge><<<grid_for(hi - lo, CT), CT, GEN_SMEM, st>>>(b, c, lo, hi);
     else k_gen_w<GenMerge><<<grid_for(hi - lo, 4), 128, 0, st>>>(b, c, lo, hi);
   }
-  static const bool done = [] {  // once per process, thread-safe
-    cudaFuncSetAttribute(k_gen_top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GenTopShared));
-    return true;
-  }();
-  (void)done;
+  static DeviceOnce once;
+  set_limits(once, {{(const void*)k_gen_top, (int)sizeof(GenTopShared)}});
   k_gen_top<<<c.n_chains, TOP_THREADS, sizeof(GenTopShared), st>>>(b, c);
   for (int l = c.n_levels - 1; l >= 0; --l) {
     const int lo = c.merge_off[l], hi = c.merge_off[l + 1];

@@ -27,6 +27,7 @@
 #include "gf_beam_gp.cuh"
 #include "gf_chain.cuh"
 #include "gf_chain_root.cuh"
+#include "gf_kernels.cuh"
 #include "gf_math.cuh"
 
 namespace gf {
@@ -655,11 +656,8 @@ void launch_sym_chains(const Batch& b, const ChainParts& c, cudaStream_t st) {
     if (hi <= c.merge_soa) k_sym<Merge><<<grid_for(hi - lo, CT), CT, 0, st>>>(b, c, lo, hi);
     else k_sym_h<Merge><<<grid_for(hi - lo, 8), 128, 0, st>>>(b, c, lo, hi);
   }
-  static const bool done = [] {  // once per process, thread-safe
-    cudaFuncSetAttribute(k_sym_top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SymTopShared));
-    return true;
-  }();
-  (void)done;
+  static DeviceOnce once;
+  set_limits(once, {{(const void*)k_sym_top, (int)sizeof(SymTopShared)}});
   k_sym_top<<<c.n_chains, TOP_THREADS, sizeof(SymTopShared), st>>>(b, c);
   for (int l = c.n_levels - 1; l >= 0; --l) {
     const int lo = c.merge_off[l], hi = c.merge_off[l + 1];

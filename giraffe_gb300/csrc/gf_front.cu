@@ -1068,16 +1068,11 @@ __global__ void k_mf_add(int n, const double* d, double* x) {
 namespace {
 constexpr int ZERO_CTAS = 8 * 152;
 
-// Shared-memory limit, once per process (thread-safe).
 template <typename T> void mf_attrs() {
-  static const bool done = [] {
-    cudaFuncSetAttribute(k_mf_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         MF_SMALL * (MF_SMALL + 1) * (int)sizeof(T));
-    cudaFuncSetAttribute(k_mf_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_mf_back<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    return true;
-  }();
-  (void)done;
+  static DeviceOnce once;
+  set_limits(once, {{(const void*)k_mf_small<T>, MF_SMALL * (MF_SMALL + 1) * (int)sizeof(T)},
+                    {(const void*)k_mf_fwd<T>, 200 * 1024},
+                    {(const void*)k_mf_back<T>, 200 * 1024}});
 }
 
 // A launch in clusters of C CTAs along x.

@@ -349,11 +349,8 @@ __global__ void __launch_bounds__(T5_THREADS, 1) k_mf_t5(Batch b, int job0, int 
 
 void launch_front_t5(const Batch& b, const FrontLevel& V, cudaStream_t st) {
   if (!V.t5_cnt) return;
-  static const bool done = [] {  // once per process, thread-safe
-    cudaFuncSetAttribute(k_mf_t5, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MF_T5_SMEM);
-    return true;
-  }();
-  (void)done;
+  static DeviceOnce once;
+  set_limits(once, {{(const void*)k_mf_t5, (int)MF_T5_SMEM}});
   for (int q = 0; q < front_grids(V.t5_cnt); ++q) {
     const int n = min(V.t5_cnt - q * MF_GRID_FRONTS, MF_GRID_FRONTS), off = V.t5_off + q * MF_GRID_FRONTS;
     k_mf_kmax<<<dim3((V.t5_s + 7) / 8, 2, n), 256, 0, st>>>(b, off);

@@ -1581,17 +1581,12 @@ void launch_commit(const Batch& b, cudaStream_t st) {
   launch_commit_nodes(b, st);
 }
 
-// Shared-memory limits of the large kernels, once per process (the served
-// path's builder thread and the caller's thread may both get here first; a
-// function-local static is initialised by exactly one of them).
+// Shared-memory limits of the large kernels (the served path's builder thread and the
+// caller's thread may both get here first).
 static void set_attrs() {
-  static const bool done = [] {
-    cudaFuncSetAttribute(k_beam_tangent<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOUNT_SMEM_SPLIT);
-    cudaFuncSetAttribute(k_band_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (RING * GF_LDB + RING) * (int)sizeof(double));
-    return true;
-  }();
-  (void)done;
+  static DeviceOnce once;
+  set_limits(once, {{(const void*)k_beam_tangent<2>, MOUNT_SMEM_SPLIT},
+                    {(const void*)k_band_solve, (RING * GF_LDB + RING) * (int)sizeof(double)}});
 }
 
 const char* kernel_class_name(int k) {
@@ -1694,9 +1689,8 @@ void launch_band_solve(const Batch& b, cudaStream_t st) {
 void launch_beam_elements(int n, const BeamConst* c, const BeamHist* h, const double* d, double* K,
                           double* f, cudaStream_t st) {
   if (n <= 0) return;
-  static const bool attr =
-      cudaFuncSetAttribute(k_beam_elements, cudaFuncAttributeMaxDynamicSharedMemorySize, BE_SMEM) == cudaSuccess;
-  (void)attr;
+  static DeviceOnce once;
+  set_limits(once, {{(const void*)k_beam_elements, BE_SMEM}});
   k_beam_elements<<<(n + 31) / 32, MOUNT_THREADS, BE_SMEM, st>>>(n, c, h, d, K, f);
 }
 

@@ -23,9 +23,29 @@
 #pragma once
 #include <nvtx3/nvToolsExt.h>
 
+#include <initializer_list>
+
+#include "gf_device_once.h"
 #include "gf_types.h"
 
 namespace gf {
+
+// set_limits(once, {...}): dynamic shared memory limits of kernels, once per device
+// (thread-safe; a failure is CUDA's last error, and tried again at the next launch).
+struct SmemLimit {
+  const void* kernel;
+  int bytes;
+};
+inline void set_limits(DeviceOnce& once, std::initializer_list<SmemLimit> limits) {
+  int device = 0;
+  cudaGetDevice(&device);
+  once(device, [&] {
+    bool ok = true;
+    for (const SmemLimit& l : limits)
+      ok = cudaFuncSetAttribute(l.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, l.bytes) == cudaSuccess && ok;
+    return ok;
+  });
+}
 
 // Optional per-kernel timing: when non-null, every launch of kernel class k
 // is bracketed by events ev[2*i], ev[2*i+1] and recorded in cls[i].

@@ -352,11 +352,8 @@ template <class Src> __global__ void __launch_bounds__(ST_THREADS) k_shell_mount
 }
 
 template <class Src> static void launch_mount(const Src& src, int n, cudaStream_t st) {
-  static const bool done = [] {  // once per process, thread-safe
-    cudaFuncSetAttribute(k_shell_mount<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SIZE * 8);
-    return true;
-  }();
-  (void)done;
+  static DeviceOnce once;
+  set_limits(once, {{(const void*)k_shell_mount<Src>, ST_SIZE * 8}});
   k_shell_mount<Src><<<(n + ST_E - 1) / ST_E, ST_THREADS, ST_SIZE * 8, st>>>(src);
 }
 

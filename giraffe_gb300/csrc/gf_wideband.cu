@@ -999,12 +999,8 @@ static void launch_bwd(const Batch& b, int p, int nrhs, cudaStream_t st) {
 static void launch_wb_update(const Batch& b, int p, int part, cudaStream_t st) {
   const int nw = b.sh.n_wide, mr = b.sh.max_kl;
   if (b.sh.wide_tc && part != 1) {
-    static const bool attr = [] {  // once per process, thread-safe
-      cudaFuncSetAttribute(k_wb_update_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OZ_SMEM);
-      cudaFuncSetAttribute(k_wb_update_t5, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T5_SMEM);
-      return true;
-    }();
-    (void)attr;
+    static DeviceOnce once;
+    set_limits(once, {{(const void*)k_wb_update_tc, (int)OZ_SMEM}, {(const void*)k_wb_update_t5, (int)T5_SMEM}});
     // the panel's slices (L21 rows and U12 columns), then the tiles
     k_wb_slice<<<dim3((mr + SL_ROWS - 1) / SL_ROWS, 2, nw), 256, 0, st>>>(b, p);
     if (b.sh.wide_tc == 1)  // GF_WIDE_TENSOR: tcgen05; 2, GF_WIDE_TENSOR_SYNC: mma.sync
