@@ -763,7 +763,7 @@ template <typename T> __device__ __forceinline__ T mf_block_fwd(const T (*D)[33]
 // plate (0.84 ms of a 6.2 ms pass), where the top fronts' U12 alone is 44 us of one
 // SM's FP64 rate, and 11 us a height and sweep on the 24x24x2 plate's FP32 fronts,
 // most of it four loads at a time from L2 over U12's columns.
-constexpr int MF_BACK_THREADS = 256, MF_PART = 512;
+constexpr int MF_BACK_THREADS = 256;
 
 template <typename T> struct MfSubst {
   T D[2][32][33];   // diagonal blocks: column j, row i
@@ -1071,8 +1071,8 @@ constexpr int ZERO_CTAS = 8 * 152;
 template <typename T> void mf_attrs() {
   static DeviceOnce once;
   set_limits(once, {{(const void*)k_mf_small<T>, MF_SMALL * (MF_SMALL + 1) * (int)sizeof(T)},
-                    {(const void*)k_mf_fwd<T>, 200 * 1024},
-                    {(const void*)k_mf_back<T>, 200 * 1024}});
+                    {(const void*)k_mf_fwd<T>, MF_SUBST_SMEM},
+                    {(const void*)k_mf_back<T>, MF_SUBST_SMEM}});
 }
 
 // A launch in clusters of C CTAs along x.

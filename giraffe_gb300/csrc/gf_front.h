@@ -38,6 +38,10 @@ struct Front {
 // in its shared memory (k_mf_small); the others run panel by panel on many.
 constexpr int MF_SMALL = 96;
 constexpr int MF_NB = 32;  // pivots per panel of a large front
+// Shared memory of the substitutions beside their static part (gf_front.cu), and the rows
+// of a front whose vector fits it with the partial sums of MF_PART rows.
+constexpr int MF_SUBST_SMEM = 200 * 1024, MF_PART = 512;
+constexpr int MF_MAX_ROWS = MF_SUBST_SMEM / 8 - 2 - 8 * MF_PART;
 // Large fronts of a height that one launch takes where they are its grid's y or z (which
 // end at 65,535): more of them, as a band of 200,000 blocks has, take several.
 constexpr int MF_GRID_FRONTS = 65535;
@@ -142,6 +146,10 @@ struct FrontPlan {
 void nd_landmark_fields(NdGraph& g);
 // The plan of a graph whose vertex v holds the DOFs dofs[dptr[v] .. dptr[v + 1]).
 FrontPlan plan_fronts(const NdGraph& g, const std::vector<int>& dptr, const std::vector<int>& dofs);
+
+// Whether the kernels take a plan: 32-bit offsets, and every front's vector in shared
+// memory.
+bool fronts_fit(const FrontPlan& P);
 
 // Plans of several structures joined into one schedule; device offsets are
 // batch-wide.

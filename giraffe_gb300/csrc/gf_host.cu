@@ -1137,8 +1137,9 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       std::vector<int> offs;
       for (int s : wide_structs) {
         const FrontPlan& F = plan[s].fronts;
-        if (F.size > INT32_MAX) {
-          set_err(ctx, "structure %d: %lld entries of its fronts exceed 32-bit offsets", s, (long long)F.size);
+        if (!fronts_fit(F)) {
+          set_err(ctx, "structure %d: its fronts (%lld entries in all) exceed 32-bit offsets or %d rows in one", s,
+                  (long long)F.size, MF_MAX_ROWS);
           return GF_ERR_ARG;
         }
         plans.push_back(&F);

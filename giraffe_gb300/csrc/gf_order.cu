@@ -271,6 +271,12 @@ FrontPlan plan_fronts(const NdGraph& g, const std::vector<int>& dptr, const std:
   return P;
 }
 
+bool fronts_fit(const FrontPlan& P) {
+  int f = 0;
+  for (const gf::Front& F : P.fronts) f = std::max(f, F.f);
+  return P.size <= INT_MAX && f <= gf::MF_MAX_ROWS;
+}
+
 // The largest front of a height that takes one CTA.  One CTA runs at its SM's FP64
 // rate (16 cycles a warp instruction) and has no launches between its steps: the
 // way for many fronts.  Panel by panel a front spreads over the SMs at about 30 us

@@ -115,14 +115,6 @@ void csr_graph(int n, const int* rp, const int* ci, NdGraph& g, std::vector<int>
   }
 }
 
-// What the multifrontal kernels take: 32-bit offsets, and a front's column of
-// the solution in shared memory.
-bool fronts_fit(const FrontPlan& P) {
-  int f = 0;
-  for (const Front& F : P.fronts) f = std::max(f, F.f);
-  return P.size < INT_MAX && f <= 16384;
-}
-
 }  // namespace
 
 namespace gfh {
