@@ -1,7 +1,7 @@
 // One standalone system on the multifrontal LU: its plan, and the batch of one
 // structure around it that the kernels of gf_front.cu take.  Everything lives
-// in one block of the context's device workspace, its host data in one block
-// of pinned staging sent by one copy.  Internal to libgiraffe_gpu.so.
+// in one block of the context's device workspace, its host data sent by one copy
+// from pinned staging.  Internal to libgiraffe_gpu.so.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -67,13 +67,20 @@ struct FrontSystem {
     const size_t off_xs = after(off_ex, (size_t)fb.oz_exp * sizeof(int)), off_r = after(off_xs, sizeof(double) * (size_t)n);
     total = off_r + sizeof(double) * (size_t)n;
     dev = static_cast<char*>(ctx->device_work(total));
-    char* pin = static_cast<char*>(ctx->pinned(sent));
-    if (!dev || !pin) {
-      set_err(ctx, "linear solve: allocation of %zu device and %zu pinned bytes failed", total, sent);
+    if (!dev) {
+      set_err(ctx, "linear solve: allocation of %zu device bytes failed", total);
       return GF_ERR_CUDA;
     }
-    for (const Part& p : parts) std::memcpy(pin + p.off, p.src, p.bytes);
-    GF_CK(cudaMemcpyAsync(dev, pin, sent, cudaMemcpyHostToDevice, ctx->stream));
+    // through the context's pinned staging; from pageable memory, a part at a time, where
+    // there is none or the parts are too large to keep page-locked
+    if (char* pin = sent <= gf_ctx::kStagePin ? static_cast<char*>(ctx->pinned(sent)) : nullptr) {
+      for (const Part& p : parts)
+        if (p.bytes) std::memcpy(pin + p.off, p.src, p.bytes);
+      GF_CK(cudaMemcpyAsync(dev, pin, sent, cudaMemcpyHostToDevice, ctx->stream));
+    } else {
+      for (const Part& p : parts)
+        if (p.bytes) GF_CK(cudaMemcpyAsync(dev + p.off, p.src, p.bytes, cudaMemcpyHostToDevice, ctx->stream));
+    }
     b.n_struct = 1;
     b.n_free = n;
     b.info = at<gf::StructInfo>(p_info);
@@ -120,17 +127,23 @@ struct FrontSystem {
     cudaStream_t st = ctx->stream;
     int* bad = reinterpret_cast<int*>(b.state + 1);
     const size_t xb = sizeof(double) * (size_t)n;
-    char* pin = static_cast<char*>(ctx->pin);  // the staging is free again once the factorization has run
+    // the staging is free again once the factorization has run
+    std::vector<char> pageable;
+    char* pin = xb + sizeof(state) <= ctx->pin_bytes ? static_cast<char*>(ctx->pin) : nullptr;
+    if (!pin) {
+      pageable.resize(xb + sizeof(state));
+      pin = pageable.data();
+    }
     assemble(b);
     gf::launch_front_lu(b, xs, st);
     *done = false;
     for (int sweep = 0;; ++sweep) {
       check(xs, r, bad);
       GF_CK(cudaGetLastError());
-      GF_CK(cudaMemcpyAsync(pin + parts[p_rhs].off, xs, xb, cudaMemcpyDeviceToHost, st));
-      GF_CK(cudaMemcpyAsync(pin + parts[p_state].off, b.state, sizeof(state), cudaMemcpyDeviceToHost, st));
+      GF_CK(cudaMemcpyAsync(pin, xs, xb, cudaMemcpyDeviceToHost, st));
+      GF_CK(cudaMemcpyAsync(pin + xb, b.state, sizeof(state), cudaMemcpyDeviceToHost, st));
       GF_CK(cudaStreamSynchronize(st));
-      std::memcpy(&state, pin + parts[p_state].off, sizeof(state));
+      std::memcpy(&state, pin + xb, sizeof(state));
       if (state.st.info_fail || !state.bad) {
         *done = !state.st.info_fail;
         break;
@@ -139,7 +152,7 @@ struct FrontSystem {
       GF_CK(cudaMemsetAsync(bad, 0, sizeof(int), st));
       gf::launch_front_refine(b, n, r, xs, st);
     }
-    if (*done) std::memcpy(x, pin + parts[p_rhs].off, xb);
+    if (*done) std::memcpy(x, pin, xb);
     ctx->trim_work();
     return GF_OK;
   }

@@ -22,8 +22,8 @@ struct gf_ctx {
   // options of the standalone solves (gf_band_solve, gf_sparse_solve):
   // wide_update picks their wide-band trailing update
   int wide_update = GF_WIDE_TENSOR;
-  // pinned staging of gf_batch_results' read-back (grown on demand, freed
-  // with the context)
+  // pinned staging of gf_batch_results' read-back and of the standalone solves up to
+  // kStagePin bytes (grown on demand, freed with the context)
   void* pin = nullptr;
   size_t pin_bytes = 0;
   // device workspace of the standalone solves (calls on one context do not
@@ -32,6 +32,7 @@ struct gf_ctx {
   void* work = nullptr;
   size_t work_bytes = 0;
   static constexpr size_t kKeepWork = (size_t)512 << 20;
+  static constexpr size_t kStagePin = (size_t)256 << 20;
   void* device_work(size_t n) {
     if (n <= work_bytes) return work;
     if (work) cudaFree(work);
@@ -59,6 +60,7 @@ struct gf_ctx {
     pin = nullptr;
     pin_bytes = 0;
     if (cudaMallocHost(&pin, n) != cudaSuccess) {
+      cudaGetLastError();
       pin = nullptr;
       return nullptr;
     }
