@@ -140,6 +140,9 @@ struct FrontPlan {
   double flops = 0.0;
 };
 
+// Graph of a CSR matrix's symmetrised pattern, consecutive rows with the same columns (the
+// DOFs of a mesh node) as one vertex: its rows are dptr[v] .. dptr[v + 1).
+void csr_graph(int n, const int* rp, const int* ci, NdGraph& g, std::vector<int>& dptr);
 // Landmark fields of a graph without coordinates: differences of squared
 // distances to far-apart vertices (linear functions of the position where the
 // graph is a mesh).

@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <atomic>
 #include <climits>
+#include <cstring>
 #include <numeric>
 #include <thread>
 
@@ -184,6 +185,84 @@ void nd_landmark_fields(NdGraph& g) {
   add([&](int i) { return sq(0, i) + sq(1, i) - sq(2, i) - sq(3, i); });
   add([&](int i) { return sq(0, i) + sq(2, i) - sq(1, i) - sq(3, i); });
   add([&](int i) { return sq(0, i) + sq(3, i) - sq(1, i) - sq(2, i); });
+}
+
+void csr_graph(int n, const int* rp, const int* ci, NdGraph& g, std::vector<int>& dptr) {
+  std::vector<int> id(n);
+  for (int i = 0; i < n; ++i) {
+    const int len = rp[i + 1] - rp[i];
+    const bool same = i > 0 && len == rp[i] - rp[i - 1] && len > 0 &&
+                      std::memcmp(ci + rp[i], ci + rp[i - 1], sizeof(int) * (size_t)len) == 0;
+    if (!same) dptr.push_back(i);
+    id[i] = (int)dptr.size() - 1;
+  }
+  g.n = (int)dptr.size();
+  dptr.push_back(n);
+  for (int v = 0; v < g.n; ++v) g.w.push_back(dptr[v + 1] - dptr[v]);
+  // Rows in ascending order of a symmetric pattern are the lists already: each column u met
+  // while the rows go by has to be the next one of row u's own list.  (A sort of both
+  // directions of every edge took 30 ns an entry, most of a call with long rows.)
+  g.ptr.assign(1, 0);
+  bool plain = true;
+  for (int v = 0; v < g.n; ++v) {
+    int last = -1;
+    for (int k = rp[dptr[v]]; plain && k < rp[dptr[v] + 1]; ++k) {
+      const int u = id[ci[k]];
+      plain = u >= last;
+      if (u != v && u != last) g.adj.push_back(u);
+      last = u;
+    }
+    g.ptr.push_back((int)g.adj.size());
+  }
+  std::vector<int> at(g.ptr.begin(), g.ptr.end() - 1);
+  for (int v = 0; v < g.n && plain; ++v)
+    for (int k = g.ptr[v]; k < g.ptr[v + 1] && plain; ++k) {
+      const int u = g.adj[k], q = at[u]++;
+      plain = q < g.ptr[u + 1] && g.adj[q] == v;
+    }
+  if (plain) return;
+  // any other: both directions of every edge, a list's transpose (which comes out sorted)
+  // transposed again and the two merged without repeats
+  struct Lists {
+    std::vector<int> ptr, to;
+  };
+  auto transpose = [&](auto each) {
+    Lists T;
+    T.ptr.assign(g.n + 1, 0);
+    each([&](int, int u) { T.ptr[u + 1]++; });
+    for (int v = 0; v < g.n; ++v) T.ptr[v + 1] += T.ptr[v];
+    T.to.resize(T.ptr[g.n]);
+    at.assign(T.ptr.begin(), T.ptr.end() - 1);
+    each([&](int v, int u) { T.to[at[u]++] = v; });
+    return T;
+  };
+  const Lists col = transpose([&](auto f) {
+    for (int v = 0; v < g.n; ++v) {
+      int last = -1;
+      for (int k = rp[dptr[v]]; k < rp[dptr[v] + 1]; ++k) {
+        const int u = id[ci[k]];
+        if (u != v && u != last) f(v, u);
+        last = u;
+      }
+    }
+  });
+  const Lists row = transpose([&](auto f) {
+    for (int v = 0; v < g.n; ++v)
+      for (int k = col.ptr[v]; k < col.ptr[v + 1]; ++k)
+        if (k == col.ptr[v] || col.to[k] != col.to[k - 1]) f(v, col.to[k]);
+  });
+  g.ptr.assign(1, 0);
+  g.adj.clear();
+  for (int v = 0; v < g.n; ++v) {
+    int i = row.ptr[v], j = col.ptr[v], last = -1;
+    const int i1 = row.ptr[v + 1], j1 = col.ptr[v + 1];
+    while (i < i1 || j < j1) {
+      const int u = j >= j1 || (i < i1 && row.to[i] <= col.to[j]) ? row.to[i++] : col.to[j++];
+      if (u != last) g.adj.push_back(u);
+      last = u;
+    }
+    g.ptr.push_back((int)g.adj.size());
+  }
 }
 
 FrontPlan plan_fronts(const NdGraph& g, const std::vector<int>& dptr, const std::vector<int>& dofs) {

@@ -70,51 +70,6 @@ int csr_bandwidth(int n, const int* rp, const int* ci, const int* pos) {
   return w;
 }
 
-// Graph of the symmetrised CSR pattern, consecutive rows with the same columns
-// (the DOFs of a mesh node) as one vertex.
-void csr_graph(int n, const int* rp, const int* ci, NdGraph& g, std::vector<int>& dptr) {
-  std::vector<int> id(n);
-  for (int i = 0; i < n; ++i) {
-    const int len = rp[i + 1] - rp[i];
-    const bool same = i > 0 && len == rp[i] - rp[i - 1] && len > 0 &&
-                      std::memcmp(ci + rp[i], ci + rp[i - 1], sizeof(int) * (size_t)len) == 0;
-    if (!same) dptr.push_back(i);
-    id[i] = (int)dptr.size() - 1;
-  }
-  g.n = (int)dptr.size();
-  dptr.push_back(n);
-  for (int v = 0; v < g.n; ++v) g.w.push_back(dptr[v + 1] - dptr[v]);
-  // both directions of every edge, then each list sorted without repeats
-  std::vector<int> cnt(g.n + 1, 0);
-  auto edges = [&](auto f) {
-    for (int v = 0; v < g.n; ++v) {
-      int last = -1;
-      for (int k = rp[dptr[v]]; k < rp[dptr[v] + 1]; ++k) {
-        const int u = id[ci[k]];
-        if (u != v && u != last) f(v, u);
-        last = u;
-      }
-    }
-  };
-  edges([&](int v, int u) {
-    cnt[v + 1]++;
-    cnt[u + 1]++;
-  });
-  for (int v = 0; v < g.n; ++v) cnt[v + 1] += cnt[v];
-  std::vector<int> all(cnt[g.n]), at(cnt.begin(), cnt.end() - 1);
-  edges([&](int v, int u) {
-    all[at[v]++] = u;
-    all[at[u]++] = v;
-  });
-  g.ptr.assign(1, 0);
-  for (int v = 0; v < g.n; ++v) {
-    std::sort(all.begin() + cnt[v], all.begin() + cnt[v + 1]);
-    for (int k = cnt[v]; k < cnt[v + 1]; ++k)
-      if (k == cnt[v] || all[k] != all[k - 1]) g.adj.push_back(all[k]);
-    g.ptr.push_back((int)g.adj.size());
-  }
-}
-
 }  // namespace
 
 namespace gfh {

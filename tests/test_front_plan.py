@@ -46,3 +46,63 @@ int main(int, char** v) {
     rows = 200 * 1024 // 8 - 2 - 8 * 512
     for f, size, fit in ((rows, 10 ** 9, 1), (rows + 1, 10 ** 9, 0), (10, 2 ** 31 - 1, 1), (10, 2 ** 31, 0)):
         assert int(run(f, size).stdout) == fit
+
+
+def test_graph_of_a_csr_pattern(compiled):
+    # symmetric and sorted rows take a way of their own: 2,000 patterns of either kind,
+    # with repeated and unsorted columns and equal neighbouring rows, against sets
+    run = compiled("graph", r"""
+#include <algorithm>
+#include <cstdio>
+#include <random>
+#include <set>
+#include "gf_front.h"
+int main() {
+  std::mt19937 r(1);
+  int wrong = 0;
+  for (int t = 0; t < 2000; ++t) {
+    const int n = 1 + r() % 60, kind = r() % 4;
+    std::vector<std::vector<int>> R(n);
+    for (auto& x : R)
+      for (int q = r() % 8; q > 0; --q) x.push_back(r() % n);
+    if (kind & 1) {  // symmetric
+      const auto S = R;
+      for (int i = 0; i < n; ++i)
+        for (int u : S[i]) R[u].push_back(i);
+    }
+    if (kind & 2)  // ascending, now and then without repeats
+      for (auto& x : R) {
+        std::sort(x.begin(), x.end());
+        if (r() % 2) x.erase(std::unique(x.begin(), x.end()), x.end());
+      }
+    if (r() % 2)
+      for (int i = 1; i < n; ++i)
+        if (r() % 3 == 0) R[i] = R[i - 1];
+    std::vector<int> rp(1, 0), ci, dptr, id(n);
+    for (auto& x : R) {
+      ci.insert(ci.end(), x.begin(), x.end());
+      rp.push_back((int)ci.size());
+    }
+    gfh::NdGraph g;
+    gfh::csr_graph(n, rp.data(), ci.data(), g, dptr);
+    bool ok = (int)dptr.size() == g.n + 1 && dptr[0] == 0 && dptr[g.n] == n && (int)g.ptr.size() == g.n + 1;
+    std::vector<std::set<int>> A(g.n);
+    for (int v = 0; v < g.n; ++v)
+      for (int i = dptr[v]; i < dptr[v + 1]; ++i) {
+        id[i] = v;
+        ok = ok && R[i] == R[dptr[v]] && g.w[v] == dptr[v + 1] - dptr[v];
+      }
+    for (int i = 0; i < n; ++i)
+      for (int u : R[i])
+        if (id[u] != id[i]) {
+          A[id[i]].insert(id[u]);
+          A[id[u]].insert(id[i]);
+        }
+    for (int v = 0; v < g.n && ok; ++v)
+      ok = std::vector<int>(A[v].begin(), A[v].end()) == std::vector<int>(g.adj.begin() + g.ptr[v], g.adj.begin() + g.ptr[v + 1]);
+    wrong += !ok;
+  }
+  std::printf("%d", wrong);
+}
+""")
+    assert run().stdout == "0"
