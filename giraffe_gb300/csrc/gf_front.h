@@ -58,10 +58,10 @@ constexpr double MF_T5_WORK = 1.5e6;
 // and beam tangents reach 1 to 8 of them in either order, a tridiagonal system with a
 // diagonal entry of 1e-3 that the dissection puts first 130, one of 1e-6 350,000.
 constexpr double MF_ERROR_LIMIT = 0x1p-49;
-// Such a front: its slices, exponents (per 128 pivots) and pivot maxima.
+// Such a front: its slices, exponents (per 64 pivots) and pivot maxima.
 struct FrontT5 {
   int64_t slices;  // L21's at oz[slices], U12's behind: [64 pivots][slice][rows][64]
-  int exps, kmax;  // [operand][128 pivots][rows], [operand][s]
+  int exps, kmax;  // [operand][64 pivots][rows], [operand][s]
   int rows;        // rows of L21 and columns of U12, padded to 128
   int front;
 };

@@ -1,7 +1,7 @@
 // The Schur complements C -= L21 U12 of the largest fronts on the 5th-generation
 // tensor cores, FP64 products from exact bf16 slices (see k_wb_update_tc's comment
-// in gf_wideband.cu for the slicing and its error; here a row's power of two holds
-// for 128 pivots, whose slice products stay exact integers: 8 * 128 * 127^2 < 2^24).
+// in gf_wideband.cu for the slicing and its error: a row's power of two holds for 64
+// pivots).
 //   k_mf_kmax    largest entry of every pivot's column of L21 and row of U12
 //   k_mf_slice   the slices, every pivot balanced by a power of two
 //   k_mf_t5      128 x 64 tiles of C
@@ -20,8 +20,7 @@ namespace gf {
 
 namespace {
 
-constexpr int T5_CHUNK = 128;  // pivots under one exponent, two 64-wide sub-chunks
-constexpr int SL_ROWS = 16;    // rows (columns) a CTA slices
+constexpr int SL_ROWS = 32;  // rows (columns) a CTA slices
 
 __device__ __forceinline__ bool mf_active(const Batch& b, int s) {
   const StructState& st = b.state[s];
@@ -32,8 +31,8 @@ __device__ __forceinline__ bool mf_active(const Batch& b, int s) {
 __device__ __forceinline__ __nv_bfloat16* t5_slices(const FrontData& d, const FrontT5& T, int s, int op, int sub) {
   return d.oz + T.slices + (int64_t)(op * ((s + OZ_K - 1) / OZ_K) + sub) * OZ_S * T.rows * OZ_K;
 }
-__device__ __forceinline__ int* t5_exps(const FrontData& d, const FrontT5& T, int s, int op, int chunk) {
-  return d.oz_exp + T.exps + (op * ((s + T5_CHUNK - 1) / T5_CHUNK) + chunk) * T.rows;
+__device__ __forceinline__ int* t5_exps(const FrontData& d, const FrontT5& T, int s, int op, int sub) {
+  return d.oz_exp + T.exps + (op * ((s + OZ_K - 1) / OZ_K) + sub) * T.rows;
 }
 
 // S 2^k
@@ -87,25 +86,25 @@ __global__ void __launch_bounds__(256) k_mf_kmax(Batch b, int off) {
   }
 }
 
-// Sixteen rows of L21 (blockIdx.y even) or columns of U12 (odd) over the 128 pivots of
-// chunk blockIdx.y / 2; rows beyond the front and pivots beyond s are zero.  The CTAs of
-// L21's first chunk also take the right-hand side of their rows.
+// SL_ROWS rows of L21 (blockIdx.y even) or columns of U12 (odd) over 64 pivots, the
+// blockIdx.y / 2-th of them; rows beyond the front and pivots beyond s are zero.  The CTAs
+// of L21's first pivots also take the right-hand side of their rows.
 __global__ void __launch_bounds__(256) k_mf_slice(Batch b, int off) {
   const FrontData& d = b.sh.mf;
   const FrontT5 T = d.t5[off + blockIdx.z];
   const Front F = d.fronts[T.front];
   if (!mf_active(b, F.slot)) return;
   const int op = blockIdx.y & 1, ch = blockIdx.y >> 1, r0 = SL_ROWS * blockIdx.x, s = F.s, ld = F.ld;
-  const int kb = T5_CHUNK * ch, kn = min(T5_CHUNK, s - kb);
+  const int kb = OZ_K * ch, kn = min(OZ_K, s - kb);
   if (r0 >= T.rows || kn <= 0) return;
   const int n = F.f - s;  // rows of L21, columns of U12
   double* G = d.F + F.off;
-  static_assert(SL_ROWS * T5_CHUNK == 8 * 256, "a chunk of eight pivots per thread");
-  __shared__ double A[SL_ROWS][T5_CHUNK + 1];
+  static_assert(SL_ROWS * OZ_K == 8 * 256, "eight pivots of a row per thread");
+  __shared__ double A[SL_ROWS][OZ_K + 1];
   __shared__ int e[SL_ROWS];
-  __shared__ double bal[T5_CHUNK];
+  __shared__ double bal[OZ_K];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < T5_CHUNK) {
+  if (tid < OZ_K) {
     // pivot k's column of L21 times 2^-f, its row of U12 times 2^f: the products
     // unchanged, the two maxima within a factor two of each other
     int f = 0;
@@ -118,9 +117,9 @@ __global__ void __launch_bounds__(256) k_mf_slice(Batch b, int off) {
   }
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < SL_ROWS * T5_CHUNK / 256; ++q) {
+  for (int q = 0; q < SL_ROWS * OZ_K / 256; ++q) {
     const int x = tid + 256 * q;
-    const int i = op ? x / T5_CHUNK : x % SL_ROWS, k = op ? x % T5_CHUNK : x / SL_ROWS;
+    const int i = op ? x / OZ_K : x % SL_ROWS, k = op ? x % OZ_K : x / SL_ROWS;
     const bool live = k < kn && r0 + i < n;
     A[i][k] = live ? G[op ? kb + k + (int64_t)(s + r0 + i) * ld : s + r0 + i + (int64_t)(kb + k) * ld] * bal[k] : 0.0;
   }
@@ -128,7 +127,7 @@ __global__ void __launch_bounds__(256) k_mf_slice(Batch b, int off) {
   for (int i = warp; i < SL_ROWS; i += 8) {
     unsigned long long m = 0;
 #pragma unroll
-    for (int q = 0; q < T5_CHUNK / 32; ++q) m = max(m, oz_mag(A[i][lane + 32 * q]));
+    for (int q = 0; q < OZ_K / 32; ++q) m = max(m, oz_mag(A[i][lane + 32 * q]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (lane == 0) e[i] = oz_exponent(m);
@@ -136,49 +135,47 @@ __global__ void __launch_bounds__(256) k_mf_slice(Batch b, int off) {
   __syncthreads();
   // eight pivots of a row per thread: a 16-byte chunk of every slice
   {
-    const int i = tid >> 4, k0 = 8 * (tid & 15), r = r0 + i;
-    if (k0 < (kn + OZ_K - 1) / OZ_K * OZ_K) {
-      uint32_t w[OZ_S][4];
+    const int i = tid >> 3, k0 = 8 * (tid & 7), r = r0 + i;
+    uint32_t w[OZ_S][4];
 #pragma unroll
-      for (int x = 0; x < 8; ++x) {
-        uint16_t v[OZ_S];
-        oz_split_bits(A[i][k0 + x], e[i], v);
+    for (int x = 0; x < 8; ++x) {
+      uint16_t v[OZ_S];
+      oz_split_bits(A[i][k0 + x], e[i], v);
 #pragma unroll
-        for (int q = 0; q < OZ_S; ++q) w[q][x >> 1] = x & 1 ? w[q][x >> 1] | (uint32_t)v[q] << 16 : v[q];
-      }
-      // the 128-byte swizzle: 16-byte chunk c of row r at chunk c ^ (r & 7)
-      __nv_bfloat16* dst = t5_slices(d, T, s, op, 2 * ch + (k0 >> 6)) + (int64_t)r * OZ_K + 8 * (((k0 >> 3) & 7) ^ (r & 7));
-#pragma unroll
-      for (int q = 0; q < OZ_S; ++q)
-        *reinterpret_cast<uint4*>(dst + (int64_t)q * T.rows * OZ_K) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+      for (int q = 0; q < OZ_S; ++q) w[q][x >> 1] = x & 1 ? w[q][x >> 1] | (uint32_t)v[q] << 16 : v[q];
     }
+    // the 128-byte swizzle: 16-byte chunk c of row r at chunk c ^ (r & 7)
+    __nv_bfloat16* dst = t5_slices(d, T, s, op, ch) + (int64_t)r * OZ_K + 8 * ((tid & 7) ^ (r & 7));
+#pragma unroll
+    for (int q = 0; q < OZ_S; ++q)
+      *reinterpret_cast<uint4*>(dst + (int64_t)q * T.rows * OZ_K) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
   }
   if (tid < SL_ROWS) t5_exps(d, T, s, op, ch)[r0 + tid] = e[tid];
   if (op || ch || r0 >= n) return;
-  // the right-hand side of these rows, in FP64: sixteen lanes a row
+  // the right-hand side of these rows, in FP64: eight lanes a row
   const int i = tid % SL_ROWS, q = tid / SL_ROWS, r = s + r0 + i;
   double acc = 0.0;
   if (r < F.f)
 #pragma unroll 4
-    for (int k = q; k < s; k += 16) acc = fma(G[r + (int64_t)k * ld], G[k + (int64_t)F.f * ld], acc);
+    for (int k = q; k < s; k += 8) acc = fma(G[r + (int64_t)k * ld], G[k + (int64_t)F.f * ld], acc);
   __syncthreads();
   A[i][q] = acc;
   __syncthreads();
   if (q == 0 && r < F.f) {
     double t = A[i][0];
 #pragma unroll
-    for (int x = 1; x < 16; ++x) t += A[i][x];
+    for (int x = 1; x < 8; ++x) t += A[i][x];
     G[r + (int64_t)F.f * ld] -= t;
   }
 }
 
-// 128 x 64 tiles of C, one after the other, all pivots of a tile, 128 at a time: eight
+// 128 x 64 tiles of C, one after the other, all pivots of a tile, 64 at a time: eight
 // accumulators of 64 columns in tensor memory (diagonal q + t of the slice products),
 // issued by one thread.  The sixteen slices of 64 pivots (192 KB) are asked for at
 // once, as soon as the products of the 64 before have run, of the next tile too, so
 // they arrive beside the epilogue.  The tile of C waits in registers (a row and 16
-// columns per thread); after every 128 pivots the diagonals are joined in 64-bit
-// integers, converted once and subtracted: two FP64 operations an entry for 128 FMA.
+// columns per thread); after every 64 pivots the diagonals are joined in 64-bit
+// integers, converted once and subtracted: two FP64 operations an entry for 64 FMA.
 // Every wait is bounded; one that gives up fails the solves of its and the CTA's
 // later tiles, and the copies in flight are waited for (bounded) before the CTA ends.
 constexpr size_t MF_T5_SMEM = 1024 + OZ_S * (T5_B_BYTES + T5_A_BYTES) + 128 + T5_N * sizeof(int);
@@ -254,13 +251,11 @@ __global__ void __launch_bounds__(T5_THREADS, 1) k_mf_t5(Batch b, int job0, int 
     double* C = d.F + F.off + s + r + (int64_t)(s + c0 + cb) * F.ld;
     double c22[T5_COLS_PER_WARP];
     for (int sub = 0; sub < nsub; ++sub, phase ^= 1) {
-      const int ch = sub >> 1;
-      if (!(sub & 1) && tid < T5_N) eU[tid] = t5_exps(d, T, s, 1, ch)[c0 + tid];
+      if (tid < T5_N) eU[tid] = t5_exps(d, T, s, 1, sub)[c0 + tid];
       if (tid == 0) {
         const int kk_n = (min(OZ_K, s - OZ_K * sub) + 15) / 16;
         bool ok = t5_wait(fullB, phase);
         int landed = 0;
-        const uint32_t first = sub & 1;  // the chunk's first 64 pivots overwrite the accumulators
 #pragma unroll
         for (int q = 0; q < OZ_S; ++q) {
           ok = ok && t5_wait(fullA + 8 * q, phase);
@@ -273,7 +268,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) k_mf_t5(Batch b, int job0, int 
             for (int t = 0; t + q < OZ_S; ++t) {
               const uint64_t db = descB + (uint64_t)(t * (T5_B_BYTES >> 4));
               const uint32_t acc = tmem + (uint32_t)((q + t) * T5_N);
-              t5_mma(acc, da, db, q == 0 ? first : 1u);
+              t5_mma(acc, da, db, q == 0 ? 0u : 1u);  // the first products overwrite the accumulators
               if (kk_n > 1) t5_mma(acc, da + 2, db + 2, 1u);
               if (kk_n > 2) t5_mma(acc, da + 4, db + 4, 1u);
               if (kk_n > 3) t5_mma(acc, da + 6, db + 6, 1u);
@@ -299,8 +294,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) k_mf_t5(Batch b, int job0, int 
         if (sub + 1 < nsub) load(job, sub + 1);
         else if (next < n_jobs) load(next, 0);
       }
-      if (!(sub & 1) && sub + 1 < nsub) continue;  // the other 64 of the chunk
-      const int eLr = t5_exps(d, T, s, 0, ch)[r];
+      const int eLr = t5_exps(d, T, s, 0, sub)[r];
       t5_fence_after();
       const uint32_t tl = tmem + ((uint32_t)(lg * 32) << 16);
 #pragma unroll
@@ -314,7 +308,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) k_mf_t5(Batch b, int job0, int 
           int ci[OZ_S];
 #pragma unroll
           for (int q = 0; q < OZ_S; ++q) ci[q] = __float2int_rn(__uint_as_float(v[q][cc]));
-          // S = sum_d c_d 2^(7 (7 - d)) with |c_d| <= (d + 1) 2^21, T = floor(S / 2^10) in
+          // S = sum_d c_d 2^(7 (7 - d)) with |c_d| <= (d + 1) 2^20, T = floor(S / 2^10) in
           // 64 bits: pairs of diagonals first (|c_d 2^7 + c_(d+1)| < 2^31)
           const int P0 = ci[0] * 128 + ci[1], P1 = ci[2] * 128 + ci[3], P2 = ci[4] * 128 + ci[5];
           const int P3 = (ci[6] * 128 + ci[7]) >> 10;
@@ -354,7 +348,7 @@ void launch_front_t5(const Batch& b, const FrontLevel& V, cudaStream_t st) {
   for (int q = 0; q < front_grids(V.t5_cnt); ++q) {
     const int n = min(V.t5_cnt - q * MF_GRID_FRONTS, MF_GRID_FRONTS), off = V.t5_off + q * MF_GRID_FRONTS;
     k_mf_kmax<<<dim3((V.t5_s + 7) / 8, 2, n), 256, 0, st>>>(b, off);
-    k_mf_slice<<<dim3(V.t5_rows / SL_ROWS, 2 * ((V.t5_s + T5_CHUNK - 1) / T5_CHUNK), n), 256, 0, st>>>(b, off);
+    k_mf_slice<<<dim3(V.t5_rows / SL_ROWS, 2 * ((V.t5_s + OZ_K - 1) / OZ_K), n), 256, 0, st>>>(b, off);
   }
   k_mf_t5<<<min(V.t5_job_cnt, 152), T5_THREADS, MF_T5_SMEM, st>>>(b, V.t5_job_off, V.t5_job_cnt);
 }

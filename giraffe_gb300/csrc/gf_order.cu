@@ -521,7 +521,7 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
       const int u = F.f - F.s, rows = (u + 127) / 128 * 128, id = (int)out.t5.size();
       out.t5.push_back(gf::FrontT5{oz, (int)exps, (int)kmax, rows, k});
       oz += (int64_t)2 * ((F.s + 63) / 64) * 8 * rows * 64;
-      exps += (int64_t)2 * ((F.s + 127) / 128) * rows;
+      exps += (int64_t)2 * ((F.s + 63) / 64) * rows;
       kmax += 2 * F.s;
       V.t5_rows = std::max(V.t5_rows, rows);
       V.t5_s = std::max(V.t5_s, F.s);

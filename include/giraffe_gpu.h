@@ -85,7 +85,7 @@ typedef struct gf_solve_opts {
                       GF_WIDE_TENSOR_SYNC runs the same emulation on warp-level
                       mma.sync where the wide-band LU is used, FP64 FMA in the
                       multifrontal LU.  The emulated product of row i of L21 and
-                      column j of U12 (K <= 128 terms at a time) errs by at most
+                      column j of U12 (K <= 64 terms at a time) errs by at most
                       about 2^-52 K max_k |L_ik 2^-f_k| max_k |2^f_k U_kj|, where
                       2^f_k is a power-of-two balancing of pivot k's column
                       of L21 against its row of U12; for

@@ -332,3 +332,37 @@ def test_more_fronts_of_a_height_than_a_grid_has_rows(gpu_ctx):
     b[:kl] = 2.0
     x, info = gpu_ctx.band_solve(ab, kl, 0, b)
     assert info == 0 and np.array_equal(x, np.ones(n))
+
+
+def test_slices_hold_an_exponent_per_64_pivots(gpu_ctx):
+    # two blocks of 128 pivots coupled to 128 rows: L21 is 1 over the first 64 pivots and
+    # 1e-8 over the others, half of U12's columns 0 and 1e-8, so their Schur complement of
+    # 1e-16 comes from the small entries alone.  An emulated product errs by 2^-52 64 max|L|
+    # max|U| over 64 pivots each: 64 x 128 of it against a diagonal of 200e-16 and sums
+    # below half of that, 2^-52 x 82; under one exponent for all 128 pivots 1e8 times that
+    rng = np.random.default_rng(11)
+    m, e = 128, 1e-8
+    n = 3 * m
+    A = np.eye(n)
+    S, half = slice(2 * m, n), 2 * m + m // 2
+    for q in range(2):
+        first, last = slice(q * m, q * m + m // 2), slice(q * m + m // 2, q * m + m)
+        A[S, first] = rng.uniform(-1.0, 1.0, (m, m // 2))
+        A[S, last] = e * rng.uniform(-1.0, 1.0, (m, m // 2))
+        A[first, 2 * m:half] = rng.uniform(-1.0, 1.0, (m // 2, m // 2))
+        A[last, half:] = e * rng.uniform(-1.0, 1.0, (m // 2, m // 2))
+    A[S, S] = np.diag(np.where(np.arange(m) < m // 2, 200.0, 200.0 * e * e))
+    # the same system with columns and rows of like size, for the reference
+    r = np.ones(n)
+    c = np.ones(n)
+    c[half:] = 1.0 / (e * e)
+    for q in range(2):
+        last = slice(q * m + m // 2, q * m + m)
+        r[last], c[last] = e, 1.0 / e
+    b = rng.normal(size=n)
+    b /= r
+    ref = np.linalg.solve(r[:, None] * A * c, r * b) * c
+    rows, cols = np.nonzero(np.kron(np.array([[1, 0, 1], [0, 1, 1], [1, 1, 1]]), np.ones((m, m))))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.int32)
+    x, info = gpu_ctx.sparse_solve(rp, cols.astype(np.int32), A[rows, cols], b)
+    assert info == 0 and (np.abs(x - ref) / c).max() <= 1e-12 * (np.abs(ref) / c).max()
