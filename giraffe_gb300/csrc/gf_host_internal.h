@@ -247,10 +247,12 @@ std::vector<int> rcm_order(int nn, const std::vector<std::vector<int>>& adj);
 // gf_band_solve for half-bandwidths above 17: the blocked wide-band LU on a
 // one-structure batch (gf_sparse.cu).
 int wide_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, int* info);
-// gf_band_solve on the multifrontal LU, and whether it takes it (gf_sparse.cu).  *done:
-// b holds the solution; false leaves b for the natural order's solvers.
+// gf_band_solve and gf_sparse_solve on the multifrontal LU, and whether the former takes
+// it (gf_sparse.cu).  *done: b holds the solution; false leaves b for the natural order's
+// solvers.
 bool band_takes_fronts(int n, int kl, int ku);
 int front_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, bool* done);
+int front_sparse_solve(gf_ctx* ctx, int n, const int* rp, const int* ci, const double* val, double* b, bool* done);
 using gf::beam_precalc;
 using gf::beam_state_in;
 using gf::cs_rows;

@@ -4,7 +4,9 @@
 #include <atomic>
 #include <climits>
 #include <cstring>
+#include <exception>
 #include <numeric>
+#include <system_error>
 #include <thread>
 
 #include "gf_front.h"
@@ -16,6 +18,36 @@ namespace {
 // A part of at most this weight (DOFs) is not split further: below it a split
 // only adds fronts (a 2-element patch of the six-node mesh weighs 6 to 50).
 constexpr int ND_LEAF = 24;
+
+// Runs f on a thread of its own, or at once where one is not wanted or cannot be had;
+// join() throws what f threw.
+struct Beside {
+  std::thread t;
+  std::exception_ptr error;
+  template <typename F> Beside(bool own, F f) {
+    if (own) {
+      try {
+        t = std::thread([this, f] {
+          try {
+            f();
+          } catch (...) {
+            error = std::current_exception();
+          }
+        });
+        return;
+      } catch (const std::system_error&) {
+      }
+    }
+    f();
+  }
+  void join() {
+    if (t.joinable()) t.join();
+    if (error) std::rethrow_exception(error);
+  }
+  ~Beside() {
+    if (t.joinable()) t.join();
+  }
+};
 
 struct Dissection {
   const NdGraph& g;
@@ -125,14 +157,10 @@ struct Dissection {
     std::copy(s.begin(), s.end(), perm.begin() + lo + a.size() + b.size());
     const int ma = lo + (int)a.size(), mb = ma + (int)b.size();
     if (!s.empty()) start[mb] = 1;
-    if (depth < 4 && m > 1000) {
-      std::thread t([&] { split(lo, ma, depth + 1); });
-      split(ma, mb, depth + 1);
-      t.join();
-    } else {
-      split(lo, ma, depth + 1);
-      split(ma, mb, depth + 1);
-    }
+    auto first = [this, lo, ma, depth] { split(lo, ma, depth + 1); };
+    Beside t(depth < 4 && m > 1000, first);
+    split(ma, mb, depth + 1);
+    t.join();
   }
 };
 

@@ -19,6 +19,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "../../include/giraffe_gpu.h"
@@ -95,8 +96,7 @@ bool band_takes_fronts(int n, int kl, int ku) {
   return t_front < t_band;
 }
 
-int front_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, bool* done) {
-  *done = false;
+static int band_on_fronts(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, bool* done) {
   // blocks of at least the half-bandwidth: their graph is a path
   const int B = std::max(std::max(kl, ku), 12), nb = (n + B - 1) / B, W = kl + ku + 1;
   NdGraph g;
@@ -125,6 +125,47 @@ int front_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int l
   return S.solve(ctx, n, [&](const Batch& q) { launch_front_band(q, n, kl, ku, W, A, ctx->stream); },
                  [&](const double* x, double* r, int* bad) { launch_band_residual(n, kl, ku, W, A, S.b.P, x, r, bad, ctx->stream); },
                  b, done);
+}
+
+static int sparse_on_fronts(gf_ctx* ctx, int n, const int* rp, const int* ci, const double* val, double* b, bool* done) {
+  if (rp[n] > INT_MAX / 2) return GF_OK;  // both directions of its edges are counted in 32 bits
+  NdGraph g;
+  std::vector<int> dptr, dofs(n);
+  csr_graph(n, rp, ci, g, dptr);
+  for (int i = 0; i < n; ++i) dofs[i] = i;
+  nd_landmark_fields(g);
+  std::vector<float> place(g.n);
+  for (int v = 0; v < g.n; ++v) place[v] = (float)v;
+  g.field.push_back(std::move(place));
+  const FrontPlan plan = plan_fronts(g, dptr, dofs);
+  if (!fronts_fit(plan)) return GF_OK;
+  const size_t nnz = rp[n];
+  FrontSystem S;
+  std::vector<int> part;
+  if (S.init(ctx, plan, n, b, {{rp, sizeof(int) * ((size_t)n + 1)}, {ci, sizeof(int) * nnz}, {val, sizeof(double) * nnz}},
+             &part) != GF_OK)
+    return GF_OK;
+  const int *drp = S.at<int>(part[0]), *dci = S.at<int>(part[1]);
+  const double* dv = S.at<double>(part[2]);
+  return S.solve(ctx, n, [&](const Batch& q) { launch_front_csr(q, n, drp, dci, dv, ctx->stream); },
+                 [&](const double* x, double* r, int* bad) { launch_csr_residual(n, drp, dci, dv, S.b.P, x, r, bad, ctx->stream); },
+                 b, done);
+}
+
+// A front solve that host memory does not allow leaves *done false too.
+template <typename Solve> static int front_solve(bool* done, Solve solve) {
+  *done = false;
+  try {
+    return solve();
+  } catch (const std::bad_alloc&) {
+    return GF_OK;
+  }
+}
+int front_band_solve(gf_ctx* ctx, int n, int kl, int ku, const double* ab, int ldab, double* b, bool* done) {
+  return front_solve(done, [&] { return band_on_fronts(ctx, n, kl, ku, ab, ldab, b, done); });
+}
+int front_sparse_solve(gf_ctx* ctx, int n, const int* rp, const int* ci, const double* val, double* b, bool* done) {
+  return front_solve(done, [&] { return sparse_on_fronts(ctx, n, rp, ci, val, b, done); });
 }
 
 // Wide branch of gf_band_solve: the GB array goes into the wide band with
@@ -191,33 +232,10 @@ int gf_sparse_solve(gf_ctx* ctx, int n, const int* row_ptr, const int* col_idx, 
   for (int i = 0; i < n && !wide; ++i)
     for (int k = row_ptr[i]; k < row_ptr[i + 1] && !wide; ++k) wide = std::abs(i - col_idx[k]) > GF_KB;
   if (wide) {
-    NdGraph g;
-    std::vector<int> dptr, dofs(n);
-    csr_graph(n, row_ptr, col_idx, g, dptr);
-    for (int i = 0; i < n; ++i) dofs[i] = i;
-    nd_landmark_fields(g);
-    std::vector<float> place(g.n);
-    for (int v = 0; v < g.n; ++v) place[v] = (float)v;
-    g.field.push_back(std::move(place));
-    const FrontPlan plan = plan_fronts(g, dptr, dofs);
-    if (fronts_fit(plan)) {
-      FrontSystem S;
-      std::vector<int> part;
-      if (S.init(ctx, plan, n, b,
-                 {{row_ptr, sizeof(int) * ((size_t)n + 1)}, {col_idx, sizeof(int) * (size_t)nnz},
-                  {val, sizeof(double) * (size_t)nnz}}, &part) == GF_OK) {
-        const int *rp = S.at<int>(part[0]), *ci = S.at<int>(part[1]);
-        const double* v = S.at<double>(part[2]);
-        bool done = false;
-        const int rc = S.solve(ctx, n, [&](const Batch& q) { launch_front_csr(q, n, rp, ci, v, ctx->stream); },
-                               [&](const double* x, double* r, int* bad) {
-                                 launch_csr_residual(n, rp, ci, v, S.b.P, x, r, bad, ctx->stream);
-                               },
-                               b, &done);
-        if (rc == GF_OK && done && info) *info = 0;
-        if (rc != GF_OK || done) return rc;
-      }
-    }
+    bool done = false;
+    const int rc = gfh::front_sparse_solve(ctx, n, row_ptr, col_idx, val, b, &done);
+    if (rc == GF_OK && done && info) *info = 0;
+    if (rc != GF_OK || done) return rc;
   }
   // a system that the multifrontal LU does not take or not solve to the accuracy that it
   // asks of it, or a narrow band: ordering natural, or reverse Cuthill-McKee on the

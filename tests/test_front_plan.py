@@ -106,3 +106,45 @@ int main() {
 }
 """)
     assert run().stdout == "0"
+
+
+def test_plan_without_threads(compiled):
+    # the dissection's threads are a help, not a need: where a thread cannot be made (its
+    # stack does not fit the address space allowed) the plan is the same
+    run = compiled("threads", r"""
+#include <cstdio>
+#include "gf_front.h"
+int main() {
+  const int m = 90, n = m * m;
+  gfh::NdGraph g;
+  g.n = n;
+  g.ptr.push_back(0);
+  std::vector<int> dptr(1, 0), dofs(2 * n);
+  for (int v = 0; v < n; ++v) {
+    if (v >= m) g.adj.push_back(v - m);
+    if (v % m) g.adj.push_back(v - 1);
+    if (v % m < m - 1) g.adj.push_back(v + 1);
+    if (v + m < n) g.adj.push_back(v + m);
+    g.ptr.push_back((int)g.adj.size());
+    g.w.push_back(2);
+    dptr.push_back(2 * v + 2);
+    dofs[2 * v] = 2 * v;
+    dofs[2 * v + 1] = 2 * v + 1;
+  }
+  gfh::nd_landmark_fields(g);
+  const gfh::FrontPlan P = gfh::plan_fronts(g, dptr, dofs);
+  unsigned long long h = 1469598103934665603ull;
+  for (int p : P.pos) h = (h ^ (unsigned)p) * 1099511628211ull;
+  std::printf("%zu %lld %llu", P.fronts.size(), (long long)P.size, h);
+}
+""")
+
+    def no_threads():
+        import resource
+
+        resource.setrlimit(resource.RLIMIT_STACK, (4 << 30, resource.RLIM_INFINITY))
+        resource.setrlimit(resource.RLIMIT_AS, (1 << 30, 1 << 30))
+
+    free, bound = run(), run(preexec_fn=no_threads)
+    assert free.returncode == 0 and bound.returncode == 0, bound.stderr
+    assert free.stdout == bound.stdout
