@@ -366,3 +366,32 @@ def test_slices_hold_an_exponent_per_64_pivots(gpu_ctx):
     rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.int32)
     x, info = gpu_ctx.sparse_solve(rp, cols.astype(np.int32), A[rows, cols], b)
     assert info == 0 and (np.abs(x - ref) / c).max() <= 1e-12 * (np.abs(ref) / c).max()
+
+
+def test_a_large_system_of_wide_fronts(gpu_ctx):
+    # a hundred full blocks of 530 DOFs, each coupled to the same six: fronts of more own
+    # DOFs than the substitution's partial sums hold at once, with a boundary; a matrix
+    # beyond the pinned staging and a workspace beyond the 512 MB that a context keeps.
+    # Rows dominant by 1.5: forward error n eps cond with cond <= 5, 1e-12
+    rng = np.random.default_rng(3)
+    k, m, h = 100, 530, 6
+    n = k * m + h
+    block = rng.uniform(-1.0, 1.0, (k * m, m + h))
+    own = np.arange(k * m) % m
+    block[np.arange(k * m), own] = 0.0
+    block[np.arange(k * m), own] = 1.5 * np.abs(block).sum(1) + 0.1
+    cols = np.concatenate([np.arange(m)[None] + m * np.arange(k)[:, None], np.full((k, h), k * m) + np.arange(h)], axis=1)
+    hub = rng.uniform(-1.0, 1.0, (h, n))
+    hub[np.arange(h), k * m + np.arange(h)] = 0.0
+    hub[np.arange(h), k * m + np.arange(h)] = 1.5 * np.abs(hub).sum(1) + 0.1
+    ref = rng.normal(size=n)
+    b = np.concatenate([np.einsum("kij,kj->ki", block.reshape(k, m, m + h), ref[cols]).ravel(), hub @ ref])
+    ci = np.concatenate([np.repeat(cols, m, axis=0).ravel(), np.tile(np.arange(n), h)]).astype(np.int32)
+    rp = np.concatenate([np.arange(k * m) * (m + h), k * m * (m + h) + np.arange(h + 1) * n]).astype(np.int32)
+    A = pattern("grid", 5)
+    small = (*to_csr(A), np.ones(len(A)))
+    before, _ = gpu_ctx.sparse_solve(*small)
+    x, info = gpu_ctx.sparse_solve(rp, ci, np.concatenate([block.ravel(), hub.ravel()]), b)
+    assert info == 0 and np.abs(x - ref).max() <= 1e-12 * np.abs(ref).max()
+    after, _ = gpu_ctx.sparse_solve(*small)
+    assert np.array_equal(before, after)
