@@ -4,16 +4,17 @@
 //
 // The right-hand side is column f of every front, so the forward substitution
 // is part of the elimination.  Per height, bottom up:
-//   k_mf_extend   the children's Schur complements added into their parents
-//                 (one launch per child ordinal: the children of a front touch
-//                 common entries)
-//   k_mf_small    fronts of at most MF_SMALL rows: one CTA each, in shared
-//                 memory
+//   k_mf_extend   the children's Schur complements added into the large fronts, all
+//                 children of a front's column by one warp
+//   k_mf_small    fronts up to the height's line (at most MF_SMALL rows): one CTA each,
+//                 in shared memory, the children's complements added as it loads
 //   larger fronts, MF_NB pivots per panel:
-//     k_mf_diag   LU of the panel's diagonal block
+//     k_mf_diag   LU of the first panel's diagonal block
 //     k_mf_trsm   L21 = A21 U11^-1 and U12 = L11^-1 A12
-//     k_mf_panel  the rest of the pivot rows and columns
-//   k_mf_schur    the boundary block, once all pivots are done: C -= L21 U12
+//     k_mf_panel  the rest of the pivot rows and columns, and the LU of the next
+//                 panel's diagonal block
+//   k_mf_schur    the boundary block, once all pivots are done: C -= L21 U12 (the largest
+//                 fronts' in gf_front_t5.cu)
 // and top down
 //   k_mf_back     x of the front's own DOFs from its boundary's.
 // The diagonal of U is stored as its reciprocal.
@@ -528,7 +529,8 @@ template <typename T, int L> __global__ void __launch_bounds__(128) k_mf_trsm(Ba
 // them factors it (mf_block_lu) while the others run: a launch per panel and 14 us less
 // on the chain of panels.  On one CTA the tile takes 8 us of its SM's FP64 rate, all of
 // them on the chain where a height has few fronts (24 us a panel with one, 17 with
-// four).
+// four).  FP32 fronts take one: their tile is a few us in either form (24x24x2 mixed
+// plate 10.49 ms with one CTA and with four).
 constexpr int MF_PANEL_THREADS = 256;
 static_assert(MF_PANEL_THREADS == MF_DIAG_THREADS, "the panel's first CTA factors a block");
 template <typename T, int C>

@@ -29,13 +29,14 @@ struct Front {
   int slot;    // structure
   int dof0;    // its first own DOF in the elimination order (batch-wide index)
   int bnd;     // boundary DOFs (batch-wide elimination positions, ascending): bnd[bnd .. bnd + f - s)
-  int rel;     // the parent's front index of every boundary DOF: rel[rel .. rel + f - s)
+  int rel;     // (host) the parent's front index of every boundary DOF: rel[rel .. rel + f - s)
   int parent;  // -1: a root
   int kid0, kid1;  // its children: kids[kid0 .. kid1)
 };
 
 // Fronts up to this size may take one CTA for the elimination, the whole matrix
-// in its shared memory (k_mf_small); the others run panel by panel on many.
+// in its shared memory (k_mf_small); the others run panel by panel on many.  The line of
+// a height is at or below it (small_limit, gf_order.cu).
 constexpr int MF_SMALL = 96;
 constexpr int MF_NB = 32;  // pivots per panel of a large front
 // Shared memory of the substitutions beside their static part (gf_front.cu), and the rows
@@ -88,10 +89,8 @@ struct FrontSchedule {
 
 // Device arrays; the schedule is host memory owned by the batch.
 struct FrontData {
-  int n_fronts;
   Front* fronts;
   int* bnd;
-  int* rel;
   Front* list;      // the fronts by height
   int2* ext_jobs;   // (front, column block)
   int2* schur_jobs; // (front, row tile | column tile << 16), tiles of FrontLevel::tile rows
@@ -137,7 +136,6 @@ struct FrontPlan {
   std::vector<int> pos;        // DOF -> elimination position
   std::vector<int> dof_front;  // elimination position -> front
   int64_t size = 0;            // doubles
-  double flops = 0.0;
 };
 
 // Graph of a CSR matrix's symmetrised pattern, consecutive rows with the same columns (the

@@ -89,7 +89,6 @@ struct FrontSystem {
     b.sh.n_wide = 1;
     b.sh.wide_structs = at<int>(p_ws);
     gf::FrontData& d = b.sh.mf;
-    d.n_fronts = (int)fb.fronts.size();
     d.fronts = at<gf::Front>(p_fr);
     d.bnd = at<int>(p_bnd);
     d.kids = at<int2>(p_kids);

@@ -1148,8 +1148,7 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
       FrontBuild fb;
       join_fronts(plans, wide_structs, offs, n, dof_off, B->opts.wide_update == GF_WIDE_TENSOR, fb);
       FrontData& md = sd.mf;
-      md.n_fronts = (int)fb.fronts.size();
-      if (!upload(B, &md.fronts, fb.fronts) || !upload(B, &md.bnd, fb.bnd) || !upload(B, &md.rel, fb.rel) ||
+      if (!upload(B, &md.fronts, fb.fronts) || !upload(B, &md.bnd, fb.bnd) ||
           !upload(B, &md.list, fb.list) || !upload(B, &md.ext_jobs, fb.ext_jobs) ||
           !upload(B, &md.schur_jobs, fb.schur_jobs) || !upload(B, &md.pos, fb.pos) ||
           !upload(B, &md.dof_front, fb.dof_front) ||

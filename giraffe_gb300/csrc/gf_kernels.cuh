@@ -92,12 +92,12 @@ struct ProfScope {
   }
 };
 
-// The wide band holds K_AA in the assembly view only (gf_batch_assemble, the
-// Newton-iteration boundary).
 // Row of a Shell_1 element's 27 DOFs for DOF k of its local node a: translations of all
 // six nodes, rotations of the midside nodes only (-1: none).
 __host__ __device__ inline int shell_dof(int a, int k) { return k < 3 ? 3 * a + k : a < 3 ? -1 : 18 + 3 * (a - 3) + k - 3; }
 
+// The wide band holds K_AA in the assembly view only (gf_batch_assemble, the
+// Newton-iteration boundary).
 __host__ __device__ inline bool wide_band_filled(const Batch& b) { return b.full_band; }
 
 void launch_iteration(const Batch& b, cudaStream_t st, bool commit_kernels = true, LaunchProf* prof = nullptr);

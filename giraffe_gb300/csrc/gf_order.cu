@@ -353,8 +353,6 @@ FrontPlan plan_fronts(const NdGraph& g, const std::vector<int>& dptr, const std:
     F.off = P.size;
     P.size += ((int64_t)F.ld * (F.f + 1) + 31) / 32 * 32;
     for (int d = F.dof0; d < F.dof0 + F.s; ++d) P.dof_front[d] = k;
-    const double s = F.s, u = F.f - F.s;
-    P.flops += 2.0 * (s * s * s / 3.0 + s * s * u + s * u * u);
     if (F.parent >= 0) P.height[F.parent] = std::max(P.height[F.parent], P.height[k] + 1);
   }
   // front index, in the parent, of every boundary DOF
@@ -510,8 +508,13 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
       V.s_at.push_back(s);
     }
     V.schur_off = (int)out.schur_jobs.size();
-    // 32 x 32 tiles, or 16 x 16 while those leave SMs idle in the last wave: a tile
-    // holds an SM's FP64 units for its whole product
+    // 32 x 32 tiles, or 16 x 16 where their waves are shorter: a tile holds an SM's FP64
+    // units for its whole product, four parts of work for the large one and one for the
+    // small, which takes 1.3 with its operands' loads for a quarter of the products.  16
+    // everywhere: FP32 fronts of the 64x64x2 plate 122.0 -> 123.5 ms (whole waves of either);
+    // 32 everywhere: four vibrating plates 18.1 -> 18.7 ms, one 6x6x2 plate 4.02 -> 4.25
+    // (a part of one wave); batches of 16 to 128 plates and the FP64 64x64x2 plate
+    // within 1 % either way
     auto on_t5 = [&](int k) {
       const double u = out.fronts[k].f - out.fronts[k].s;
       return tensor && out.fronts[k].s * u * u >= gf::MF_T5_WORK;
