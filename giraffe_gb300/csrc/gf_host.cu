@@ -718,7 +718,11 @@ int build_batch(gf_batch* B, int n, const gf_model_desc* models) {
   size_t work = 0;
   for (int s = 0; s < n; ++s) work += (size_t)std::max(models[s].n_nodes, 0) + std::max(models[s].n_beams, 0) +
                                       std::max(models[s].n_shells, 0);
-  parallel_structures(n, work, [&](int s) { plan_structure(models[s], s, !B->band_view, plan[s]); });
+  // a shell's share of its structure's numbering and dissection, 3 to 4 us, is worth some
+  // forty beam nodes (16 plates of 16x16x2 on one thread 30 ms, on sixteen 4)
+  size_t plan_work = work;
+  for (int s = 0; s < n && !B->band_view; ++s) plan_work += 40 * (size_t)std::max(models[s].n_shells, 0);
+  parallel_structures(n, plan_work, [&](int s) { plan_structure(models[s], s, !B->band_view, plan[s]); });
   for (int s = 0; s < n; ++s)
     if (!plan[s].err.empty()) {
       set_err(ctx, "%s", plan[s].err.c_str());

@@ -426,9 +426,21 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
   out.base.assign(n_struct, 0);
   out.size.assign(n_struct, 0);
   std::vector<int> height;
+  {
+    size_t nf = 0, nb = 0;
+    for (const FrontPlan* P : plans) {
+      nf += P->fronts.size();
+      nb += P->bnd.size();
+    }
+    out.fronts.reserve(nf);
+    height.reserve(nf);
+    out.bnd.resize(nb);
+    out.rel.reserve(nb);
+  }
+  int b0 = 0;
   for (size_t q = 0; q < plans.size(); ++q) {
     const FrontPlan& P = *plans[q];
-    const int f0 = (int)out.fronts.size(), b0 = (int)out.bnd.size(), d0 = dof_off[q];
+    const int f0 = (int)out.fronts.size(), d0 = dof_off[q];
     out.base[slots[q]] = out.total;
     out.size[slots[q]] = P.size;
     for (gf::Front F : P.fronts) {
@@ -440,7 +452,8 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
       if (F.parent >= 0) F.parent += f0;
       out.fronts.push_back(F);
     }
-    for (int d : P.bnd) out.bnd.push_back(d + d0);
+    for (size_t i = 0; i < P.bnd.size(); ++i) out.bnd[b0 + i] = P.bnd[i] + d0;
+    b0 += (int)P.bnd.size();
     out.rel.insert(out.rel.end(), P.rel.begin(), P.rel.end());
     height.insert(height.end(), P.height.begin(), P.height.end());
     for (size_t i = 0; i < P.pos.size(); ++i) out.pos[d0 + i] = P.pos[i] + d0;
@@ -450,22 +463,37 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
   const int nf = (int)out.fronts.size();
   int nl = 0;
   for (int h : height) nl = std::max(nl, h + 1);
-  std::vector<std::vector<int>> at(nl), kids(nf);
+  std::vector<std::vector<int>> at(nl);
+  auto parent = [&](int k) { return out.fronts[k].f > out.fronts[k].s ? out.fronts[k].parent : -1; };
+  size_t n_inv = 0;
   for (int k = 0; k < nf; ++k) {
     at[height[k]].push_back(k);
-    if (out.fronts[k].parent >= 0 && out.fronts[k].f > out.fronts[k].s) kids[out.fronts[k].parent].push_back(k);
+    out.fronts[k].kid0 = out.fronts[k].kid1 = 0;
   }
-  for (int k = 0; k < nf; ++k) {
-    out.fronts[k].kid0 = (int)out.kids.size();
-    for (int c : kids[k]) {
-      const gf::Front& C = out.fronts[c];
-      out.kids.push_back(make_int2(c, (int)out.inv.size()));
-      out.inv.resize(out.inv.size() + out.fronts[k].f, -1);
-      int* inv = out.inv.data() + out.inv.size() - out.fronts[k].f;
-      for (int i = 0; i < C.f - C.s; ++i) inv[out.rel[C.rel + i]] = i;
+  for (int k = 0; k < nf; ++k)
+    if (parent(k) >= 0) {
+      ++out.fronts[parent(k)].kid1;
+      n_inv += out.fronts[parent(k)].f;
     }
-    out.fronts[k].kid1 = (int)out.kids.size();
+  int n_kids = 0;
+  for (int k = 0; k < nf; ++k) {
+    const int n = out.fronts[k].kid1;
+    out.fronts[k].kid0 = out.fronts[k].kid1 = n_kids;
+    n_kids += n;
   }
+  out.kids.resize(n_kids);
+  for (int k = 0; k < nf; ++k)
+    if (parent(k) >= 0) out.kids[out.fronts[parent(k)].kid1++].x = k;
+  out.inv.assign(n_inv, -1);
+  n_inv = 0;
+  for (int k = 0; k < nf; ++k)
+    for (int q = out.fronts[k].kid0; q < out.fronts[k].kid1; ++q) {
+      const gf::Front& C = out.fronts[out.kids[q].x];
+      out.kids[q].y = (int)n_inv;
+      int* inv = out.inv.data() + n_inv;
+      for (int i = 0; i < C.f - C.s; ++i) inv[out.rel[C.rel + i]] = i;
+      n_inv += out.fronts[k].f;
+    }
   out.dof_at.assign(n_dofs, -1);
   for (int i = 0; i < n_dofs; ++i)
     if (out.pos[i] >= 0) out.dof_at[out.pos[i]] = i;
@@ -492,7 +520,7 @@ void join_fronts(const std::vector<const FrontPlan*>& plans, const std::vector<i
     for (int k : big) out.list.push_back(out.fronts[k]);
     V.ext_off = (int)out.ext_jobs.size();
     for (int k : big)
-      if (!kids[k].empty())
+      if (out.fronts[k].kid1 > out.fronts[k].kid0)
         for (int c = 0; c <= out.fronts[k].f; c += 8) out.ext_jobs.push_back(make_int2(k, c));
     V.ext_cnt = (int)out.ext_jobs.size() - V.ext_off;
     const int panels = big.empty() ? 0 : (out.fronts[big[0]].s + gf::MF_NB - 1) / gf::MF_NB;
