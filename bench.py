@@ -34,9 +34,9 @@ import numpy as np  # noqa: E402
 
 METRIC = "Newton solves/sec (batched static Beam_1 chains, FP64, converged load steps)"
 UNIT = "Newton solves/s"
-# DRAM bytes per element mount of k_beam_tangent, from one ncu capture on 128
-# chains: (54.9 MB read + 173.1 MB written) / 79,322 elements
-TANGENT_DRAM_BYTES_PER_ELEMENT = (55.088384e6 + 202.853120e6) / 79322
+# DRAM bytes per element mount of k_beam_tangent, from one launch on the 512-chain
+# workload under ncu: (206.2 MB read + 270.7 MB written) / 299,042 elements
+TANGENT_DRAM_BYTES_PER_ELEMENT = (206.164736e6 + 270.698240e6) / 299042
 # FP64 flops of one element in k_beam_tangent (an FMA counts two)
 TANGENT_FLOPS = 3270.0
 
@@ -720,7 +720,7 @@ def run_ours(args, rank, world):
                 "frac": achieved / fp64.value,
                 "traffic": TANGENT_DRAM_BYTES_PER_ELEMENT * mounts_per_launch,
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_beam_tangent "
-                                  "launch on 128 chains (profiles/k_beam_tangent_128chains.md): "
+                                  "launch on 512 chains (profiles/launches_batched_static_512chains.md): "
                                   f"{TANGENT_DRAM_BYTES_PER_ELEMENT:.0f} B per element, scaled by the "
                                   f"{mounts_per_launch:.0f} element mounts of an average launch here",
                 "note": "FP64 CUDA-core bound (no HBM or tensor-core bound applies: per-element 18x18 algebra); "
