@@ -1012,7 +1012,7 @@ __global__ void k_mf_band(Batch b, int n, int kl, int ku, int ldab, const double
 
 // r = rhs - A x and whether a row's backward error is above the limit; a non-finite
 // one is.  mx: the largest |x_j| of the row's columns as its bits.
-__device__ __forceinline__ void mf_judge(int i, double rhs, double ax, double sum, unsigned long long mx, double* r, int* bad) {
+__device__ __forceinline__ void mf_row_error(int i, double rhs, double ax, double sum, unsigned long long mx, double* r, int* bad) {
   const double res = rhs - ax, d = fma(sum, __longlong_as_double((long long)mx), fabs(rhs));
   r[i] = res;
   if (!(fabs(res) <= MF_ERROR_LIMIT * d && d <= DBL_MAX)) *bad = 1;
@@ -1040,7 +1040,7 @@ __global__ void __launch_bounds__(128) k_csr_residual(int n, const int* rp, cons
     sum += __shfl_xor_sync(0xffffffffu, sum, o);
     mx = max(mx, (unsigned long long)__shfl_xor_sync(0xffffffffu, mx, o));
   }
-  if (i < n && lane == 0) mf_judge(i, rhs[i], ax, sum, mx, r, bad);
+  if (i < n && lane == 0) mf_row_error(i, rhs[i], ax, sum, mx, r, bad);
 }
 
 // A thread a row of LAPACK GB columns.
@@ -1058,7 +1058,7 @@ __global__ void __launch_bounds__(64) k_band_residual(int n, int kl, int ku, int
     sum += fabs(a);
     mx = max(mx, mf_mag(xj));
   }
-  mf_judge(i, rhs[i], ax, sum, mx, r, bad);
+  mf_row_error(i, rhs[i], ax, sum, mx, r, bad);
 }
 
 __global__ void k_mf_add(int n, const double* d, double* x) {

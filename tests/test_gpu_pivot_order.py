@@ -81,3 +81,22 @@ def test_grid_with_a_weak_row(gpu_ctx, weak):
         assert info == 0, r
         res, d = np.abs(b - B @ x), np.abs(B).sum(1) * np.abs(x).max() + np.abs(b)
         assert (res / d).max() <= 2.0 ** -44, r
+
+
+@pytest.mark.parametrize("g,shift", [(100, 0.0), (60, 0.37)])
+def test_refinement_on_the_fronts(gpu_ctx, g, shift):
+    # five-point Laplacians, one of them indefinite: the tensor-core products leave rows of 36
+    # and 6,000 roundings, refined with the factor to within the limit
+    n = g * g
+    at = np.arange(n)
+    cols = np.stack([at - g, at - 1, at, at + 1, at + g], axis=1)
+    live = np.stack([at >= g, at % g > 0, at >= 0, at % g < g - 1, at < n - g], axis=1)
+    vals = np.where(np.arange(5) == 2, 4.0 - shift, -1.0) * live
+    b = np.random.default_rng(5).normal(size=n)
+    rp = np.concatenate([[0], np.cumsum(live.sum(1))]).astype(np.int32)
+    x, info = gpu_ctx.sparse_solve(rp, cols[live].astype(np.int32), vals[live], b)
+    xc = np.where(live, x[np.clip(cols, 0, n - 1)], 0.0).astype(np.longdouble)
+    r = np.abs(b - (vals * xc).sum(1))
+    d = np.abs(vals).sum(1) * np.abs(xc).max(1) + np.abs(b)
+    # the limit, and the residual's own five roundings
+    assert info == 0 and float((r / d).max()) <= 2.0 ** -49 + 5 * 2.0 ** -53
